@@ -1008,72 +1008,306 @@ __global__ void __launch_bounds__(256) pool2d_bwd_kernel(const T* __restrict__ x
 }
 
 // ============================================================== direct conv2d NHWC x RSCF (small C)
-// y[n,oh,ow,f] = sum_{r,s,c} x[n, oh*sh - pt + r*dh, ow*sw - pl + s*dw, c] * w[r,s,c,f] (+ bias[f])
+// y[n,oh,ow,f] = sum_{r,s,c} x[n, oh*sh - pt + r, ow*sw - pl + s, c] * w[r,s,c,f] (+ bias[f])
+//
+// An implicit matrix product over k = (r, s, c) in fp32 FMAs: a block owns 2 * PG output positions and
+// 4 * FG channels, each thread a 2 x 4 tile of them. CONV_KC values of k are staged at a time (the gathered
+// input and the filter rows, as floats), so a thread does 8 FMAs for two shared loads; one thread per
+// output value with both operands from global memory was bound by its two loads per FMA. (A 4 x 4 tile
+// leaves too few warps: 50,000 threads for 256 images of 14 x 14 x 16.)
+// Measured (fp32, 3x3): 256 x 28 x 28 x 1 -> 16 83 -> 19 us, 256 x 14 x 14 x 16 -> 32 133 -> 38 us; still some
+// five times its FMAs' time, which goes to staging the gathered input.
+// The terms are added in the same order (bias, then k ascending), so fp32 results are unchanged.
+// A padded position counts as absent, not as 0 * w: where the staged filter holds an infinity or a NaN
+// the block falls back to conv_point, which skips such positions.
+struct ConvGeom {
+  int N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl;
+};
+
 template <typename T>
+__device__ __noinline__ float conv_point(const T* __restrict__ x, const T* __restrict__ w, float acc, const ConvGeom g,
+                                         long long m, int f) {
+  const int ow = (int)(m % g.OW);
+  const long long q = m / g.OW;
+  const int oh = (int)(q % g.OH), n = (int)(q / g.OH);
+  for (int r = 0; r < g.R; ++r) {
+    const int ih = oh * g.sh - g.pt + r;
+    if (ih < 0 || ih >= g.H) continue;
+    for (int s = 0; s < g.S; ++s) {
+      const int iw = ow * g.sw - g.pl + s;
+      if (iw < 0 || iw >= g.W) continue;
+      if (!NB_IN_BOUNDS(NB_SITE_CONV_INPUT, (((size_t)n * g.H + ih) * g.W + iw) * g.C, (size_t)g.N * g.H * g.W * g.C)) continue;
+      const T* xp = x + (((size_t)n * g.H + ih) * g.W + iw) * g.C;
+      const T* wp = w + ((size_t)(r * g.S + s) * g.C) * g.F + f;
+      for (int c = 0; c < g.C; ++c) acc = fmaf(to_f<T>(xp[c]), to_f<T>(wp[(size_t)c * g.F]), acc);
+    }
+  }
+  return acc;
+}
+
+// Four consecutive elements (16 bytes of fp32, 8 of bf16).
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 r = *reinterpret_cast<const float4*>(p);
+  v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+}
+__device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xffff0000u);
+  v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xffff0000u);
+}
+
+constexpr int CONV_KC = 32;      // values of k staged at a time
+
+template <typename T, int FG, bool VEC>
 __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                           const T* __restrict__ bias, T* __restrict__ y, int N, int H,
-                                                           int W, int C, int R, int S, int F, int OH, int OW, int sh,
-                                                           int sw, int pt, int pl) {
-  const size_t total = (size_t)N * OH * OW * F;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int f = i % F;
-    size_t r_ = i / F;
-    const int ow = r_ % OW; r_ /= OW;
-    const int oh = r_ % OH;
-    const int n = r_ / OH;
-    float acc = bias ? to_f<T>(bias[f]) : 0.f;
-    for (int r = 0; r < R; ++r) {
-      const int ih = oh * sh - pt + r;
-      if (ih < 0 || ih >= H) continue;
-      for (int s = 0; s < S; ++s) {
-        const int iw = ow * sw - pl + s;
-        if (iw < 0 || iw >= W) continue;
-        if (!NB_IN_BOUNDS(NB_SITE_CONV_INPUT, (((size_t)n * H + ih) * W + iw) * C, (size_t)N * H * W * C)) continue;
-        const T* xp = x + (((size_t)n * H + ih) * W + iw) * C;
-        const T* wp = w + ((size_t)(r * S + s) * C) * F + f;
-        for (int c = 0; c < C; ++c) acc += to_f<T>(xp[c]) * to_f<T>(wp[(size_t)c * F]);
+                                                           const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g) {
+  constexpr int PG = 128 / FG, MT = 2 * PG, FT = 4 * FG, PER = (MT + 127) / 128, KSTEP = MT < 128 ? 128 / MT : 1;
+  __shared__ __align__(16) float xs[CONV_KC][MT + 4];
+  __shared__ __align__(16) float ws[CONV_KC][FT];
+  __shared__ int krs[CONV_KC], koff[CONV_KC];       // (r << 16 | s) and the offset of (r, s, c) from a window's first pixel
+  const int tid = threadIdx.x;
+  const long long positions = (long long)g.N * g.OH * g.OW;
+  const long long m0 = (long long)blockIdx.x * MT;
+  const int f0 = blockIdx.y * FT;
+  const int K = g.R * g.S * g.C;
+  // the positions whose input this thread stages
+  int ih0[PER], iw0[PER];
+  long long base[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const long long m = m0 + (tid % (MT < 128 ? MT : 128)) + j * 128;
+    ih0[j] = -0x40000000;                            // a position past the end: every row of its window is out of range
+    iw0[j] = 0;
+    base[j] = 0;
+    if (m < positions) {
+      const int ow = (int)(m % g.OW);
+      const long long q = m / g.OW;
+      const int oh = (int)(q % g.OH);
+      ih0[j] = oh * g.sh - g.pt;
+      iw0[j] = ow * g.sw - g.pl;
+      base[j] = (((q / g.OH) * g.H + ih0[j]) * g.W + iw0[j]) * g.C;
+    }
+  }
+  const int fg = tid % FG, pg = tid / FG;
+  float acc[2][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int f = f0 + fg * 4 + j;
+    const float b = bias && f < g.F ? to_f<T>(bias[f]) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) acc[i][j] = b;
+  }
+  int odd = 0;                                       // a filter value that is not finite was staged
+  for (int k0 = 0; k0 < K; k0 += CONV_KC) {
+    const int kn = min(CONV_KC, K - k0);
+    __syncthreads();
+    if (tid < kn) {
+      const int k = k0 + tid, rs = k / g.C, r = rs / g.S;
+      krs[tid] = r << 16 | (rs - r * g.S);
+      koff[tid] = (r * g.W + (rs - r * g.S)) * g.C + (k - rs * g.C);
+    }
+    for (int e = tid; e < kn * FT; e += 128) {
+      const int k = e / FT, f = f0 + e % FT;
+      const float v = f < g.F ? to_f<T>(w[(size_t)(k0 + k) * g.F + f]) : 0.f;
+      odd |= !isfinite(v);
+      ws[k][e % FT] = v;
+    }
+    __syncthreads();
+    constexpr int KV = VEC ? 4 : 1;                  // VEC (C % 4 == 0): four channels of one pixel per load
+#pragma unroll 8
+    for (int k = (MT < 128 ? tid / MT : 0) * KV; k < kn; k += KSTEP * KV) {
+      const int rs = krs[k], off = koff[k];
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int ih = ih0[j] + (rs >> 16), iw = iw0[j] + (rs & 0xffff);
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W &&
+            NB_IN_BOUNDS(NB_SITE_CONV_INPUT, base[j] + off + KV - 1, (long long)g.N * g.H * g.W * g.C)) {
+          if (VEC) load4(x + base[j] + off, v);
+          else v[0] = to_f<T>(x[base[j] + off]);
+        }
+#pragma unroll
+        for (int i = 0; i < KV; ++i) xs[k + i][(tid % (MT < 128 ? MT : 128)) + j * 128] = v[i];
       }
     }
-    y[i] = from_f<T>(acc);
+    __syncthreads();
+    auto step = [&](int k) {
+      const float2 a = *reinterpret_cast<const float2*>(&xs[k][pg * 2]);
+      const float4 b = *reinterpret_cast<const float4*>(&ws[k][fg * 4]);
+      const float av[2] = {a.x, a.y}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    };
+    if (kn == CONV_KC) {
+#pragma unroll 8
+      for (int k = 0; k < CONV_KC; ++k) step(k);
+    } else {
+      for (int k = 0; k < kn; ++k) step(k);
+    }
+  }
+  odd = __syncthreads_or(odd);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const long long m = m0 + pg * 2 + i;
+    if (m >= positions) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int f = f0 + fg * 4 + j;
+      if (f >= g.F) break;
+      if (odd) acc[i][j] = conv_point<T>(x, w, bias ? to_f<T>(bias[f]) : 0.f, g, m, f);
+      y[m * g.F + f] = from_f<T>(acc[i][j]);
+    }
   }
 }
 
 // Filter gradient of the direct convolution (small channel counts, fp32 or bf16):
 //   dw[r,s,c,f] = sum_{n,oh,ow} x[n, oh*sh - pt + r, ow*sw - pl + s, c] * dy[n,oh,ow,f]
-// One block per (r, s, c) and tile of 32 output channels. Lane = output channel (coalesced reads
-// of dy, one broadcast read of x per position), the 8 warps split the N*OH*OW positions and are
-// summed through shared memory: plain stores, no atomics, deterministic.
-template <typename T>
-__global__ void __launch_bounds__(256) conv2d_wgrad_direct_kernel(const T* __restrict__ x, const T* __restrict__ dy,
-                                                                 T* __restrict__ dw, int N, int H, int W, int C, int R,
-                                                                 int S, int F, int OH, int OW, int sh, int sw, int pt,
-                                                                 int pl) {
-  __shared__ float part[8][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int f = blockIdx.y * 32 + lane;
-  int rsc = blockIdx.x;
-  const int c = rsc % C; rsc /= C;
-  const int s = rsc % S;
-  const int r = rsc / S;
-  const long long positions = (long long)N * OH * OW;
-  float acc = 0.f;
-  for (long long p = warp; p < positions; p += 8) {
-    const int ow = (int)(p % OW);
-    long long q = p / OW;
-    const int oh = (int)(q % OH);
-    const int n = (int)(q / OH);
-    const int ih = oh * sh - pt + r, iw = ow * sw - pl + s;
-    if (ih < 0 || ih >= H || iw < 0 || iw >= W) continue;
-    const float xv = to_f<T>(x[(((size_t)n * H + ih) * W + iw) * C + c]);
-    if (f < F) acc += xv * to_f<T>(dy[(size_t)p * F + f]);
+// The same implicit product with the output positions as the summed index, which is long (N * OH * OW)
+// while the result is tiny: the positions are split over gridDim.z blocks, each writing its fp32 partial
+// sums to part[z][k][f], and fold_slices_kernel adds those in a fixed order (no atomics:
+// deterministic). Inside a block the 128 threads are SL slices of KG x FG threads; each thread owns
+// 4 x 4 values of (k, f) and its slice takes every SL-th position. One block per (r, s, c), as it was
+// before, left 9 blocks walking 200,000 positions for a 3x3 filter over one plane. Measured with the sizes
+// above: 15.8 ms -> 38 us and 3.5 ms -> 42 us.
+// Padded positions are absent (see above): a chunk whose dy holds an infinity or a NaN is added by the
+// branch that tests every term.
+constexpr int WG_MC = 64;        // positions staged at a time
+
+template <typename T, int KG, int FG, bool VEC>
+__global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __restrict__ x, const T* __restrict__ dy,
+                                                                 float* __restrict__ part, const ConvGeom g,
+                                                                 long long per_block) {
+  constexpr int SL = 128 / (KG * FG), KT = 4 * KG, FT = 4 * FG;
+  constexpr int RED = SL > 1 ? 128 * 16 : 4, STAGE = WG_MC * (KT + FT);
+  __shared__ __align__(16) float sm[RED > STAGE ? RED : STAGE];
+  __shared__ int krs[KT], koff[KT];
+  __shared__ int mh[WG_MC], mw[WG_MC];
+  __shared__ long long mb[WG_MC];
+  float (*xs)[KT] = reinterpret_cast<float (*)[KT]>(sm);
+  float (*ds)[FT] = reinterpret_cast<float (*)[FT]>(sm + WG_MC * KT);
+  const int tid = threadIdx.x;
+  const int K = g.R * g.S * g.C, k0 = blockIdx.x * KT, f0 = blockIdx.y * FT;
+  const long long positions = (long long)g.N * g.OH * g.OW;
+  const long long p0 = blockIdx.z * per_block, p1 = min(positions, p0 + per_block);
+  if (tid < KT) {
+    const int k = min(k0 + tid, K - 1), rs = k / g.C, r = rs / g.S;
+    krs[tid] = r << 16 | (rs - r * g.S);
+    koff[tid] = (r * g.W + (rs - r * g.S)) * g.C + (k - rs * g.C);
   }
-  part[warp][lane] = acc;
-  __syncthreads();
-  if (warp == 0 && f < F) {
-    float t = 0.f;
+  const int fg = tid % FG, kg = (tid / FG) % KG, sl = tid / (FG * KG);
+  float acc[4][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t += part[i][lane];
-    dw[((size_t)(r * S + s) * C + c) * F + f] = from_f<T>(t);
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  for (long long pc = p0; pc < p1; pc += WG_MC) {
+    const int mn = (int)min((long long)WG_MC, p1 - pc);
+    __syncthreads();
+    if (tid < WG_MC) {
+      const long long m = pc + min(tid, mn - 1);
+      const int ow = (int)(m % g.OW);
+      const long long q = m / g.OW;
+      const int oh = (int)(q % g.OH);
+      mh[tid] = oh * g.sh - g.pt;
+      mw[tid] = ow * g.sw - g.pl;
+      mb[tid] = (((q / g.OH) * g.H + mh[tid]) * g.W + mw[tid]) * g.C;
+    }
+    int odd = 0;
+#pragma unroll 8
+    for (int e = tid; e < WG_MC * FT; e += 128) {
+      const int m = e / FT, f = f0 + e % FT;
+      const float v = m < mn && f < g.F ? to_f<T>(dy[(pc + m) * g.F + f]) : 0.f;
+      odd |= !isfinite(v);
+      ds[m][e % FT] = v;
+    }
+    odd = __syncthreads_or(odd);
+    constexpr int KV = VEC ? 4 : 1;                  // VEC (C % 4 == 0): four channels of one pixel per load
+#pragma unroll 8
+    for (int e = tid; e < WG_MC * KT / KV; e += 128) {
+      const int m = e / (KT / KV), k = e % (KT / KV) * KV, rs = krs[k];
+      const int ih = mh[m] + (rs >> 16), iw = mw[m] + (rs & 0xffff);
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (m < mn && k0 + k < K && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W &&
+          NB_IN_BOUNDS(NB_SITE_CONV_INPUT, mb[m] + koff[k] + KV - 1, (long long)g.N * g.H * g.W * g.C)) {
+        if (VEC) load4(x + mb[m] + koff[k], v);
+        else v[0] = to_f<T>(x[mb[m] + koff[k]]);
+      }
+      if (VEC) *reinterpret_cast<float4*>(&xs[m][k]) = make_float4(v[0], v[1], v[2], v[3]);
+      else xs[m][k] = v[0];
+    }
+    __syncthreads();
+    if (!odd) {
+#pragma unroll 8
+      for (int m = sl; m < WG_MC; m += SL) {
+        const float4 a = *reinterpret_cast<const float4*>(&xs[m][kg * 4]);
+        const float4 b = *reinterpret_cast<const float4*>(&ds[m][fg * 4]);
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      }
+    } else {
+      for (int m = sl; m < mn; m += SL)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rs = krs[kg * 4 + i], ih = mh[m] + (rs >> 16), iw = mw[m] + (rs & 0xffff);
+          if (ih < 0 || ih >= g.H || iw < 0 || iw >= g.W) continue;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[m][kg * 4 + i], ds[m][fg * 4 + j], acc[i][j]);
+        }
+    }
+  }
+  if (SL > 1) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sm[(i * 4 + j) * 128 + tid] = acc[i][j];
+    __syncthreads();
+    if (sl != 0) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < SL; ++q) t += sm[(i * 4 + j) * 128 + q * (KG * FG) + tid];
+        acc[i][j] = t;
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = k0 + kg * 4 + i;
+    if (k >= K) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int f = f0 + fg * 4 + j;
+      if (f < g.F) part[((size_t)blockIdx.z * K + k) * g.F + f] = acc[i][j];
+    }
+  }
+}
+// out[i] = sum_z part[z][i], fp32 slices of n: 32 results per block, its 8 warps take every 8th slice.
+template <typename T>
+__global__ void __launch_bounds__(256) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
+                                                         int slices) {
+  __shared__ float sh[8][32];
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+  const size_t i = (size_t)blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (i < n) {
+#pragma unroll 8
+    for (int z = wq; z < slices; z += 8) s += part[(size_t)z * n + i];
+  }
+  sh[wq][lane] = s;
+  __syncthreads();
+  if (wq == 0 && i < n) {
+    s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += sh[q][lane];
+    out[i] = from_f<T>(s);
   }
 }
 
@@ -1404,11 +1638,17 @@ int nb_pool2d_select(const void* x, const void* t, void* y, int N, int H, int W,
 
 int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int R, int S,
                      int F, int OH, int OW, int sh, int sw, int pt, int pl, int dtype, void* stream) {
-  const size_t total = (size_t)N * OH * OW * F;
-  if (!total) return 0;
-  const int grid = grid_for(total, 128, 148 * 32);
-  if (dtype) conv2d_direct_kernel<bf16><<<grid, 128, 0, STREAM>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl);
-  else conv2d_direct_kernel<float><<<grid, 128, 0, STREAM>>>((const float*)x, (const float*)w, (const float*)bias, (float*)y, N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl);
+  const size_t positions = (size_t)N * OH * OW;
+  if (!positions || !F) return 0;
+  const ConvGeom g{N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl};
+  // the narrowest channel tile that holds F, so that lanes of absent channels are few
+  const bool vec = C % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & (dtype ? 7 : 15)) == 0;
+#define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<dim3((unsigned)((positions + 256 / FG - 1) / (256 / FG)), (F + 4 * FG - 1) / (4 * FG)), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g)
+#define CONV(T, FG) do { if (vec) CONV_V(T, FG, true); else CONV_V(T, FG, false); } while (0)
+  if (dtype) { if (F <= 8) CONV(bf16, 2); else if (F <= 16) CONV(bf16, 4); else CONV(bf16, 8); }
+  else { if (F <= 8) CONV(float, 2); else if (F <= 16) CONV(float, 4); else CONV(float, 8); }
+#undef CONV
+#undef CONV_V
   return CHECK_LAUNCH();
 }
 
@@ -1421,12 +1661,39 @@ int nb_sum_slices(const float* part, void* out, long long n, int slices, int dty
   return CHECK_LAUNCH();
 }
 
-int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, int N, int H, int W, int C, int R, int S, int F,
+// Position slices of the filter gradient: enough blocks for four per SM, at least 256 positions each.
+int nb_conv2d_wgrad_slices(long long positions, int K, int F) {
+  const int kt = K <= 16 ? 16 : K <= 32 ? 32 : 64, ft = F <= 16 ? 16 : 32;
+  const long long tiles = (long long)((K + kt - 1) / kt) * ((F + ft - 1) / ft);
+  long long z = (148 * 4 + tiles - 1) / tiles;
+  if (z > (positions + 255) / 256) z = (positions + 255) / 256;
+  return (int)(z < 1 ? 1 : z);
+}
+// part: fp32 scratch of nb_conv2d_wgrad_slices(N * OH * OW, R * S * C, F) * R * S * C * F elements.
+int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part, int N, int H, int W, int C, int R, int S, int F,
                            int OH, int OW, int sh, int sw, int pt, int pl, int dtype, void* stream) {
-  if ((size_t)R * S * C * F == 0) return 0;
-  const dim3 grid(R * S * C, (F + 31) / 32);
-  if (dtype) conv2d_wgrad_direct_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (const bf16*)dy, (bf16*)dw, N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl);
-  else conv2d_wgrad_direct_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (const float*)dy, (float*)dw, N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl);
+  const size_t n = (size_t)R * S * C * F;
+  if (n == 0) return 0;
+  const int K = R * S * C;
+  const long long positions = (long long)N * OH * OW;
+  const int z = nb_conv2d_wgrad_slices(positions, K, F);
+  const long long per = (positions + z - 1) / z;
+  const ConvGeom g{N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl};
+  const bool vec = C % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & (dtype ? 7 : 15)) == 0;
+#define WGRAD(T, KG, FG) do { if (vec) WGRAD_V(T, KG, FG, true); else WGRAD_V(T, KG, FG, false); } while (0)
+#define WGRAD_V(T, KG, FG, VEC) conv2d_wgrad_direct_kernel<T, KG, FG, VEC><<<dim3((K + 4 * KG - 1) / (4 * KG), (F + 4 * FG - 1) / (4 * FG), z), 128, 0, STREAM>>>((const T*)x, (const T*)dy, part, g, per)
+#define WGRAD_T(T)                                                                            \
+  do {                                                                                        \
+    if (K <= 16) { if (F <= 16) WGRAD(T, 4, 4); else WGRAD(T, 4, 8); }                        \
+    else if (K <= 32) { if (F <= 16) WGRAD(T, 8, 4); else WGRAD(T, 8, 8); }                   \
+    else { if (F <= 16) WGRAD(T, 16, 4); else WGRAD(T, 16, 8); }                              \
+    fold_slices_kernel<T><<<(unsigned)((n + 31) / 32), 256, 0, STREAM>>>(part, (T*)dw, n, z); \
+  } while (0)
+  if (dtype) WGRAD_T(bf16);
+  else WGRAD_T(float);
+#undef WGRAD_T
+#undef WGRAD
+#undef WGRAD_V
   return CHECK_LAUNCH();
 }
 

@@ -47,7 +47,8 @@ def _L():
             "nb_pool2d_bwd": [c_vp] * 3 + [c_int] * 14 + [c_vp],
             "nb_pool2d_select": [c_vp] * 3 + [c_int] * 13 + [c_vp],
             "nb_conv2d_direct": [c_vp] * 4 + [c_int] * 14 + [c_vp],
-            "nb_conv2d_wgrad_direct": [c_vp] * 3 + [c_int] * 14 + [c_vp],
+            "nb_conv2d_wgrad_slices": [c_ll, c_int, c_int],
+            "nb_conv2d_wgrad_direct": [c_vp] * 4 + [c_int] * 14 + [c_vp],
             "nb_sum_slices": [c_vp, c_vp, c_ll, c_int, c_int, c_vp],
             "nb_binary": [c_vp, c_vp, c_vp, c_ll, c_int, c_int, c_ll, c_int, c_int, c_vp],
             "nb_unary": [c_vp, c_vp, c_ll, c_int, c_int, c_vp],
@@ -391,14 +392,18 @@ def conv2d_direct(x, w, bias, stride, padding):
 def conv2d_wgrad_direct(x, dy, w_shape, stride, padding):
     """Filter gradient of the NHWC x RSCF convolution: ``dw[r,s,c,f] = sum x[...] * dy[...]`` over
     the batch and all output pixels (deterministic, no atomics)."""
+    global launch_count
     x = x.contiguous()
     dy = dy.contiguous().to(x.dtype)
     N, H, W, C = x.shape
     R, S, _, F = w_shape
     OH, OW = dy.shape[1], dy.shape[2]
     dw = torch.empty((R, S, C, F), dtype=x.dtype, device=x.device)
-    _ok(_L().nb_conv2d_wgrad_direct(ptr(x), ptr(dy), ptr(dw), N, H, W, C, R, S, F, OH, OW, stride[0], stride[1],
+    slices = _L().nb_conv2d_wgrad_slices(N * OH * OW, R * S * C, F)
+    part = torch.empty(slices * dw.numel(), dtype=torch.float32, device=x.device)
+    _ok(_L().nb_conv2d_wgrad_direct(ptr(x), ptr(dy), ptr(dw), ptr(part), N, H, W, C, R, S, F, OH, OW, stride[0], stride[1],
                                     padding[0], padding[2], _dt(x), stream_ptr()), "conv2d_wgrad_direct")
+    launch_count += 1
     return dw
 
 
