@@ -19,6 +19,7 @@ CUDA bf16 tensors:
   ``adamw_reduce`` steps, set up by ``transforms/compile.py``).
 * ``all_gather(rows) -> linear | matmul [-> dact_mul]``: one launch that pulls the peers' rows while the tensor
   cores already work on the rows that are there; the gathered tensor is still produced.
+* ``zeros -> scatter-add``: the gradient of an embedding table without the table of zeros.
 
 Every other node is a plain 'op' step. Fusion never changes which tensors exist: fused-away
 intermediates that are still referenced are simply not fusable.
@@ -91,6 +92,15 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
                                 a.op.name == "gelu" and a.kwargs.get("approximate", "none") not in ("none", "tanh")):
                             chain = [i, j, k]
         kind = "linear_epilogue"
+        if chain is None and n.op.name == "full":
+            # zeros -> scatter-add (the gradient of an embedding): the kernel writes every row once and
+            # takes no base at all, so the zeros are neither written nor read
+            o = sole_output(n)
+            if fusable_intermediate(o) and _is_zero_table(n, o):
+                j = cons[id(o)][0]
+                if not used[j] and _is_scatter_add_into(nodes[j], o):
+                    chain = [i, j]
+                    kind = "scatter_zeros"
         if chain is None and n.op.name == "matmul" and _is_local_gemm(n):
             dk = _dact_consumer(n, nodes, cons, target_ids, used)
             if dk is not None:
@@ -182,6 +192,22 @@ def _is_cuda_bf16_2d(n: OpNode) -> bool:
 
     return (a.device.label == "gpu" and a.dtype is DType.bfloat16 and b.dtype is DType.bfloat16
             and len(b._shape) == 2 and len(a._shape) >= 2)
+
+
+def _is_zero_table(n: OpNode, o: TensorImpl) -> bool:
+    from ...types import DType
+
+    v = n.kwargs.get("value")
+    return (isinstance(v, (int, float)) and v == 0 and o.device.label == "gpu" and len(o._shape) == 2
+            and o.dtype in (DType.bfloat16, DType.float32))
+
+
+def _is_scatter_add_into(n: OpNode, table: TensorImpl) -> bool:
+    if n.op.name != "scatter" or n.kwargs.get("mode") != "add" or n.kwargs.get("axis") != 0 or n.kwargs.get("bd", 0):
+        return False
+    ins = n.input_impls()
+    return len(ins) == 3 and ins[0] is table and all(x is not table for x in ins[1:]) \
+        and all(x.sharding is None and not x.batch_dims for x in ins)
 
 
 def _is_local_gemm(n: OpNode) -> bool:
@@ -380,6 +406,20 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
                 o._buffers = [out]
         else:
             store_outputs(last, [[out]])
+        return
+    if kind == "scatter_zeros":
+        from ... import native
+
+        z, sc = group
+        _, idx, upd = [x._buffers[0] if x._buffers else None for x in sc.input_impls()]
+        shape, dt = tuple(sc.input_impls()[0]._shape), sc.input_impls()[0].dtype.to_torch()
+        if native.use_native(upd) and upd.dim() and upd.shape[-1] == shape[1] and all(shape):
+            from ...native import kernels
+
+            _store(sc, [[kernels.embedding_scatter_add(None, idx, upd, shape[0], dt)]], keep_graph)
+        else:
+            _plain(z, keep_graph)
+            _plain(sc, keep_graph)
         return
     if kind == "gemm_residual":
         from ...native.gemm import gemm_bf16

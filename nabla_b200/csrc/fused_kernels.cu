@@ -673,19 +673,213 @@ __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restri
     for (int c = threadIdx.x; c < D; c += blockDim.x) dst[c] = ok ? src[c] : from_f<T>(0.f);
   }
 }
-// acc[ids[i]] += upd[i]  (fp32 accumulation table)
-template <typename T>
-__global__ void __launch_bounds__(128) embedding_scatter_add_kernel(float* __restrict__ acc,
-                                                                   const long long* __restrict__ ids,
-                                                                   const T* __restrict__ upd, int n_ids, int D,
-                                                                   int vocab) {
+// out = base + scatter_add(ids, upd): the gradient of an embedding.
+// Large tables: `out` starts as a copy of base (or zeros, by memset), the ids are bucketed by row (three short
+// launches over the integers), and every row that occurs is written once more, as the fp32 sum of its updates
+// in registers: no fp32 table that is zeroed, added to with atomics and converted. A row with more than SCAT_SEG
+// entries (frequent tokens: ids of text fall off about as 1 / rank) is cut into segments, one block each, whose
+// fp32 partial rows the last block of the row adds up; one block per row would leave the most frequent id,
+// some 1000 of 16384 tokens, to one block.
+// Bound by HBM (updates read once, `out` written once and its rows once more). 16384 ids into 32000 x 2048 bf16
+// with a base table: 257 us with the fp32 table, 114 now; 48 for the rows, 11 for the bucketing.
+constexpr int SCAT_SEG = 32;
+struct ScatWs {
+  int *counts, *done, *total, *nseg, *nheavy;   // zeroed by the launcher
+  int *start, *rank, *list;                     // first list slot per row; place of an entry in its row; entries by row
+  int4* seg;                                    // (row, first list slot, entries, partial row or -1)
+};
+// Segments of one row: `c` entries from list slot `at` on, written from seg[sg] on.
+__device__ __forceinline__ void scatter_segments(const ScatWs& ws, int v, int c, int at, int sg) {
+  const int k = (c + SCAT_SEG - 1) / SCAT_SEG;
+  int h = -1;
+  if (k > 1) h = atomicAdd(ws.nheavy, k);
+  for (int q = 0; q < k; ++q) ws.seg[sg + q] = make_int4(v, at + q * SCAT_SEG, min(SCAT_SEG, c - q * SCAT_SEG), h < 0 ? -1 : h + q);
+}
+// Lanes of a warp with the same id share one atomic; returns the entry's place among those of its row.
+__device__ __forceinline__ int scatter_rank(int* counts, long long id, bool ok) {
+  const unsigned same = __match_any_sync(0xffffffffu, ok ? (int)id : -1);
+  const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+  int base = 0;
+  if (ok && lane == leader) base = atomicAdd(counts + id, __popc(same));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  return base + __popc(same & ((1u << lane) - 1u));
+}
+// Inclusive scan over the block of (entries, segments), packed in the halves of 64 bits.
+template <int NW>
+__device__ __forceinline__ unsigned long long scatter_scan(unsigned long long x, unsigned long long* wsum,
+                                                           unsigned long long& total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += t;
+  }
+  if (lane == 31) wsum[w] = x;
+  __syncthreads();
+  unsigned long long before = 0, all = 0;
+#pragma unroll
+  for (int i = 0; i < NW; ++i) {
+    if (i < w) before += wsum[i];
+    all += wsum[i];
+  }
+  total = all;
+  return x + before;
+}
+
+__global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const long long id = i < n_ids ? ids[i] : -1;
+  const bool ok = id >= 0 && id < vocab;
+  const int rank = scatter_rank(ws.counts, id, ok);
+  if (ok) ws.rank[i] = rank;
+}
+// List slots and segments of every row; the rows of a block come in order, the blocks in any.
+__global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int vocab) {
+  __shared__ unsigned long long wsum[8];
+  __shared__ int base_at, base_sg;
+  const int v = blockIdx.x * 256 + threadIdx.x;
+  const int c = v < vocab ? ws.counts[v] : 0;
+  const unsigned long long t = (unsigned long long)((c + SCAT_SEG - 1) / SCAT_SEG) << 32 | (unsigned)c;
+  unsigned long long total;
+  const unsigned long long at0 = scatter_scan<8>(t, wsum, total) - t;
+  if (total == 0) return;                            // the same in every thread
+  if (threadIdx.x == 0) {
+    base_at = atomicAdd(ws.total, (int)(unsigned)total);
+    base_sg = atomicAdd(ws.nseg, (int)(total >> 32));
+  }
+  __syncthreads();
+  if (c) {
+    const int at = base_at + (int)(unsigned)at0;
+    ws.start[v] = at;
+    scatter_segments(ws, v, c, at, base_sg + (int)(at0 >> 32));
+  }
+}
+__global__ void __launch_bounds__(256) scatter_place_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n_ids) return;
+  const long long id = ids[i];
+  if (id >= 0 && id < vocab) ws.list[ws.start[id] + ws.rank[i]] = i;
+}
+
+// Columns [c, c + VN) of the fp32 sum of `n` rows of upd. SCAT_U rows are in flight: the rows lie anywhere, so
+// each is a full memory latency.
+constexpr int SCAT_U = 8;
+template <typename T, int VN>
+__device__ __forceinline__ void scatter_sum(const T* __restrict__ upd, const int* __restrict__ list, int n, size_t D, int c,
+                                            int n_ids, float (&acc)[VN]) {
+#pragma unroll
+  for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+  for (int k = 0; k < n; k += SCAT_U) {
+    uint4 raw[SCAT_U];
+    T one[SCAT_U];
+#pragma unroll
+    for (int u = 0; u < SCAT_U; ++u) {
+      if (k + u < n) {
+        const int i = list[k + u];
+        if (!NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, i, n_ids)) return;
+        if (VN > 1) raw[u] = *reinterpret_cast<const uint4*>(upd + i * D + c);
+        else one[u] = upd[i * D + c];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < SCAT_U; ++u) {
+      if (k + u < n) {
+        float v[VN];
+        if constexpr (VN > 1) unpack_vec<T>(raw[u], v);
+        else v[0] = to_f<T>(one[u]);
+#pragma unroll
+        for (int j = 0; j < VN; ++j) acc[j] += v[j];
+      }
+    }
+  }
+}
+template <typename T, int VN>
+__device__ __forceinline__ void scatter_write(const T* __restrict__ base, T* __restrict__ out, size_t at, float (&acc)[VN]) {
+  if (base != nullptr) {
+    float b[VN];
+    if (VN > 1) load_vec<T>(base + at, b);
+    else b[0] = to_f<T>(base[at]);
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j] += b[j];
+  }
+  if (VN > 1) store_vec<T>(out + at, acc);
+  else out[at] = from_f<T>(acc[0]);
+}
+// Adds up the `nseg` fp32 partial rows of row v from partial row h0 on.
+template <typename T, int VN>
+__device__ __forceinline__ void scatter_join(const T* __restrict__ base, T* __restrict__ out, const float* __restrict__ part,
+                                             int v, int h0, int nseg, int D) {
+  for (int c = threadIdx.x * VN; c < D; c += blockDim.x * VN) {
+    float acc[VN];
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+#pragma unroll 4
+    for (int q = 0; q < nseg; ++q)
+#pragma unroll
+      for (int j = 0; j < VN; ++j) acc[j] += __ldcg(part + (size_t)(h0 + q) * D + c + j);
+    scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
+  }
+}
+// The blocks walk the segments, the next descriptor on its way while one is worked on. VN: elements per access
+// (16 bytes, or 1 where rows are not 16-byte aligned).
+template <typename T, int VN>
+__global__ void __launch_bounds__(256) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
+                                                          T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
+                                                          int D) {
+  __shared__ int last;
+  const int total = *ws.nseg;
+  int4 next = ws.seg[blockIdx.x];                    // not written past the last segment: read, then dropped
+  for (int s = blockIdx.x; s < total; s += gridDim.x) {
+    const int4 sg = next;
+    if (s + (int)gridDim.x < total) next = ws.seg[s + gridDim.x];
+    const int v = sg.x;
+    for (int c = threadIdx.x * VN; c < D; c += blockDim.x * VN) {
+      float acc[VN];
+      scatter_sum<T, VN>(upd, ws.list + sg.y, sg.z, D, c, n_ids, acc);
+      if (sg.w < 0) {
+        scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
+      } else {
+#pragma unroll
+        for (int j = 0; j < VN; ++j) part[(size_t)sg.w * D + c + j] = acc[j];
+      }
+    }
+    if (sg.w < 0) continue;
+    const int nseg = (ws.counts[v] + SCAT_SEG - 1) / SCAT_SEG, h0 = sg.w - (sg.y - ws.start[v]) / SCAT_SEG;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ws.done + v, 1) == nseg - 1;
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      scatter_join<T, VN>(base, out, part, v, h0, nseg, D);
+    }
+  }
+}
+// Small tables: acc[ids[i]] += upd[i] in an fp32 table that stays in L2, four columns per atomic (VEC).
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(128) embedding_scatter_add_kernel(float* __restrict__ acc, const long long* __restrict__ ids,
+                                                                   const T* __restrict__ upd, int n_ids, int D, int vocab) {
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
   const long long id = ids[i];
   if (id < 0 || id >= vocab) return;
   float* dst = acc + (size_t)id * D;
   const T* src = upd + (size_t)i * D;
-  for (int c = threadIdx.x; c < D; c += blockDim.x) atomicAdd(dst + c, to_f<T>(src[c]));
+  if constexpr (VEC) {
+    for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) {
+      float4 v;
+      if constexpr (sizeof(T) == 4) {
+        v = *reinterpret_cast<const float4*>(src + c);
+      } else {
+        const uint2 w = *reinterpret_cast<const uint2*>(src + c);
+        v = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
+                        __uint_as_float(w.y & 0xffff0000u));
+      }
+      atomicAdd(reinterpret_cast<float4*>(dst + c), v);
+    }
+  } else {
+    for (int c = threadIdx.x; c < D; c += blockDim.x) atomicAdd(dst + c, to_f<T>(src[c]));
+  }
 }
 // The same sum without atomics, for runs that must repeat bit for bit: the ids come sorted (stable,
 // `perm[k]` = position of the k-th sorted id in the original order); the block at the head of each
@@ -1502,17 +1696,67 @@ int nb_embedding_gather(const void* table, const long long* ids, void* out, int 
   else embedding_gather_kernel<float><<<n_ids, 128, 0, STREAM>>>((const float*)table, ids, (float*)out, n_ids, D, vocab);
   return CHECK_LAUNCH();
 }
-// acc (fp32, [vocab][D]) must be zeroed by the caller; out = base + acc, cast to dtype.
-int nb_embedding_scatter_add(float* acc, const long long* ids, const void* upd, const void* base, void* out, int n_ids,
-                             int D, int vocab, int dtype, void* stream) {
-  if (n_ids > 0) {
-    if (dtype) embedding_scatter_add_kernel<bf16><<<n_ids, 128, 0, STREAM>>>(acc, ids, (const bf16*)upd, n_ids, D, vocab);
-    else embedding_scatter_add_kernel<float><<<n_ids, 128, 0, STREAM>>>(acc, ids, (const float*)upd, n_ids, D, vocab);
+// out = base + scatter_add(ids, upd); base null: zeros. `work`: nb_embedding_scatter_work(...) 32-bit words of
+// 16-byte aligned scratch.
+static long long scat_max_heavy(long long n_ids) { return 2 * (n_ids / SCAT_SEG); }   // segments of rows with > SCAT_SEG entries
+static long long scat_ints(long long n_ids, long long vocab) { return (3 * vocab + 3 + 2 * n_ids + 3) / 4 * 4; }
+// Atomics into an fp32 table while it stays in L2 and its rows are not crowded: the bucketing's launches
+// have no large table to win against there (5000 ids into 1000 x 256 fp32: 17 us with atomics, 42 bucketed; 4000
+// into 8192 x 768 bf16: 34 and 44), but 20000 ids into 50 x 2048 take 91 us with atomics and 82 bucketed.
+static bool scat_atomics(long long n_ids, long long D, long long vocab) { return vocab * D <= (8ll << 20) && n_ids <= 16 * vocab; }
+long long nb_embedding_scatter_work(int n_ids, int D, int vocab) {
+  if (scat_atomics(n_ids, D, vocab)) return (long long)vocab * D;
+  return scat_ints(n_ids, vocab) + 4ll * n_ids + scat_max_heavy(n_ids) * D;
+}
+int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, const void* base, void* out, int n_ids, int D,
+                             int vocab, int dtype, void* stream) {
+  if (vocab <= 0 || D <= 0) return 0;
+  if (n_ids < 0) return -2;
+  if (n_ids > 0 && scat_atomics(n_ids, D, vocab)) {
+    const size_t n = (size_t)vocab * D;
+    const bool direct = !dtype && base == nullptr;   // the sum is the result
+    float* acc = direct ? (float*)out : reinterpret_cast<float*>(work);
+    if (cudaMemsetAsync(acc, 0, n * sizeof(float), STREAM) != cudaSuccess) return -1;
+    const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(acc)) & 15) == 0;
+#define SCAT(T, VEC) embedding_scatter_add_kernel<T, VEC><<<n_ids, 128, 0, STREAM>>>(acc, ids, (const T*)upd, n_ids, D, vocab)
+    if (dtype) { if (vec) SCAT(bf16, true); else SCAT(bf16, false); }
+    else { if (vec) SCAT(float, true); else SCAT(float, false); }
+#undef SCAT
+    const int grid = grid_for(n, 256);
+    if (dtype) cast_kernel<float, bf16><<<grid, 256, 0, STREAM>>>(acc, (bf16*)out, n, (const bf16*)base);
+    else if (!direct) cast_kernel<float, float><<<grid, 256, 0, STREAM>>>(acc, (float*)out, n, (const float*)base);
+    return CHECK_LAUNCH();
   }
-  const size_t n = (size_t)vocab * D;
-  const int grid = grid_for(n, 256);
-  if (dtype) cast_kernel<float, bf16><<<grid, 256, 0, STREAM>>>(acc, (bf16*)out, n, (const bf16*)base);
-  else cast_kernel<float, float><<<grid, 256, 0, STREAM>>>(acc, (float*)out, n, (const float*)base);
+  const size_t bytes = (size_t)vocab * D * (dtype ? 2 : 4);
+  if ((base != nullptr ? cudaMemcpyAsync(out, base, bytes, cudaMemcpyDeviceToDevice, STREAM)
+                       : cudaMemsetAsync(out, 0, bytes, STREAM)) != cudaSuccess)
+    return -1;
+  if (n_ids == 0) return 0;
+  ScatWs ws;
+  ws.counts = work;
+  ws.done = ws.counts + vocab;
+  ws.total = ws.done + vocab;
+  ws.nseg = ws.total + 1;
+  ws.nheavy = ws.nseg + 1;
+  ws.start = ws.nheavy + 1;
+  ws.rank = ws.start + vocab;
+  ws.list = ws.rank + n_ids;
+  ws.seg = reinterpret_cast<int4*>(work + scat_ints(n_ids, vocab));
+  float* part = reinterpret_cast<float*>(ws.seg + n_ids);
+  const int idb = (n_ids + 255) / 256;
+  if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 3) * sizeof(int), STREAM) != cudaSuccess) return -1;
+  scatter_count_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
+  scatter_slots_kernel<<<(vocab + 255) / 256, 256, 0, STREAM>>>(ws, vocab);
+  scatter_place_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
+  const int V = dtype ? 8 : 4;
+  const bool vec = D % V == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  int threads = 32;                                  // the power of two that covers a row in one pass, at most 256
+  while (threads < 256 && threads * (vec ? V : 1) < D) threads *= 2;
+  const int grid = (int)(n_ids < 148ll * 2048 / threads ? n_ids : 148ll * 2048 / threads);
+#define SCAT(T, VN) scatter_rows_kernel<T, VN><<<grid, threads, 0, STREAM>>>((const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D)
+  if (dtype) { if (vec) SCAT(bf16, 8); else SCAT(bf16, 1); }
+  else { if (vec) SCAT(float, 4); else SCAT(float, 1); }
+#undef SCAT
   return CHECK_LAUNCH();
 }
 

@@ -60,6 +60,8 @@ def _L():
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = c_int
+        lib.nb_embedding_scatter_work.argtypes = [c_int] * 3
+        lib.nb_embedding_scatter_work.restype = c_ll
         lib.nb_layernorm_bwd_two_kernels.argtypes = [c_int]
         lib.nb_layernorm_bwd_two_kernels.restype = None
         # NABLA_B200_LN_BWD=two_kernels: dx and dgamma / dbeta in separate passes (the layout for rows
@@ -217,14 +219,21 @@ def embedding_gather(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
     return out.view(*ids.shape, D)
 
 
-def embedding_scatter_add(base: torch.Tensor, ids: torch.Tensor, upd: torch.Tensor) -> torch.Tensor:
-    """base + scatter_add(ids, upd) with fp32 accumulation (embedding backward)."""
+def embedding_scatter_add(base: torch.Tensor | None, ids: torch.Tensor, upd: torch.Tensor, vocab: int = 0,
+                          dtype: torch.dtype | None = None) -> torch.Tensor:
+    """base + scatter_add(ids, upd) with fp32 accumulation (embedding backward). ``base`` None: a table of
+    ``vocab`` rows of zeros in ``dtype``, which is neither made nor read."""
     global launch_count
-    base = base.contiguous()
-    V, D = base.shape
-    flat = ids.contiguous().view(-1).to(torch.int64)
-    u = upd.contiguous().view(-1, D).to(base.dtype)
     from .. import config
+
+    if base is None and config.is_deterministic():
+        base = torch.zeros((vocab, upd.shape[-1]), dtype=dtype, device=upd.device)
+    if base is not None:
+        base = base.contiguous()
+        vocab, dtype = base.shape[0], base.dtype
+    V, D = vocab, upd.shape[-1]
+    flat = ids.contiguous().view(-1).to(torch.int64)
+    u = upd.contiguous().view(-1, D).to(dtype)
 
     if config.is_deterministic():
         # no atomics: stable sort of the ids, then one block per run of equal ids adds the run's rows
@@ -235,9 +244,9 @@ def embedding_scatter_add(base: torch.Tensor, ids: torch.Tensor, upd: torch.Tens
                                              _dt(base), stream_ptr()), "embedding_scatter_sorted")
         launch_count += 1
         return out
-    acc = torch.zeros((V, D), dtype=torch.float32, device=base.device)
-    out = torch.empty_like(base)
-    _ok(_L().nb_embedding_scatter_add(ptr(acc), ptr(flat), ptr(u), ptr(base), ptr(out), flat.numel(), D, V, _dt(base),
+    work = torch.empty(_L().nb_embedding_scatter_work(flat.numel(), D, V), dtype=torch.int32, device=u.device)
+    out = torch.empty((V, D), dtype=dtype, device=u.device)
+    _ok(_L().nb_embedding_scatter_add(ptr(work), ptr(flat), ptr(u), ptr(base), ptr(out), flat.numel(), D, V, _dt(u),
                                       stream_ptr()), "embedding_scatter_add")
     launch_count += 1
     return out

@@ -81,3 +81,44 @@ def test_direct_convolution_skips_padding_under_infinite_operands():
     zero = torch.zeros((), dtype=torch.float64, device="cuda")
     ref = torch.where(ok.unsqueeze(-1), win.unsqueeze(-1) * dy.double()[:, :, :, None, None, None, :], zero).sum((0, 1, 2))
     torch.testing.assert_close(dw.double(), ref, rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
+# ---------------------------------------------------------------- embedding gradient
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab,dim,n,hot", [
+    (1, 8, 1, 0.0), (50, 33, 700, 0.0), (100, 256, 33, 1.0), (300, 64, 4096, 0.3), (300, 64, 4801, 0.3), (300, 33, 4801, 0.3),
+    (4096, 2048, 500, 0.1), (4097, 2048, 500, 0.1), (4080, 2056, 3000, 0.05), (4097, 2056, 3000, 0.05), (50, 40, 801, 1.0),
+    (8200, 1032, 9000, 0.5), (9000, 1001, 700, 0.5)])
+def test_embedding_scatter_add(dtype, vocab, dim, n, hot):
+    """Both ways of adding (an fp32 table of at most 8M elements, the bucketed ids), rows of one to thousands of
+    entries (segments of 32), ids out of range, rows that are and are not whole 16-byte vectors, with and without a base table."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(n)
+    ids = torch.randint(-2, vocab + 2, (n,), device="cuda")
+    ids[torch.rand(n, device="cuda") < hot] = vocab // 2
+    upd = torch.randn(n, dim, device="cuda").to(dtype)
+    base = torch.randn(vocab, dim, device="cuda").to(dtype)
+    ok = (ids >= 0) & (ids < vocab)
+    ref = torch.zeros(vocab, dim, dtype=torch.float64, device="cuda").index_add_(0, ids[ok], upd[ok].double())
+    assert _rel2(kernels.embedding_scatter_add(base, ids, upd), ref + base.double()) < STORED[dtype]
+    got = kernels.embedding_scatter_add(None, ids, upd, vocab, dtype)
+    assert got.shape == (vocab, dim) and got.dtype is dtype and _rel2(got, ref) < STORED[dtype]
+    empty = kernels.embedding_scatter_add(base, ids[:0], upd[:0])
+    assert torch.equal(empty, base)
+
+
+def test_gradient_of_an_embedding_takes_no_table_of_zeros():
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    torch.manual_seed(0)
+    table = torch.randn(500, 64, device="cuda")
+    ids = torch.randint(0, 500, (3, 70), device="cuda")
+    w = torch.randn(3, 70, 64, device="cuda")
+    wt, it, tt = nb.Tensor.from_torch(w), nb.Tensor.from_torch(ids), nb.Tensor.from_torch(table)
+    f = nb.compile(lambda t: nb.grad(lambda a: nb.reduce_sum(F.embedding(it, a) * wt), create_graph=False)(t))
+    ref = torch.zeros(500, 64, dtype=torch.float64, device="cuda").index_add_(0, ids.reshape(-1), w.double().reshape(-1, 64))
+    for _ in range(2):
+        assert _rel2(f(tt).to_torch(), ref) < STORED[torch.float32]
+    assert "scatter_zeros" in f.dump_plan()
