@@ -20,6 +20,7 @@ CUDA bf16 tensors:
 * ``all_gather(rows) -> linear | matmul [-> dact_mul]``: one launch that pulls the peers' rows while the tensor
   cores already work on the rows that are there; the gathered tensor is still produced.
 * ``zeros -> scatter-add``: the gradient of an embedding table without the table of zeros.
+* ``sum -> sum ...`` over neighbouring axes: one reduction over the joined axes.
 
 Every other node is a plain 'op' step. Fusion never changes which tensors exist: fused-away
 intermediates that are still referenced are simply not fusable.
@@ -101,6 +102,30 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
                 if not used[j] and _is_scatter_add_into(nodes[j], o):
                     chain = [i, j]
                     kind = "scatter_zeros"
+        if chain is None and n.op.name == "reduce_sum" and _is_plain_sum(n) \
+                and n.kwargs["axis"] < len(n.input_impls()[0]._shape) - 1:
+            # sums over neighbouring axes, one after the other (``sum(axis=(0, 1, 2))``): one reduction over
+            # the joined axes, without the partial results and their rounding. Not where the last axis is
+            # among them: one long row would be left to one warp
+            idxs, lo, hi = [i], n.kwargs["axis"], n.kwargs["axis"]
+            last_axis = len(n.input_impls()[0]._shape) - 1
+            while True:
+                o = sole_output(nodes[idxs[-1]])
+                if not fusable_intermediate(o):
+                    break
+                j = cons[id(o)][0]
+                m = nodes[j]
+                if used[j] or m.op.name != "reduce_sum" or not _is_plain_sum(m) or m.kwargs["axis"] not in (lo - 1, lo) \
+                        or (m.kwargs["axis"] == lo and hi + 1 == last_axis):
+                    break
+                if m.kwargs["axis"] == lo:
+                    hi += 1
+                else:
+                    lo -= 1
+                idxs.append(j)
+            if len(idxs) > 1:
+                chain = idxs
+                kind = "sum_axes"
         if chain is None and n.op.name == "matmul" and _is_local_gemm(n):
             dk = _dact_consumer(n, nodes, cons, target_ids, used)
             if dk is not None:
@@ -208,6 +233,16 @@ def _is_scatter_add_into(n: OpNode, table: TensorImpl) -> bool:
     ins = n.input_impls()
     return len(ins) == 3 and ins[0] is table and all(x is not table for x in ins[1:]) \
         and all(x.sharding is None and not x.batch_dims for x in ins)
+
+
+def _is_plain_sum(n: OpNode) -> bool:
+    """Unsharded floating-point GPU sum that drops its axis."""
+    from ...types import DType
+
+    ins = n.input_impls()
+    return (len(ins) == 1 and ins[0].sharding is None and not ins[0].batch_dims and ins[0].device.label == "gpu"
+            and ins[0].dtype in (DType.bfloat16, DType.float32) and not n.kwargs.get("keepdims", False)
+            and set(n.kwargs) <= {"axis", "keepdims"} and n.kwargs["axis"] >= 0)
 
 
 def _is_local_gemm(n: OpNode) -> bool:
@@ -420,6 +455,23 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         else:
             _plain(z, keep_graph)
             _plain(sc, keep_graph)
+        return
+    if kind == "sum_axes":
+        from ...native import kernels
+
+        x = group[0].input_impls()[0]._buffers[0]
+        lo = hi = group[0].kwargs["axis"]
+        for n_ in group[1:]:
+            if n_.kwargs["axis"] == lo:
+                hi += 1
+            else:
+                lo -= 1
+        out = kernels.reduce(x.contiguous().reshape(*x.shape[:lo], -1, *x.shape[hi + 1:]), lo, "sum") if x.numel() else None
+        if out is not None:
+            _store(group[-1], [[out]], keep_graph)
+        else:
+            for n_ in group:
+                _plain(n_, keep_graph)
         return
     if kind == "gemm_residual":
         from ...native.gemm import gemm_bf16

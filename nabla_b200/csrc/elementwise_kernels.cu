@@ -324,6 +324,48 @@ __global__ void __launch_bounds__(256) col_reduce_kernel(const T* __restrict__ x
   }
 }
 
+// The same for few rows and many columns (a sum over the batch: R = 8, inner = seq * dim): one thread per
+// 16-byte vector of columns walks the R rows, four loads in flight, no shared memory and no barrier. The
+// tile kernel above reads 2-byte elements there, and with R / 8 rows per warp spends its time at the
+// barriers. Bound by HBM; (8, 2048, 2048) bf16 over dim 0: 239 us with the tile kernel, 23 here.
+template <typename T, int OP>
+__global__ void __launch_bounds__(256) thin_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
+                                                         int R, long long inner) {
+  constexpr int V = Vec<T>::N;
+  const long long nv = inner / V, t = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (t >= outer * nv) return;
+  const long long o = t / nv, i = (t - o * nv) * V;
+  const T* p = x + o * R * inner + i;
+  if (!NB_IN_BOUNDS(NB_SITE_REDUCE_INDEX, (o * R + (R - 1)) * inner + i + V - 1, outer * R * inner)) return;
+  float acc[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = OP == R_MAX ? -INFINITY : OP == R_MIN ? INFINITY : 0.f;
+  auto take = [&](const uint4& raw) {
+    float f[V];
+    unpack<T>(raw, f);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      if (OP == R_MAX) acc[j] = (f[j] > acc[j] || f[j] != f[j]) ? f[j] : acc[j];      // NaN wins, and stays
+      else if (OP == R_MIN) acc[j] = (f[j] < acc[j] || f[j] != f[j]) ? f[j] : acc[j];
+      else acc[j] += f[j];
+    }
+  };
+  int r = 0;
+  for (; r + 4 <= R; r += 4) {
+    uint4 raw[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) raw[u] = *reinterpret_cast<const uint4*>(p + (long long)(r + u) * inner);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) take(raw[u]);
+  }
+  for (; r < R; ++r) take(*reinterpret_cast<const uint4*>(p + (long long)r * inner));
+  if (OP == R_MEAN) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] /= (float)R;
+  }
+  *reinterpret_cast<uint4*>(out + o * inner + i) = pack<T>(acc);
+}
+
 template <typename T, typename O>
 __global__ void __launch_bounds__(256) col_reduce_finish_kernel(const float* __restrict__ pv, const long long* __restrict__ pi,
                                                                O* __restrict__ out, long long outer, long long R,
@@ -411,6 +453,12 @@ int nb_reduce_splits(long long outer, long long R, long long inner) {
   return (int)(s < 1 ? 1 : s);
 }
 
+// thin_reduce_kernel: value reductions over at most 256 rows (a longer sum keeps the tile kernel's parallel
+// partial sums) with enough column vectors for a block on every SM.
+static bool thin_reduce(long long outer, long long R, long long inner, int V) {
+  return R <= 256 && inner % V == 0 && outer * (inner / V) >= 148 * 256 && (outer * (inner / V) + 255) / 256 <= 0x7fffffffll;
+}
+
 int nb_reduce(const void* x, void* out, void* scratch, long long outer, long long R, long long inner, int op, int dtype,
               void* stream) {
   if (outer <= 0 || inner <= 0 || R <= 0) return 0;
@@ -425,6 +473,17 @@ int nb_reduce(const void* x, void* out, void* scratch, long long outer, long lon
       if (arg) row_reduce_kernel<float, long long><<<grid, 256, 0, STREAM>>>((const float*)x, (long long*)out, outer, R, op);
       else row_reduce_kernel<float, float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)out, outer, R, op);
     }
+    return CHECK_LAUNCH();
+  }
+  const int V = dtype ? 8 : 4;
+  if (!arg && thin_reduce(outer, R, inner, V) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    const unsigned grid_t = (unsigned)((outer * (inner / V) + 255) / 256);
+#define NB_THIN(T, OP) thin_reduce_kernel<T, OP><<<grid_t, 256, 0, STREAM>>>((const T*)x, (T*)out, outer, (int)R, inner)
+#define NB_THIN_T(T) do { if (op == R_SUM) NB_THIN(T, R_SUM); else if (op == R_MAX) NB_THIN(T, R_MAX); \
+                          else if (op == R_MIN) NB_THIN(T, R_MIN); else NB_THIN(T, R_MEAN); } while (0)
+    if (dtype) NB_THIN_T(bf16); else NB_THIN_T(float);
+#undef NB_THIN_T
+#undef NB_THIN
     return CHECK_LAUNCH();
   }
   const int splits = nb_reduce_splits(outer, R, inner);

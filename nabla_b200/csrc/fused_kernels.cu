@@ -422,6 +422,28 @@ __global__ void __launch_bounds__(256) colsum_partials_kernel(const float* __res
   }
 }
 
+// out[i] = sum_z part[z][i], fp32 slices of n: 32 results per block, its 8 warps take every 8th slice.
+template <typename T>
+__global__ void __launch_bounds__(256) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
+                                                         int slices) {
+  __shared__ float sh[8][32];
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+  const size_t i = (size_t)blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (i < n) {
+#pragma unroll 8
+    for (int z = wq; z < slices; z += 8) s += part[(size_t)z * n + i];
+  }
+  sh[wq][lane] = s;
+  __syncthreads();
+  if (wq == 0 && i < n) {
+    s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += sh[q][lane];
+    out[i] = from_f<T>(s);
+  }
+}
+
 // ============================================================== column sum (bias gradient)
 // x [rows][N] -> partial[gridDim.y][N] ; each block sums a slab of rows for 32*V columns.
 template <typename T>
@@ -461,6 +483,38 @@ __global__ void colsum_final_kernel(const float* __restrict__ partial, T* __rest
   float s = 0.f;
   for (int i = 0; i < nparts; ++i) s += partial[(size_t)i * N + c];
   out[c] = from_f<T>(s);
+}
+
+// Column sums of a tall, narrow matrix (the bias gradient of a convolution: 200704 x 16): the block's 256
+// threads cover 256 / (N / V) whole rows at a time, so every lane loads whatever N is; colsum_kernel gives a
+// warp one row's 32 vectors and leaves 28 of 32 lanes without one there. 200704 x 16 fp32: 81 -> 17 us.
+template <typename T>
+__global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
+                                                           int N, int rows_per_block) {
+  constexpr int V = Vec<T>::N;
+  __shared__ float sh[256 * V];
+  const int nv = N / V, rpp = 256 / nv, r_in = threadIdx.x / nv, c = threadIdx.x % nv;
+  const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
+  float acc[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = 0.f;
+  if (r_in < rpp) {
+#pragma unroll 4
+    for (int r = r0 + r_in; r < r1; r += rpp) {
+      float v[V];
+      load_vec<T>(x + (size_t)r * N + c * V, v);
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[j] += v[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < V; ++j) sh[threadIdx.x * V + j] = acc[j];
+  __syncthreads();
+  for (int i = threadIdx.x; i < N; i += 256) {        // element i of row slot k sits at k * N + i
+    float s = 0.f;
+    for (int k = 0; k < rpp; ++k) s += sh[k * N + i];
+    partial[(size_t)blockIdx.x * N + i] = s;
+  }
 }
 
 // ============================================================== softmax / log-softmax (last dim)
@@ -1483,28 +1537,6 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __
     }
   }
 }
-// out[i] = sum_z part[z][i], fp32 slices of n: 32 results per block, its 8 warps take every 8th slice.
-template <typename T>
-__global__ void __launch_bounds__(256) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
-                                                         int slices) {
-  __shared__ float sh[8][32];
-  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  const size_t i = (size_t)blockIdx.x * 32 + lane;
-  float s = 0.f;
-  if (i < n) {
-#pragma unroll 8
-    for (int z = wq; z < slices; z += 8) s += part[(size_t)z * n + i];
-  }
-  sh[wq][lane] = s;
-  __syncthreads();
-  if (wq == 0 && i < n) {
-    s = 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) s += sh[q][lane];
-    out[i] = from_f<T>(s);
-  }
-}
-
 // out[i] = sum_j part[j][i] for `slices` fp32 slices of n elements (n % 4 == 0): the second half of
 // a split-K GEMM, whose partial products are written as fp32 by the tensor-core kernel.
 template <typename T>
@@ -1618,16 +1650,27 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
   return CHECK_LAUNCH();
 }
 
-int nb_colsum_nparts(int rows) {
-  int np = (rows + 511) / 512;
-  if (np > 64) np = 64;
+// Narrow: fewer vectors per row than a warp has lanes, and rows enough for many blocks (256 rows each at least).
+static bool colsum_narrow(int rows, int N, int V) { return N / V < 32 && rows >= 4096; }
+int nb_colsum_nparts(int rows, int N, int in_dtype) {
+  int np = (rows + 511) / 512, most = 64;
+  if (colsum_narrow(rows, N, in_dtype ? 8 : 4)) { np = (rows + 255) / 256; most = 148 * 4; }
+  if (np > most) np = most;
   return np < 1 ? 1 : np;
 }
+// partial: fp32 scratch of nb_colsum_nparts(rows, N, in_dtype) * N elements.
 int nb_colsum(const void* x, void* out, float* partial, int rows, int N, int in_dtype, int out_dtype, void* stream) {
   const int V = in_dtype ? 8 : 4;
   if (N % V) return -2;
-  const int np = nb_colsum_nparts(rows);
+  const int np = nb_colsum_nparts(rows, N, in_dtype);
   const int rpb = (rows + np - 1) / np;
+  if (colsum_narrow(rows, N, V)) {
+    if (in_dtype) colsum_narrow_kernel<bf16><<<np, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
+    else colsum_narrow_kernel<float><<<np, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
+    if (out_dtype) fold_slices_kernel<bf16><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (bf16*)out, (size_t)N, np);
+    else fold_slices_kernel<float><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (float*)out, (size_t)N, np);
+    return CHECK_LAUNCH();
+  }
   dim3 grid((N + 32 * V - 1) / (32 * V), np);
   if (in_dtype) colsum_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
   else colsum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);

@@ -25,7 +25,7 @@ def _L():
             "nb_layernorm_fwd": [c_vp] * 6 + [c_int, c_int, c_f, c_int, c_vp],
             "nb_layernorm_bwd_nblocks": [c_int, c_int, c_int],
             "nb_layernorm_bwd": [c_vp] * 9 + [c_int, c_int, c_int, c_vp],
-            "nb_colsum_nparts": [c_int],
+            "nb_colsum_nparts": [c_int] * 3,
             "nb_colsum": [c_vp] * 3 + [c_int] * 4 + [c_vp],
             "nb_softmax": [c_vp, c_vp, c_int, c_int, c_int, c_int, c_vp],
             "nb_lse_pick_fwd": [c_vp] * 4 + [c_int, c_int, c_int, c_vp],
@@ -140,7 +140,7 @@ def colsum(x: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tenso
     x2 = x.contiguous().view(-1, N)
     rows = x2.shape[0]
     out = torch.empty(N, dtype=out_dtype or x.dtype, device=x.device)
-    np_ = _L().nb_colsum_nparts(rows)
+    np_ = _L().nb_colsum_nparts(rows, N, _dt(x))
     partial = torch.empty((np_, N), dtype=torch.float32, device=x.device)
     _ok(_L().nb_colsum(ptr(x2), ptr(out), ptr(partial), rows, N, _dt(x), _dt(out), stream_ptr()), "colsum")
     launch_count += 1

@@ -122,3 +122,37 @@ def test_gradient_of_an_embedding_takes_no_table_of_zeros():
     for _ in range(2):
         assert _rel2(f(tt).to_torch(), ref) < STORED[torch.float32]
     assert "scatter_zeros" in f.dump_plan()
+
+
+# ---------------------------------------------------------------- reductions
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape,axis", [((1, 40, 8192), 0), ((5, 37, 8192), 0), ((256, 40, 8192), 0), ((257, 40, 8192), 0), ((3, 6, 128, 1024), 1),
+                                        ((4, 300, 1001), 0), ((4095, 16), 0), ((4097, 8), 0), ((70001, 24), 0), ((9000, 248), 0)])
+def test_reductions_over_leading_axes(dtype, shape, axis):
+    """The kernel for few rows and its neighbours (257 rows, columns that are no whole vectors), and the column
+    sums of narrow matrices around the row count where they take over."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(1)
+    x = torch.randn(shape, device="cuda").to(dtype)
+    for op, ref in (("sum", x.double().sum(axis)), ("mean", x.double().mean(axis))):
+        assert _rel2(kernels.reduce(x, axis, op), ref) < STORED[dtype]
+    x.view(-1)[::977] = float("-inf")
+    x.view(-1)[5::3001] = float("nan")
+    for op, fn in (("max", torch.amax), ("min", torch.amin)):
+        torch.testing.assert_close(kernels.reduce(x, axis, op), fn(x, axis), rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("axes", [(0, 1), (0, 1, 2), (1, 2), (0, 2), (0, 1, 2, 3)])
+def test_sums_over_neighbouring_axes(axes):
+    import nabla_b200 as nb
+
+    x = torch.randn(6, 7, 50, 16, device="cuda")
+    t = nb.Tensor.from_torch(x)
+    for keep in (False, True):
+        got = nb.reduce_sum(t, axis=axes, keepdims=keep).to_torch()
+        ref = x.double().sum(axes, keepdim=keep)
+        assert got.shape == ref.shape and _rel2(got, ref) < STORED[torch.float32]
+    f = nb.compile(lambda a: nb.reduce_sum(a, axis=axes))
+    f(t)
+    assert ("sum_axes" in f.dump_plan()) == (axes in ((0, 1), (0, 1, 2), (1, 2)))
