@@ -156,3 +156,35 @@ def test_sums_over_neighbouring_axes(axes):
     f = nb.compile(lambda a: nb.reduce_sum(a, axis=axes))
     f(t)
     assert ("sum_axes" in f.dump_plan()) == (axes in ((0, 1), (0, 1, 2), (1, 2)))
+
+
+# ---------------------------------------------------------------- attention
+def _attention64(q, k, v, causal, mask=None):
+    s = q.double() @ k.double().transpose(-1, -2) * q.shape[-1] ** -0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(s.shape[-2:], dtype=torch.bool, device="cuda").tril(s.shape[-1] - s.shape[-2]), float("-inf"))
+    return torch.softmax(s if mask is None else s + mask.double(), -1) @ v.double()
+
+
+def _attention_check(q, k, v, causal, mask=None, grads=True):
+    """Products of bf16 operands with bf16 probabilities: each of the two roundings adds up to 2^-9 relative."""
+    from nabla_b200.native import attention
+
+    scale = q.shape[-1] ** -0.5
+    o, lse = attention.sdpa_fwd(q, k, v, causal=causal, scale=scale, mask=mask)
+    a, b, c = (t.double().requires_grad_(True) for t in (q, k, v))
+    ref = _attention64(a, b, c, causal, mask)
+    assert _rel2(o, ref) < 6e-3
+    if grads:
+        do = torch.randn_like(q)
+        got = attention.sdpa_bwd(do, q, k, v, o, lse, causal=causal, scale=scale, mask=mask)
+        for x, y in zip(got, torch.autograd.grad(ref, (a, b, c), do.double())):
+            assert _rel2(x, y) < 8e-3
+
+
+@pytest.mark.parametrize("B,H,S,D", [(5, 14, 1030, 128), (9, 16, 1030, 64), (1, 1, 129, 128), (3, 1, 2100, 64)])
+def test_causal_attention_in_tile_order(B, H, S, D):
+    """More (batch, head) pairs than one chunk of the launch order holds (and a last chunk that is not full)."""
+    torch.manual_seed(0)
+    q, k, v = (torch.randn(B, H, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    _attention_check(q, k, v, True)
