@@ -485,11 +485,14 @@ struct DkvSmem {
   static constexpr int TILE_BYTES = BT * HD * 2;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = OFF_K + TILE_BYTES;
-  static constexpr int OFF_Q = OFF_V + TILE_BYTES;        // 2 stages
-  static constexpr int OFF_DO = OFF_Q + 2 * TILE_BYTES;   // 2 stages
-  static constexpr int OFF_STAT = OFF_DO + 2 * TILE_BYTES;   // lse2[2][128], delta[2][128]
-  static constexpr int OFF_BAR = OFF_STAT + 4 * BT * 4;
-  static constexpr int RAW = OFF_BAR + 24 * 8 + 16 + 1024;
+  static constexpr int QST = 3;                           // Q stages: a Q tile is held from S^T until dK has read it,
+                                                          // so two would leave its load half a tile's time
+                                                          // (forward and backward at 64 heads x 2048: 461 -> 453 us)
+  static constexpr int OFF_Q = OFF_V + TILE_BYTES;        // QST stages
+  static constexpr int OFF_DO = OFF_Q + QST * TILE_BYTES; // 2 stages
+  static constexpr int OFF_STAT = OFF_DO + 2 * TILE_BYTES;   // lse2[QST][128], delta[2][128]
+  static constexpr int OFF_BAR = OFF_STAT + (QST + 2) * BT * 4;
+  static constexpr int RAW = OFF_BAR + 18 * 8 + 16;       // no slack: the kernel's shared memory is 1024-byte aligned
   static constexpr int TOTAL = RAW < 120 * 1024 ? 120 * 1024 : RAW;
 };
 
@@ -499,33 +502,34 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                      const BwdArgs args) {
   using L = DkvSmem<HD>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int QST = L::QST;
+  extern __shared__ __align__(1024) uint8_t smem_tiles[];
+  uint8_t* smem = smem_tiles;
   uint8_t* sK = smem + L::OFF_K;
   uint8_t* sV = smem + L::OFF_V;
   uint8_t* sQ = smem + L::OFF_Q;
   uint8_t* sDO = smem + L::OFF_DO;
-  float* s_nlse2 = reinterpret_cast<float*>(smem + L::OFF_STAT);   // [2][128]
-  float* s_ndelta = s_nlse2 + 2 * BT;                              // [2][128]
+  float* s_nlse2 = reinterpret_cast<float*>(smem + L::OFF_STAT);   // [QST][128]
+  float* s_ndelta = s_nlse2 + QST * BT;                            // [2][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* kv_full = bars + 0;
-  uint64_t* q_full = bars + 1;     // [2]  Q_i and its lse2 landed in stage i & 1
-  uint64_t* q_empty = bars + 3;    // [2]
-  uint64_t* do_full = bars + 5;    // [2]  dO_i and its delta landed
-  uint64_t* do_empty = bars + 7;   // [2]
-  uint64_t* s_full = bars + 9;     //      S^T of the current tile is in TMEM
-  uint64_t* dp_full = bars + 10;   //      dP^T of the current tile is in TMEM
-  uint64_t* p_full = bars + 11;    //      P^T written back (256 arrivals)
-  uint64_t* ds_full = bars + 12;   //      dS^T written back (256 arrivals)
-  uint64_t* all_done = bars + 13;
+  uint64_t* q_full = bars + 1;     // [QST] Q_i and its lse2 landed in stage i % QST
+  uint64_t* q_empty = bars + 4;    // [QST]
+  uint64_t* do_full = bars + 7;    // [2]  dO_i and its delta landed
+  uint64_t* do_empty = bars + 9;   // [2]
+  uint64_t* s_full = bars + 11;    //      S^T of the current tile is in TMEM
+  uint64_t* dp_full = bars + 12;   //      dP^T of the current tile is in TMEM
+  uint64_t* p_full = bars + 13;    //      P^T written back (256 arrivals)
+  uint64_t* ds_full = bars + 14;   //      dS^T written back (256 arrivals)
+  uint64_t* all_done = bars + 15;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  {
-    __shared__ int s_abort;
-    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(args.status);
-    __syncthreads();
-    if (s_abort != 0) return;
+  // an earlier bounded wait on this device already failed: leave (uniformly)
+  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return;
+  if (smem_u32(smem) & 1023u) {     // the swizzled tiles need it, and the size above leaves no room to align
+    if (threadIdx.x == 0) atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER);
+    return;
   }
   int bh_, jt;             // key tile 0 sees every query tile, the last one only a few
   tile_order(blockIdx.x, args.H * args.B, args.q_chunk, (args.Skv + BT - 1) / BT, bh_, jt);
@@ -548,9 +552,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
     mbar_init(kv_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < QST; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&q_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
       mbar_init(&do_full[i], 1);
       mbar_init(&do_empty[i], 1);
     }
@@ -581,16 +587,16 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tma_load_4d(sV + c * (BT * 128), &tmV, kv_full, c * 64, k0, h, b, args.Skv, args.H, args.B);
       }
       for (int it = 0; it < n_it; ++it) {
-        const int st = it & 1;
+        const int st = it & 1, qs = it % QST;
         const uint32_t ph = ((it >> 1) & 1) ^ 1;
         const int q0 = (i_start + it) * BT;
-        if (!mbar_wait(&q_empty[st], ph)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
-        mbar_arrive_expect_tx(&q_full[st], L::TILE_BYTES + BT * 4);
+        if (!mbar_wait(&q_empty[qs], ((it / QST) & 1) ^ 1)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
+        mbar_arrive_expect_tx(&q_full[qs], L::TILE_BYTES + BT * 4);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
-          tma_load_4d(sQ + st * L::TILE_BYTES + c * (BT * 128), &tmQ, &q_full[st], c * 64, q0, h, b, args.Sq, args.H, args.B);
+          tma_load_4d(sQ + qs * L::TILE_BYTES + c * (BT * 128), &tmQ, &q_full[qs], c * 64, q0, h, b, args.Sq, args.H, args.B);
         if (!NB_IN_BOUNDS(NB_SITE_ATTN_STAT_INDEX, q0 + BT - 1, args.Sq_pad)) break;   // debug build only
-        bulk_load_1d(s_nlse2 + st * BT, args.nlse2 + bh * args.Sq_pad + q0, BT * 4, &q_full[st]);
+        bulk_load_1d(s_nlse2 + qs * BT, args.nlse2 + bh * args.Sq_pad + q0, BT * 4, &q_full[qs]);
         if (!mbar_wait(&do_empty[st], ph)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
         mbar_arrive_expect_tx(&do_full[st], L::TILE_BYTES + BT * 4);
 #pragma unroll
@@ -614,22 +620,22 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         umma_commit(dp_full);
       }
       for (int it = 0; it < n_it && ok; ++it) {
-        const int st = it & 1;
+        const int st = it & 1, qs = it % QST, qn = (it + 1) % QST;
         const bool more = it + 1 < n_it;
         if (!mbar_wait(p_full, it & 1)) { ok = false; break; }
         tc_fence_after();
         mma_accum<HD>(t_dv, t_st, true, smem_u32(sDO + st * L::TILE_BYTES), it != 0);     // dV += P^T dO_i
         umma_commit(&do_empty[st]);
         if (more) {
-          if (!mbar_wait(&q_full[st ^ 1], ((it + 1) >> 1) & 1)) { ok = false; break; }
+          if (!mbar_wait(&q_full[qn], ((it + 1) / QST) & 1)) { ok = false; break; }
           tc_fence_after();
-          mma_scores<HD>(t_st, smem_u32(sK), smem_u32(sQ + (st ^ 1) * L::TILE_BYTES));
+          mma_scores<HD>(t_st, smem_u32(sK), smem_u32(sQ + qn * L::TILE_BYTES));
           umma_commit(s_full);
         }
         if (!mbar_wait(ds_full, it & 1)) { ok = false; break; }
         tc_fence_after();
-        mma_accum<HD>(t_dk, t_dpt, true, smem_u32(sQ + st * L::TILE_BYTES), it != 0);     // dK += dS^T Q_i
-        umma_commit(&q_empty[st]);
+        mma_accum<HD>(t_dk, t_dpt, true, smem_u32(sQ + qs * L::TILE_BYTES), it != 0);     // dK += dS^T Q_i
+        umma_commit(&q_empty[qs]);
         if (more) {
           if (!mbar_wait(&do_full[st ^ 1], ((it + 1) >> 1) & 1)) { ok = false; break; }
           tc_fence_after();
@@ -651,9 +657,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const float* mbase = args.mask.ptr == nullptr ? nullptr : args.mask.ptr + b * args.mask.sb + h * args.mask.sh + key;
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
-      const int st = it & 1;
+      const int st = it & 1, qs = it % QST;
       const int q0 = (i_start + it) * BT + grp * 64;
-      if (ok && !(mbar_wait(&q_full[st], (it >> 1) & 1) && mbar_wait(s_full, it & 1))) {
+      if (ok && !(mbar_wait(&q_full[qs], (it / QST) & 1) && mbar_wait(s_full, it & 1))) {
         atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
         ok = false;
       }
@@ -681,7 +687,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         tmem_st_wait();
       }
-      const float2* nl2 = reinterpret_cast<const float2*>(s_nlse2 + st * BT + grp * 64);
+      const float2* nl2 = reinterpret_cast<const float2*>(s_nlse2 + qs * BT + grp * 64);
       const float2 sc2 = make_float2(args.scale_log2, args.scale_log2);
       float2 p[32];
       uint32_t va[32], vb[32];
