@@ -188,3 +188,30 @@ def test_causal_attention_in_tile_order(B, H, S, D):
     torch.manual_seed(0)
     q, k, v = (torch.randn(B, H, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
     _attention_check(q, k, v, True)
+
+
+@pytest.mark.parametrize("S,D,causal", [(130, 64, False), (257, 128, False), (777, 64, True), (64, 128, False)])
+@pytest.mark.parametrize("shape", ["b11k", "bh1k", "11qk"])
+def test_attention_with_additive_masks(S, D, causal, shape):
+    """One mask row for all queries (shared memory in the kernels) and one per query, hidden keys as -1e9 and as
+    -inf."""
+    torch.manual_seed(2)
+    B, H = 2, 3
+    q, k, v = (torch.randn(B, H, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    mask = torch.randn({"b11k": (B, 1, 1, S), "bh1k": (B, H, 1, S), "11qk": (1, 1, S, S)}[shape], device="cuda")
+    hide = torch.rand(mask.shape, device="cuda") < 0.3
+    hide[..., 0] = False                              # every row keeps a key, the causal ones too
+    _attention_check(q, k, v, causal, mask.masked_fill(hide, -1e9))
+    _attention_check(q, k, v, causal, mask.masked_fill(hide, float("-inf")))
+
+
+def test_attention_rows_without_a_visible_key_are_zero():
+    from nabla_b200.native import attention
+
+    q, k, v = (torch.randn(2, 2, 150, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    mask = torch.zeros(2, 1, 1, 150, device="cuda")
+    mask[1] = float("-inf")
+    o, lse = attention.sdpa_fwd(q, k, v, causal=False, scale=0.125, mask=mask)
+    assert bool((o[1] == 0).all()) and bool((lse[1] == float("-inf")).all()) and bool(torch.isfinite(lse[0]).all())
+    for g in attention.sdpa_bwd(torch.randn_like(q), q, k, v, o, lse, causal=False, scale=0.125, mask=mask):
+        assert bool(torch.isfinite(g).all()) and bool((g[1] == 0).all())
