@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(128, 4) layernorm_bwd_dx_kernel(const T* __res
   }
 }
 
-// Backward in one pass (rows of up to 8 vectors per lane): a persistent grid of warps walks the rows,
+// Backward in one pass (rows of one vector per lane): a persistent grid of warps walks the rows,
 // each warp computing dx of its row as above while it also adds the row's dy * xhat and dy into
 // per-lane register accumulators for the columns it holds, so dy and x are read from DRAM once
 // instead of twice. At the end the four warps of a block fold their accumulators through shared
@@ -349,7 +349,122 @@ __global__ void __launch_bounds__(128, (VPL * Vec<T>::N >= 64 ? 2 : VPL * Vec<T>
   }
 }
 
-// Backward, part 2 (rows wider than that): dgamma = sum_rows dy * xhat, dbeta = sum_rows dy. Block = 32*V columns x a
+// Backward in one pass for wider rows: NW warps share a row, one 16-byte vector of x and dy per thread, so
+// gamma and the column sums of a thread's V columns sit in registers for the whole launch and 32 warps fit
+// an SM (a warp per row holds 8 vectors per lane and their sums in 200 registers: 8 warps per SM, and half
+// of HBM's rate left unused). RB = 8 / NW rows per block at a time, two of them in flight per thread; the row
+// sums meet in shared memory, double buffered, one barrier per two rows. 16384 x 2048 bf16: 83 -> 52 us with the
+// column sums' second launch; 8192 x 4096: 165 -> 65 us. Each block writes one row of
+// `partial` as above.
+constexpr int LN_MAX_WARPS = 16;
+template <typename T>
+__global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
+    layernorm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
+                              const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
+                              float* __restrict__ partial, int rows, int D, int NW, int RB) {
+  constexpr int V = Vec<T>::N, P = V / 2;
+  __shared__ float4 red[2][LN_MAX_WARPS];
+  __shared__ float sh[2][4 * 32 * V];                // RB > 1 means NW <= 4
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, slot = wid / NW, c = ((wid - slot * NW) * 32 + lane) * V;
+  const bool act = c < D;
+  const float inv_d = 1.f / D;
+  float2 gm[P], ag[P], ab[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) { gm[k] = make_float2(1.f, 1.f); ag[k] = ab[k] = make_float2(0.f, 0.f); }
+  if (gamma && act) unpack_pairs<T>(*reinterpret_cast<const uint4*>(gamma + c), gm);
+  const int stride = gridDim.x * RB;
+  int buf = 0;
+  for (int base = blockIdx.x * RB; base < rows; base += 2 * stride, buf ^= 1) {
+    uint4 xr[2], dr[2];
+    float rs[2], nmr[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int row = base + u * stride + slot;
+      xr[u] = dr[u] = make_uint4(0, 0, 0, 0);
+      rs[u] = nmr[u] = 0.f;
+      if (row < rows) {
+        if (act) {
+          xr[u] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + c);
+          dr[u] = *reinterpret_cast<const uint4*>(dy + (size_t)row * D + c);
+        }
+        rs[u] = rstd[row];
+        nmr[u] = -mean[row] * rs[u];
+      }
+    }
+    float s[4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), xv[P], dv[P];
+      const float2 rs2 = make_float2(rs[u], rs[u]), nmr2 = make_float2(nmr[u], nmr[u]);
+      unpack_pairs<T>(xr[u], xv);
+      unpack_pairs<T>(dr[u], dv);
+      if (act) {
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          const float2 xh = __ffma2_rn(xv[k], rs2, nmr2);              // (x - mean) * rstd
+          const float2 g = __fmul2_rn(dv[k], gm[k]);
+          s1 = __fadd2_rn(s1, g);
+          s2 = __ffma2_rn(g, xh, s2);
+          ag[k] = __ffma2_rn(dv[k], xh, ag[k]);
+          ab[k] = __fadd2_rn(ab[k], dv[k]);
+        }
+      }
+      s[2 * u] = s1.x + s1.y;
+      s[2 * u + 1] = s2.x + s2.y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+    if (lane == 0) red[buf][wid] = make_float4(s[0], s[1], s[2], s[3]);
+    __syncthreads();
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < NW; ++k) {
+      const float4 r = red[buf][slot * NW + k];
+      t.x += r.x; t.y += r.y; t.z += r.z; t.w += r.w;
+    }
+    const float m1[2] = {t.x * inv_d, t.z * inv_d}, m2[2] = {t.y * inv_d, t.w * inv_d};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int row = base + u * stride + slot;
+      if (act && row < rows) {
+        // dx = rstd * (g - m1 - xhat * m2) = g * rstd + (xhat * (-rstd * m2) + (-rstd * m1))
+        const float2 rs2 = make_float2(rs[u], rs[u]), nmr2 = make_float2(nmr[u], nmr[u]);
+        const float2 a2 = make_float2(-rs[u] * m2[u], -rs[u] * m2[u]), b2 = make_float2(-rs[u] * m1[u], -rs[u] * m1[u]);
+        float2 xv[P], dv[P], o[P];
+        unpack_pairs<T>(xr[u], xv);
+        unpack_pairs<T>(dr[u], dv);
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+          o[k] = __ffma2_rn(__fmul2_rn(dv[k], gm[k]), rs2, __ffma2_rn(__ffma2_rn(xv[k], rs2, nmr2), a2, b2));
+        *reinterpret_cast<uint4*>(dx + (size_t)row * D + c) = pack_pairs<T>(o);
+      }
+    }
+  }
+  float* prow = partial + (size_t)blockIdx.x * 2 * D;
+  for (int r = 0; r < RB; ++r) {                     // fold the row slots, in order
+    if (slot == r && act) {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        float2 g = ag[k], b = ab[k];
+        if (r > 0) {
+          g.x += sh[0][c + 2 * k]; g.y += sh[0][c + 2 * k + 1];
+          b.x += sh[1][c + 2 * k]; b.y += sh[1][c + 2 * k + 1];
+        }
+        if (r == RB - 1) {
+          *reinterpret_cast<float2*>(prow + c + 2 * k) = g;
+          *reinterpret_cast<float2*>(prow + D + c + 2 * k) = b;
+        } else {
+          sh[0][c + 2 * k] = g.x; sh[0][c + 2 * k + 1] = g.y;
+          sh[1][c + 2 * k] = b.x; sh[1][c + 2 * k + 1] = b.y;
+        }
+      }
+    }
+    if (RB > 1) __syncthreads();
+  }
+}
+
+// Backward, part 2 of the two-kernel layout: dgamma = sum_rows dy * xhat, dbeta = sum_rows dy. Block = 32*V columns x a
 // slab of rows; 8 warps stride over the slab's rows with register accumulators; partial sums go
 // to `partial` ([gridDim.y][2][D] fp32) and are folded by colsum_partials_kernel.
 template <typename T>
@@ -395,31 +510,24 @@ __global__ void __launch_bounds__(256) layernorm_bwd_dgb_kernel(const T* __restr
 }
 
 // out0[c] = sum_b partial[b][0][c], out1[c] = sum_b partial[b][1][c]  (two planes of width D per row
-// of `partial`). A block covers 32 columns; its 8 warps take every 8th row, so a few hundred rows of
-// partials are a few dozen dependent loads per thread instead of a few hundred.
+// of `partial`). A block covers 32 columns of one plane; its 32 warps take every 32nd row, so several hundred
+// rows of partials are a dozen or two loads per thread.
 template <typename T>
-__global__ void __launch_bounds__(256) colsum_partials_kernel(const float* __restrict__ partial, T* __restrict__ out0,
-                                                             T* __restrict__ out1, int nblocks, int D) {
-  __shared__ float sh[2][8][32];
+__global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __restrict__ partial, T* __restrict__ out0,
+                                                              T* __restrict__ out1, int nblocks, int D) {
+  __shared__ float sh[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
-  float a = 0.f, b = 0.f;
+  float a = 0.f;
   if (c < D) {
-    for (int i = w; i < nblocks; i += 8) {
-      a += partial[(size_t)i * 2 * D + c];
-      b += partial[(size_t)i * 2 * D + D + c];
-    }
+#pragma unroll 8
+    for (int i = w; i < nblocks; i += 32) a += partial[((size_t)i * 2 + blockIdx.y) * D + c];
   }
-  sh[0][w][lane] = a;
-  sh[1][w][lane] = b;
+  sh[w][lane] = a;
   __syncthreads();
-  if (w == 0 && c < D) {
-    float sa = 0.f, sb = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { sa += sh[0][k][lane]; sb += sh[1][k][lane]; }
-    if (out0) out0[c] = from_f<T>(sa);
-    if (out1) out1[c] = from_f<T>(sb);
-  }
+  a = warp_sum(sh[lane][w]);                         // warp w: column w of the block's 32
+  T* out = blockIdx.y ? out1 : out0;
+  if (lane == 0 && blockIdx.x * 32 + w < D && out) out[blockIdx.x * 32 + w] = from_f<T>(a);
 }
 
 // out[i] = sum_z part[z][i], fp32 slices of n: 32 results per block, its 8 warps take every 8th slice.
@@ -1588,23 +1696,26 @@ int nb_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y
 }
 
 // Number of rows of the `partial` scratch buffer (each 2*D floats) that nb_layernorm_bwd writes for
-// this problem: the grid of the one-pass kernel when the row fits 8 vectors per lane, else the
-// number of row slabs of the two-kernel path.
+// this problem: the grid of the one-pass kernels, or the number of row slabs of the two-kernel path.
 static int ln_bwd_vpl(int D, int dtype) { const int V = dtype ? 8 : 4; return (D / V + 31) / 32; }
 static int g_ln_bwd_two_kernels = 0;
 // 1: always take the two-kernel path (dx, then dgamma / dbeta), for comparisons.
 void nb_layernorm_bwd_two_kernels(int on) { g_ln_bwd_two_kernels = on; }
 int nb_layernorm_bwd_nblocks(int rows, int D, int dtype) {
-  const int vpl = ln_bwd_vpl(D, dtype);
-  if (vpl <= 8 && !g_ln_bwd_two_kernels) {
-    const int V = dtype ? 8 : 4;
-    const int cap = 148 * (vpl * V >= 64 ? 2 : vpl * V >= 32 ? 3 : 4);   // resident blocks of the kernel
-    int nb = (rows + 3) / 4;
-    if (nb > cap) nb = cap;
-    return nb < 1 ? 1 : nb;
+  const int vpl = ln_bwd_vpl(D, dtype);              // = warps that share a row in layernorm_bwd_rows_kernel
+  int nb, cap;
+  if (g_ln_bwd_two_kernels || vpl > LN_MAX_WARPS) {
+    nb = (rows + 255) / 256;
+    cap = 128;
+  } else if (vpl == 1) {
+    nb = (rows + 3) / 4;
+    cap = 148 * 4;
+  } else {                                           // 32 warps per SM, two rows per slot and iteration
+    const int rb = vpl < 8 ? 8 / vpl : 1;
+    nb = (rows + 2 * rb - 1) / (2 * rb);
+    cap = 148 * (32 / (vpl * rb));
   }
-  int nb = (rows + 255) / 256;
-  if (nb > 128) nb = 128;
+  if (nb > cap) nb = cap;
   return nb < 1 ? 1 : nb;
 }
 
@@ -1614,39 +1725,43 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
   const int V = dtype ? 8 : 4;
   if (D % V) return -2;
   const int vpl = ln_bwd_vpl(D, dtype);
+  if (vpl > LN_MAX_WARPS) return -3;
   const int nb = nb_layernorm_bwd_nblocks(rows, D, dtype);
   const int rpb = (rows + nb - 1) / nb;
   dim3 grid_dx((rows + 3) / 4);
   dim3 grid_gb((D + 32 * V - 1) / (32 * V), nb);
-#define LN_BWD1(T, VPL)                                                                                               \
-  {                                                                                                                   \
-    layernorm_bwd_fused_kernel<T, VPL><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
-                                                               (T*)dx, partial, rows, D);                            \
-    colsum_partials_kernel<T><<<(D + 31) / 32, 256, 0, STREAM>>>(partial, (T*)dgamma, (T*)dbeta, nb, D);            \
-  }
 #define LN_BWD(T, VPL)                                                                                                \
   {                                                                                                                   \
     layernorm_bwd_dx_kernel<T, VPL><<<grid_dx, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean,    \
                                                                   rstd, (T*)dx, rows, D);                            \
     layernorm_bwd_dgb_kernel<T><<<grid_gb, 256, 0, STREAM>>>((const T*)dy, (const T*)x, mean, rstd, partial, rows, D, \
                                                               rpb);                                                   \
-    colsum_partials_kernel<T><<<(D + 31) / 32, 256, 0, STREAM>>>(partial, (T*)dgamma, (T*)dbeta, nb, D);            \
   }
-  if (g_ln_bwd_two_kernels) {
-    if (dtype) {
-      if (vpl <= 1) LN_BWD(bf16, 1) else if (vpl <= 2) LN_BWD(bf16, 2) else if (vpl <= 4) LN_BWD(bf16, 4)
-      else if (vpl <= 8) LN_BWD(bf16, 8) else if (vpl <= 16) LN_BWD(bf16, 16) else return -3;
-    } else {
-      if (vpl <= 1) LN_BWD(float, 1) else if (vpl <= 2) LN_BWD(float, 2) else if (vpl <= 4) LN_BWD(float, 4)
-      else if (vpl <= 8) LN_BWD(float, 8) else if (vpl <= 16) LN_BWD(float, 16) else return -3;
-    }
+#define LN_BWD_ONE_PASS(T)                                                                                            \
+  {                                                                                                                   \
+    if (vpl == 1)                                                                                                     \
+      layernorm_bwd_fused_kernel<T, 1><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean,      \
+                                                               rstd, (T*)dx, partial, rows, D);                      \
+    else {                                                                                                            \
+      const int rb = vpl < 8 ? 8 / vpl : 1;                                                                           \
+      layernorm_bwd_rows_kernel<T><<<nb, 32 * vpl * rb, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma,      \
+                                                                     mean, rstd, (T*)dx, partial, rows, D, vpl, rb); \
+    }                                                                                                                 \
+  }
+  if (!g_ln_bwd_two_kernels) {
+    if (dtype) LN_BWD_ONE_PASS(bf16) else LN_BWD_ONE_PASS(float)
   } else if (dtype) {
-    if (vpl <= 1) LN_BWD1(bf16, 1) else if (vpl <= 2) LN_BWD1(bf16, 2) else if (vpl <= 4) LN_BWD1(bf16, 4)
-    else if (vpl <= 8) LN_BWD1(bf16, 8) else if (vpl <= 16) LN_BWD(bf16, 16) else return -3;
+    if (vpl <= 1) LN_BWD(bf16, 1) else if (vpl <= 2) LN_BWD(bf16, 2) else if (vpl <= 4) LN_BWD(bf16, 4)
+    else if (vpl <= 8) LN_BWD(bf16, 8) else LN_BWD(bf16, 16)
   } else {
-    if (vpl <= 1) LN_BWD1(float, 1) else if (vpl <= 2) LN_BWD1(float, 2) else if (vpl <= 4) LN_BWD1(float, 4)
-    else if (vpl <= 8) LN_BWD1(float, 8) else if (vpl <= 16) LN_BWD(float, 16) else return -3;
+    if (vpl <= 1) LN_BWD(float, 1) else if (vpl <= 2) LN_BWD(float, 2) else if (vpl <= 4) LN_BWD(float, 4)
+    else if (vpl <= 8) LN_BWD(float, 8) else LN_BWD(float, 16)
   }
+#undef LN_BWD
+#undef LN_BWD_ONE_PASS
+  const dim3 grid_fold((D + 31) / 32, 2);
+  if (dtype) colsum_partials_kernel<bf16><<<grid_fold, 1024, 0, STREAM>>>(partial, (bf16*)dgamma, (bf16*)dbeta, nb, D);
+  else colsum_partials_kernel<float><<<grid_fold, 1024, 0, STREAM>>>(partial, (float*)dgamma, (float*)dbeta, nb, D);
   return CHECK_LAUNCH();
 }
 

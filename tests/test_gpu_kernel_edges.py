@@ -215,3 +215,25 @@ def test_attention_rows_without_a_visible_key_are_zero():
     assert bool((o[1] == 0).all()) and bool((lse[1] == float("-inf")).all()) and bool(torch.isfinite(lse[0]).all())
     for g in attention.sdpa_bwd(torch.randn_like(q), q, k, v, o, lse, causal=False, scale=0.125, mask=mask):
         assert bool(torch.isfinite(g).all()) and bool((g[1] == 0).all())
+
+
+# ---------------------------------------------------------------- layer norm backward
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,vectors", [(1, 32), (5, 33), (2, 64), (1000, 65), (3, 96), (777, 125), (4, 128), (9, 160), (300, 224), (6, 256), (5000, 256),
+                                          (2, 257), (33, 512)])
+def test_layer_norm_backward_by_row_width(dtype, rows, vectors):
+    """One warp per row, 2 to 16 warps per row with one or several rows per block, last warps that are partly
+    idle, fewer rows than a block holds and many times the grid."""
+    from nabla_b200.native import kernels
+
+    D = vectors * (8 if dtype is torch.bfloat16 else 4)
+    torch.manual_seed(4)
+    x, dy = (torch.randn(rows, D, device="cuda").add_(0.5).to(dtype) for _ in range(2))
+    for g in (torch.randn(D, device="cuda").to(dtype), None):
+        _, mean, rstd = kernels.layernorm_fwd(x, g, None, 1e-5)
+        got = kernels.layernorm_bwd(dy, x, g, mean, rstd)
+        a, b, c = x.double().requires_grad_(True), (torch.ones(D, device="cuda") if g is None else g).double().requires_grad_(True), \
+            torch.zeros(D, dtype=torch.float64, device="cuda").requires_grad_(True)
+        ref = torch.autograd.grad(TF.layer_norm(a, (D,), b, c, 1e-5), (a, b, c), dy.double())
+        for y, r in zip(got, ref):
+            assert _rel2(y, r) < STORED[dtype]
