@@ -1662,6 +1662,53 @@ __global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict
   }
 }
 
+// ============================================================== many copies, one launch
+// The inputs of a captured step are copied into the graph's buffers and its results out of them: dozens of
+// tensors of a few KB, for which a launch each is the whole cost. Up to COPY_MAX copies ride in one launch's
+// parameters; a block moves one COPY_CHUNK of one of them, found by bisection over the chunk counts.
+constexpr int COPY_MAX = 128, COPY_CHUNK = 32 * 1024;
+struct CopyBatch {
+  void* dst[COPY_MAX];
+  const void* src[COPY_MAX];
+  unsigned long long bytes[COPY_MAX];
+  unsigned first[COPY_MAX + 1];        // first block of every copy; first[n] = blocks
+  int n;
+};
+template <typename W>
+__device__ __forceinline__ void copy_words(void* dst, const void* src, unsigned bytes) {
+  const unsigned words = bytes / sizeof(W);
+  W* d = reinterpret_cast<W*>(dst);
+  const W* s = reinterpret_cast<const W*>(src);
+  unsigned i = threadIdx.x;
+  for (; i + 3 * 256 < words; i += 4 * 256) {
+    W v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = s[i + u * 256];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) d[i + u * 256] = v[u];
+  }
+  for (; i < words; i += 256) d[i] = s[i];
+  for (unsigned b = words * sizeof(W) + threadIdx.x; b < bytes; b += 256)
+    reinterpret_cast<uint8_t*>(dst)[b] = reinterpret_cast<const uint8_t*>(src)[b];
+}
+__global__ void __launch_bounds__(256) copy_batch_kernel(const __grid_constant__ CopyBatch c) {
+  int lo = 0, hi = c.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (c.first[mid] <= blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const unsigned long long at = (unsigned long long)(blockIdx.x - c.first[lo]) * COPY_CHUNK, total = c.bytes[lo];
+  if (at >= total) return;
+  char* dst = static_cast<char*>(c.dst[lo]) + at;
+  const char* src = static_cast<const char*>(c.src[lo]) + at;
+  const unsigned n = (unsigned)(total - at < COPY_CHUNK ? total - at : COPY_CHUNK);
+  const unsigned align = (unsigned)((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u);
+  if (align == 0) copy_words<uint4>(dst, src, n);
+  else if ((align & 3u) == 0) copy_words<unsigned>(dst, src, n);
+  else if ((align & 1u) == 0) copy_words<unsigned short>(dst, src, n);
+  else copy_words<uint8_t>(dst, src, n);
+}
+
 static inline int grid_for(size_t n, int per_block, int cap = 148 * 16) {
   size_t g = (n + per_block - 1) / per_block;
   if (g < 1) g = 1;
@@ -1925,6 +1972,35 @@ int nb_embedding_scatter_sorted(const long long* sorted_ids, const long long* pe
   if (dtype) embedding_scatter_sorted_kernel<bf16><<<n_ids, 128, 0, STREAM>>>(sorted_ids, perm, (const bf16*)upd, (const bf16*)base, (bf16*)out, n_ids, D, vocab);
   else embedding_scatter_sorted_kernel<float><<<n_ids, 128, 0, STREAM>>>(sorted_ids, perm, (const float*)upd, (const float*)base, (float*)out, n_ids, D, vocab);
   return CHECK_LAUNCH();
+}
+
+// n copies of bytes[i] bytes from src[i] to dst[i] (host arrays; the ranges do not overlap), as few launches as
+// the parameter space allows. Returns the number of launches, or a negative code.
+int nb_copy_batch(void* const* dst, const void* const* src, const unsigned long long* bytes, int n, void* stream) {
+  int launches = 0;
+  for (int i = 0; i < n;) {
+    CopyBatch c;
+    unsigned long long blocks = 0;
+    c.n = 0;
+    for (; i < n && c.n < COPY_MAX; ++i) {
+      const unsigned long long k = (bytes[i] + COPY_CHUNK - 1) / COPY_CHUNK;
+      if (k == 0) continue;
+      if (blocks + k > 0x7fffffffull) {
+        if (c.n == 0) return -4;
+        break;
+      }
+      c.dst[c.n] = dst[i];
+      c.src[c.n] = src[i];
+      c.bytes[c.n] = bytes[i];
+      c.first[c.n++] = (unsigned)blocks;
+      blocks += k;
+    }
+    if (c.n == 0) break;
+    c.first[c.n] = (unsigned)blocks;
+    copy_batch_kernel<<<(unsigned)blocks, 256, 0, STREAM>>>(c);
+    ++launches;
+  }
+  return cudaGetLastError() == cudaSuccess ? launches : -1;
 }
 
 int nb_cast(const void* in, void* out, long long n, int in_dtype, int out_dtype, void* stream) {

@@ -36,6 +36,7 @@ def _L():
             "nb_embedding_scatter_add": [c_vp] * 5 + [c_int] * 4 + [c_vp],
             "nb_embedding_scatter_sorted": [c_vp] * 5 + [c_int] * 4 + [c_vp],
             "nb_cast": [c_vp, c_vp, c_ll, c_int, c_int, c_vp],
+            "nb_copy_batch": [c_vp, c_vp, c_vp, c_int, c_vp],
             "nb_activation": [c_vp] * 3 + [c_ll, c_int, c_int, c_int, c_vp],
             "nb_rng": [c_vp, c_ll, c_ull, c_ull, c_int, c_f, c_f, c_int, c_vp],
             "nb_dropout": [c_vp] * 3 + [c_ll, c_f, c_ull, c_ull, c_int, c_vp],
@@ -250,6 +251,67 @@ def embedding_scatter_add(base: torch.Tensor | None, ids: torch.Tensor, upd: tor
                                       stream_ptr()), "embedding_scatter_add")
     launch_count += 1
     return out
+
+
+def _is_dense(t: torch.Tensor) -> bool:
+    """No gaps and no overlaps between the elements, in any order of the dims: one run of bytes."""
+    want = 1
+    for st, n in sorted((st, n) for st, n in zip(t.stride(), t.shape) if n != 1):
+        if st != want:
+            return False
+        want *= n
+    return True
+
+
+class CopyBatch:
+    """Copies between a fixed list of tensors and equally laid out ones that come with each call, all in one
+    launch (or one per 128 tensors). ``shared``: callers may hold views of the fixed tensors' memory."""
+
+    def __init__(self, fixed: list[torch.Tensor], shared: bool = False):
+        n = len(fixed)
+        dev = torch.cuda.current_device()
+        self.fixed = fixed
+        self.strides = [t.stride() for t in fixed]
+        self.fixed_ptrs = (c_vp * n)(*[t.data_ptr() for t in fixed])
+        self.own = [t.data_ptr() for t in fixed]
+        self.other_ptrs = (c_vp * n)()
+        self.size = [t.numel() * t.element_size() for t in fixed]
+        self.bytes = (c_ull * n)()
+        # what one launch can move: dense tensors of this device (a CPU scalar among the inputs is not one)
+        self.plain = [t.is_cuda and t.device.index == dev and _is_dense(t) for t in fixed]
+        self.storages = {t.untyped_storage().data_ptr() for t in fixed} if shared else None
+
+    def run(self, others: list[torch.Tensor], into_fixed: bool) -> None:
+        """``fixed <- others`` (``into_fixed``) or ``others <- fixed``. A pair that shares its storage is left
+        alone; one whose layouts differ goes through torch's copy, and so does every pair, in order, when a
+        source lies in the memory of another pair's destination."""
+        global launch_count
+        ptrs, nbytes, own, copies = self.other_ptrs, self.bytes, self.own, False
+        for i, o in enumerate(others):
+            p = o.data_ptr()
+            nbytes[i] = 0
+            if p == own[i]:
+                continue
+            f = self.fixed[i]
+            if self.storages is not None and o.untyped_storage().data_ptr() in self.storages:
+                for f, o in zip(self.fixed, others):
+                    if f.data_ptr() != o.data_ptr():
+                        f.copy_(o) if into_fixed else o.copy_(f)
+                return
+            if self.plain[i] and o.dtype is f.dtype and o.stride() == self.strides[i] and o.device == f.device:
+                ptrs[i] = p
+                nbytes[i] = self.size[i]
+                copies = True
+        for i, o in enumerate(others):
+            if nbytes[i] == 0 and self.size[i] and o.data_ptr() != own[i]:
+                self.fixed[i].copy_(o) if into_fixed else o.copy_(self.fixed[i])
+        if not copies:
+            return
+        dst, src = (self.fixed_ptrs, ptrs) if into_fixed else (ptrs, self.fixed_ptrs)
+        k = _L().nb_copy_batch(dst, src, nbytes, len(own), stream_ptr())
+        if k < 0:
+            raise RuntimeError(f"copy_batch failed with code {k}")
+        launch_count += k
 
 
 def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:

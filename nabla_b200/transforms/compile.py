@@ -182,6 +182,8 @@ class _Recorded:
         self.out_cached: list | None = None         # Tensor objects of outputs that alias donated inputs
         self.static_inputs: list[list[torch.Tensor]] | None = None
         self.static_outputs: list[list[torch.Tensor]] | None = None
+        self.copy_in = None                         # (CopyBatch) one-launch copies into the graph's inputs / out of its results
+        self.copy_out = None
         self.side_steps: set[int] = set()           # optimizer updates that run on a side stream, under the backward
         self.host_sync = False                      # holds a node that reads a device value on the host
         self.sizes: dict[str, int] = {}             # value of every named dynamic dimension in this recording
@@ -261,7 +263,7 @@ class CompiledFunction:
                 if not isinstance(rec, _Recorded):
                     continue
                 rec.cuda_graph = None
-                rec.static_inputs = rec.static_outputs = rec.out_cached = None
+                rec.static_inputs = rec.static_outputs = rec.out_cached = rec.copy_in = rec.copy_out = None
                 for ph in rec.placeholders:
                     ph._buffers = None
                 for outs in rec.keep:
@@ -780,10 +782,11 @@ class CompiledFunction:
             # those buffers up. The static copy of any other argument is overwritten by the next
             # call's copy-in, so a result that aliases it is cloned out below.
             rec.static_ptrs = {b.data_ptr() for bufs, d in zip(rec.static_inputs, rec.donated) if d for b in bufs}
-        for bufs, t in zip(rec.static_inputs, tensors):
-            for dst, src in zip(bufs, t._impl._buffers):
-                if dst.data_ptr() != src.data_ptr():
-                    dst.copy_(src)
+            from ..native.kernels import CopyBatch
+
+            rec.copy_in = CopyBatch([b for bufs in rec.static_inputs for b in bufs], shared=any(rec.donated))
+            rec.copy_out = None
+        rec.copy_in.run([b for t in tensors for b in t._impl._buffers], into_fixed=True)
         rec.cuda_graph.replay()
         if rec.out_cached is None:
             # results that live entirely in a donated input's buffers are the same storage on
@@ -796,6 +799,14 @@ class CompiledFunction:
                                                                 batch_dims=impl.batch_dims)))
                 else:
                     rec.out_cached.append(None)
+            from ..native.kernels import CopyBatch
+
+            rec.copy_out = CopyBatch([b for impl, bufs, cached in zip(rec.out_impls, rec.static_outputs, rec.out_cached)
+                                      if impl is not None and cached is None for b in bufs if b.data_ptr() not in rec.static_ptrs])
+        # every other result leaves the graph's memory: fresh tensors, filled by one launch
+        fresh = [torch.empty_like(b) for b in rec.copy_out.fixed]
+        rec.copy_out.run(fresh, into_fixed=False)
+        taken = iter(fresh)
         outs = []
         for impl, static, bufs, cached in zip(rec.out_impls, rec.out_static, rec.static_outputs, rec.out_cached):
             if impl is None:
@@ -803,7 +814,7 @@ class CompiledFunction:
             elif cached is not None:
                 outs.append(cached)
             else:
-                res = [b if b.data_ptr() in rec.static_ptrs else b.clone() for b in bufs]
+                res = [b if b.data_ptr() in rec.static_ptrs else next(taken) for b in bufs]
                 new = TensorImpl(res, shape=impl._shape, dtype=impl.dtype, device=impl.device,
                                  sharding=impl.sharding, batch_dims=impl.batch_dims)
                 outs.append(Tensor(impl=new))

@@ -237,3 +237,50 @@ def test_layer_norm_backward_by_row_width(dtype, rows, vectors):
         ref = torch.autograd.grad(TF.layer_norm(a, (D,), b, c, 1e-5), (a, b, c), dy.double())
         for y, r in zip(got, ref):
             assert _rel2(y, r) < STORED[dtype]
+
+
+# ---------------------------------------------------------------- copies around a captured step
+def test_copy_batch_moves_every_size_alignment_and_type():
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(5)
+    pool = torch.randint(0, 255, (1 << 20,), dtype=torch.uint8, device="cuda")
+    src = [pool[o:o + n] for o in (0, 1, 2, 3, 4, 8, 16) for n in (0, 1, 2, 3, 15, 16, 17, 4095, 32768, 32769, 100001)]
+    src += [torch.randn(n, device="cuda") for n in (1, 7, 300)] + [torch.randn(5, 9, device="cuda", dtype=torch.bfloat16).t() for _ in range(70)]
+    src += [torch.randn(6, 8, device="cuda")[:, :5], torch.tensor(3.0), torch.arange(4, device="cuda")]
+    fixed = [torch.empty_like(t) for t in src]
+    assert len(src) > 128
+    batch = kernels.CopyBatch(fixed)
+    for _ in range(2):
+        batch.run(src, into_fixed=True)
+        assert all(torch.equal(a, b) for a, b in zip(src, fixed))
+        src = [t if t.dtype is not torch.float32 else t + 1 for t in src]
+    out = [torch.empty_like(t) for t in fixed]
+    batch.run(out, into_fixed=False)
+    assert all(torch.equal(a, b) for a, b in zip(out, fixed))
+
+
+def test_copy_batch_keeps_the_order_where_pairs_share_memory():
+    from nabla_b200.native import kernels
+
+    a, b = torch.zeros(8, device="cuda"), torch.ones(8, device="cuda")
+    kernels.CopyBatch([a, b], shared=True).run([b, a], into_fixed=True)     # one after the other: a <- b, then b <- a
+    assert bool((a == 1).all()) and bool((b == 1).all())
+
+
+def test_captured_function_with_odd_inputs():
+    """Views, a CPU scalar, an input returned as it is and one returned twice, and results that stay valid."""
+    import nabla_b200 as nb
+
+    f = nb.compile(lambda x, y, s: (x @ y, x, nb.relu(y), y + s, y), cuda_graph=True)
+    first = None
+    for i in range(4):
+        x = torch.randn(33, 40, device="cuda").t()[:, :17]
+        y = torch.randn(17, 24, device="cuda")[:, ::2]
+        s = torch.randn(12, device="cuda")
+        out = [t.to_torch() for t in f(*(nb.Tensor.from_torch(t) for t in (x, y, s)))]
+        for got, ref in zip(out, (x @ y, x, y.relu(), y + s, y)):
+            torch.testing.assert_close(got, ref, rtol=1e-4, atol=1e-4)
+        if first is not None:
+            assert torch.equal(first[0], first[1])
+        first = (out[1], x)
