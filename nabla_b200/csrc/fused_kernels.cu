@@ -1239,9 +1239,11 @@ __global__ void __launch_bounds__(256) nf4_dequant_kernel(const uint8_t* __restr
 }
 
 // One code per byte (the layout of the QLoRA weight dict: `indices` uint8 [padded_numel], `scales`
-// fp32 per block) and the 16-entry codebook passed by the caller. 16 codes per thread: one 16-byte
-// load of codes, the block scale read once per run of codes in the same block.
-template <typename T>
+// fp32 per block) and the 16-entry codebook passed by the caller. 16 codes per thread: one 16-byte load of
+// codes and, where the scale blocks are whole multiples of 16 codes (WHOLE), one scale; the results leave as
+// 16-byte stores. A 64-bit division and a 2- or 4-byte store per element, as it was before, bound the kernel
+// by instructions instead of the 1 + sizeof(T) bytes per weight that it has to move.
+template <typename T, bool WHOLE>
 __global__ void __launch_bounds__(256) nf4_dequant_codes_kernel(const uint8_t* __restrict__ codes,
                                                                const float* __restrict__ absmax,
                                                                const float* __restrict__ codebook, T* __restrict__ out,
@@ -1251,16 +1253,19 @@ __global__ void __launch_bounds__(256) nf4_dequant_codes_kernel(const uint8_t* _
   __syncthreads();
   const size_t stride = (size_t)gridDim.x * blockDim.x * 16;
   for (size_t i0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 16; i0 < n; i0 += stride) {
-    uint8_t c[16];
-    if (i0 + 16 <= n && (reinterpret_cast<uintptr_t>(codes + i0) & 15) == 0) {
-      *reinterpret_cast<uint4*>(c) = *reinterpret_cast<const uint4*>(codes + i0);
+    if (WHOLE && i0 + 16 <= n) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(codes + i0);
+      const float scale = absmax[i0 <= 0xffffffffull ? (size_t)((unsigned)i0 / (unsigned)block) : i0 / block];
+      const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
+      float o[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) o[j] = cb[(w[j >> 2] >> (8 * (j & 3))) & 15] * scale;
+#pragma unroll
+      for (int j = 0; j < 16; j += Vec<T>::N) store_vec<T>(out + i0 + j, o + j);
     } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) c[j] = i0 + j < n ? codes[i0 + j] : 0;
+      for (int j = 0; j < 16; ++j)
+        if (i0 + j < n) out[i0 + j] = from_f<T>(cb[codes[i0 + j] & 15] * absmax[(i0 + j) / block]);
     }
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (i0 + j < n) out[i0 + j] = from_f<T>(cb[c[j] & 15] * absmax[(i0 + j) / block]);
   }
 }
 
@@ -2079,8 +2084,11 @@ int nb_nf4_dequant_codes(const unsigned char* codes, const float* absmax, const 
                          int block, int dtype, void* stream) {
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)(n + 15) / 16, 256);
-  if (dtype) nf4_dequant_codes_kernel<bf16><<<grid, 256, 0, STREAM>>>(codes, absmax, codebook, (bf16*)out, (size_t)n, block);
-  else nf4_dequant_codes_kernel<float><<<grid, 256, 0, STREAM>>>(codes, absmax, codebook, (float*)out, (size_t)n, block);
+  const bool whole = block % 16 == 0 && ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+#define NF4(T, W) nf4_dequant_codes_kernel<T, W><<<grid, 256, 0, STREAM>>>(codes, absmax, codebook, (T*)out, (size_t)n, block)
+  if (dtype) { if (whole) NF4(bf16, true); else NF4(bf16, false); }
+  else { if (whole) NF4(float, true); else NF4(float, false); }
+#undef NF4
   return CHECK_LAUNCH();
 }
 

@@ -284,3 +284,17 @@ def test_captured_function_with_odd_inputs():
         if first is not None:
             assert torch.equal(first[0], first[1])
         first = (out[1], x)
+
+
+# ---------------------------------------------------------------- NF4
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,block,offset", [(1, 64, 0), (16, 16, 0), (1000, 64, 0), (4096, 128, 0), (4113, 10, 0), (4096, 64, 3), (70000, 48, 0)])
+def test_nf4_codes(dtype, n, block, offset):
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(6)
+    codes = torch.randint(0, 16, (n + offset,), device="cuda", dtype=torch.uint8)[offset:]
+    scales = torch.rand((n + block - 1) // block, device="cuda") + 0.01
+    book = torch.linspace(-1, 1, 16, device="cuda")
+    got = kernels.nf4_dequant_codes(codes, scales, book, n, block, dtype)
+    assert torch.equal(got, (book[codes.long()] * scales.repeat_interleave(block)[:n]).to(dtype))
