@@ -654,6 +654,14 @@ __global__ void __launch_bounds__(256) softmax_kernel(const T* __restrict__ x, T
 // Per row: lse = logsumexp(logits_row); picked = logits_row[target] when 0 <= target < D else 0.
 // A vocabulary shard passes targets shifted by its offset, so out-of-range simply means
 // "another shard holds this class"; the caller combines shards with max/sum reductions.
+//
+// Rows of any width and alignment move in 16-byte vectors: the elements before a row's first 16-byte
+// boundary and behind its last are taken one by one (a vocabulary that is not a multiple of 8 gives every
+// row another offset; all-scalar rows cost several times the vector loop's time).
+template <typename T>
+__device__ __forceinline__ int row_head(const T* row, int D) {       // elements before the first 16-byte boundary
+  return min(D, (int)(((16u - (unsigned)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) / sizeof(T)));
+}
 template <typename T>
 __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__ logits,
                                                           const long long* __restrict__ tgt, float* __restrict__ lse_out,
@@ -664,26 +672,26 @@ __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__
   const T* xr = logits + (size_t)row * D;
   float m = -INFINITY, s = 0.f;
   constexpr int V = Vec<T>::N;
-  if ((D % V) == 0) {
-    for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
-      float v[V];
-      load_vec<T>(xr + c, v);
-      float lm = v[0];
+  const int head = row_head(xr, D), body = (D - head) / V * V, tail = head + body;
+  const int edge = threadIdx.x < head ? (int)threadIdx.x : tail + (int)threadIdx.x - head;     // one edge element per thread
+  if (edge < D) {
+    m = to_f<T>(xr[edge]);
+    s = m == -INFINITY ? 0.f : 1.f;                            // exp(m - m); NaN stays in s
+    if (m != m) s = m;
+  }
+  for (int c = head + threadIdx.x * V; c < tail; c += blockDim.x * V) {
+    float v[V];
+    load_vec<T>(xr + c, v);
+    float lm = v[0];
 #pragma unroll
-      for (int j = 1; j < V; ++j) lm = fmaxf(lm, v[j]);
-      if (lm > m) { s = s * __expf(m - lm); m = lm; }
+    for (int j = 1; j < V; ++j) lm = fmaxf(lm, v[j]);
+    if (lm > m) { s = s * __expf(m - lm); m = lm; }
+    const float ms = m == -INFINITY ? 0.f : m;                 // only -inf so far: each adds exp(-inf) = 0
 #pragma unroll
-      for (int j = 0; j < V; ++j) s += __expf(v[j] - m);
-    }
-  } else {
-    for (int c = threadIdx.x; c < D; c += blockDim.x) {
-      const float v = to_f<T>(xr[c]);
-      if (v > m) { s = s * __expf(m - v); m = v; }
-      s += __expf(v - m);
-    }
+    for (int j = 0; j < V; ++j) s += __expf(v[j] - ms);
   }
   const float gm = block_max<8>(m, sh);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
+  s = (m == -INFINITY) ? s : s * __expf(m - gm);               // 0 (or NaN) where the thread saw only -inf
   const float gs = block_sum<8>(s, sh);
   if (threadIdx.x == 0) {
     const long long t = tgt[row];
@@ -707,17 +715,20 @@ __global__ void __launch_bounds__(256) lse_pick_bwd_kernel(const T* __restrict__
   const float gl = g_lse ? g_lse[row] : 0.f;
   const float gp = g_pick ? g_pick[row] : 0.f;
   constexpr int V = Vec<T>::N;
-  if ((D % V) == 0) {
-    for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
-      float v[V], o[V];
-      load_vec<T>(xr + c, v);
+  // both rows have the same offset from a 16-byte boundary unless a caller's base pointers differ in it
+  const int head = row_head(xr, D) == row_head(dr, D) ? row_head(xr, D) : D;
+  const int body = (D - head) / V * V, tail = head + body;
+  auto grad = [&](float v, int c) { return __expf(v - l) * gl + (c == t ? gp : 0.f); };
+  for (int e = threadIdx.x; e < D - body; e += blockDim.x) {
+    const int c = e < head ? e : body + e;
+    dr[c] = from_f<T>(grad(to_f<T>(xr[c]), c));
+  }
+  for (int c = head + threadIdx.x * V; c < tail; c += blockDim.x * V) {
+    float v[V], o[V];
+    load_vec<T>(xr + c, v);
 #pragma unroll
-      for (int j = 0; j < V; ++j) o[j] = __expf(v[j] - l) * gl + ((c + j) == t ? gp : 0.f);
-      store_vec<T>(dr + c, o);
-    }
-  } else {
-    for (int c = threadIdx.x; c < D; c += blockDim.x)
-      dr[c] = from_f<T>(__expf(to_f<T>(xr[c]) - l) * gl + (c == t ? gp : 0.f));
+    for (int j = 0; j < V; ++j) o[j] = grad(v[j], c + j);
+    store_vec<T>(dr + c, o);
   }
 }
 

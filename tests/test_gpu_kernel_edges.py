@@ -298,3 +298,26 @@ def test_nf4_codes(dtype, n, block, offset):
     book = torch.linspace(-1, 1, 16, device="cuda")
     got = kernels.nf4_dequant_codes(codes, scales, book, n, block, dtype)
     assert torch.equal(got, (book[codes.long()] * scales.repeat_interleave(block)[:n]).to(dtype))
+
+
+# ---------------------------------------------------------------- cross-entropy rows
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,D", [(3, 1), (5, 7), (4, 8), (9, 33), (6, 1000), (7, 2051), (3, 10001), (2, 32000)])
+def test_logsumexp_and_gradient_at_any_row_alignment(dtype, rows, D):
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(7)
+    x = (torch.randn(rows, D, device="cuda") * 3).to(dtype)
+    x[0, D // 3: D // 3 + 20] = float("-inf")          # masked classes, here and there a whole vector of them
+    if D > 1:
+        x[0, D - 1] = 1.0
+    t = torch.randint(-1, D + 1, (rows,), device="cuda")
+    lse, picked = kernels.lse_pick_fwd(x, t)
+    torch.testing.assert_close(lse.double(), torch.logsumexp(x.double(), -1), rtol=1e-5, atol=1e-5)
+    ok = (t >= 0) & (t < D)
+    assert torch.equal(picked, torch.where(ok, x.float().gather(1, t.clamp(0, D - 1)[:, None])[:, 0], torch.zeros((), device="cuda")))
+    gl, gp = torch.rand(rows, device="cuda"), torch.randn(rows, device="cuda")
+    safe = torch.where(lse == float("-inf"), torch.zeros_like(lse), lse)
+    ref = torch.exp(x.double() - safe.double()[:, None]) * gl.double()[:, None]
+    ref[ok] = ref[ok].scatter_add(1, t[ok][:, None], gp.double()[ok][:, None])
+    assert _rel2(kernels.lse_pick_bwd(x, t, safe, gl, gp), ref) < STORED[dtype]
