@@ -441,7 +441,11 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
     // two epilogue groups share every tile: group g takes the 64-column pairs with (pair & 1) == g,
     // so the per-element math of the gelu / d-gelu epilogues fits under the tile's MMAs
     const int grp = (warp - 4) >> 2;
-    const bool heavy = args.epi == EPI_BIAS_GELU || args.aux == AUX_MUL_DGELU;
+    // bf16 rows that are not 16-byte aligned (N or ldc not a multiple of 8: an odd vocabulary) leave through
+    // shared memory as runs of 64 columns of one row. A lane storing its own row would touch 32 rows, 32
+    // sectors, per 2-byte store.
+    const bool staged = MODE == MODE_NONE && !args.vec_ok && !args.out_fp32 && !args.accumulate;
+    const bool heavy = (args.epi == EPI_BIAS_GELU || args.aux == AUX_MUL_DGELU) && !staged;
     bool ok = true;
     int it = 0;
     for (int t = cta; t < num_tiles; t += nctas, ++it) {
@@ -629,6 +633,37 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
                 const uint4 v = *reinterpret_cast<const uint4*>(mine + r * L::OUT_ROW_BYTES + piece * 16);
                 *reinterpret_cast<uint4*>(base + (long long)r * args.N + col) = v;
               }
+            }
+            __syncwarp();
+          }
+        } else if (staged) {
+          uint8_t* mine = out_stage + wq * (32 * L::OUT_ROW_BYTES);
+          uint8_t* rowp = mine + lane * L::OUT_ROW_BYTES + (c & 1) * 64;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint4 pk;
+            uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              __nv_bfloat162 h = __floats2bfloat162_rn(f[q * 8 + 2 * j], f[q * 8 + 2 * j + 1]);
+              pw[j] = *reinterpret_cast<uint32_t*>(&h);
+            }
+            *reinterpret_cast<uint4*>(rowp + q * 16) = pk;
+          }
+          if ((c & 1) || c == BN / 32 - 1 || nb0 + 32 >= args.N) {
+            __syncwarp();
+            const int col0 = n0 + (c & ~1) * 32, cols = min(args.N - col0, (c & 1) ? 64 : 32), r0 = m0 + wq * 32;
+            __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(out_ptr) + (out_off - (long long)lane * args.ldc) + col0;
+            const int nr = min(32, args.M - r0);
+#pragma unroll 4
+            for (int r = 0; r < nr; ++r) {
+              if (!NB_IN_BOUNDS(NB_SITE_GEMM_STORE, out_off + (r - lane) * args.ldc,
+                                static_cast<long long>(args.batch - 1) * args.stride_c +
+                                    static_cast<long long>(args.M - 1) * args.ldc + 1))
+                break;
+              const __nv_bfloat16* sr = reinterpret_cast<const __nv_bfloat16*>(mine + r * L::OUT_ROW_BYTES);
+              if (lane < cols) base[r * args.ldc + lane] = sr[lane];
+              if (lane + 32 < cols) base[r * args.ldc + lane + 32] = sr[lane + 32];
             }
             __syncwarp();
           }

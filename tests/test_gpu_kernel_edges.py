@@ -321,3 +321,25 @@ def test_logsumexp_and_gradient_at_any_row_alignment(dtype, rows, D):
     ref = torch.exp(x.double() - safe.double()[:, None]) * gl.double()[:, None]
     ref[ok] = ref[ok].scatter_add(1, t[ok][:, None], gp.double()[ok][:, None])
     assert _rel2(kernels.lse_pick_bwd(x, t, safe, gl, gp), ref) < STORED[dtype]
+
+
+# ---------------------------------------------------------------- GEMM rows that are not 16-byte aligned
+@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (130, 33, 72), (257, 77, 200), (100, 255, 64), (300, 513, 128), (4097, 1001, 264), (5000, 4999, 64)])
+def test_gemm_with_odd_output_rows(M, N, K):
+    from nabla_b200.native import gemm
+
+    torch.manual_seed(8)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(K, N, device="cuda", dtype=torch.bfloat16) * 0.1
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    z = a.double() @ b.double() + bias.double()
+    assert _rel2(gemm.gemm_bf16(a, b), a.double() @ b.double()) < STORED[torch.bfloat16]
+    assert _rel2(gemm.gemm_bf16(a, b, bias=bias, epilogue="relu"), z.relu()) < STORED[torch.bfloat16]
+    y, pre = gemm.gemm_bf16(a, b, bias=bias, epilogue="gelu", aux="store_preact")
+    assert _rel2(pre, z) < STORED[torch.bfloat16] and _rel2(y, TF.gelu(z)) < STORED[torch.bfloat16]
+    three = gemm.gemm_bf16(torch.stack([a, a * 2]), torch.stack([b, b]))
+    assert _rel2(three[1], 2 * (a.double() @ b.double())) < STORED[torch.bfloat16]
+    guard = torch.full((M, N + 3), 7.0, device="cuda", dtype=torch.bfloat16)      # rows with another stride: nothing beside them
+    gemm.gemm_bf16(a, b, out=guard[:, 1:1 + N])
+    assert _rel2(guard[:, 1:1 + N], a.double() @ b.double()) < STORED[torch.bfloat16]
+    assert bool((guard[:, 0] == 7).all()) and bool((guard[:, 1 + N:] == 7).all())
