@@ -89,6 +89,12 @@ def _prep(t: torch.Tensor):
     def ok(ld, sbatch):
         return ld % 8 == 0 and (b == 1 or sbatch % 8 == 0) and t.data_ptr() % 16 == 0 and ld > 0
 
+    # a single row or column has no second stride that could be misaligned: any multiple of 8 will do, and
+    # the vector is read in place (it took a zero fill and a copy into a padded buffer)
+    if r == 1 and sc == 1 and ok(8, sb):
+        return t, "row", (c + 7) // 8 * 8, sb
+    if c == 1 and sr == 1 and ok(8, sb):
+        return t, "col", (r + 7) // 8 * 8, sb
     if sc == 1 and ok(sr, sb) and sr >= c:
         return t, "row", sr, sb
     if sr == 1 and ok(sc, sb) and sc >= r:

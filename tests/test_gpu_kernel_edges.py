@@ -343,3 +343,16 @@ def test_gemm_with_odd_output_rows(M, N, K):
     gemm.gemm_bf16(a, b, out=guard[:, 1:1 + N])
     assert _rel2(guard[:, 1:1 + N], a.double() @ b.double()) < STORED[torch.bfloat16]
     assert bool((guard[:, 0] == 7).all()) and bool((guard[:, 1 + N:] == 7).all())
+
+
+# ---------------------------------------------------------------- GEMM operands of one row or column
+def test_gemm_operands_of_one_row_or_column():
+    from nabla_b200.native import gemm
+
+    torch.manual_seed(11)
+    for M, N, K in ((512, 1, 256), (1, 300, 77), (1, 1, 9), (300, 40, 1), (256, 1, 513), (1, 2056, 4096)):
+        for ta in (False, True):
+            for tb in (False, True):
+                a = torch.randn(K, M, device="cuda", dtype=torch.bfloat16).t() if ta else torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+                b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16).t() if tb else torch.randn(K, N, device="cuda", dtype=torch.bfloat16)
+                assert _rel2(gemm.gemm_bf16(a, b), a.double() @ b.double()) < STORED[torch.bfloat16]
