@@ -807,6 +807,16 @@ __global__ void __launch_bounds__(256) adamw_kernel(const TP* __restrict__ p, co
     }
   }
 }
+// hyper = {lr, 1 - b1^t, 1 - b2^t, 1} for a step count t that lives on the device (in 64 bits: 1 - b2^t of the
+// first steps cancels). One thread; the same four numbers took ten launches of elementwise kernels, as much
+// as the updates of a small model.
+__global__ void adam_hyper_kernel(const float* __restrict__ step, float* __restrict__ hyper, float lr, double b1, double b2) {
+  const double t = (double)step[0];
+  hyper[0] = lr;
+  hyper[1] = (float)(1.0 - pow(b1, t));
+  hyper[2] = (float)(1.0 - pow(b2, t));
+  hyper[3] = 1.f;
+}
 template <typename TP, typename TG>
 __global__ void __launch_bounds__(256) sgd_kernel(const TP* __restrict__ p, const TG* __restrict__ g,
                                                  const float* __restrict__ buf, TP* __restrict__ p_out,
@@ -1896,6 +1906,10 @@ int nb_adamw(const void* p, const void* g, const float* m, const float* v, void*
   else if (p_dtype) ADAMW(bf16, float);
   else if (g_dtype) ADAMW(float, bf16);
   else ADAMW(float, float);
+  return CHECK_LAUNCH();
+}
+int nb_adam_hyper(const float* step, float* hyper, float lr, double b1, double b2, void* stream) {
+  adam_hyper_kernel<<<1, 1, 0, STREAM>>>(step, hyper, lr, b1, b2);
   return CHECK_LAUNCH();
 }
 int nb_sgd(const void* p, const void* g, const float* buf, void* p_out, float* buf_out, long long n, float lr,

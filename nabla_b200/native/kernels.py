@@ -31,6 +31,7 @@ def _L():
             "nb_lse_pick_fwd": [c_vp] * 4 + [c_int, c_int, c_int, c_vp],
             "nb_lse_pick_bwd": [c_vp] * 6 + [c_int, c_int, c_int, c_vp],
             "nb_adamw": [c_vp] * 7 + [c_ll] + [c_f] * 8 + [c_vp, c_int, c_int, c_vp],
+            "nb_adam_hyper": [c_vp, c_vp, c_f, ctypes.c_double, ctypes.c_double, c_vp],
             "nb_sgd": [c_vp] * 5 + [c_ll] + [c_f] * 4 + [c_int, c_int, c_vp],
             "nb_embedding_gather": [c_vp] * 3 + [c_int] * 4 + [c_vp],
             "nb_embedding_scatter_add": [c_vp] * 5 + [c_int] * 4 + [c_vp],
@@ -197,6 +198,13 @@ def adamw(p, g, m, v, *, lr, b1, b2, eps, wd, step: int | None = None, hyper: to
                       float(b2), float(eps), float(wd), float(bc1), float(bc2), float(grad_scale), ptr(hyper), _dt(p),
                       _dt(g), stream_ptr()), "adamw")
     return po, mo, vo
+
+
+def adam_hyper(step: torch.Tensor, lr: float, b1: float, b2: float) -> torch.Tensor:
+    """[lr, 1 - b1^t, 1 - b2^t, 1] for the fp32 step count ``t`` on the device (one element)."""
+    out = torch.empty(4, dtype=torch.float32, device=step.device)
+    _ok(_L().nb_adam_hyper(ptr(step), ptr(out), float(lr), float(b1), float(b2), stream_ptr()), "adam_hyper")
+    return out
 
 
 def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):

@@ -854,6 +854,10 @@ class AdamHyperOp(Operation):
 
     def kernel(self, step, *, lr: float, beta1: float, beta2: float):
         s = step.reshape(()).float()
+        if _native(s):
+            from ..native import kernels
+
+            return kernels.adam_hyper(s, lr, beta1, beta2)
         one = torch.ones((), device=step.device)
         return torch.stack([one * lr, 1 - beta1 ** s, 1 - beta2 ** s, one]).float()
 

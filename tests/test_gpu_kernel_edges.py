@@ -356,3 +356,13 @@ def test_gemm_operands_of_one_row_or_column():
                 a = torch.randn(K, M, device="cuda", dtype=torch.bfloat16).t() if ta else torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
                 b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16).t() if tb else torch.randn(K, N, device="cuda", dtype=torch.bfloat16)
                 assert _rel2(gemm.gemm_bf16(a, b), a.double() @ b.double()) < STORED[torch.bfloat16]
+
+
+# ---------------------------------------------------------------- AdamW bias corrections
+def test_adam_hyper():
+    from nabla_b200.native import kernels
+
+    for t in (1.0, 2.0, 101.0, 12345.0):
+        got = kernels.adam_hyper(torch.tensor(t, device="cuda"), 1e-3, 0.9, 0.999).double().tolist()
+        for a, b in zip(got, (1e-3, 1 - 0.9 ** t, 1 - 0.999 ** t, 1.0)):
+            assert abs(a - b) <= 1e-7 * abs(b)
