@@ -566,6 +566,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
 #pragma unroll
   for (int j = 0; j < V; ++j) acc[j] = 0.f;
   if (c < N) {
+#pragma unroll 4
     for (int r = r0 + warp; r < r1; r += 8) {
       float v[V];
       load_vec<T>(x + (size_t)r * N + c, v);
@@ -584,15 +585,6 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
     if (col < N) partial[(size_t)blockIdx.y * N + col] = s;
   }
 }
-template <typename T>
-__global__ void colsum_final_kernel(const float* __restrict__ partial, T* __restrict__ out, int nparts, int N) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
-  float s = 0.f;
-  for (int i = 0; i < nparts; ++i) s += partial[(size_t)i * N + c];
-  out[c] = from_f<T>(s);
-}
-
 // Column sums of a tall, narrow matrix (the bias gradient of a convolution: 200704 x 16): the block's 256
 // threads cover 256 / (N / V) whole rows at a time, so every lane loads whatever N is; colsum_kernel gives a
 // warp one row's 32 vectors and leaves 28 of 32 lanes without one there. 200704 x 16 fp32: 81 -> 17 us.
@@ -1840,9 +1832,20 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
 
 // Narrow: fewer vectors per row than a warp has lanes, and rows enough for many blocks (256 rows each at least).
 static bool colsum_narrow(int rows, int N, int V) { return N / V < 32 && rows >= 4096; }
+// Row slabs. Otherwise 512 rows each and at most 64 slabs, but no fewer than give every SM two blocks while a
+// warp still has eight rows: at 2002 x 512 four slabs of two column tiles were 8 blocks, each warp of which
+// read 64 rows one after the other.
 int nb_colsum_nparts(int rows, int N, int in_dtype) {
+  const int V = in_dtype ? 8 : 4, tiles = (N + 32 * V - 1) / (32 * V);
   int np = (rows + 511) / 512, most = 64;
-  if (colsum_narrow(rows, N, in_dtype ? 8 : 4)) { np = (rows + 255) / 256; most = 148 * 4; }
+  if (colsum_narrow(rows, N, V)) {
+    np = (rows + 255) / 256;
+    most = 148 * 4;
+  } else {
+    int fill = (2 * 148 + tiles - 1) / tiles;
+    if (fill > (rows + 63) / 64) fill = (rows + 63) / 64;
+    if (np < fill) np = fill;
+  }
   if (np > most) np = most;
   return np < 1 ? 1 : np;
 }
@@ -1855,15 +1858,13 @@ int nb_colsum(const void* x, void* out, float* partial, int rows, int N, int in_
   if (colsum_narrow(rows, N, V)) {
     if (in_dtype) colsum_narrow_kernel<bf16><<<np, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
     else colsum_narrow_kernel<float><<<np, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
-    if (out_dtype) fold_slices_kernel<bf16><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (bf16*)out, (size_t)N, np);
-    else fold_slices_kernel<float><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (float*)out, (size_t)N, np);
-    return CHECK_LAUNCH();
+  } else {
+    const dim3 grid((N + 32 * V - 1) / (32 * V), np);
+    if (in_dtype) colsum_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
+    else colsum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
   }
-  dim3 grid((N + 32 * V - 1) / (32 * V), np);
-  if (in_dtype) colsum_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
-  else colsum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
-  if (out_dtype) colsum_final_kernel<bf16><<<(N + 255) / 256, 256, 0, STREAM>>>(partial, (bf16*)out, np, N);
-  else colsum_final_kernel<float><<<(N + 255) / 256, 256, 0, STREAM>>>(partial, (float*)out, np, N);
+  if (out_dtype) fold_slices_kernel<bf16><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (bf16*)out, (size_t)N, np);
+  else fold_slices_kernel<float><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (float*)out, (size_t)N, np);
   return CHECK_LAUNCH();
 }
 

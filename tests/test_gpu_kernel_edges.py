@@ -366,3 +366,14 @@ def test_adam_hyper():
         got = kernels.adam_hyper(torch.tensor(t, device="cuda"), 1e-3, 0.9, 0.999).double().tolist()
         for a, b in zip(got, (1e-3, 1 - 0.9 ** t, 1 - 0.999 ** t, 1.0)):
             assert abs(a - b) <= 1e-7 * abs(b)
+
+
+# ---------------------------------------------------------------- column sums
+def test_column_sums_around_the_slab_counts():
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(10)
+    for rows, N in ((1, 8), (63, 512), (64, 512), (65, 256), (512, 256), (2002, 1536), (16384, 264), (5000, 8192)):
+        for dtype in (torch.bfloat16, torch.float32):
+            x = torch.randn(rows, N, device="cuda").to(dtype)
+            assert _rel2(kernels.colsum(x), x.double().sum(0)) < STORED[dtype]
