@@ -1306,6 +1306,83 @@ __global__ void __launch_bounds__(256) pool2d_fwd_kernel(const T* __restrict__ x
     y[i] = from_f<T>(mode == 0 ? acc / (kh * kw) : acc);
   }
 }
+// Pooling whose windows do not overlap and lie in the image (kernel <= stride, no padding: the usual 2 x 2), C a
+// multiple of the 16-byte vector: one thread per vector of channels of a stride x stride cell. Forward: the
+// window's elements are read once. Backward: so are x and dy, and the cell's dx is written whole, zeros where
+// no window reaches (the gather form below finds every window's arg-max again for each of its pixels, with
+// six 64-bit divisions per element). Same values, first arg-max included. 2 x 2 over 256 x 28 x 28 x 16 fp32:
+// forward 10 -> 3.6 us, backward 52 -> 5.4 us.
+struct CellGeom {
+  int H, W, CV, OH, OW, kh, kw, sh, sw, cells_h, cells_w;
+};
+template <typename T, bool MAX>
+__global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, const CellGeom g, unsigned total) {
+  constexpr int V = Vec<T>::N;
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= total) return;
+  const unsigned c = i % g.CV, p = i / g.CV, ow = p % g.OW, q = p / g.OW, oh = q % g.OH, n = q / g.OH;
+  const T* xp = x + (((size_t)n * g.H + oh * g.sh) * g.W + ow * g.sw) * g.CV * V + c * V;
+  float acc[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = MAX ? -INFINITY : 0.f;
+  for (int a = 0; a < g.kh; ++a)
+    for (int b = 0; b < g.kw; ++b) {
+      float v[V];
+      load_vec<T>(xp + ((size_t)a * g.W + b) * g.CV * V, v);
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[j] = MAX ? fmaxf(acc[j], v[j]) : acc[j] + v[j];
+    }
+  if (!MAX) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] /= g.kh * g.kw;
+  }
+  store_vec<T>(y + (size_t)i * V, acc);
+}
+template <typename T, bool MAX>
+__global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dx,
+                                                             const CellGeom g, unsigned total) {
+  constexpr int V = Vec<T>::N;
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= total) return;
+  const unsigned c = i % g.CV, p = i / g.CV, cw = p % g.cells_w, q = p / g.cells_w, ch = q % g.cells_h, n = q / g.cells_h;
+  const size_t at = (((size_t)n * g.H + ch * g.sh) * g.W + cw * g.sw) * g.CV * V + c * V, down = (size_t)g.W * g.CV * V;
+  const bool window = (int)ch < g.OH && (int)cw < g.OW;
+  float d[V], best[V];
+  int where[V];                                      // position of the first maximum in the window, -1: none
+#pragma unroll
+  for (int j = 0; j < V; ++j) { d[j] = 0.f; best[j] = -INFINITY; where[j] = -1; }
+  if (window) {
+    load_vec<T>(dy + (((size_t)n * g.OH + ch) * g.OW + cw) * g.CV * V + c * V, d);
+    if (MAX) {
+      for (int a = 0; a < g.kh; ++a)
+        for (int b = 0; b < g.kw; ++b) {
+          float v[V];
+          load_vec<T>(x + at + a * down + (size_t)b * g.CV * V, v);
+#pragma unroll
+          for (int j = 0; j < V; ++j)
+            if (v[j] > best[j]) { best[j] = v[j]; where[j] = a * g.kw + b; }
+        }
+    }
+  }
+  const float inv = 1.f / (g.kh * g.kw);
+  const int hh = min(g.sh, g.H - (int)ch * g.sh), ww = min(g.sw, g.W - (int)cw * g.sw);
+  for (int a = 0; a < hh; ++a)
+    for (int b = 0; b < ww; ++b) {
+      const bool in = window && a < g.kh && b < g.kw;
+      float o[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j) o[j] = !in ? 0.f : MAX ? (where[j] == a * g.kw + b ? d[j] : 0.f) : d[j] * inv;
+      store_vec<T>(dx + at + a * down + (size_t)b * g.CV * V, o);
+    }
+}
+// Whether the two kernels above take a problem.
+static inline bool pool_cells(const void* x, const void* y, const void* z, int N, int H, int W, int C, int OH, int OW, int kh, int kw,
+                              int sh, int sw, int ph, int pw, int V, CellGeom& g) {
+  g = CellGeom{H, W, C / V, OH, OW, kh, kw, sh, sw, (H + sh - 1) / sh, (W + sw - 1) / sw};
+  return ph == 0 && pw == 0 && kh <= sh && kw <= sw && C % V == 0 && (long long)N * g.cells_h * g.cells_w * g.CV < 0x7fffff00ll &&
+         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z)) & 15) == 0;
+}
+
 // out[window] = t[first arg-max of x over the window] (0 for a window that lies in the padding): the
 // forward-mode derivative of max pooling, and the transpose of its backward routing.
 template <typename T>
@@ -2122,16 +2199,35 @@ int nb_pool2d_fwd(const void* x, void* y, int N, int H, int W, int C, int OH, in
                   int ph, int pw, int mode, int dtype, void* stream) {
   const size_t total = (size_t)N * OH * OW * C;
   if (!total) return 0;
+  const int V = dtype ? 8 : 4;
+  CellGeom g;
+  if (pool_cells(x, y, nullptr, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g)) {
+    const unsigned n = (unsigned)(total / V);
+#define POOL(T, MAX) pool2d_cell_fwd_kernel<T, MAX><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (T*)y, g, n)
+    if (dtype) { if (mode) POOL(bf16, true); else POOL(bf16, false); }
+    else { if (mode) POOL(float, true); else POOL(float, false); }
+#undef POOL
+    return CHECK_LAUNCH();
+  }
   const int grid = grid_for(total, 256);
   if (dtype) pool2d_fwd_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (bf16*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
   else pool2d_fwd_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
   return CHECK_LAUNCH();
 }
-// dx must be a zeroed fp32 buffer of the input's shape.
 int nb_pool2d_bwd(const void* x, const void* dy, void* dx, int N, int H, int W, int C, int OH, int OW, int kh, int kw,
                   int sh, int sw, int ph, int pw, int mode, int dtype, void* stream) {
   const size_t total = (size_t)N * H * W * C;
   if (!total) return 0;
+  const int V = dtype ? 8 : 4;
+  CellGeom g;
+  if (pool_cells(x, dy, dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g)) {
+    const unsigned n = (unsigned)((size_t)N * g.cells_h * g.cells_w * g.CV);
+#define POOL(T, MAX) pool2d_cell_bwd_kernel<T, MAX><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (const T*)dy, (T*)dx, g, n)
+    if (dtype) { if (mode) POOL(bf16, true); else POOL(bf16, false); }
+    else { if (mode) POOL(float, true); else POOL(float, false); }
+#undef POOL
+    return CHECK_LAUNCH();
+  }
   const int grid = grid_for(total, 256);
   if (dtype) pool2d_bwd_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (const bf16*)dy, (bf16*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
   else pool2d_bwd_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (const float*)dy, (float*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);

@@ -377,3 +377,29 @@ def test_column_sums_around_the_slab_counts():
         for dtype in (torch.bfloat16, torch.float32):
             x = torch.randn(rows, N, device="cuda").to(dtype)
             assert _rel2(kernels.colsum(x), x.double().sum(0)) < STORED[dtype]
+
+
+# ---------------------------------------------------------------- pooling
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("mode", ["max", "avg"])
+@pytest.mark.parametrize("N,H,W,C,k,s,p", [(2, 8, 8, 16, (2, 2), (2, 2), 0), (1, 7, 9, 8, (2, 2), (2, 2), 0), (3, 5, 11, 24, (1, 2), (2, 3), 0), (2, 9, 9, 8, (3, 3), (3, 3), 0),
+                                           (1, 2, 2, 8, (2, 2), (5, 4), 0), (2, 6, 6, 12, (2, 2), (2, 2), 0), (2, 6, 6, 5, (2, 2), (2, 2), 0),
+                                           (2, 8, 8, 8, (3, 3), (2, 2), 0), (2, 8, 8, 8, (2, 2), (2, 2), 1)])
+def test_pooling_cells(dtype, mode, N, H, W, C, k, s, p):
+    """Windows that do not overlap (whole images and ragged edges, strides wider than the window) and the sizes
+    beside the rule; ties go to the first maximum, a window of -inf routes nothing."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(9)
+    x = torch.randint(-3, 4, (N, H, W, C), device="cuda").to(dtype)
+    x[0, :k[0], :k[1], 0] = float("-inf") if mode == "max" and p == 0 else 0.0
+    y = kernels.pool2d_fwd(x, *k, *s, p, p, mode)
+    xr = x.double().permute(0, 3, 1, 2).requires_grad_(True)
+    xp = TF.pad(xr, (p, p, p, p), value=float("-inf") if mode == "max" else 0.0)
+    ref = TF.max_pool2d(xp, k, s) if mode == "max" else TF.avg_pool2d(xp, k, s)
+    torch.testing.assert_close(y.double(), ref.permute(0, 2, 3, 1), rtol=2.0 ** -8, atol=0)
+    dy = torch.randn(y.shape, device="cuda").to(dtype)
+    if mode == "max" and p == 0:
+        dy[0, 0, 0, 0] = 0.0                           # torch routes a window of -inf to its first element
+    (g,) = torch.autograd.grad(ref, xr, dy.double().permute(0, 3, 1, 2))
+    torch.testing.assert_close(kernels.pool2d_bwd(x, dy, *k, *s, p, p, mode).double(), g.permute(0, 2, 3, 1), rtol=2.0 ** -7, atol=1e-6)
