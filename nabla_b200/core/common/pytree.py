@@ -9,6 +9,7 @@ from __future__ import annotations
 from typing import Any, Callable
 
 _registry: dict[type, tuple[Callable, Callable]] = {}
+_leaf_types: set[type] = set()      # types already found to be leaves (emptied by every registration)
 
 
 def register_pytree_node(cls: type, flatten_fn: Callable, unflatten_fn: Callable) -> None:
@@ -17,6 +18,7 @@ def register_pytree_node(cls: type, flatten_fn: Callable, unflatten_fn: Callable
     if not isinstance(cls, type):
         raise TypeError("cls must be a type")
     _registry[cls] = (flatten_fn, unflatten_fn)
+    _leaf_types.clear()
 
 
 def _freeze(v: Any) -> Any:
@@ -92,6 +94,9 @@ def _flatten(tree: Any, leaves: list, is_leaf) -> PyTreeDef:
     if tree is None:
         return _NONE
     t = type(tree)
+    if t in _leaf_types:
+        leaves.append(tree)
+        return _LEAF
     if t is list or t is tuple:
         ch = tuple(_flatten(x, leaves, is_leaf) for x in tree)
         return PyTreeDef("list" if t is list else "tuple", None, ch, sum(c.num_leaves for c in ch))
@@ -112,6 +117,8 @@ def _flatten(tree: Any, leaves: list, is_leaf) -> PyTreeDef:
     if isinstance(tree, tuple) and hasattr(tree, "_fields"):  # namedtuple
         ch = tuple(_flatten(x, leaves, is_leaf) for x in tree)
         return PyTreeDef("custom", (t, "namedtuple"), ch, sum(c.num_leaves for c in ch))
+    if not isinstance(tree, tuple):
+        _leaf_types.add(t)
     leaves.append(tree)
     return _LEAF
 

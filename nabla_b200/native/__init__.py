@@ -159,7 +159,15 @@ def use_native(t: torch.Tensor) -> bool:
     return t.is_cuda and os.environ.get("NABLA_B200_DISABLE_NATIVE", "0") != "1"
 
 
+try:                               # the raw handle, without a Stream object per launch
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+except AttributeError:             # a torch build without CUDA
+    _raw_stream = None
+
+
 def stream_ptr() -> ctypes.c_void_p:
+    if _raw_stream is not None:
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 

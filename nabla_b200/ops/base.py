@@ -319,11 +319,10 @@ class Operation:
     def execute(self, node: OpNode) -> list[list[torch.Tensor]]:
         """Run the kernel once per local shard. Returns per-output lists of shard buffers."""
         leaves = node.arg_leaves
-        impls = [a for a in leaves if isinstance(a, TensorImpl)]
         n_shards = 1
         mesh = None
-        for im in impls:
-            if im.sharding is not None:
+        for im in leaves:
+            if isinstance(im, TensorImpl) and im.sharding is not None:
                 mesh = im.sharding.mesh
                 n_shards = mesh.num_local
                 break
@@ -346,10 +345,14 @@ class Operation:
                     shard_leaves.append(bufs[s] if len(bufs) > 1 else bufs[0])
                 else:
                     shard_leaves.append(a)
-            args = pytree.tree_unflatten(node.arg_treedef, shard_leaves)
+            td = node.arg_treedef
+            if td.kind == "tuple" and all(c.kind == "leaf" for c in td.children):      # no nested arguments
+                args = shard_leaves
+            else:
+                args = pytree.tree_unflatten(td, shard_leaves)
             kw = self.shard_kwargs(node.kwargs, node, s, local_ids[s]) if mesh is not None else node.kwargs
             out = self.kernel(*args, **kw)
-            flat = pytree.tree_leaves(out)
+            flat = [out] if isinstance(out, torch.Tensor) else pytree.tree_leaves(out)
             if per_output is None:
                 per_output = [[] for _ in flat]
             for i, o in enumerate(flat):

@@ -244,6 +244,7 @@ class CompiledFunction:
         self.op_profile: dict[str, list] = {}
         self._cache: "OrderedDict[Any, dict[Any, _Recorded]]" = OrderedDict()
         self._stats = CompilationStats()
+        self._latest = None             # (structure, signatures, recording, deterministic) of the most recent call
         self.__name__ = getattr(fn, "__name__", "compiled")
         self.__doc__ = getattr(fn, "__doc__", None)
 
@@ -253,6 +254,7 @@ class CompiledFunction:
 
     def clear_cache(self) -> None:
         self._cache.clear()
+        self._latest = None
 
     def release(self) -> None:
         """Drop every recorded schedule together with its CUDA graphs and the buffers they own.
@@ -270,6 +272,7 @@ class CompiledFunction:
                     for o in outs:
                         o._buffers = None
         self._cache.clear()
+        self._latest = None
 
     def dump_plan(self, file=None) -> str:
         """Text listing of every recorded schedule: one line per step with its kind (``op`` or
@@ -350,9 +353,47 @@ class CompiledFunction:
         return (td, tuple(sym), config.is_deterministic()), tuple(conc), leaves, td
 
     # ---- call
+    @staticmethod
+    def _same_as(latest: tuple, args: tuple) -> list | None:
+        """The argument leaves when this call has the structure and, leaf by leaf, the signature of the call
+        before it (then that call's recording serves, and neither keys are built nor hashed); else None."""
+        tds, conc, _, deterministic = latest
+        if deterministic != config.is_deterministic() or len(args) != len(tds):
+            return None
+        leaves: list = []
+        for a, td in zip(args, tds):
+            if type(a) is Tensor:
+                if td.kind != "leaf":
+                    return None
+                leaves.append(a)
+                continue
+            lv, td_a = pytree.tree_flatten(a)
+            if td_a != td:
+                return None
+            leaves += lv
+        for leaf, c in zip(leaves, conc):
+            if type(leaf) is not Tensor:
+                return None
+            im = leaf._impl
+            # conc: (shape, dtype, sharding signature, batch dims, device); only unsharded calls are kept
+            if im._shape != c[0] or im._dtype is not c[1] or im.sharding is not None or im.batch_dims != c[3] \
+                    or im._device != c[4] or im._buffers is None:
+                return None
+        return leaves
+
     def __call__(self, *args, **kwargs):
         args = tuple(_normalize_step_scalars(a) for a in args)
         kwargs = {k: _normalize_step_scalars(v) for k, v in kwargs.items()}
+        latest = self._latest           # read once: another thread may replace it
+        if latest is not None and not kwargs:
+            leaves = self._same_as(latest, args)
+            if leaves is not None:
+                self._stats.hits += 1              # the entry is the most recently used one already
+                t0 = time.perf_counter()
+                out = self._replay(latest[2], leaves)
+                self._stats.replay_time_s += time.perf_counter() - t0
+                return out
+        self._latest = None
         key, conc, leaves, td = self._keys(args, kwargs)
         pending = [t for t in leaves if isinstance(t, Tensor) and not t._impl.is_realized]
         if pending:
@@ -397,6 +438,8 @@ class CompiledFunction:
         t0 = time.perf_counter()
         out = self._replay(rec, [l for l in leaves if isinstance(l, Tensor)])
         self._stats.replay_time_s += time.perf_counter() - t0
+        if not kwargs and self.max_cache_size > 0 and all(type(l) is Tensor and l._impl.sharding is None for l in leaves):
+            self._latest = (td[0], conc, rec, config.is_deterministic())
         return out
 
     # ---- trace

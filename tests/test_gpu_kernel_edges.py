@@ -403,3 +403,50 @@ def test_pooling_cells(dtype, mode, N, H, W, C, k, s, p):
         dy[0, 0, 0, 0] = 0.0                           # torch routes a window of -inf to its first element
     (g,) = torch.autograd.grad(ref, xr, dy.double().permute(0, 3, 1, 2))
     torch.testing.assert_close(kernels.pool2d_bwd(x, dy, *k, *s, p, p, mode).double(), g.permute(0, 2, 3, 1), rtol=2.0 ** -7, atol=1e-6)
+
+
+# ---------------------------------------------------------------- compiled calls
+def test_compiled_calls_that_change_between_calls():
+    """The path for a call like the one before it: other shapes, types, structures and deterministic mode in
+    between, and two threads on one function."""
+    import threading
+
+    import nabla_b200 as nb
+    from nabla_b200 import config
+
+    f = nb.compile(lambda d, x: {"y": d["w"] * x + d["b"], "n": x})
+
+    def call(n, dtype, extra=False):
+        w, b, x = (torch.randn(n, device="cuda").to(dtype) for _ in range(3))
+        d = {"w": nb.Tensor.from_torch(w), "b": nb.Tensor.from_torch(b)}
+        if extra:
+            d["unused"] = nb.Tensor.from_torch(x)
+        out = f(d, nb.Tensor.from_torch(x))
+        torch.testing.assert_close(out["y"].to_torch().float(), (w * x + b).float(), rtol=2e-2, atol=2e-2)
+        assert torch.equal(out["n"].to_torch(), x)
+
+    for args in [(8, torch.float32), (8, torch.float32), (16, torch.float32), (16, torch.bfloat16), (16, torch.bfloat16), (8, torch.float32),
+                 (8, torch.float32, True), (8, torch.float32)] * 2:
+        call(*args)
+    misses = f.stats.misses
+    with config.deterministic():
+        call(8, torch.float32)
+    assert f.stats.misses == misses + 1
+    f.clear_cache()
+    call(8, torch.float32)
+    assert f.stats.misses == misses + 2
+    errors = []
+
+    def worker(n):
+        try:
+            for _ in range(20):
+                call(n, torch.float32)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    for n in (8, 16):
+        call(n, torch.float32)
+    threads = [threading.Thread(target=worker, args=(n,)) for n in (8, 16)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors
