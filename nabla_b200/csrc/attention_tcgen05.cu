@@ -166,6 +166,9 @@ struct FwdArgs {
   MaskArg mask;
   int* status;
   int bh_chunk;                 // see tile_order
+  int nsplit;                   // the keys are cut into this many ranges, one CTA each (1: no split)
+  float* part_o;                // nsplit > 1: [nsplit][B][H][Sq][HD] output over each range, fp32
+  float* part_lse;              //             [nsplit][B][H][Sq] natural-log sum of exponentials of each range
 };
 
 template <int HD>
@@ -210,8 +213,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return;
   const int nqt = (args.Sq + 2 * BT - 1) / (2 * BT);
   int bh_, rank;
-  tile_order(blockIdx.x, args.H * args.B, args.bh_chunk, nqt, bh_, rank);
+  tile_order(blockIdx.x, args.H * args.B * args.nsplit, args.bh_chunk, nqt, bh_, rank);
   const int qt = nqt - 1 - rank;          // the late tiles of a causal problem see the most keys
+  const int sp = bh_ % args.nsplit;
+  bh_ /= args.nsplit;
   const int h = bh_ % args.H;
   const int b = bh_ / args.H;
   const int q0 = qt * 2 * BT;
@@ -227,6 +232,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     n_t[t] = q0t < args.Sq ? n : 0;
   }
+  // this CTA's range of key tiles: [kt0, kt0 + n_t[t]) of query tile t
+  const int per = (max(n_t[0], n_t[1]) + args.nsplit - 1) / args.nsplit;
+  const int kt0 = sp * per;
+  n_t[0] = min(max(n_t[0] - kt0, 0), per);
+  n_t[1] = min(max(n_t[1] - kt0, 0), per);
   const int n_max = max(n_t[0], n_t[1]);
 
   if (threadIdx.x == 0) {
@@ -274,12 +284,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mbar_arrive_expect_tx(&k_full[st], L::TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
-          tma_load_4d(sK + st * L::TILE_BYTES + c * (BT * 128), &tmK, &k_full[st], c * 64, j * BT, h, b, args.Skv, args.H, args.B);
+          tma_load_4d(sK + st * L::TILE_BYTES + c * (BT * 128), &tmK, &k_full[st], c * 64, (kt0 + j) * BT, h, b, args.Skv, args.H, args.B);
         if (!mbar_wait(&v_empty[st], ph)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
         mbar_arrive_expect_tx(&v_full[st], L::TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
-          tma_load_4d(sV + st * L::TILE_BYTES + c * (BT * 128), &tmV, &v_full[st], c * 64, j * BT, h, b, args.Skv, args.H, args.B);
+          tma_load_4d(sV + st * L::TILE_BYTES + c * (BT * 128), &tmV, &v_full[st], c * 64, (kt0 + j) * BT, h, b, args.Skv, args.H, args.B);
       }
     }
   } else if (warp == 1) {
@@ -341,12 +351,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float* smask = reinterpret_cast<float*>(smem + L::OFF_MASK) + t * 2 * BT;
     const float mask_mul = LOG2E / args.scale_log2;
     float mnext = 0.f;
-    if (mshared && n > 0 && r < args.Skv) mnext = mrow[r];
+    if (mshared && n > 0 && kt0 * BT + r < args.Skv) mnext = mrow[kt0 * BT + r];
     const float2 sc2 = make_float2(args.scale_log2, args.scale_log2);
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      const int kv0 = j * BT;
+      const int kv0 = (kt0 + j) * BT;
       if (mshared) {
         smask[(j & 1) * BT + r] = mnext;
         named_bar_sync(2 + t, 128);
@@ -504,7 +514,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
-        if (q_idx < args.Sq) {
+        if (q_idx < args.Sq && args.nsplit > 1) {
+          float4* prow = reinterpret_cast<float4*>(args.part_o + ((((long long)sp * args.B + b) * args.H + h) * args.Sq + q_idx) * HD + c * 32);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            prow[u] = make_float4(__uint_as_float(v[4 * u]) * inv, __uint_as_float(v[4 * u + 1]) * inv,
+                                  __uint_as_float(v[4 * u + 2]) * inv, __uint_as_float(v[4 * u + 3]) * inv);
+        } else if (q_idx < args.Sq) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             uint4 pk;
@@ -516,9 +532,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
         }
       }
-      if (q_idx < args.Sq)
-        args.lse[((long long)b * args.H + h) * args.Sq + q_idx] =
-            have ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+      if (q_idx < args.Sq) {
+        const long long row = ((long long)b * args.H + h) * args.Sq + q_idx;
+        float* dst = args.nsplit > 1 ? args.part_lse + (long long)sp * args.B * args.H * args.Sq + row : args.lse + row;
+        *dst = have ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+      }
     }
   }
 
@@ -527,6 +545,187 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// O = sum_s w_s O_s with w_s = exp(lse_s - lse): joins the key ranges of a split forward pass. One warp per row; a range
+// in which the row sees no key has lse = -inf and weight 0.
+template <int HD>
+__global__ void __launch_bounds__(128) attn_fwd_combine_kernel(const FwdArgs args) {
+  constexpr int E = HD / 32;
+  const long long rows = (long long)args.B * args.H * args.Sq;
+  const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  float mx = -INFINITY;
+  bool nan = false;                                  // a NaN range makes the row NaN (fmaxf would drop it)
+  for (int s = lane; s < args.nsplit; s += 32) {
+    const float v = args.part_lse[s * rows + row];
+    mx = fmaxf(mx, v);
+    nan |= v != v;
+  }
+  if (__any_sync(0xffffffffu, nan)) mx = NAN;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = mx != mx ? mx : fmaxf(mx, v);
+  }
+  float acc[E], sum = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
+  if (mx != -INFINITY) {
+    for (int s = 0; s < args.nsplit; ++s) {
+      const float w = ex2((args.part_lse[s * rows + row] - mx) * LOG2E);
+      const float* p = args.part_o + (s * rows + row) * HD + lane * E;
+      sum += w;
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[e] = fmaf(w, p[e], acc[e]);
+    }
+  }
+  const bool have = !(sum <= 0.f);
+  const float inv = have ? 1.f / sum : 0.f;
+  const int q = (int)(row % args.Sq);
+  const long long bh = row / args.Sq;
+  __nv_bfloat16* orow = args.O + (bh / args.H) * args.o_sb + (bh % args.H) * args.o_sh + q * args.o_ss + lane * E;
+#pragma unroll
+  for (int e = 0; e < E; e += 2) *reinterpret_cast<uint32_t*>(orow + e) = pack_bf16(acc[e] * inv, acc[e + 1] * inv);
+  if (lane == 0) args.lse[row] = have ? mx + logf(sum) : -INFINITY;
+}
+
+// A few queries (at most 4 per head: decoding) against many keys, without a user mask. The work is one read of K
+// and V: no tile of 128 query rows, no tensor core; K and V go from global memory to registers, 16 bytes per
+// lane, HD / 8 lanes per key, DEC_U keys of K and of V in flight per lane, and every group of lanes keeps its
+// own running maximum, sum and output (fp32), joined at the end of the block and, over the key ranges
+// (gridDim.x), by attn_fwd_combine_kernel. 592 blocks (four per SM) of 4 x 16 B x 8 x 32 lanes hold the bytes
+// in flight that HBM needs. 64 heads, 1 query, 4001 keys of 128: 68 us with the tile kernel, 42 here with the join
+// (3.1 TB/s); 16 heads, 8000 keys: 120 -> 36 us.
+struct DecodeArgs {
+  FwdArgs f;
+  const __nv_bfloat16 *q, *k, *v;
+  long long q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss;
+};
+constexpr int DEC_MAX_Q = 4, DEC_U = 4;
+
+template <int HD, int NQ>
+__global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeArgs a) {
+  constexpr int LPK = HD / 8, KPW = 32 / LPK, G = 4 * KPW;      // lanes per key, keys per warp, lane groups per block
+  const FwdArgs& f = a.f;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LPK, d0 = (lane % LPK) * 8;
+  const int grp = warp * KPW + sub;
+  const int sp = blockIdx.x, h = blockIdx.y % f.H, b = blockIdx.y / f.H;
+  const int per = (f.Skv + f.nsplit - 1) / f.nsplit;
+  const int k0 = sp * per, k1 = min(f.Skv, k0 + per);
+  float q[NQ][8], acc[NQ][8], m[NQ], l[NQ];
+#pragma unroll
+  for (int i = 0; i < NQ; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+    uint4 raw = make_uint4(0, 0, 0, 0);
+    if (i < f.Sq) raw = *reinterpret_cast<const uint4*>(a.q + b * a.q_sb + h * a.q_sh + i * a.q_ss + d0);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      q[i][e] = __uint_as_float(e & 1 ? w[e >> 1] & 0xffff0000u : w[e >> 1] << 16) * f.scale_log2;
+      acc[i][e] = 0.f;
+    }
+  }
+  const __nv_bfloat16* kp = a.k + b * a.k_sb + h * a.k_sh + d0;
+  const __nv_bfloat16* vp = a.v + b * a.v_sb + h * a.v_sh + d0;
+  for (int kb = k0 + grp; kb - grp < k1; kb += G * DEC_U) {
+    uint4 kr[DEC_U], vr[DEC_U];
+#pragma unroll
+    for (int u = 0; u < DEC_U; ++u) {
+      const int k = kb + u * G;
+      kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
+      if (k < k1) {
+        kr[u] = *reinterpret_cast<const uint4*>(kp + k * a.k_ss);
+        vr[u] = *reinterpret_cast<const uint4*>(vp + k * a.v_ss);
+      }
+    }
+    float s[NQ][DEC_U];
+#pragma unroll
+    for (int u = 0; u < DEC_U; ++u) {
+      const uint32_t w[4] = {kr[u].x, kr[u].y, kr[u].z, kr[u].w};
+#pragma unroll
+      for (int i = 0; i < NQ; ++i) s[i][u] = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = __uint_as_float(e & 1 ? w[e >> 1] & 0xffff0000u : w[e >> 1] << 16);
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) s[i][u] = fmaf(q[i][e], x, s[i][u]);
+      }
+    }
+#pragma unroll
+    for (int o = LPK / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < NQ; ++i)
+#pragma unroll
+        for (int u = 0; u < DEC_U; ++u) s[i][u] += __shfl_xor_sync(0xffffffffu, s[i][u], o);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const int lim = min(k1, f.causal ? f.Skv - f.Sq + i + 1 : f.Skv);      // keys below lim are visible
+      float mx = m[i];
+#pragma unroll
+      for (int u = 0; u < DEC_U; ++u) {
+        if (kb + u * G >= lim) s[i][u] = -INFINITY;
+        mx = fmaxf(mx, s[i][u]);
+      }
+      const float ms = mx == -INFINITY ? 0.f : mx;
+      const float corr = ex2(m[i] - ms);
+      m[i] = mx;
+      l[i] *= corr;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[i][e] *= corr;
+#pragma unroll
+      for (int u = 0; u < DEC_U; ++u) {
+        s[i][u] = ex2(s[i][u] - ms);
+        l[i] += s[i][u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < DEC_U; ++u) {
+      const uint32_t w[4] = {vr[u].x, vr[u].y, vr[u].z, vr[u].w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = __uint_as_float(e & 1 ? w[e >> 1] & 0xffff0000u : w[e >> 1] << 16);
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) acc[i][e] = fmaf(s[i][u], x, acc[i][e]);
+      }
+    }
+  }
+  __shared__ float sm[G][NQ], sl[G][NQ], so[G][NQ][HD];
+#pragma unroll
+  for (int i = 0; i < NQ; ++i) {
+    if (d0 == 0) { sm[grp][i] = m[i]; sl[grp][i] = l[i]; }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) so[grp][i][d0 + e] = acc[i][e];
+  }
+  __syncthreads();
+  const long long rows = (long long)f.B * f.H * f.Sq;
+  for (int t = threadIdx.x; t < NQ * HD; t += 128) {
+    const int i = t / HD, d = t % HD;
+    if (i >= f.Sq) break;
+    float mx = -INFINITY, sum = 0.f, o = 0.f;
+#pragma unroll
+    for (int g = 0; g < G; ++g) mx = fmaxf(mx, sm[g][i]);
+    const float ms = mx == -INFINITY ? 0.f : mx;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const float w = ex2(sm[g][i] - ms);
+      sum = fmaf(w, sl[g][i], sum);
+      o = fmaf(w, so[g][i][d], o);
+    }
+    const bool have = !(sum <= 0.f);                 // NaN counts: it has to show
+    o = have ? o / sum : 0.f;
+    const float lse = have ? (mx + log2f(sum)) * 0.6931471805599453f : -INFINITY;
+    const long long row = ((long long)b * f.H + h) * f.Sq + i;
+    if (f.nsplit > 1) {
+      f.part_o[(sp * rows + row) * HD + d] = o;
+      if (d == 0) f.part_lse[sp * rows + row] = lse;
+    } else {
+      f.O[b * f.o_sb + h * f.o_sh + i * f.o_ss + d] = __float2bfloat16(o);
+      if (d == 0) f.lse[row] = lse;
+    }
   }
 }
 
@@ -1250,6 +1449,22 @@ static int l2_chunk(int nbh, long long rows, int hd) {
   return (int)(n < 1 ? 1 : n > nbh ? nbh : n);
 }
 
+template <int HD>
+static void combine(const FwdArgs& a, cudaStream_t stream) {
+  const long long rows = (long long)a.B * a.H * a.Sq;
+  attn_fwd_combine_kernel<HD><<<(unsigned)((rows + 3) / 4), 128, 0, stream>>>(a);
+}
+
+template <int HD>
+static int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
+  const dim3 grid(a.f.nsplit, a.f.B * a.f.H);
+  if (a.f.Sq == 1) attn_decode_kernel<HD, 1><<<grid, 128, 0, stream>>>(a);
+  else if (a.f.Sq == 2) attn_decode_kernel<HD, 2><<<grid, 128, 0, stream>>>(a);
+  else attn_decode_kernel<HD, 4><<<grid, 128, 0, stream>>>(a);
+  if (a.f.nsplit > 1) combine<HD>(a.f, stream);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 template <int HD, bool MASK>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a,
                       cudaStream_t stream) {
@@ -1260,9 +1475,10 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     configured = true;
   }
   const int nqt = (a.Sq + 2 * BT - 1) / (2 * BT);
-  const long long grid = (long long)nqt * a.H * a.B;
+  const long long grid = (long long)nqt * a.H * a.B * a.nsplit;
   if (grid <= 0) return 0;
   attn_fwd_kernel<HD, MASK><<<(unsigned)grid, NTHREADS, L::TOTAL, stream>>>(tq, tk, tv, a);
+  if (a.nsplit > 1) combine<HD>(a, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -1284,19 +1500,55 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 
 }  // namespace nba
 
+// Few queries and no user mask: the decode kernel (gridDim.y holds the (batch, head) pairs).
+static bool attn_decode(int B, int H, int Sq, bool mask) { return Sq <= nba::DEC_MAX_Q && !mask && (long long)B * H <= 65535; }
+
+// Key ranges that a forward pass is cut into (1: none).
+// Decode kernel: ranges of at least 128 keys, for four blocks per SM.
+// Otherwise a CTA owns 256 queries of one (batch, head), so a short query block against a long prefix gives one
+// CTA per (batch, head), each walking all key tiles alone. The rule counts what the busiest SM walks: waves *
+// (key tiles per CTA + 3), the 3 standing for a CTA's start and end, and splits only where that falls below
+// 0.8 of the unsplit count (the partial results cost a second launch). With more than one block of 256 queries
+// it stays as it is: 64 such CTAs (2 x 8 heads x 1001 queries, causal) took 25.6 us, split and joined 27.6.
+extern "C" int nb_attn_fwd_splits(int B, int H, int Sq, int Skv, int has_mask) {
+  constexpr int SMS = 148;
+  if (B <= 0 || H <= 0 || Sq <= 0 || Skv <= 0) return 1;
+  if (attn_decode(B, H, Sq, has_mask != 0)) {
+    long long s = (4ll * SMS + (long long)B * H - 1) / ((long long)B * H);
+    if (s > Skv / 128) s = Skv / 128;
+    return (int)(s < 1 ? 1 : s > 64 ? 64 : s);
+  }
+  const long long ctas = (long long)B * H;
+  const int n = (Skv + nba::BT - 1) / nba::BT;
+  if (Sq > 2 * nba::BT || ctas >= SMS || n < 4) return 1;
+  int best = 1;
+  long long best_cost = n + 3;
+  for (int s = 2; s <= 32 && s <= n; ++s) {
+    const long long cost = ((ctas * s + SMS - 1) / SMS) * ((n + s - 1) / s + 3);
+    if (cost < best_cost && 10 * cost < 8 * (n + 3)) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 // q, k, v: bf16 (B, H, S, D) views, D contiguous, strides in elements (multiples of 8, 16-byte
 // aligned bases). o: bf16 with its own strides. lse: fp32 [B][H][Sq]. D in {64, 128}.
 // mask: optional fp32 additive mask (null = none), element strides m_sb, m_sh, m_sq (0 = broadcast),
-// key stride 1.
+// key stride 1. nsplit = nb_attn_fwd_splits(...) or 1; above 1 part_o / part_lse are fp32 scratch of
+// nsplit * B * H * Sq * D and nsplit * B * H * Sq elements (16-byte aligned).
 extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H, int Sq,
                            int Skv, int D, long long q_sb, long long q_sh, long long q_ss, long long k_sb,
                            long long k_sh, long long k_ss, long long v_sb, long long v_sh, long long v_ss,
                            long long o_sb, long long o_sh, long long o_ss, float scale, int causal, const float* mask,
-                           long long m_sb, long long m_sh, long long m_sq, int* status, void* stream) {
+                           long long m_sb, long long m_sh, long long m_sq, int nsplit, float* part_o,
+                           float* part_lse, int* status, void* stream) {
   using namespace nba;
   if (D != 64 && D != 128) return -10;
   if (!(scale > 0.f)) return -13;
   if (B <= 0 || H <= 0 || Sq <= 0) return 0;
+  if (nsplit < 1 || (nsplit > 1 && (part_o == nullptr || part_lse == nullptr || (reinterpret_cast<uintptr_t>(part_o) & 15)))) return -14;
   const long long strides[] = {q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_ss, o_sh, o_sb};
   for (long long s : strides)
     if (s & 7) return -12;
@@ -1312,8 +1564,14 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   a.lse = lse;
   a.mask = MaskArg{mask, m_sb, m_sh, m_sq};
   a.status = status;
-  a.bh_chunk = causal ? l2_chunk(B * H, Skv, D) : 1;
+  a.bh_chunk = causal ? l2_chunk(B * H, Skv, D) * nsplit : 1;
+  a.nsplit = nsplit; a.part_o = part_o; a.part_lse = part_lse;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (Skv > 0 && attn_decode(B, H, Sq, mask != nullptr)) {
+    const DecodeArgs d{a, reinterpret_cast<const __nv_bfloat16*>(q), reinterpret_cast<const __nv_bfloat16*>(k),
+                       reinterpret_cast<const __nv_bfloat16*>(v), q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss};
+    return D == 128 ? launch_decode<128>(d, s) : launch_decode<64>(d, s);
+  }
   CUtensorMap tq, tk, tv;
   int r;
   if ((r = make_map4(&tq, q, B, H, Sq, D, q_sb, q_sh, q_ss))) return r;

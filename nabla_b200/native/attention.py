@@ -14,13 +14,14 @@ import torch
 
 launch_count = 0
 _fwd = None
+_splits = None
 _bwd = None
 _checked = False
 c_int, c_ll, c_f, c_vp = ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p
 
 
 def _lib():
-    global _fwd, _bwd, _checked
+    global _fwd, _splits, _bwd, _checked
     if not _checked:
         _checked = True
         from . import available, load
@@ -29,7 +30,10 @@ def _lib():
             lib = load("libnb_attention.so")
             f = lib.nb_attn_fwd
             f.restype = c_int
-            f.argtypes = [c_vp] * 5 + [c_int] * 5 + [c_ll] * 12 + [c_f, c_int, c_vp, c_ll, c_ll, c_ll, c_vp, c_vp]
+            f.argtypes = [c_vp] * 5 + [c_int] * 5 + [c_ll] * 12 + [c_f, c_int, c_vp, c_ll, c_ll, c_ll, c_int, c_vp, c_vp, c_vp, c_vp]
+            lib.nb_attn_fwd_splits.restype = c_int
+            lib.nb_attn_fwd_splits.argtypes = [c_int] * 5
+            _splits = lib.nb_attn_fwd_splits
             _fwd = f
             if hasattr(lib, "nb_attn_bwd"):
                 g = lib.nb_attn_bwd
@@ -106,13 +110,19 @@ def sdpa_fwd(q, k, v, *, causal: bool, scale: float, mask=None):
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
     st = status_word(q.device)
     m, m_sb, m_sh, m_sq = _mask_args(mask, B, H, Sq, Skv)
+    ns = _splits(B, H, Sq, Skv, int(m is not None))
+    # fp32 results of the key ranges: nsplit x (output, log-sum-exp)
+    part = torch.empty(ns * B * H * Sq * (D + 1), dtype=torch.float32, device=q.device) if ns > 1 else None
+    p_o = 0 if part is None else part.data_ptr()
+    p_lse = 0 if part is None else p_o + ns * B * H * Sq * D * 4
     rc = _lib()(ptr(q), ptr(k), ptr(v), ptr(o_mem), ptr(lse), B, H, Sq, Skv, D,
               q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
               v.stride(0), v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2),
-              float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()), m_sb, m_sh, m_sq, ptr(st), stream_ptr())
+              float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()), m_sb, m_sh, m_sq, ns, c_vp(p_o), c_vp(p_lse),
+              ptr(st), stream_ptr())
     if rc != 0:
         raise RuntimeError(f"nb_attn_fwd failed with code {rc}")
-    launch_count += 1
+    launch_count += 1 if ns == 1 else 2
     return o, lse
 
 

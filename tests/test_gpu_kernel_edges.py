@@ -450,3 +450,26 @@ def test_compiled_calls_that_change_between_calls():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not errors
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Sq,Skv", [(1, 1, 1, 1), (2, 3, 1, 31), (1, 2, 2, 127), (1, 2, 3, 128), (2, 1, 4, 257), (1, 4, 1, 4001), (3, 5, 4, 700),
+                                        (40, 16, 1, 300), (1, 1, 5, 4000), (2, 4, 33, 2500), (1, 2, 130, 1500), (1, 1, 300, 3000)])
+def test_attention_of_few_queries_over_a_long_prefix(B, H, Sq, Skv, D):
+    """The decode kernel (up to 4 queries), one key range and many, and the split of the tile kernel; keys and
+    values as slices of a longer cache."""
+    torch.manual_seed(3)
+    q = torch.randn(B, H, Sq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(B, H, Skv + 8, D, device="cuda", dtype=torch.bfloat16)[:, :, 5:5 + Skv] for _ in range(2))
+    for causal in ([False, True] if Sq <= Skv else [False]):
+        _attention_check(q, k, v, causal, grads=1 < Skv and Sq * Skv < 100000)    # (one key: the score gradients are 0)
+
+
+def test_attention_shows_a_nan_key_in_every_split():
+    from nabla_b200.native import attention
+
+    q = torch.randn(1, 2, 1, 128, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(1, 2, 3000, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    k[0, 1, 2500] = float("nan")
+    o, lse = attention.sdpa_fwd(q, k, v, causal=True, scale=0.09)
+    assert bool(torch.isfinite(o[0, 0]).all()) and bool(torch.isnan(o[0, 1]).all()) and bool(torch.isnan(lse[0, 1]).all())
