@@ -9,7 +9,10 @@ from __future__ import annotations
 from typing import Any, Callable
 
 _registry: dict[type, tuple[Callable, Callable]] = {}
-_leaf_types: set[type] = set()      # types already found to be leaves (emptied by every registration)
+# Types already found to be leaves, so that a leaf does not walk the registry. A registration puts a new set in its
+# place: a thread that looked a type up before it adds the type to the old one.
+_leaf_types: set[type] = set()
+_MAX_LEAF_TYPES = 256
 
 
 def register_pytree_node(cls: type, flatten_fn: Callable, unflatten_fn: Callable) -> None:
@@ -17,8 +20,9 @@ def register_pytree_node(cls: type, flatten_fn: Callable, unflatten_fn: Callable
     ``unflatten_fn(aux, children) -> obj``."""
     if not isinstance(cls, type):
         raise TypeError("cls must be a type")
+    global _leaf_types
     _registry[cls] = (flatten_fn, unflatten_fn)
-    _leaf_types.clear()
+    _leaf_types = set()
 
 
 def _freeze(v: Any) -> Any:
@@ -94,7 +98,8 @@ def _flatten(tree: Any, leaves: list, is_leaf) -> PyTreeDef:
     if tree is None:
         return _NONE
     t = type(tree)
-    if t in _leaf_types:
+    known = _leaf_types
+    if t in known:
         leaves.append(tree)
         return _LEAF
     if t is list or t is tuple:
@@ -117,8 +122,8 @@ def _flatten(tree: Any, leaves: list, is_leaf) -> PyTreeDef:
     if isinstance(tree, tuple) and hasattr(tree, "_fields"):  # namedtuple
         ch = tuple(_flatten(x, leaves, is_leaf) for x in tree)
         return PyTreeDef("custom", (t, "namedtuple"), ch, sum(c.num_leaves for c in ch))
-    if not isinstance(tree, tuple):
-        _leaf_types.add(t)
+    if not isinstance(tree, tuple) and len(known) < _MAX_LEAF_TYPES:
+        known.add(t)
     leaves.append(tree)
     return _LEAF
 
