@@ -443,7 +443,7 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
     const int grp = (warp - 4) >> 2;
     // bf16 rows that are not 16-byte aligned (N or ldc not a multiple of 8: an odd vocabulary) leave through
     // shared memory as runs of 64 columns of one row. A lane storing its own row would touch 32 rows, 32
-    // sectors, per 2-byte store.
+    // sectors, per 2-byte store: 4096 x 10001 x 512 took 554 us, 153 this way.
     const bool staged = MODE == MODE_NONE && !args.vec_ok && !args.out_fp32 && !args.accumulate;
     const bool heavy = (args.epi == EPI_BIAS_GELU || args.aux == AUX_MUL_DGELU) && !staged;
     bool ok = true;
