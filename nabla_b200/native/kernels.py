@@ -277,14 +277,12 @@ class CopyBatch:
 
     def __init__(self, fixed: list[torch.Tensor], shared: bool = False):
         n = len(fixed)
-        dev = torch.cuda.current_device()
+        self.dev = dev = torch.cuda.current_device()
         self.fixed = fixed
         self.strides = [t.stride() for t in fixed]
         self.fixed_ptrs = (c_vp * n)(*[t.data_ptr() for t in fixed])
         self.own = [t.data_ptr() for t in fixed]
-        self.other_ptrs = (c_vp * n)()
         self.size = [t.numel() * t.element_size() for t in fixed]
-        self.bytes = (c_ull * n)()
         # what one launch can move: dense tensors of this device (a CPU scalar among the inputs is not one)
         self.plain = [t.is_cuda and t.device.index == dev and _is_dense(t) for t in fixed]
         self.storages = {t.untyped_storage().data_ptr() for t in fixed} if shared else None
@@ -294,10 +292,12 @@ class CopyBatch:
         alone; one whose layouts differ goes through torch's copy, and so does every pair, in order, when a
         source lies in the memory of another pair's destination."""
         global launch_count
-        ptrs, nbytes, own, copies = self.other_ptrs, self.bytes, self.own, False
+        own, copies = self.own, False
+        n = len(own)
+        ptrs, nbytes = (c_vp * n)(), (c_ull * n)()          # of this call: another thread may be in here too
+        here = torch.cuda.current_device() == self.dev
         for i, o in enumerate(others):
             p = o.data_ptr()
-            nbytes[i] = 0
             if p == own[i]:
                 continue
             f = self.fixed[i]
@@ -306,7 +306,7 @@ class CopyBatch:
                     if f.data_ptr() != o.data_ptr():
                         f.copy_(o) if into_fixed else o.copy_(f)
                 return
-            if self.plain[i] and o.dtype is f.dtype and o.stride() == self.strides[i] and o.device == f.device:
+            if here and self.plain[i] and o.dtype is f.dtype and o.stride() == self.strides[i] and o.device == f.device:
                 ptrs[i] = p
                 nbytes[i] = self.size[i]
                 copies = True
@@ -316,7 +316,7 @@ class CopyBatch:
         if not copies:
             return
         dst, src = (self.fixed_ptrs, ptrs) if into_fixed else (ptrs, self.fixed_ptrs)
-        k = _L().nb_copy_batch(dst, src, nbytes, len(own), stream_ptr())
+        k = _L().nb_copy_batch(dst, src, nbytes, n, stream_ptr())
         if k < 0:
             raise RuntimeError(f"copy_batch failed with code {k}")
         launch_count += k
