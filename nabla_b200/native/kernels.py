@@ -289,11 +289,15 @@ class CopyBatch:
 
     def run(self, others: list[torch.Tensor], into_fixed: bool) -> None:
         """``fixed <- others`` (``into_fixed``) or ``others <- fixed``. A pair that shares its storage is left
-        alone; one whose layouts differ goes through torch's copy, and so does every pair, in order, when a
-        source lies in the memory of another pair's destination."""
+        alone; one whose layouts differ goes through torch's copy. A source that lies in the memory of the fixed
+        tensors (a result of the captured step that comes back in another place) is copied aside first, so that
+        every pair reads what was there before the call."""
         global launch_count
         own, copies = self.own, False
         n = len(own)
+        if self.storages is not None and into_fixed:
+            others = [o.clone() if o.data_ptr() != own[i] and o.untyped_storage().data_ptr() in self.storages else o
+                      for i, o in enumerate(others)]
         ptrs, nbytes = (c_vp * n)(), (c_ull * n)()          # of this call: another thread may be in here too
         here = torch.cuda.current_device() == self.dev
         for i, o in enumerate(others):
@@ -301,11 +305,6 @@ class CopyBatch:
             if p == own[i]:
                 continue
             f = self.fixed[i]
-            if self.storages is not None and o.untyped_storage().data_ptr() in self.storages:
-                for f, o in zip(self.fixed, others):
-                    if f.data_ptr() != o.data_ptr():
-                        f.copy_(o) if into_fixed else o.copy_(f)
-                return
             if here and self.plain[i] and o.dtype is f.dtype and o.stride() == self.strides[i] and o.device == f.device:
                 ptrs[i] = p
                 nbytes[i] = self.size[i]

@@ -260,12 +260,37 @@ def test_copy_batch_moves_every_size_alignment_and_type():
     assert all(torch.equal(a, b) for a, b in zip(out, fixed))
 
 
-def test_copy_batch_keeps_the_order_where_pairs_share_memory():
+def test_copy_batch_reads_before_it_writes_where_pairs_share_memory():
     from nabla_b200.native import kernels
 
     a, b = torch.zeros(8, device="cuda"), torch.ones(8, device="cuda")
-    kernels.CopyBatch([a, b], shared=True).run([b, a], into_fixed=True)     # one after the other: a <- b, then b <- a
-    assert bool((a == 1).all()) and bool((b == 1).all())
+    kernels.CopyBatch([a, b], shared=True).run([b, a], into_fixed=True)
+    assert bool((a == 1).all()) and bool((b == 0).all())
+    c = torch.arange(12.0, device="cuda").view(3, 4)
+    d = torch.zeros(4, device="cuda")
+    kernels.CopyBatch([c, d], shared=True).run([torch.full((3, 4), 5.0, device="cuda"), c[1]], into_fixed=True)   # a view of another pair
+    assert bool((c == 5).all()) and d.tolist() == [4.0, 5.0, 6.0, 7.0]
+
+
+@pytest.mark.parametrize("order", [(1, 0, 2), (1, 2, 0), (0, 1, 2)])
+def test_captured_function_whose_donated_results_come_back_in_other_places(order):
+    import nabla_b200 as nb
+
+    def step(x, y, z):
+        return x, y, z, x * 2.0 + y          # the first three live in the donated buffers
+
+    start = [torch.randn(40, device="cuda") for _ in range(3)]
+    got = {}
+    for graph in (False, True):
+        f = nb.compile(step, cuda_graph=graph, donate_argnums=(0, 1, 2))
+        state, seen = [nb.Tensor.from_torch(t.clone()) for t in start], []
+        for _ in range(5):
+            *out, extra = f(*state)
+            seen.append(extra.to_torch().clone())
+            state = [out[i] for i in order]
+        got[graph] = seen + [t.to_torch().clone() for t in state]
+    for a, b in zip(got[True], got[False]):
+        assert torch.equal(a, b)
 
 
 def test_captured_function_with_odd_inputs():
