@@ -1510,13 +1510,24 @@ __device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
 
 constexpr int CONV_KC = 32;      // values of k staged at a time
 
+// Filter tap k = (r, s, c) and its offset from the first pixel of a window, 16 bytes. The offset is
+// 64 bits wide: r * W * C may pass 2^31 where the image is large, or low but padded to a tall filter.
+struct __align__(16) ConvTap {
+  int r, s;
+  long long off;
+};
+__device__ __forceinline__ ConvTap conv_tap(int k, const ConvGeom& g) {
+  const int rs = k / g.C, r = rs / g.S, s = rs - r * g.S;
+  return ConvTap{r, s, ((long long)r * g.W + s) * g.C + (k - rs * g.C)};
+}
+
 template <typename T, int FG, bool VEC>
 __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                            const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g) {
   constexpr int PG = 128 / FG, MT = 2 * PG, FT = 4 * FG, PER = (MT + 127) / 128, KSTEP = MT < 128 ? 128 / MT : 1;
   __shared__ __align__(16) float xs[CONV_KC][MT + 4];
   __shared__ __align__(16) float ws[CONV_KC][FT];
-  __shared__ int krs[CONV_KC], koff[CONV_KC];       // (r << 16 | s) and the offset of (r, s, c) from a window's first pixel
+  __shared__ ConvTap taps[CONV_KC];
   const int tid = threadIdx.x;
   const long long positions = (long long)g.N * g.OH * g.OW;
   const long long m0 = (long long)blockIdx.x * MT;
@@ -1553,11 +1564,7 @@ __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict_
   for (int k0 = 0; k0 < K; k0 += CONV_KC) {
     const int kn = min(CONV_KC, K - k0);
     __syncthreads();
-    if (tid < kn) {
-      const int k = k0 + tid, rs = k / g.C, r = rs / g.S;
-      krs[tid] = r << 16 | (rs - r * g.S);
-      koff[tid] = (r * g.W + (rs - r * g.S)) * g.C + (k - rs * g.C);
-    }
+    if (tid < kn) taps[tid] = conv_tap(k0 + tid, g);
     for (int e = tid; e < kn * FT; e += 128) {
       const int k = e / FT, f = f0 + e % FT;
       const float v = f < g.F ? to_f<T>(w[(size_t)(k0 + k) * g.F + f]) : 0.f;
@@ -1568,15 +1575,15 @@ __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict_
     constexpr int KV = VEC ? 4 : 1;                  // VEC (C % 4 == 0): four channels of one pixel per load
 #pragma unroll 8
     for (int k = (MT < 128 ? tid / MT : 0) * KV; k < kn; k += KSTEP * KV) {
-      const int rs = krs[k], off = koff[k];
+      const ConvTap tap = taps[k];
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
-        const int ih = ih0[j] + (rs >> 16), iw = iw0[j] + (rs & 0xffff);
+        const int ih = ih0[j] + tap.r, iw = iw0[j] + tap.s;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W &&
-            NB_IN_BOUNDS(NB_SITE_CONV_INPUT, base[j] + off + KV - 1, (long long)g.N * g.H * g.W * g.C)) {
-          if (VEC) load4(x + base[j] + off, v);
-          else v[0] = to_f<T>(x[base[j] + off]);
+            NB_IN_BOUNDS(NB_SITE_CONV_INPUT, base[j] + tap.off + KV - 1, (long long)g.N * g.H * g.W * g.C)) {
+          if (VEC) load4(x + base[j] + tap.off, v);
+          else v[0] = to_f<T>(x[base[j] + tap.off]);
         }
 #pragma unroll
         for (int i = 0; i < KV; ++i) xs[k + i][(tid % (MT < 128 ? MT : 128)) + j * 128] = v[i];
@@ -1634,7 +1641,8 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __
   constexpr int SL = 128 / (KG * FG), KT = 4 * KG, FT = 4 * FG;
   constexpr int RED = SL > 1 ? 128 * 16 : 4, STAGE = WG_MC * (KT + FT);
   __shared__ __align__(16) float sm[RED > STAGE ? RED : STAGE];
-  __shared__ int krs[KT], koff[KT];
+  constexpr int KV = VEC ? 4 : 1;                    // VEC (C % 4 == 0): four channels of one pixel per load
+  __shared__ int tap_r[KT / KV], tap_s[KT / KV];
   __shared__ int mh[WG_MC], mw[WG_MC];
   __shared__ long long mb[WG_MC];
   float (*xs)[KT] = reinterpret_cast<float (*)[KT]>(sm);
@@ -1643,10 +1651,12 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __
   const int K = g.R * g.S * g.C, k0 = blockIdx.x * KT, f0 = blockIdx.y * FT;
   const long long positions = (long long)g.N * g.OH * g.OW;
   const long long p0 = blockIdx.z * per_block, p1 = min(positions, p0 + per_block);
-  if (tid < KT) {
-    const int k = min(k0 + tid, K - 1), rs = k / g.C, r = rs / g.S;
-    krs[tid] = r << 16 | (rs - r * g.S);
-    koff[tid] = (r * g.W + (rs - r * g.S)) * g.C + (k - rs * g.C);
+  // the tap that this thread stages, of every (128 KV / KT)-th position
+  const int kq = tid % (KT / KV), kt = k0 + kq * KV;
+  const ConvTap tap = conv_tap(min(kt, K - KV), g);
+  if (tid < KT / KV) {
+    tap_r[tid] = tap.r;
+    tap_s[tid] = tap.s;
   }
   const int fg = tid % FG, kg = (tid / FG) % KG, sl = tid / (FG * KG);
   float acc[4][4];
@@ -1675,19 +1685,17 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __
       ds[m][e % FT] = v;
     }
     odd = __syncthreads_or(odd);
-    constexpr int KV = VEC ? 4 : 1;                  // VEC (C % 4 == 0): four channels of one pixel per load
 #pragma unroll 8
-    for (int e = tid; e < WG_MC * KT / KV; e += 128) {
-      const int m = e / (KT / KV), k = e % (KT / KV) * KV, rs = krs[k];
-      const int ih = mh[m] + (rs >> 16), iw = mw[m] + (rs & 0xffff);
+    for (int m = tid / (KT / KV); m < WG_MC; m += 128 / (KT / KV)) {
+      const int ih = mh[m] + tap.r, iw = mw[m] + tap.s;
       float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (m < mn && k0 + k < K && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W &&
-          NB_IN_BOUNDS(NB_SITE_CONV_INPUT, mb[m] + koff[k] + KV - 1, (long long)g.N * g.H * g.W * g.C)) {
-        if (VEC) load4(x + mb[m] + koff[k], v);
-        else v[0] = to_f<T>(x[mb[m] + koff[k]]);
+      if (m < mn && kt < K && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W &&
+          NB_IN_BOUNDS(NB_SITE_CONV_INPUT, mb[m] + tap.off + KV - 1, (long long)g.N * g.H * g.W * g.C)) {
+        if (VEC) load4(x + mb[m] + tap.off, v);
+        else v[0] = to_f<T>(x[mb[m] + tap.off]);
       }
-      if (VEC) *reinterpret_cast<float4*>(&xs[m][k]) = make_float4(v[0], v[1], v[2], v[3]);
-      else xs[m][k] = v[0];
+      if (VEC) *reinterpret_cast<float4*>(&xs[m][kq * KV]) = make_float4(v[0], v[1], v[2], v[3]);
+      else xs[m][kq * KV] = v[0];
     }
     __syncthreads();
     if (!odd) {
@@ -1705,7 +1713,7 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __
       for (int m = sl; m < mn; m += SL)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int rs = krs[kg * 4 + i], ih = mh[m] + (rs >> 16), iw = mw[m] + (rs & 0xffff);
+          const int ih = mh[m] + tap_r[(kg * 4 + i) / KV], iw = mw[m] + tap_s[(kg * 4 + i) / KV];
           if (ih < 0 || ih >= g.H || iw < 0 || iw >= g.W) continue;
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[m][kg * 4 + i], ds[m][fg * 4 + j], acc[i][j]);
@@ -2272,11 +2280,12 @@ int nb_sum_slices(const float* part, void* out, long long n, int slices, int dty
   return CHECK_LAUNCH();
 }
 
-// Position slices of the filter gradient: enough blocks for four per SM, at least 256 positions each.
+// Position slices of the filter gradient: four blocks per SM and no more, since a few blocks above that would
+// be a wave of their own (8 x 224 x 224 x 3 -> 64, 7 x 7: 594 blocks 310 us, 588 blocks 218); at least 256 positions each.
 int nb_conv2d_wgrad_slices(long long positions, int K, int F) {
   const int kt = K <= 16 ? 16 : K <= 32 ? 32 : 64, ft = F <= 16 ? 16 : 32;
   const long long tiles = (long long)((K + kt - 1) / kt) * ((F + ft - 1) / ft);
-  long long z = (148 * 4 + tiles - 1) / tiles;
+  long long z = 148 * 4 / tiles;
   if (z > (positions + 255) / 256) z = (positions + 255) / 256;
   return (int)(z < 1 ? 1 : z);
 }

@@ -83,6 +83,38 @@ def test_direct_convolution_skips_padding_under_infinite_operands():
     torch.testing.assert_close(dw.double(), ref, rtol=1e-5, atol=1e-5, equal_nan=True)
 
 
+@pytest.mark.parametrize("H,W,R,S,pad", [(1, 1 << 20, 2100, 1, (2099, 0, 0, 0)), (2, 4, 40000, 1, (39999, 0, 0, 0)), (1, 2, 1, 70000, (0, 0, 69999, 0))])
+def test_direct_convolution_with_tall_and_wide_filters(H, W, R, S, pad):
+    """Filter taps whose offset in the image passes 2^31 (only the last rows of the filter meet the image), and
+    more rows and columns than 16 bits hold. Small whole values: every sum is exact."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(1)
+    x = torch.randint(-3, 4, (1, H, W, 1), device="cuda").float()
+    w = torch.randint(-3, 4, (R, S, 1, 1), device="cuda").float()
+    y = kernels.conv2d_direct(x, w, None, (1, 1), pad)
+    dy = torch.randint(-1, 2, y.shape, device="cuda").float()
+    dw = kernels.conv2d_wgrad_direct(x, dy, tuple(w.shape), (1, 1), pad)
+    ref, ref_dw = torch.zeros_like(y, dtype=torch.float64), torch.zeros_like(w, dtype=torch.float64)
+    for oh in range(y.shape[1]):
+        for ow in range(y.shape[2]) if S > 1 else [slice(None)]:
+            # the window's first row (column) lies pad above (left of) output row oh (column ow)
+            rows = slice(max(0, pad[0] - oh), min(R, H + pad[0] - oh))
+            top = rows.start - (pad[0] - oh)
+            n = rows.stop - rows.start
+            if S > 1:
+                cols = slice(max(0, pad[2] - ow), min(S, W + pad[2] - ow))
+                left, m = cols.start - (pad[2] - ow), cols.stop - cols.start
+                part = x[0, top:top + n, left:left + m, 0].double()
+                ref[0, oh, ow, 0] = (w[rows, cols, 0, 0].double() * part).sum()
+                ref_dw[rows, cols, 0, 0] += part * dy[0, oh, ow, 0].double()
+            else:
+                part = x[0, top:top + n, :, 0].double()
+                ref[0, oh, :, 0] = (w[rows, 0, 0, 0].double()[:, None] * part).sum(0)
+                ref_dw[rows, 0, 0, 0] += (part * dy[0, oh, :, 0].double()).sum(1)
+    assert torch.equal(y.double(), ref) and torch.equal(dw.double(), ref_dw)
+
+
 # ---------------------------------------------------------------- embedding gradient
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab,dim,n,hot", [
