@@ -1531,7 +1531,9 @@ __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict_
   const int tid = threadIdx.x;
   const long long positions = (long long)g.N * g.OH * g.OW;
   const long long m0 = (long long)blockIdx.x * MT;
-  const int f0 = blockIdx.y * FT;
+  // channel tile; a grid holds 65535 in y, more go on in z
+  if ((blockIdx.z * 65535ll + blockIdx.y) * FT >= g.F) return;
+  const int f0 = (blockIdx.z * 65535 + blockIdx.y) * FT;
   const int K = g.R * g.S * g.C;
   // the positions whose input this thread stages
   int ih0[PER], iw0[PER];
@@ -2262,7 +2264,11 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
   const ConvGeom g{N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl};
   // the narrowest channel tile that holds F, so that lanes of absent channels are few
   const bool vec = C % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & (dtype ? 7 : 15)) == 0;
-#define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<dim3((unsigned)((positions + 256 / FG - 1) / (256 / FG)), (F + 4 * FG - 1) / (4 * FG)), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g)
+  const auto grid = [&](int fg) {
+    const unsigned tiles = (unsigned)((F + 4ll * fg - 1) / (4 * fg));
+    return dim3((unsigned)((positions + 256 / fg - 1) / (256 / fg)), tiles < 65535u ? tiles : 65535u, (tiles + 65534u) / 65535u);
+  };
+#define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<grid(FG), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g)
 #define CONV(T, FG) do { if (vec) CONV_V(T, FG, true); else CONV_V(T, FG, false); } while (0)
   if (dtype) { if (F <= 8) CONV(bf16, 2); else if (F <= 16) CONV(bf16, 4); else CONV(bf16, 8); }
   else { if (F <= 8) CONV(float, 2); else if (F <= 16) CONV(float, 4); else CONV(float, 8); }

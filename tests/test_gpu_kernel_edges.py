@@ -115,6 +115,16 @@ def test_direct_convolution_with_tall_and_wide_filters(H, W, R, S, pad):
     assert torch.equal(y.double(), ref) and torch.equal(dw.double(), ref_dw)
 
 
+@pytest.mark.parametrize("F", [32 * 65535, 32 * 65535 + 1, 3 * 32 * 65535 + 77])
+def test_direct_convolution_to_more_channel_tiles_than_a_grid_holds_in_y(F):
+    from nabla_b200.native import kernels
+
+    x = torch.tensor([2.0, 3.0], device="cuda").view(1, 1, 2, 1)
+    w = torch.randint(-3, 4, (1, 1, 1, F), device="cuda").float()
+    y = kernels.conv2d_direct(x, w, None, (1, 1), (0, 0, 0, 0))
+    assert torch.equal(y, x * w.view(F))
+
+
 # ---------------------------------------------------------------- embedding gradient
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab,dim,n,hot", [
