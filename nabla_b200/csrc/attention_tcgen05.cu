@@ -919,10 +919,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t lane_addr = static_cast<uint32_t>(wq * 32) << 16;
     const uint32_t a_s = t_st + lane_addr + grp * 64, a_dp = t_dpt + lane_addr + grp * 64;
     const float* mbase = !MASK ? nullptr : args.mask.ptr + b * args.mask.sb + h * args.mask.sh + key;
-    // a mask with one row for all queries is one number per key here: added in the exponent, no mask pass
+    // a mask with one row for all queries is one number per key here: added on the way into the exponent, no mask
+    // pass, with the forward's roundings ((s + mask / scale) * scale_log2 - lse: where all keys of a row share
+    // a large offset, any other order rounds the offset and the log-sum-exp apart)
     const bool mkey = MASK && args.mask.sq == 0;
-    const float mval = mkey && key_ok ? mbase[0] * LOG2E : 0.f;
-    const float2 mval2 = make_float2(mval, mval);
+    const float mval = mkey && key_ok ? mbase[0] : 0.f;
+    const float mask_mul = LOG2E / args.scale_log2;
+    const float2 mval2 = make_float2(mval, mval), mul2 = make_float2(mask_mul, mask_mul);
     if (mkey) mbase = nullptr;
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
@@ -938,7 +941,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const bool general = (args.causal && (k0 + BT - 1 > q0 + off)) || (k0 + BT > args.Skv) || (mbase != nullptr);
       if (general) {
         // masked tile: rewrite S^T in place with -inf where (key, query) is not visible
-        const float mask_mul = LOG2E / args.scale_log2;
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
           uint32_t v[32];
@@ -969,8 +971,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          float2 x = __ffma2_rn(f2(v[2 * i], v[2 * i + 1]), sc2, nl2[c * 16 + i]);
-          if (mkey) x = __fadd2_rn(x, mval2);
+          float2 x = f2(v[2 * i], v[2 * i + 1]);
+          if (mkey) x = __ffma2_rn(mval2, mul2, x);
+          x = __ffma2_rn(x, sc2, nl2[c * 16 + i]);
           p[c * 16 + i] = make_float2(ex2(x.x), ex2(x.y));
           pk[i] = pack_bf16(p[c * 16 + i].x, p[c * 16 + i].y);
         }
@@ -1224,20 +1227,23 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const float nlse2 = stat_ok ? args.nlse2[bh * args.Sq_pad + q_idx] : -INFINITY;
     const float ndelta = stat_ok ? args.ndelta[bh * args.Sq_pad + q_idx] : 0.f;
     // user mask: one row for all queries goes through shared memory (64 values per group and key tile) and is
-    // added in the exponent; a row per query is read by its own thread in the mask pass
+    // added on the way into the exponent, with the forward's roundings (see the dK / dV kernel); a row per query is
+    // read by its own thread in the mask pass
     const float* mrow = nullptr;
     const bool mkey = MASK && args.mask.sq == 0;
     const float* mkeys = mkey ? args.mask.ptr + b * args.mask.sb + h * args.mask.sh : nullptr;
     if (MASK && !mkey && q_idx < args.Sq)
       mrow = args.mask.ptr + b * args.mask.sb + h * args.mask.sh + (long long)q_idx * args.mask.sq;
     float* smask = reinterpret_cast<float*>(smem + L::OFF_MASK) + grp * 128;
+    const float mask_mul = LOG2E / args.scale_log2;
+    const float2 mul2 = make_float2(mask_mul, mask_mul);
     float mnext = mkey && r < 64 && grp * 64 + r < args.Skv ? mkeys[grp * 64 + r] : 0.f;
     const int lim = args.causal ? min(args.Skv - 1, q_idx + off) : args.Skv - 1;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
       const int kv0 = j * BT + grp * 64;
       if (mkey) {
-        if (r < 64) smask[(j & 1) * 64 + r] = mnext * LOG2E;
+        if (r < 64) smask[(j & 1) * 64 + r] = mnext;
         named_bar_sync(2 + grp, 128);
         mnext = j + 1 < n && r < 64 && kv0 + BT + r < args.Skv ? mkeys[kv0 + BT + r] : 0.f;
       }
@@ -1255,7 +1261,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t a_s = tmem_base + (j & 1) * BT + lane_addr + grp * 64;
       if (general) {
         // masked tile: rewrite the scores in place with -inf where the key is not visible
-        const float mask_mul = LOG2E / args.scale_log2;
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
           uint32_t v[32];
@@ -1283,8 +1288,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (c == 0) tmem_ld_32x32(a_s + 32, vb);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          float2 x = __ffma2_rn(f2(v[2 * i], v[2 * i + 1]), sc2, nl2);
-          if (mkey) x = __fadd2_rn(x, *reinterpret_cast<const float2*>(smask + (j & 1) * 64 + c * 32 + 2 * i));
+          float2 x = f2(v[2 * i], v[2 * i + 1]);
+          if (mkey) x = __ffma2_rn(*reinterpret_cast<const float2*>(smask + (j & 1) * 64 + c * 32 + 2 * i), mul2, x);
+          x = __ffma2_rn(x, sc2, nl2);
           p[c * 16 + i] = make_float2(ex2(x.x), ex2(x.y));
         }
       }

@@ -247,6 +247,26 @@ def test_attention_with_additive_masks(S, D, causal, shape):
     _attention_check(q, k, v, causal, mask.masked_fill(hide, float("-inf")))
 
 
+@pytest.mark.parametrize("S,D,causal", [(130, 64, False), (257, 128, False), (777, 64, True), (64, 128, False)])
+def test_attention_with_a_large_common_offset_in_the_mask(S, D, causal):
+    """One mask row for all queries gives what the same mask with a row per query gives, bit for bit: both add it
+    to the scores with one rounding. An offset that all keys share leaves the softmax as it is, but it is
+    rounded away from the scores in fp32 and any second rounding shows in the probabilities."""
+    from nabla_b200.native import attention
+
+    torch.manual_seed(12)
+    B, H = 2, 3
+    q, k, v, do = (torch.randn(B, H, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    for offset in (0.0, -1e4, 65504.0):
+        mask = torch.randn(B, 1, 1, S, device="cuda") + offset
+        got = []
+        for m in (mask, mask.expand(B, 1, S, S).contiguous()):
+            o, lse = attention.sdpa_fwd(q, k, v, causal=causal, scale=D ** -0.5, mask=m)
+            got.append((o, lse, *attention.sdpa_bwd(do, q, k, v, o, lse, causal=causal, scale=D ** -0.5, mask=m)))
+        for a, b in zip(*got):
+            assert torch.equal(a, b), offset
+
+
 def test_attention_rows_without_a_visible_key_are_zero():
     from nabla_b200.native import attention
 
