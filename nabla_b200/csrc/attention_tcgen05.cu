@@ -950,6 +950,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int i = 0; i < 32; ++i) {
             const int q = q0 + c * 32 + i;
             float x = __uint_as_float(v[i]);
+            if (mkey) x = fmaf(mval, mask_mul, x);
             if (mbase != nullptr && key_ok && q < args.Sq) x = fmaf(mbase[(long long)q * args.mask.sq], mask_mul, x);
             if (!key_ok || (args.causal && key > q + off)) x = -INFINITY;
             v[i] = __float_as_uint(x);
@@ -972,7 +973,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float2 x = f2(v[2 * i], v[2 * i + 1]);
-          if (mkey) x = __ffma2_rn(mval2, mul2, x);
+          if (mkey && !general) x = __ffma2_rn(mval2, mul2, x);      // else the mask pass has added it, under the -inf
           x = __ffma2_rn(x, sc2, nl2[c * 16 + i]);
           p[c * 16 + i] = make_float2(ex2(x.x), ex2(x.y));
           pk[i] = pack_bf16(p[c * 16 + i].x, p[c * 16 + i].y);
@@ -1270,6 +1271,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int i = 0; i < 32; ++i) {
             const int kc = kv0 + c * 32 + i;
             float x = __uint_as_float(v[i]);
+            if (mkey) x = fmaf(smask[(j & 1) * 64 + c * 32 + i], mask_mul, x);
             if (mrow != nullptr && kc < args.Skv) x = fmaf(mrow[kc], mask_mul, x);
             v[i] = __float_as_uint(kc <= lim ? x : -INFINITY);
           }
@@ -1289,7 +1291,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float2 x = f2(v[2 * i], v[2 * i + 1]);
-          if (mkey) x = __ffma2_rn(*reinterpret_cast<const float2*>(smask + (j & 1) * 64 + c * 32 + 2 * i), mul2, x);
+          if (mkey && !general) x = __ffma2_rn(*reinterpret_cast<const float2*>(smask + (j & 1) * 64 + c * 32 + 2 * i), mul2, x);
           x = __ffma2_rn(x, sc2, nl2);
           p[c * 16 + i] = make_float2(ex2(x.x), ex2(x.y));
         }

@@ -267,6 +267,26 @@ def test_attention_with_a_large_common_offset_in_the_mask(S, D, causal):
             assert torch.equal(a, b), offset
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("S,D", [(130, 64), (300, 128)])
+def test_attention_hides_a_masked_key_that_is_not_finite(S, D, value):
+    """Causal: rows before a key never see its mask value, whatever it is; with a row per query the same."""
+    from nabla_b200.native import attention
+
+    torch.manual_seed(13)
+    q, k, v, do = (torch.randn(1, 2, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    mask = torch.randn(1, 1, 1, S, device="cuda")
+    mask[..., S - 20] = value
+    got = []
+    for m in (mask, mask.expand(1, 1, S, S).contiguous()):
+        o, lse = attention.sdpa_fwd(q, k, v, causal=True, scale=D ** -0.5, mask=m)
+        dq, _, _ = attention.sdpa_bwd(do, q, k, v, o, lse, causal=True, scale=D ** -0.5, mask=m)
+        assert bool(torch.isfinite(o[:, :, :S - 20]).all()) and bool(torch.isfinite(dq[:, :, :S - 20]).all())
+        got.append((o, lse, dq))
+    for a, b in zip(*got):
+        assert torch.equal(a[:, :, :S - 20], b[:, :, :S - 20])
+
+
 def test_attention_rows_without_a_visible_key_are_zero():
     from nabla_b200.native import attention
 
