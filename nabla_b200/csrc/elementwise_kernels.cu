@@ -327,43 +327,58 @@ __global__ void __launch_bounds__(256) col_reduce_kernel(const T* __restrict__ x
 // The same for few rows and many columns (a sum over the batch: R = 8, inner = seq * dim): one thread per
 // 16-byte vector of columns walks the R rows, four loads in flight, no shared memory and no barrier. The
 // tile kernel above reads 2-byte elements there, and with R / 8 rows per warp spends its time at the
-// barriers. Bound by HBM; (8, 2048, 2048) bf16 over dim 0: 239 us with the tile kernel, 23 here.
-template <typename T, int OP>
-__global__ void __launch_bounds__(256) thin_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
+// barriers. Sums keep its eight chains (row r adds to chain r % 8, the chains are joined in order), so an
+// fp32 result is the same bit for bit; a single chain had 1.5 times its error at 32 rows and 2.4 times at 256.
+// (CH = 1: up to 8 rows, where one chain is the same additions, and the order-free maximum and minimum.)
+// Bound by HBM; (8, 2048, 2048) bf16 over dim 0: 241 us with the tile kernel, 21 here; (256, 40, 8192) fp32: 102 and 74.
+constexpr int THIN_THREADS = 128, THIN_CHAINS = 8;
+template <typename T, int OP, int CH>
+__global__ void __launch_bounds__(THIN_THREADS) thin_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
                                                          int R, long long inner) {
-  constexpr int V = Vec<T>::N;
-  const long long nv = inner / V, t = (long long)blockIdx.x * 256 + threadIdx.x;
+  constexpr int V = Vec<T>::N, U = 4, STEP = CH > U ? CH : U;
+  const long long nv = inner / V, t = (long long)blockIdx.x * THIN_THREADS + threadIdx.x;
   if (t >= outer * nv) return;
   const long long o = t / nv, i = (t - o * nv) * V;
   const T* p = x + o * R * inner + i;
   if (!NB_IN_BOUNDS(NB_SITE_REDUCE_INDEX, (o * R + (R - 1)) * inner + i + V - 1, outer * R * inner)) return;
-  float acc[V];
+  float acc[CH][V];
 #pragma unroll
-  for (int j = 0; j < V; ++j) acc[j] = OP == R_MAX ? -INFINITY : OP == R_MIN ? INFINITY : 0.f;
-  auto take = [&](const uint4& raw) {
+  for (int k = 0; k < CH; ++k)
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[k][j] = OP == R_MAX ? -INFINITY : OP == R_MIN ? INFINITY : 0.f;
+  auto take = [&](const uint4& raw, float (&a)[V]) {
     float f[V];
     unpack<T>(raw, f);
 #pragma unroll
     for (int j = 0; j < V; ++j) {
-      if (OP == R_MAX) acc[j] = (f[j] > acc[j] || f[j] != f[j]) ? f[j] : acc[j];      // NaN wins, and stays
-      else if (OP == R_MIN) acc[j] = (f[j] < acc[j] || f[j] != f[j]) ? f[j] : acc[j];
-      else acc[j] += f[j];
+      if (OP == R_MAX) a[j] = (f[j] > a[j] || f[j] != f[j]) ? f[j] : a[j];      // NaN wins, and stays
+      else if (OP == R_MIN) a[j] = (f[j] < a[j] || f[j] != f[j]) ? f[j] : a[j];
+      else a[j] += f[j];
     }
   };
   int r = 0;
-  for (; r + 4 <= R; r += 4) {
-    uint4 raw[4];
+  for (; r + STEP <= R; r += STEP) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) raw[u] = *reinterpret_cast<const uint4*>(p + (long long)(r + u) * inner);
+    for (int g = 0; g < STEP; g += U) {
+      uint4 raw[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) take(raw[u]);
+      for (int u = 0; u < U; ++u) raw[u] = *reinterpret_cast<const uint4*>(p + (long long)(r + g + u) * inner);
+#pragma unroll
+      for (int u = 0; u < U; ++u) take(raw[u], acc[(g + u) % CH]);
+    }
   }
-  for (; r < R; ++r) take(*reinterpret_cast<const uint4*>(p + (long long)r * inner));
+#pragma unroll
+  for (int u = 0; u < STEP - 1; ++u)
+    if (r + u < R) take(*reinterpret_cast<const uint4*>(p + (long long)(r + u) * inner), acc[u % CH]);
+#pragma unroll
+  for (int k = 1; k < CH; ++k)
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[0][j] += acc[k][j];
   if (OP == R_MEAN) {
 #pragma unroll
-    for (int j = 0; j < V; ++j) acc[j] /= (float)R;
+    for (int j = 0; j < V; ++j) acc[0][j] /= (float)R;
   }
-  *reinterpret_cast<uint4*>(out + o * inner + i) = pack<T>(acc);
+  *reinterpret_cast<uint4*>(out + o * inner + i) = pack<T>(acc[0]);
 }
 
 template <typename T, typename O>
@@ -456,7 +471,8 @@ int nb_reduce_splits(long long outer, long long R, long long inner) {
 // thin_reduce_kernel: value reductions over at most 256 rows (a longer sum keeps the tile kernel's parallel
 // partial sums) with enough column vectors for a block on every SM.
 static bool thin_reduce(long long outer, long long R, long long inner, int V) {
-  return R <= 256 && inner % V == 0 && outer * (inner / V) >= 148 * 256 && (outer * (inner / V) + 255) / 256 <= 0x7fffffffll;
+  const long long threads = outer * (inner / V);
+  return R <= 256 && inner % V == 0 && threads >= 148 * 256 && (threads + THIN_THREADS - 1) / THIN_THREADS <= 0x7fffffffll;
 }
 
 int nb_reduce(const void* x, void* out, void* scratch, long long outer, long long R, long long inner, int op, int dtype,
@@ -477,12 +493,14 @@ int nb_reduce(const void* x, void* out, void* scratch, long long outer, long lon
   }
   const int V = dtype ? 8 : 4;
   if (!arg && thin_reduce(outer, R, inner, V) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-    const unsigned grid_t = (unsigned)((outer * (inner / V) + 255) / 256);
-#define NB_THIN(T, OP) thin_reduce_kernel<T, OP><<<grid_t, 256, 0, STREAM>>>((const T*)x, (T*)out, outer, (int)R, inner)
-#define NB_THIN_T(T) do { if (op == R_SUM) NB_THIN(T, R_SUM); else if (op == R_MAX) NB_THIN(T, R_MAX); \
-                          else if (op == R_MIN) NB_THIN(T, R_MIN); else NB_THIN(T, R_MEAN); } while (0)
+    const unsigned grid_t = (unsigned)((outer * (inner / V) + THIN_THREADS - 1) / THIN_THREADS);
+#define NB_THIN(T, OP, CH) thin_reduce_kernel<T, OP, CH><<<grid_t, THIN_THREADS, 0, STREAM>>>((const T*)x, (T*)out, outer, (int)R, inner)
+#define NB_THIN_S(T, OP) do { if (R <= THIN_CHAINS) NB_THIN(T, OP, 1); else NB_THIN(T, OP, THIN_CHAINS); } while (0)
+#define NB_THIN_T(T) do { if (op == R_SUM) NB_THIN_S(T, R_SUM); else if (op == R_MAX) NB_THIN(T, R_MAX, 1); \
+                          else if (op == R_MIN) NB_THIN(T, R_MIN, 1); else NB_THIN_S(T, R_MEAN); } while (0)
     if (dtype) NB_THIN_T(bf16); else NB_THIN_T(float);
 #undef NB_THIN_T
+#undef NB_THIN_S
 #undef NB_THIN
     return CHECK_LAUNCH();
   }

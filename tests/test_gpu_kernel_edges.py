@@ -185,6 +185,27 @@ def test_reductions_over_leading_axes(dtype, shape, axis):
         torch.testing.assert_close(kernels.reduce(x, axis, op), fn(x, axis), rtol=0, atol=0, equal_nan=True)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape,axis", [((1, 40, 8192), 0), ((7, 40, 8192), 0), ((8, 40, 8192), 0), ((33, 40, 8192), 0), ((256, 40, 8192), 0),
+                                        ((5000, 21, 64), 1)])
+def test_sums_over_few_rows_in_eight_chains(dtype, shape, axis):
+    """Row r adds to chain r % 8 and the chains are joined in order, as in the kernel for longer sums: the
+    same fp32 additions one by one."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(14)
+    x = torch.randn(shape, device="cuda").to(dtype)
+    rows = x.movedim(axis, 0).float()
+    chains = torch.zeros(8, *rows.shape[1:], device="cuda")
+    for r, row in enumerate(rows):
+        chains[r % 8] += row
+    ref = chains[0]
+    for c in chains[1:]:
+        ref = ref + c
+    assert torch.equal(kernels.reduce(x, axis, "sum"), ref.to(dtype))
+    assert torch.equal(kernels.reduce(x, axis, "mean"), (ref / torch.full_like(ref, rows.shape[0])).to(dtype))
+
+
 @pytest.mark.parametrize("axes", [(0, 1), (0, 1, 2), (1, 2), (0, 2), (0, 1, 2, 3)])
 def test_sums_over_neighbouring_axes(axes):
     import nabla_b200 as nb
