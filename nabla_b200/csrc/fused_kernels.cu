@@ -530,26 +530,40 @@ __global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __re
   if (lane == 0 && blockIdx.x * 32 + w < D && out) out[blockIdx.x * 32 + w] = from_f<T>(a);
 }
 
-// out[i] = sum_z part[z][i], fp32 slices of n: 32 results per block, its 8 warps take every 8th slice.
-template <typename T>
-__global__ void __launch_bounds__(256) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
-                                                         int slices) {
-  __shared__ float sh[8][32];
+// Sum of eight numbers in pairs: three roundings deep.
+__device__ __forceinline__ float sum8(const float (&a)[8]) { return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])); }
+
+// out[i] = sum_z part[z][i], fp32 slices of n: 32 results per block, its WARPS warps take every WARPS-th slice and meet
+// in a tree. 32 warps from 64 slices on, so that no chain of additions is long: several hundred slices added by 8
+// warps rounded more than the blocks that made them.
+template <typename T, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
+                                                                int slices) {
+  __shared__ float sh[WARPS][33];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  const size_t i = (size_t)blockIdx.x * 32 + lane;
+  const size_t i0 = (size_t)blockIdx.x * 32, i = i0 + lane;
   float s = 0.f;
   if (i < n) {
 #pragma unroll 8
-    for (int z = wq; z < slices; z += 8) s += part[(size_t)z * n + i];
+    for (int z = wq; z < slices; z += WARPS) s += part[(size_t)z * n + i];
   }
   sh[wq][lane] = s;
   __syncthreads();
-  if (wq == 0 && i < n) {
-    s = 0.f;
+  if constexpr (WARPS == 32) {                       // warp w: result w of the block's 32
+    s = warp_sum(sh[lane][wq]);
+    if (lane == 0 && i0 + wq < n) out[i0 + wq] = from_f<T>(s);
+  } else if (wq == 0 && i < n) {
+    float a[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) s += sh[q][lane];
-    out[i] = from_f<T>(s);
+    for (int q = 0; q < 8; ++q) a[q] = sh[q][lane];
+    out[i] = from_f<T>(sum8(a));
   }
+}
+template <typename T>
+static void fold_slices(const float* part, void* out, size_t n, int slices, cudaStream_t stream) {
+  const unsigned grid = (unsigned)((n + 31) / 32);
+  if (slices < 64) fold_slices_kernel<T, 8><<<grid, 256, 0, stream>>>(part, (T*)out, n, slices);
+  else fold_slices_kernel<T, 32><<<grid, 1024, 0, stream>>>(part, (T*)out, n, slices);
 }
 
 // ============================================================== column sum (bias gradient)
@@ -578,16 +592,16 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
   for (int j = 0; j < V; ++j) sh[warp][lane * V + j] = acc[j];
   __syncthreads();
   for (int i = threadIdx.x; i < 32 * V; i += blockDim.x) {
-    float s = 0.f;
+    float a[8];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s += sh[w][i];
+    for (int w = 0; w < 8; ++w) a[w] = sh[w][i];
     const int col = blockIdx.x * 32 * V + i;
-    if (col < N) partial[(size_t)blockIdx.y * N + col] = s;
+    if (col < N) partial[(size_t)blockIdx.y * N + col] = sum8(a);
   }
 }
 // Column sums of a tall, narrow matrix (the bias gradient of a convolution: 200704 x 16): the block's 256
 // threads cover 256 / (N / V) whole rows at a time, so every lane loads whatever N is; colsum_kernel gives a
-// warp one row's 32 vectors and leaves 28 of 32 lanes without one there. 200704 x 16 fp32: 81 -> 17 us.
+// warp one row's 32 vectors and leaves 28 of 32 lanes without one there. 200704 x 16 fp32: 81 -> 15 us.
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
                                                            int N, int rows_per_block) {
@@ -611,9 +625,16 @@ __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict_
   for (int j = 0; j < V; ++j) sh[threadIdx.x * V + j] = acc[j];
   __syncthreads();
   for (int i = threadIdx.x; i < N; i += 256) {        // element i of row slot k sits at k * N + i
+    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int k = 0;
+    for (; k + 8 <= rpp; k += 8) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a[u] += sh[(k + u) * N + i];
+    }
     float s = 0.f;
-    for (int k = 0; k < rpp; ++k) s += sh[k * N + i];
-    partial[(size_t)blockIdx.x * N + i] = s;
+    for (; k < rpp; ++k) s += sh[k * N + i];
+    a[0] += s;
+    partial[(size_t)blockIdx.x * N + i] = sum8(a);
   }
 }
 
@@ -1953,8 +1974,8 @@ int nb_colsum(const void* x, void* out, float* partial, int rows, int N, int in_
     if (in_dtype) colsum_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
     else colsum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
   }
-  if (out_dtype) fold_slices_kernel<bf16><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (bf16*)out, (size_t)N, np);
-  else fold_slices_kernel<float><<<(N + 31) / 32, 256, 0, STREAM>>>(partial, (float*)out, (size_t)N, np);
+  if (out_dtype) fold_slices<bf16>(partial, out, (size_t)N, np, STREAM);
+  else fold_slices<float>(partial, out, (size_t)N, np, STREAM);
   return CHECK_LAUNCH();
 }
 
@@ -2313,7 +2334,7 @@ int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part,
     if (K <= 16) { if (F <= 16) WGRAD(T, 4, 4); else WGRAD(T, 4, 8); }                        \
     else if (K <= 32) { if (F <= 16) WGRAD(T, 8, 4); else WGRAD(T, 8, 8); }                   \
     else { if (F <= 16) WGRAD(T, 16, 4); else WGRAD(T, 16, 8); }                              \
-    fold_slices_kernel<T><<<(unsigned)((n + 31) / 32), 256, 0, STREAM>>>(part, (T*)dw, n, z); \
+    fold_slices<T>(part, dw, n, z, STREAM);                                                   \
   } while (0)
   if (dtype) WGRAD_T(bf16);
   else WGRAD_T(float);

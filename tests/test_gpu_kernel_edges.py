@@ -507,6 +507,47 @@ def test_column_sums_around_the_slab_counts():
             assert _rel2(kernels.colsum(x), x.double().sum(0)) < STORED[dtype]
 
 
+@pytest.mark.parametrize("rows,N", [(4096, 8), (4099, 124), (12544, 48), (50176, 32), (200704, 16), (700001, 120)])
+def test_narrow_column_sums_are_short_chains(rows, N):
+    """The additions one by one: a slab's rows to the slots of a block, the slots in eight sums and in pairs, the slabs to
+    8 or 32 warps and in a tree. No chain is longer than a slot's rows or rpp / 8 or 18."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(16)
+    x = torch.randn(rows, N, device="cuda")
+
+    def chain(t):                                     # one after the other over dim 0
+        acc = torch.zeros(t.shape[1:], device="cuda")
+        for row in t:
+            acc = acc + row
+        return acc
+
+    def slots(t, n):                                  # (k, ...) -> (steps, n, ...), zeros behind the last
+        pad = torch.zeros(-t.shape[0] % n, *t.shape[1:], device="cuda")
+        return torch.cat([t, pad]).view(-1, n, *t.shape[1:])
+
+    def sum8(a):
+        return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]))
+
+    parts = kernels._L().nb_colsum_nparts(rows, N, 0)
+    per, rpp = -(-rows // parts), 256 // (N // 4)
+    slabs = []
+    for b in range(parts):
+        a = chain(slots(x[b * per:(b + 1) * per], rpp))
+        eight = chain(a[:rpp // 8 * 8].view(-1, 8, N)) if rpp >= 8 else torch.zeros(8, N, device="cuda")
+        eight[0] = eight[0] + chain(a[rpp // 8 * 8:]) if rpp % 8 else eight[0] + 0.0
+        slabs.append(sum8(eight))
+    slabs = torch.stack(slabs)
+    if parts < 64:
+        ref = sum8(chain(slots(slabs, 8)))
+    else:
+        ref = chain(slots(slabs, 32))
+        for o in (16, 8, 4, 2, 1):
+            ref = ref + ref[torch.arange(32, device="cuda") ^ o]
+        ref = ref[0]
+    assert torch.equal(kernels.colsum(x), ref)
+
+
 # ---------------------------------------------------------------- pooling
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("mode", ["max", "avg"])
