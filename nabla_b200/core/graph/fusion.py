@@ -27,6 +27,7 @@ intermediates that are still referenced are simply not fusable.
 """
 from __future__ import annotations
 
+import math
 import os
 
 import torch
@@ -105,10 +106,13 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
         if chain is None and n.op.name == "reduce_sum" and _is_plain_sum(n) \
                 and n.kwargs["axis"] < len(n.input_impls()[0]._shape) - 1:
             # sums over neighbouring axes, one after the other (``sum(axis=(0, 1, 2))``): one reduction over
-            # the joined axes, without the partial results and their rounding. Not where the last axis is
-            # among them: one long row would be left to one warp
+            # as many joined axes as the kernels' rule takes, without the partial results and their rounding.
+            # Not where the last axis is among them: one long row would be left to one warp
+            from ...native import kernels
+
             idxs, lo, hi = [i], n.kwargs["axis"], n.kwargs["axis"]
-            last_axis = len(n.input_impls()[0]._shape) - 1
+            x0 = n.input_impls()[0]
+            last_axis, joined = len(x0._shape) - 1, 1
             while True:
                 o = sole_output(nodes[idxs[-1]])
                 if not fusable_intermediate(o):
@@ -123,8 +127,11 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
                 else:
                     lo -= 1
                 idxs.append(j)
-            if len(idxs) > 1:
-                chain = idxs
+                if kernels.joined_sum(math.prod(x0._shape[:lo]), math.prod(x0._shape[lo:hi + 1]), math.prod(x0._shape[hi + 1:]),
+                                      x0.dtype.to_torch()):
+                    joined = len(idxs)
+            if joined > 1:
+                chain = idxs[:joined]
                 kind = "sum_axes"
         if chain is None and n.op.name == "matmul" and _is_local_gemm(n):
             dk = _dact_consumer(n, nodes, cons, target_ids, used)

@@ -575,6 +575,31 @@ def _outer_r_inner(x: torch.Tensor, axis: int):
     return outer, int(x.shape[axis]), inner
 
 
+def joined_sum(outer: int, rows: int, inner: int, dtype: torch.dtype) -> bool:
+    """Whether one sum over ``rows`` = several neighbouring axes serves better than one sum per axis.
+
+    Column sums of a tall narrow matrix (a convolution's bias gradient) always do: their chains of additions are
+    short and they fill the chip (256 x 28 x 28 x 16 fp32 over its leading axes: 45 us as three sums, 13 as one).
+    Otherwise fp32 stays with one sum per axis: each has R / 8 rows in a chain, one over all axes has the
+    product (64 x 64 x 32768: 1.1e-7 from 64 bits as two sums, 4.1e-7 as one, 198 and 188 us), while bf16 loses a rounding
+    of its partial results to 16 bits by joining, and joins where the one kernel has two blocks per SM or the
+    tensor is small: 100 x 30 x 8192 81 -> 36 us, but 1000 x 1000 x 256, where 64 slabs of 2 column tiles are 128 blocks,
+    243 as two sums and 566 as one, 1.4 M x 8 in two outer parts 56 and 196."""
+    v = 8 if dtype == torch.bfloat16 else 4
+    column_sums = outer == 1 and rows > 4096 and inner % v == 0 and inner <= 4096 * (v // 4)      # as in reduce()
+    if column_sums and inner // v < 32:
+        return True
+    if dtype != torch.bfloat16:
+        return False
+    if outer * rows * inner <= 1 << 20 or (rows <= 256 and inner % v == 0 and outer * (inner // v) >= 148 * 256):
+        return True
+    if column_sums:
+        blocks = -(-inner // (32 * v)) * _L().nb_colsum_nparts(rows, inner, 1)
+    else:
+        blocks = outer * -(-inner // 32) * _L().nb_reduce_splits(outer, rows, inner)
+    return blocks >= 2 * 148
+
+
 def reduce(x: torch.Tensor, axis: int, op: str, keepdims: bool = False):
     """sum / max / min / mean / argmax / argmin over one axis in one kernel (fp32 / bf16 CUDA, non-empty
     axis); None otherwise."""

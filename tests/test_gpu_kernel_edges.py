@@ -207,18 +207,50 @@ def test_sums_over_few_rows_in_eight_chains(dtype, shape, axis):
 
 
 @pytest.mark.parametrize("axes", [(0, 1), (0, 1, 2), (1, 2), (0, 2), (0, 1, 2, 3)])
-def test_sums_over_neighbouring_axes(axes):
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_sums_over_neighbouring_axes(axes, dtype):
     import nabla_b200 as nb
 
-    x = torch.randn(6, 7, 50, 16, device="cuda")
+    x = torch.randn(6, 7, 50, 16, device="cuda").to(dtype)
     t = nb.Tensor.from_torch(x)
     for keep in (False, True):
         got = nb.reduce_sum(t, axis=axes, keepdims=keep).to_torch()
         ref = x.double().sum(axes, keepdim=keep)
-        assert got.shape == ref.shape and _rel2(got, ref) < STORED[torch.float32]
+        assert got.shape == ref.shape and _rel2(got, ref) < len(axes) * STORED[dtype]
     f = nb.compile(lambda a: nb.reduce_sum(a, axis=axes))
     f(t)
-    assert ("sum_axes" in f.dump_plan()) == (axes in ((0, 1), (0, 1, 2), (1, 2)))
+    assert _rel2(f(t).to_torch(), x.double().sum(axes)) < len(axes) * STORED[dtype]
+    assert ("sum_axes" in f.dump_plan()) == (dtype is torch.bfloat16 and axes in ((0, 1), (0, 1, 2), (1, 2)))
+
+
+@pytest.mark.parametrize("shape,axes,joined", [((20, 15, 14, 32), (0, 1, 2), True), ((16, 16, 4096), (0, 1), False), ((4, 60, 50, 24), (1, 2), False),
+                                               ((64, 65, 128), (0, 1), False), ((2, 64, 65, 16), (0, 1, 2), True)])
+def test_joined_sums_round_no_more_than_one_sum_per_axis(shape, axes, joined):
+    """fp32: one reduction takes over only where its chains of additions are short (see ``kernels.joined_sum``)."""
+    import nabla_b200 as nb
+    from nabla_b200.native import kernels
+
+    f = nb.compile(lambda a: nb.reduce_sum(a, axis=axes))
+    one = each = 0.0
+    for seed in range(8):                             # 8 draws: the error of a sum of few results scatters
+        torch.manual_seed(seed)
+        x = torch.randn(shape, device="cuda")
+        f(nb.Tensor.from_torch(x))
+        got, ref = f(nb.Tensor.from_torch(x)).to_torch(), x.double().sum(axes)
+        y = x
+        for axis in reversed(axes):
+            y = kernels.reduce(y, axis, "sum")
+        one, each = one + _rel2(got, ref) ** 2, each + _rel2(y, ref) ** 2
+    assert one <= 1.1 ** 2 * each
+    assert ("sum_axes" in f.dump_plan()) == joined
+
+
+@pytest.mark.parametrize("args,joined", [((1, 200704, 16, torch.float32), True), ((1, 4096, 16, torch.float32), False), ((1, 1 << 20, 256, torch.bfloat16), False),
+                                         ((2, 700000, 8, torch.bfloat16), False), ((1, 16384, 2048, torch.bfloat16), True), ((1, 16, 1 << 20, torch.bfloat16), True)])
+def test_rule_of_joined_sums(args, joined):
+    from nabla_b200.native import kernels
+
+    assert kernels.joined_sum(*args) == joined
 
 
 # ---------------------------------------------------------------- attention
