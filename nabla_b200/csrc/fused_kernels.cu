@@ -1333,7 +1333,12 @@ __global__ void __launch_bounds__(256) pool2d_fwd_kernel(const T* __restrict__ x
 // window's elements are read once. Backward: so are x and dy, and the cell's dx is written whole, zeros where
 // no window reaches (the gather form below finds every window's arg-max again for each of its pixels, with
 // six 64-bit divisions per element). Same values, first arg-max included. 2 x 2 over 256 x 28 x 28 x 16 fp32:
-// forward 10 -> 3.6 us, backward 52 -> 5.4 us.
+// forward 10 -> 3.6 us, backward 52 -> 5.4 us. A thread walks its cell alone, so large cells leave few threads.
+// Forward and max backward are faster all the same (the gather forms walk the window too, the latter once per
+// pixel: 8 x 56 x 56 x 64 in one window fp32 1.25 -> 0.45 ms and 6.2 -> 0.94 ms), but average backward has only one
+// load per pixel to do there and keeps the gather form where cells of more than 9 pixels times channels are below
+// 8192: that image 20 us by pixels, 108 by cells (512 cells); 1 x 256 x 256 x 16 in 16 x 16 18 and 23 (4096); 64 x 14 x 14 x
+// 256 in one window each 35 and 19 (16384).
 struct CellGeom {
   int H, W, CV, OH, OW, kh, kw, sh, sw, cells_h, cells_w;
 };
@@ -1397,12 +1402,15 @@ __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restric
       store_vec<T>(dx + at + a * down + (size_t)b * g.CV * V, o);
     }
 }
-// Whether the two kernels above take a problem.
+// Whether the two kernels above can take a problem.
 static inline bool pool_cells(const void* x, const void* y, const void* z, int N, int H, int W, int C, int OH, int OW, int kh, int kw,
                               int sh, int sw, int ph, int pw, int V, CellGeom& g) {
   g = CellGeom{H, W, C / V, OH, OW, kh, kw, sh, sw, (H + sh - 1) / sh, (W + sw - 1) / sw};
   return ph == 0 && pw == 0 && kh <= sh && kw <= sw && C % V == 0 && (long long)N * g.cells_h * g.cells_w * g.CV < 0x7fffff00ll &&
          ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z)) & 15) == 0;
+}
+static inline bool pool_cells_avg_bwd(int N, int C, const CellGeom& g) {
+  return (long long)(g.sh < g.H ? g.sh : g.H) * (g.sw < g.W ? g.sw : g.W) <= 9 || (long long)N * g.cells_h * g.cells_w * C >= 8192;
 }
 
 // out[window] = t[first arg-max of x over the window] (0 for a window that lies in the padding): the
@@ -2254,7 +2262,7 @@ int nb_pool2d_bwd(const void* x, const void* dy, void* dx, int N, int H, int W, 
   if (!total) return 0;
   const int V = dtype ? 8 : 4;
   CellGeom g;
-  if (pool_cells(x, dy, dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g)) {
+  if (pool_cells(x, dy, dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g) && (mode == 1 || pool_cells_avg_bwd(N, C, g))) {
     const unsigned n = (unsigned)((size_t)N * g.cells_h * g.cells_w * g.CV);
 #define POOL(T, MAX) pool2d_cell_bwd_kernel<T, MAX><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (const T*)dy, (T*)dx, g, n)
     if (dtype) { if (mode) POOL(bf16, true); else POOL(bf16, false); }

@@ -585,7 +585,9 @@ def test_narrow_column_sums_are_short_chains(rows, N):
 @pytest.mark.parametrize("mode", ["max", "avg"])
 @pytest.mark.parametrize("N,H,W,C,k,s,p", [(2, 8, 8, 16, (2, 2), (2, 2), 0), (1, 7, 9, 8, (2, 2), (2, 2), 0), (3, 5, 11, 24, (1, 2), (2, 3), 0), (2, 9, 9, 8, (3, 3), (3, 3), 0),
                                            (1, 2, 2, 8, (2, 2), (5, 4), 0), (2, 6, 6, 12, (2, 2), (2, 2), 0), (2, 6, 6, 5, (2, 2), (2, 2), 0),
-                                           (2, 8, 8, 8, (3, 3), (2, 2), 0), (2, 8, 8, 8, (2, 2), (2, 2), 1)])
+                                           (2, 8, 8, 8, (3, 3), (2, 2), 0), (2, 8, 8, 8, (2, 2), (2, 2), 1),
+                                           (2, 20, 20, 8, (20, 20), (20, 20), 0), (3, 11, 13, 16, (11, 13), (40, 50), 0), (64, 7, 7, 128, (7, 7), (7, 7), 0),
+                                           (16, 9, 14, 256, (4, 7), (4, 7), 0)])
 def test_pooling_cells(dtype, mode, N, H, W, C, k, s, p):
     """Windows that do not overlap (whole images and ragged edges, strides wider than the window) and the sizes
     beside the rule; ties go to the first maximum, a window of -inf routes nothing."""
@@ -604,6 +606,30 @@ def test_pooling_cells(dtype, mode, N, H, W, C, k, s, p):
         dy[0, 0, 0, 0] = 0.0                           # torch routes a window of -inf to its first element
     (g,) = torch.autograd.grad(ref, xr, dy.double().permute(0, 3, 1, 2))
     torch.testing.assert_close(kernels.pool2d_bwd(x, dy, *k, *s, p, p, mode).double(), g.permute(0, 2, 3, 1), rtol=2.0 ** -7, atol=1e-6)
+
+
+def test_average_pooling_over_few_large_windows_uses_a_thread_per_pixel():
+    """The gradient of global average pooling is one load and one store per pixel. Against the gradient of max
+    pooling over the same windows, which threads walk whole cells for, it takes a 19th by pixels and a 4th by cells
+    (20, 92 and 395 us); the line is between the two."""
+    from nabla_b200.native import kernels
+
+    x = torch.randn(8, 56, 56, 64, device="cuda")
+    dy = torch.randn(8, 1, 1, 64, device="cuda")
+
+    def fastest(mode):
+        times = []
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(200000)                  # both events and the launch are queued before the first runs
+            a.record()
+            kernels.pool2d_bwd(x, dy, 56, 56, 56, 56, 0, 0, mode)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert 9 * fastest("avg") < fastest("max")
 
 
 # ---------------------------------------------------------------- compiled calls
