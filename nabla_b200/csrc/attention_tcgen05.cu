@@ -88,12 +88,6 @@ __device__ __forceinline__ void tmem_ld_wait32(uint32_t (&v)[32]) {
 // the increase never waits.
 __device__ __forceinline__ void service_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 80;"); }
 __device__ __forceinline__ void math_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); }
-// One arrival per warp on a barrier that counts warps. Every lane has waited for its own TMEM stores.
-__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
-  tc_fence_before();
-  __syncwarp();
-  if (lane == 0) mbar_arrive(bar);
-}
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -175,27 +169,32 @@ struct FwdArgs {
   float* part_lse;              //             [nsplit][B][H][Sq] natural-log sum of exponentials of each range
 };
 
-template <int HD>
+template <int HD, bool KEYS>
 struct FwdSmem {
   static constexpr int TILE_BYTES = BT * HD * 2;
   static constexpr int OFF_Q = 0;                          // 2 query tiles
   static constexpr int OFF_K = OFF_Q + 2 * TILE_BYTES;     // 2 stages
   static constexpr int OFF_V = OFF_K + 2 * TILE_BYTES;     // 2 stages
-  static constexpr int OFF_MASK = OFF_V + 2 * TILE_BYTES;  // [2 math groups][2][128] mask values of a key tile
-  static constexpr int OFF_BAR = OFF_MASK + 4 * BT * 4;
+  static constexpr int OFF_MASK = OFF_V + 2 * TILE_BYTES;  // key mask: [2 math groups][2][128] values of a key tile. Not for
+  static constexpr int OFF_BAR = OFF_MASK + (KEYS ? 4 * BT * 4 : 0);   // the others: at 196 KB (head_dim 128) the 2 KB cost
+                                                           // half of the L1 that holds a row mask's lines
   static constexpr int RAW = OFF_BAR + 18 * 8 + 16 + 1024;
   static constexpr int TOTAL = RAW < 120 * 1024 ? 120 * 1024 : RAW;   // one CTA per SM (it takes all of TMEM)
 };
+static_assert(FwdSmem<128, false>::TOTAL + 1024 <= 196 * 1024, "with a row mask or none 60 KB of L1 are left");
 
-// MASK: a user mask is given. Its kernel reads a row's scores once and keeps them in registers for the mask, the
-// maximum and the exponentials; without a mask, reading them twice (maximum, exponentials), each load under the
-// work on the one before, measured 5 % faster at head_dim 128. 96 heads x 777 x 64 with a key mask: forward
-// 134 -> 84 us, backward 318 -> 199 us.
-template <int HD, bool MASK>
+// MASK_KEYS: a user mask with one row for all queries (padding). Its kernel reads a row's scores once and keeps them in
+// registers for the mask, the maximum and the exponentials; without a mask, reading them twice (maximum,
+// exponentials), each load under the work on the one before, measured 5 % faster at head_dim 128. 96 heads x 777 x
+// 64 with a key mask: forward 134 -> 84 us, backward 318 -> 199 us.
+// MASK_ROWS: a mask row per query, 128 loads per thread and key tile. They are added in the pass that hides keys, the
+// kernel otherwise that without a mask: with the scores in registers fewer of those loads are in flight
+// (96 x 777 x 64: 243 us that way, 212 this way; 16 heads x 300 x 128: 74 and 47, the L1 space included).
+template <int HD, UserMask MASK>
 __global__ void __launch_bounds__(NTHREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs args) {
-  using L = FwdSmem<HD>;
+  using L = FwdSmem<HD, MASK == MASK_KEYS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::OFF_Q;
@@ -208,7 +207,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* v_full = bars + 6;     // [2]
   uint64_t* v_empty = bars + 8;    // [2]
   uint64_t* s_full = bars + 10;    // [2] per query tile: scores of the next key tile are in TMEM
-  uint64_t* p_full = bars + 12;    // [2] per query tile: probabilities are in TMEM (one arrival per math warp)
+  uint64_t* p_full = bars + 12;    // [2] per query tile: probabilities are in TMEM (128 arrivals)
   uint64_t* o_done = bars + 14;    // [2] per query tile: last PV product has retired
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
@@ -254,7 +253,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 4);
+      mbar_init(&p_full[i], 128);
       mbar_init(&o_done[i], 1);
     }
     fence_mbar_init();
@@ -271,7 +270,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   // tile t: scores (and P over their first 64 columns) at t * 128, output accumulator at 256 + t * HD
 
   if (warp < 4) {
-  if (MASK) service_registers();
+  if (MASK == MASK_KEYS) service_registers();
   if (warp == 0) {
     if (lane == 0 && n_max > 0) {
       for (int t = 0; t < 2; ++t) {
@@ -337,7 +336,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   }
   } else {
-    if (MASK) math_registers();
+    if (MASK == MASK_KEYS) math_registers();
     const int t = (warp - 4) >> 2;          // query tile of this math group
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
@@ -349,8 +348,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // user mask: one row for all queries (padding masks) goes through shared memory, 128 coalesced values
     // per key tile; a row per query is read by its own thread
     const float* mrow = nullptr;
-    const bool mshared = MASK && args.mask.sq == 0;
-    if (MASK && (mshared || q_idx < args.Sq))
+    constexpr bool mshared = MASK == MASK_KEYS;
+    if (mshared || (MASK == MASK_ROWS && q_idx < args.Sq))
       mrow = args.mask.ptr + b * args.mask.sb + h * args.mask.sh + (mshared ? 0ll : (long long)q_idx * args.mask.sq);
     float* smask = reinterpret_cast<float*>(smem + L::OFF_MASK) + t * 2 * BT;
     const float mask_mul = LOG2E / args.scale_log2;
@@ -377,10 +376,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       tc_fence_after();
       const bool edge = kv0 + BT > args.Skv || (args.causal && kv0 + BT - 1 > q0 + t * BT + off);
-      const int lim = (args.causal ? min(args.Skv - 1, q_idx + off) : args.Skv - 1) - kv0;
+      const int last = args.causal ? min(args.Skv - 1, q_idx + off) : args.Skv - 1;      // this row's last visible key
       float mxa[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      uint32_t v4[MASK ? 4 : 2][32];     // MASK: the row's 128 scores; else two chunks of 32, one of them in flight
-      if constexpr (MASK) {
+      uint32_t v4[mshared ? 4 : 2][32];  // key mask: the row's 128 scores; else two chunks of 32, one of them in flight
+      if constexpr (mshared) {
         auto& v = v4;
         // the load of the next 32 columns runs under the work on the current ones
         tmem_ld_32x32(t_s, v[0]);
@@ -388,38 +387,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int c = 0; c < 4; ++c) {
           tmem_ld_wait32(v[c]);
           if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, v[c + 1]);
-          if (mrow != nullptr) {
-            if (mshared) {
-              const float4* m4 = reinterpret_cast<const float4*>(smask + (j & 1) * BT + c * 32);
+          const float4* m4 = reinterpret_cast<const float4*>(smask + (j & 1) * BT + c * 32);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const float4 mv = m4[i];
-                uint32_t* w = &v[c][i * 4];
-                w[0] = __float_as_uint(fmaf(mv.x, mask_mul, __uint_as_float(w[0])));
-                w[1] = __float_as_uint(fmaf(mv.y, mask_mul, __uint_as_float(w[1])));
-                w[2] = __float_as_uint(fmaf(mv.z, mask_mul, __uint_as_float(w[2])));
-                w[3] = __float_as_uint(fmaf(mv.w, mask_mul, __uint_as_float(w[3])));
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (kv0 + c * 32 + i < args.Skv)
-                  v[c][i] = __float_as_uint(fmaf(mrow[kv0 + c * 32 + i], mask_mul, __uint_as_float(v[c][i])));
-            }
+          for (int i = 0; i < 8; ++i) {
+            const float4 mv = m4[i];
+            uint32_t* w = &v[c][i * 4];
+            w[0] = __float_as_uint(fmaf(mv.x, mask_mul, __uint_as_float(w[0])));
+            w[1] = __float_as_uint(fmaf(mv.y, mask_mul, __uint_as_float(w[1])));
+            w[2] = __float_as_uint(fmaf(mv.z, mask_mul, __uint_as_float(w[2])));
+            w[3] = __float_as_uint(fmaf(mv.w, mask_mul, __uint_as_float(w[3])));
           }
           if (edge) {
             // diagonal or tail tile: -inf where a key is not visible
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (c * 32 + i > lim) v[c][i] = __float_as_uint(-INFINITY);
+              if (c * 32 + i > last - kv0) v[c][i] = __float_as_uint(-INFINITY);
           }
 #pragma unroll
           for (int i = 0; i < 16; ++i) mxa[i & 3] = max3(mxa[i & 3], __uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1]));
         }
       } else {
         uint32_t (&va)[32] = v4[0], (&vb)[32] = v4[1];
-        if (edge) {
-          // diagonal or tail tile: rewrite the scores in place, -inf where a key is
+        if (edge || MASK == MASK_ROWS) {
+          // diagonal or tail tile, or a mask: rewrite the scores in place, -inf where a key is
           // not visible, so that the two passes below carry no mask logic
 #pragma unroll 1
           for (int c = 0; c < BT / 32; ++c) {
@@ -427,8 +417,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             tmem_ld_32x32(t_s + c * 32, v);
             tmem_ld_wait32(v);
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c * 32 + i > lim) v[i] = __float_as_uint(-INFINITY);
+            for (int i = 0; i < 32; ++i) {
+              const int kc = kv0 + c * 32 + i;
+              float x = __uint_as_float(v[i]);
+              if (MASK == MASK_ROWS && mrow != nullptr && kc < args.Skv) x = fmaf(mrow[kc], mask_mul, x);
+              v[i] = __float_as_uint(kc <= last ? x : -INFINITY);
+            }
             tmem_st_32x32(t_s + c * 32, v);
           }
           tmem_st_wait();
@@ -476,8 +470,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
       for (int c = 0; c < BT / 32; ++c) {
-        uint32_t (&v)[32] = v4[MASK ? c : c & 1];
-        if constexpr (!MASK) {
+        uint32_t (&v)[32] = v4[mshared ? c : c & 1];
+        if constexpr (!mshared) {
           tmem_ld_wait32(v);
           if (c + 1 < BT / 32) tmem_ld_32x32(t_s + (c + 1) * 32, v4[(c + 1) & 1]);
         }
@@ -494,7 +488,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const float sum = (acc[0].x + acc[0].y) + (acc[1].x + acc[1].y);
       l = l * alpha + sum;
       tmem_st_wait();
-      warp_arrive(&p_full[t], lane);
+      tc_fence_before();
+      mbar_arrive(&p_full[t]);
     }
     if (ok && n > 0) {
       if (!mbar_wait(&o_done[t], 0)) {
@@ -1476,10 +1471,10 @@ static int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-template <int HD, bool MASK>
+template <int HD, UserMask MASK>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdArgs& a,
                       cudaStream_t stream) {
-  using L = FwdSmem<HD>;
+  using L = FwdSmem<HD, MASK == MASK_KEYS>;
   static bool configured = false;
   if (!configured) {
     if (set_smem(attn_fwd_kernel<HD, MASK>, L::TOTAL)) return -2;
@@ -1588,8 +1583,9 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   if ((r = make_map4(&tq, q, B, H, Sq, D, q_sb, q_sh, q_ss))) return r;
   if ((r = make_map4(&tk, k, B, H, Skv, D, k_sb, k_sh, k_ss))) return r;
   if ((r = make_map4(&tv, v, B, H, Skv, D, v_sb, v_sh, v_ss))) return r;
-  if (mask != nullptr) return D == 128 ? launch_fwd<128, true>(tq, tk, tv, a, s) : launch_fwd<64, true>(tq, tk, tv, a, s);
-  return D == 128 ? launch_fwd<128, false>(tq, tk, tv, a, s) : launch_fwd<64, false>(tq, tk, tv, a, s);
+  if (mask == nullptr) return D == 128 ? launch_fwd<128, MASK_NONE>(tq, tk, tv, a, s) : launch_fwd<64, MASK_NONE>(tq, tk, tv, a, s);
+  if (m_sq == 0) return D == 128 ? launch_fwd<128, MASK_KEYS>(tq, tk, tv, a, s) : launch_fwd<64, MASK_KEYS>(tq, tk, tv, a, s);
+  return D == 128 ? launch_fwd<128, MASK_ROWS>(tq, tk, tv, a, s) : launch_fwd<64, MASK_ROWS>(tq, tk, tv, a, s);
 }
 
 // Backward. All tensors are (B, H, S, D) bf16 views with the head dim contiguous (element strides
