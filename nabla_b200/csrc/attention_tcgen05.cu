@@ -1507,32 +1507,52 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 
 }  // namespace nba
 
-// Few queries and no user mask: the decode kernel (gridDim.y holds the (batch, head) pairs).
-static bool attn_decode(int B, int H, int Sq, bool mask) { return Sq <= nba::DEC_MAX_Q && !mask && (long long)B * H <= 65535; }
+// Few queries and no user mask: the decode kernel (gridDim.y holds the (batch, head) pairs) or the tile kernel, by
+// what was faster over 4 .. 1024 pairs and 64 .. 16384 keys. The decode kernel's FMAs grow with the queries and head_dim,
+// where the tile kernel's time does not; it starts sooner (12 -> 8 us over 64 keys), and a tile kernel of more CTAs than
+// SMs takes a wave per 148 pairs.
+// head_dim 64: one and two queries (256 pairs x 1000 keys: 26 and 32 us, 41 with tiles); three and four up to one tile
+// of keys and from 256 pairs on (128 x 1000: 28 and 25 with tiles, 256 x 1000: 38 and 41).
+// head_dim 128: one query, but for up to a wave of pairs over short prefixes (64 x 300: 17.4 and 16.4; 128 x 1000: 27.7 and
+// 26.6; 64 x 1000: 21.5 and 23.6); two from 512 pairs on (256 x 4096: 142 and 129, 512 x 4096: 226 and 246); up to
+// four over 64 keys, or below 256 keys where the pairs are more than a wave. Four over 128 x 4096: 114 and 68.
+static bool attn_decode(int B, int H, int Sq, int Skv, int D, bool mask) {
+  const long long bh = (long long)B * H;
+  const bool one_wave = bh <= 148;
+  if (mask || Sq > nba::DEC_MAX_Q || bh > 65535) return false;
+  if (D == 64) return Sq <= 2 || Skv <= nba::BT || bh >= 256;
+  if (Skv <= 64 || (!one_wave && Skv < 256)) return true;
+  if (Sq == 1) return !one_wave || Skv > (bh > 64 ? 8 * bh : 512);
+  return Sq == 2 && bh >= 512;
+}
 
 // Key ranges that a forward pass is cut into (1: none).
-// Decode kernel: ranges of at least 128 keys, for four blocks per SM.
+// Decode kernel: ranges of at least 128 keys, for four blocks per SM; at head_dim 64 none below 512 keys, where a block walks
+// them before a second launch would have started (64 pairs x 300 keys: 12.3 us whole, 15.4 in two ranges; 16.4 and 15.4 at
+// head_dim 128).
 // Otherwise a CTA owns 256 queries of one (batch, head), so a short query block against a long prefix gives one
 // CTA per (batch, head), each walking all key tiles alone. The rule counts what the busiest SM walks: waves *
-// (key tiles per CTA + 3), the 3 standing for a CTA's start and end, and splits only where that falls below
-// 0.8 of the unsplit count (the partial results cost a second launch). With more than one block of 256 queries
-// it stays as it is: 64 such CTAs (2 x 8 heads x 1001 queries, causal) took 25.6 us, split and joined 27.6.
-extern "C" int nb_attn_fwd_splits(int B, int H, int Sq, int Skv, int has_mask) {
+// (key tiles per CTA + 3), the 3 standing for a CTA's start and end, and 3 more for the launch that joins the
+// ranges (a tile is 1.7 us at head_dim 128, the join 5): 500 keys 16.4 us whole and 17.4 in four ranges, 520 keys 18.4 and
+// 15.4, 4096 keys of 64 pairs 65 and 44. With more than one block of 256 queries it stays as it is (2 x 8 heads x 1001
+// queries, causal: 25.6 us, 27.6 in two ranges; few heads over long prefixes would gain, 8 heads x 512 queries x 8192 keys 129 -> 38).
+extern "C" int nb_attn_fwd_splits(int B, int H, int Sq, int Skv, int D, int has_mask) {
   constexpr int SMS = 148;
   if (B <= 0 || H <= 0 || Sq <= 0 || Skv <= 0) return 1;
-  if (attn_decode(B, H, Sq, has_mask != 0)) {
+  if (attn_decode(B, H, Sq, Skv, D, has_mask != 0)) {
+    if (D == 64 && Skv < 512) return 1;
     long long s = (4ll * SMS + (long long)B * H - 1) / ((long long)B * H);
     if (s > Skv / 128) s = Skv / 128;
     return (int)(s < 1 ? 1 : s > 64 ? 64 : s);
   }
   const long long ctas = (long long)B * H;
   const int n = (Skv + nba::BT - 1) / nba::BT;
-  if (Sq > 2 * nba::BT || ctas >= SMS || n < 4) return 1;
+  if (Sq > 2 * nba::BT || ctas >= SMS) return 1;
   int best = 1;
   long long best_cost = n + 3;
   for (int s = 2; s <= 32 && s <= n; ++s) {
-    const long long cost = ((ctas * s + SMS - 1) / SMS) * ((n + s - 1) / s + 3);
-    if (cost < best_cost && 10 * cost < 8 * (n + 3)) {
+    const long long cost = ((ctas * s + SMS - 1) / SMS) * ((n + s - 1) / s + 3) + 3;
+    if (cost < best_cost) {
       best = s;
       best_cost = cost;
     }
@@ -1574,7 +1594,7 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   a.bh_chunk = causal ? l2_chunk(B * H, Skv, D) * nsplit : 1;
   a.nsplit = nsplit; a.part_o = part_o; a.part_lse = part_lse;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (Skv > 0 && attn_decode(B, H, Sq, mask != nullptr)) {
+  if (Skv > 0 && attn_decode(B, H, Sq, Skv, D, mask != nullptr)) {
     const DecodeArgs d{a, reinterpret_cast<const __nv_bfloat16*>(q), reinterpret_cast<const __nv_bfloat16*>(k),
                        reinterpret_cast<const __nv_bfloat16*>(v), q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss};
     return D == 128 ? launch_decode<128>(d, s) : launch_decode<64>(d, s);

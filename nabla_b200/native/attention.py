@@ -32,7 +32,7 @@ def _lib():
             f.restype = c_int
             f.argtypes = [c_vp] * 5 + [c_int] * 5 + [c_ll] * 12 + [c_f, c_int, c_vp, c_ll, c_ll, c_ll, c_int, c_vp, c_vp, c_vp, c_vp]
             lib.nb_attn_fwd_splits.restype = c_int
-            lib.nb_attn_fwd_splits.argtypes = [c_int] * 5
+            lib.nb_attn_fwd_splits.argtypes = [c_int] * 6
             _splits = lib.nb_attn_fwd_splits
             _fwd = f
             if hasattr(lib, "nb_attn_bwd"):
@@ -110,7 +110,7 @@ def sdpa_fwd(q, k, v, *, causal: bool, scale: float, mask=None):
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
     st = status_word(q.device)
     m, m_sb, m_sh, m_sq = _mask_args(mask, B, H, Sq, Skv)
-    ns = _splits(B, H, Sq, Skv, int(m is not None))
+    ns = _splits(B, H, Sq, Skv, D, int(m is not None))
     # fp32 results of the key ranges: nsplit x (output, log-sum-exp)
     part = torch.empty(ns * B * H * Sq * (D + 1), dtype=torch.float32, device=q.device) if ns > 1 else None
     p_o = 0 if part is None else part.data_ptr()

@@ -692,6 +692,25 @@ def test_attention_of_few_queries_over_a_long_prefix(B, H, Sq, Skv, D):
         _attention_check(q, k, v, causal, grads=1 < Skv and Sq * Skv < 100000)    # (one key: the score gradients are 0)
 
 
+@pytest.mark.parametrize("B,H,Sq,Skv,D,decode,splits", [
+    (1, 16, 1, 4001, 128, True, 31), (4, 16, 1, 4001, 128, True, 10), (1, 64, 1, 500, 128, False, 1), (1, 64, 1, 513, 128, True, 4),
+    (1, 64, 1, 300, 64, True, 1), (1, 128, 3, 1000, 64, False, 1), (1, 256, 4, 1000, 64, True, 3), (8, 16, 4, 4096, 128, False, 1),
+    (2, 256, 2, 4096, 128, True, 2), (1, 256, 2, 4096, 128, False, 1), (1, 16, 4, 64, 128, True, 1), (1, 16, 5, 500, 64, False, 1),
+    (1, 16, 5, 520, 64, False, 5), (1, 64, 33, 4096, 64, False, 2), (1, 8, 300, 4000, 128, False, 1)])
+def test_kernel_and_key_ranges_of_few_queries(B, H, Sq, Skv, D, decode, splits):
+    """On both sides of the rules' lines: the number of ranges, and whether the call is the decode kernel (it keeps
+    the probabilities in fp32, the tile kernel rounds them to bf16: 1.65e-3 and 2.1e-3 or more from 64 bits)."""
+    from nabla_b200.native import attention
+
+    attention._lib()
+    assert attention._splits(B, H, Sq, Skv, D, 0) == splits
+    torch.manual_seed(17)
+    q = torch.randn(B, H, Sq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(B, H, Skv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    o, _ = attention.sdpa_fwd(q, k, v, causal=False, scale=D ** -0.5)
+    assert (_rel2(o, _attention64(q, k, v, False)) < 1.85e-3) == decode
+
+
 def test_attention_shows_a_nan_key_in_every_split():
     from nabla_b200.native import attention
 
