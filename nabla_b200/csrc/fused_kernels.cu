@@ -874,22 +874,23 @@ __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restri
 // launches over the integers), and every row that occurs is written once more, as the fp32 sum of its updates
 // in registers: no fp32 table that is zeroed, added to with atomics and converted. A row with more than SCAT_SEG
 // entries (frequent tokens: ids of text fall off about as 1 / rank) is cut into segments, one block each, whose
-// fp32 partial rows the last block of the row adds up; one block per row would leave the most frequent id,
-// some 1000 of 16384 tokens, to one block.
-// Bound by HBM (updates read once, `out` written once and its rows once more). 16384 ids into 32000 x 2048 bf16
-// with a base table: 257 us with the fp32 table, 114 now; 48 for the rows, 11 for the bucketing.
-constexpr int SCAT_SEG = 32;
+// fp32 partial rows are added up in two steps: the last block of every SCAT_GROUP segments adds those, the last
+// group of a row the groups. One block per row would leave the most frequent id, some 1000 of 16384 tokens, to one
+// block, and joining them in one step the padding id of a batch (29700 of 33000 ids into 4097 x 2048 fp32: 881 us
+// in one step, 128 in two).
+// Bound by latency in the rows (dependent loads of a segment, its list, its rows of updates; 1.4 TB/s) after an HBM-bound
+// fill of `out`. 16384 ids into 32000 x 2048 bf16 with a base table: 257 us with the fp32 table, 114 now; 48 for the
+// rows, 11 for the bucketing.
+constexpr int SCAT_SEG = 32, SCAT_GROUP = 32;
 struct ScatWs {
   int *counts, *done, *total, *nseg, *nheavy;   // zeroed by the launcher
+  int* gdone;                                   // likewise: finished segments of a group, at its first partial row
   int *start, *rank, *list;                     // first list slot per row; place of an entry in its row; entries by row
   int4* seg;                                    // (row, first list slot, entries, partial row or -1)
 };
-// Segments of one row: `c` entries from list slot `at` on, written from seg[sg] on.
-__device__ __forceinline__ void scatter_segments(const ScatWs& ws, int v, int c, int at, int sg) {
-  const int k = (c + SCAT_SEG - 1) / SCAT_SEG;
-  int h = -1;
-  if (k > 1) h = atomicAdd(ws.nheavy, k);
-  for (int q = 0; q < k; ++q) ws.seg[sg + q] = make_int4(v, at + q * SCAT_SEG, min(SCAT_SEG, c - q * SCAT_SEG), h < 0 ? -1 : h + q);
+// Segment q of a row of `c` entries from list slot `at` on; h: its first partial row, or -1.
+__device__ __forceinline__ int4 scatter_segment(int v, int c, int at, int h, int q) {
+  return make_int4(v, at + q * SCAT_SEG, min(SCAT_SEG, c - q * SCAT_SEG), h < 0 ? -1 : h + q);
 }
 // Lanes of a warp with the same id share one atomic; returns the entry's place among those of its row.
 __device__ __forceinline__ int scatter_rank(int* counts, long long id, bool ok) {
@@ -929,10 +930,15 @@ __global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __r
   const int rank = scatter_rank(ws.counts, id, ok);
   if (ok) ws.rank[i] = rank;
 }
-// List slots and segments of every row; the rows of a block come in order, the blocks in any.
+// List slots and segments of every row; the rows of a block come in order, the blocks in any. A row of many
+// segments is written by the whole block.
 __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int vocab) {
+  constexpr int FEW = 4;
+  struct Row { int v, c, at, sg, h; };
   __shared__ unsigned long long wsum[8];
-  __shared__ int base_at, base_sg;
+  __shared__ int base_at, base_sg, nmany;
+  __shared__ Row many[256];
+  if (threadIdx.x == 0) nmany = 0;                   // (the scan below has the barrier)
   const int v = blockIdx.x * 256 + threadIdx.x;
   const int c = v < vocab ? ws.counts[v] : 0;
   const unsigned long long t = (unsigned long long)((c + SCAT_SEG - 1) / SCAT_SEG) << 32 | (unsigned)c;
@@ -945,9 +951,19 @@ __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int vocab
   }
   __syncthreads();
   if (c) {
-    const int at = base_at + (int)(unsigned)at0;
+    const int at = base_at + (int)(unsigned)at0, sg = base_sg + (int)(at0 >> 32), k = (c + SCAT_SEG - 1) / SCAT_SEG;
     ws.start[v] = at;
-    scatter_segments(ws, v, c, at, base_sg + (int)(at0 >> 32));
+    const int h = k > 1 ? atomicAdd(ws.nheavy, k) : -1;
+    if (k <= FEW) {
+      for (int q = 0; q < k; ++q) ws.seg[sg + q] = scatter_segment(v, c, at, h, q);
+    } else {
+      many[atomicAdd(&nmany, 1)] = Row{v, c, at, sg, h};
+    }
+  }
+  __syncthreads();
+  for (int r = 0; r < nmany; ++r) {
+    const Row w = many[r];
+    for (int q = threadIdx.x; q < (w.c + SCAT_SEG - 1) / SCAT_SEG; q += 256) ws.seg[w.sg + q] = scatter_segment(w.v, w.c, w.at, w.h, q);
   }
 }
 __global__ void __launch_bounds__(256) scatter_place_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
@@ -1001,25 +1017,37 @@ __device__ __forceinline__ void scatter_write(const T* __restrict__ base, T* __r
   if (VN > 1) store_vec<T>(out + at, acc);
   else out[at] = from_f<T>(acc[0]);
 }
-// Adds up the `nseg` fp32 partial rows of row v from partial row h0 on.
-template <typename T, int VN>
-__device__ __forceinline__ void scatter_join(const T* __restrict__ base, T* __restrict__ out, const float* __restrict__ part,
-                                             int v, int h0, int nseg, int D) {
-  for (int c = threadIdx.x * VN; c < D; c += blockDim.x * VN) {
-    float acc[VN];
+// Columns [c, c + VN) of the sum of `n` fp32 partial rows, `step` rows apart, from p on.
+template <int VN>
+__device__ __forceinline__ void scatter_join(const float* p, int n, size_t step, int c, float (&acc)[VN]) {
 #pragma unroll
-    for (int j = 0; j < VN; ++j) acc[j] = 0.f;
-#pragma unroll 4
-    for (int q = 0; q < nseg; ++q)
+  for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+  constexpr int U = 8;                               // rows in flight
+  int q = 0;
+  if constexpr (VN > 1) {                            // rows are 16-byte aligned
+    for (; q + U <= n; q += U) {
+      float4 r[U][VN / 4];
 #pragma unroll
-      for (int j = 0; j < VN; ++j) acc[j] += __ldcg(part + (size_t)(h0 + q) * D + c + j);
-    scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < VN / 4; ++j) r[u][j] = __ldcg(reinterpret_cast<const float4*>(p + (q + u) * step + c) + j);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < VN / 4; ++j) {
+          acc[4 * j] += r[u][j].x; acc[4 * j + 1] += r[u][j].y; acc[4 * j + 2] += r[u][j].z; acc[4 * j + 3] += r[u][j].w;
+        }
+    }
   }
+#pragma unroll 8
+  for (; q < n; ++q)
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j] += __ldcg(p + q * step + c + j);
 }
 // The blocks walk the segments, the next descriptor on its way while one is worked on. VN: elements per access
 // (16 bytes, or 1 where rows are not 16-byte aligned).
 template <typename T, int VN>
-__global__ void __launch_bounds__(256) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
+__global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
                                                           T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
                                                           int D) {
   __shared__ int last;
@@ -1040,14 +1068,37 @@ __global__ void __launch_bounds__(256) scatter_rows_kernel(const T* __restrict__
       }
     }
     if (sg.w < 0) continue;
-    const int nseg = (ws.counts[v] + SCAT_SEG - 1) / SCAT_SEG, h0 = sg.w - (sg.y - ws.start[v]) / SCAT_SEG;
+    const int nseg = (ws.counts[v] + SCAT_SEG - 1) / SCAT_SEG, ngroups = (nseg + SCAT_GROUP - 1) / SCAT_GROUP;
+    const int q = (sg.y - ws.start[v]) / SCAT_SEG, h0 = sg.w - q, g0 = h0 + q / SCAT_GROUP * SCAT_GROUP;
+    const int gsize = min(SCAT_GROUP, h0 + nseg - g0);
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ws.done + v, 1) == nseg - 1;
+    if (threadIdx.x == 0) last = atomicAdd(ws.gdone + g0, 1) == gsize - 1;
     __syncthreads();
-    if (last) {
-      __threadfence();
-      scatter_join<T, VN>(base, out, part, v, h0, nseg, D);
+    if (!last) continue;                             // the same in every thread
+    __threadfence();
+    float* grow = part + (size_t)g0 * D;
+    for (int c = threadIdx.x * VN; c < D; c += blockDim.x * VN) {
+      float acc[VN];
+      scatter_join<VN>(grow, gsize, D, c, acc);
+      if (ngroups == 1) {
+        scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
+      } else {
+#pragma unroll
+        for (int j = 0; j < VN; ++j) grow[c + j] = acc[j];       // this thread alone reads and writes these columns
+      }
+    }
+    if (ngroups == 1) continue;
+    __threadfence();
+    __syncthreads();                                 // also: every thread has read `last`
+    if (threadIdx.x == 0) last = atomicAdd(ws.done + v, 1) == ngroups - 1;
+    __syncthreads();
+    if (!last) continue;
+    __threadfence();
+    for (int c = threadIdx.x * VN; c < D; c += blockDim.x * VN) {
+      float acc[VN];
+      scatter_join<VN>(part + (size_t)h0 * D, ngroups, (size_t)SCAT_GROUP * D, c, acc);
+      scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
     }
   }
 }
@@ -2054,20 +2105,27 @@ int nb_embedding_gather(const void* table, const long long* ids, void* out, int 
 // out = base + scatter_add(ids, upd); base null: zeros. `work`: nb_embedding_scatter_work(...) 32-bit words of
 // 16-byte aligned scratch.
 static long long scat_max_heavy(long long n_ids) { return 2 * (n_ids / SCAT_SEG); }   // segments of rows with > SCAT_SEG entries
-static long long scat_ints(long long n_ids, long long vocab) { return (3 * vocab + 3 + 2 * n_ids + 3) / 4 * 4; }
-// Atomics into an fp32 table while it stays in L2 and its rows are not crowded: the bucketing's launches
-// have no large table to win against there (5000 ids into 1000 x 256 fp32: 17 us with atomics, 42 bucketed; 4000
-// into 8192 x 768 bf16: 34 and 44), but 20000 ids into 50 x 2048 take 91 us with atomics and 82 bucketed.
-static bool scat_atomics(long long n_ids, long long D, long long vocab) { return vocab * D <= (8ll << 20) && n_ids <= 16 * vocab; }
-long long nb_embedding_scatter_work(int n_ids, int D, int vocab) {
-  if (scat_atomics(n_ids, D, vocab)) return (long long)vocab * D;
+static long long scat_ints(long long n_ids, long long vocab) { return (3 * vocab + 3 + scat_max_heavy(n_ids) + 2 * n_ids + 3) / 4 * 4; }
+// Atomics into an fp32 table, or bucketed ids, by times over tables of 2 .. 32000 rows of 8 .. 2048, 100 .. 100000 ids,
+// spread or crowded on one row. The bucketing is 25 to 35 us of short launches: it wins where the table is more than the
+// L2 keeps (32000 x 2048 bf16, 16384 ids: 263 us with atomics, 136), where much is added to few rows (1000 x
+// 2048, 16384 ids: 83 and 46, all on one row 189 and 58; 2 x 256, 100000 ids: 433 and 56), and for many ids, each of
+// which is a block of the atomics' grid (1000 x 64, 100000 ids: 64 and 46), not for small sums (16 x 8, 1000 ids: 11 and
+// 31; 100 x 256, 10000 ids: 19 and 39; 100 x 64, 100000 ids: 64 and 71). Rows that are not whole vectors are read by
+// elements, where it wins only with few ids in a large table (32000 x 1001: 1000 ids 110 and 62, 100000 ids 312 and 355).
+static bool scat_atomics(long long n_ids, long long D, long long vocab, int dtype) {
+  if (D % (dtype ? 8 : 4) != 0) return vocab * D <= (16ll << 20) || n_ids > vocab;
+  return vocab * D <= (8ll << 20) && n_ids * D <= (24ll << 20) && (n_ids <= 49152 || (vocab <= 256 && n_ids * D <= (8ll << 20)));
+}
+long long nb_embedding_scatter_work(int n_ids, int D, int vocab, int dtype) {
+  if (scat_atomics(n_ids, D, vocab, dtype)) return (long long)vocab * D;
   return scat_ints(n_ids, vocab) + 4ll * n_ids + scat_max_heavy(n_ids) * D;
 }
 int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, const void* base, void* out, int n_ids, int D,
                              int vocab, int dtype, void* stream) {
   if (vocab <= 0 || D <= 0) return 0;
   if (n_ids < 0) return -2;
-  if (n_ids > 0 && scat_atomics(n_ids, D, vocab)) {
+  if (n_ids > 0 && scat_atomics(n_ids, D, vocab, dtype)) {
     const size_t n = (size_t)vocab * D;
     const bool direct = !dtype && base == nullptr;   // the sum is the result
     float* acc = direct ? (float*)out : reinterpret_cast<float*>(work);
@@ -2093,13 +2151,14 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
   ws.total = ws.done + vocab;
   ws.nseg = ws.total + 1;
   ws.nheavy = ws.nseg + 1;
-  ws.start = ws.nheavy + 1;
+  ws.gdone = ws.nheavy + 1;
+  ws.start = ws.gdone + scat_max_heavy(n_ids);
   ws.rank = ws.start + vocab;
   ws.list = ws.rank + n_ids;
   ws.seg = reinterpret_cast<int4*>(work + scat_ints(n_ids, vocab));
   float* part = reinterpret_cast<float*>(ws.seg + n_ids);
   const int idb = (n_ids + 255) / 256;
-  if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 3) * sizeof(int), STREAM) != cudaSuccess) return -1;
+  if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 3 + scat_max_heavy(n_ids)) * sizeof(int), STREAM) != cudaSuccess) return -1;
   scatter_count_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
   scatter_slots_kernel<<<(vocab + 255) / 256, 256, 0, STREAM>>>(ws, vocab);
   scatter_place_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);

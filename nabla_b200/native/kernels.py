@@ -62,7 +62,7 @@ def _L():
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = c_int
-        lib.nb_embedding_scatter_work.argtypes = [c_int] * 3
+        lib.nb_embedding_scatter_work.argtypes = [c_int] * 4
         lib.nb_embedding_scatter_work.restype = c_ll
         lib.nb_layernorm_bwd_two_kernels.argtypes = [c_int]
         lib.nb_layernorm_bwd_two_kernels.restype = None
@@ -253,7 +253,7 @@ def embedding_scatter_add(base: torch.Tensor | None, ids: torch.Tensor, upd: tor
                                              _dt(base), stream_ptr()), "embedding_scatter_sorted")
         launch_count += 1
         return out
-    work = torch.empty(_L().nb_embedding_scatter_work(flat.numel(), D, V), dtype=torch.int32, device=u.device)
+    work = torch.empty(_L().nb_embedding_scatter_work(flat.numel(), D, V, _dt(u)), dtype=torch.int32, device=u.device)
     out = torch.empty((V, D), dtype=dtype, device=u.device)
     _ok(_L().nb_embedding_scatter_add(ptr(work), ptr(flat), ptr(u), ptr(base), ptr(out), flat.numel(), D, V, _dt(u),
                                       stream_ptr()), "embedding_scatter_add")

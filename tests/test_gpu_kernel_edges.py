@@ -130,10 +130,10 @@ def test_direct_convolution_to_more_channel_tiles_than_a_grid_holds_in_y(F):
 @pytest.mark.parametrize("vocab,dim,n,hot", [
     (1, 8, 1, 0.0), (50, 33, 700, 0.0), (100, 256, 33, 1.0), (300, 64, 4096, 0.3), (300, 64, 4801, 0.3), (300, 33, 4801, 0.3),
     (4096, 2048, 500, 0.1), (4097, 2048, 500, 0.1), (4080, 2056, 3000, 0.05), (4097, 2056, 3000, 0.05), (50, 40, 801, 1.0),
-    (8200, 1032, 9000, 0.5), (9000, 1001, 700, 0.5)])
+    (8200, 1032, 9000, 0.5), (9000, 1001, 700, 0.5), (9000, 1040, 1030, 1.0), (9000, 1040, 1060, 1.0), (4097, 2056, 33000, 0.9), (40, 1032, 70000, 0.5)])
 def test_embedding_scatter_add(dtype, vocab, dim, n, hot):
-    """Both ways of adding (an fp32 table of at most 8M elements, the bucketed ids), rows of one to thousands of
-    entries (segments of 32), ids out of range, rows that are and are not whole 16-byte vectors, with and without a base table."""
+    """Both ways of adding (an fp32 table, the bucketed ids), rows of one to thousands of entries (segments of 32, groups
+    of 32 segments), ids out of range, rows that are and are not whole 16-byte vectors, with and without a base table."""
     from nabla_b200.native import kernels
 
     torch.manual_seed(n)
@@ -148,6 +148,17 @@ def test_embedding_scatter_add(dtype, vocab, dim, n, hot):
     assert got.shape == (vocab, dim) and got.dtype is dtype and _rel2(got, ref) < STORED[dtype]
     empty = kernels.embedding_scatter_add(base, ids[:0], upd[:0])
     assert torch.equal(empty, base)
+
+
+@pytest.mark.parametrize("vocab,dim,n,dtype,atomics", [
+    (16, 8, 1000, 1, True), (4096, 2048, 12288, 1, True), (4097, 2048, 100, 1, False), (4096, 2048, 12289, 1, False), (1000, 64, 49152, 0, True),
+    (1000, 64, 49153, 0, False), (256, 64, 100000, 0, True), (256, 64, 131073, 0, False), (9000, 1001, 700, 1, True), (32000, 1001, 700, 1, False),
+    (32000, 1001, 32001, 1, True), (9000, 1004, 700, 1, True), (9000, 1004, 700, 0, False)])
+def test_ways_of_adding_an_embedding_gradient(vocab, dim, n, dtype, atomics):
+    """On both sides of the rule's lines: the atomics' scratch is the table in fp32."""
+    from nabla_b200.native import kernels
+
+    assert (kernels._L().nb_embedding_scatter_work(n, dim, vocab, dtype) == vocab * dim) == atomics
 
 
 def test_gradient_of_an_embedding_takes_no_table_of_zeros():
