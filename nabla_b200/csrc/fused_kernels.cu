@@ -13,6 +13,7 @@
 // All of them are bandwidth bound: 16-byte vector accesses, fp32 math, one pass over DRAM
 // where the row fits in registers / L1.
 #include <cuda_runtime.h>
+#include <cfloat>
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -670,12 +671,14 @@ __global__ void __launch_bounds__(256) softmax_kernel(const T* __restrict__ x, T
 //
 // Rows of any width and alignment move in 16-byte vectors: the elements before a row's first 16-byte
 // boundary and behind its last are taken one by one (a vocabulary that is not a multiple of 8 gives every
-// row another offset). 4096 x 10001 bf16: forward 95 us with scalar rows, 33 so; gradient 98 and 37.
+// row another offset). 4096 x 10001 bf16: forward 95 us with scalar rows, 33 so; gradient 98 and 37. WHOLE: all rows are
+// whole aligned vectors, with no such offsets to work out. Of other rows those of up to 256 elements take one element
+// per thread (65536 x 9: gradient 37 us, 43 by vectors and edges).
 template <typename T>
 __device__ __forceinline__ int row_head(const T* row, int D) {       // elements before the first 16-byte boundary
   return min(D, (int)(((16u - (unsigned)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) / sizeof(T)));
 }
-template <typename T>
+template <typename T, bool WHOLE>
 __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__ logits,
                                                           const long long* __restrict__ tgt, float* __restrict__ lse_out,
                                                           float* __restrict__ picked, int rows, int D) {
@@ -683,14 +686,15 @@ __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
   const T* xr = logits + (size_t)row * D;
-  float m = -INFINITY, s = 0.f;
+  // the maximum starts at the lowest finite value: elements of -inf then add exp(-inf) = 0 without a test
+  float m = -FLT_MAX, s = 0.f;
   constexpr int V = Vec<T>::N;
-  const int head = row_head(xr, D), body = (D - head) / V * V, tail = head + body;
+  const int head = WHOLE ? 0 : D <= 256 ? D : row_head(xr, D), body = WHOLE ? D : (D - head) / V * V, tail = head + body;
   const int edge = threadIdx.x < head ? (int)threadIdx.x : tail + (int)threadIdx.x - head;     // one edge element per thread
-  if (edge < D) {
-    m = to_f<T>(xr[edge]);
-    s = m == -INFINITY ? 0.f : 1.f;                            // exp(m - m); NaN stays in s
-    if (m != m) s = m;
+  if (!WHOLE && edge < D) {
+    const float v = to_f<T>(xr[edge]);
+    m = fmaxf(m, v);
+    s = __expf(v - m);                                         // NaN stays in s
   }
   for (int c = head + threadIdx.x * V; c < tail; c += blockDim.x * V) {
     float v[V];
@@ -699,12 +703,11 @@ __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__
 #pragma unroll
     for (int j = 1; j < V; ++j) lm = fmaxf(lm, v[j]);
     if (lm > m) { s = s * __expf(m - lm); m = lm; }
-    const float ms = m == -INFINITY ? 0.f : m;                 // only -inf so far: each adds exp(-inf) = 0
 #pragma unroll
-    for (int j = 0; j < V; ++j) s += __expf(v[j] - ms);
+    for (int j = 0; j < V; ++j) s += __expf(v[j] - m);
   }
   const float gm = block_max<8>(m, sh);
-  s = (m == -INFINITY) ? s : s * __expf(m - gm);               // 0 (or NaN) where the thread saw only -inf
+  s *= __expf(m - gm);
   const float gs = block_sum<8>(s, sh);
   if (threadIdx.x == 0) {
     const long long t = tgt[row];
@@ -713,7 +716,7 @@ __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__
   }
 }
 // dlogits = exp(logits - lse) * g_lse[row] + onehot(target) * g_pick[row]
-template <typename T>
+template <typename T, bool WHOLE>
 __global__ void __launch_bounds__(256) lse_pick_bwd_kernel(const T* __restrict__ logits,
                                                           const long long* __restrict__ tgt,
                                                           const float* __restrict__ lse, const float* __restrict__ g_lse,
@@ -728,11 +731,16 @@ __global__ void __launch_bounds__(256) lse_pick_bwd_kernel(const T* __restrict__
   const float gl = g_lse ? g_lse[row] : 0.f;
   const float gp = g_pick ? g_pick[row] : 0.f;
   constexpr int V = Vec<T>::N;
-  // both rows have the same offset from a 16-byte boundary unless a caller's base pointers differ in it
-  const int head = row_head(xr, D) == row_head(dr, D) ? row_head(xr, D) : D;
-  const int body = (D - head) / V * V, tail = head + body;
   auto grad = [&](float v, int c) { return __expf(v - l) * gl + (c == t ? gp : 0.f); };
-  for (int e = threadIdx.x; e < D - body; e += blockDim.x) {
+  if (!WHOLE && D <= 256) {
+    const int c = threadIdx.x;
+    if (c < D) dr[c] = from_f<T>(grad(to_f<T>(xr[c]), c));
+    return;
+  }
+  // both rows have the same offset from a 16-byte boundary unless a caller's base pointers differ in it
+  const int head = WHOLE ? 0 : row_head(xr, D) == row_head(dr, D) ? row_head(xr, D) : D;
+  const int body = WHOLE ? D : (D - head) / V * V, tail = head + body;
+  for (int e = threadIdx.x; !WHOLE && e < D - body; e += blockDim.x) {
     const int c = e < head ? e : body + e;
     dr[c] = from_f<T>(grad(to_f<T>(xr[c]), c));
   }
@@ -2053,17 +2061,21 @@ int nb_softmax(const void* x, void* y, int rows, int D, int log, int dtype, void
 int nb_lse_pick_fwd(const void* logits, const long long* tgt, float* lse, float* picked, int rows, int D, int dtype,
                     void* stream) {
   if (rows <= 0) return 0;
-  if (dtype) lse_pick_fwd_kernel<bf16><<<rows, 256, 0, STREAM>>>((const bf16*)logits, tgt, lse, picked, rows, D);
-  else lse_pick_fwd_kernel<float><<<rows, 256, 0, STREAM>>>((const float*)logits, tgt, lse, picked, rows, D);
+  const bool whole = D % (dtype ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+#define LSE(T, W) lse_pick_fwd_kernel<T, W><<<rows, 256, 0, STREAM>>>((const T*)logits, tgt, lse, picked, rows, D)
+  if (dtype) { if (whole) LSE(bf16, true); else LSE(bf16, false); }
+  else { if (whole) LSE(float, true); else LSE(float, false); }
+#undef LSE
   return CHECK_LAUNCH();
 }
 int nb_lse_pick_bwd(const void* logits, const long long* tgt, const float* lse, const float* g_lse, const float* g_pick,
                     void* dlogits, int rows, int D, int dtype, void* stream) {
   if (rows <= 0) return 0;
-  if (dtype)
-    lse_pick_bwd_kernel<bf16><<<rows, 256, 0, STREAM>>>((const bf16*)logits, tgt, lse, g_lse, g_pick, (bf16*)dlogits, rows, D);
-  else
-    lse_pick_bwd_kernel<float><<<rows, 256, 0, STREAM>>>((const float*)logits, tgt, lse, g_lse, g_pick, (float*)dlogits, rows, D);
+  const bool whole = D % (dtype ? 8 : 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0;
+#define LSE(T, W) lse_pick_bwd_kernel<T, W><<<rows, 256, 0, STREAM>>>((const T*)logits, tgt, lse, g_lse, g_pick, (T*)dlogits, rows, D)
+  if (dtype) { if (whole) LSE(bf16, true); else LSE(bf16, false); }
+  else { if (whole) LSE(float, true); else LSE(float, false); }
+#undef LSE
   return CHECK_LAUNCH();
 }
 

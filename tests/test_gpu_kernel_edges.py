@@ -473,12 +473,15 @@ def test_nf4_codes(dtype, n, block, offset):
 
 # ---------------------------------------------------------------- cross-entropy rows
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,D", [(3, 1), (5, 7), (4, 8), (9, 33), (6, 1000), (7, 2051), (3, 10001), (2, 32000)])
-def test_logsumexp_and_gradient_at_any_row_alignment(dtype, rows, D):
+@pytest.mark.parametrize("rows,D,offset", [(3, 1, 0), (5, 7, 0), (4, 8, 0), (9, 33, 0), (4, 255, 0), (4, 256, 0), (4, 257, 0), (6, 1000, 0), (7, 2051, 0),
+                                           (3, 10001, 0), (2, 32000, 0), (6, 1000, 1), (5, 256, 3), (4, 64, 8)])
+def test_logsumexp_and_gradient_at_any_row_alignment(dtype, rows, D, offset):
+    """Whole aligned vectors, an element per thread, and vectors between edges; logits that start inside a vector."""
     from nabla_b200.native import kernels
 
     torch.manual_seed(7)
-    x = (torch.randn(rows, D, device="cuda") * 3).to(dtype)
+    x = torch.empty(rows * D + offset, device="cuda", dtype=dtype)[offset:].view(rows, D)
+    x.copy_(torch.randn(rows, D, device="cuda") * 3)
     x[0, D // 3: D // 3 + 20] = float("-inf")          # masked classes, here and there a whole vector of them
     if D > 1:
         x[0, D - 1] = 1.0
@@ -492,6 +495,28 @@ def test_logsumexp_and_gradient_at_any_row_alignment(dtype, rows, D):
     ref = torch.exp(x.double() - safe.double()[:, None]) * gl.double()[:, None]
     ref[ok] = ref[ok].scatter_add(1, t[ok][:, None], gp.double()[ok][:, None])
     assert _rel2(kernels.lse_pick_bwd(x, t, safe, gl, gp), ref) < STORED[dtype]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D", [5, 256, 1001, 4096])
+def test_logsumexp_of_rows_at_the_ends_of_the_range(dtype, D):
+    """Rows of -inf, of the type's lowest value, of -inf but for the lowest or for one element, with +inf and NaN."""
+    from nabla_b200.native import kernels
+
+    low, inf = torch.finfo(dtype).min, float("inf")
+    x = torch.full((7, D), -inf, device="cuda", dtype=dtype)
+    x[1] = low
+    x[2, D // 2] = low
+    x[3, D - 1] = -3.0
+    x[4] = 1.0
+    x[4, D // 3] = inf
+    x[5] = 1.0
+    x[5, 0] = float("nan")
+    x[6] = torch.finfo(dtype).max / 4
+    lse, _ = kernels.lse_pick_fwd(x, torch.zeros(7, dtype=torch.int64, device="cuda"))
+    ref = torch.logsumexp(x.double(), -1)
+    assert lse[0] == -inf and not bool(torch.isfinite(lse[4])) and bool(torch.isnan(lse[5]))
+    torch.testing.assert_close(lse[[1, 2, 3, 6]].double(), ref[[1, 2, 3, 6]], rtol=1e-5, atol=1e-5)
 
 
 # ---------------------------------------------------------------- GEMM rows that are not 16-byte aligned
