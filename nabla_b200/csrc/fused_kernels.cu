@@ -1356,9 +1356,22 @@ __global__ void __launch_bounds__(256) nf4_dequant_codes_kernel(const uint8_t* _
       for (int j = 0; j < 16; ++j) o[j] = cb[(w[j >> 2] >> (8 * (j & 3))) & 15] * scale;
 #pragma unroll
       for (int j = 0; j < 16; j += Vec<T>::N) store_vec<T>(out + i0 + j, o + j);
-    } else {
+    } else if constexpr (WHOLE) {                    // the last codes
       for (int j = 0; j < 16; ++j)
         if (i0 + j < n) out[i0 + j] = from_f<T>(cb[codes[i0 + j] & 15] * absmax[(i0 + j) / block]);
+    } else {
+      // any block size and alignment: one division per thread, then the scale moves on where a block ends
+      size_t b = i0 / block;
+      int left = block - (int)(i0 - b * block);
+      float scale = absmax[b];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (i0 + j < n) {
+          if (left == 0) { scale = absmax[++b]; left = block; }
+          out[i0 + j] = from_f<T>(cb[codes[i0 + j] & 15] * scale);
+          --left;
+        }
+      }
     }
   }
 }
