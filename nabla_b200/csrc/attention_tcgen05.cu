@@ -586,6 +586,7 @@ __global__ void __launch_bounds__(128) attn_fwd_combine_kernel(const FwdArgs arg
   const float inv = have ? 1.f / sum : 0.f;
   const int q = (int)(row % args.Sq);
   const long long bh = row / args.Sq;
+  if (!NB_IN_BOUNDS(NB_SITE_ATTN_STORE, bh, (long long)args.B * args.H)) return;
   __nv_bfloat16* orow = args.O + (bh / args.H) * args.o_sb + (bh % args.H) * args.o_sh + q * args.o_ss + lane * E;
 #pragma unroll
   for (int e = 0; e < E; e += 2) *reinterpret_cast<uint32_t*>(orow + e) = pack_bf16(acc[e] * inv, acc[e + 1] * inv);
@@ -637,7 +638,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeArgs a) {
     for (int u = 0; u < DEC_U; ++u) {
       const int k = kb + u * G;
       kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
-      if (k < k1) {
+      if (k < k1 && NB_IN_BOUNDS(NB_SITE_ATTN_TMA_COORD, k, f.Skv)) {
         kr[u] = *reinterpret_cast<const uint4*>(kp + k * a.k_ss);
         vr[u] = *reinterpret_cast<const uint4*>(vp + k * a.v_ss);
       }
@@ -719,6 +720,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeArgs a) {
     o = have ? o / sum : 0.f;
     const float lse = have ? (mx + log2f(sum)) * 0.6931471805599453f : -INFINITY;
     const long long row = ((long long)b * f.H + h) * f.Sq + i;
+    if (!NB_IN_BOUNDS(NB_SITE_ATTN_STORE, row, rows) || !NB_IN_BOUNDS(NB_SITE_ATTN_STORE, sp, f.nsplit)) continue;
     if (f.nsplit > 1) {
       f.part_o[(sp * rows + row) * HD + d] = o;
       if (d == 0) f.part_lse[sp * rows + row] = lse;

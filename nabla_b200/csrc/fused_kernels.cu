@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
       xr[u] = dr[u] = make_uint4(0, 0, 0, 0);
       rs[u] = nmr[u] = 0.f;
       if (row < rows) {
-        if (act) {
+        if (act && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, (long long)row * D + c + V - 1, (long long)rows * D)) {
           xr[u] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + c);
           dr[u] = *reinterpret_cast<const uint4*>(dy + (size_t)row * D + c);
         }
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int row = base + u * stride + slot;
-      if (act && row < rows) {
+      if (act && row < rows && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, (long long)row * D + c + V - 1, (long long)rows * D)) {
         // dx = rstd * (g - m1 - xhat * m2) = g * rstd + (xhat * (-rstd * m2) + (-rstd * m1))
         const float2 rs2 = make_float2(rs[u], rs[u]), nmr2 = make_float2(nmr[u], nmr[u]);
         const float2 a2 = make_float2(-rs[u] * m2[u], -rs[u] * m2[u]), b2 = make_float2(-rs[u] * m1[u], -rs[u] * m1[u]);
@@ -616,6 +616,7 @@ __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict_
   if (r_in < rpp) {
 #pragma unroll 4
     for (int r = r0 + r_in; r < r1; r += rpp) {
+      if (!NB_IN_BOUNDS(NB_SITE_REDUCE_INDEX, ((long long)r * N + c * V) + V - 1, (long long)rows * N)) break;
       float v[V];
       load_vec<T>(x + (size_t)r * N + c * V, v);
 #pragma unroll
@@ -936,11 +937,11 @@ __global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __r
   const long long id = i < n_ids ? ids[i] : -1;
   const bool ok = id >= 0 && id < vocab;
   const int rank = scatter_rank(ws.counts, id, ok);
-  if (ok) ws.rank[i] = rank;
+  if (ok && NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, rank, n_ids)) ws.rank[i] = rank;
 }
 // List slots and segments of every row; the rows of a block come in order, the blocks in any. A row of many
 // segments is written by the whole block.
-__global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int vocab) {
+__global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int n_ids, int vocab) {
   constexpr int FEW = 4;
   struct Row { int v, c, at, sg, h; };
   __shared__ unsigned long long wsum[8];
@@ -958,7 +959,7 @@ __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int vocab
     base_sg = atomicAdd(ws.nseg, (int)(total >> 32));
   }
   __syncthreads();
-  if (c) {
+  if (c && NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, base_at + (int)(unsigned)at0 + c - 1, n_ids)) {      // as many segments at most
     const int at = base_at + (int)(unsigned)at0, sg = base_sg + (int)(at0 >> 32), k = (c + SCAT_SEG - 1) / SCAT_SEG;
     ws.start[v] = at;
     const int h = k > 1 ? atomicAdd(ws.nheavy, k) : -1;
@@ -978,7 +979,9 @@ __global__ void __launch_bounds__(256) scatter_place_kernel(const long long* __r
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n_ids) return;
   const long long id = ids[i];
-  if (id >= 0 && id < vocab) ws.list[ws.start[id] + ws.rank[i]] = i;
+  if (id < 0 || id >= vocab) return;
+  const int slot = ws.start[id] + ws.rank[i];
+  if (NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, slot, n_ids)) ws.list[slot] = i;
 }
 
 // Columns [c, c + VN) of the fp32 sum of `n` rows of upd. SCAT_U rows are in flight: the rows lie anywhere, so
@@ -1065,6 +1068,7 @@ __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(cons
     const int4 sg = next;
     if (s + (int)gridDim.x < total) next = ws.seg[s + gridDim.x];
     const int v = sg.x;
+    if (!NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, sg.w < 0 ? 0 : sg.w, 2 * (n_ids / SCAT_SEG) + 1)) continue;   // partial row
     for (int c = threadIdx.x * VN; c < D; c += blockDim.x * VN) {
       float acc[VN];
       scatter_sum<T, VN>(upd, ws.list + sg.y, sg.z, D, c, n_ids, acc);
@@ -1367,7 +1371,11 @@ __global__ void __launch_bounds__(256) nf4_dequant_codes_kernel(const uint8_t* _
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         if (i0 + j < n) {
-          if (left == 0) { scale = absmax[++b]; left = block; }
+          if (left == 0) {
+            if (!NB_IN_BOUNDS(NB_SITE_NF4_BLOCK, b + 1, (n + block - 1) / block)) return;
+            scale = absmax[++b];
+            left = block;
+          }
           out[i0 + j] = from_f<T>(cb[codes[i0 + j] & 15] * scale);
           --left;
         }
@@ -1412,7 +1420,7 @@ __global__ void __launch_bounds__(256) pool2d_fwd_kernel(const T* __restrict__ x
 // 8192: that image 20 us by pixels, 108 by cells (512 cells); 1 x 256 x 256 x 16 in 16 x 16 18 and 23 (4096); 64 x 14 x 14 x
 // 256 in one window each 35 and 19 (16384).
 struct CellGeom {
-  int H, W, CV, OH, OW, kh, kw, sh, sw, cells_h, cells_w;
+  int N, H, W, CV, OH, OW, kh, kw, sh, sw, cells_h, cells_w;
 };
 template <typename T, bool MAX>
 __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, const CellGeom g, unsigned total) {
@@ -1420,7 +1428,10 @@ __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restric
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
   const unsigned c = i % g.CV, p = i / g.CV, ow = p % g.OW, q = p / g.OW, oh = q % g.OH, n = q / g.OH;
-  const T* xp = x + (((size_t)n * g.H + oh * g.sh) * g.W + ow * g.sw) * g.CV * V + c * V;
+  const size_t at = (((size_t)n * g.H + oh * g.sh) * g.W + ow * g.sw) * g.CV * V + c * V;
+  if (!NB_IN_BOUNDS(NB_SITE_POOL_INPUT, at + ((size_t)(g.kh - 1) * g.W + g.kw - 1) * g.CV * V + V - 1, (size_t)g.N * g.H * g.W * g.CV * V))
+    return;
+  const T* xp = x + at;
   float acc[V];
 #pragma unroll
   for (int j = 0; j < V; ++j) acc[j] = MAX ? -INFINITY : 0.f;
@@ -1446,6 +1457,11 @@ __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restric
   const unsigned c = i % g.CV, p = i / g.CV, cw = p % g.cells_w, q = p / g.cells_w, ch = q % g.cells_h, n = q / g.cells_h;
   const size_t at = (((size_t)n * g.H + ch * g.sh) * g.W + cw * g.sw) * g.CV * V + c * V, down = (size_t)g.W * g.CV * V;
   const bool window = (int)ch < g.OH && (int)cw < g.OW;
+  const int hh = min(g.sh, g.H - (int)ch * g.sh), ww = min(g.sw, g.W - (int)cw * g.sw);      // the cell's part of the image
+  if (!NB_IN_BOUNDS(NB_SITE_POOL_INPUT, at + (hh - 1) * down + (size_t)(ww - 1) * g.CV * V + V - 1, (size_t)g.N * g.H * g.W * g.CV * V) ||
+      (window && !NB_IN_BOUNDS(NB_SITE_POOL_INPUT, ((((size_t)n * g.OH + ch) * g.OW + cw) * g.CV + c) * V + V - 1,
+                               (size_t)g.N * g.OH * g.OW * g.CV * V)))
+    return;
   float d[V], best[V];
   int where[V];                                      // position of the first maximum in the window, -1: none
 #pragma unroll
@@ -1464,7 +1480,6 @@ __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restric
     }
   }
   const float inv = 1.f / (g.kh * g.kw);
-  const int hh = min(g.sh, g.H - (int)ch * g.sh), ww = min(g.sw, g.W - (int)cw * g.sw);
   for (int a = 0; a < hh; ++a)
     for (int b = 0; b < ww; ++b) {
       const bool in = window && a < g.kh && b < g.kw;
@@ -1477,7 +1492,7 @@ __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restric
 // Whether the two kernels above can take a problem.
 static inline bool pool_cells(const void* x, const void* y, const void* z, int N, int H, int W, int C, int OH, int OW, int kh, int kw,
                               int sh, int sw, int ph, int pw, int V, CellGeom& g) {
-  g = CellGeom{H, W, C / V, OH, OW, kh, kw, sh, sw, (H + sh - 1) / sh, (W + sw - 1) / sw};
+  g = CellGeom{N, H, W, C / V, OH, OW, kh, kw, sh, sw, (H + sh - 1) / sh, (W + sw - 1) / sw};
   return ph == 0 && pw == 0 && kh <= sh && kw <= sw && C % V == 0 && (long long)N * g.cells_h * g.cells_w * g.CV < 0x7fffff00ll &&
          ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z)) & 15) == 0;
 }
@@ -2185,7 +2200,7 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
   const int idb = (n_ids + 255) / 256;
   if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 3 + scat_max_heavy(n_ids)) * sizeof(int), STREAM) != cudaSuccess) return -1;
   scatter_count_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
-  scatter_slots_kernel<<<(vocab + 255) / 256, 256, 0, STREAM>>>(ws, vocab);
+  scatter_slots_kernel<<<(vocab + 255) / 256, 256, 0, STREAM>>>(ws, n_ids, vocab);
   scatter_place_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
   const int V = dtype ? 8 : 4;
   const bool vec = D % V == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;

@@ -52,6 +52,28 @@ def test_every_kernel_source_includes_the_check_header_and_uses_it():
     assert "#define NB_ALIGNED(site, value, align) true" in header
 
 
+@pytest.mark.parametrize("source,kernels", [
+    ("fused_kernels.cu", ["layernorm_bwd_rows_kernel", "colsum_narrow_kernel", "scatter_count_kernel", "scatter_slots_kernel", "scatter_place_kernel",
+                          "scatter_rows_kernel", "nf4_dequant_codes_kernel", "pool2d_cell_fwd_kernel", "pool2d_cell_bwd_kernel", "pool2d_bwd_kernel",
+                          "conv2d_direct_kernel", "conv2d_wgrad_direct_kernel", "embedding_gather_kernel", "lse_pick_fwd_kernel", "lse_pick_bwd_kernel"]),
+    ("elementwise_kernels.cu", ["thin_reduce_kernel", "col_reduce_kernel"]),
+    ("attention_tcgen05.cu", ["attn_decode_kernel", "attn_fwd_combine_kernel"])])
+def test_kernels_with_computed_indexes_check_them(source, kernels):
+    """The body of each of these kernels passes its indexes through the debug build's check."""
+    import re
+    from pathlib import Path
+
+    import nabla_b200
+
+    src = (Path(nabla_b200.__file__).parent / "csrc" / source).read_text()
+    for name in kernels:
+        m = re.search(r"__global__[^;{]*\b" + name + r"\(", src)
+        assert m, name
+        body = src[m.end():src.index("\n}\n", m.end())]
+        assert "NB_IN_BOUNDS(" in body, name
+
+
+
 def test_site_table_matches_the_header():
     from nabla_b200 import native
 
