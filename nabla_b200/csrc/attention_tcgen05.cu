@@ -1509,23 +1509,19 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 
 }  // namespace nba
 
-// Few queries and no user mask: the decode kernel (gridDim.y holds the (batch, head) pairs) or the tile kernel, by
-// what was faster over 4 .. 1024 pairs and 64 .. 16384 keys. The decode kernel's FMAs grow with the queries and head_dim,
-// where the tile kernel's time does not; it starts sooner (12 -> 8 us over 64 keys), and a tile kernel of more CTAs than
-// SMs takes a wave per 148 pairs.
-// head_dim 64: one and two queries (256 pairs x 1000 keys: 26 and 32 us, 41 with tiles); three and four up to one tile
-// of keys and from 256 pairs on (128 x 1000: 28 and 25 with tiles, 256 x 1000: 38 and 41).
-// head_dim 128: one query, but for up to a wave of pairs over short prefixes (64 x 300: 17.4 and 16.4; 128 x 1000: 27.7 and
-// 26.6; 64 x 1000: 21.5 and 23.6); two from 512 pairs on (256 x 4096: 142 and 129, 512 x 4096: 226 and 246); up to
-// four over 64 keys, or below 256 keys where the pairs are more than a wave. Four over 128 x 4096: 114 and 68.
+// Few queries and no user mask: the decode kernel (gridDim.y holds the (batch, head) pairs), which keeps the probabilities
+// in fp32 (1.65e-3 from 64 bits, 2.1e-3 to 2.4e-3 with tiles). Times of both over 4 .. 1024 pairs and 64 .. 16384 keys: its
+// FMAs grow with the queries and head_dim, where the tile kernel's time does not; it starts sooner (12 -> 8 us over 64
+// keys), and a tile kernel of more CTAs than SMs takes a wave per 148 pairs.
+// One and two queries: most lengths are faster (256 pairs x 1000 keys x 64: 26 and 32 us, 41 with tiles; 64 x 4096 x 128: 42
+// and 44, 46 and 44 in key ranges, 65 whole), two of head_dim 128 over 128 to 256 pairs up to 3 us or a tenth slower.
+// Three and four, head_dim 64: one tile of keys, or from 256 pairs on (128 x 1000: 28 and 25 with tiles, 256 x 1000: 38 and
+// 41). Head_dim 128: 64 keys, or below 256 where the pairs are more than a wave (4 queries, 128 x 4096: 114 and 68).
 static bool attn_decode(int B, int H, int Sq, int Skv, int D, bool mask) {
   const long long bh = (long long)B * H;
-  const bool one_wave = bh <= 148;
   if (mask || Sq > nba::DEC_MAX_Q || bh > 65535) return false;
-  if (D == 64) return Sq <= 2 || Skv <= nba::BT || bh >= 256;
-  if (Skv <= 64 || (!one_wave && Skv < 256)) return true;
-  if (Sq == 1) return !one_wave || Skv > (bh > 64 ? 8 * bh : 512);
-  return Sq == 2 && bh >= 512;
+  if (Sq <= 2) return true;
+  return D == 64 ? Skv <= nba::BT || bh >= 256 : Skv <= 64 || (bh > 148 && Skv < 256);
 }
 
 // Key ranges that a forward pass is cut into (1: none).

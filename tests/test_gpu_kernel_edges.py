@@ -729,10 +729,11 @@ def test_attention_of_few_queries_over_a_long_prefix(B, H, Sq, Skv, D):
 
 
 @pytest.mark.parametrize("B,H,Sq,Skv,D,decode,splits", [
-    (1, 16, 1, 4001, 128, True, 31), (4, 16, 1, 4001, 128, True, 10), (1, 64, 1, 500, 128, False, 1), (1, 64, 1, 513, 128, True, 4),
-    (1, 64, 1, 300, 64, True, 1), (1, 128, 3, 1000, 64, False, 1), (1, 256, 4, 1000, 64, True, 3), (8, 16, 4, 4096, 128, False, 1),
-    (2, 256, 2, 4096, 128, True, 2), (1, 256, 2, 4096, 128, False, 1), (1, 16, 4, 64, 128, True, 1), (1, 16, 5, 500, 64, False, 1),
-    (1, 16, 5, 520, 64, False, 5), (1, 64, 33, 4096, 64, False, 2), (1, 8, 300, 4000, 128, False, 1)])
+    (1, 16, 1, 4001, 128, True, 31), (4, 16, 1, 4001, 128, True, 10), (1, 64, 1, 500, 128, True, 3), (1, 64, 1, 300, 64, True, 1),
+    (1, 64, 1, 512, 64, True, 4), (1, 128, 3, 1000, 64, False, 1), (1, 128, 3, 128, 64, True, 1), (1, 256, 4, 1000, 64, True, 3), (8, 16, 4, 4096, 128, False, 1),
+    (2, 256, 2, 4096, 128, True, 2), (1, 128, 3, 65, 128, False, 1), (1, 16, 4, 64, 128, True, 1), (1, 149, 4, 255, 128, True, 1),
+    (1, 149, 4, 256, 128, False, 1), (1, 16, 5, 500, 64, False, 1), (1, 16, 5, 520, 64, False, 5), (1, 64, 33, 4096, 64, False, 2),
+    (1, 8, 300, 4000, 128, False, 1)])
 def test_kernel_and_key_ranges_of_few_queries(B, H, Sq, Skv, D, decode, splits):
     """On both sides of the rules' lines: the number of ranges, and whether the call is the decode kernel (it keeps
     the probabilities in fp32, the tile kernel rounds them to bf16: 1.65e-3 and 2.1e-3 or more from 64 bits)."""
