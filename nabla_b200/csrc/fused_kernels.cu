@@ -224,12 +224,6 @@ __global__ void __launch_bounds__(128, 4) layernorm_bwd_dx_kernel(const T* __res
   }
 }
 
-// Backward in one pass (rows of one vector per lane): a persistent grid of warps walks the rows,
-// each warp computing dx of its row as above while it also adds the row's dy * xhat and dy into
-// per-lane register accumulators for the columns it holds, so dy and x are read from DRAM once
-// instead of twice. At the end the four warps of a block fold their accumulators through shared
-// memory and the block writes one row of `partial` ([gridDim.x][2][D] fp32), which
-// colsum_partials_kernel adds up into dgamma / dbeta.
 // 16-byte vector <-> pairs of floats, for the packed two-wide fp32 instructions (fma.rn.f32x2).
 template <typename T> __device__ __forceinline__ void unpack_pairs(const uint4& raw, float2* out);
 template <> __device__ __forceinline__ void unpack_pairs<float>(const uint4& raw, float2* out) {
@@ -255,98 +249,78 @@ template <> __device__ __forceinline__ uint4 pack_pairs<bf16>(const float2* in) 
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-template <typename T, int VPL>
-__global__ void __launch_bounds__(128, (VPL * Vec<T>::N >= 64 ? 2 : VPL * Vec<T>::N >= 32 ? 3 : 4))
+// Backward in one pass (rows of one vector per lane): a persistent grid of warps walks the rows,
+// each warp computing dx of its row as above while it also adds the row's dy * xhat and dy into
+// register accumulators of its lanes' columns, so dy and x are read from DRAM once
+// instead of twice. At the end the four warps of a block fold their accumulators through shared
+// memory and the block writes one row of `partial` ([gridDim.x][2][D] fp32), which
+// colsum_partials_kernel adds up into dgamma / dbeta.
+template <typename T>
+__global__ void __launch_bounds__(128, 4)
     layernorm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                                const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
                                float* __restrict__ partial, int rows, int D) {
   constexpr int V = Vec<T>::N, P = V / 2;
-  __shared__ float sh[2][32 * V * VPL];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float2 ag[VPL][P], ab[VPL][P];
+  __shared__ float sh[2][32 * V];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = lane * V;
+  const bool act = c < D;
+  float2 ag[P], ab[P];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i)
-#pragma unroll
-    for (int k = 0; k < P; ++k) { ag[i][k] = make_float2(0.f, 0.f); ab[i][k] = make_float2(0.f, 0.f); }
+  for (int k = 0; k < P; ++k) ag[k] = ab[k] = make_float2(0.f, 0.f);
   for (int row = blockIdx.x * 4 + warp; row < rows; row += gridDim.x * 4) {
-    const T* xr = x + (size_t)row * D;
-    const T* dyr = dy + (size_t)row * D;
-    uint4 xraw[VPL], draw[VPL];
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int c = (i * 32 + lane) * V;
-      if (c < D) {
-        xraw[i] = *reinterpret_cast<const uint4*>(xr + c);
-        draw[i] = *reinterpret_cast<const uint4*>(dyr + c);
-      }
+    uint4 xraw, draw;
+    if (act) {
+      xraw = *reinterpret_cast<const uint4*>(x + (size_t)row * D + c);
+      draw = *reinterpret_cast<const uint4*>(dy + (size_t)row * D + c);
     }
     const float mu = mean[row], rs = rstd[row];
     const float2 rs2 = make_float2(rs, rs), nmr2 = make_float2(-mu * rs, -mu * rs);
-    float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f);
+    float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), xv[P], dv[P], gm[P];
+    if (act) {
+      unpack_pairs<T>(xraw, xv);
+      unpack_pairs<T>(draw, dv);
+      if (gamma) unpack_pairs<T>(*reinterpret_cast<const uint4*>(gamma + c), gm);
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int c = (i * 32 + lane) * V;
-      if (c < D) {
-        float2 xv[P], dv[P], gm[P];
-        unpack_pairs<T>(xraw[i], xv);
-        unpack_pairs<T>(draw[i], dv);
-        if (gamma) unpack_pairs<T>(*reinterpret_cast<const uint4*>(gamma + c), gm);
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-          const float2 xh = __ffma2_rn(xv[k], rs2, nmr2);              // (x - mean) * rstd
-          const float2 g = gamma ? __fmul2_rn(dv[k], gm[k]) : dv[k];
-          s1 = __fadd2_rn(s1, g);
-          s2 = __ffma2_rn(g, xh, s2);
-          ag[i][k] = __ffma2_rn(dv[k], xh, ag[i][k]);
-          ab[i][k] = __fadd2_rn(ab[i][k], dv[k]);
-        }
+      for (int k = 0; k < P; ++k) {
+        const float2 xh = __ffma2_rn(xv[k], rs2, nmr2);              // (x - mean) * rstd
+        const float2 g = gamma ? __fmul2_rn(dv[k], gm[k]) : dv[k];
+        s1 = __fadd2_rn(s1, g);
+        s2 = __ffma2_rn(g, xh, s2);
+        ag[k] = __ffma2_rn(dv[k], xh, ag[k]);
+        ab[k] = __fadd2_rn(ab[k], dv[k]);
       }
     }
     const float m1 = warp_sum(s1.x + s1.y) / D;
     const float m2 = warp_sum(s2.x + s2.y) / D;
-    // dx = rstd * (g - m1 - xhat * m2) = g * rstd + (xhat * (-rstd * m2) + (-rstd * m1))
-    const float2 a2 = make_float2(-rs * m2, -rs * m2), b2 = make_float2(-rs * m1, -rs * m1);
-    T* dxr = dx + (size_t)row * D;
+    if (act) {
+      // dx = rstd * (g - m1 - xhat * m2) = g * rstd + (xhat * (-rstd * m2) + (-rstd * m1))
+      const float2 a2 = make_float2(-rs * m2, -rs * m2), b2 = make_float2(-rs * m1, -rs * m1);
+      float2 o[P];
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int c = (i * 32 + lane) * V;
-      if (c < D) {
-        float2 xv[P], dv[P], gm[P], o[P];
-        unpack_pairs<T>(xraw[i], xv);
-        unpack_pairs<T>(draw[i], dv);
-        if (gamma) unpack_pairs<T>(*reinterpret_cast<const uint4*>(gamma + c), gm);
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-          const float2 xh = __ffma2_rn(xv[k], rs2, nmr2);
-          const float2 g = gamma ? __fmul2_rn(dv[k], gm[k]) : dv[k];
-          o[k] = __ffma2_rn(g, rs2, __ffma2_rn(xh, a2, b2));
-        }
-        *reinterpret_cast<uint4*>(dxr + c) = pack_pairs<T>(o);
+      for (int k = 0; k < P; ++k) {
+        const float2 xh = __ffma2_rn(xv[k], rs2, nmr2);
+        const float2 g = gamma ? __fmul2_rn(dv[k], gm[k]) : dv[k];
+        o[k] = __ffma2_rn(g, rs2, __ffma2_rn(xh, a2, b2));
       }
+      *reinterpret_cast<uint4*>(dx + (size_t)row * D + c) = pack_pairs<T>(o);
     }
   }
   for (int w = 0; w < 4; ++w) {
-    if (warp == w) {
+    if (warp == w && act) {
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int c = (i * 32 + lane) * V;
-        if (c < D) {
-#pragma unroll
-          for (int k = 0; k < P; ++k) {
-            sh[0][c + 2 * k] = (w == 0 ? 0.f : sh[0][c + 2 * k]) + ag[i][k].x;
-            sh[0][c + 2 * k + 1] = (w == 0 ? 0.f : sh[0][c + 2 * k + 1]) + ag[i][k].y;
-            sh[1][c + 2 * k] = (w == 0 ? 0.f : sh[1][c + 2 * k]) + ab[i][k].x;
-            sh[1][c + 2 * k + 1] = (w == 0 ? 0.f : sh[1][c + 2 * k + 1]) + ab[i][k].y;
-          }
-        }
+      for (int k = 0; k < P; ++k) {
+        sh[0][c + 2 * k] = (w == 0 ? 0.f : sh[0][c + 2 * k]) + ag[k].x;
+        sh[0][c + 2 * k + 1] = (w == 0 ? 0.f : sh[0][c + 2 * k + 1]) + ag[k].y;
+        sh[1][c + 2 * k] = (w == 0 ? 0.f : sh[1][c + 2 * k]) + ab[k].x;
+        sh[1][c + 2 * k + 1] = (w == 0 ? 0.f : sh[1][c + 2 * k + 1]) + ab[k].y;
       }
     }
     __syncthreads();
   }
   float* prow = partial + (size_t)blockIdx.x * 2 * D;
-  for (int c = threadIdx.x; c < D; c += blockDim.x) {
-    prow[c] = sh[0][c];
-    prow[D + c] = sh[1][c];
+  for (int i = threadIdx.x; i < D; i += blockDim.x) {
+    prow[i] = sh[0][i];
+    prow[D + i] = sh[1][i];
   }
 }
 
@@ -465,7 +439,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
   }
 }
 
-// Backward, part 2 of the two-kernel layout: dgamma = sum_rows dy * xhat, dbeta = sum_rows dy. Block = 32*V columns x a
+// Backward, part 2 of the two-kernel layout (comparisons only): dgamma = sum_rows dy * xhat, dbeta = sum_rows dy. Block = 32*V columns x a
 // slab of rows; 8 warps stride over the slab's rows with register accumulators; partial sums go
 // to `partial` ([gridDim.y][2][D] fp32) and are folded by colsum_partials_kernel.
 template <typename T>
@@ -1969,7 +1943,7 @@ int nb_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y
 // this problem: the grid of the one-pass kernels, or the number of row slabs of the two-kernel path.
 static int ln_bwd_vpl(int D, int dtype) { const int V = dtype ? 8 : 4; return (D / V + 31) / 32; }
 static int g_ln_bwd_two_kernels = 0;
-// 1: always take the two-kernel path (dx, then dgamma / dbeta), for comparisons.
+// 1: always take the two-kernel path (dx, then dgamma / dbeta). For comparisons only: no row needs it.
 void nb_layernorm_bwd_two_kernels(int on) { g_ln_bwd_two_kernels = on; }
 int nb_layernorm_bwd_nblocks(int rows, int D, int dtype) {
   const int vpl = ln_bwd_vpl(D, dtype);              // = warps that share a row in layernorm_bwd_rows_kernel
@@ -2010,7 +1984,7 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
 #define LN_BWD_ONE_PASS(T)                                                                                            \
   {                                                                                                                   \
     if (vpl == 1)                                                                                                     \
-      layernorm_bwd_fused_kernel<T, 1><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean,      \
+      layernorm_bwd_fused_kernel<T><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean,      \
                                                                rstd, (T*)dx, partial, rows, D);                      \
     else {                                                                                                            \
       const int rb = vpl < 8 ? 8 / vpl : 1;                                                                           \

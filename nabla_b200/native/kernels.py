@@ -66,8 +66,8 @@ def _L():
         lib.nb_embedding_scatter_work.restype = c_ll
         lib.nb_layernorm_bwd_two_kernels.argtypes = [c_int]
         lib.nb_layernorm_bwd_two_kernels.restype = None
-        # NABLA_B200_LN_BWD=two_kernels: dx and dgamma / dbeta in separate passes (the layout for rows
-        # wider than 8 vectors per lane), instead of the one-pass kernel
+        # NABLA_B200_LN_BWD=two_kernels: dx and dgamma / dbeta in separate passes instead of the one-pass
+        # kernels, for comparisons (no row width needs them)
         lib.nb_layernorm_bwd_two_kernels(1 if os.environ.get("NABLA_B200_LN_BWD", "fused") == "two_kernels" else 0)
         _lib = lib
     return _lib

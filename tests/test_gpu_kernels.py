@@ -133,7 +133,7 @@ def test_layernorm_fwd_bwd(dtype, rows, D):
     assert _rel(y, ref) < tol
     dx, dg, db = kernels.layernorm_bwd(dy, x, g, mean, rstd)
     assert _rel(dx, xr.grad) < tol and _rel(dg, gr.grad) < tol and _rel(db, br.grad) < tol
-    # the same through the dx + dgamma/dbeta kernel pair (the path of rows wider than 8 vectors per lane)
+    # the same through the dx + dgamma/dbeta kernel pair (kept for comparisons)
     lib = kernels._L()
     lib.nb_layernorm_bwd_two_kernels(1)
     try:
@@ -144,8 +144,8 @@ def test_layernorm_fwd_bwd(dtype, rows, D):
 
 
 def test_layernorm_backward_many_rows_and_wide_rows():
-    """More rows than the persistent grid of the one-pass kernel holds at once (every warp walks
-    several rows), no gamma, and a row too wide for it (4096 bf16 = 16 vectors per lane)."""
+    """More rows than the persistent grid of the one-pass kernels holds at once (every warp walks
+    several rows), no gamma, and the widest row they take (4096 bf16: 16 warps per row)."""
     from nabla_b200.native import kernels
 
     torch.manual_seed(3)
