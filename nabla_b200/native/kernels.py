@@ -276,6 +276,8 @@ class CopyBatch:
     launch (or one per 128 tensors). ``shared``: callers may hold views of the fixed tensors' memory."""
 
     def __init__(self, fixed: list[torch.Tensor], shared: bool = False):
+        from . import use_native
+
         n = len(fixed)
         self.dev = dev = torch.cuda.current_device()
         self.fixed = fixed
@@ -283,8 +285,9 @@ class CopyBatch:
         self.fixed_ptrs = (c_vp * n)(*[t.data_ptr() for t in fixed])
         self.own = [t.data_ptr() for t in fixed]
         self.size = [t.numel() * t.element_size() for t in fixed]
-        # what one launch can move: dense tensors of this device (a CPU scalar among the inputs is not one)
-        self.plain = [t.is_cuda and t.device.index == dev and _is_dense(t) for t in fixed]
+        # what one launch can move: dense tensors of this device (a CPU scalar among the inputs is not one), and none
+        # where the native kernels are switched off
+        self.plain = [use_native(t) and t.device.index == dev and _is_dense(t) for t in fixed]
         self.storages = {t.untyped_storage().data_ptr() for t in fixed} if shared else None
 
     def run(self, others: list[torch.Tensor], into_fixed: bool) -> None:

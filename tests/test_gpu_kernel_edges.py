@@ -418,6 +418,16 @@ def test_copy_batch_reads_before_it_writes_where_pairs_share_memory():
     assert bool((c == 5).all()) and d.tolist() == [4.0, 5.0, 6.0, 7.0]
 
 
+def test_copy_batch_without_native_kernels(monkeypatch):
+    from nabla_b200.native import kernels
+
+    monkeypatch.setenv("NABLA_B200_DISABLE_NATIVE", "1")
+    fixed, src = [torch.zeros(9, device="cuda") for _ in range(3)], [torch.randn(9, device="cuda") for _ in range(3)]
+    n = kernels.launch_count
+    kernels.CopyBatch(fixed).run(src, into_fixed=True)
+    assert kernels.launch_count == n and all(torch.equal(a, b) for a, b in zip(fixed, src))
+
+
 @pytest.mark.parametrize("order", [(1, 0, 2), (1, 2, 0), (0, 1, 2)])
 def test_captured_function_whose_donated_results_come_back_in_other_places(order):
     import nabla_b200 as nb
