@@ -453,14 +453,16 @@ def test_captured_function_with_odd_inputs():
     """Views, a CPU scalar, an input returned as it is and one returned twice, and results that stay valid."""
     import nabla_b200 as nb
 
-    f = nb.compile(lambda x, y, s: (x @ y, x, nb.relu(y), y + s, y), cuda_graph=True)
+    f = nb.compile(lambda x, y, s, c: (x @ y, x, nb.relu(y), y + s, y, y, c), cuda_graph=True)
     first = None
     for i in range(4):
         x = torch.randn(33, 40, device="cuda").t()[:, :17]
         y = torch.randn(17, 24, device="cuda")[:, ::2]
         s = torch.randn(12, device="cuda")
-        out = [t.to_torch() for t in f(*(nb.Tensor.from_torch(t) for t in (x, y, s)))]
-        for got, ref in zip(out, (x @ y, x, y.relu(), y + s, y)):
+        c = torch.tensor(float(i))                     # stays on the CPU
+        out = [t.to_torch() for t in f(*(nb.Tensor.from_torch(t) for t in (x, y, s, c)))]
+        assert out[6].device.type == "cpu"
+        for got, ref in zip(out, (x @ y, x, y.relu(), y + s, y, y, c)):
             torch.testing.assert_close(got, ref, rtol=1e-4, atol=1e-4)
         if first is not None:
             assert torch.equal(first[0], first[1])
@@ -756,6 +758,30 @@ def test_kernel_and_key_ranges_of_few_queries(B, H, Sq, Skv, D, decode, splits):
     k, v = (torch.randn(B, H, Skv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
     o, _ = attention.sdpa_fwd(q, k, v, causal=False, scale=D ** -0.5)
     assert (_rel2(o, _attention64(q, k, v, False)) < 1.85e-3) == decode
+
+
+@pytest.mark.parametrize("kind", ["keys", "rows", "range hidden"])
+@pytest.mark.parametrize("B,H,Sq,Skv,D,splits", [(1, 3, 1, 4001, 128, 32), (2, 1, 4, 700, 64, 6), (2, 4, 33, 2500, 64, 10), (1, 2, 130, 1500, 128, 12),
+                                                 (3, 16, 256, 2049, 128, 3)])
+def test_masked_attention_over_split_keys(B, H, Sq, Skv, D, splits, kind):
+    """Masks are indexed by the key tile of a CTA's range, also where one whole range is hidden from all queries;
+    a few queries with a mask take the tile kernel."""
+    from nabla_b200.native import attention
+
+    attention._lib()
+    assert attention._splits(B, H, Sq, Skv, D, 1) == splits
+    torch.manual_seed(15)
+    q = torch.randn(B, H, Sq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(B, H, Skv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    mask = torch.randn((1, 1, Sq, Skv) if kind == "rows" else (B, 1, 1, Skv), device="cuda")
+    hide = torch.rand(mask.shape, device="cuda") < 0.3
+    hide[..., 0] = False
+    if kind == "range hidden":
+        per = -(-(-(-Skv // 128)) // splits) * 128           # keys of a range
+        hide[..., per:2 * per] = True
+    for value in (-1e9, float("-inf")):
+        for causal in (False, True):
+            _attention_check(q, k, v, causal, mask.masked_fill(hide, value), grads=Sq * Skv < 100000)
 
 
 def test_attention_shows_a_nan_key_in_every_split():
