@@ -20,7 +20,7 @@ CUDA bf16 tensors:
 * ``all_gather(rows) -> linear | matmul [-> dact_mul]``: one launch that pulls the peers' rows while the tensor
   cores already work on the rows that are there; the gathered tensor is still produced.
 * ``zeros -> scatter-add``: the gradient of an embedding table without the table of zeros.
-* ``sum -> sum ...`` over neighbouring axes: one reduction over the joined axes.
+* ``sum -> sum ...`` over neighbouring axes: one reduction over the joined axes, where ``kernels.joined_sum`` takes it.
 
 Every other node is a plain 'op' step. Fusion never changes which tensors exist: fused-away
 intermediates that are still referenced are simply not fusable.
