@@ -20,6 +20,7 @@ CUDA bf16 tensors:
 * ``all_gather(rows) -> linear | matmul [-> dact_mul]``: one launch that pulls the peers' rows while the tensor
   cores already work on the rows that are there; the gathered tensor is still produced.
 * ``zeros -> scatter-add``: the gradient of an embedding table without the table of zeros.
+* ``gather -> add`` of a tensor over the trailing dims (token plus position embedding): one pass (compiled replays).
 * ``sum -> sum ...`` over neighbouring axes: one reduction over the joined axes, where ``kernels.joined_sum`` takes it.
 
 Every other node is a plain 'op' step. Fusion never changes which tensors exist: fused-away
@@ -52,7 +53,9 @@ def _single_consumer_map(nodes: list[OpNode], targets) -> dict[int, list[int]]:
     return cons
 
 
-def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
+def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = False):
+    """``private``: nobody outside ``nodes`` can ask for an intermediate later (a compiled recording), so values that
+    autodiff traced through may be fused away too when no node reads them."""
     from .engine import Plan
 
     cons = _single_consumer_map(nodes, targets)
@@ -75,6 +78,10 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
         return (impl is not None and id(impl) not in target_ids and not impl.is_traced
                 and len(cons.get(id(impl), [])) == 1 and impl.sharding is None and impl.batch_dims == 0)
 
+    def private_intermediate(impl: TensorImpl) -> bool:
+        return (impl is not None and id(impl) not in target_ids and len(cons.get(id(impl), [])) == 1
+                and impl.sharding is None and impl.batch_dims == 0)
+
     for i, n in enumerate(nodes):
         if used[i]:
             continue
@@ -94,6 +101,14 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl]):
                                 a.op.name == "gelu" and a.kwargs.get("approximate", "none") not in ("none", "tanh")):
                             chain = [i, j, k]
         kind = "linear_epilogue"
+        if chain is None and private and n.op.name == "gather" and _is_table_gather(n):
+            o = sole_output(n)
+            if private_intermediate(o):
+                j = cons[id(o)][0]
+                m = nodes[j]
+                if not used[j] and m.op.name == "add" and _is_trailing_add(m, o):
+                    chain = [i, j]
+                    kind = "gather_add"
         if chain is None and n.op.name == "full":
             # zeros -> scatter-add (the gradient of an embedding): the kernel writes every row once and
             # takes no base at all, so the zeros are neither written nor read
@@ -224,6 +239,31 @@ def _is_cuda_bf16_2d(n: OpNode) -> bool:
 
     return (a.device.label == "gpu" and a.dtype is DType.bfloat16 and b.dtype is DType.bfloat16
             and len(b._shape) == 2 and len(a._shape) >= 2)
+
+
+def _is_table_gather(n: OpNode) -> bool:
+    """Rows of an unsharded fp32 / bf16 GPU table."""
+    from ...types import DType
+
+    ins = n.input_impls()
+    return (len(ins) == 2 and n.kwargs.get("axis") == 0 and not n.kwargs.get("bd", 0) and len(ins[0]._shape) == 2
+            and all(x.sharding is None and not x.batch_dims for x in ins) and ins[0].device.label == "gpu"
+            and ins[0].dtype in (DType.bfloat16, DType.float32))
+
+
+def _is_trailing_add(add: OpNode, x: TensorImpl) -> bool:
+    """``x`` plus a tensor of its dtype over its trailing dims (the last one at least)."""
+    ins = add.input_impls()
+    if len(ins) != 2:
+        return False
+    other = ins[1] if ins[0] is x else ins[0] if ins[1] is x else None
+    if other is None or other is x or other.sharding is not None or other.batch_dims or other.dtype is not x.dtype \
+            or other.device != x.device or len(other._shape) > len(x._shape):
+        return False
+    shp = tuple(other._shape)
+    while len(shp) > 1 and shp[0] == 1:
+        shp = shp[1:]
+    return len(shp) >= 1 and tuple(x._shape)[len(x._shape) - len(shp):] == shp
 
 
 def _is_zero_table(n: OpNode, o: TensorImpl) -> bool:
@@ -448,6 +488,24 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
                 o._buffers = [out]
         else:
             store_outputs(last, [[out]])
+        return
+    if kind == "gather_add":
+        from ... import native
+
+        ga, add = group
+        table, idx = [x._buffers[0] for x in ga.input_impls()]
+        rows = ga.outputs()[0]
+        other = [x for x in add.input_impls() if x is not rows][0]._buffers[0]
+        out = None
+        if native.use_native(table) and idx.numel() and table.numel():
+            from ...native import kernels
+
+            out = kernels.embedding_gather(table, idx, other)
+        if out is not None:
+            _store(add, [[out]], keep_graph)
+        else:
+            _plain(ga, keep_graph)
+            _plain(add, keep_graph)
         return
     if kind == "scatter_zeros":
         from ... import native

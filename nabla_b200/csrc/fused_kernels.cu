@@ -832,44 +832,62 @@ __global__ void __launch_bounds__(256) sgd_kernel(const TP* __restrict__ p, cons
 }
 
 // ============================================================== embedding
-template <typename T>
+// out[i] = table[ids[i]] (+ add[i % period]: a position embedding, or one row for all). Ids outside the table give zeros.
+// Bound by the write of `out` and the table's rows. 16384 ids, 32000 x 2048 bf16, 2048 positions: gather 16 us and the
+// add behind it 30, 20 together.
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restrict__ table,
-                                                              const long long* __restrict__ ids, T* __restrict__ out,
-                                                              int n_ids, int D, int vocab) {
+                                                              const long long* __restrict__ ids, const T* __restrict__ add,
+                                                              T* __restrict__ out, int n_ids, int D, int vocab, int period) {
   constexpr int V = Vec<T>::N;
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
   long long id = ids[i];
   const bool ok = id >= 0 && id < vocab;
   const T* src = table + (size_t)(ok ? id : 0) * D;
+  const T* pos = ADD ? add + (size_t)(i % period) * D : nullptr;
   T* dst = out + (size_t)i * D;
   if ((D % V) == 0) {
     for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
       uint4 raw = ok ? *reinterpret_cast<const uint4*>(src + c) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(dst + c) = raw;
+      if constexpr (ADD) {
+        float x[V], p[V];
+        load_vec<T>(pos + c, p);
+        unpack_vec<T>(raw, x);
+#pragma unroll
+        for (int j = 0; j < V; ++j) x[j] += p[j];
+        store_vec<T>(dst + c, x);
+      } else {
+        *reinterpret_cast<uint4*>(dst + c) = raw;
+      }
     }
   } else {
-    for (int c = threadIdx.x; c < D; c += blockDim.x) dst[c] = ok ? src[c] : from_f<T>(0.f);
+    for (int c = threadIdx.x; c < D; c += blockDim.x) {
+      const T x = ok ? src[c] : from_f<T>(0.f);
+      dst[c] = ADD ? from_f<T>(to_f<T>(x) + to_f<T>(pos[c])) : x;
+    }
   }
 }
 // out = base + scatter_add(ids, upd): the gradient of an embedding.
-// Large tables: `out` starts as a copy of base (or zeros, by memset), the ids are bucketed by row (three short
-// launches over the integers), and every row that occurs is written once more, as the fp32 sum of its updates
-// in registers: no fp32 table that is zeroed, added to with atomics and converted. A row with more than SCAT_SEG
-// entries (frequent tokens: ids of text fall off about as 1 / rank) is cut into segments, one block each, whose
-// fp32 partial rows are added up in two steps: the last block of every SCAT_GROUP segments adds those, the last
-// group of a row the groups. One block per row would leave the most frequent id, some 1000 of 16384 tokens, to one
-// block, and joining them in one step the padding id of a batch (29700 of 33000 ids into 4097 x 2048 fp32: 881 us
-// in one step, 128 in two).
-// Bound by latency in the rows (dependent loads of a segment, its list, its rows of updates; 1.4 TB/s) after an HBM-bound
-// fill of `out`. 16384 ids into 32000 x 2048 bf16 with a base table: 257 us with the fp32 table, 114 now; 48 for the
-// rows, 11 for the bucketing.
-constexpr int SCAT_SEG = 32, SCAT_GROUP = 32;
+// Large tables: the ids are bucketed by row (three short launches over the integers), and one launch writes every
+// row of the table once: rows that occur as the fp32 sum of their updates in registers, the others as zeros or as the
+// base's row. No fp32 table that is zeroed, added to with atomics and converted, and no fill of `out` before it.
+// A row with at most SCAT_LIGHT entries is one warp's work (its loads are a list entry and then the rows, two
+// latencies in a chain, so what counts is how many rows the chip has on its way: 4 KB rows by a block each were 1.4 TB/s);
+// a row with more takes the whole block, in segments of SCAT_SEG entries whose fp32 partial rows are added up in two
+// steps where there are several: the last block of every SCAT_GROUP segments adds those, the last group of a row the
+// groups. One block per row would leave the most frequent id, some 1000 of 16384 tokens (ids of text fall off about as
+// 1 / rank), to one block, and joining them in one step the padding id of a batch (29700 of 33000 ids into 4097 x 2048
+// fp32: 881 us in one step, 128 in two).
+// 16384 ids of text into 32000 x 2048 bf16: fill 23 + rows 34 us before, 49 now (131 MB written, 67 read: 30 us at the
+// copy rate).
+constexpr int SCAT_SEG = 32, SCAT_GROUP = 32, SCAT_LIGHT = 4;
 struct ScatWs {
-  int *counts, *done, *total, *nseg, *nheavy;   // zeroed by the launcher
+  int *counts, *done, *total, *nseg, *nheavy, *nlight;   // zeroed by the launcher
   int* gdone;                                   // likewise: finished segments of a group, at its first partial row
   int *start, *rank, *list;                     // first list slot per row; place of an entry in its row; entries by row
-  int4* seg;                                    // (row, first list slot, entries, partial row or -1)
+  int4* seg;                                    // (row, first list slot, entries, partial row or -1): the rows of at most
+                                                // SCAT_LIGHT entries from the end backwards, the others from the start on
 };
 // Segment q of a row of `c` entries from list slot `at` on; h: its first partial row, or -1.
 __device__ __forceinline__ int4 scatter_segment(int v, int c, int at, int h, int q) {
@@ -884,7 +902,7 @@ __device__ __forceinline__ int scatter_rank(int* counts, long long id, bool ok) 
   base = __shfl_sync(0xffffffffu, base, leader);
   return base + __popc(same & ((1u << lane) - 1u));
 }
-// Inclusive scan over the block of (entries, segments), packed in the halves of 64 bits.
+// Inclusive scan over the block, two numbers packed in the halves of 64 bits.
 template <int NW>
 __device__ __forceinline__ unsigned long long scatter_scan(unsigned long long x, unsigned long long* wsum,
                                                            unsigned long long& total) {
@@ -918,26 +936,32 @@ __global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __r
 __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int n_ids, int vocab) {
   constexpr int FEW = 4;
   struct Row { int v, c, at, sg, h; };
-  __shared__ unsigned long long wsum[8];
-  __shared__ int base_at, base_sg, nmany;
+  __shared__ unsigned long long wsum[8], wsum2[8];
+  __shared__ int base_at, base_lt, base_sg, nmany;
   __shared__ Row many[256];
   if (threadIdx.x == 0) nmany = 0;                   // (the scan below has the barrier)
   const int v = blockIdx.x * 256 + threadIdx.x;
   const int c = v < vocab ? ws.counts[v] : 0;
-  const unsigned long long t = (unsigned long long)((c + SCAT_SEG - 1) / SCAT_SEG) << 32 | (unsigned)c;
-  unsigned long long total;
+  const bool light = c <= SCAT_LIGHT;
+  const int k = light ? 0 : (c + SCAT_SEG - 1) / SCAT_SEG;
+  const unsigned long long t = (unsigned long long)(c > 0 && light) << 32 | (unsigned)c;     // (light rows, entries)
+  unsigned long long total, heavy = 0;
   const unsigned long long at0 = scatter_scan<8>(t, wsum, total) - t;
   if (total == 0) return;                            // the same in every thread
+  const unsigned long long sg0 = scatter_scan<8>((unsigned)k, wsum2, heavy) - (unsigned)k;
   if (threadIdx.x == 0) {
     base_at = atomicAdd(ws.total, (int)(unsigned)total);
-    base_sg = atomicAdd(ws.nseg, (int)(total >> 32));
+    base_lt = total >> 32 ? atomicAdd(ws.nlight, (int)(total >> 32)) : 0;
+    base_sg = heavy ? atomicAdd(ws.nseg, (int)heavy) : 0;
   }
   __syncthreads();
   if (c && NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, base_at + (int)(unsigned)at0 + c - 1, n_ids)) {      // as many segments at most
-    const int at = base_at + (int)(unsigned)at0, sg = base_sg + (int)(at0 >> 32), k = (c + SCAT_SEG - 1) / SCAT_SEG;
+    const int at = base_at + (int)(unsigned)at0, sg = base_sg + (int)sg0;
     ws.start[v] = at;
     const int h = k > 1 ? atomicAdd(ws.nheavy, k) : -1;
-    if (k <= FEW) {
+    if (light) {
+      ws.seg[n_ids - 1 - (base_lt + (int)(at0 >> 32))] = make_int4(v, at, c, -1);
+    } else if (k <= FEW) {
       for (int q = 0; q < k; ++q) ws.seg[sg + q] = scatter_segment(v, c, at, h, q);
     } else {
       many[atomicAdd(&nmany, 1)] = Row{v, c, at, sg, h};
@@ -1029,15 +1053,89 @@ __device__ __forceinline__ void scatter_join(const float* p, int n, size_t step,
 #pragma unroll
     for (int j = 0; j < VN; ++j) acc[j] += __ldcg(p + q * step + c + j);
 }
-// The blocks walk the segments, the next descriptor on its way while one is worked on. VN: elements per access
-// (16 bytes, or 1 where rows are not 16-byte aligned).
+// A row of `n` <= R entries by one warp: R rows times SCAT_U / R vectors of each on their way per lane.
+template <typename T, int VN, int R>
+__device__ __forceinline__ void scatter_light(const T* __restrict__ upd, const T* __restrict__ base, T* __restrict__ out,
+                                              const int* __restrict__ list, int n, size_t v, int D, int n_ids, int lane) {
+  constexpr int CU = SCAT_U / R;
+  const T* row[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = list[r < n ? r : 0];
+    if (!NB_IN_BOUNDS(NB_SITE_EMB_SCATTER_ID, i, n_ids)) return;
+    row[r] = upd + (size_t)i * D;
+  }
+#pragma unroll 1
+  for (int c0 = lane * VN; c0 < D; c0 += 32 * VN * CU) {
+    uint4 raw[CU][R];
+#pragma unroll
+    for (int u = 0; u < CU; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int c = c0 + u * 32 * VN;
+        raw[u][r] = make_uint4(0, 0, 0, 0);
+        if (r < n && c < D) {
+          if (VN > 1) raw[u][r] = *reinterpret_cast<const uint4*>(row[r] + c);
+          else raw[u][r].x = __float_as_uint(to_f<T>(row[r][c]));
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < CU; ++u) {
+      const int c = c0 + u * 32 * VN;
+      float acc[VN];
+#pragma unroll
+      for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float x[VN];
+        if constexpr (VN > 1) unpack_vec<T>(raw[u][r], x);
+        else x[0] = __uint_as_float(raw[u][r].x);
+#pragma unroll
+        for (int j = 0; j < VN; ++j) acc[j] += x[j];
+      }
+      if (c < D) scatter_write<T, VN>(base, out, v * D + c, acc);
+    }
+  }
+}
+// Rows without an entry, one warp per SCAT_IDLE rows: zeros, or the base's row.
+constexpr int SCAT_IDLE = 8;
+template <typename T, int VN>
+__device__ __forceinline__ void scatter_idle(const T* __restrict__ base, T* __restrict__ out, const int* __restrict__ counts,
+                                             int vocab, size_t D, int warp, int nwarps, int lane) {
+  for (int v0 = warp * SCAT_IDLE; v0 < vocab; v0 += nwarps * SCAT_IDLE) {
+    const bool idle = lane < SCAT_IDLE && v0 + lane < vocab && counts[v0 + lane] == 0;
+    for (unsigned m = __ballot_sync(0xffffffffu, idle); m; m &= m - 1) {
+      const size_t at = (size_t)(v0 + __ffs(m) - 1) * D;
+      if (base != nullptr) {
+        for (size_t c = lane * VN; c < D; c += 32 * VN) {
+          if (VN > 1) *reinterpret_cast<uint4*>(out + at + c) = *reinterpret_cast<const uint4*>(base + at + c);
+          else out[at + c] = base[at + c];
+        }
+      } else {
+        for (size_t c = lane * VN; c < D; c += 32 * VN) {
+          if (VN > 1) *reinterpret_cast<uint4*>(out + at + c) = make_uint4(0, 0, 0, 0);
+          else out[at + c] = from_f<T>(0.f);
+        }
+      }
+    }
+    if (v0 > vocab - nwarps * SCAT_IDLE) break;      // (the next v0 may not fit an int)
+  }
+}
+// Every row of the table, once. The blocks walk the segments of crowded rows, the next descriptor on its way while one is
+// worked on; then their warps the rows of few entries. Every other block writes its rows without an entry first, the rest
+// last, so that stores and dependent loads run side by side. VN: elements per access (16 bytes, or 1 where rows are not
+// 16-byte aligned).
 template <typename T, int VN>
 __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
                                                           T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
-                                                          int D) {
+                                                          int D, int vocab) {
   __shared__ int last;
-  const int total = *ws.nseg;
-  int4 next = ws.seg[blockIdx.x];                    // not written past the last segment: read, then dropped
+  const int total = *ws.nseg, lights = *ws.nlight;
+  const int lane = threadIdx.x & 31, nwarps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;         // few rows: spread over the blocks
+  if (blockIdx.x & 1) scatter_idle<T, VN>(base, out, ws.counts, vocab, D, warp, nwarps, lane);
+  int4 next = make_int4(0, 0, 0, -1);
+  if ((int)blockIdx.x < total) next = ws.seg[blockIdx.x];
   for (int s = blockIdx.x; s < total; s += gridDim.x) {
     const int4 sg = next;
     if (s + (int)gridDim.x < total) next = ws.seg[s + gridDim.x];
@@ -1087,6 +1185,18 @@ __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(cons
       scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
     }
   }
+  const int4* lseg = ws.seg + n_ids - 1;
+  int4 lnext = make_int4(0, 0, 0, -1);
+  if (lwarp < lights) lnext = lseg[-lwarp];
+  for (int s = lwarp; s < lights; s += nwarps) {
+    const int4 sg = lnext;
+    if (nwarps < lights - s) lnext = lseg[-(s + nwarps)];
+    const int* list = ws.list + sg.y;
+    if (sg.z == 1) scatter_light<T, VN, 1>(upd, base, out, list, 1, sg.x, D, n_ids, lane);
+    else scatter_light<T, VN, SCAT_LIGHT>(upd, base, out, list, sg.z, sg.x, D, n_ids, lane);
+    if (nwarps >= lights - s) break;
+  }
+  if (!(blockIdx.x & 1)) scatter_idle<T, VN>(base, out, ws.counts, vocab, D, warp, nwarps, lane);
 }
 // Small tables: acc[ids[i]] += upd[i] in an fp32 table that stays in L2, four columns per atomic (VEC).
 template <typename T, bool VEC>
@@ -2109,17 +2219,20 @@ int nb_sgd(const void* p, const void* g, const float* buf, void* p_out, float* b
   return CHECK_LAUNCH();
 }
 
-int nb_embedding_gather(const void* table, const long long* ids, void* out, int n_ids, int D, int vocab, int dtype,
-                        void* stream) {
+int nb_embedding_gather(const void* table, const long long* ids, const void* add, void* out, int n_ids, int D, int vocab,
+                        int period, int dtype, void* stream) {
   if (n_ids <= 0) return 0;
-  if (dtype) embedding_gather_kernel<bf16><<<n_ids, 128, 0, STREAM>>>((const bf16*)table, ids, (bf16*)out, n_ids, D, vocab);
-  else embedding_gather_kernel<float><<<n_ids, 128, 0, STREAM>>>((const float*)table, ids, (float*)out, n_ids, D, vocab);
+  if (add != nullptr && period <= 0) return -2;
+#define GATHER(T, ADD) embedding_gather_kernel<T, ADD><<<n_ids, 128, 0, STREAM>>>((const T*)table, ids, (const T*)add, (T*)out, n_ids, D, vocab, period)
+  if (dtype) { if (add) GATHER(bf16, true); else GATHER(bf16, false); }
+  else { if (add) GATHER(float, true); else GATHER(float, false); }
+#undef GATHER
   return CHECK_LAUNCH();
 }
 // out = base + scatter_add(ids, upd); base null: zeros. `work`: nb_embedding_scatter_work(...) 32-bit words of
 // 16-byte aligned scratch.
 static long long scat_max_heavy(long long n_ids) { return 2 * (n_ids / SCAT_SEG); }   // segments of rows with > SCAT_SEG entries
-static long long scat_ints(long long n_ids, long long vocab) { return (3 * vocab + 3 + scat_max_heavy(n_ids) + 2 * n_ids + 3) / 4 * 4; }
+static long long scat_ints(long long n_ids, long long vocab) { return (3 * vocab + 4 + scat_max_heavy(n_ids) + 2 * n_ids + 3) / 4 * 4; }
 // Atomics into an fp32 table, or bucketed ids, by times over tables of 2 .. 32000 rows of 8 .. 2048, 100 .. 100000 ids,
 // spread or crowded on one row. The bucketing is 25 to 35 us of short launches: it wins where the table is more than the
 // L2 keeps (32000 x 2048 bf16, 16384 ids: 263 us with atomics, 136), where much is added to few rows (1000 x
@@ -2154,25 +2267,26 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
     else if (!direct) cast_kernel<float, float><<<grid, 256, 0, STREAM>>>(acc, (float*)out, n, (const float*)base);
     return CHECK_LAUNCH();
   }
-  const size_t bytes = (size_t)vocab * D * (dtype ? 2 : 4);
-  if ((base != nullptr ? cudaMemcpyAsync(out, base, bytes, cudaMemcpyDeviceToDevice, STREAM)
-                       : cudaMemsetAsync(out, 0, bytes, STREAM)) != cudaSuccess)
-    return -1;
-  if (n_ids == 0) return 0;
+  if (n_ids == 0) {
+    const size_t bytes = (size_t)vocab * D * (dtype ? 2 : 4);
+    return (base != nullptr ? cudaMemcpyAsync(out, base, bytes, cudaMemcpyDeviceToDevice, STREAM)
+                            : cudaMemsetAsync(out, 0, bytes, STREAM)) == cudaSuccess ? 0 : -1;
+  }
   ScatWs ws;
   ws.counts = work;
   ws.done = ws.counts + vocab;
   ws.total = ws.done + vocab;
   ws.nseg = ws.total + 1;
   ws.nheavy = ws.nseg + 1;
-  ws.gdone = ws.nheavy + 1;
+  ws.nlight = ws.nheavy + 1;
+  ws.gdone = ws.nlight + 1;
   ws.start = ws.gdone + scat_max_heavy(n_ids);
   ws.rank = ws.start + vocab;
   ws.list = ws.rank + n_ids;
   ws.seg = reinterpret_cast<int4*>(work + scat_ints(n_ids, vocab));
   float* part = reinterpret_cast<float*>(ws.seg + n_ids);
   const int idb = (n_ids + 255) / 256;
-  if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 3 + scat_max_heavy(n_ids)) * sizeof(int), STREAM) != cudaSuccess) return -1;
+  if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 4 + scat_max_heavy(n_ids)) * sizeof(int), STREAM) != cudaSuccess) return -1;
   scatter_count_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
   scatter_slots_kernel<<<(vocab + 255) / 256, 256, 0, STREAM>>>(ws, n_ids, vocab);
   scatter_place_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
@@ -2180,8 +2294,10 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
   const bool vec = D % V == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   int threads = 32;                                  // the power of two that covers a row in one pass, at most 256
   while (threads < 256 && threads * (vec ? V : 1) < D) threads *= 2;
-  const int grid = (int)(n_ids < 148ll * 2048 / threads ? n_ids : 148ll * 2048 / threads);
-#define SCAT(T, VN) scatter_rows_kernel<T, VN><<<grid, threads, 0, STREAM>>>((const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D)
+  // blocks: what the chip holds, or as many as there are entries and groups of SCAT_IDLE rows for their warps
+  const long long held = 148ll * (vec && dtype ? 768 : 1024) / threads, want = ((long long)vocab / SCAT_IDLE + 1) * 32 / threads + 1;
+  const int grid = (int)(held < n_ids || held < want ? held : n_ids > want ? n_ids : want);
+#define SCAT(T, VN) scatter_rows_kernel<T, VN><<<grid, threads, 0, STREAM>>>((const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D, vocab)
   if (dtype) { if (vec) SCAT(bf16, 8); else SCAT(bf16, 1); }
   else { if (vec) SCAT(float, 4); else SCAT(float, 1); }
 #undef SCAT

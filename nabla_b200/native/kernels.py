@@ -33,7 +33,7 @@ def _L():
             "nb_adamw": [c_vp] * 7 + [c_ll] + [c_f] * 8 + [c_vp, c_int, c_int, c_vp],
             "nb_adam_hyper": [c_vp, c_vp, c_f, ctypes.c_double, ctypes.c_double, c_vp],
             "nb_sgd": [c_vp] * 5 + [c_ll] + [c_f] * 4 + [c_int, c_int, c_vp],
-            "nb_embedding_gather": [c_vp] * 3 + [c_int] * 4 + [c_vp],
+            "nb_embedding_gather": [c_vp] * 4 + [c_int] * 5 + [c_vp],
             "nb_embedding_scatter_add": [c_vp] * 5 + [c_int] * 4 + [c_vp],
             "nb_embedding_scatter_sorted": [c_vp] * 5 + [c_int] * 4 + [c_vp],
             "nb_cast": [c_vp, c_vp, c_ll, c_int, c_int, c_vp],
@@ -218,12 +218,27 @@ def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):
 
 
 # ---------------------------------------------------------------- embedding
-def embedding_gather(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
+def embedding_gather(table: torch.Tensor, ids: torch.Tensor, add: torch.Tensor | None = None) -> torch.Tensor | None:
+    """Rows of ``table`` (vocab, D) by id. ``add``: a tensor over the trailing dims of the result (at least the
+    last), added in the same pass; None when that pass does not take it (the caller then gathers and adds)."""
+    period = 0
+    if add is not None:
+        shape = tuple(add.shape)
+        while len(shape) > 1 and shape[0] == 1:
+            shape = shape[1:]
+        full = (*ids.shape, table.shape[1])
+        if add.dtype != table.dtype or not shape or full[len(full) - len(shape):] != shape or not add.numel() \
+                or not elementwise_enabled():
+            return None
+        add = add.contiguous()
+        period = add.numel() // table.shape[1]
     table = table.contiguous()
+    if add is not None and (add.data_ptr() | table.data_ptr()) & 15:
+        return None
     flat = ids.contiguous().view(-1).to(torch.int64)
     D = table.shape[1]
     out = torch.empty((flat.numel(), D), dtype=table.dtype, device=table.device)
-    _ok(_L().nb_embedding_gather(ptr(table), ptr(flat), ptr(out), flat.numel(), D, table.shape[0], _dt(table),
+    _ok(_L().nb_embedding_gather(ptr(table), ptr(flat), ptr(add), ptr(out), flat.numel(), D, table.shape[0], period, _dt(table),
                                  stream_ptr()), "embedding_gather")
     return out.view(*ids.shape, D)
 

@@ -511,7 +511,7 @@ class CompiledFunction:
         """Fused schedule, liveness and in-place marking of a recorded node list."""
         nodes, targets = rec.nodes, rec.targets
         rec.host_sync = any(getattr(n.op, "host_sync", False) for n in nodes)
-        plan = fusion.build_plan(nodes, targets) if fusion.enabled() else None
+        plan = fusion.build_plan(nodes, targets, private=True) if fusion.enabled() else None
         rec.steps = plan.steps if plan is not None else [("op", (i,)) for i in range(len(nodes))]
         if any(rec.donated):
             rec.steps = _optimizer_steps_last(rec.steps, nodes)

@@ -150,6 +150,59 @@ def test_embedding_scatter_add(dtype, vocab, dim, n, hot):
     assert torch.equal(empty, base)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab,dim", [(40000, 264), (9000, 1048), (9001, 2056), (20000, 517), (1100000, 8)])
+def test_embedding_gradient_by_row_counts(dtype, vocab, dim):
+    """Rows of 0 to 4 entries (a warp's work), of 5 and more (a block's), at the ends of the segments of 32, spread over the
+    table; the rows without an entry are the base's bit for bit."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(dim)
+    counts = [1, 2, 3, 4, 5, 31, 32, 33, 64, 65] * 12 + [1] * 200 + [1100]
+    rows = torch.randperm(vocab - 2, device="cuda")[:len(counts)] + 1
+    rows[0], rows[1] = 0, vocab - 1
+    ids = torch.repeat_interleave(rows, torch.tensor(counts, device="cuda"))
+    ids = ids[torch.randperm(ids.numel(), device="cuda")]
+    n = ids.numel()
+    assert kernels._L().nb_embedding_scatter_work(n, dim, vocab, 1 if dtype == torch.bfloat16 else 0) != vocab * dim
+    upd = torch.randn(n, dim, device="cuda").to(dtype)
+    base = torch.randn(vocab, dim, device="cuda").to(dtype)
+    ref = torch.zeros(vocab, dim, dtype=torch.float64, device="cuda").index_add_(0, ids, upd.double())
+    idle = torch.ones(vocab, dtype=torch.bool, device="cuda")
+    idle[rows] = False
+    got = kernels.embedding_scatter_add(base, ids, upd)
+    assert torch.equal(got[idle], base[idle]) and _rel2(got[rows], ref[rows] + base[rows].double()) < STORED[dtype]
+    got = kernels.embedding_scatter_add(None, ids, upd, vocab, dtype)
+    assert not got[idle].any() and _rel2(got[rows], ref[rows]) < STORED[dtype]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("ids,add,fused", [
+    ((3, 70), (70, 64), True), ((3, 70), (64,), True), ((3, 70), (1, 70, 64), True), ((3, 70), (1, 1, 64), True), ((7,), (7, 64), True),
+    ((3, 70), (3, 70, 64), True), ((3, 70), (3, 70, 33), True), ((3, 70), (3, 1, 64), False), ((3, 70), (70, 1), False), ((2, 3), (4, 2, 3, 64), False)])
+def test_embedding_plus_a_tensor_over_trailing_dims(dtype, ids, add, fused):
+    """One pass where the added tensor covers trailing dims (the sum is the one of two passes, bit for bit), two elsewhere, also
+    where the rows are asked for on their own."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    torch.manual_seed(1)
+    dim = add[-1] if add[-1] > 1 else 64
+    table = torch.randn(50, dim, device="cuda").to(dtype)
+    pos = torch.randn(add, device="cuda").to(dtype)
+    idx = torch.randint(0, 50, ids, device="cuda")
+    ref = (table[idx].float() + pos.float()).to(dtype)
+    tt, pt, it = nb.Tensor.from_torch(table), nb.Tensor.from_torch(pos), nb.Tensor.from_torch(idx)
+    for order in (lambda a, b: a + b, lambda a, b: b + a):
+        f = nb.compile(lambda t, p, i: nb.vjp(lambda a, b: order(F.embedding(i, a), b), t, p, create_graph=False)[0])
+        g = nb.compile(lambda t, p, i: (lambda rows: (rows, order(rows, p)))(F.embedding(i, t)))
+        for _ in range(2):
+            assert torch.equal(f(tt, pt, it).to_torch(), ref)
+            rows, out = g(tt, pt, it)
+            assert torch.equal(rows.to_torch(), table[idx]) and torch.equal(out.to_torch(), ref)
+        assert ("gather_add" in f.dump_plan()) == fused and "gather_add" not in g.dump_plan()
+
+
 @pytest.mark.parametrize("vocab,dim,n,dtype,atomics", [
     (16, 8, 1000, 1, True), (4096, 2048, 12288, 1, True), (4097, 2048, 100, 1, False), (4096, 2048, 12289, 1, False), (1000, 64, 49152, 0, True),
     (1000, 64, 49153, 0, False), (256, 64, 100000, 0, True), (256, 64, 131073, 0, False), (9000, 1001, 700, 1, True), (32000, 1001, 700, 1, False),
