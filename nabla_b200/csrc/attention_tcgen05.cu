@@ -272,7 +272,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp < 4) {
   if (MASK == MASK_KEYS) service_registers();
   if (warp == 0) {
-    if (lane == 0 && n_max > 0) {
+    if (n_max > 0 && elect_one()) {
       for (int t = 0; t < 2; ++t) {
         if (n_t[t] == 0) continue;
         mbar_arrive_expect_tx(&q_full[t], L::TILE_BYTES);
@@ -296,7 +296,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_max > 0) {
+    if (n_max > 0 && elect_one()) {
       bool ok = true;
       auto qk = [&](int t, int j) {
         mma_scores<HD>(tmem_base + t * BT, smem_u32(sQ + t * L::TILE_BYTES), smem_u32(sK + (j & 1) * L::TILE_BYTES));
@@ -845,7 +845,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t t_st = tmem_base, t_dpt = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 256 + HD;
 
   if (warp == 0) {
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       mbar_arrive_expect_tx(kv_full, 2 * L::TILE_BYTES);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c) {
@@ -872,7 +872,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       bool ok = mbar_wait(kv_full, 0) && mbar_wait(&q_full[0], 0);
       if (ok) {
         tc_fence_after();
@@ -1149,7 +1149,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t t_dp = tmem_base + 256, t_dq = tmem_base + 384;   // S buffers at 0 and 128
 
   if (warp == 0) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && elect_one()) {
       mbar_arrive_expect_tx(qdo_full, 2 * L::TILE_BYTES);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c) {
@@ -1171,7 +1171,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && elect_one()) {
       auto scores = [&](int j) {          // S_j = Q K_j^T into buffer j & 1
         mma_scores<HD>(tmem_base + (j & 1) * BT, smem_u32(sQ), smem_u32(sK + (j % KST) * L::TILE_BYTES));
         umma_commit(&s_full[j & 1]);

@@ -275,7 +275,7 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -381,7 +381,7 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
     // ------------------------------------------------------------ MMA issuer
     if (PAIR && !leader) {
       // the other CTA of the pair issues nothing: the leader's thread drives both tensor cores
-    } else if (lane == 0) {
+    } else if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(TILE_M, BN, args.a_mn, args.b_mn);
       // Per-operand descriptor constants.
       const uint32_t a_lbo = args.a_mn ? BLOCK_K * 128 : 16, a_sbo = 1024;
