@@ -35,6 +35,20 @@
 namespace nba {
 using namespace nb;
 
+// named_bar_sync whose threads also learn whether `any` holds in one of them.
+__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool any) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %3, 0;\n\t"
+      "barrier.cta.red.or.pred p, %1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"(nthreads), "r"((uint32_t)any)
+      : "memory");
+  return r != 0;
+}
+
 constexpr int BT = 128;          // tile edge, queries and keys
 constexpr int NTHREADS = 384;
 constexpr float LOG2E = 1.4426950408889634f;
@@ -104,6 +118,21 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 __device__ __forceinline__ float2 f2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
 
+// 32 values of a row times `mul` as bf16. vec32: the address is 32-byte aligned, and a lane writes whole sectors (in
+// 16-byte pieces of 32 different rows the end of a dK / dV block took 5200 clocks, 3000 this way).
+__device__ __forceinline__ void store_row32(__nv_bfloat16* p, const uint32_t (&v)[32], float mul, int vec32) {
+  uint32_t w[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) w[e] = pack_bf16(__uint_as_float(v[2 * e]) * mul, __uint_as_float(v[2 * e + 1]) * mul);
+  if (vec32) {
+    st_global_v8(p, w);
+    st_global_v8(p + 16, w + 8);
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) reinterpret_cast<uint4*>(p)[u] = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
+  }
+}
+
 // D[128 x 128] = A[128 x HD] B[128 x HD]^T : both operands K-major tiles of HD / 64 swizzled chunks.
 template <int HD>
 __device__ __forceinline__ void mma_scores(uint32_t d_tmem, uint32_t a0, uint32_t b0) {
@@ -163,6 +192,7 @@ struct FwdArgs {
   float* lse;                   // [B][H][Sq]
   MaskArg mask;
   int* status;
+  int vec32;                    // rows of O start on 32-byte boundaries
   int bh_chunk;                 // see tile_order
   int nsplit;                   // the keys are cut into this many ranges, one CTA each (1: no split)
   float* part_o;                // nsplit > 1: [nsplit][B][H][Sq][HD] output over each range, fp32
@@ -178,7 +208,7 @@ struct FwdSmem {
   static constexpr int OFF_MASK = OFF_V + 2 * TILE_BYTES;  // key mask: [2 math groups][2][128] values of a key tile. Not for
   static constexpr int OFF_BAR = OFF_MASK + (KEYS ? 4 * BT * 4 : 0);   // the others: at 196 KB (head_dim 128) the 2 KB cost
                                                            // half of the L1 that holds a row mask's lines
-  static constexpr int RAW = OFF_BAR + 18 * 8 + 16 + 1024;
+  static constexpr int RAW = OFF_BAR + 20 * 8 + 16 + 1024;
   static constexpr int TOTAL = RAW < 120 * 1024 ? 120 * 1024 : RAW;   // one CTA per SM (it takes all of TMEM)
 };
 static_assert(FwdSmem<128, false>::TOTAL + 1024 <= 196 * 1024, "with a row mask or none 60 KB of L1 are left");
@@ -190,11 +220,16 @@ static_assert(FwdSmem<128, false>::TOTAL + 1024 <= 196 * 1024, "with a row mask 
 // MASK_ROWS: a mask row per query, 128 loads per thread and key tile. They are added in the pass that hides keys, the
 // kernel otherwise that without a mask: with the scores in registers fewer of those loads are in flight
 // (96 x 777 x 64: 243 us that way, 212 this way; 16 heads x 300 x 128: 74 and 47, the L1 space included).
+// SPARE (head_dim 64 but for MASK_ROWS): the two outputs take 128 columns of tensor memory, which leaves 128 of the 512 for
+// the probabilities. A tile's scores are read into registers at once and the next key tile's QK^T overwrites them while
+// the exponentials run, so the softmax does not wait for a product.
 template <int HD, UserMask MASK>
 __global__ void __launch_bounds__(NTHREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs args) {
   using L = FwdSmem<HD, MASK == MASK_KEYS>;
+  constexpr bool SPARE = HD == 64 && MASK != MASK_ROWS;
+  constexpr bool REGS = SPARE || MASK == MASK_KEYS;      // a row's 128 scores stay in registers
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::OFF_Q;
@@ -208,8 +243,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* v_empty = bars + 8;    // [2]
   uint64_t* s_full = bars + 10;    // [2] per query tile: scores of the next key tile are in TMEM
   uint64_t* p_full = bars + 12;    // [2] per query tile: probabilities are in TMEM (128 arrivals)
-  uint64_t* o_done = bars + 14;    // [2] per query tile: last PV product has retired
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* o_done = bars + 14;    // [2] per query tile: last PV product has retired (SPARE: every PV product)
+  uint64_t* s_read = bars + 16;    // [2] per query tile, SPARE: scores are in registers (128 arrivals)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
@@ -249,12 +285,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int i = 0; i < 2; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
+      mbar_init(&k_empty[i], SPARE ? 2 : 1);       // SPARE: one arrival per query tile
       mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
+      mbar_init(&v_empty[i], SPARE ? 2 : 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 128);
       mbar_init(&o_done[i], 1);
+      mbar_init(&s_read[i], 128);
     }
     fence_mbar_init();
     fence_proxy_async_smem();
@@ -267,10 +304,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // tile t: scores (and P over their first 64 columns) at t * 128, output accumulator at 256 + t * HD
+  // tile t: scores (and P over their first 64 columns) at t * 128, output accumulator at 256 + t * HD; SPARE: P at 384 + t * 64
 
   if (warp < 4) {
-  if (MASK == MASK_KEYS) service_registers();
+  if (REGS) service_registers();
   if (warp == 0) {
     if (n_max > 0 && elect_one()) {
       for (int t = 0; t < 2; ++t) {
@@ -294,6 +331,43 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int c = 0; c < HD / 64; ++c)
           tma_load_4d(sV + st * L::TILE_BYTES + c * (BT * 128), &tmV, &v_full[st], c * 64, (kt0 + j) * BT, h, b, args.Skv, args.H, args.B);
       }
+    }
+  } else if (SPARE) {
+    // warps 1 and 3 issue for one query tile each, so that neither group's softmax waits for the other's
+    const int t = warp >> 1;
+    if (warp != 2 && n_max > 0 && elect_one()) {
+      bool ok = n_t[t] == 0 || mbar_wait(&q_full[t], 0);
+      for (int j = 0; j <= n_max && ok; ++j) {
+        if (j < n_max) {                   // scores of key tile j, as soon as those before are in registers
+          const int st = j & 1;
+          ok = mbar_wait(&k_full[st], (j >> 1) & 1);
+          if (ok && j < n_t[t]) {
+            ok = j == 0 || mbar_wait(&s_read[t], (j - 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            mma_scores<HD>(tmem_base + t * BT, smem_u32(sQ + t * L::TILE_BYTES), smem_u32(sK + st * L::TILE_BYTES));
+            umma_commit(&s_full[t]);
+            umma_commit(&k_empty[st]);
+          } else if (ok) {
+            mbar_arrive(&k_empty[st]);     // this query tile sees no key of the tile
+          }
+        }
+        if (ok && j > 0) {                 // PV of key tile j - 1
+          const int i = j - 1, st = i & 1;
+          ok = mbar_wait(&v_full[st], (i >> 1) & 1);
+          if (ok && i < n_t[t]) {
+            ok = mbar_wait(&p_full[t], i & 1);
+            if (!ok) break;
+            tc_fence_after();
+            mma_accum<HD>(tmem_base + 256 + t * HD, tmem_base + 384 + t * 64, false, smem_u32(sV + st * L::TILE_BYTES), i != 0);
+            umma_commit(&o_done[t]);
+            umma_commit(&v_empty[st]);
+          } else if (ok) {
+            mbar_arrive(&v_empty[st]);
+          }
+        }
+      }
+      if (!ok) atomicExch(args.status, NB_ERR_TIMEOUT_MMA);
     }
   } else if (warp == 1) {
     if (n_max > 0 && elect_one()) {
@@ -336,7 +410,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   }
   } else {
-    if (MASK == MASK_KEYS) math_registers();
+    if (REGS) math_registers();
     const int t = (warp - 4) >> 2;          // query tile of this math group
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
@@ -345,6 +419,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_addr = static_cast<uint32_t>(wq * 32) << 16;
     const uint32_t t_s = tmem_base + t * BT + lane_addr;
     const uint32_t t_o = tmem_base + 256 + t * HD + lane_addr;
+    const uint32_t t_p = SPARE ? tmem_base + 384 + t * 64 + lane_addr : t_s;
     // user mask: one row for all queries (padding masks) goes through shared memory, 128 coalesced values
     // per key tile; a row per query is read by its own thread
     const float* mrow = nullptr;
@@ -359,9 +434,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     bool ok = true;
     for (int j = 0; j < n; ++j) {
       const int kv0 = (kt0 + j) * BT;
+      bool masked = false;                 // a tile whose 128 mask values are all zero (most of a padded batch) adds nothing
       if (mshared) {
         smask[(j & 1) * BT + r] = mnext;
-        named_bar_sync(2 + t, 128);
+        masked = named_bar_or(2 + t, 128, mnext != 0.f);
         mnext = j + 1 < n && kv0 + BT + r < args.Skv ? mrow[kv0 + BT + r] : 0.f;
       }
       if (ok && !mbar_wait(&s_full[t], j & 1)) {
@@ -376,24 +452,36 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       const bool edge = kv0 + BT > args.Skv || (args.causal && kv0 + BT - 1 > q0 + t * BT + off);
       float mxa[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      uint32_t v4[mshared ? 4 : 2][32];  // key mask: the row's 128 scores; else two chunks of 32, one of them in flight
-      if constexpr (mshared) {
+      uint32_t v4[REGS ? 4 : 2][32];     // the row's 128 scores, or two chunks of 32, one of them in flight
+      if constexpr (REGS) {
         auto& v = v4;
-        // the load of the next 32 columns runs under the work on the current ones
-        tmem_ld_32x32(t_s, v[0]);
+        if constexpr (SPARE) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld_wait32(v[c]);
+          tc_fence_before();
+          mbar_arrive(&s_read[t]);
+        } else {
+          tmem_ld_32x32(t_s, v[0]);        // the load of the next 32 columns runs under the work on the current ones
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          tmem_ld_wait32(v[c]);
-          if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, v[c + 1]);
-          const float4* m4 = reinterpret_cast<const float4*>(smask + (j & 1) * BT + c * 32);
+          if constexpr (!SPARE) {
+            tmem_ld_wait32(v[c]);
+            if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, v[c + 1]);
+          }
+          if (mshared && masked) {
+            const float4* m4 = reinterpret_cast<const float4*>(smask + (j & 1) * BT + c * 32);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 mv = m4[i];
-            uint32_t* w = &v[c][i * 4];
-            w[0] = __float_as_uint(fmaf(mv.x, mask_mul, __uint_as_float(w[0])));
-            w[1] = __float_as_uint(fmaf(mv.y, mask_mul, __uint_as_float(w[1])));
-            w[2] = __float_as_uint(fmaf(mv.z, mask_mul, __uint_as_float(w[2])));
-            w[3] = __float_as_uint(fmaf(mv.w, mask_mul, __uint_as_float(w[3])));
+            for (int i = 0; i < 8; ++i) {
+              const float4 mv = m4[i];
+              uint32_t* w = &v[c][i * 4];
+              w[0] = __float_as_uint(fmaf(mv.x, mask_mul, __uint_as_float(w[0])));
+              w[1] = __float_as_uint(fmaf(mv.y, mask_mul, __uint_as_float(w[1])));
+              w[2] = __float_as_uint(fmaf(mv.z, mask_mul, __uint_as_float(w[2])));
+              w[3] = __float_as_uint(fmaf(mv.w, mask_mul, __uint_as_float(w[3])));
+            }
           }
           if (edge) {
             // diagonal or tail tile: -inf where a key is not visible
@@ -453,8 +541,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         resc = true;
       }
       const float m_sub = m_used == -INFINITY ? 0.f : m_used;
+      if (SPARE && j > 0) {
+        // the previous PV product has read P and written O
+        if (!mbar_wait(&o_done[t], (j - 1) & 1)) {
+          atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (mshared) continue;
+          break;
+        }
+        tc_fence_after();
+      }
       if (__any_sync(0xffffffffu, resc)) {
-        // s_full of this tile also tracks the previous PV product: O is not being written now
+        // O is not being written now (without SPARE s_full of this tile also tracks the previous PV product)
 #pragma unroll 1
         for (int c = 0; c < HD / 32; ++c) {
           uint32_t o[32];
@@ -471,8 +572,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
       for (int c = 0; c < BT / 32; ++c) {
-        uint32_t (&v)[32] = v4[mshared ? c : c & 1];
-        if constexpr (!mshared) {
+        uint32_t (&v)[32] = v4[REGS ? c : c & 1];
+        if constexpr (!REGS) {
           tmem_ld_wait32(v);
           if (c + 1 < BT / 32) tmem_ld_32x32(t_s + (c + 1) * 32, v4[(c + 1) & 1]);
         }
@@ -484,7 +585,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           acc[i & 1] = __fadd2_rn(acc[i & 1], pr);
           pk[i] = pack_bf16(pr.x, pr.y);
         }
-        tmem_st_32x16(t_s + c * 16, pk);
+        tmem_st_32x16(t_p + c * 16, pk);
       }
       const float sum = (acc[0].x + acc[0].y) + (acc[1].x + acc[1].y);
       l = l * alpha + sum;
@@ -493,7 +594,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_arrive(&p_full[t]);
     }
     if (ok && n > 0) {
-      if (!mbar_wait(&o_done[t], 0)) {
+      if (!mbar_wait(&o_done[t], SPARE ? (n - 1) & 1 : 0)) {
         atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
         ok = false;
       }
@@ -521,15 +622,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             prow[u] = make_float4(__uint_as_float(v[4 * u]) * inv, __uint_as_float(v[4 * u + 1]) * inv,
                                   __uint_as_float(v[4 * u + 2]) * inv, __uint_as_float(v[4 * u + 3]) * inv);
         } else if (q_idx < args.Sq) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 pk;
-            uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              pw[e] = pack_bf16(__uint_as_float(v[u * 8 + 2 * e]) * inv, __uint_as_float(v[u * 8 + 2 * e + 1]) * inv);
-            *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = pk;
-          }
+          store_row32(orow + c * 32, v, inv, args.vec32);
         }
       }
       if (q_idx < args.Sq) {
@@ -742,6 +835,7 @@ struct BwdArgs {
   long long dq_sb, dq_sh, dq_ss, dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
   MaskArg mask;
   int* status;
+  int vec32;               // rows of dQ, dK and dV start on 32-byte boundaries
   int q_chunk, kv_chunk;   // see tile_order: of the dK / dV kernel (Q and dO shared) and of the dQ kernel (K and V)
 };
 
@@ -762,6 +856,12 @@ struct DkvSmem {
   static constexpr int TOTAL = RAW < 120 * 1024 ? 120 * 1024 : RAW;
 };
 
+// Tensor memory: dV, dK and NREG regions of 128 columns (three where head_dim 64 leaves room, else two), which S^T and dP^T
+// of the tiles take in turn. P^T and dS^T (bf16, 32 columns each per group) go over the score columns that their own threads
+// have read. So a region that held dP^T is free once that is in registers: S^T of the next tile is multiplied while dS^T is
+// made (three regions: from when P^T is written); dP^T of the next tile follows dK in the issue order and is ready before
+// its exponentials are. With S^T and dP^T in fixed places a thread waited 1700 of 4050 clocks per tile for
+// scores, 850 of 3250 this way (64 heads x 2048 x 128, causal: dK and dV 177 -> 149 us, with the 32-byte stores).
 template <int HD, UserMask MASK>
 __global__ void __launch_bounds__(NTHREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -788,7 +888,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* p_full = bars + 13;    //      P^T written back (256 arrivals)
   uint64_t* ds_full = bars + 14;   //      dS^T written back (256 arrivals)
   uint64_t* all_done = bars + 15;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* dp_read = bars + 16;   //      two regions: dP^T of the current tile is in registers (256 arrivals)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
@@ -831,6 +932,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(p_full, 256);
     mbar_init(ds_full, 256);
     mbar_init(all_done, 1);
+    mbar_init(dp_read, 256);
     fence_mbar_init();
     fence_proxy_async_smem();
   }
@@ -842,7 +944,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t t_st = tmem_base, t_dpt = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 256 + HD;
+  constexpr int NREG = HD == 64 ? 3 : 2;
+  const uint32_t t_dv = tmem_base + NREG * 128, t_dk = t_dv + HD;
+  auto t_s = [&](int it) { return tmem_base + (NREG == 3 ? 2 * it % 3 : it & 1) * 128; };            // S^T of tile it
+  auto t_dp = [&](int it) { return tmem_base + (NREG == 3 ? (2 * it + 1) % 3 : (it + 1) & 1) * 128; };
 
   if (warp == 0) {
     if (n_it > 0 && elect_one()) {
@@ -876,36 +981,40 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       bool ok = mbar_wait(kv_full, 0) && mbar_wait(&q_full[0], 0);
       if (ok) {
         tc_fence_after();
-        mma_scores<HD>(t_st, smem_u32(sK), smem_u32(sQ));            // S^T_0 = K Q_0^T
+        mma_scores<HD>(t_s(0), smem_u32(sK), smem_u32(sQ));          // S^T_0 = K Q_0^T
         umma_commit(s_full);
         ok = mbar_wait(&do_full[0], 0);
       }
       if (ok) {
         tc_fence_after();
-        mma_scores<HD>(t_dpt, smem_u32(sV), smem_u32(sDO));          // dP^T_0 = V dO_0^T
+        mma_scores<HD>(t_dp(0), smem_u32(sV), smem_u32(sDO));        // dP^T_0 = V dO_0^T
         umma_commit(dp_full);
       }
       for (int it = 0; it < n_it && ok; ++it) {
         const int st = it & 1, qs = it % QST, qn = (it + 1) % QST;
         const bool more = it + 1 < n_it;
-        if (!mbar_wait(p_full, it & 1)) { ok = false; break; }
-        tc_fence_after();
-        mma_accum<HD>(t_dv, t_st, true, smem_u32(sDO + st * L::TILE_BYTES), it != 0);     // dV += P^T dO_i
-        umma_commit(&do_empty[st]);
+        // Scores of the next tile: their region held dP^T of this tile (two regions: once all threads have read it) or of
+        // the one before (three: once all have written P^T, so that none can arrive a second time on a barrier where
+        // another has yet to arrive)
+        if (NREG == 3 && !mbar_wait(p_full, it & 1)) { ok = false; break; }
         if (more) {
-          if (!mbar_wait(&q_full[qn], ((it + 1) / QST) & 1)) { ok = false; break; }
+          if (!(mbar_wait(&q_full[qn], ((it + 1) / QST) & 1) && (NREG == 3 || mbar_wait(dp_read, it & 1)))) { ok = false; break; }
           tc_fence_after();
-          mma_scores<HD>(t_st, smem_u32(sK), smem_u32(sQ + qn * L::TILE_BYTES));
+          mma_scores<HD>(t_s(it + 1), smem_u32(sK), smem_u32(sQ + qn * L::TILE_BYTES));
           umma_commit(s_full);
         }
+        if (NREG == 2 && !mbar_wait(p_full, it & 1)) { ok = false; break; }
+        tc_fence_after();
+        mma_accum<HD>(t_dv, t_s(it), true, smem_u32(sDO + st * L::TILE_BYTES), it != 0);         // dV += P^T dO_i
+        umma_commit(&do_empty[st]);
         if (!mbar_wait(ds_full, it & 1)) { ok = false; break; }
         tc_fence_after();
-        mma_accum<HD>(t_dk, t_dpt, true, smem_u32(sQ + qs * L::TILE_BYTES), it != 0);     // dK += dS^T Q_i
+        mma_accum<HD>(t_dk, t_s(it) + 32, true, smem_u32(sQ + qs * L::TILE_BYTES), it != 0);     // dK += dS^T Q_i
         umma_commit(&q_empty[qs]);
         if (more) {
           if (!mbar_wait(&do_full[st ^ 1], ((it + 1) >> 1) & 1)) { ok = false; break; }
           tc_fence_after();
-          mma_scores<HD>(t_dpt, smem_u32(sV), smem_u32(sDO + (st ^ 1) * L::TILE_BYTES));
+          mma_scores<HD>(t_dp(it + 1), smem_u32(sV), smem_u32(sDO + (st ^ 1) * L::TILE_BYTES));
           umma_commit(dp_full);
         }
       }
@@ -919,7 +1028,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int key = k0 + r;
     const bool key_ok = key < args.Skv;
     const uint32_t lane_addr = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t a_s = t_st + lane_addr + grp * 64, a_dp = t_dpt + lane_addr + grp * 64;
     const float* mbase = MASK == MASK_NONE ? nullptr : args.mask.ptr + b * args.mask.sb + h * args.mask.sh + key;
     // a mask with one row for all queries is one number per key here: added on the way into the exponent, no mask
     // pass, with the forward's roundings ((s + mask / scale) * scale_log2 - lse: where all keys of a row share
@@ -932,16 +1040,18 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     for (int it = 0; it < n_it; ++it) {
       const int st = it & 1, qs = it % QST;
       const int q0 = (i_start + it) * BT + grp * 64;
-      if (ok && !(mbar_wait(&q_full[qs], (it / QST) & 1) && mbar_wait(s_full, it & 1))) {
+      // (dO and its delta have landed by the time the scores are there)
+      if (ok && !(mbar_wait(&q_full[qs], (it / QST) & 1) && mbar_wait(&do_full[st], (it >> 1) & 1) && mbar_wait(s_full, it & 1))) {
         atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
         ok = false;
       }
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
+      const uint32_t a_s = t_s(it) + lane_addr + grp * 64, a_dp = t_dp(it) + lane_addr + grp * 64;
       const bool general = (args.causal && (k0 + BT - 1 > q0 + off)) || (k0 + BT > args.Skv) || MASK == MASK_ROWS;
-      if (general) {
-        // masked tile: rewrite S^T in place with -inf where (key, query) is not visible
+      if (MASK == MASK_ROWS) {
+        // rewrite S^T in place with the mask, -inf where (key, query) is not visible
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
           uint32_t v[32];
@@ -951,8 +1061,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int i = 0; i < 32; ++i) {
             const int q = q0 + c * 32 + i;
             float x = __uint_as_float(v[i]);
-            if (mkey) x = fmaf(mval, mask_mul, x);
-            if (MASK == MASK_ROWS && key_ok && q < args.Sq) x = fmaf(mbase[(long long)q * args.mask.sq], mask_mul, x);
+            if (key_ok && q < args.Sq) x = fmaf(mbase[(long long)q * args.mask.sq], mask_mul, x);
             if (!key_ok || (args.causal && key > q + off)) x = -INFINITY;
             v[i] = __float_as_uint(x);
           }
@@ -965,11 +1074,27 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       float2 p[32];
       uint32_t va[32], vb[32];
       tmem_ld_32x32(a_s, va);
+      tmem_ld_32x32(a_s + 32, vb);
+      tmem_ld_wait32(va);
+      tmem_ld_wait32(vb);
+      if (MASK != MASK_ROWS && general) {
+        // diagonal or tail tile: -inf below the first query of this group that sees the key (one bound, so that the
+        // compiler selects; two conditions per element became branches, 3400 clocks a tile)
+        const int first = !key_ok ? 64 : args.causal ? key - off - q0 : 0;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t (&v)[32] = c ? vb : va;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            float x = __uint_as_float(v[i]);
+            if (mkey) x = fmaf(mval, mask_mul, x);
+            v[i] = __float_as_uint(c * 32 + i < first ? -INFINITY : x);
+          }
+        }
+      }
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t (&v)[32] = c ? vb : va;
-        tmem_ld_wait32(v);
-        if (c == 0) tmem_ld_32x32(a_s + 32, vb);
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -984,7 +1109,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(p_full);
-      if (!(mbar_wait(&do_full[st], (it >> 1) & 1) && mbar_wait(dp_full, it & 1))) {
+      if (!mbar_wait(dp_full, it & 1)) {
         atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
         ok = false;
       }
@@ -993,11 +1118,16 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_after();
       const float2* nd2 = reinterpret_cast<const float2*>(s_ndelta + st * BT + grp * 64);
       tmem_ld_32x32(a_dp, va);
+      tmem_ld_32x32(a_dp + 32, vb);
+      tmem_ld_wait32(va);
+      tmem_ld_wait32(vb);
+      if (NREG == 2) {
+        tc_fence_before();
+        mbar_arrive(dp_read);
+      }
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t (&v)[32] = c ? vb : va;
-        tmem_ld_wait32(v);
-        if (c == 0) tmem_ld_32x32(a_dp + 32, vb);
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -1005,7 +1135,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const float2 d = __fmul2_rn(p[c * 16 + i], __fadd2_rn(f2(v[2 * i], v[2 * i + 1]), nd2[c * 16 + i]));
           pk[i] = pack_bf16(d.x, d.y);
         }
-        tmem_st_32x16(a_dp + c * 16, pk);
+        tmem_st_32x16(a_s + 32 + c * 16, pk);
       }
       tmem_st_wait();
       tc_fence_before();
@@ -1037,15 +1167,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
         if (key_ok) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 pk;
-            uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              pw[e] = pack_bf16(__uint_as_float(v[u * 8 + 2 * e]) * mul, __uint_as_float(v[u * 8 + 2 * e + 1]) * mul);
-            *reinterpret_cast<uint4*>(dst + c * 32 + u * 8) = pk;
-          }
+          store_row32(dst + c * 32, v, mul, args.vec32);
         }
       }
     }
@@ -1070,10 +1192,13 @@ struct DqSmem {
   static constexpr int OFF_V = OFF_K + KST * TILE_BYTES;    // 2 stages
   static constexpr int OFF_MASK = OFF_V + 2 * TILE_BYTES;   // [2 math groups][2][64] mask values of a key tile
   static constexpr int OFF_BAR = OFF_MASK + 4 * 64 * 4;
-  static constexpr int RAW = OFF_BAR + 18 * 8 + 16 + 1024;
+  static constexpr int RAW = OFF_BAR + 21 * 8 + 16 + 1024;
   static constexpr int TOTAL = RAW < 120 * 1024 ? 120 * 1024 : RAW;
 };
 
+// dS goes over the score columns that its own threads have read, so dP of the next tile needs its region only after dP was
+// read, and S of the tile after next follows dQ in the issue order: with dS over dP a thread waited 1200 of 3100 clocks per
+// tile for scores, 300 of 2190 this way (64 heads x 2048 x 128, causal: 127 -> 111 us).
 template <int HD, UserMask MASK>
 __global__ void __launch_bounds__(NTHREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -1088,16 +1213,19 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint8_t* sK = smem + L::OFF_K;
   uint8_t* sV = smem + L::OFF_V;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* qdo_full = bars + 0;
+  uint64_t* q_full = bars + 0;
   uint64_t* k_full = bars + 1;     // [3]
   uint64_t* k_empty = bars + 4;    // [3]
   uint64_t* v_full = bars + 7;     // [2]
   uint64_t* v_empty = bars + 9;    // [2]
   uint64_t* s_full = bars + 11;    // [2]  score buffer j & 1 holds S_j
   uint64_t* dp_full = bars + 13;   //      dP_j is in TMEM
-  uint64_t* ds_full = bars + 14;   //      dS_j written back (256 arrivals)
+  uint64_t* ds_full = bars + 18;   // [2]  dS_j written back (256 arrivals); two, because dP_j+1 may let a thread come here again
+                                   //      before another has arrived for dS_j
   uint64_t* dq_done = bars + 15;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* dp_read = bars + 16;   //      dP_j is in registers (256 arrivals)
+  uint64_t* do_full = bars + 17;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
@@ -1122,7 +1250,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
-    mbar_init(qdo_full, 1);
+    mbar_init(q_full, 1);
+    mbar_init(do_full, 1);
     for (int i = 0; i < KST; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_empty[i], 1);
@@ -1133,8 +1262,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(&s_full[i], 1);
     }
     mbar_init(dp_full, 1);
-    mbar_init(ds_full, 256);
+    mbar_init(&ds_full[0], 256);
+    mbar_init(&ds_full[1], 256);
     mbar_init(dq_done, 1);
+    mbar_init(dp_read, 256);
     fence_mbar_init();
     fence_proxy_async_smem();
   }
@@ -1150,12 +1281,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 0) {
     if (n > 0 && elect_one()) {
-      mbar_arrive_expect_tx(qdo_full, 2 * L::TILE_BYTES);
+      mbar_arrive_expect_tx(q_full, L::TILE_BYTES);
 #pragma unroll
-      for (int c = 0; c < HD / 64; ++c) {
-        tma_load_4d(sQ + c * (BT * 128), &tmQ, qdo_full, c * 64, q0, h, b, args.Sq, args.H, args.B);
-        tma_load_4d(sDO + c * (BT * 128), &tmDO, qdo_full, c * 64, q0, h, b, args.Sq, args.H, args.B);
-      }
+      for (int c = 0; c < HD / 64; ++c)
+        tma_load_4d(sQ + c * (BT * 128), &tmQ, q_full, c * 64, q0, h, b, args.Sq, args.H, args.B);
       for (int j = 0; j < n; ++j) {
         const int ks = j % KST, vs = j & 1;
         if (!mbar_wait(&k_empty[ks], ((j / KST) & 1) ^ 1)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
@@ -1163,6 +1292,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
           tma_load_4d(sK + ks * L::TILE_BYTES + c * (BT * 128), &tmK, &k_full[ks], c * 64, j * BT, h, b, args.Skv, args.H, args.B);
+        if (j == 0) {                      // behind Q and K, which the first scores wait for
+          mbar_arrive_expect_tx(do_full, L::TILE_BYTES);
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c)
+            tma_load_4d(sDO + c * (BT * 128), &tmDO, do_full, c * 64, q0, h, b, args.Sq, args.H, args.B);
+        }
         if (!mbar_wait(&v_empty[vs], ((j >> 1) & 1) ^ 1)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
         mbar_arrive_expect_tx(&v_full[vs], L::TILE_BYTES);
 #pragma unroll
@@ -1181,11 +1316,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         umma_commit(dp_full);
         umma_commit(&v_empty[j & 1]);
       };
-      bool ok = mbar_wait(qdo_full, 0) && mbar_wait(&k_full[0], 0);
+      bool ok = mbar_wait(q_full, 0) && mbar_wait(&k_full[0], 0);
       if (ok) {
         tc_fence_after();
         scores(0);
-        ok = mbar_wait(&v_full[0], 0);
+        ok = mbar_wait(do_full, 0) && mbar_wait(&v_full[0], 0);
       }
       if (ok) {
         tc_fence_after();
@@ -1199,15 +1334,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       for (int j = 0; j < n && ok; ++j) {
-        if (!mbar_wait(ds_full, j & 1)) { ok = false; break; }
-        tc_fence_after();
-        mma_accum<HD>(t_dq, t_dp, true, smem_u32(sK + (j % KST) * L::TILE_BYTES), j != 0);   // dQ += dS_j K_j
-        umma_commit(&k_empty[j % KST]);
         if (j + 1 < n) {
-          if (!mbar_wait(&v_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) { ok = false; break; }
+          if (!(mbar_wait(&v_full[(j + 1) & 1], ((j + 1) >> 1) & 1) && mbar_wait(dp_read, j & 1))) { ok = false; break; }
           tc_fence_after();
           dprobs(j + 1);
         }
+        if (!mbar_wait(&ds_full[j & 1], (j >> 1) & 1)) { ok = false; break; }
+        tc_fence_after();
+        mma_accum<HD>(t_dq, tmem_base + (j & 1) * BT, true, smem_u32(sK + (j % KST) * L::TILE_BYTES), j != 0);   // dQ += dS_j K_j
+        umma_commit(&k_empty[j % KST]);
         if (j + 2 < n) {
           if (!mbar_wait(&k_full[(j + 2) % KST], ((j + 2) / KST) & 1)) { ok = false; break; }
           tc_fence_after();
@@ -1244,9 +1379,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     bool ok = true;
     for (int j = 0; j < n; ++j) {
       const int kv0 = j * BT + grp * 64;
+      bool masked = false;
       if (mkey) {
         if (r < 64) smask[(j & 1) * 64 + r] = mnext;
-        named_bar_sync(2 + grp, 128);
+        masked = named_bar_or(2 + grp, 128, mnext != 0.f);
         mnext = j + 1 < n && r < 64 && kv0 + BT + r < args.Skv ? mkeys[kv0 + BT + r] : 0.f;
       }
       if (ok && !mbar_wait(&s_full[j & 1], (j >> 1) & 1)) {
@@ -1261,8 +1397,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_after();
       const bool general = (kv0 + 64 > args.Skv) || (args.causal && (kv0 + 63 > q0 + off)) || MASK == MASK_ROWS;
       const uint32_t a_s = tmem_base + (j & 1) * BT + lane_addr + grp * 64;
-      if (general) {
-        // masked tile: rewrite the scores in place with -inf where the key is not visible
+      if (MASK == MASK_ROWS) {
+        // rewrite the scores in place with the mask, -inf where the key is not visible
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
           uint32_t v[32];
@@ -1272,8 +1408,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int i = 0; i < 32; ++i) {
             const int kc = kv0 + c * 32 + i;
             float x = __uint_as_float(v[i]);
-            if (mkey) x = fmaf(smask[(j & 1) * 64 + c * 32 + i], mask_mul, x);
-            if (MASK == MASK_ROWS && mrow != nullptr && kc < args.Skv) x = fmaf(mrow[kc], mask_mul, x);
+            if (mrow != nullptr && kc < args.Skv) x = fmaf(mrow[kc], mask_mul, x);
             v[i] = __float_as_uint(kc <= lim ? x : -INFINITY);
           }
           tmem_st_32x32(a_s + c * 32, v);
@@ -1284,15 +1419,37 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       float2 p[32];
       uint32_t va[32], vb[32];
       tmem_ld_32x32(a_s, va);
+      tmem_ld_32x32(a_s + 32, vb);
+      tmem_ld_wait32(va);
+      tmem_ld_wait32(vb);
+      if (mkey && masked) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t (&v)[32] = c ? vb : va;
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float2 x = __ffma2_rn(*reinterpret_cast<const float2*>(smask + (j & 1) * 64 + c * 32 + i), mul2, f2(v[i], v[i + 1]));
+            v[i] = __float_as_uint(x.x);
+            v[i + 1] = __float_as_uint(x.y);
+          }
+        }
+      }
+      if (MASK != MASK_ROWS && general) {
+        // diagonal or tail tile: -inf where the key is not visible
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t (&v)[32] = c ? vb : va;
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i > lim - kv0) v[i] = __float_as_uint(-INFINITY);
+        }
+      }
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t (&v)[32] = c ? vb : va;
-        tmem_ld_wait32(v);
-        if (c == 0) tmem_ld_32x32(a_s + 32, vb);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float2 x = f2(v[2 * i], v[2 * i + 1]);
-          if (mkey && !general) x = __ffma2_rn(*reinterpret_cast<const float2*>(smask + (j & 1) * 64 + c * 32 + 2 * i), mul2, x);
           x = __ffma2_rn(x, sc2, nl2);
           p[c * 16 + i] = make_float2(ex2(x.x), ex2(x.y));
         }
@@ -1309,11 +1466,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_after();
       const float2 nd2 = make_float2(ndelta, ndelta);
       tmem_ld_32x32(a_dp, va);
+      tmem_ld_32x32(a_dp + 32, vb);
+      tmem_ld_wait32(va);
+      tmem_ld_wait32(vb);
+      tc_fence_before();
+      mbar_arrive(dp_read);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t (&v)[32] = c ? vb : va;
-        tmem_ld_wait32(v);
-        if (c == 0) tmem_ld_32x32(a_dp + 32, vb);
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -1321,11 +1481,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const float2 d = __fmul2_rn(p[c * 16 + i], __fadd2_rn(f2(v[2 * i], v[2 * i + 1]), nd2));
           pk[i] = pack_bf16(d.x, d.y);
         }
-        tmem_st_32x16(a_dp + c * 16, pk);
+        tmem_st_32x16(a_s + c * 16, pk);
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(ds_full);
+      mbar_arrive(&ds_full[j & 1]);
     }
     if (ok && n > 0) {
       if (!mbar_wait(dq_done, 0)) {
@@ -1351,15 +1511,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
         if (q_idx < args.Sq) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 pk;
-            uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              pw[e] = pack_bf16(__uint_as_float(v[u * 8 + 2 * e]) * args.scale, __uint_as_float(v[u * 8 + 2 * e + 1]) * args.scale);
-            *reinterpret_cast<uint4*>(dst + c * 32 + u * 8) = pk;
-          }
+          store_row32(dst + c * 32, v, args.scale, args.vec32);
         }
       }
     }
@@ -1375,43 +1527,50 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
 // ndelta[b][h][q] = -sum_d dO * O and nlse2 = -lse * log2(e), both padded to Sq_pad rows per
 // (b, h): padding rows and rows whose lse is -inf (no visible key) get nlse2 = -inf (probability 0)
-// and ndelta = 0. D / 8 lanes per row, 16-byte loads.
+// and ndelta = 0. D / 8 lanes per row, 16-byte loads, PREP_U rows per group of lanes on their way; a block's rows lie in
+// one (b, h) (they divide a tile of 128), so there is one division per block. 64 heads x 2048 x 128: 21.8 us with a row and two
+// 64-bit divisions per group, 17.8 so.
+constexpr int PREP_U = 4;
+template <int D>
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dO,
                                                            const __nv_bfloat16* __restrict__ O,
                                                            const float* __restrict__ lse, float* __restrict__ ndelta,
-                                                           float* __restrict__ nlse2, int B, int H, int Sq, int Sq_pad, int D,
+                                                           float* __restrict__ nlse2, int H, int Sq, int Sq_pad,
                                                            long long do_sb, long long do_sh, long long do_ss,
                                                            long long o_sb, long long o_sh, long long o_ss) {
-  const int lpr = D / 8;                                  // lanes per row: 16 (D = 128) or 8 (D = 64)
-  const int rows_per_block = 256 / lpr;
-  const long long row = (long long)blockIdx.x * rows_per_block + threadIdx.x / lpr;
-  const int sub = threadIdx.x % lpr;
-  const bool in_range = row < (long long)B * H * Sq_pad;
-  const int q = in_range ? (int)(row % Sq_pad) : 0;
-  const long long bh = in_range ? row / Sq_pad : 0;
-  const int h = bh % H;
-  const int b = bh / H;
-  float acc = 0.f;
-  if (in_range && q < Sq) {
-    const uint4 ra = *reinterpret_cast<const uint4*>(dO + b * do_sb + h * do_sh + q * do_ss + sub * 8);
-    const uint4 rc = *reinterpret_cast<const uint4*>(O + b * o_sb + h * o_sh + q * o_ss + sub * 8);
-    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&ra);
-    const __nv_bfloat162* pc = reinterpret_cast<const __nv_bfloat162*>(&rc);
+  constexpr int LPR = D / 8, RPB = 256 / LPR * PREP_U;    // lanes per row: 16 or 8; rows per block: 64 or 128
+  static_assert(BT % RPB == 0, "a block stays inside a (batch, head)");
+  const int per_bh = Sq_pad / RPB, bh = blockIdx.x / per_bh, q0 = (blockIdx.x - bh * per_bh) * RPB + threadIdx.x / LPR;
+  const int b = bh / H, h = bh - b * H, sub = threadIdx.x % LPR;
+  const __nv_bfloat16* pd = dO + b * do_sb + h * do_sh + sub * 8;
+  const __nv_bfloat16* po = O + b * o_sb + h * o_sh + sub * 8;
+  uint4 ra[PREP_U], rc[PREP_U];
+#pragma unroll
+  for (int u = 0; u < PREP_U; ++u) {
+    const int q = q0 + u * (256 / LPR);
+    ra[u] = rc[u] = make_uint4(0, 0, 0, 0);
+    if (q < Sq) {
+      ra[u] = *reinterpret_cast<const uint4*>(pd + q * do_ss);
+      rc[u] = *reinterpret_cast<const uint4*>(po + q * o_ss);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < PREP_U; ++u) {
+    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&ra[u]);
+    const __nv_bfloat162* pc = reinterpret_cast<const __nv_bfloat162*>(&rc[u]);
+    float acc = 0.f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 x = __bfloat1622float2(pa[e]), y = __bfloat1622float2(pc[e]);
       acc += x.x * y.x + x.y * y.y;
     }
-  }
-  for (int o = lpr / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (in_range && sub == 0) {
-    if (q < Sq) {
-      const float l = lse[bh * Sq + q];
-      ndelta[row] = -acc;
-      nlse2[row] = (l == -INFINITY) ? -INFINITY : -l * LOG2E;
-    } else {
-      ndelta[row] = 0.f;
-      nlse2[row] = -INFINITY;
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const int q = q0 + u * (256 / LPR);
+    if (sub == 0) {
+      const float l = q < Sq ? lse[(long long)bh * Sq + q] : -INFINITY;
+      ndelta[(long long)bh * Sq_pad + q] = q < Sq ? -acc : 0.f;
+      nlse2[(long long)bh * Sq_pad + q] = l == -INFINITY ? -INFINITY : -l * LOG2E;
     }
   }
 }
@@ -1589,6 +1748,7 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   a.lse = lse;
   a.mask = MaskArg{mask, m_sb, m_sh, m_sq};
   a.status = status;
+  a.vec32 = ((reinterpret_cast<uintptr_t>(o) & 31) | ((o_sb | o_sh | o_ss) & 15)) == 0;
   a.bh_chunk = causal ? l2_chunk(B * H, Skv, D) * nsplit : 1;
   a.nsplit = nsplit; a.part_o = part_o; a.part_lse = part_lse;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
@@ -1635,10 +1795,14 @@ extern "C" int nb_attn_bwd(const void* dO, const void* q, const void* k, const v
   const long long rows = (long long)B * H * Sq_pad;
   float* ndelta = stats;
   float* nlse2 = stats + rows;
-  const int rpb = 256 / (D / 8);
-  attn_bwd_prep_kernel<<<(unsigned)((rows + rpb - 1) / rpb), 256, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(dO), reinterpret_cast<const __nv_bfloat16*>(o), lse, ndelta, nlse2, B, H, Sq,
-      Sq_pad, D, do_sb, do_sh, do_ss, o_sb, o_sh, o_ss);
+  const long long prep = rows / (256 / (D / 8) * PREP_U);
+  if (prep > 0x7fffffffll) return -15;
+#define PREP(HD) attn_bwd_prep_kernel<HD><<<(unsigned)prep, 256, 0, s>>>( \
+      reinterpret_cast<const __nv_bfloat16*>(dO), reinterpret_cast<const __nv_bfloat16*>(o), lse, ndelta, nlse2, H, Sq, Sq_pad, \
+      do_sb, do_sh, do_ss, o_sb, o_sh, o_ss)
+  if (D == 128) PREP(128);
+  else PREP(64);
+#undef PREP
   CUtensorMap tq, tk, tv, tdo;
   int r;
   if ((r = make_map4(&tq, q, B, H, Sq, D, q_sb, q_sh, q_ss))) return r;
@@ -1656,6 +1820,8 @@ extern "C" int nb_attn_bwd(const void* dO, const void* q, const void* k, const v
   a.dk_sb = dk_sb; a.dk_sh = dk_sh; a.dk_ss = dk_ss; a.dv_sb = dv_sb; a.dv_sh = dv_sh; a.dv_ss = dv_ss;
   a.mask = MaskArg{mask, m_sb, m_sh, m_sq};
   a.status = status;
+  a.vec32 = (((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 31) |
+             ((dq_sb | dq_sh | dq_ss | dk_sb | dk_sh | dk_ss | dv_sb | dv_sh | dv_ss) & 15)) == 0;
   a.q_chunk = causal ? l2_chunk(B * H, Sq, D) : B * H;
   a.kv_chunk = causal ? l2_chunk(B * H, Skv, D) : 1;
   if (mask == nullptr) return D == 128 ? launch_bwd<128, MASK_NONE>(tq, tk, tv, tdo, a, s) : launch_bwd<64, MASK_NONE>(tq, tk, tv, tdo, a, s);

@@ -182,13 +182,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu_u32(const unsigned* p) {
   return v;
 }
 
-// 32-byte store (one whole sector per lane and instruction; the address must be 32-byte aligned).
-__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-               : "memory");
-}
-
 // One CTA's share of the GEMM. `cta` / `nctas` replace blockIdx / gridDim so that the fused
 // kernel can dedicate some CTAs to communication. Returns false if the CTA left early.
 // PAIR: this CTA is one of a cluster of two (cta_group::2). `cta` / `nctas` then count pairs; a pair

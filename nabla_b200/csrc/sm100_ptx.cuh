@@ -321,6 +321,12 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, int a_mn, i
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// 32-byte store (one whole sector per lane and instruction; the address must be 32-byte aligned).
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 // erf(t) and exp(-t*t) together (Abramowitz & Stegun 7.1.26, |error| < 1.5e-7): one approximate
 // reciprocal, one ex2 and a degree-5 polynomial -- about half the instructions of erff() plus a
 // separate expf(), which matters because the exact-gelu epilogues run on four warps per CTA next
