@@ -24,6 +24,8 @@ CUDA bf16 tensors:
 * ``sum -> sum ...`` over neighbouring axes: one reduction over the joined axes, where ``kernels.joined_sum`` takes it.
 
 Every other node is a plain 'op' step. Fusion never changes which tensors exist: fused-away
+* ``adamw_group``: the updates of small parameters with the same hyperparameters, one launch at the end of a compiled
+  schedule (grouped by ``transforms/compile.py``).
 intermediates that are still referenced are simply not fusable.
 """
 from __future__ import annotations
@@ -574,6 +576,27 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         return
     if kind == "all_reduce_bucket":
         # many small partial sums over the same device group: one flat all-reduce
+    if kind == "adamw_group":
+        from ... import native
+
+        leaves = [[x._buffers[0] for x in n_.input_impls()] for n_ in group]
+        kw = group[0].kwargs
+        outs = None
+        if all(native.use_native(b[0]) for b in leaves):
+            from ...native import kernels
+
+            flags = [bool(n_.kwargs.get("inplace")) and all(t.is_contiguous() for t in (b[0], b[2], b[3])) for n_, b in zip(group, leaves)]
+            corrected = kw.get("bias_correction", True)
+            outs = kernels.adamw_group([(b[0], b[1], b[2], b[3], f) for b, f in zip(leaves, flags)], lr=kw["lr"], b1=kw["beta1"],
+                                       b2=kw["beta2"], eps=kw["eps"], wd=kw["weight_decay"],
+                                       step=kw.get("step_value") if corrected else None,
+                                       hyper=leaves[0][4].contiguous() if len(leaves[0]) > 4 and corrected else None)
+        for n_, o in zip(group, outs if outs is not None else group):
+            if outs is not None:
+                _store(n_, [[t] for t in o], keep_graph)
+            else:
+                _plain(n_, keep_graph)
+        return
         from ...parallel import backend
 
         first = group[0]

@@ -31,6 +31,7 @@ def _L():
             "nb_lse_pick_fwd": [c_vp] * 4 + [c_int, c_int, c_int, c_vp],
             "nb_lse_pick_bwd": [c_vp] * 6 + [c_int, c_int, c_int, c_vp],
             "nb_adamw": [c_vp] * 7 + [c_ll] + [c_f] * 8 + [c_vp, c_int, c_int, c_vp],
+            "nb_adamw_group": [c_vp] * 8 + [c_int] + [c_f] * 8 + [c_vp, c_int, c_int, c_vp],
             "nb_adam_hyper": [c_vp, c_vp, c_f, ctypes.c_double, ctypes.c_double, c_vp],
             "nb_sgd": [c_vp] * 5 + [c_ll] + [c_f] * 4 + [c_int, c_int, c_vp],
             "nb_embedding_gather": [c_vp] * 4 + [c_int] * 5 + [c_vp],
@@ -208,6 +209,26 @@ def adam_hyper(step: torch.Tensor, lr: float, b1: float, b2: float) -> torch.Ten
 
 
 def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):
+def adamw_group(leaves: list, *, lr, b1, b2, eps, wd, step: int | None = None, hyper: torch.Tensor | None = None):
+    """``adamw`` of several small tensors that share their hyperparameters and types, in one launch per 48: ``leaves``
+    holds (p, g, m, v, inplace); returns [(p', m', v')], or None where a tensor is not 16-byte aligned."""
+    n = len(leaves)
+    ins, outs = [], []
+    for p, g, m, v, inplace in leaves:
+        p, g, m, v = p.contiguous(), g.contiguous(), m.contiguous(), v.contiguous()
+        ins.append((p, g, m, v))
+        outs.append((p, m, v) if inplace else (torch.empty_like(p), torch.empty_like(m), torch.empty_like(v)))
+    cols = [(c_vp * n)(*[t[i].data_ptr() for t in ins]) for i in range(4)] + [(c_vp * n)(*[t[i].data_ptr() for t in outs]) for i in range(3)]
+    if any((a or 0) & 15 for col in cols for a in col):
+        return None
+    bc1 = 1.0 - b1 ** step if step is not None else 1.0
+    bc2 = 1.0 - b2 ** step if step is not None else 1.0
+    sizes = (c_int * n)(*[t[0].numel() for t in ins])
+    _ok(_L().nb_adamw_group(*cols, sizes, n, float(lr), float(b1), float(b2), float(eps), float(wd), float(bc1), float(bc2), 1.0,
+                            ptr(hyper), _dt(ins[0][0]), _dt(ins[0][1]), stream_ptr()), "adamw_group")
+    return outs
+
+
     p = p.contiguous()
     g = g.contiguous()
     po = torch.empty_like(p)

@@ -519,6 +519,8 @@ class CompiledFunction:
         # liveness: free an intermediate after the last step that reads it
         out_ids = {id(i) for i in rec.out_impls if i is not None}
         produced = {id(o): o for outs in rec.keep for o in outs}
+        if plan is not None:
+            rec.steps = _group_small_updates(rec.steps, nodes)
         last_use: dict[int, int] = {}
         ph_ids = {id(p) for p in rec.placeholders}
         ph_last_use: dict[int, int] = {}
@@ -911,15 +913,17 @@ def _hoist_optimizer_steps(rec: "_Recorded", last_use: dict[int, int], produced:
     for si in movable:
         n = nodes[steps[si][1][0]]
         ready = -1
-        for a in n.input_impls():
-            ready = max(ready, producer.get(id(a), -1), readers.get(id(a), -1))
+        ins = n.input_impls()
+        for a in ins:
+            ready = max(ready, producer.get(id(a), -1))
+        for i in n.op.inplace_inputs:           # a tensor that is only read may have readers behind it
+            ready = max(ready, readers.get(id(ins[i]), -1) if i < len(ins) else -1)
         ready = min(ready, si)              # never later than where it already was
         after.setdefault(ready, []).append(si)
     order: list[int] = list(after.get(-1, []))
     for si in range(len(steps)):
-        if si in mov:
-            continue
-        order.append(si)
+        if si not in mov:
+            order.append(si)
         order += after.get(si, [])
     new_index = {old: new for new, old in enumerate(order)}
     rec.steps = [steps[o] for o in order]
@@ -1064,17 +1068,58 @@ def compute_local(impl) -> tuple:
 def _mark_inplace_updates(rec: _Recorded, last_use: dict[int, int]) -> None:
     donated = {id(ph) for ph, d in zip(rec.placeholders, rec.donated) if d}
     for si, (kind, idxs) in enumerate(rec.steps):
-        if kind != "op":
+        if kind not in ("op", "adamw_group"):
             continue
-        n = rec.nodes[idxs[0]]
-        which = getattr(n.op, "inplace_inputs", None)
-        if not which:
+        for ni in idxs:
+            n = rec.nodes[ni]
+            which = getattr(n.op, "inplace_inputs", None)
+            if not which:
+                continue
+            ins = n.input_impls()
+            targets = [ins[i] for i in which if i < len(ins)]
+            # in place only when every overwritten input was donated and nothing reads it later
+            if targets and all(id(t) in donated and last_use.get(id(t), si) <= si for t in targets):
+                n.kwargs = dict(n.kwargs, inplace=True)
+
+
+def _group_small_updates(steps: list, nodes: list[OpNode], max_elems: int = 1 << 18) -> list:
+    """AdamW updates of small unsharded parameters on one GPU become one step, one launch, at the end of the schedule: each
+    is a launch of some 3 us whatever its size. Only updates with the same hyperparameters and types, whose results feed no
+    other node, and whose tensors no other update of the group reads (one may then still be done in place)."""
+    from ..ops.fused import AdamWStepOp
+    from ..types import DType
+
+    readers: dict[int, int] = {}
+    for n in nodes:
+        for a in n.input_impls():
+            readers[id(a)] = readers.get(id(a), 0) + 1
+    groups: dict[tuple, list[int]] = {}
+    for si, (kind, idxs) in enumerate(steps):
+        n = nodes[idxs[0]]
+        if kind != "op" or not isinstance(n.op, AdamWStepOp) or any(o is not None and id(o) in readers for o in n.outputs()):
             continue
         ins = n.input_impls()
-        targets = [ins[i] for i in which if i < len(ins)]
-        # in place only when every overwritten input was donated and nothing reads it later
-        if targets and all(id(t) in donated and last_use.get(id(t), si) <= si for t in targets):
-            n.kwargs = dict(n.kwargs, inplace=True)
+        numel = 1
+        for d in ins[0]._shape:
+            numel *= int(d)
+        if not 0 < numel <= max_elems or any(x.sharding is not None or x.batch_dims or x.device.label != "gpu" for x in ins) \
+                or any(tuple(x._shape) != tuple(ins[0]._shape) for x in ins[1:4]) or ins[2].dtype is not DType.float32 \
+                or ins[3].dtype is not DType.float32 or any(x.dtype not in (DType.bfloat16, DType.float32) for x in ins[:2]):
+            continue
+        key = (tuple(sorted(n.kwargs.items())), ins[0].device, ins[0].dtype, ins[1].dtype, id(ins[4]) if len(ins) > 4 else None)
+        groups.setdefault(key, []).append(si)
+    out, gone = [], set()
+    for members in groups.values():
+        seen: dict[int, int] = {}
+        for si in members:
+            for x in {id(x): x for x in nodes[steps[si][1][0]].input_impls()[:4]}.values():
+                seen[id(x)] = seen.get(id(x), 0) + 1
+        members = [si for si in members if len({id(x) for x in nodes[steps[si][1][0]].input_impls()[:4]}) == 4
+                   and all(seen[id(x)] == 1 for x in nodes[steps[si][1][0]].input_impls()[:4])]
+        if len(members) > 1:
+            gone.update(members)
+            out.append(("adamw_group", tuple(steps[si][1][0] for si in members)))
+    return [st for si, st in enumerate(steps) if si not in gone] + out if gone else steps
 
 
 def compile(fn: Callable | None = None, *, fullgraph: bool = False, max_cache_size: int = 64,

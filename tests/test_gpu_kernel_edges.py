@@ -767,6 +767,60 @@ def test_compiled_calls_that_change_between_calls():
 
     def worker(n):
         try:
+@pytest.mark.parametrize("p_dtype,g_dtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_small_adamw_updates_in_one_launch(p_dtype, g_dtype):
+    """More tensors than a launch holds, sizes around a block's 2048 elements and the eight of a thread: the bits of one launch
+    each, in place or not; a misaligned tensor is refused."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(0)
+    sizes = [1, 7, 8, 9, 2047, 2048, 2049, 4096, 65537, 1 << 18] + list(range(11, 56))
+    mk = lambda n, dt: torch.randn(n, device="cuda").to(dt)  # noqa: E731
+    leaves = [(mk(n, p_dtype), mk(n, g_dtype), mk(n, torch.float32), mk(n, torch.float32).abs()) for n in sizes]
+    hyper = kernels.adam_hyper(torch.tensor(7.0, device="cuda"), 1e-3, 0.9, 0.999)
+    kw = dict(lr=1e-3, b1=0.9, b2=0.999, eps=1e-8, wd=0.01)
+    for extra in ({"hyper": hyper}, {"step": 7}, {}):
+        ref = [kernels.adamw(*leaf, **kw, **extra) for leaf in leaves]
+        flags = [i % 2 == 0 for i in range(len(sizes))]
+        mine = [tuple(t.clone() for t in leaf) for leaf in leaves]
+        got = kernels.adamw_group([(*leaf, f) for leaf, f in zip(mine, flags)], **kw, **extra)
+        for r, g, leaf, old, f in zip(ref, got, mine, leaves, flags):
+            assert all(torch.equal(a, b) for a, b in zip(r, g))
+            assert (g[0].data_ptr() == leaf[0].data_ptr()) == f and (f or torch.equal(leaf[0], old[0]))
+    odd = mk(17, torch.float32)[1:]
+    assert kernels.adamw_group([(mk(16, p_dtype), mk(16, g_dtype), odd, odd.clone(), False)], **kw) is None
+
+
+@pytest.mark.parametrize("donate", [False, True])
+def test_compiled_step_groups_its_small_updates(donate):
+    import nabla_b200 as nb
+    from nabla_b200 import nn
+
+    torch.manual_seed(0)
+    shapes = {"a": (64, 40), "b": (40,), "big": (600, 512), "c": (3,), "d": (512, 512)}
+    wrap = lambda d: {k: nb.Tensor.from_torch(v.clone()) for k, v in d.items()}  # noqa: E731
+    p = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
+    g = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
+    z = {k: torch.zeros(v, device="cuda") for k, v in shapes.items()}
+
+    def step(params, state, grads):
+        return nn.adamw_update(params, grads, state, lr=1e-2, weight_decay=0.1, realize=False)
+
+    f = nb.compile(step, cuda_graph=True, donate_argnums=(0, 1) if donate else ())
+    new, st = wrap(p), {"m": wrap(z), "v": wrap(z), "step": nb.Tensor.from_torch(torch.tensor(0.0, device="cuda"))}
+    ref = {k: v.double() for k, v in p.items()}
+    m = {k: v.double() for k, v in z.items()}
+    v2 = {k: v.double() for k, v in z.items()}
+    for t in range(1, 5):
+        new, st = f(new, st, wrap(g))
+        for k in p:
+            m[k] = 0.9 * m[k] + 0.1 * g[k].double()
+            v2[k] = 0.999 * v2[k] + 0.001 * g[k].double() ** 2
+            ref[k] = ref[k] - 1e-2 * ((m[k] / (1 - 0.9 ** t)) / ((v2[k] / (1 - 0.999 ** t)).sqrt() + 1e-8) + 0.1 * ref[k])
+            assert _rel2(new[k].to_torch(), ref[k]) < t * STORED[torch.float32]      # a rounding of p, m and v per step
+    assert sum("adamw_group" in line for line in str(f.dump_plan()).splitlines()) == 1
+
+
             for _ in range(20):
                 call(n, torch.float32)
         except Exception as e:  # noqa: BLE001
