@@ -556,6 +556,84 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
   for (int j = 0; j < V; ++j) acc[j] = 0.f;
   if (c < N) {
 #pragma unroll 4
+// ============================================================== small fp32 products
+// out[M][N] = A B + bias for fp32 operands of any strides: the linear layers of small fp32 networks, few results of long
+// sums, whose time is latency. 32 x 32 results per block, 32 steps of K staged through shared memory, the next
+// ones on their way meanwhile; K is cut into gridDim.z slices (fp32 partial sums, folded by a second launch) so that the
+// chip has some 300 blocks. What the library took 24.2 us for (256 x 1568 times 1568 x 10: 64-wide tiles, its own slices and
+// an add for the bias) takes 7.5; 1568 x 256 times 256 x 10: 8.1 -> 7.2.
+constexpr int SG = 32;
+struct SgemmArgs {
+  const float *a, *b, *bias;
+  float* out;                                        // [M][N], or [gridDim.z][M][N] partial sums
+  int M, N, K, per;                                  // per: K of a slice, a multiple of SG
+  long long a_m, a_k, b_k, b_n;
+};
+__global__ void __launch_bounds__(256) sgemm_kernel(const SgemmArgs g) {
+  __shared__ float sa[SG][SG + 1], sb[SG][SG + 1];   // [k][m], [k][n]
+  const int t = threadIdx.x, m0 = blockIdx.y * SG, n0 = blockIdx.x * SG;
+  const int k_lo = blockIdx.z * g.per, k_hi = min(g.K, k_lo + g.per);
+  // consecutive threads along the operand's unit stride
+  const bool a_along_k = g.a_k == 1, b_along_n = g.b_n == 1;
+  float ra[4], rb[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = t & 31, j = (t >> 5) + u * 8;
+      const int am = m0 + (a_along_k ? j : i), ak = k0 + (a_along_k ? i : j);
+      ra[u] = am < g.M && ak < k_hi && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, ak, g.K) ? g.a[am * g.a_m + ak * g.a_k] : 0.f;
+      const int bn = n0 + (b_along_n ? i : j), bk = k0 + (b_along_n ? j : i);
+      rb[u] = bn < g.N && bk < k_hi && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, bk, g.K) ? g.b[bk * g.b_k + bn * g.b_n] : 0.f;
+    }
+  };
+  // thread: rows ty and ty + 16, columns tx and tx + 16
+  const int tx = t & 15, ty = t >> 4;
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  fetch(k_lo);
+  for (int k0 = k_lo; k0 < k_hi; k0 += SG) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = t & 31, j = (t >> 5) + u * 8;
+      if (a_along_k) sa[i][j] = ra[u]; else sa[j][i] = ra[u];
+      if (b_along_n) sb[j][i] = rb[u]; else sb[i][j] = rb[u];
+    }
+    __syncthreads();
+    if (k0 + SG < k_hi) fetch(k0 + SG);
+    const int steps = min(SG, k_hi - k0);            // (a padded step would turn an infinite operand into NaN)
+    for (int k = 0; k < steps; ++k) {
+      const float a0 = sa[k][ty], a1 = sa[k][ty + 16], b0 = sb[k][tx], b1 = sb[k][tx + 16];
+      acc[0][0] = fmaf(a0, b0, acc[0][0]); acc[0][1] = fmaf(a0, b1, acc[0][1]);
+      acc[1][0] = fmaf(a1, b0, acc[1][0]); acc[1][1] = fmaf(a1, b1, acc[1][1]);
+    }
+    __syncthreads();
+  }
+  float* out = g.out + (size_t)blockIdx.z * g.M * g.N;
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int m = m0 + ty + 16 * r, n = n0 + tx + 16 * c;
+      if (m < g.M && n < g.N) out[(size_t)m * g.N + n] = acc[r][c] + (g.bias != nullptr && gridDim.z == 1 ? g.bias[n] : 0.f);
+    }
+}
+// out[m][n] = sum of the slices + bias[n]; eight lanes per result.
+__global__ void __launch_bounds__(256) sgemm_fold_kernel(const float* __restrict__ part, const float* __restrict__ bias,
+                                                        float* __restrict__ out, int MN, int N, int slices) {
+  const int i = (blockIdx.x * 256 + threadIdx.x) % 32 + blockIdx.x * 32, q = threadIdx.x >> 5;
+  __shared__ float sh[8][33];
+  float s = 0.f;
+  if (i < MN)
+    for (int z = q; z < slices; z += 8) s += part[(size_t)z * MN + i];
+  sh[q][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (q == 0 && i < MN) {
+    float a[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[k] = sh[k][threadIdx.x];
+    out[i] = sum8(a) + (bias != nullptr ? bias[i % N] : 0.f);
+  }
+}
+
     for (int r = r0 + warp; r < r1; r += 8) {
       float v[V];
       load_vec<T>(x + (size_t)r * N + c, v);
@@ -2571,6 +2649,28 @@ int nb_conv2d_wgrad_slices(long long positions, int K, int F) {
   long long z = 148 * 4 / tiles;
   if (z > (positions + 255) / 256) z = (positions + 255) / 256;
   return (int)(z < 1 ? 1 : z);
+// Slices of K for sgemm_kernel: as many as bring the grid to 300 blocks, of at least 64 steps.
+int nb_sgemm_slices(int M, int N, int K) {
+  const long long tiles = (long long)((M + SG - 1) / SG) * ((N + SG - 1) / SG);
+  long long z = 300 / (tiles < 1 ? 1 : tiles);
+  if (z > K / 64) z = K / 64;
+  if (z > 32) z = 32;
+  return z < 1 ? 1 : (int)z;
+}
+// partial: fp32 scratch of nb_sgemm_slices(M, N, K) * M * N elements, unused for one slice. Strides in elements.
+int nb_sgemm(const float* a, const float* b, const float* bias, float* out, float* partial, int M, int N, int K, long long a_m,
+             long long a_k, long long b_k, long long b_n, void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || (M + SG - 1) / SG > 65535 || (long long)M * N > 0x7fffffffll) return -2;
+  int z = nb_sgemm_slices(M, N, K);
+  const int per = ((K + z - 1) / z + SG - 1) / SG * SG;
+  z = (K + per - 1) / per;
+  const SgemmArgs g{a, b, bias, z > 1 ? partial : out, M, N, K, per, a_m, a_k, b_k, b_n};
+  sgemm_kernel<<<dim3((N + SG - 1) / SG, (M + SG - 1) / SG, z), 256, 0, STREAM>>>(g);
+  if (z > 1) sgemm_fold_kernel<<<(M * N + 31) / 32, 256, 0, STREAM>>>(partial, bias, out, M * N, N, z);
+  return CHECK_LAUNCH();
+}
+
 }
 // part: fp32 scratch of nb_conv2d_wgrad_slices(N * OH * OW, R * S * C, F) * R * S * C * F elements.
 int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part, int N, int H, int W, int C, int R, int S, int F,

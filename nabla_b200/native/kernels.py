@@ -52,6 +52,8 @@ def _L():
             "nb_conv2d_direct": [c_vp] * 4 + [c_int] * 14 + [c_vp],
             "nb_conv2d_wgrad_slices": [c_ll, c_int, c_int],
             "nb_conv2d_wgrad_direct": [c_vp] * 4 + [c_int] * 14 + [c_vp],
+            "nb_sgemm_slices": [c_int] * 3,
+            "nb_sgemm": [c_vp] * 5 + [c_int] * 3 + [c_ll] * 4 + [c_vp],
             "nb_sum_slices": [c_vp, c_vp, c_ll, c_int, c_int, c_vp],
             "nb_binary": [c_vp, c_vp, c_vp, c_ll, c_int, c_int, c_ll, c_int, c_int, c_vp],
             "nb_unary": [c_vp, c_vp, c_ll, c_int, c_int, c_vp],
@@ -559,6 +561,30 @@ def elementwise_enabled() -> bool:
 
 def binary(a: torch.Tensor, b: torch.Tensor, op: str):
     """``a (op) b`` in one kernel when both are fp32 / bf16 CUDA tensors of one dtype and ``b`` (or
+def sgemm_pays(M: int, N: int, K: int) -> bool:
+    """Where ``sgemm`` beats the library (us, library and this, over 45 sizes and both orders): few results of long sums. 256 x 10
+    over 1568 21.7 and 6.9, 128 x 128 over 512 10.5 and 5.6, 256 x 100 over 256 6.8 and 5.7, over 2048 21.9 and 16.5; not 256 x
+    256 over 256 (6.6 and 7.9), 1568 x 100 over 256 (7.4 and 14.1), 256 x 1568 over 10 (3.0 and 3.3), 8 x 1024 over 1024 (8.1 and 9.6)."""
+    return min(M, N) > 8 and M * N <= 32768 and 256 <= K <= 4096
+
+
+def sgemm(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor | None:
+    """``a @ b [+ bias]`` of small 2-D fp32 matrices of any strides on the CUDA cores; None for anything else."""
+    if not (a.is_cuda and a.device == b.device and a.dim() == 2 and b.dim() == 2 and a.dtype == b.dtype == torch.float32
+            and elementwise_enabled()):
+        return None
+    M, K, N = a.shape[0], a.shape[1], b.shape[1]
+    if b.shape[0] != K or not 0 < M * N * K < 1 << 31 or M > 1 << 20 or (bias is not None and (bias.numel() != N or bias.dtype != torch.float32)):
+        return None
+    z = _L().nb_sgemm_slices(M, N, K)
+    out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    part = torch.empty((z, M, N), dtype=torch.float32, device=a.device) if z > 1 else None
+    bias = bias.reshape(-1).contiguous() if bias is not None else None
+    _ok(_L().nb_sgemm(ptr(a), ptr(b), ptr(bias), ptr(out), ptr(part), M, N, K, a.stride(0), a.stride(1), b.stride(0), b.stride(1),
+                      stream_ptr()), "sgemm")
+    return out
+
+
     ``a``) has the other's shape, is a single element, or is a vector over the trailing dims (bias
     style). Returns None for anything else (mixed dtypes, general broadcasting, integers): the caller
     then uses the framework's generic path."""

@@ -155,6 +155,12 @@ class MatmulOp(Operation):
 
         if native.use_native(a) and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.numel() and b.numel():
             return native.gemm_bf16(a, b) if (a.dim() <= 3 and b.dim() <= 3) else _bmm_nd(a, b)
+        if native.use_native(a) and a.dtype == torch.float32 and a.dim() == 2 and b.dim() == 2:
+            from ..native import kernels
+
+            y = kernels.sgemm(a, b) if kernels.sgemm_pays(a.shape[0], b.shape[1], a.shape[1]) else None
+            if y is not None:
+                return y
         return torch.matmul(a, b)
 
     def sharding_rule(self, input_shapes, output_shapes, **kw):

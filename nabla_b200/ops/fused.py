@@ -86,9 +86,15 @@ class LinearOp(_Fused):
                              epilogue=epi, aux="store_preact", gelu_tanh=activation == "gelu_tanh")
             shp = (*x.shape[:-1], w.shape[-1])
             return y.reshape(shp), z.reshape(shp)
-        z = torch.matmul(x, w)
-        if b is not None:
-            z = z + b.reshape(-1).to(z.dtype)
+        z = None
+        if _native(x) and x.dtype == torch.float32 and x.dim() == 2 and w.dim() == 2:
+            from ..native import kernels
+
+            z = kernels.sgemm(x, w, b) if kernels.sgemm_pays(x.shape[0], w.shape[1], x.shape[1]) else None
+        if z is None:
+            z = torch.matmul(x, w)
+            if b is not None:
+                z = z + b.reshape(-1).to(z.dtype)
         if activation is None:
             return z
         return _apply_act(z, activation), z

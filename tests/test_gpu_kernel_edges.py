@@ -125,6 +125,144 @@ def test_direct_convolution_to_more_channel_tiles_than_a_grid_holds_in_y(F):
     assert torch.equal(y, x * w.view(F))
 
 
+# ---------------------------------------------------------------- adds and factors that GEMMs and the layer norm take
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,D", [(1, 8), (5, 128), (777, 256), (9, 264), (33, 1000), (1001, 512), (300, 2048), (4, 1024)])
+def test_layer_norm_backward_plus_a_gradient(dtype, rows, D):
+    """dx + add, rounded once, by the kernel of narrow rows and the one of wide rows; dgamma and dbeta as without it."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(rows)
+    x, dy, add = (torch.randn(rows, D, device="cuda").to(dtype) for _ in range(3))
+    g, b = torch.randn(D, device="cuda").to(dtype), torch.randn(D, device="cuda").to(dtype)
+    _, mean, rstd = kernels.layernorm_fwd(x, g, b, 1e-5)
+    plain, got = kernels.layernorm_bwd(dy, x, g, mean, rstd), kernels.layernorm_bwd(dy, x, g, mean, rstd, add=add)
+    x64 = x.double().requires_grad_(True)
+    ref, = torch.autograd.grad(TF.layer_norm(x64, (D,), g.double(), b.double()), x64, dy.double())
+    assert _rel2(got[0], ref + add.double()) < STORED[dtype]
+    assert torch.equal(got[1], plain[1]) and torch.equal(got[2], plain[2])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (130, 64, 72), (257, 77, 200), (2048, 16, 6144), (16, 512, 2048), (300, 1024, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gemm_with_a_factor_on_the_device(M, N, K, dtype):
+    """Also where the product is cut into K slices, and beside a bias and a residual."""
+    from nabla_b200.native.gemm import gemm_bf16
+
+    torch.manual_seed(0)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    s = torch.tensor([1.7], device="cuda").to(dtype)
+    ref = (a.double() @ b.double()) * s.double()
+    assert _rel2(gemm_bf16(a, b, alpha=s), ref) < STORED[torch.bfloat16]
+    bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    got = gemm_bf16(a, b, alpha=s, bias=bias, aux="add", aux_in=res)
+    assert _rel2(got, ref + bias.double() + res.double()) < STORED[torch.bfloat16]
+
+
+@pytest.mark.parametrize("tokens,dim,out,rank", [(100, 64, 192, 8), (333, 128, 77, 16), (1, 64, 64, 8), (2, 4096, 64, 8)])
+def test_compiled_products_take_their_adds_and_factors(tokens, dim, out, rank):
+    """x w + (x a) b s, a residual and a layer norm between them: values and gradients against 64 bits, with the steps that the
+    schedule has to have; a product that is asked for on its own stays on its own."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    torch.manual_seed(tokens)
+    mk = lambda *s: torch.randn(*s, device="cuda").mul(s[0] ** -0.5 if len(s) == 2 else 1.0).bfloat16()  # noqa: E731
+    x, w, a, b = torch.randn(tokens, dim, device="cuda").bfloat16(), mk(dim, out), mk(dim, rank), mk(rank, out)
+    g, be, w2, dy = mk(dim), mk(dim), mk(out, dim), torch.randn(tokens, dim, device="cuda").bfloat16()
+
+    def layer(x, w, a, b, g, be, w2):
+        h = F.layer_norm(x, g, be)
+        y = h @ w + ((h @ a) @ b) * 0.75
+        return x + F.linear(y, w2)
+
+    def layer64(x, w, a, b, g, be, w2):
+        h = TF.layer_norm(x, (dim,), g, be)
+        return x + (h @ w + ((h @ a) @ b) * 0.75) @ w2
+
+    args = (x, w, a, b, g, be, w2)
+    ps = [t.double().requires_grad_(True) for t in args]
+    y64 = layer64(*ps)
+    want = [y64] + list(torch.autograd.grad(y64, ps, dy.double()))
+    ts, dt = [nb.Tensor.from_torch(t) for t in args], nb.Tensor.from_torch(dy)
+
+    def run(*ps):
+        y, pull = nb.vjp(layer, *ps[:-1], create_graph=False)
+        return (y, *pull(ps[-1]))
+
+    f = nb.compile(run)
+    for _ in range(2):
+        for got, ref in zip(f(*ts, dt), want):
+            assert _rel2(got.to_torch(), ref) < 2.5e-2          # five products of bf16 operands and results, 2^-9 each, in a chain
+    plan = str(f.dump_plan())
+    for kind in ("gemm_residual", "gemm_scale", "scale_gemm", "ln_bwd_add"):
+        assert (kind in plan) or (tokens == 1 and kind == "gemm_residual"), (kind, plan)
+    h = nb.compile(lambda x, w, r: (lambda p: (p, p + r))(x @ w))
+    p, q = h(ts[0], ts[1], nb.Tensor.from_torch(mk(tokens, out)))
+    assert "gemm_residual" not in str(h.dump_plan()) and _rel2(p.to_torch(), x.double() @ w.double()) < STORED[torch.bfloat16]
+
+
+@pytest.mark.parametrize("M,N,K,sliced", [(2048, 16, 2048, True), (1, 512, 2048, True), (130, 77, 1800, True), (2002, 512, 2048, True), (512, 512, 2002, True),
+                                          (100, 1000, 8192, True), (257, 130, 4100, True), (16, 6144, 2048, True), (64, 64, 8193, False), (512, 512, 256, False),
+                                          (4096, 4096, 2048, False)])
+def test_products_on_clusters_of_k_slices(M, N, K, sliced):
+    """Both orders of both operands, remainders in every dimension, a bias and a residual of odd rows, a factor, fp32 results; and
+    the rule's lines. Against 64 bits, and the sum of the slices is the same bits on every run."""
+    from nabla_b200.native import gemm as G
+
+    assert (G.cluster_slices(M, N, K) > 1) == sliced
+    torch.manual_seed(0)
+    mk = lambda r, c: torch.randn(r, c, device="cuda").bfloat16()  # noqa: E731
+    orders = [(mk(M, K), mk(K, N)), (mk(K, M).t(), mk(K, N)), (mk(M, K), mk(N, K).t()), (mk(K, M).t(), mk(N, K).t())]
+    bias, res, s = torch.randn(N, device="cuda"), mk(M, N), torch.tensor([0.5], device="cuda")
+    for a, b in orders if M * N < 1 << 22 else orders[:1]:
+        ref = a.double() @ b.double()
+        got = G.gemm_bf16(a, b)
+        assert _rel2(got, ref) < STORED[torch.bfloat16] and torch.equal(got, G.gemm_bf16(a, b))
+        # fp32 sums of K products of unit variance
+        assert _rel2(G.gemm_bf16(a, b, out_dtype=torch.float32), ref) < 4e-6
+        got = G.gemm_bf16(a, b, alpha=s, bias=bias, aux="add", aux_in=res)
+        assert _rel2(got, 0.5 * ref + bias.double() + res.double()) < STORED[torch.bfloat16]
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (256, 10, 1568), (33, 31, 32), (32, 32, 33), (65, 10, 4097), (7, 1000, 3), (1, 4000, 500), (3000, 1, 65), (255, 255, 255)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+def test_small_fp32_products(M, N, K, ta, tb):
+    """Every order of the operands, tiles and slices with remainders, a bias, an infinite operand beside the padding, and what the
+    kernel leaves to the library. 2e-6: the rounding of sums of some hundred terms."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(K)
+    a = torch.randn(K, M, device="cuda").t() if ta else torch.randn(M, K, device="cuda")
+    b = torch.randn(N, K, device="cuda").t() if tb else torch.randn(K, N, device="cuda")
+    bias = torch.randn(1, N, device="cuda")
+    ref = a.double() @ b.double()
+    bound = 2e-6 * (a.double().abs() @ b.double().abs() + bias.double().abs())
+    assert ((kernels.sgemm(a, b).double() - ref).abs() <= bound).all()
+    assert ((kernels.sgemm(a, b, bias).double() - ref - bias.double()).abs() <= bound).all()
+    a[0, K - 1] = float("inf")
+    got = kernels.sgemm(a, b)
+    assert torch.isinf(got[0]).all() and torch.isfinite(got[1:]).all()
+    assert kernels.sgemm(a.bfloat16(), b.bfloat16()) is None and kernels.sgemm(a[None], b[None]) is None
+    assert kernels.sgemm(a, b, bias.bfloat16()) is None and kernels.sgemm(a[:0], b) is None
+
+
+def test_rule_of_small_fp32_products():
+    """Both sides of the rule's lines, and that both entry points take the same bits from either side's kernel."""
+    from nabla_b200.native import kernels
+    from nabla_b200.ops import binary, fused
+
+    for args, pays in (((9, 9, 256), True), ((8, 100, 512), False), ((100, 8, 512), False), ((256, 128, 256), True), ((257, 128, 256), False),
+                       ((64, 10, 255), False), ((64, 10, 4096), True), ((64, 10, 4097), False)):
+        assert kernels.sgemm_pays(*args) == pays
+    torch.manual_seed(0)
+    x, w, b = torch.randn(64, 300, device="cuda"), torch.randn(300, 10, device="cuda"), torch.randn(10, device="cuda")
+    assert torch.equal(binary.MatmulOp().kernel(x, w), kernels.sgemm(x, w))
+    assert torch.equal(fused.LinearOp().kernel(x, w, b), kernels.sgemm(x, w, b))
+    y, z = fused.LinearOp().kernel(x, w, b, activation="relu")
+    assert torch.equal(z, kernels.sgemm(x, w, b)) and torch.equal(y, z.clamp_min(0))
+
+
 # ---------------------------------------------------------------- embedding gradient
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab,dim,n,hot", [
