@@ -10,7 +10,10 @@ CUDA bf16 tensors:
 * ``matmul | linear (no bias) -> all_reduce(sum) | reduce_scatter`` on a mesh that runs one
   process per GPU: one launch of the fused GEMM + collective kernel (tiles are reduced over
   NVLink while later tiles are still being multiplied).
-* ``linear (+bias) -> add(residual)``: the residual is added in the GEMM epilogue.
+* ``linear (+bias) | matmul -> add(residual)``: the residual is added in the GEMM epilogue (compiled replays).
+* ``matmul -> mul(one element)`` and ``mul(one element) -> matmul ...`` (the scale of a LoRA adapter and its gradient): the
+  factor is applied in the GEMM epilogue (compiled replays).
+* ``layer norm backward -> add``: the gradient that joins dx is added in the same pass (compiled replays).
 * ``matmul -> dact_mul`` (backward of linear + relu/gelu): the activation derivative is applied in
   the GEMM epilogue.
 * compiled replays with donated optimizer state: ``matmul -> all_reduce(dp) -> adam_wstep`` becomes a
@@ -21,11 +24,11 @@ CUDA bf16 tensors:
   cores already work on the rows that are there; the gathered tensor is still produced.
 * ``zeros -> scatter-add``: the gradient of an embedding table without the table of zeros.
 * ``gather -> add`` of a tensor over the trailing dims (token plus position embedding): one pass (compiled replays).
+* ``adamw_group``: the updates of small parameters with the same hyperparameters, one launch at the end of a compiled
+  schedule (grouped by ``transforms/compile.py``).
 * ``sum -> sum ...`` over neighbouring axes: one reduction over the joined axes, where ``kernels.joined_sum`` takes it.
 
 Every other node is a plain 'op' step. Fusion never changes which tensors exist: fused-away
-* ``adamw_group``: the updates of small parameters with the same hyperparameters, one launch at the end of a compiled
-  schedule (grouped by ``transforms/compile.py``).
 intermediates that are still referenced are simply not fusable.
 """
 from __future__ import annotations
@@ -155,6 +158,53 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
             if dk is not None:
                 chain = [i, dk]
                 kind = "gemm_dact"
+        if chain is None and private and n.op.name == "matmul" and _is_cuda_bf16_2d(n):
+            # x @ w * s with one element s
+            o = sole_output(n)
+            if private_intermediate(o):
+                j = cons[id(o)][0]
+                if not used[j] and nodes[j].op.name == "mul" and _scalar_factor(nodes[j], o) is not None:
+                    chain = [i, j]
+                    kind = "gemm_scale"
+        if chain is None and private and n.op.name == "mul":
+            # x * s with one element s, read by nothing but GEMMs
+            o = sole_output(n)
+            readers = cons.get(id(o), []) if o is not None else []
+            if readers and id(o) not in target_ids and o.sharding is None and not o.batch_dims and len(set(readers)) == len(readers) \
+                    and any(_scalar_factor(n, x) is not None for x in n.input_impls()) \
+                    and all(not used[j] and nodes[j].op.name == "matmul" and _is_cuda_bf16_2d(nodes[j]) for j in readers):
+                used[i] = True
+                for j in readers:
+                    used[j] = True
+                    steps.append((j, ("scale_gemm", (i, j))))
+                continue
+        if chain is None and private and n.op.name in ("linear", "matmul") and n.kwargs.get("activation") is None \
+                and _is_plain_gemm(n):
+            # a residual of the same shape goes into the epilogue; of two products that are added, into the one with more to
+            # multiply
+            o = sole_output(n)
+            if private_intermediate(o):
+                k = cons[id(o)][0]
+                a_ = nodes[k]
+                if not used[k] and a_.op.name == "add" and _same_layout_addend(a_, o):
+                    other = [x for x in a_.input_impls() if x is not o][0]
+                    p = nodes[producer[id(other)]] if id(other) in producer else None
+                    if p is None or p.op.name not in ("linear", "matmul") or not _is_plain_gemm(p) or used[producer[id(other)]] \
+                            or p.input_impls()[0]._shape[-1] <= n.input_impls()[0]._shape[-1]:
+                        chain = [i, k]
+                        kind = "gemm_residual"
+        if chain is None and private and n.op.name == _LN_BWD_NAME and _is_plain_ln_bwd(n):
+            o = n.outputs()[0]
+            if private_intermediate(o):
+                k = cons[id(o)][0]
+                a_ = nodes[k]
+                if not used[k] and a_.op.name == "add" and _same_layout_addend(a_, o):
+                    other = [x for x in a_.input_impls() if x is not o][0]
+                    # the step runs where the layer norm's does, so that dgamma and dbeta are no later than before
+                    if producer.get(id(other), -1) < i:
+                        used[i] = used[k] = True
+                        steps.append((i, ("ln_bwd_add", (i, k))))
+                        continue
         if chain is None and _FUSE_RESIDUAL and n.op.name == "linear" and n.kwargs.get("activation") is None \
                 and _is_local_linear(n):
             # y = x @ w + b followed by "+ residual" of the same shape: the residual is added in the epilogue
@@ -319,6 +369,41 @@ def _is_local_linear(n: OpNode) -> bool:
 
     return (a.device.label == "gpu" and a.dtype is DType.bfloat16 and b.dtype is DType.bfloat16
             and len(b._shape) == 2 and len(a._shape) >= 2 and a.batch_dims == 0 and b.batch_dims == 0)
+
+
+def _is_plain_gemm(n: OpNode) -> bool:
+    """Unsharded bf16 GPU ``x @ w [+ b]`` (w 2-D)."""
+    ins = n.input_impls()
+    from ...types import DType
+
+    return (len(ins) in (2, 3) and all(x.sharding is None and not x.batch_dims and x.device.label == "gpu" for x in ins)
+            and all(x.dtype is DType.bfloat16 for x in ins[:2]) and len(ins[1]._shape) == 2 and len(ins[0]._shape) >= 2)
+
+
+def _scalar_factor(mul: OpNode, x: TensorImpl) -> TensorImpl | None:
+    """The one-element GPU tensor that ``mul`` multiplies the bf16 tensor ``x`` with, if that is what it does."""
+    from ...types import DType
+
+    ins = mul.input_impls()
+    if len(ins) != 2 or x.dtype is not DType.bfloat16:
+        return None
+    other = ins[1] if ins[0] is x else ins[0] if ins[1] is x else None
+    outs = mul.outputs()
+    o = outs[0] if len(outs) == 1 else None
+    if other is None or other is x or o is None or other.sharding is not None or other.batch_dims or x.sharding is not None \
+            or x.batch_dims or other.device != x.device or other.dtype is not x.dtype or tuple(o._shape) != tuple(x._shape) \
+            or any(int(d) != 1 for d in other._shape) or all(int(d) == 1 for d in x._shape):
+        return None
+    return other
+
+
+_LN_BWD_NAME = "layer_norm_bwd"
+
+
+def _is_plain_ln_bwd(n: OpNode) -> bool:
+    ins = n.input_impls()
+    return (len(ins) in (4, 5) and all(x.sharding is None and not x.batch_dims and x.device.label == "gpu" for x in ins)
+            and ins[0].dtype is ins[1].dtype)
 
 
 def _same_layout_addend(add: OpNode, x: TensorImpl) -> bool:
@@ -491,6 +576,27 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         else:
             store_outputs(last, [[out]])
         return
+    if kind == "adamw_group":
+        from ... import native
+
+        leaves = [[x._buffers[0] for x in n_.input_impls()] for n_ in group]
+        kw = group[0].kwargs
+        outs = None
+        if all(native.use_native(b[0]) for b in leaves):
+            from ...native import kernels
+
+            flags = [bool(n_.kwargs.get("inplace")) and all(t.is_contiguous() for t in (b[0], b[2], b[3])) for n_, b in zip(group, leaves)]
+            corrected = kw.get("bias_correction", True)
+            outs = kernels.adamw_group([(b[0], b[1], b[2], b[3], f) for b, f in zip(leaves, flags)], lr=kw["lr"], b1=kw["beta1"],
+                                       b2=kw["beta2"], eps=kw["eps"], wd=kw["weight_decay"],
+                                       step=kw.get("step_value") if corrected else None,
+                                       hyper=leaves[0][4].contiguous() if len(leaves[0]) > 4 and corrected else None)
+        for n_, o in zip(group, outs if outs is not None else group):
+            if outs is not None:
+                _store(n_, [[t] for t in o], keep_graph)
+            else:
+                _plain(n_, keep_graph)
+        return
     if kind == "gather_add":
         from ... import native
 
@@ -540,8 +646,49 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
             for n_ in group:
                 _plain(n_, keep_graph)
         return
-    if kind == "gemm_residual":
+    if kind in ("gemm_scale", "scale_gemm"):
+        from ... import native
         from ...native.gemm import gemm_bf16
+
+        mm, mul = group if kind == "gemm_scale" else (group[1], group[0])
+        if kind == "gemm_scale":
+            a, b = [x._buffers[0] for x in mm.input_impls()]
+            factor = _scalar_factor(mul, mm.outputs()[0])
+        else:
+            factor = [f for f in (_scalar_factor(mul, x) for x in mul.input_impls()) if f is not None][0]
+            scaled = [x for x in mul.input_impls() if x is not factor][0]
+            product = mul.outputs()[0]
+            a, b = [(scaled if x is product else x)._buffers[0] for x in mm.input_impls()]
+        if native.use_native(a) and a.numel() and b.numel():
+            out = gemm_bf16(a.reshape(-1, a.shape[-1]), b, alpha=factor._buffers[0]).reshape(*a.shape[:-1], b.shape[-1])
+            _store(group[-1], [[out]], keep_graph)
+        elif kind == "gemm_scale":
+            _plain(mm, keep_graph)
+            _plain(mul, keep_graph)
+        else:
+            _plain(mul, keep_graph)
+            _plain(mm, keep_graph)
+        return
+    if kind == "ln_bwd_add":
+        from ... import native
+        from ...native import kernels
+
+        ln, add = group
+        dx_out = ln.outputs()[0]
+        other = [x for x in add.input_impls() if x is not dx_out][0]._buffers[0]
+        ins = [x._buffers[0] for x in ln.input_impls()]
+        dy, x = ins[0], ins[1]
+        if native.use_native(x) and x.numel() and x.dtype in (torch.bfloat16, torch.float32) and dy.dtype == x.dtype \
+                and kernels.supports_rows(x, 2048):
+            dx, dg, db = kernels.layernorm_bwd(dy, x, ins[4] if len(ins) > 4 else None, ins[2].reshape(-1), ins[3].reshape(-1), add=other)
+            _store(ln, [None, [dg], [db]], keep_graph)
+            _store(add, [[dx]], keep_graph)
+        else:
+            _plain(ln, keep_graph)
+            _plain(add, keep_graph)
+        return
+    if kind == "gemm_residual":
+        from ...native.gemm import gemm_bf16, split_k_factor
 
         lin, add = group
         ins = lin.input_impls()
@@ -549,7 +696,8 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         bias = ins[2]._buffers[0] if len(ins) > 2 else None
         lin_out = lin.outputs()[0]
         res = [x for x in add.input_impls() if x is not lin_out][0]._buffers[0]
-        if a.is_cuda and a.numel() and b.numel():
+        # (a product that is worth cutting into K slices keeps its own launch: the slices are summed by another)
+        if a.is_cuda and a.numel() and b.numel() and not (bias is None and split_k_factor(a.numel() // a.shape[-1], b.shape[-1], a.shape[-1]) > 1):
             n_out = b.shape[-1]
             out = gemm_bf16(a.reshape(-1, a.shape[-1]), b, bias=bias, aux="add",
                             aux_in=res.reshape(-1, n_out)).reshape(*a.shape[:-1], n_out)
@@ -576,27 +724,6 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         return
     if kind == "all_reduce_bucket":
         # many small partial sums over the same device group: one flat all-reduce
-    if kind == "adamw_group":
-        from ... import native
-
-        leaves = [[x._buffers[0] for x in n_.input_impls()] for n_ in group]
-        kw = group[0].kwargs
-        outs = None
-        if all(native.use_native(b[0]) for b in leaves):
-            from ...native import kernels
-
-            flags = [bool(n_.kwargs.get("inplace")) and all(t.is_contiguous() for t in (b[0], b[2], b[3])) for n_, b in zip(group, leaves)]
-            corrected = kw.get("bias_correction", True)
-            outs = kernels.adamw_group([(b[0], b[1], b[2], b[3], f) for b, f in zip(leaves, flags)], lr=kw["lr"], b1=kw["beta1"],
-                                       b2=kw["beta2"], eps=kw["eps"], wd=kw["weight_decay"],
-                                       step=kw.get("step_value") if corrected else None,
-                                       hyper=leaves[0][4].contiguous() if len(leaves[0]) > 4 and corrected else None)
-        for n_, o in zip(group, outs if outs is not None else group):
-            if outs is not None:
-                _store(n_, [[t] for t in o], keep_graph)
-            else:
-                _plain(n_, keep_graph)
-        return
         from ...parallel import backend
 
         first = group[0]

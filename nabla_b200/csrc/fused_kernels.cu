@@ -255,11 +255,12 @@ template <> __device__ __forceinline__ uint4 pack_pairs<bf16>(const float2* in) 
 // instead of twice. At the end the four warps of a block fold their accumulators through shared
 // memory and the block writes one row of `partial` ([gridDim.x][2][D] fp32), which
 // colsum_partials_kernel adds up into dgamma / dbeta.
-template <typename T>
+// ADD: dx += add, the gradient that reaches x beside the norm (a residual connection), rounded once.
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(128, 4)
     layernorm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
-                               const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
-                               float* __restrict__ partial, int rows, int D) {
+                               const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
+                               T* __restrict__ dx, float* __restrict__ partial, int rows, int D) {
   constexpr int V = Vec<T>::N, P = V / 2;
   __shared__ float sh[2][32 * V];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = lane * V;
@@ -268,8 +269,9 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
   for (int k = 0; k < P; ++k) ag[k] = ab[k] = make_float2(0.f, 0.f);
   for (int row = blockIdx.x * 4 + warp; row < rows; row += gridDim.x * 4) {
-    uint4 xraw, draw;
+    uint4 xraw, draw, araw;
     if (act) {
+      if (ADD) araw = *reinterpret_cast<const uint4*>(add + (size_t)row * D + c);
       xraw = *reinterpret_cast<const uint4*>(x + (size_t)row * D + c);
       draw = *reinterpret_cast<const uint4*>(dy + (size_t)row * D + c);
     }
@@ -302,6 +304,12 @@ __global__ void __launch_bounds__(128, 4)
         const float2 g = gamma ? __fmul2_rn(dv[k], gm[k]) : dv[k];
         o[k] = __ffma2_rn(g, rs2, __ffma2_rn(xh, a2, b2));
       }
+      if (ADD) {
+        float2 e[P];
+        unpack_pairs<T>(araw, e);
+#pragma unroll
+        for (int k = 0; k < P; ++k) o[k] = __fadd2_rn(o[k], e[k]);
+      }
       *reinterpret_cast<uint4*>(dx + (size_t)row * D + c) = pack_pairs<T>(o);
     }
   }
@@ -332,11 +340,11 @@ __global__ void __launch_bounds__(128, 4)
 // column sums' second launch; 8192 x 4096: 165 -> 65 us. Each block writes one row of
 // `partial` as above.
 constexpr int LN_MAX_WARPS = 16;
-template <typename T>
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
     layernorm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
-                              const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
-                              float* __restrict__ partial, int rows, int D, int NW, int RB) {
+                              const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
+                              T* __restrict__ dx, float* __restrict__ partial, int rows, int D, int NW, int RB) {
   constexpr int V = Vec<T>::N, P = V / 2;
   __shared__ float4 red[2][LN_MAX_WARPS];
   __shared__ float sh[2][4 * 32 * V];                // RB > 1 means NW <= 4
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
   const int stride = gridDim.x * RB;
   int buf = 0;
   for (int base = blockIdx.x * RB; base < rows; base += 2 * stride, buf ^= 1) {
-    uint4 xr[2], dr[2];
+    uint4 xr[2], dr[2], ar[2];
     float rs[2], nmr[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -361,6 +369,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
         if (act && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, (long long)row * D + c + V - 1, (long long)rows * D)) {
           xr[u] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + c);
           dr[u] = *reinterpret_cast<const uint4*>(dy + (size_t)row * D + c);
+          if (ADD) ar[u] = *reinterpret_cast<const uint4*>(add + (size_t)row * D + c);
         }
         rs[u] = rstd[row];
         nmr[u] = -mean[row] * rs[u];
@@ -412,6 +421,12 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
 #pragma unroll
         for (int k = 0; k < P; ++k)
           o[k] = __ffma2_rn(__fmul2_rn(dv[k], gm[k]), rs2, __ffma2_rn(__ffma2_rn(xv[k], rs2, nmr2), a2, b2));
+        if (ADD) {
+          float2 e[P];
+          unpack_pairs<T>(ar[u], e);
+#pragma unroll
+          for (int k = 0; k < P; ++k) o[k] = __fadd2_rn(o[k], e[k]);
+        }
         *reinterpret_cast<uint4*>(dx + (size_t)row * D + c) = pack_pairs<T>(o);
       }
     }
@@ -541,21 +556,6 @@ static void fold_slices(const float* part, void* out, size_t n, int slices, cuda
   else fold_slices_kernel<T, 32><<<grid, 1024, 0, stream>>>(part, (T*)out, n, slices);
 }
 
-// ============================================================== column sum (bias gradient)
-// x [rows][N] -> partial[gridDim.y][N] ; each block sums a slab of rows for 32*V columns.
-template <typename T>
-__global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
-                                                    int N, int rows_per_block) {
-  constexpr int V = Vec<T>::N;
-  __shared__ float sh[8][32 * V];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = (blockIdx.x * 32 + lane) * V;
-  const int r0 = blockIdx.y * rows_per_block, r1 = min(rows, r0 + rows_per_block);
-  float acc[V];
-#pragma unroll
-  for (int j = 0; j < V; ++j) acc[j] = 0.f;
-  if (c < N) {
-#pragma unroll 4
 // ============================================================== small fp32 products
 // out[M][N] = A B + bias for fp32 operands of any strides: the linear layers of small fp32 networks, few results of long
 // sums, whose time is latency. 32 x 32 results per block, 32 steps of K staged through shared memory, the next
@@ -634,6 +634,21 @@ __global__ void __launch_bounds__(256) sgemm_fold_kernel(const float* __restrict
   }
 }
 
+// ============================================================== column sum (bias gradient)
+// x [rows][N] -> partial[gridDim.y][N] ; each block sums a slab of rows for 32*V columns.
+template <typename T>
+__global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
+                                                    int N, int rows_per_block) {
+  constexpr int V = Vec<T>::N;
+  __shared__ float sh[8][32 * V];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = (blockIdx.x * 32 + lane) * V;
+  const int r0 = blockIdx.y * rows_per_block, r1 = min(rows, r0 + rows_per_block);
+  float acc[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = 0.f;
+  if (c < N) {
+#pragma unroll 4
     for (int r = r0 + warp; r < r1; r += 8) {
       float v[V];
       load_vec<T>(x + (size_t)r * N + c, v);
@@ -834,6 +849,51 @@ struct AdamHyper { float lr, b1, b2, eps, wd, bc1, bc2, grad_scale; };
 // Elements [i, i + 8) of one tensor with 16-byte accesses (all tensors come from the caching allocator and
 // are at least 16-byte aligned); the ragged tail is handled element-wise.
 template <typename TP, typename TG>
+__device__ __forceinline__ void adamw_update8(const TP* __restrict__ p, const TG* __restrict__ g, const float* __restrict__ m,
+                                              const float* __restrict__ v, TP* __restrict__ p_out, float* __restrict__ m_out,
+                                              float* __restrict__ v_out, size_t i, size_t n, const AdamHyper& h, float ibc1,
+                                              float ibc2) {
+  float pv[8], gv[8], mv[8], vv[8];
+  const bool full = i + 8 <= n;
+  if (full) {
+    load8<TP>(p + i, pv);
+    load8<TG>(g + i, gv);
+    load8<float>(m + i, mv);
+    load8<float>(v + i, vv);
+  } else {
+    for (int j = 0; j < 8; ++j) {
+      const bool ok = i + j < n;
+      pv[j] = ok ? to_f<TP>(p[i + j]) : 0.f;
+      gv[j] = ok ? to_f<TG>(g[i + j]) : 0.f;
+      mv[j] = ok ? m[i + j] : 0.f;
+      vv[j] = ok ? v[i + j] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float gr = gv[j] * h.grad_scale;
+    mv[j] = h.b1 * mv[j] + (1.f - h.b1) * gr;
+    vv[j] = h.b2 * vv[j] + (1.f - h.b2) * gr * gr;
+    const float upd = (mv[j] * ibc1) / (sqrtf(vv[j] * ibc2) + h.eps) + h.wd * pv[j];
+    pv[j] -= h.lr * upd;
+  }
+  if (full) {
+    store8<TP>(p_out + i, pv);
+    store8<float>(m_out + i, mv);
+    store8<float>(v_out + i, vv);
+  } else {
+    for (int j = 0; j < 8; ++j)
+      if (i + j < n) {
+        p_out[i + j] = from_f<TP>(pv[j]);
+        m_out[i + j] = mv[j];
+        v_out[i + j] = vv[j];
+      }
+  }
+}
+__device__ __forceinline__ void adamw_device_hyper(AdamHyper& h, const float* __restrict__ hyper) {
+  if (hyper) { h.lr = hyper[0]; h.bc1 = hyper[1]; h.bc2 = hyper[2]; h.grad_scale = hyper[3]; }
+}
+template <typename TP, typename TG>
 __global__ void __launch_bounds__(256) adamw_kernel(const TP* __restrict__ p, const TG* __restrict__ g,
                                                    const float* __restrict__ m, const float* __restrict__ v,
                                                    TP* __restrict__ p_out, float* __restrict__ m_out,
@@ -913,51 +973,6 @@ __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restri
   const T* src = table + (size_t)(ok ? id : 0) * D;
   const T* pos = ADD ? add + (size_t)(i % period) * D : nullptr;
   T* dst = out + (size_t)i * D;
-__device__ __forceinline__ void adamw_update8(const TP* __restrict__ p, const TG* __restrict__ g, const float* __restrict__ m,
-                                              const float* __restrict__ v, TP* __restrict__ p_out, float* __restrict__ m_out,
-                                              float* __restrict__ v_out, size_t i, size_t n, const AdamHyper& h, float ibc1,
-                                              float ibc2) {
-  float pv[8], gv[8], mv[8], vv[8];
-  const bool full = i + 8 <= n;
-  if (full) {
-    load8<TP>(p + i, pv);
-    load8<TG>(g + i, gv);
-    load8<float>(m + i, mv);
-    load8<float>(v + i, vv);
-  } else {
-    for (int j = 0; j < 8; ++j) {
-      const bool ok = i + j < n;
-      pv[j] = ok ? to_f<TP>(p[i + j]) : 0.f;
-      gv[j] = ok ? to_f<TG>(g[i + j]) : 0.f;
-      mv[j] = ok ? m[i + j] : 0.f;
-      vv[j] = ok ? v[i + j] : 0.f;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float gr = gv[j] * h.grad_scale;
-    mv[j] = h.b1 * mv[j] + (1.f - h.b1) * gr;
-    vv[j] = h.b2 * vv[j] + (1.f - h.b2) * gr * gr;
-    const float upd = (mv[j] * ibc1) / (sqrtf(vv[j] * ibc2) + h.eps) + h.wd * pv[j];
-    pv[j] -= h.lr * upd;
-  }
-  if (full) {
-    store8<TP>(p_out + i, pv);
-    store8<float>(m_out + i, mv);
-    store8<float>(v_out + i, vv);
-  } else {
-    for (int j = 0; j < 8; ++j)
-      if (i + j < n) {
-        p_out[i + j] = from_f<TP>(pv[j]);
-        m_out[i + j] = mv[j];
-        v_out[i + j] = vv[j];
-      }
-  }
-}
-__device__ __forceinline__ void adamw_device_hyper(AdamHyper& h, const float* __restrict__ hyper) {
-  if (hyper) { h.lr = hyper[0]; h.bc1 = hyper[1]; h.bc2 = hyper[2]; h.grad_scale = hyper[3]; }
-}
-template <typename TP, typename TG>
   if ((D % V) == 0) {
     for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
       uint4 raw = ok ? *reinterpret_cast<const uint4*>(src + c) : make_uint4(0, 0, 0, 0);
@@ -2184,13 +2199,14 @@ int nb_layernorm_bwd_nblocks(int rows, int D, int dtype) {
   return nb < 1 ? 1 : nb;
 }
 
-int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
+int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* add, void* dx,
                      void* dgamma, void* dbeta, float* partial, int rows, int D, int dtype, void* stream) {
   if (rows <= 0) return 0;
   const int V = dtype ? 8 : 4;
   if (D % V) return -2;
   const int vpl = ln_bwd_vpl(D, dtype);
   if (vpl > LN_MAX_WARPS) return -3;
+  if (add != nullptr && (g_ln_bwd_two_kernels || (reinterpret_cast<uintptr_t>(add) & 15))) return -4;
   const int nb = nb_layernorm_bwd_nblocks(rows, D, dtype);
   const int rpb = (rows + nb - 1) / nb;
   dim3 grid_dx((rows + 3) / 4);
@@ -2202,19 +2218,20 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
     layernorm_bwd_dgb_kernel<T><<<grid_gb, 256, 0, STREAM>>>((const T*)dy, (const T*)x, mean, rstd, partial, rows, D, \
                                                               rpb);                                                   \
   }
-#define LN_BWD_ONE_PASS(T)                                                                                            \
+#define LN_BWD_ONE_PASS(T, ADD)                                                                                       \
   {                                                                                                                   \
     if (vpl == 1)                                                                                                     \
-      layernorm_bwd_fused_kernel<T><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean,      \
-                                                               rstd, (T*)dx, partial, rows, D);                      \
+      layernorm_bwd_fused_kernel<T, ADD><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
+                                                                 (const T*)add, (T*)dx, partial, rows, D);            \
     else {                                                                                                            \
       const int rb = vpl < 8 ? 8 / vpl : 1;                                                                           \
-      layernorm_bwd_rows_kernel<T><<<nb, 32 * vpl * rb, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma,      \
-                                                                     mean, rstd, (T*)dx, partial, rows, D, vpl, rb); \
+      layernorm_bwd_rows_kernel<T, ADD><<<nb, 32 * vpl * rb, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
+                                                                          (const T*)add, (T*)dx, partial, rows, D, vpl, rb); \
     }                                                                                                                 \
   }
   if (!g_ln_bwd_two_kernels) {
-    if (dtype) LN_BWD_ONE_PASS(bf16) else LN_BWD_ONE_PASS(float)
+    if (dtype) { if (add) LN_BWD_ONE_PASS(bf16, true) else LN_BWD_ONE_PASS(bf16, false) }
+    else { if (add) LN_BWD_ONE_PASS(float, true) else LN_BWD_ONE_PASS(float, false) }
   } else if (dtype) {
     if (vpl <= 1) LN_BWD(bf16, 1) else if (vpl <= 2) LN_BWD(bf16, 2) else if (vpl <= 4) LN_BWD(bf16, 4)
     else if (vpl <= 8) LN_BWD(bf16, 8) else LN_BWD(bf16, 16)
@@ -2632,23 +2649,6 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
   return CHECK_LAUNCH();
 }
 
-int nb_sum_slices(const float* part, void* out, long long n, int slices, int dtype, void* stream) {
-  if (n <= 0 || slices <= 0) return 0;
-  if (n & 3) return -2;
-  const int grid = grid_for((size_t)n / 4, 256, 148 * 8);
-  if (dtype) sum_slices_kernel<bf16><<<grid, 256, 0, STREAM>>>(part, (bf16*)out, (size_t)n, slices);
-  else sum_slices_kernel<float><<<grid, 256, 0, STREAM>>>(part, (float*)out, (size_t)n, slices);
-  return CHECK_LAUNCH();
-}
-
-// Position slices of the filter gradient: four blocks per SM and no more, since a few blocks above that would
-// be a wave of their own (8 x 224 x 224 x 3 -> 64, 7 x 7: 594 blocks 310 us, 588 blocks 218); at least 256 positions each.
-int nb_conv2d_wgrad_slices(long long positions, int K, int F) {
-  const int kt = K <= 16 ? 16 : K <= 32 ? 32 : 64, ft = F <= 16 ? 16 : 32;
-  const long long tiles = (long long)((K + kt - 1) / kt) * ((F + ft - 1) / ft);
-  long long z = 148 * 4 / tiles;
-  if (z > (positions + 255) / 256) z = (positions + 255) / 256;
-  return (int)(z < 1 ? 1 : z);
 // Slices of K for sgemm_kernel: as many as bring the grid to 300 blocks, of at least 64 steps.
 int nb_sgemm_slices(int M, int N, int K) {
   const long long tiles = (long long)((M + SG - 1) / SG) * ((N + SG - 1) / SG);
@@ -2671,6 +2671,23 @@ int nb_sgemm(const float* a, const float* b, const float* bias, float* out, floa
   return CHECK_LAUNCH();
 }
 
+int nb_sum_slices(const float* part, void* out, long long n, int slices, int dtype, void* stream) {
+  if (n <= 0 || slices <= 0) return 0;
+  if (n & 3) return -2;
+  const int grid = grid_for((size_t)n / 4, 256, 148 * 8);
+  if (dtype) sum_slices_kernel<bf16><<<grid, 256, 0, STREAM>>>(part, (bf16*)out, (size_t)n, slices);
+  else sum_slices_kernel<float><<<grid, 256, 0, STREAM>>>(part, (float*)out, (size_t)n, slices);
+  return CHECK_LAUNCH();
+}
+
+// Position slices of the filter gradient: four blocks per SM and no more, since a few blocks above that would
+// be a wave of their own (8 x 224 x 224 x 3 -> 64, 7 x 7: 594 blocks 310 us, 588 blocks 218); at least 256 positions each.
+int nb_conv2d_wgrad_slices(long long positions, int K, int F) {
+  const int kt = K <= 16 ? 16 : K <= 32 ? 32 : 64, ft = F <= 16 ? 16 : 32;
+  const long long tiles = (long long)((K + kt - 1) / kt) * ((F + ft - 1) / ft);
+  long long z = 148 * 4 / tiles;
+  if (z > (positions + 255) / 256) z = (positions + 255) / 256;
+  return (int)(z < 1 ? 1 : z);
 }
 // part: fp32 scratch of nb_conv2d_wgrad_slices(N * OH * OW, R * S * C, F) * R * S * C * F elements.
 int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part, int N, int H, int W, int C, int R, int S, int F,

@@ -48,6 +48,8 @@ struct GemmArgs {
   int vec_ok;               // output/aux rows are 16-byte aligned
   int vec32_ok;             // ... and 32-byte aligned: a lane's 32 columns go out as 32-byte stores (whole sectors)
   float alpha;              // scale applied to the accumulator before the epilogue
+  const void* alpha_dev;    // one more factor, read on the device (bf16 or fp32; may be null)
+  int alpha_fp32;
   int* status;              // device status word (0 = ok)
 };
 
@@ -216,13 +218,10 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
   const int lane = threadIdx.x & 31;
   // a previous bounded wait failed on this device: do not pile more waits on top of it
   // (a pair does not leave early: both CTAs must reach the cluster barriers below, and their waits
-  // are bounded anyway)
-  if (!PAIR) {
-    __shared__ int s_abort;
-    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(args.status);
-    __syncthreads();
-    if (s_abort != 0) return false;   // uniform for the whole CTA
-  }
+  // are bounded anyway). The word is fetched under the set-up below and looked at after it: half a microsecond of a small
+  // product's five
+  __shared__ int s_abort;
+  if (!PAIR && threadIdx.x == 96) s_abort = *reinterpret_cast<volatile int*>(args.status);
 
   // pair: tiles are counted in pairs of 128-row tiles; an odd last tile leaves the second CTA a tile
   // past the edge (its loads read the fill value and its epilogue stores nothing)
@@ -265,6 +264,10 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
   if (PAIR) cluster_sync_all();      // the other CTA's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!PAIR && s_abort != 0) {               // uniform for the whole CTA
+    if (warp == 2) tmem_dealloc(tmem_base, 2 * BN);
+    return false;
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -439,6 +442,10 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
     // sectors, per 2-byte store: 4096 x 10001 x 512 took 554 us, 153 this way.
     const bool staged = MODE == MODE_NONE && !args.vec_ok && !args.out_fp32 && !args.accumulate;
     const bool heavy = (args.epi == EPI_BIAS_GELU || args.aux == AUX_MUL_DGELU) && !staged;
+    float alpha = args.alpha;
+    if (args.alpha_dev != nullptr)
+      alpha *= args.alpha_fp32 ? *reinterpret_cast<const float*>(args.alpha_dev)
+                               : __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(args.alpha_dev));
     bool ok = true;
     int it = 0;
     for (int t = cta; t < num_tiles; t += nctas, ++it) {
@@ -512,7 +519,7 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
         tmem_ld_wait_regs(v);
         float f[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * args.alpha + sbias[c * 32 + j];
+        for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * alpha + sbias[c * 32 + j];
         const int c_next = next_chunk(c);
         if (c_next < BN / 32) tmem_ld_32x32(taddr + c_next * 32, v);
         const bool full = (nb0 + 32 <= args.N) && args.vec_ok;
@@ -1350,7 +1357,7 @@ extern "C" int nb_gemm_bf16(const void* A, const void* B, void* C, const void* b
                             long long ldc, long long stride_a, long long stride_b, long long stride_c,
                             long long ld_aux, long long stride_aux, int a_mn, int b_mn, int out_fp32,
                             int bias_fp32, int epi, int aux, int accumulate, int gelu_tanh, float alpha,
-                            int block_n, int max_ctas, int* status, void* stream) {
+                            const void* alpha_dev, int alpha_fp32, int block_n, int max_ctas, int* status, void* stream) {
   using namespace nb;
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (K <= 0) return -10;
@@ -1390,6 +1397,7 @@ extern "C" int nb_gemm_bf16(const void* A, const void* B, void* C, const void* b
   g.a_mn = a_mn; g.b_mn = b_mn; g.out_fp32 = out_fp32; g.bias_fp32 = bias_fp32;
   g.epi = epi; g.aux = aux; g.accumulate = accumulate; g.gelu_tanh = gelu_tanh;
   g.alpha = alpha;
+  g.alpha_dev = alpha_dev; g.alpha_fp32 = alpha_fp32;
   g.status = status;
   const int oes = out_fp32 ? 4 : 2;
   bool vec = ((reinterpret_cast<uintptr_t>(C) & 15) == 0) && ((ldc * oes) % 16 == 0) &&

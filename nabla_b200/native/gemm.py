@@ -22,7 +22,7 @@ def _get():
         fn = lib.nb_gemm_bf16
         fn.restype = ctypes.c_int
         fn.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int] * 4 + [ctypes.c_longlong] * 8 + [ctypes.c_int] * 8 + [
-            ctypes.c_float, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+            ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
         lib.nb_gemm_set_pair_mode.argtypes = [ctypes.c_int]
         lib.nb_gemm_set_pair_mode.restype = ctypes.c_int
         lib.nb_gemm_pair_alloc_probe.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
@@ -172,11 +172,12 @@ def _k_slices(t3: torch.Tensor, kind: str, ld: int, s: int, k_dim: int) -> torch
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = None, epilogue: str = "none",
               aux: str = "none", aux_in: torch.Tensor | None = None, out: torch.Tensor | None = None,
               out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False, gelu_tanh: bool = False,
-              alpha: float = 1.0, block_n: int = 0, max_ctas: int = 0, split_k: int | None = None):
+              alpha: float | torch.Tensor = 1.0, block_n: int = 0, max_ctas: int = 0, split_k: int | None = None):
     """``out = epilogue(alpha * a @ b + bias)`` for bf16 ``a`` (..., M, K) and ``b`` (..., K, N).
 
     ``a`` and ``b`` may be arbitrary 2-D/3-D strided views (e.g. ``.transpose(-1, -2)``); views
-    whose rows or columns are contiguous are consumed in place through TMA descriptors.
+    whose rows or columns are contiguous are consumed in place through TMA descriptors. ``alpha`` may be a one-element
+    bf16 / fp32 tensor, which the kernel reads on the device.
     Returns ``out`` or ``(out, preact)`` when ``aux == 'store_preact'``.
     """
     global launch_count
@@ -211,13 +212,13 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
     # split-K: few output tiles and a long K (weight gradients): the K range is cut into slices that
     # run as a batch (each slice an fp32 partial product), and one pass adds the slices
     if (batch == 1 and bias is None and epilogue == "none" and aux == "none" and out is None and not accumulate
-            and alpha == 1.0 and block_n == 0 and split_k != 1 and out_dtype in (torch.bfloat16, torch.float32)):
+            and (isinstance(alpha, torch.Tensor) or alpha == 1.0) and block_n == 0 and split_k != 1 and out_dtype in (torch.bfloat16, torch.float32)):
         s_ = split_k if split_k else split_k_factor(M, N, K)
         if s_ > 1 and K % (s_ * 64) == 0:
             from . import kernels
 
             part = gemm_bf16(_k_slices(a3, akind, lda, s_, 1), _k_slices(b3, bkind, ldb, s_, 0),
-                             out_dtype=torch.float32, split_k=1, max_ctas=max_ctas)
+                             out_dtype=torch.float32, split_k=1, max_ctas=max_ctas, alpha=alpha)
             res = kernels.sum_slices(part, out_dtype)
             return res if squeeze else res.unsqueeze(0)
     a_mn = 0 if akind == "row" else 1
@@ -250,12 +251,16 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
     if bias is not None and bias.dtype not in (torch.float32, torch.bfloat16):
         bias = bias.to(torch.bfloat16)
     st = status_word(a.device)
+    alpha_t = alpha if isinstance(alpha, torch.Tensor) else None
+    if alpha_t is not None:
+        assert alpha_t.numel() == 1 and alpha_t.dtype in (torch.float32, torch.bfloat16)
+        alpha = 1.0
     rc = _get()(
         ptr(a3), ptr(b3), ptr(out), ptr(bias), ptr(aux_t if aux not in ("none", "store_preact") else None),
         ptr(aux_out), M, N, K, batch, lda, ldb, out.stride(1), sa, sb, out.stride(0) if batch > 1 else M * out.stride(1),
         aux_t.stride(1) if aux_t is not None else 0, aux_t.stride(0) if aux_t is not None else 0,
         a_mn, b_mn, out_fp32, bias_fp32, EPI[epilogue], AUX[aux], int(accumulate), int(gelu_tanh), float(alpha),
-        block_n, max_ctas, ptr(st), stream_ptr())
+        ptr(alpha_t), int(alpha_t is not None and alpha_t.dtype == torch.float32), block_n, max_ctas, ptr(st), stream_ptr())
     if rc != 0:
         raise RuntimeError(f"nb_gemm_bf16 failed with code {rc} for {tuple(a.shape)} @ {tuple(b.shape)}")
     launch_count += 1

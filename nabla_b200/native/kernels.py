@@ -24,7 +24,7 @@ def _L():
         sig = {
             "nb_layernorm_fwd": [c_vp] * 6 + [c_int, c_int, c_f, c_int, c_vp],
             "nb_layernorm_bwd_nblocks": [c_int, c_int, c_int],
-            "nb_layernorm_bwd": [c_vp] * 9 + [c_int, c_int, c_int, c_vp],
+            "nb_layernorm_bwd": [c_vp] * 10 + [c_int, c_int, c_int, c_vp],
             "nb_colsum_nparts": [c_int] * 3,
             "nb_colsum": [c_vp] * 3 + [c_int] * 4 + [c_vp],
             "nb_softmax": [c_vp, c_vp, c_int, c_int, c_int, c_int, c_vp],
@@ -120,8 +120,14 @@ def layernorm_fwd(x: torch.Tensor, gamma, beta, eps: float):
     return y.view(x.shape), mean, rstd
 
 
-def layernorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma, mean: torch.Tensor, rstd: torch.Tensor):
+def layernorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma, mean: torch.Tensor, rstd: torch.Tensor, add: torch.Tensor | None = None):
+    """(dx, dgamma, dbeta); ``add`` (x's shape and dtype) is added to dx in the same pass."""
     global launch_count
+    if add is not None:
+        add = add.contiguous()
+        if add.data_ptr() & 15 or os.environ.get("NABLA_B200_LN_BWD") == "two_kernels":
+            dx, dgamma, dbeta = layernorm_bwd(dy, x, gamma, mean, rstd)
+            return dx + add, dgamma, dbeta
     D = x.shape[-1]
     x2 = x.contiguous().view(-1, D)
     dy2 = dy.contiguous().view(-1, D)
@@ -132,7 +138,7 @@ def layernorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma, mean: torch.Tensor, 
     nb = _L().nb_layernorm_bwd_nblocks(rows, D, _dt(x))
     partial = torch.empty((nb, 2, D), dtype=torch.float32, device=x.device)
     g = gamma.contiguous().to(x.dtype) if gamma is not None else None
-    _ok(_L().nb_layernorm_bwd(ptr(dy2), ptr(x2), ptr(g), ptr(mean), ptr(rstd), ptr(dx), ptr(dgamma), ptr(dbeta),
+    _ok(_L().nb_layernorm_bwd(ptr(dy2), ptr(x2), ptr(g), ptr(mean), ptr(rstd), ptr(add), ptr(dx), ptr(dgamma), ptr(dbeta),
                               ptr(partial), rows, D, _dt(x), stream_ptr()), "layernorm_bwd")
     launch_count += 2
     return dx.view(x.shape), dgamma, dbeta
@@ -203,14 +209,6 @@ def adamw(p, g, m, v, *, lr, b1, b2, eps, wd, step: int | None = None, hyper: to
     return po, mo, vo
 
 
-def adam_hyper(step: torch.Tensor, lr: float, b1: float, b2: float) -> torch.Tensor:
-    """[lr, 1 - b1^t, 1 - b2^t, 1] for the fp32 step count ``t`` on the device (one element)."""
-    out = torch.empty(4, dtype=torch.float32, device=step.device)
-    _ok(_L().nb_adam_hyper(ptr(step), ptr(out), float(lr), float(b1), float(b2), stream_ptr()), "adam_hyper")
-    return out
-
-
-def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):
 def adamw_group(leaves: list, *, lr, b1, b2, eps, wd, step: int | None = None, hyper: torch.Tensor | None = None):
     """``adamw`` of several small tensors that share their hyperparameters and types, in one launch per 48: ``leaves``
     holds (p, g, m, v, inplace); returns [(p', m', v')], or None where a tensor is not 16-byte aligned."""
@@ -231,6 +229,14 @@ def adamw_group(leaves: list, *, lr, b1, b2, eps, wd, step: int | None = None, h
     return outs
 
 
+def adam_hyper(step: torch.Tensor, lr: float, b1: float, b2: float) -> torch.Tensor:
+    """[lr, 1 - b1^t, 1 - b2^t, 1] for the fp32 step count ``t`` on the device (one element)."""
+    out = torch.empty(4, dtype=torch.float32, device=step.device)
+    _ok(_L().nb_adam_hyper(ptr(step), ptr(out), float(lr), float(b1), float(b2), stream_ptr()), "adam_hyper")
+    return out
+
+
+def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):
     p = p.contiguous()
     g = g.contiguous()
     po = torch.empty_like(p)
@@ -327,6 +333,23 @@ class CopyBatch:
         # where the native kernels are switched off
         self.plain = [use_native(t) and t.device.index == dev and _is_dense(t) for t in fixed]
         self.storages = {t.untyped_storage().data_ptr() for t in fixed} if shared else None
+        self.all_sizes = (c_ull * n)(*self.size) if all(self.plain) else None
+
+    def fresh(self) -> list[torch.Tensor]:
+        """New tensors like the fixed ones with their contents: what was just allocated for the purpose needs none of the
+        checks of ``run``."""
+        global launch_count
+        others = [torch.empty_like(t) for t in self.fixed]
+        if self.all_sizes is None or not others or torch.cuda.current_device() != self.dev or any(
+                o.stride() != s for o, s in zip(others, self.strides)):
+            self.run(others, into_fixed=False)
+            return others
+        n = len(others)
+        k = _L().nb_copy_batch((c_vp * n)(*[o.data_ptr() for o in others]), self.fixed_ptrs, self.all_sizes, n, stream_ptr())
+        if k < 0:
+            raise RuntimeError(f"copy_batch failed with code {k}")
+        launch_count += k
+        return others
 
     def run(self, others: list[torch.Tensor], into_fixed: bool) -> None:
         """``fixed <- others`` (``into_fixed``) or ``others <- fixed``. A pair that shares its storage is left
@@ -336,23 +359,24 @@ class CopyBatch:
         global launch_count
         own, copies = self.own, False
         n = len(own)
+        rest = []                                           # pairs that torch copies
         if self.storages is not None and into_fixed:
             others = [o.clone() if o.data_ptr() != own[i] and o.untyped_storage().data_ptr() in self.storages else o
                       for i, o in enumerate(others)]
         ptrs, nbytes = (c_vp * n)(), (c_ull * n)()          # of this call: another thread may be in here too
         here = torch.cuda.current_device() == self.dev
-        for i, o in enumerate(others):
+        for i, (o, f, q, plain, stride, size) in enumerate(zip(others, self.fixed, own, self.plain, self.strides, self.size)):
             p = o.data_ptr()
-            if p == own[i]:
+            if p == q:
                 continue
-            f = self.fixed[i]
-            if here and self.plain[i] and o.dtype is f.dtype and o.stride() == self.strides[i] and o.device == f.device:
+            if here and plain and o.dtype is f.dtype and o.stride() == stride and o.get_device() == self.dev:
                 ptrs[i] = p
-                nbytes[i] = self.size[i]
-                copies = True
-        for i, o in enumerate(others):
-            if nbytes[i] == 0 and self.size[i] and o.data_ptr() != own[i]:
-                self.fixed[i].copy_(o) if into_fixed else o.copy_(self.fixed[i])
+                nbytes[i] = size
+                copies = copies or size > 0
+            elif size:
+                rest.append(i)
+        for i in rest:
+            self.fixed[i].copy_(others[i]) if into_fixed else others[i].copy_(self.fixed[i])
         if not copies:
             return
         dst, src = (self.fixed_ptrs, ptrs) if into_fixed else (ptrs, self.fixed_ptrs)
@@ -537,30 +561,6 @@ def nf4_dequant_codes(codes: torch.Tensor, absmax: torch.Tensor, codebook: torch
     return out
 
 
-def sum_slices(part: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
-    """Sum a contiguous fp32 tensor over its leading dim (the partial products of a split-K GEMM)."""
-    s_ = part.shape[0]
-    out = torch.empty(part.shape[1:], dtype=out_dtype, device=part.device)
-    _ok(_L().nb_sum_slices(ptr(part), ptr(out), out.numel(), s_, _dt(out), stream_ptr()), "sum_slices")
-    return out
-
-
-# ---------------------------------------------------------------- pointwise / reduction families
-BINARY_OPS = {"add": 0, "sub": 1, "mul": 2, "div": 3, "maximum": 4, "minimum": 5, "pow": 6}
-UNARY_OPS = {"neg": 0, "abs": 1, "exp": 2, "log": 3, "sqrt": 4, "rsqrt": 5, "tanh": 6, "sigmoid": 7, "sin": 8, "cos": 9,
-             "erf": 10, "log1p": 11, "floor": 12, "trunc": 13, "round": 14, "square": 15, "reciprocal": 16}
-REDUCE_OPS = {"sum": 0, "max": 1, "min": 2, "mean": 3, "argmax": 4, "argmin": 5}
-_FLOATS = (torch.float32, torch.bfloat16)
-
-
-def elementwise_enabled() -> bool:
-    import os
-
-    return os.environ.get("NABLA_B200_ELEMENTWISE", "native") == "native"
-
-
-def binary(a: torch.Tensor, b: torch.Tensor, op: str):
-    """``a (op) b`` in one kernel when both are fp32 / bf16 CUDA tensors of one dtype and ``b`` (or
 def sgemm_pays(M: int, N: int, K: int) -> bool:
     """Where ``sgemm`` beats the library (us, library and this, over 45 sizes and both orders): few results of long sums. 256 x 10
     over 1568 21.7 and 6.9, 128 x 128 over 512 10.5 and 5.6, 256 x 100 over 256 6.8 and 5.7, over 2048 21.9 and 16.5; not 256 x
@@ -585,6 +585,30 @@ def sgemm(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) ->
     return out
 
 
+def sum_slices(part: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
+    """Sum a contiguous fp32 tensor over its leading dim (the partial products of a split-K GEMM)."""
+    s_ = part.shape[0]
+    out = torch.empty(part.shape[1:], dtype=out_dtype, device=part.device)
+    _ok(_L().nb_sum_slices(ptr(part), ptr(out), out.numel(), s_, _dt(out), stream_ptr()), "sum_slices")
+    return out
+
+
+# ---------------------------------------------------------------- pointwise / reduction families
+BINARY_OPS = {"add": 0, "sub": 1, "mul": 2, "div": 3, "maximum": 4, "minimum": 5, "pow": 6}
+UNARY_OPS = {"neg": 0, "abs": 1, "exp": 2, "log": 3, "sqrt": 4, "rsqrt": 5, "tanh": 6, "sigmoid": 7, "sin": 8, "cos": 9,
+             "erf": 10, "log1p": 11, "floor": 12, "trunc": 13, "round": 14, "square": 15, "reciprocal": 16}
+REDUCE_OPS = {"sum": 0, "max": 1, "min": 2, "mean": 3, "argmax": 4, "argmin": 5}
+_FLOATS = (torch.float32, torch.bfloat16)
+
+
+def elementwise_enabled() -> bool:
+    import os
+
+    return os.environ.get("NABLA_B200_ELEMENTWISE", "native") == "native"
+
+
+def binary(a: torch.Tensor, b: torch.Tensor, op: str):
+    """``a (op) b`` in one kernel when both are fp32 / bf16 CUDA tensors of one dtype and ``b`` (or
     ``a``) has the other's shape, is a single element, or is a vector over the trailing dims (bias
     style). Returns None for anything else (mixed dtypes, general broadcasting, integers): the caller
     then uses the framework's generic path."""

@@ -202,29 +202,6 @@ def test_compiled_products_take_their_adds_and_factors(tokens, dim, out, rank):
     assert "gemm_residual" not in str(h.dump_plan()) and _rel2(p.to_torch(), x.double() @ w.double()) < STORED[torch.bfloat16]
 
 
-@pytest.mark.parametrize("M,N,K,sliced", [(2048, 16, 2048, True), (1, 512, 2048, True), (130, 77, 1800, True), (2002, 512, 2048, True), (512, 512, 2002, True),
-                                          (100, 1000, 8192, True), (257, 130, 4100, True), (16, 6144, 2048, True), (64, 64, 8193, False), (512, 512, 256, False),
-                                          (4096, 4096, 2048, False)])
-def test_products_on_clusters_of_k_slices(M, N, K, sliced):
-    """Both orders of both operands, remainders in every dimension, a bias and a residual of odd rows, a factor, fp32 results; and
-    the rule's lines. Against 64 bits, and the sum of the slices is the same bits on every run."""
-    from nabla_b200.native import gemm as G
-
-    assert (G.cluster_slices(M, N, K) > 1) == sliced
-    torch.manual_seed(0)
-    mk = lambda r, c: torch.randn(r, c, device="cuda").bfloat16()  # noqa: E731
-    orders = [(mk(M, K), mk(K, N)), (mk(K, M).t(), mk(K, N)), (mk(M, K), mk(N, K).t()), (mk(K, M).t(), mk(N, K).t())]
-    bias, res, s = torch.randn(N, device="cuda"), mk(M, N), torch.tensor([0.5], device="cuda")
-    for a, b in orders if M * N < 1 << 22 else orders[:1]:
-        ref = a.double() @ b.double()
-        got = G.gemm_bf16(a, b)
-        assert _rel2(got, ref) < STORED[torch.bfloat16] and torch.equal(got, G.gemm_bf16(a, b))
-        # fp32 sums of K products of unit variance
-        assert _rel2(G.gemm_bf16(a, b, out_dtype=torch.float32), ref) < 4e-6
-        got = G.gemm_bf16(a, b, alpha=s, bias=bias, aux="add", aux_in=res)
-        assert _rel2(got, 0.5 * ref + bias.double() + res.double()) < STORED[torch.bfloat16]
-
-
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (256, 10, 1568), (33, 31, 32), (32, 32, 33), (65, 10, 4097), (7, 1000, 3), (1, 4000, 500), (3000, 1, 65), (255, 255, 255)])
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
 def test_small_fp32_products(M, N, K, ta, tb):
@@ -767,6 +744,60 @@ def test_adam_hyper():
             assert abs(a - b) <= 1e-7 * abs(b)
 
 
+@pytest.mark.parametrize("p_dtype,g_dtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_small_adamw_updates_in_one_launch(p_dtype, g_dtype):
+    """More tensors than a launch holds, sizes around a block's 2048 elements and the eight of a thread: the bits of one launch
+    each, in place or not; a misaligned tensor is refused."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(0)
+    sizes = [1, 7, 8, 9, 2047, 2048, 2049, 4096, 65537, 1 << 18] + list(range(11, 56))
+    mk = lambda n, dt: torch.randn(n, device="cuda").to(dt)  # noqa: E731
+    leaves = [(mk(n, p_dtype), mk(n, g_dtype), mk(n, torch.float32), mk(n, torch.float32).abs()) for n in sizes]
+    hyper = kernels.adam_hyper(torch.tensor(7.0, device="cuda"), 1e-3, 0.9, 0.999)
+    kw = dict(lr=1e-3, b1=0.9, b2=0.999, eps=1e-8, wd=0.01)
+    for extra in ({"hyper": hyper}, {"step": 7}, {}):
+        ref = [kernels.adamw(*leaf, **kw, **extra) for leaf in leaves]
+        flags = [i % 2 == 0 for i in range(len(sizes))]
+        mine = [tuple(t.clone() for t in leaf) for leaf in leaves]
+        got = kernels.adamw_group([(*leaf, f) for leaf, f in zip(mine, flags)], **kw, **extra)
+        for r, g, leaf, old, f in zip(ref, got, mine, leaves, flags):
+            assert all(torch.equal(a, b) for a, b in zip(r, g))
+            assert (g[0].data_ptr() == leaf[0].data_ptr()) == f and (f or torch.equal(leaf[0], old[0]))
+    odd = mk(17, torch.float32)[1:]
+    assert kernels.adamw_group([(mk(16, p_dtype), mk(16, g_dtype), odd, odd.clone(), False)], **kw) is None
+
+
+@pytest.mark.parametrize("donate", [False, True])
+def test_compiled_step_groups_its_small_updates(donate):
+    import nabla_b200 as nb
+    from nabla_b200 import nn
+
+    torch.manual_seed(0)
+    shapes = {"a": (64, 40), "b": (40,), "big": (600, 512), "c": (3,), "d": (512, 512)}
+    wrap = lambda d: {k: nb.Tensor.from_torch(v.clone()) for k, v in d.items()}  # noqa: E731
+    p = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
+    g = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
+    z = {k: torch.zeros(v, device="cuda") for k, v in shapes.items()}
+
+    def step(params, state, grads):
+        return nn.adamw_update(params, grads, state, lr=1e-2, weight_decay=0.1, realize=False)
+
+    f = nb.compile(step, cuda_graph=True, donate_argnums=(0, 1) if donate else ())
+    new, st = wrap(p), {"m": wrap(z), "v": wrap(z), "step": nb.Tensor.from_torch(torch.tensor(0.0, device="cuda"))}
+    ref = {k: v.double() for k, v in p.items()}
+    m = {k: v.double() for k, v in z.items()}
+    v2 = {k: v.double() for k, v in z.items()}
+    for t in range(1, 5):
+        new, st = f(new, st, wrap(g))
+        for k in p:
+            m[k] = 0.9 * m[k] + 0.1 * g[k].double()
+            v2[k] = 0.999 * v2[k] + 0.001 * g[k].double() ** 2
+            ref[k] = ref[k] - 1e-2 * ((m[k] / (1 - 0.9 ** t)) / ((v2[k] / (1 - 0.999 ** t)).sqrt() + 1e-8) + 0.1 * ref[k])
+            assert _rel2(new[k].to_torch(), ref[k]) < t * STORED[torch.float32]      # a rounding of p, m and v per step
+    assert sum("adamw_group" in line for line in str(f.dump_plan()).splitlines()) == 1
+
+
 # ---------------------------------------------------------------- column sums
 def test_column_sums_around_the_slab_counts():
     from nabla_b200.native import kernels
@@ -905,60 +936,6 @@ def test_compiled_calls_that_change_between_calls():
 
     def worker(n):
         try:
-@pytest.mark.parametrize("p_dtype,g_dtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
-def test_small_adamw_updates_in_one_launch(p_dtype, g_dtype):
-    """More tensors than a launch holds, sizes around a block's 2048 elements and the eight of a thread: the bits of one launch
-    each, in place or not; a misaligned tensor is refused."""
-    from nabla_b200.native import kernels
-
-    torch.manual_seed(0)
-    sizes = [1, 7, 8, 9, 2047, 2048, 2049, 4096, 65537, 1 << 18] + list(range(11, 56))
-    mk = lambda n, dt: torch.randn(n, device="cuda").to(dt)  # noqa: E731
-    leaves = [(mk(n, p_dtype), mk(n, g_dtype), mk(n, torch.float32), mk(n, torch.float32).abs()) for n in sizes]
-    hyper = kernels.adam_hyper(torch.tensor(7.0, device="cuda"), 1e-3, 0.9, 0.999)
-    kw = dict(lr=1e-3, b1=0.9, b2=0.999, eps=1e-8, wd=0.01)
-    for extra in ({"hyper": hyper}, {"step": 7}, {}):
-        ref = [kernels.adamw(*leaf, **kw, **extra) for leaf in leaves]
-        flags = [i % 2 == 0 for i in range(len(sizes))]
-        mine = [tuple(t.clone() for t in leaf) for leaf in leaves]
-        got = kernels.adamw_group([(*leaf, f) for leaf, f in zip(mine, flags)], **kw, **extra)
-        for r, g, leaf, old, f in zip(ref, got, mine, leaves, flags):
-            assert all(torch.equal(a, b) for a, b in zip(r, g))
-            assert (g[0].data_ptr() == leaf[0].data_ptr()) == f and (f or torch.equal(leaf[0], old[0]))
-    odd = mk(17, torch.float32)[1:]
-    assert kernels.adamw_group([(mk(16, p_dtype), mk(16, g_dtype), odd, odd.clone(), False)], **kw) is None
-
-
-@pytest.mark.parametrize("donate", [False, True])
-def test_compiled_step_groups_its_small_updates(donate):
-    import nabla_b200 as nb
-    from nabla_b200 import nn
-
-    torch.manual_seed(0)
-    shapes = {"a": (64, 40), "b": (40,), "big": (600, 512), "c": (3,), "d": (512, 512)}
-    wrap = lambda d: {k: nb.Tensor.from_torch(v.clone()) for k, v in d.items()}  # noqa: E731
-    p = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
-    g = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
-    z = {k: torch.zeros(v, device="cuda") for k, v in shapes.items()}
-
-    def step(params, state, grads):
-        return nn.adamw_update(params, grads, state, lr=1e-2, weight_decay=0.1, realize=False)
-
-    f = nb.compile(step, cuda_graph=True, donate_argnums=(0, 1) if donate else ())
-    new, st = wrap(p), {"m": wrap(z), "v": wrap(z), "step": nb.Tensor.from_torch(torch.tensor(0.0, device="cuda"))}
-    ref = {k: v.double() for k, v in p.items()}
-    m = {k: v.double() for k, v in z.items()}
-    v2 = {k: v.double() for k, v in z.items()}
-    for t in range(1, 5):
-        new, st = f(new, st, wrap(g))
-        for k in p:
-            m[k] = 0.9 * m[k] + 0.1 * g[k].double()
-            v2[k] = 0.999 * v2[k] + 0.001 * g[k].double() ** 2
-            ref[k] = ref[k] - 1e-2 * ((m[k] / (1 - 0.9 ** t)) / ((v2[k] / (1 - 0.999 ** t)).sqrt() + 1e-8) + 0.1 * ref[k])
-            assert _rel2(new[k].to_torch(), ref[k]) < t * STORED[torch.float32]      # a rounding of p, m and v per step
-    assert sum("adamw_group" in line for line in str(f.dump_plan()).splitlines()) == 1
-
-
             for _ in range(20):
                 call(n, torch.float32)
         except Exception as e:  # noqa: BLE001
