@@ -134,6 +134,32 @@ def tree_flatten(tree: Any, is_leaf: Callable[[Any], bool] | None = None) -> tup
     return leaves, td
 
 
+def leaves_as(td: PyTreeDef, tree: Any, out: list) -> bool:
+    """Append the leaves of ``tree`` in the order of ``td``, if it has that structure as far as lists, tuples, dicts and None
+    go (what stands in the place of a leaf is the caller's to look at); False for another structure and for registered
+    containers. A third of the time of ``tree_flatten`` and a comparison: no keys are sorted and no structure is built."""
+    k = td.kind
+    if k == "leaf":
+        out.append(tree)
+        return True
+    if k == "none":
+        return tree is None
+    if k == "dict":
+        if type(tree) is not dict or len(tree) != len(td.children):
+            return False
+        for key, c in zip(td.meta, td.children):
+            if key not in tree:
+                return False
+            if c is _LEAF:
+                out.append(tree[key])
+            elif not leaves_as(c, tree[key], out):
+                return False
+        return True
+    if (k == "list" and type(tree) is list or k == "tuple" and type(tree) is tuple) and len(tree) == len(td.children):
+        return all(leaves_as(c, x, out) for c, x in zip(td.children, tree))
+    return False
+
+
 def _unflatten(td: PyTreeDef, it) -> Any:
     k = td.kind
     if k == "leaf":

@@ -64,6 +64,19 @@ class TensorImpl:
         self._dtype = dtype
         self._device = device
 
+    @classmethod
+    def result_like(cls, like: "TensorImpl", buffers: list[torch.Tensor]) -> "TensorImpl":
+        """A realized impl with the shape, type and layout of ``like`` and nothing of its history (results of a replay)."""
+        new = cls.__new__(cls)
+        new._buffers = buffers
+        new._shape, new._dtype, new._device = like._shape, like._dtype, like._device
+        new.sharding, new.batch_dims = like.sharding, like.batch_dims
+        new.is_traced = new.requires_grad = False
+        new.sharding_constraint = new.grad = new.tangent = new.cotangent = new.dual = None
+        new.output_refs = new._local_shapes = new._keepalive = None
+        new.output_index = 0
+        return new
+
     # ---- state
     @property
     def is_realized(self) -> bool:

@@ -8,6 +8,7 @@ which makes the following head-merge reshape free.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -33,7 +34,7 @@ def _lib():
             f.argtypes = [c_vp] * 5 + [c_int] * 5 + [c_ll] * 12 + [c_f, c_int, c_vp, c_ll, c_ll, c_ll, c_int, c_vp, c_vp, c_vp, c_vp]
             lib.nb_attn_fwd_splits.restype = c_int
             lib.nb_attn_fwd_splits.argtypes = [c_int] * 6
-            _splits = lib.nb_attn_fwd_splits
+            _splits = functools.lru_cache(1024)(lib.nb_attn_fwd_splits)      # a function of the sizes alone
             _fwd = f
             if hasattr(lib, "nb_attn_bwd"):
                 g = lib.nb_attn_bwd
@@ -44,7 +45,10 @@ def _lib():
 
 
 def _ok_view(t: torch.Tensor) -> bool:
-    return (t.dim() == 4 and t.stride(3) == 1 and all(s % 8 == 0 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0)
+    if t.dim() != 4:
+        return False
+    sb, sh, ss, sd = t.stride()
+    return sd == 1 and not (sb | sh | ss) & 7 and not t.data_ptr() & 15
 
 
 def supported(q, k, v, mask, dropout_p) -> bool:
@@ -116,8 +120,7 @@ def sdpa_fwd(q, k, v, *, causal: bool, scale: float, mask=None):
     p_o = 0 if part is None else part.data_ptr()
     p_lse = 0 if part is None else p_o + ns * B * H * Sq * D * 4
     rc = _lib()(ptr(q), ptr(k), ptr(v), ptr(o_mem), ptr(lse), B, H, Sq, Skv, D,
-              q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
-              v.stride(0), v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2),
+              *q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *o.stride()[:3],
               float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()), m_sb, m_sh, m_sq, ns, c_vp(p_o), c_vp(p_lse),
               ptr(st), stream_ptr())
     if rc != 0:
@@ -149,7 +152,7 @@ def sdpa_bwd(do, q, k, v, o, lse, *, causal: bool, scale: float, out=None, mask=
     args = [ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse.contiguous()), ptr(dq), ptr(dk), ptr(dv), ptr(stats)]
     strides = []
     for t in (q, k, v, do, o, dq, dk, dv):
-        strides += [t.stride(0), t.stride(1), t.stride(2)]
+        strides += t.stride()[:3]
     rc = _bwd(*args, B, H, Sq, Skv, D, *strides, float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()),
               m_sb, m_sh, m_sq, ptr(st), stream_ptr())
     if rc != 0:

@@ -222,10 +222,10 @@ def _normalize_step_scalars(tree: Any, depth: int = 0) -> Any:
             out = dict(tree)
             out["step"] = constant(float(step), dtype=DType.float32, device=first.device if first is not None else None)
             return out
-        if depth < 1:
+        if depth < 1 and (type(tree) is not dict or any(isinstance(v, dict) for v in tree.values())):      # nothing else is looked into one level down
             return {k: _normalize_step_scalars(v, depth + 1) for k, v in tree.items()}
         return tree
-    if depth < 1 and isinstance(tree, (list, tuple)) and not hasattr(tree, "_fields"):
+    if depth < 1 and isinstance(tree, (list, tuple)) and not hasattr(tree, "_fields") and any(isinstance(v, dict) for v in tree):
         return type(tree)(_normalize_step_scalars(v, depth + 1) for v in tree)
     return tree
 
@@ -367,17 +367,20 @@ class CompiledFunction:
                     return None
                 leaves.append(a)
                 continue
-            lv, td_a = pytree.tree_flatten(a)
-            if td_a != td:
-                return None
-            leaves += lv
+            at = len(leaves)
+            if not pytree.leaves_as(td, a, leaves):
+                del leaves[at:]
+                lv, td_a = pytree.tree_flatten(a)
+                if td_a != td:
+                    return None
+                leaves += lv
         for leaf, c in zip(leaves, conc):
             if type(leaf) is not Tensor:
                 return None
             im = leaf._impl
             # conc: (shape, dtype, sharding signature, batch dims, device); only unsharded calls are kept
             if im._shape != c[0] or im._dtype is not c[1] or im.sharding is not None or im.batch_dims != c[3] \
-                    or im._device != c[4] or im._buffers is None:
+                    or im._buffers is None or (im._device is not c[4] and im._device != c[4]):
                 return None
         return leaves
 
@@ -516,11 +519,11 @@ class CompiledFunction:
         if any(rec.donated):
             rec.steps = _optimizer_steps_last(rec.steps, nodes)
             rec.steps = _bucket_small_all_reduces(rec.steps, nodes)
+        if plan is not None:
+            rec.steps = _group_small_updates(rec.steps, nodes)
         # liveness: free an intermediate after the last step that reads it
         out_ids = {id(i) for i in rec.out_impls if i is not None}
         produced = {id(o): o for outs in rec.keep for o in outs}
-        if plan is not None:
-            rec.steps = _group_small_updates(rec.steps, nodes)
         last_use: dict[int, int] = {}
         ph_ids = {id(p) for p in rec.placeholders}
         ph_last_use: dict[int, int] = {}
@@ -773,9 +776,7 @@ class CompiledFunction:
             if impl is None:
                 outs.append(static)
                 continue
-            new = TensorImpl(list(impl._buffers), shape=impl._shape, dtype=impl.dtype, device=impl.device,
-                             sharding=impl.sharding, batch_dims=impl.batch_dims)
-            outs.append(Tensor(impl=new))
+            outs.append(Tensor(impl=TensorImpl.result_like(impl, list(impl._buffers))))
         # drop our references to output buffers produced by nodes (placeholders are re-bound per call)
         ph = {id(p) for p in rec.placeholders}
         for impl in rec.out_impls:
@@ -849,9 +850,7 @@ class CompiledFunction:
             rec.copy_out = CopyBatch([b for impl, bufs, cached in zip(rec.out_impls, rec.static_outputs, rec.out_cached)
                                       if impl is not None and cached is None for b in bufs if b.data_ptr() not in rec.static_ptrs])
         # every other result leaves the graph's memory: fresh tensors, filled by one launch
-        fresh = [torch.empty_like(b) for b in rec.copy_out.fixed]
-        rec.copy_out.run(fresh, into_fixed=False)
-        taken = iter(fresh)
+        taken = iter(rec.copy_out.fresh())
         outs = []
         for impl, static, bufs, cached in zip(rec.out_impls, rec.out_static, rec.static_outputs, rec.out_cached):
             if impl is None:
@@ -859,10 +858,8 @@ class CompiledFunction:
             elif cached is not None:
                 outs.append(cached)
             else:
-                res = [b if b.data_ptr() in rec.static_ptrs else next(taken) for b in bufs]
-                new = TensorImpl(res, shape=impl._shape, dtype=impl.dtype, device=impl.device,
-                                 sharding=impl.sharding, batch_dims=impl.batch_dims)
-                outs.append(Tensor(impl=new))
+                res = [b if b.data_ptr() in rec.static_ptrs else next(taken) for b in bufs] if rec.static_ptrs else [next(taken) for _ in bufs]
+                outs.append(Tensor(impl=TensorImpl.result_like(impl, res)))
         return pytree.tree_unflatten(rec.out_treedef, outs)
 
 
