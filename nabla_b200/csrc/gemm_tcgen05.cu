@@ -783,6 +783,179 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   gemm_cta<BN, MODE_NONE, true>(&tmA, &tmB, args, none, blockIdx.x >> 1, gridDim.x >> 1);
 }
 
+// The K range of a tile on a cluster of SLICES CTAs: each multiplies its k-blocks and lays its fp32 tile over the ring that
+// has been read; then each adds up 128 / SLICES rows of all of them, read through distributed shared memory in whole rows
+// (sending the rows instead, 16 bytes of each by a lane, cost some 4 us more). For products with too few tiles for the chip:
+// what bounds a CTA there is the rate at which it loads operands (64 bytes a clock, 384 clocks for the k-block of a 128 x 64
+// tile whose MMAs take 176). One launch, no fp32 partial results in memory, the slices added in order. Bias and residual are
+// added by the sum; no other epilogue.
+// us, whole tiles of the best width and slices: 2048 x 16 x 2048 11.1, 5.9; 2002 x 512 x 2048 10.8, 9.7; 777 x 1024 x 4096 17.1,
+// 13.2; 100 x 512 x 2048 10.1, 5.4; 64 x 256 x 512 5.3, 4.5.
+template <int BN, int SLICES>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_bf16_slices_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs args) {
+  using L = SmemLayout<BN>;
+  constexpr int STAGES = L::STAGES, LDP = BN + 4;      // floats per partial row, padded against bank conflicts
+  static_assert(BLOCK_M * LDP * 4 <= L::RING_BYTES, "the partial rows fit the ring");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring + L::RING_BYTES);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tmem_full = empty_bar + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_ctarank();
+  const int num_m = (args.M + BLOCK_M - 1) / BLOCK_M, num_n = (args.N + BN - 1) / BN;
+  int b, tm, tn;
+  tile_coords(blockIdx.x / SLICES, num_m, num_n, b, tm, tn);
+  const int m0 = tm * BLOCK_M, n0 = tn * BN;
+  // (the launcher leaves no slice without a k-block)
+  const int num_kb = (args.K + BLOCK_K - 1) / BLOCK_K, per = (num_kb + SLICES - 1) / SLICES;
+  const int kb0 = (int)crank * per, kb1 = min(num_kb, kb0 + per);
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(&full_bar[i], 1);
+      mbar_init(&empty_bar[i], 1);
+    }
+    mbar_init(tmem_full, 1);
+    fence_mbar_init();
+    fence_proxy_async_smem();
+  }
+  if (warp == 2) {
+    tmem_alloc(tmem_slot, BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      for (int i = 0; i < kb1 - kb0; ++i) {
+        const int st = i % STAGES, k0 = (kb0 + i) * BLOCK_K;
+        if (!mbar_wait(&empty_bar[st], ((i / STAGES) & 1) ^ 1)) { atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER); break; }
+        if (!(NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, k0, args.K) && NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, m0, args.M) &&
+              NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, n0, args.N) &&
+              NB_ALIGNED(NB_SITE_GEMM_TMA_ALIGN, (args.a_mn ? m0 : k0) * 2, 16) &&
+              NB_ALIGNED(NB_SITE_GEMM_TMA_ALIGN, (args.b_mn ? n0 : k0) * 2, 16)))
+          break;
+        uint8_t* sA = ring + st * L::STAGE_BYTES;
+        uint8_t* sB = sA + L::A_BYTES;
+        mbar_arrive_expect_tx(&full_bar[st], L::STAGE_BYTES);
+        if (!args.a_mn) {
+          tma_load_3d(sA, &tmA, &full_bar[st], k0, m0, 0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_3d(sA + j * (BLOCK_K * 128), &tmA, &full_bar[st], m0 + j * 64, k0, 0);
+        }
+        if (!args.b_mn) {
+          tma_load_3d(sB, &tmB, &full_bar[st], k0, n0, 0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j) tma_load_3d(sB + j * (BLOCK_K * 128), &tmB, &full_bar[st], n0 + j * 64, k0, 0);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(BLOCK_M, BN, args.a_mn, args.b_mn);
+      const uint32_t a_lbo = args.a_mn ? BLOCK_K * 128 : 16, b_lbo = args.b_mn ? BLOCK_K * 128 : 16;
+      const uint32_t a_kstep = args.a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      const uint32_t b_kstep = args.b_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      bool ok = true;
+      for (int i = 0; i < kb1 - kb0 && ok; ++i) {
+        const int st = i % STAGES;
+        ok = mbar_wait(&full_bar[st], (i / STAGES) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sA = smem_u32(ring + st * L::STAGE_BYTES);
+        const uint64_t da = make_smem_desc_sw128(sA, a_lbo, 1024), db = make_smem_desc_sw128(sA + L::A_BYTES, b_lbo, 1024);
+#pragma unroll
+        for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+          umma_f16_ss(tmem_base, da + static_cast<uint64_t>(k * a_kstep), db + static_cast<uint64_t>(k * b_kstep), idesc,
+                      (i | k) != 0 ? 1u : 0u);
+        umma_commit(&empty_bar[st]);
+      }
+      if (ok) umma_commit(tmem_full);
+      else atomicExch(args.status, NB_ERR_TIMEOUT_MMA);
+    }
+  } else if (warp >= 4 && warp < 8) {
+    // every load of the ring is read by an MMA that this barrier waits for
+    if (!mbar_wait(tmem_full, 0)) atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
+    tc_fence_after();
+    float* row = reinterpret_cast<float*>(ring) + ((warp & 3) * 32 + lane) * LDP;
+#pragma unroll
+    for (int c = 0; c < BN; c += 32) {
+      uint32_t v[32];
+      tmem_ld_32x32(tmem_base + c + (static_cast<uint32_t>((warp & 3) * 32) << 16), v);
+      tmem_ld_wait_regs(v);
+#pragma unroll
+      for (int q = 0; q < 32; q += 4) *reinterpret_cast<uint4*>(row + c + q) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  cluster_sync_all();                    // the tiles of all slices are laid out
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BN);
+  }
+  float alpha = args.alpha;
+  if (args.alpha_dev != nullptr)
+    alpha *= args.alpha_fp32 ? *reinterpret_cast<const float*>(args.alpha_dev)
+                             : __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(args.alpha_dev));
+  constexpr int ROWS = BLOCK_M / SLICES;   // rows that a CTA adds up
+  uint32_t part[SLICES];
+#pragma unroll
+  for (int z = 0; z < SLICES; ++z) part[z] = mapa_shared(smem_u32(ring) + crank * (ROWS * LDP * 4), z);
+#pragma unroll 2
+  for (int i = threadIdx.x; i < ROWS * (BN / 4); i += NUM_THREADS) {
+    const int r = i / (BN / 4), c = (i - r * (BN / 4)) * 4, m = m0 + (int)crank * ROWS + r, n = n0 + c;
+    if (m >= args.M || n >= args.N) continue;
+    float4 p[SLICES];
+#pragma unroll
+    for (int z = 0; z < SLICES; ++z)
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(p[z].x), "=f"(p[z].y), "=f"(p[z].z), "=f"(p[z].w)
+                   : "r"(part[z] + (r * LDP + c) * 4)
+                   : "memory");
+    float4 t = p[0];
+#pragma unroll
+    for (int z = 1; z < SLICES; ++z) { t.x += p[z].x; t.y += p[z].y; t.z += p[z].z; t.w += p[z].w; }
+    float f[4] = {t.x * alpha, t.y * alpha, t.z * alpha, t.w * alpha};
+    const long long at = static_cast<long long>(m) * args.ldc + n;
+    if (!NB_IN_BOUNDS(NB_SITE_GEMM_STORE, at, static_cast<long long>(args.M - 1) * args.ldc + args.N)) continue;
+    const int cols = min(4, args.N - n);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j >= cols) continue;
+      if (args.bias != nullptr && args.epi == EPI_BIAS)
+        f[j] += args.bias_fp32 ? reinterpret_cast<const float*>(args.bias)[n + j]
+                               : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(args.bias)[n + j]);
+      if (args.aux == AUX_ADD) f[j] += __bfloat162float(args.aux_in[static_cast<long long>(m) * args.ld_aux + n + j]);
+    }
+    if (args.out_fp32) {
+      float* o = reinterpret_cast<float*>(args.out) + at;
+      if (cols == 4 && args.vec_ok) *reinterpret_cast<float4*>(o) = make_float4(f[0], f[1], f[2], f[3]);
+      else for (int j = 0; j < cols; ++j) o[j] = f[j];
+    } else {
+      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(args.out) + at;
+      if (cols == 4 && args.vec_ok) {
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(f[0], f[1]), __floats2bfloat162_rn(f[2], f[3])};
+        *reinterpret_cast<uint2*>(o) = *reinterpret_cast<uint2*>(h);
+      } else {
+        for (int j = 0; j < cols; ++j) o[j] = __float2bfloat16(f[j]);
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();                    // the others have read this CTA's rows
+}
+
 // Probe of the tensor-memory allocator for CTA pairs, run once before the pair GEMM is used: both
 // CTAs of one cluster ask for 256 columns with cta_group::2 and report the base they were given.
 // 2 x 256 columns fit the 512 of an SM, so neither request can wait for the other whichever way the
@@ -1279,6 +1452,87 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+// Largest tile that still gives every SM a tile; small problems use narrower tiles.
+static int tile_width(int M, int N, int batch) {
+  const long long m_tiles = (M + BLOCK_M - 1) / BLOCK_M;
+  int bn = 256;
+  if (N <= 64 || m_tiles * ((N + 255) / 256) * batch < g_num_sms / 2) bn = 128;
+  if (N <= 64 || (bn == 128 && m_tiles * ((N + 127) / 128) * batch < g_num_sms / 2)) bn = 64;
+  return bn;
+}
+
+// Slices of K that a product is given to clusters for (1: none), and their tile width. In clocks: a CTA loads a k-block in
+// 2 (128 + bn) and stores a tile in 16 bn; the exchange of the slices and its two barriers take some 1400. Only where all
+// slices run at once and a tenth and 600 clocks are saved (us, whole and sliced: 1 x 512 x 512 5.2, 4.1; 100 x 768 x 768 6.2,
+// 5.6; outside the line 100 x 2048 x 512 5.5, 5.3; 1332 x 512 x 512 5.7, 6.6; slices that do not run at once 5.9, 10.1). The clusters that fit are asked for once (-1: not yet).
+struct SlicePlan { int bn, slices; };
+static int g_slice_clusters[2][4] = {{-1, -1, -1, -1}, {-1, -1, -1, -1}};   // [bn 64, 128][log2 slices]
+template <int BN, int SLICES>
+static int slice_clusters() {
+  int& n = g_slice_clusters[BN == 128][SLICES == 2 ? 1 : SLICES == 4 ? 2 : 3];
+  if (n < 0) {
+    n = 0;
+    const auto kernel = gemm_bf16_slices_kernel<BN, SLICES>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemLayout<BN>::TOTAL) == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = SLICES;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(SLICES);
+      cfg.blockDim = dim3(NUM_THREADS);
+      cfg.dynamicSmemBytes = SmemLayout<BN>::TOTAL;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int k = 0;
+      if (cudaOccupancyMaxActiveClusters(&k, kernel, &cfg) == cudaSuccess) n = k;
+    }
+    if (n == 0) cudaGetLastError();      // the query's own error: the other kernels serve
+  }
+  return n;
+}
+template <int BN>
+static int slice_clusters(int slices) {
+  return slices == 2 ? slice_clusters<BN, 2>() : slices == 4 ? slice_clusters<BN, 4>() : slice_clusters<BN, 8>();
+}
+static SlicePlan slice_plan(int M, int N, int K, int bn) {
+  SlicePlan best{bn, 1};
+  if (bn == 256 || K > 8192) return best;              // (wide tiles: enough of them for the chip)
+  const long long kb = (K + BLOCK_K - 1) / BLOCK_K, m_t = (M + BLOCK_M - 1) / BLOCK_M;
+  const long long tiles0 = m_t * ((N + bn - 1) / bn);
+  const double t0 = (double)((tiles0 + g_num_sms - 1) / g_num_sms) * kb * 2 * (BLOCK_M + bn) + 16 * bn;
+  double t_best = 0.9 * t0 < t0 - 600 ? 0.9 * t0 : t0 - 600;
+  for (int w = 64; w <= 128; w *= 2)
+    for (int z = 2; z <= 8; z *= 2) {
+      const long long tiles = m_t * ((N + w - 1) / w), per = (kb + z - 1) / z;
+      if ((z - 1) * per >= kb || tiles * z > g_num_sms) continue;
+      const double t = (double)per * 2 * (BLOCK_M + w) + 16 * w + 1400;
+      if (t < t_best && tiles <= (w == 64 ? slice_clusters<64>(z) : slice_clusters<128>(z))) {
+        t_best = t;
+        best = SlicePlan{w, z};
+      }
+    }
+  return best;
+}
+template <int BN>
+static int launch_slices(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, int slices, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = slices;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(((a.M + BLOCK_M - 1) / BLOCK_M) * ((a.N + BN - 1) / BN) * slices));
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SmemLayout<BN>::TOTAL;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const auto kernel = slices == 2 ? gemm_bf16_slices_kernel<BN, 2> : slices == 4 ? gemm_bf16_slices_kernel<BN, 4> : gemm_bf16_slices_kernel<BN, 8>;
+  return cudaLaunchKernelEx(&cfg, kernel, ta, tb, a) == cudaSuccess ? 0 : -3;
+}
+
 // bit 0: CTA pairs for 256-wide tiles of plain GEMMs with at least one tile pair per two SMs;
 // bit 1: CTA pairs in the fused GEMM + collective kernels (even number of 128-row tiles). 0: lone CTAs only
 static int g_pair_mode = 0;
@@ -1347,6 +1601,18 @@ extern "C" int nb_gemm_pair_alloc_probe(unsigned* out2, void* stream) {
   return cudaLaunchKernelEx(&cfg, nb::pair_alloc_probe_kernel, out2) == cudaSuccess ? 0 : -3;
 }
 
+// Slices of K that nb_gemm_bf16 cuts a plain product of one batch into by itself (1: none).
+extern "C" int nb_gemm_slices(int M, int N, int K) {
+  using namespace nb;
+  if (M <= 0 || N <= 0 || K <= 0) return 1;
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return slice_plan(M, N, K, tile_width(M, N, 1)).slices;
+}
+
 // C entry point. All leading dimensions / strides are in elements.
 //   A: a_mn == 0 -> [batch][M][K] (K contiguous, row stride lda); a_mn == 1 -> [batch][K][M]
 //   B: b_mn == 0 -> [batch][N][K] (K contiguous, row stride ldb); b_mn == 1 -> [batch][K][N]
@@ -1370,13 +1636,11 @@ extern "C" int nb_gemm_bf16(const void* A, const void* B, void* C, const void* b
   }
   if (max_ctas <= 0 || max_ctas > g_num_sms) max_ctas = g_num_sms;
   int bn = block_n;
-  if (bn != 256 && bn != 128 && bn != 64) {
-    // Largest tile that still gives every SM a tile; small problems use narrower tiles.
-    const long long m_tiles = (M + BLOCK_M - 1) / BLOCK_M;
-    bn = 256;
-    if (N <= 64 || m_tiles * ((N + 255) / 256) * batch < g_num_sms / 2) bn = 128;
-    if (N <= 64 || (bn == 128 && m_tiles * ((N + 127) / 128) * batch < g_num_sms / 2)) bn = 64;
-  }
+  if (bn != 256 && bn != 128 && bn != 64) bn = tile_width(M, N, batch);
+  const bool sliceable = batch == 1 && !accumulate && (epi == EPI_NONE || epi == EPI_BIAS) && (aux == AUX_NONE || aux == AUX_ADD) &&
+                         block_n == 0 && max_ctas == g_num_sms;
+  const SlicePlan plan = sliceable ? slice_plan(M, N, K, bn) : SlicePlan{bn, 1};
+  bn = plan.bn;
   CUtensorMap ta, tb;
   int r;
   if (!a_mn) r = make_map(&ta, A, K, M, batch, lda, stride_a, BLOCK_M);
@@ -1415,6 +1679,7 @@ extern "C" int nb_gemm_bf16(const void* A, const void* B, void* C, const void* b
             (batch == 1 || (stride_aux * 2) % 32 == 0);
   g.vec32_ok = vec32 ? 1 : 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (plan.slices > 1) return bn == 64 ? launch_slices<64>(ta, tb, g, plan.slices, s) : launch_slices<128>(ta, tb, g, plan.slices, s);
   if (pair) return launch_pair<256>(ta, tb, g, max_ctas, s);
   if (bn == 256) return launch<256>(ta, tb, g, max_ctas, s);
   if (bn == 128) return launch<128>(ta, tb, g, max_ctas, s);

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -23,6 +24,8 @@ def _get():
         fn.restype = ctypes.c_int
         fn.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int] * 4 + [ctypes.c_longlong] * 8 + [ctypes.c_int] * 8 + [
             ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+        lib.nb_gemm_slices.argtypes = [ctypes.c_int] * 3
+        lib.nb_gemm_slices.restype = ctypes.c_int
         lib.nb_gemm_set_pair_mode.argtypes = [ctypes.c_int]
         lib.nb_gemm_set_pair_mode.restype = ctypes.c_int
         lib.nb_gemm_pair_alloc_probe.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
@@ -116,6 +119,15 @@ def gemm_supported(a: torch.Tensor, b: torch.Tensor) -> bool:
 _SMS = 0
 
 
+@functools.lru_cache(1024)
+def cluster_slices(M: int, N: int, K: int) -> int:
+    """Slices of K that the kernel itself cuts this product into, on a cluster of CTAs each (1: none)."""
+    from . import load
+
+    _get()
+    return load("libnb_gemm.so").nb_gemm_slices(M, N, K)
+
+
 def split_k_factor(M: int, N: int, K: int) -> int:
     """How many K slices a weight-gradient-shaped GEMM (few output tiles, long K) is cut into: 1 (no
     split), 2, 4 or 8. A small cost model of the kernel picks it: whole waves of tiles over the SMs,
@@ -153,7 +165,9 @@ def split_k_factor(M: int, N: int, K: int) -> int:
         t = est(s)
         if t < 0.93 * best_t:
             best, best_t = s, t
-    return best
+    # Slices on clusters need no second launch (us, this split and those: 64 x 256 x 8192 11.3, 7.6; 1024 x 1024 x 4096 19.1, 12.9);
+    # fewer of them would be longer fp32 sums.
+    return 1 if best > 1 and cluster_slices(M, N, K) >= best else best
 
 
 def _k_slices(t3: torch.Tensor, kind: str, ld: int, s: int, k_dim: int) -> torch.Tensor:

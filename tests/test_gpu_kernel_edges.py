@@ -202,6 +202,33 @@ def test_compiled_products_take_their_adds_and_factors(tokens, dim, out, rank):
     assert "gemm_residual" not in str(h.dump_plan()) and _rel2(p.to_torch(), x.double() @ w.double()) < STORED[torch.bfloat16]
 
 
+@pytest.mark.parametrize("M,N,K,sliced", [(2048, 16, 2048, True), (1, 512, 2048, True), (130, 77, 1800, True), (2002, 512, 2048, True), (512, 512, 2002, True),
+                                          (100, 1000, 8192, True), (257, 130, 4100, True), (16, 6144, 2048, True), (64, 64, 8193, False), (512, 512, 256, False), (64, 256, 512, True),
+                                          (70, 100, 449, True), (512, 512, 8192, True), (4096, 4096, 2048, False)])
+def test_products_on_clusters_of_k_slices(M, N, K, sliced):
+    """Both orders of both operands, remainders in every dimension, a bias and a residual of odd rows, a factor, fp32 results; and
+    the rule's lines. Against 64 bits, and the sum of the slices is the same bits on every run."""
+    from nabla_b200.native import gemm as G
+
+    assert (G.cluster_slices(M, N, K) > 1) == sliced
+    assert G.split_k_factor(M, N, K) in (1, 8) and (G.split_k_factor(M, N, K) == 8) == ((M, N, K) == (512, 512, 8192))
+    torch.manual_seed(0)
+    mk = lambda r, c: torch.randn(r, c, device="cuda").bfloat16()  # noqa: E731
+    orders = [(mk(M, K), mk(K, N)), (mk(K, M).t(), mk(K, N)), (mk(M, K), mk(N, K).t()), (mk(K, M).t(), mk(N, K).t())]
+    bias, res, s = torch.randn(N, device="cuda"), mk(M, N), torch.tensor([0.5], device="cuda")
+    for a, b in orders if M * N < 1 << 22 else orders[:1]:
+        ref = a.double() @ b.double()
+        got = G.gemm_bf16(a, b)
+        assert _rel2(got, ref) < STORED[torch.bfloat16] and torch.equal(got, G.gemm_bf16(a, b))
+        # each MMA of 16 products cuts its fp32 sum by less than one unit in the last place: a slice has fewer of them
+        err = _rel2(G.gemm_bf16(a, b, out_dtype=torch.float32), ref)
+        assert err < (K / 16 / G.cluster_slices(M, N, K) + 8) * 2.0**-23
+        if sliced:
+            assert err <= _rel2(G.gemm_bf16(a, b, out_dtype=torch.float32, block_n=64, split_k=1), ref)
+        got = G.gemm_bf16(a, b, alpha=s, bias=bias, aux="add", aux_in=res)
+        assert _rel2(got, 0.5 * ref + bias.double() + res.double()) < STORED[torch.bfloat16]
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (256, 10, 1568), (33, 31, 32), (32, 32, 33), (65, 10, 4097), (7, 1000, 3), (1, 4000, 500), (3000, 1, 65), (255, 255, 255)])
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
 def test_small_fp32_products(M, N, K, ta, tb):
