@@ -1833,6 +1833,13 @@ __device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
   v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xffff0000u);
   v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xffff0000u);
 }
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void store4(bf16* p, const float (&v)[4]) {
+  const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+  *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
+}
 
 constexpr int CONV_KC = 32;      // values of k staged at a time
 
@@ -1945,6 +1952,136 @@ __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict_
       if (f >= g.F) break;
       if (odd) acc[i][j] = conv_point<T>(x, w, bias ? to_f<T>(bias[f]) : 0.f, g, m, f);
       y[m * g.F + f] = from_f<T>(acc[i][j]);
+    }
+  }
+}
+
+// Input patch of `rows` x pw pixels whose first is (ih0, iw0) of an image, nq groups of KV channels from group q0 on, to xs as
+// [nq][rows][pw] of KV floats; zeros outside the image. The coordinates of a thread's next pixel follow from those of the last (two divisions per value took as long
+// as the loads).
+template <typename T, bool VEC>
+__device__ __forceinline__ void stage_patch(const T* __restrict__ image, float* __restrict__ xs, const ConvGeom& g, int n, int ih0,
+                                            int iw0, int rows, int pw, int q0, int nq) {
+  constexpr int KV = VEC ? 4 : 1;
+  const int plane = rows * pw, step = 128 / nq, dq = 128 - step * nq, dr = step / pw, dc = step - dr * pw;
+  int pix = threadIdx.x / nq, q = threadIdx.x - pix * nq, pr = pix / pw, pc = pix - pr * pw;
+#pragma unroll 4
+  while (pix < plane) {
+    const int ih = ih0 + pr, iw = iw0 + pc;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W && NB_IN_BOUNDS(NB_SITE_CONV_INPUT, n, g.N)) {
+      const T* p = image + ((size_t)ih * g.W + iw) * g.C + (q0 + q) * KV;
+      if (VEC) load4(p, v);
+      else v[0] = to_f<T>(*p);
+    }
+    if (VEC) *reinterpret_cast<float4*>(xs + (q * plane + pix) * 4) = make_float4(v[0], v[1], v[2], v[3]);
+    else xs[q * plane + pix] = v[0];
+    const int carry = q + dq >= nq;
+    q += dq - carry * nq;
+    pix += step + carry;
+    pc += dc + carry;
+    pr += dr;
+    if (pc >= pw) { pc -= pw; ++pr; }
+  }
+}
+
+// The same sums from a patch: a block stages the input of TH rows of one image's output once, with its halo, and the whole
+// filter tile, and walks (r, s, c) by addresses, where the kernel above stages every input value once per filter tap. A
+// thread has PX positions (lanes take consecutive ones) and 4 channels; VEC: four input channels per shared load, kept as
+// float4 planes so that lanes read consecutive ones. The additions are those of the kernel above, in its order: the same bits.
+// Bound by the shared-memory pipe (71 % of its active time) under 2 PX + 4 wavefronts per 16 PX FMAs, and by the staging before
+// them; 128 registers, so that 512 blocks run at once. us, tiled and from patches, fp32, 3 x 3: 256 x 14 x 14 x 16 -> 32
+// 28.8, 23.2; 256 x 14 x 14 x 32 -> 16 (an input gradient) 40.2, 24.9; 256 x 28 x 28 x 1 -> 16 14.0, 12.5; 16 x 32 x 32 x 8 -> 16
+// 7.5, 5.5; bf16 within a tenth of these.
+template <typename T, int FG, int PX, bool VEC>
+__global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restrict__ x, const T* __restrict__ w,
+                                                          const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g,
+                                                          int TH, int bands, int wvec, int yvec) {
+  constexpr int PG = 128 / FG, FT = 4 * FG, KV = VEC ? 4 : 1;
+  extern __shared__ __align__(16) float conv_smem[];
+  const int tid = threadIdx.x, K = g.R * g.S * g.C, CQ = g.C / KV;
+  const int pw = (g.OW - 1) * g.sw + g.S, ph = (TH - 1) * g.sh + g.R, plane = pw * ph;
+  float* ws = conv_smem;                             // [K][FT]
+  float* xs = conv_smem + K * FT;                    // [CQ][ph][pw] of KV floats
+  const int n = blockIdx.x / bands, oh0 = (blockIdx.x - n * bands) * TH, f0 = blockIdx.y * FT;
+  int odd = 0;                                       // a filter value that is not finite was staged
+  if (wvec) {
+#pragma unroll 4
+    for (int e = tid; e < K * (FT / 4); e += 128) {
+      const int f = f0 + e % (FT / 4) * 4;
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (f < g.F) load4(w + (size_t)(e / (FT / 4)) * g.F + f, v);
+      odd |= !isfinite(v[0]) | !isfinite(v[1]) | !isfinite(v[2]) | !isfinite(v[3]);
+      *reinterpret_cast<float4*>(ws + e * 4) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  } else {
+#pragma unroll 4
+    for (int e = tid; e < K * FT; e += 128) {
+      const int f = f0 + e % FT;
+      const float v = f < g.F ? to_f<T>(w[(size_t)(e / FT) * g.F + f]) : 0.f;
+      odd |= !isfinite(v);
+      ws[e] = v;
+    }
+  }
+  stage_patch<T, VEC>(x + (size_t)n * g.H * g.W * g.C, xs, g, n, oh0 * g.sh - g.pt, -g.pl, ph, pw, 0, CQ);
+  const int pg = tid % PG, fg = tid / PG;
+  int at[PX];
+  float acc[PX][4];
+#pragma unroll
+  for (int i = 0; i < PX; ++i) {
+    const int p = pg + i * PG, r = p / g.OW, c = p - r * g.OW;
+    at[i] = r < TH ? r * g.sh * pw + c * g.sw : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int f = f0 + fg * 4 + j;
+      acc[i][j] = bias && f < g.F ? to_f<T>(bias[f]) : 0.f;
+    }
+  }
+  __syncthreads();
+  const float* wp = ws + fg * 4;
+  for (int r = 0; r < g.R; ++r)
+    for (int s = 0; s < g.S; ++s)
+      for (int q = 0; q < CQ; ++q) {
+        const float* xp = xs + (q * plane + r * pw + s) * KV;
+        float a[PX][KV];
+#pragma unroll
+        for (int i = 0; i < PX; ++i) {
+          if constexpr (VEC) {
+            const float4 t = *reinterpret_cast<const float4*>(xp + at[i] * 4);
+            a[i][0] = t.x; a[i][1] = t.y; a[i][2] = t.z; a[i][3] = t.w;
+          } else {
+            a[i][0] = xp[at[i]];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < KV; ++k) {
+          const float4 b = *reinterpret_cast<const float4*>(wp);
+          wp += FT;
+#pragma unroll
+          for (int i = 0; i < PX; ++i) {
+            acc[i][0] = fmaf(a[i][k], b.x, acc[i][0]);
+            acc[i][1] = fmaf(a[i][k], b.y, acc[i][1]);
+            acc[i][2] = fmaf(a[i][k], b.z, acc[i][2]);
+            acc[i][3] = fmaf(a[i][k], b.w, acc[i][3]);
+          }
+        }
+      }
+  odd = __syncthreads_or(odd);
+#pragma unroll
+  for (int i = 0; i < PX; ++i) {
+    const int p = pg + i * PG, r = p / g.OW, c = p - r * g.OW, oh = oh0 + r, f = f0 + fg * 4;
+    if (r >= TH || oh >= g.OH || f >= g.F) continue;
+    const long long m = ((long long)n * g.OH + oh) * g.OW + c;
+    if (odd) {
+      for (int j = 0; j < 4 && f + j < g.F; ++j) acc[i][j] = conv_point<T>(x, w, bias ? to_f<T>(bias[f + j]) : 0.f, g, m, f + j);
+    }
+    T* o = y + m * g.F + f;
+    if (yvec) {
+      store4(o, acc[i]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (f + j < g.F) o[j] = from_f<T>(acc[i][j]);
     }
   }
 }
@@ -2640,6 +2777,35 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
     const unsigned tiles = (unsigned)((F + 4ll * fg - 1) / (4 * fg));
     return dim3((unsigned)((positions + 256 / fg - 1) / (256 / fg)), tiles < 65535u ? tiles : 65535u, (tiles + 65534u) / 65535u);
   };
+  // Patches where they and the filter tile fit 48 KB, positions fill the threads to 60 % (rows of one image only) and there are
+  // blocks enough, but not one channel at a time with a stride (bank conflicts: 16 x 112 x 112 x 3 -> 64, 7 x 7 of stride 2, 59.5 us
+  // tiled, 67.2 from patches): 8 positions per thread from two blocks per SM on, 4 from 48 blocks on (148
+  // where a sum has few terms or strides widen the patches: 1 x 224 x 224 x 3 -> 16 of stride 2 5.6 us, 7.7 from 112 patches).
+  const int fg_w = F <= 8 ? 2 : F <= 16 ? 4 : 8;
+  const long long f_tiles = (F + 4 * fg_w - 1) / (4 * fg_w);
+  int px = 0, th = 0, bands = 0;
+  for (int c = 8; c >= 4 && !px && (vec || sw == 1); c -= 4) {
+    const int mt = 128 / fg_w * c;
+    if (OW > mt) continue;
+    const int nb = (OH + mt / OW - 1) / (mt / OW), rows = (OH + nb - 1) / nb;
+    const long long smem = 4ll * R * S * C * 4 * fg_w + 4ll * (((long long)(rows - 1) * sh + R) * ((long long)(OW - 1) * sw + S) * C);
+    if (5ll * OH * OW < 3ll * nb * mt || smem > 48 * 1024 || N * (long long)nb * f_tiles < (c == 8 ? 2 * 148 : R * S * C >= 32 && sh * sw == 1 ? 48 : 148)) continue;
+    px = c; th = rows; bands = (OH + rows - 1) / rows;
+  }
+  if (px && (long long)N * bands < 0x7fffffffll && f_tiles <= 65535) {
+    const size_t smem = 4 * ((size_t)R * S * C * 4 * fg_w + (size_t)((th - 1) * sh + R) * ((OW - 1) * sw + S) * C);
+    const int low = dtype ? 7 : 15, wvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & low) == 0, yvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & low) == 0;
+    const dim3 pgrid((unsigned)(N * bands), (unsigned)f_tiles);
+#define PATCH_V(T, FG, PX, VEC) conv2d_patch_kernel<T, FG, PX, VEC><<<pgrid, 128, smem, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec)
+#define PATCH_P(T, FG, PX) do { if (vec) PATCH_V(T, FG, PX, true); else PATCH_V(T, FG, PX, false); } while (0)
+#define PATCH(T, FG) do { if (px == 8) PATCH_P(T, FG, 8); else PATCH_P(T, FG, 4); } while (0)
+    if (dtype) { if (fg_w == 2) PATCH(bf16, 2); else if (fg_w == 4) PATCH(bf16, 4); else PATCH(bf16, 8); }
+    else { if (fg_w == 2) PATCH(float, 2); else if (fg_w == 4) PATCH(float, 4); else PATCH(float, 8); }
+#undef PATCH
+#undef PATCH_P
+#undef PATCH_V
+    return CHECK_LAUNCH();
+  }
 #define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<grid(FG), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g)
 #define CONV(T, FG) do { if (vec) CONV_V(T, FG, true); else CONV_V(T, FG, false); } while (0)
   if (dtype) { if (F <= 8) CONV(bf16, 2); else if (F <= 16) CONV(bf16, 4); else CONV(bf16, 8); }

@@ -64,6 +64,43 @@ def test_direct_convolution_and_filter_gradient(dtype, N, H, W, C, F, R, S, stri
     assert _rel2(dw, torch.einsum("nhwrsc,nhwf->rscf", win, dy.double())) < STORED[dtype]
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,H,W,C,F,R,S,stride,pad", [
+    (3, 14, 14, 16, 32, 3, 3, (1, 1), (1, 1, 1, 1)), (2, 14, 14, 32, 16, 3, 3, (1, 1), (1, 1, 1, 1)), (2, 28, 28, 1, 16, 3, 3, (1, 1), (1, 1, 1, 1)),
+    (2, 15, 31, 3, 8, 3, 3, (1, 1), (1, 1, 1, 1)), (1, 32, 32, 8, 17, 3, 3, (1, 1), (2, 0, 0, 2)), (2, 29, 33, 4, 6, 3, 3, (2, 2), (1, 1, 1, 1)),
+    (5, 8, 8, 12, 33, 1, 5, (1, 1), (0, 0, 2, 2)), (2, 16, 16, 5, 64, 2, 2, (1, 1), (0, 0, 0, 0)), (300, 16, 16, 8, 16, 3, 3, (1, 1), (1, 1, 1, 1)),
+    (1, 64, 64, 4, 8, 3, 3, (1, 1), (1, 1, 1, 1)), (1, 3, 256, 4, 16, 3, 3, (1, 1), (1, 1, 1, 1)), (2, 20, 20, 36, 40, 3, 3, (1, 1), (1, 1, 1, 1))])
+def test_direct_convolution_from_patches(dtype, N, H, W, C, F, R, S, stride, pad):
+    """Bands of rows with and without a remainder, both counts of positions per thread, channels in fours and not, halos, strides,
+    channel tiles with a remainder, filters and gradients that are not finite under padding; output and filter gradient."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(0)
+    x = torch.randn(N, H, W, C, device="cuda").to(dtype)
+    w = torch.randn(R, S, C, F, device="cuda").to(dtype)
+    b = torch.randn(F, device="cuda").to(dtype)
+    ref, _, _ = _conv64(x, w, b, stride, pad)
+    y = kernels.conv2d_direct(x, w, b, stride, pad)
+    assert y.shape == ref.shape and _rel2(y, ref) < STORED[dtype]
+    ref, _, _ = _conv64(x, w, torch.zeros_like(b), stride, pad)
+    assert _rel2(kernels.conv2d_direct(x, w, None, stride, pad), ref) < STORED[dtype]
+    _, win, ok = _conv64(x, w, b, stride, pad)
+    dy = torch.randn(ref.shape, device="cuda").to(dtype)
+    dw = kernels.conv2d_wgrad_direct(x, dy, tuple(w.shape), stride, pad)
+    assert _rel2(dw, torch.einsum("nhwrsc,nhwf->rscf", win, dy.double())) < STORED[dtype]
+    if N < 10:
+        dy[0, 0, 0, F - 1], dy[N - 1, -1, -1, 0] = float("inf"), float("nan")
+        ref = torch.where(ok.unsqueeze(-1), win.unsqueeze(-1) * dy.double()[:, :, :, None, None, None], torch.zeros((), dtype=torch.float64, device="cuda")).sum((0, 1, 2))
+        dw = kernels.conv2d_wgrad_direct(x, dy, tuple(w.shape), stride, pad).double()
+        fin = torch.isfinite(ref)
+        assert torch.equal(torch.isfinite(dw), fin) and torch.equal(torch.isnan(dw), torch.isnan(ref)) and _rel2(dw[fin], ref[fin]) < STORED[dtype]
+        w[0, 0, 0, F - 1], w[R - 1, S - 1, C - 1, 0] = float("inf"), float("nan")
+        ref, _, _ = _conv64(x, w, b, stride, pad)
+        y = kernels.conv2d_direct(x, w, b, stride, pad).double()
+        ok = torch.isfinite(ref)
+        assert torch.equal(torch.isfinite(y), ok) and torch.equal(torch.isnan(y), torch.isnan(ref)) and _rel2(y[ok], ref[ok]) < STORED[dtype]
+
+
 def test_direct_convolution_skips_padding_under_infinite_operands():
     from nabla_b200.native import kernels
 
