@@ -1078,3 +1078,25 @@ def test_attention_shows_a_nan_key_in_every_split():
     k[0, 1, 2500] = float("nan")
     o, lse = attention.sdpa_fwd(q, k, v, causal=True, scale=0.09)
     assert bool(torch.isfinite(o[0, 0]).all()) and bool(torch.isnan(o[0, 1]).all()) and bool(torch.isnan(lse[0, 1]).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [1023, 4097, 8191, 8192, 8197, 9216, 10241, 16383, 16384, 16391, 18432, 20488, 32000])
+def test_log_sum_of_rows_around_three_vectors_per_thread(dtype, D):
+    """Rows below, at and above the line (8192 and 16384 elements) and multiples of three vectors of 256 threads, whole and ragged;
+    infinities of either sign, a NaN, the type's lowest value, and maxima in the first and the last vector. 4e-6: fp32 sums of D terms by 256 threads, rounded
+    logarithm and exponentials."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(D)
+    x = torch.randn(9, D, device="cuda").to(dtype)
+    x[1, 0], x[2, D - 1], x[3, D // 2] = 40.0, 40.0, -float("inf")
+    x[4, :], x[5, 1], x[6, D - 2] = torch.finfo(dtype).min, float("nan"), float("inf")
+    x[7, : D - 1] = -float("inf")
+    t = torch.randint(0, D, (9,), device="cuda")
+    lse, picked = kernels.lse_pick_fwd(x, t)
+    ref = torch.logsumexp(x.double(), 1)
+    rows = [0, 1, 2, 3, 7, 8]
+    assert ((lse.double() - ref)[rows].abs() <= 4e-6 * (1 + ref[rows].abs())).all() and torch.isnan(lse[5])
+    assert torch.equal(picked[rows], x[torch.arange(9, device="cuda"), t].float()[rows])
+    assert lse[4].item() <= torch.finfo(dtype).min / 2 and not torch.isfinite(lse[6])
