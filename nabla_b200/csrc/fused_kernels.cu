@@ -2933,7 +2933,7 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
   const int fg_w = F <= 8 ? 2 : F <= 16 ? 4 : 8;
   const long long f_tiles = (F + 4 * fg_w - 1) / (4 * fg_w);
   int px = 0, th = 0, bands = 0;
-  for (int c = 8; c >= 4 && !px && (vec || sw == 1); c -= 4) {
+  for (int c = 8; c >= 4 && !px && R * S * C > 0 && (vec || sw == 1); c -= 4) {   // (an empty sum stays tiled)
     const int mt = 128 / fg_w * c;
     if (OW > mt) continue;
     const int nb = (OH + mt / OW - 1) / (mt / OW), rows = (OH + nb - 1) / nb;
