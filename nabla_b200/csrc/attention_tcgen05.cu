@@ -882,7 +882,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* q_full = bars + 1;     // [QST] Q_i and its lse2 landed in stage i % QST
   uint64_t* q_empty = bars + 4;    // [QST]
   uint64_t* do_full = bars + 7;    // [2]  dO_i and its delta landed
-  uint64_t* do_empty = bars + 9;   // [2]
+  uint64_t* do_empty = bars + 9;   // [2]  dV has read dO_i, and all threads their deltas of it
   uint64_t* s_full = bars + 11;    //      S^T of the current tile is in TMEM
   uint64_t* dp_full = bars + 12;   //      dP^T of the current tile is in TMEM
   uint64_t* p_full = bars + 13;    //      P^T written back (256 arrivals)
@@ -1006,8 +1006,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (NREG == 2 && !mbar_wait(p_full, it & 1)) { ok = false; break; }
         tc_fence_after();
         mma_accum<HD>(t_dv, t_s(it), true, smem_u32(sDO + st * L::TILE_BYTES), it != 0);         // dV += P^T dO_i
-        umma_commit(&do_empty[st]);
         if (!mbar_wait(ds_full, it & 1)) { ok = false; break; }
+        umma_commit(&do_empty[st]);        // behind ds_full: dS^T is made with the deltas that the next load into this stage replaces
         tc_fence_after();
         mma_accum<HD>(t_dk, t_s(it) + 32, true, smem_u32(sQ + qs * L::TILE_BYTES), it != 0);     // dK += dS^T Q_i
         umma_commit(&q_empty[qs]);
