@@ -993,17 +993,16 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int it = 0; it < n_it && ok; ++it) {
         const int st = it & 1, qs = it % QST, qn = (it + 1) % QST;
         const bool more = it + 1 < n_it;
-        // Scores of the next tile: their region held dP^T of this tile (two regions: once all threads have read it) or of
-        // the one before (three: once all have written P^T, so that none can arrive a second time on a barrier where
-        // another has yet to arrive)
-        if (NREG == 3 && !mbar_wait(p_full, it & 1)) { ok = false; break; }
+        // Scores of the next tile: their region held dP^T of this tile (two regions: free once all threads have read it) or
+        // of the one before (three). Never before all have written P^T of this tile, so that none can arrive a second time
+        // on a barrier where another has yet to arrive, or where this thread has yet to look.
+        if (!mbar_wait(p_full, it & 1)) { ok = false; break; }
         if (more) {
           if (!(mbar_wait(&q_full[qn], ((it + 1) / QST) & 1) && (NREG == 3 || mbar_wait(dp_read, it & 1)))) { ok = false; break; }
           tc_fence_after();
           mma_scores<HD>(t_s(it + 1), smem_u32(sK), smem_u32(sQ + qn * L::TILE_BYTES));
           umma_commit(s_full);
         }
-        if (NREG == 2 && !mbar_wait(p_full, it & 1)) { ok = false; break; }
         tc_fence_after();
         mma_accum<HD>(t_dv, t_s(it), true, smem_u32(sDO + st * L::TILE_BYTES), it != 0);         // dV += P^T dO_i
         if (!mbar_wait(ds_full, it & 1)) { ok = false; break; }

@@ -36,3 +36,16 @@ def test_statistics_of_a_stage_are_read_before_it_is_loaded_again(regions, relea
     order, threads = _issuer_order(regions), _kernel()[1]
     later = [b for b in ("p_full", "ds_full") if threads.index(f"mbar_arrive({b})") > threads.rindex(read)]
     assert later and any(order[f"wait {b}"] < order[f"commit {release}"] for b in later)
+
+
+@pytest.mark.parametrize("regions", [2, 3])
+@pytest.mark.parametrize("barrier,published", [("p_full", "s_full"), ("ds_full", "dp_full"), ("dp_read", "dp_full")])
+def test_issuer_looks_at_a_barrier_before_the_threads_can_arrive_for_the_next_tile(regions, barrier, published):
+    """Threads arrive for the next tile once ``published`` of it is there; a second arrival of all flips the parity that the
+    issuer's wait for this tile looks for."""
+    order, threads = _issuer_order(regions), _kernel()[1]
+    assert threads.index(f"mbar_wait({published}") < threads.index(f"mbar_arrive({barrier})")
+    if barrier == "dp_read" and regions == 3:
+        assert "wait dp_read" not in order
+    else:
+        assert order[f"wait {barrier}"] < order[f"commit {published}"]
