@@ -411,7 +411,8 @@ def _same_layout_addend(add: OpNode, x: TensorImpl) -> bool:
     if len(ins) != 2:
         return False
     other = ins[1] if ins[0] is x else ins[0] if ins[1] is x else None
-    if other is None or other is x or other.batch_dims or other.dtype is not x.dtype or tuple(other._shape) != tuple(x._shape):
+    if other is None or other is x or other.batch_dims or other.dtype is not x.dtype or other.device != x.device \
+            or tuple(other._shape) != tuple(x._shape):
         return False
     sa = [tuple(d.axes) for d in other.sharding.dim_specs] if other.sharding is not None else None
     sb = [tuple(d.axes) for d in x.sharding.dim_specs] if x.sharding is not None else None

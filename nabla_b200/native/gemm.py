@@ -198,6 +198,9 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
     from . import ptr, status_word, stream_ptr
 
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "gemm_bf16 needs bf16 operands"
+    dev = a.get_device()                                    # the kernel takes plain pointers
+    if dev < 0 or b.get_device() != dev or any(isinstance(t, torch.Tensor) and t.get_device() != dev for t in (bias, aux_in, out, alpha)):
+        raise RuntimeError("gemm_bf16: expected all tensors to be on the same GPU")
     squeeze = a.dim() == 2 and b.dim() == 2
     a3 = a if a.dim() == 3 else a.unsqueeze(0)
     b3 = b if b.dim() == 3 else b.unsqueeze(0)

@@ -124,6 +124,8 @@ def layernorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma, mean: torch.Tensor, 
     """(dx, dgamma, dbeta); ``add`` (x's shape and dtype) is added to dx in the same pass."""
     global launch_count
     if add is not None:
+        if add.device != x.device:
+            raise RuntimeError("layernorm_bwd: expected all tensors to be on the same GPU")
         add = add.contiguous()
         if add.data_ptr() & 15 or os.environ.get("NABLA_B200_LN_BWD") == "two_kernels":
             dx, dgamma, dbeta = layernorm_bwd(dy, x, gamma, mean, rstd)
@@ -574,7 +576,8 @@ def sgemm(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) ->
             and elementwise_enabled()):
         return None
     M, K, N = a.shape[0], a.shape[1], b.shape[1]
-    if b.shape[0] != K or not 0 < M * N * K < 1 << 31 or M > 1 << 20 or (bias is not None and (bias.numel() != N or bias.dtype != torch.float32)):
+    if b.shape[0] != K or not 0 < M * N * K < 1 << 31 or M > 1 << 20 \
+            or (bias is not None and (bias.numel() != N or bias.dtype != torch.float32 or bias.device != a.device)):
         return None
     z = _L().nb_sgemm_slices(M, N, K)
     out = torch.empty((M, N), dtype=torch.float32, device=a.device)

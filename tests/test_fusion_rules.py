@@ -1,0 +1,83 @@
+"""Rules of the fused schedules of compiled recordings, asked on the CPU: a plan looks at shapes, types and devices alone."""
+import weakref
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from nabla_b200.core.graph import fusion
+from nabla_b200.core.graph.tracing import OpNode
+from nabla_b200.core.tensor.impl import TensorImpl
+from nabla_b200.types import Device, DType
+
+GPU, GPU1, HOST = Device("gpu", 0), Device("gpu", 1), Device("cpu", 0)
+
+
+class _Graph:
+    """Recorded nodes whose tensors have no values."""
+
+    def __init__(self):
+        self.nodes, self.keep = [], []
+
+    def tensor(self, *shape, device=GPU, dtype=DType.bfloat16):
+        t = TensorImpl(None, shape=shape, dtype=dtype, device=device)
+        self.keep.append(t)
+        return t
+
+    def op(self, name, args, *shapes, dtype=DType.bfloat16, **kwargs):
+        n = OpNode(SimpleNamespace(name=name), list(args), None, kwargs, kwargs)
+        outs = [self.tensor(*s, dtype=dtype) for s in shapes]
+        for o in outs:
+            o.output_refs = n
+        n.out_refs = [weakref.ref(o) for o in outs]
+        self.nodes.append(n)
+        return outs[0] if len(outs) == 1 else outs
+
+    def plan(self, *targets):
+        return [(kind, tuple(self.nodes[i].op.name for i in idxs))
+                for kind, idxs in fusion.build_plan(self.nodes, list(targets), private=True).steps]
+
+
+@pytest.mark.parametrize("device,fused", [(GPU, True), (GPU1, False), (HOST, False)])
+@pytest.mark.parametrize("name", ["matmul", "linear"])
+def test_residual_on_another_device_stays_an_add(name, device, fused):
+    g = _Graph()
+    y = g.op(name, [g.tensor(64, 32), g.tensor(32, 64)], (64, 64))
+    z = g.op("add", [y, g.tensor(64, 64, device=device)], (64, 64))
+    assert g.plan(z) == ([("gemm_residual", (name, "add"))] if fused else [("op", (name,)), ("op", ("add",))])
+
+
+@pytest.mark.parametrize("device,fused", [(GPU, True), (GPU1, False), (HOST, False)])
+def test_gradient_on_another_device_does_not_join_the_layer_norm(device, fused):
+    g = _Graph()
+    stat = lambda: g.tensor(64, dtype=DType.float32)  # noqa: E731
+    dx, dg, db = g.op("layer_norm_bwd", [g.tensor(64, 32), g.tensor(64, 32), stat(), stat(), g.tensor(32)], (64, 32), (32,), (32,))
+    z = g.op("add", [g.tensor(64, 32, device=device), dx], (64, 32))
+    assert (g.plan(z, dg, db)[0][0] == "ln_bwd_add") == fused
+
+
+class _Fake:
+    """A tensor of the GPU as far as a wrapper looks before it launches."""
+
+    def __init__(self, *shape, dtype):
+        self.shape, self.dtype, self.is_cuda, self.device = shape, dtype, True, torch.device("cuda", 0)
+
+    def dim(self):
+        return len(self.shape)
+
+    def get_device(self):
+        return 0
+
+
+def test_wrappers_refuse_operands_on_the_host():
+    from nabla_b200.native import gemm, kernels
+
+    a, b = _Fake(64, 512, dtype=torch.float32), _Fake(512, 64, dtype=torch.float32)
+    assert kernels.sgemm(a, b, torch.zeros(64)) is None                # the caller's torch call then raises
+    x, w, host = _Fake(64, 32, dtype=torch.bfloat16), _Fake(32, 64, dtype=torch.bfloat16), torch.zeros(32, 64, dtype=torch.bfloat16)
+    for args, kw in (((x, host), {}), ((x, w), {"bias": host[0]}), ((x, w), {"aux": "add", "aux_in": torch.zeros(64, 64, dtype=torch.bfloat16)}),
+                     ((x, w), {"alpha": torch.ones(1)}), ((host.t(), host), {})):
+        with pytest.raises(RuntimeError, match="same GPU"):
+            gemm.gemm_bf16(*args, **kw)
+    with pytest.raises(RuntimeError, match="same GPU"):
+        kernels.layernorm_bwd(x, x, None, None, None, add=host)

@@ -239,6 +239,21 @@ def test_compiled_products_take_their_adds_and_factors(tokens, dim, out, rank):
     assert "gemm_residual" not in str(h.dump_plan()) and _rel2(p.to_torch(), x.double() @ w.double()) < STORED[torch.bfloat16]
 
 
+def test_operands_on_the_host_are_refused():
+    """A residual of a compiled product and a bias that live on the host, where the fused kernels would take them."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    t = lambda *s, d="cuda", ty=torch.bfloat16: nb.Tensor.from_torch(torch.ones(*s, device=d, dtype=ty))  # noqa: E731
+    f32 = torch.float32
+    for call, args in ((lambda x, w, r: x @ w + r, (t(64, 32), t(32, 64), t(64, 64, d="cpu"))),
+                       (lambda x, w, b: F.linear(x, w, b), (t(64, 32), t(32, 64), t(64, d="cpu"))),
+                       (lambda x, w, b: F.linear(x, w, b), (t(64, 512, ty=f32), t(512, 64, ty=f32), t(64, d="cpu", ty=f32)))):
+        for fn in (call, nb.compile(call)):
+            with pytest.raises(RuntimeError):
+                fn(*args).to_torch()
+
+
 @pytest.mark.parametrize("M,N,K,sliced", [(2048, 16, 2048, True), (1, 512, 2048, True), (130, 77, 1800, True), (2002, 512, 2048, True), (512, 512, 2002, True),
                                           (100, 1000, 8192, True), (257, 130, 4100, True), (16, 6144, 2048, True), (64, 64, 8193, False), (512, 512, 256, False), (64, 256, 512, True),
                                           (70, 100, 449, True), (512, 512, 8192, True), (4096, 4096, 2048, False)])
