@@ -557,11 +557,16 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
     from .engine import store_outputs
 
     if kind == "linear_epilogue":
+        from ... import native
         from ...native.gemm import gemm_bf16
 
         mm, add = group[0], group[1]
         act = group[2] if len(group) > 2 else None
         a, b = [x._buffers[0] for x in mm.input_impls()]
+        if not native.use_native(a):
+            for n_ in group:
+                _plain(n_, keep_graph)
+            return
         mm_out = mm.outputs()[0]
         bias_impl = [x for x in add.input_impls() if x is not mm_out][0]
         bias = bias_impl._buffers[0]
@@ -689,6 +694,7 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
             _plain(add, keep_graph)
         return
     if kind == "gemm_residual":
+        from ... import native
         from ...native.gemm import gemm_bf16, split_k_factor
 
         lin, add = group
@@ -698,7 +704,7 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         lin_out = lin.outputs()[0]
         res = [x for x in add.input_impls() if x is not lin_out][0]._buffers[0]
         # (a product that is worth cutting into K slices keeps its own launch: the slices are summed by another)
-        if a.is_cuda and a.numel() and b.numel() and not (bias is None and split_k_factor(a.numel() // a.shape[-1], b.shape[-1], a.shape[-1]) > 1):
+        if native.use_native(a) and a.numel() and b.numel() and not (bias is None and split_k_factor(a.numel() // a.shape[-1], b.shape[-1], a.shape[-1]) > 1):
             n_out = b.shape[-1]
             out = gemm_bf16(a.reshape(-1, a.shape[-1]), b, bias=bias, aux="add",
                             aux_in=res.reshape(-1, n_out)).reshape(*a.shape[:-1], n_out)
@@ -708,13 +714,14 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
             _plain(add, keep_graph)
         return
     if kind == "gemm_dact":
+        from ... import native
         from ...native.gemm import gemm_bf16
 
         mm, da = group
         a, b = [x._buffers[0] for x in mm.input_impls()]
         z = da.input_impls()[1]._buffers[0]
         act = da.kwargs["activation"]
-        if a.is_cuda and a.numel() and b.numel():
+        if native.use_native(a) and a.numel() and b.numel():
             n_out = b.shape[-1]
             out = gemm_bf16(a.reshape(-1, a.shape[-1]), b, aux="drelu" if act == "relu" else "dgelu",
                             aux_in=z.reshape(-1, n_out), gelu_tanh=act == "gelu_tanh").reshape(*a.shape[:-1], n_out)

@@ -239,6 +239,33 @@ def test_compiled_products_take_their_adds_and_factors(tokens, dim, out, rank):
     assert "gemm_residual" not in str(h.dump_plan()) and _rel2(p.to_torch(), x.double() @ w.double()) < STORED[torch.bfloat16]
 
 
+@pytest.mark.parametrize("kind", ["gemm_residual", "linear_epilogue", "gemm_dact"])
+def test_compiled_products_without_native_kernels(kind, monkeypatch):
+    """The switch that turns the native kernels off holds for the steps that fuse a product with what follows it."""
+    import nabla_b200 as nb
+    from nabla_b200.native import gemm
+    from nabla_b200.nn import functional as F
+
+    monkeypatch.setenv("NABLA_B200_DISABLE_NATIVE", "1")
+    torch.manual_seed(0)
+    x, w, w2, r, b = (torch.randn(*s, device="cuda").bfloat16() for s in ((48, 32), (32, 64), (64, 64), (48, 64), (1, 64)))
+
+    def mlp(x, w, w2, r, b):
+        return nb.vjp(lambda t: F.linear(F.linear(t, w, b, activation="gelu"), w2), x, create_graph=False)[1](r)[0]
+
+    call, ref = {"gemm_residual": (lambda x, w, w2, r, b: x @ w + r, x.double() @ w.double() + r.double()),
+                 "linear_epilogue": (lambda x, w, w2, r, b: nb.relu(x @ w + b), torch.relu(x.double() @ w.double() + b.double())),
+                 "gemm_dact": (mlp, None)}[kind]
+    if ref is None:
+        x64 = x.double().requires_grad_(True)
+        ref = torch.autograd.grad(TF.gelu(x64 @ w.double() + b.double()) @ w2.double(), x64, r.double())[0]
+    f, n = nb.compile(call), gemm.launch_count
+    args = [nb.Tensor.from_torch(t) for t in (x, w, w2, r, b)]
+    for _ in range(2):
+        assert _rel2(f(*args).to_torch(), ref) < 4 * STORED[torch.bfloat16]      # up to three roundings of a value and a product's
+    assert kind in str(f.dump_plan()) and gemm.launch_count == n
+
+
 def test_operands_on_the_host_are_refused():
     """A residual of a compiled product and a bias that live on the host, where the fused kernels would take them."""
     import nabla_b200 as nb
