@@ -21,6 +21,7 @@
 // matmul + add + relu/gelu composition of nabla/nn/functional/layers.py:30-35.
 #include "sm100_ptx.cuh"
 #include "nb_debug.cuh"
+#include <atomic>
 #include <stdio.h>
 
 namespace nb {
@@ -1464,32 +1465,36 @@ static int tile_width(int M, int N, int batch) {
 // Slices of K that a product is given to clusters for (1: none), and their tile width. In clocks: a CTA loads a k-block in
 // 2 (128 + bn) and stores a tile in 16 bn; the exchange of the slices and its two barriers take some 1400. Only where all
 // slices run at once and a tenth and 600 clocks are saved (us, whole and sliced: 1 x 512 x 512 5.2, 4.1; 100 x 768 x 768 6.2,
-// 5.6; outside the line 100 x 2048 x 512 5.5, 5.3; 1332 x 512 x 512 5.7, 6.6; slices that do not run at once 5.9, 10.1). The clusters that fit are asked for once (-1: not yet).
-struct SlicePlan { int bn, slices; };
-static int g_slice_clusters[2][4] = {{-1, -1, -1, -1}, {-1, -1, -1, -1}};   // [bn 64, 128][log2 slices]
+// 5.6; outside the line 100 x 2048 x 512 5.5, 5.3; 1332 x 512 x 512 5.7, 6.6; slices that do not run at once 5.9, 10.1).
+struct SlicePlan { int bn, slices; bool sure; };       // sure: no device query failed on the way
+// Clusters that run at once on the current device, or -1 where it cannot be asked now (an answer is kept, a failure is not).
+// Threads that ask at the same time all ask; none sees another's half-made answer.
 template <int BN, int SLICES>
 static int slice_clusters() {
-  int& n = g_slice_clusters[BN == 128][SLICES == 2 ? 1 : SLICES == 4 ? 2 : 3];
-  if (n < 0) {
-    n = 0;
-    const auto kernel = gemm_bf16_slices_kernel<BN, SLICES>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemLayout<BN>::TOTAL) == cudaSuccess) {
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = SLICES;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3(SLICES);
-      cfg.blockDim = dim3(NUM_THREADS);
-      cfg.dynamicSmemBytes = SmemLayout<BN>::TOTAL;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int k = 0;
-      if (cudaOccupancyMaxActiveClusters(&k, kernel, &cfg) == cudaSuccess) n = k;
-    }
-    if (n == 0) cudaGetLastError();      // the query's own error: the other kernels serve
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES];              // answer + 1; 0: not yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= DEVICES) return -1;
+  if (const int k = known[dev].load(std::memory_order_acquire)) return k - 1;
+  const auto kernel = gemm_bf16_slices_kernel<BN, SLICES>;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SLICES;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(SLICES);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SmemLayout<BN>::TOTAL;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemLayout<BN>::TOTAL) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();                                // the query's own error: the other kernels serve
+    return -1;
   }
+  known[dev].store(n + 1, std::memory_order_release);
   return n;
 }
 template <int BN>
@@ -1497,7 +1502,7 @@ static int slice_clusters(int slices) {
   return slices == 2 ? slice_clusters<BN, 2>() : slices == 4 ? slice_clusters<BN, 4>() : slice_clusters<BN, 8>();
 }
 static SlicePlan slice_plan(int M, int N, int K, int bn) {
-  SlicePlan best{bn, 1};
+  SlicePlan best{bn, 1, true};
   if (bn == 256 || K > 8192) return best;              // (wide tiles: enough of them for the chip)
   const long long kb = (K + BLOCK_K - 1) / BLOCK_K, m_t = (M + BLOCK_M - 1) / BLOCK_M;
   const long long tiles0 = m_t * ((N + bn - 1) / bn);
@@ -1508,10 +1513,12 @@ static SlicePlan slice_plan(int M, int N, int K, int bn) {
       const long long tiles = m_t * ((N + w - 1) / w), per = (kb + z - 1) / z;
       if ((z - 1) * per >= kb || tiles * z > g_num_sms) continue;
       const double t = (double)per * 2 * (BLOCK_M + w) + 16 * w + 1400;
-      if (t < t_best && tiles <= (w == 64 ? slice_clusters<64>(z) : slice_clusters<128>(z))) {
-        t_best = t;
-        best = SlicePlan{w, z};
-      }
+      if (t >= t_best) continue;
+      const int clusters = w == 64 ? slice_clusters<64>(z) : slice_clusters<128>(z);
+      if (clusters < 0) best.sure = false;
+      if (tiles > clusters) continue;
+      t_best = t;
+      best = SlicePlan{w, z, best.sure};
     }
   return best;
 }
@@ -1601,7 +1608,7 @@ extern "C" int nb_gemm_pair_alloc_probe(unsigned* out2, void* stream) {
   return cudaLaunchKernelEx(&cfg, nb::pair_alloc_probe_kernel, out2) == cudaSuccess ? 0 : -3;
 }
 
-// Slices of K that nb_gemm_bf16 cuts a plain product of one batch into by itself (1: none).
+// Slices of K that nb_gemm_bf16 cuts a plain product of one batch into by itself (1: none; 0: the device cannot be asked now).
 extern "C" int nb_gemm_slices(int M, int N, int K) {
   using namespace nb;
   if (M <= 0 || N <= 0 || K <= 0) return 1;
@@ -1609,8 +1616,10 @@ extern "C" int nb_gemm_slices(int M, int N, int K) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (g_num_sms <= 0) return 0;
   }
-  return slice_plan(M, N, K, tile_width(M, N, 1)).slices;
+  const SlicePlan plan = slice_plan(M, N, K, tile_width(M, N, 1));
+  return plan.sure ? plan.slices : 0;
 }
 
 // C entry point. All leading dimensions / strides are in elements.
@@ -1639,7 +1648,7 @@ extern "C" int nb_gemm_bf16(const void* A, const void* B, void* C, const void* b
   if (bn != 256 && bn != 128 && bn != 64) bn = tile_width(M, N, batch);
   const bool sliceable = batch == 1 && !accumulate && (epi == EPI_NONE || epi == EPI_BIAS) && (aux == AUX_NONE || aux == AUX_ADD) &&
                          block_n == 0 && max_ctas == g_num_sms;
-  const SlicePlan plan = sliceable ? slice_plan(M, N, K, bn) : SlicePlan{bn, 1};
+  const SlicePlan plan = sliceable ? slice_plan(M, N, K, bn) : SlicePlan{bn, 1, true};
   bn = plan.bn;
   CUtensorMap ta, tb;
   int r;

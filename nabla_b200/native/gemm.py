@@ -119,13 +119,27 @@ def gemm_supported(a: torch.Tensor, b: torch.Tensor) -> bool:
 _SMS = 0
 
 
+class _NoAnswer(Exception):
+    pass
+
+
 @functools.lru_cache(1024)
-def cluster_slices(M: int, N: int, K: int) -> int:
-    """Slices of K that the kernel itself cuts this product into, on a cluster of CTAs each (1: none)."""
+def _known_slices(M: int, N: int, K: int) -> int:
     from . import load
 
     _get()
-    return load("libnb_gemm.so").nb_gemm_slices(M, N, K)
+    n = load("libnb_gemm.so").nb_gemm_slices(M, N, K)
+    if n <= 0:
+        raise _NoAnswer                     # the device could not be asked: not to be kept
+    return n
+
+
+def cluster_slices(M: int, N: int, K: int) -> int:
+    """Slices of K that the kernel itself cuts this product into, on a cluster of CTAs each (1: none)."""
+    try:
+        return _known_slices(M, N, K)
+    except _NoAnswer:
+        return 1
 
 
 def split_k_factor(M: int, N: int, K: int) -> int:

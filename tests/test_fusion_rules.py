@@ -1,4 +1,5 @@
-"""Rules of the fused schedules of compiled recordings, asked on the CPU: a plan looks at shapes, types and devices alone."""
+"""Rules of the fused schedules of compiled recordings and of the wrappers around kernels, asked on the CPU: they look at
+shapes, types and devices alone."""
 import weakref
 from types import SimpleNamespace
 
@@ -81,3 +82,14 @@ def test_wrappers_refuse_operands_on_the_host():
             gemm.gemm_bf16(*args, **kw)
     with pytest.raises(RuntimeError, match="same GPU"):
         kernels.layernorm_bwd(x, x, None, None, None, add=host)
+
+
+def test_a_slice_count_that_could_not_be_asked_for_is_not_kept(monkeypatch):
+    from nabla_b200 import native
+    from nabla_b200.native import gemm
+
+    answers = [0, 4, 1]
+    monkeypatch.setattr(gemm, "_get", lambda: None)
+    monkeypatch.setattr(native, "load", lambda name: SimpleNamespace(nb_gemm_slices=lambda *a: answers.pop(0)))
+    sizes = (123457, 11, 13)                       # nobody else's
+    assert [gemm.cluster_slices(*sizes) for _ in range(3)] == [1, 4, 4]

@@ -1,5 +1,9 @@
 """Kernels and dispatch rules at the sizes where they can go wrong (tile edges, remainders, the smallest and
 largest of a rule's range) against 64-bit torch results. Needs a B200 (sm_100a)."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 import torch.nn.functional as TF
@@ -264,6 +268,28 @@ def test_compiled_products_without_native_kernels(kind, monkeypatch):
     for _ in range(2):
         assert _rel2(f(*args).to_torch(), ref) < 4 * STORED[torch.bfloat16]      # up to three roundings of a value and a product's
     assert kind in str(f.dump_plan()) and gemm.launch_count == n
+
+
+def test_threads_that_ask_first_agree_on_the_slices():
+    """Eight threads of a new process plan their first product at the same time; each has to get what a later call gets."""
+    code = """
+import threading, torch
+torch.zeros(1, device="cuda")
+from nabla_b200.native import gemm, load
+gemm._get()
+ask = load("libnb_gemm.so").nb_gemm_slices
+start, got = threading.Barrier(8), [None] * 8
+def one(i):
+    start.wait()
+    got[i] = ask(64, 256, 8192)
+threads = [threading.Thread(target=one, args=(i,)) for i in range(8)]
+for t in threads: t.start()
+for t in threads: t.join()
+assert got == [ask(64, 256, 8192)] * 8 and got[0] > 1, got
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 def test_operands_on_the_host_are_refused():
