@@ -929,7 +929,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const TP* __restrict__ p, co
 }
 // The same update of many small tensors in one launch, 2048 elements per block. A launch of one of them is 2.5 to 4 us
 // whatever its size: the eight of a 64-256-256-256-1 MLP took 24 us of a 165 us step, 4.2 together.
-constexpr int ADAM_GROUP = 48;
+constexpr int ADAM_GROUP = 48, ADAM_GROUP_MAX = 1 << 20;     // tensors of a launch, elements of one
 struct AdamGroup {
   struct Leaf {
     const void *p, *g;
@@ -2617,21 +2617,23 @@ int nb_adamw(const void* p, const void* g, const float* m, const float* v, void*
 #undef ADAMW
   return CHECK_LAUNCH();
 }
-// The updates of `count` tensors (host arrays of device pointers and element counts) with one set of hyperparameters.
+// The updates of `count` tensors (host arrays of device pointers and element counts) with one set of hyperparameters. -2, and
+// nothing updated, where one is not 16-byte aligned or has more than ADAM_GROUP_MAX elements.
 int nb_adamw_group(const void* const* p, const void* const* g, const float* const* m, const float* const* v, void* const* p_out,
                    float* const* m_out, float* const* v_out, const int* n, int count, float lr, float b1, float b2, float eps,
                    float wd, float bc1, float bc2, float grad_scale, const float* hyper, int p_dtype, int g_dtype, void* stream) {
   const AdamHyper h{lr, b1, b2, eps, wd, bc1, bc2, grad_scale};
+  for (int k = 0; k < count; ++k)                      // all of them, before the first launch updates any
+    if (n[k] > 0 && (((reinterpret_cast<uintptr_t>(p[k]) | reinterpret_cast<uintptr_t>(g[k]) | reinterpret_cast<uintptr_t>(m[k]) |
+                       reinterpret_cast<uintptr_t>(v[k]) | reinterpret_cast<uintptr_t>(p_out[k]) | reinterpret_cast<uintptr_t>(m_out[k]) |
+                       reinterpret_cast<uintptr_t>(v_out[k])) & 15) || n[k] > ADAM_GROUP_MAX))
+      return -2;
   for (int k = 0; k < count;) {
     AdamGroup c;
     unsigned blocks = 0;
     c.count = 0;
     for (; k < count && c.count < ADAM_GROUP; ++k) {
       if (n[k] <= 0) continue;
-      if (((reinterpret_cast<uintptr_t>(p[k]) | reinterpret_cast<uintptr_t>(g[k]) | reinterpret_cast<uintptr_t>(m[k]) |
-            reinterpret_cast<uintptr_t>(v[k]) | reinterpret_cast<uintptr_t>(p_out[k]) | reinterpret_cast<uintptr_t>(m_out[k]) |
-            reinterpret_cast<uintptr_t>(v_out[k])) & 15) || n[k] > (1 << 20))
-        return -2;
       c.leaf[c.count++] = AdamGroup::Leaf{p[k], g[k], m[k], v[k], p_out[k], m_out[k], v_out[k], (unsigned)n[k], blocks};
       blocks += ((unsigned)n[k] + 2047) / 2048;
     }

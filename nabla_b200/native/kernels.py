@@ -213,8 +213,11 @@ def adamw(p, g, m, v, *, lr, b1, b2, eps, wd, step: int | None = None, hyper: to
 
 def adamw_group(leaves: list, *, lr, b1, b2, eps, wd, step: int | None = None, hyper: torch.Tensor | None = None):
     """``adamw`` of several small tensors that share their hyperparameters and types, in one launch per 48: ``leaves``
-    holds (p, g, m, v, inplace); returns [(p', m', v')], or None where a tensor is not 16-byte aligned."""
+    holds (p, g, m, v, inplace); returns [(p', m', v')], or None (nothing updated) where a tensor is not 16-byte aligned
+    or has more than 2^20 elements, which the kernel is not made for."""
     n = len(leaves)
+    if any(leaf[0].numel() > 1 << 20 for leaf in leaves):
+        return None
     ins, outs = [], []
     for p, g, m, v, inplace in leaves:
         p, g, m, v = p.contiguous(), g.contiguous(), m.contiguous(), v.contiguous()

@@ -93,3 +93,10 @@ def test_a_slice_count_that_could_not_be_asked_for_is_not_kept(monkeypatch):
     monkeypatch.setattr(native, "load", lambda name: SimpleNamespace(nb_gemm_slices=lambda *a: answers.pop(0)))
     sizes = (123457, 11, 13)                       # nobody else's
     assert [gemm.cluster_slices(*sizes) for _ in range(3)] == [1, 4, 4]
+
+
+def test_a_group_with_a_large_tensor_is_left_to_single_updates():
+    from nabla_b200.native import kernels
+
+    leaves = [tuple(torch.zeros(n) for _ in range(4)) + (True,) for n in (8, (1 << 20) + 8)]
+    assert kernels.adamw_group(leaves, lr=1e-3, b1=0.9, b2=0.99, eps=1e-8, wd=0.0, step=1) is None

@@ -900,6 +900,25 @@ def test_small_adamw_updates_in_one_launch(p_dtype, g_dtype):
     assert kernels.adamw_group([(mk(16, p_dtype), mk(16, g_dtype), odd, odd.clone(), False)], **kw) is None
 
 
+@pytest.mark.parametrize("fault", ["alignment", "size"])
+def test_a_group_that_is_refused_updates_nothing(fault):
+    """The last of 49 tensors, which a second launch would take, is one that the entry point refuses."""
+    import ctypes
+
+    from nabla_b200.native import kernels, ptr, stream_ptr
+
+    n = 49
+    leaves = [[torch.full((16,), 0.5, device="cuda") for _ in range(4)] for _ in range(n)]
+    sizes = [8] * (n - 1) + [(1 << 20) + 1 if fault == "size" else 8]
+    cols = [[t[i].data_ptr() for t in leaves] for i in range(4)]
+    if fault == "alignment":
+        cols[1][-1] += 4
+    arr = [(ctypes.c_void_p * n)(*c) for c in cols + [cols[0], cols[2], cols[3]]]
+    rc = kernels._L().nb_adamw_group(*arr, (ctypes.c_int * n)(*sizes), n, 0.1, 0.9, 0.99, 1e-8, 0.0, 0.1, 0.01, 1.0, ptr(None), 0, 0, stream_ptr())
+    torch.cuda.synchronize()
+    assert rc == -2 and all(bool((t == 0.5).all()) for leaf in leaves for t in leaf)
+
+
 @pytest.mark.parametrize("donate", [False, True])
 def test_compiled_step_groups_its_small_updates(donate):
     import nabla_b200 as nb
