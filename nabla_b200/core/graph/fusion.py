@@ -87,6 +87,16 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
         return (impl is not None and id(impl) not in target_ids and len(cons.get(id(impl), [])) == 1
                 and impl.sharding is None and impl.batch_dims == 0)
 
+    def heads_epilogue(j: int) -> bool:
+        """Is product ``j`` to be fused with the activation gradient or the bias behind it?"""
+        o = sole_output(nodes[j])
+        if _is_local_gemm(nodes[j]) and _dact_consumer(nodes[j], nodes, cons, target_ids, used) is not None:
+            return True
+        if not fusable_intermediate(o):
+            return False
+        k = cons[id(o)][0]
+        return not used[k] and nodes[k].op.name == "add" and _is_bias_add(nodes[k], o)
+
     for i, n in enumerate(nodes):
         if used[i]:
             continue
@@ -167,12 +177,12 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
                     chain = [i, j]
                     kind = "gemm_scale"
         if chain is None and private and n.op.name == "mul":
-            # x * s with one element s, read by nothing but GEMMs
+            # x * s with one element s, read by nothing but GEMMs, none of which takes more than this pass into its own epilogue
             o = sole_output(n)
             readers = cons.get(id(o), []) if o is not None else []
             if readers and id(o) not in target_ids and o.sharding is None and not o.batch_dims and len(set(readers)) == len(readers) \
                     and any(_scalar_factor(n, x) is not None for x in n.input_impls()) \
-                    and all(not used[j] and nodes[j].op.name == "matmul" and _is_cuda_bf16_2d(nodes[j]) for j in readers):
+                    and all(not used[j] and nodes[j].op.name == "matmul" and _is_cuda_bf16_2d(nodes[j]) and not heads_epilogue(j) for j in readers):
                 used[i] = True
                 for j in readers:
                     used[j] = True

@@ -57,6 +57,31 @@ def test_gradient_on_another_device_does_not_join_the_layer_norm(device, fused):
     assert (g.plan(z, dg, db)[0][0] == "ln_bwd_add") == fused
 
 
+@pytest.mark.parametrize("shape", [(1,), ()])
+def test_a_factor_leaves_products_their_own_epilogues(shape):
+    """Backward of gelu(x w1) w2 * s: the scaled gradient is read by two products, one of which ends in the gelu's gradient. That
+    pass is over tokens x hidden, the factor's over tokens x dim."""
+    g = _Graph()
+    dy = g.op("mul", [g.tensor(64, 32), g.tensor(*shape)], (64, 32))
+    dw = g.op("matmul", [g.tensor(128, 64), dy], (128, 32))
+    dz = g.op("dact_mul", [g.op("matmul", [dy, g.tensor(32, 128)], (64, 128)), g.tensor(64, 128)], (64, 128), activation="gelu")
+    assert g.plan(dw, dz) == [("op", ("mul",)), ("op", ("matmul",)), ("gemm_dact", ("matmul", "dact_mul"))]
+
+
+def test_a_factor_leaves_products_their_bias_and_activation():
+    g = _Graph()
+    x = g.op("mul", [g.tensor(64, 32), g.tensor(1)], (64, 32))
+    y = g.op("relu", [g.op("add", [g.op("matmul", [x, g.tensor(32, 128)], (64, 128)), g.tensor(1, 128)], (64, 128))], (64, 128))
+    assert g.plan(y) == [("op", ("mul",)), ("linear_epilogue", ("matmul", "add", "relu"))]
+
+
+def test_a_factor_of_plain_products_goes_into_their_epilogues():
+    g = _Graph()
+    x = g.op("mul", [g.tensor(1), g.tensor(64, 32)], (64, 32))
+    y, z = g.op("matmul", [x, g.tensor(32, 128)], (64, 128)), g.op("matmul", [g.tensor(16, 64), x], (16, 32))
+    assert g.plan(y, z) == [("scale_gemm", ("mul", "matmul"))] * 2
+
+
 class _Fake:
     """A tensor of the GPU as far as a wrapper looks before it launches."""
 
