@@ -705,7 +705,7 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         return
     if kind == "gemm_residual":
         from ... import native
-        from ...native.gemm import gemm_bf16, split_k_factor
+        from ...native.gemm import gemm_bf16, residual_in_epilogue, split_k_factor
 
         lin, add = group
         ins = lin.input_impls()
@@ -713,11 +713,14 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         bias = ins[2]._buffers[0] if len(ins) > 2 else None
         lin_out = lin.outputs()[0]
         res = [x for x in add.input_impls() if x is not lin_out][0]._buffers[0]
-        # (a product that is worth cutting into K slices keeps its own launch: the slices are summed by another)
-        if native.use_native(a) and a.numel() and b.numel() and not (bias is None and split_k_factor(a.numel() // a.shape[-1], b.shape[-1], a.shape[-1]) > 1):
-            n_out = b.shape[-1]
-            out = gemm_bf16(a.reshape(-1, a.shape[-1]), b, bias=bias, aux="add",
-                            aux_in=res.reshape(-1, n_out)).reshape(*a.shape[:-1], n_out)
+        fits = native.use_native(a) and a.numel() > 0 and b.numel() > 0
+        if fits:
+            m, k, n_out = a.numel() // a.shape[-1], a.shape[-1], b.shape[-1]
+            res = res.reshape(-1, n_out)
+            # (a product that is worth cutting into K slices in memory keeps its own launch: the slices are summed by another)
+            fits = (bias is not None or split_k_factor(m, n_out, k) == 1) and residual_in_epilogue(m, n_out, k, res)
+        if fits:
+            out = gemm_bf16(a.reshape(-1, k), b, bias=bias, aux="add", aux_in=res).reshape(*a.shape[:-1], n_out)
             _store(add, [[out]], keep_graph)
         else:
             _plain(lin, keep_graph)

@@ -142,6 +142,18 @@ def cluster_slices(M: int, N: int, K: int) -> int:
         return 1
 
 
+def residual_in_epilogue(M: int, N: int, K: int, res: torch.Tensor) -> bool:
+    """Is ``a @ b + res`` one launch, or is the sum better left to another? An epilogue reads the addend in 16-byte pieces only
+    where its rows and the result's start on 16-byte boundaries; of other rows it reads 2 bytes at a time from 32 rows at once (us,
+    two launches and one: 4096 x 10001 x 512 136, 811; 333 x 1001 x 512 9.8, 17.6; 4096 x 512 x 512 with rows of 515 15, 32). The
+    sum of K slices reads whole rows whatever their alignment (4096 x 77 x 2048 10.5, 8.6)."""
+    if cluster_slices(M, N, K) > 1:
+        return True
+    if N % 8:
+        return False
+    return res.stride(-1) != 1 or (res.stride(0) % 8 == 0 and res.data_ptr() % 16 == 0)     # (strided columns are copied first)
+
+
 def split_k_factor(M: int, N: int, K: int) -> int:
     """How many K slices a weight-gradient-shaped GEMM (few output tiles, long K) is cut into: 1 (no
     split), 2, 4 or 8. A small cost model of the kernel picks it: whole waves of tiles over the SMs,

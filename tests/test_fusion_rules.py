@@ -125,3 +125,15 @@ def test_a_group_with_a_large_tensor_is_left_to_single_updates():
 
     leaves = [tuple(torch.zeros(n) for _ in range(4)) + (True,) for n in (8, (1 << 20) + 8)]
     assert kernels.adamw_group(leaves, lr=1e-3, b1=0.9, b2=0.99, eps=1e-8, wd=0.0, step=1) is None
+
+
+@pytest.mark.parametrize("slices,shape,view,fused", [
+    (1, (64, 512), lambda r: r, True), (1, (64, 77), lambda r: r, False), (1, (64, 515), lambda r: r[:, :512], False), (1, (65, 512), lambda r: r[1:], True),
+    (1, (64, 513), lambda r: r.reshape(-1)[1:64 * 512 + 1].view(64, 512), False), (1, (512, 64), lambda r: r.t(), True), (1, (77, 64), lambda r: r.t(), False),
+    (2, (64, 77), lambda r: r, True), (2, (64, 515), lambda r: r[:, :512], True)])
+def test_residual_rows_that_the_epilogue_reads_in_pieces_of_two_bytes_are_added_behind_it(monkeypatch, slices, shape, view, fused):
+    from nabla_b200.native import gemm
+
+    monkeypatch.setattr(gemm, "cluster_slices", lambda *a: slices)
+    r = view(torch.zeros(shape, dtype=torch.bfloat16))
+    assert gemm.residual_in_epilogue(r.shape[0], r.shape[1], 512, r) == fused
