@@ -8,9 +8,9 @@
 //   warp 2       TMEM allocator (2 accumulator buffers of BN columns each)
 //   warps 4..11  epilogue, two groups of four warps (a warp reads the TMEM lane quarter warp % 4):
 //                tcgen05.ld the accumulator, bias / relu / gelu / d-activation / residual add, cast
-//                and store. For the erf-gelu and d-gelu epilogues the groups take alternate
-//                64-column pairs of the tile, which keeps them shorter than the tile's MMAs; plain
-//                epilogues run on group 0 alone. The epilogue overlaps the next tile's MMAs
+//                and store. For the gelu and d-gelu epilogues and for a residual the groups take
+//                alternate 64-column pairs of the tile, which keeps them shorter than the tile's MMAs;
+//                plain epilogues run on group 0 alone. The epilogue overlaps the next tile's MMAs
 //                (double-buffered TMEM).
 //
 // Both operands may be K-major (row = M or N index, K contiguous) or MN-major (row = K index,
@@ -436,13 +436,16 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
     const int wq = warp & 3;                 // TMEM lane quarter this warp may read
     const int et = threadIdx.x - 128;        // 0..255
     // two epilogue groups share every tile: group g takes the 64-column pairs with (pair & 1) == g,
-    // so the per-element math of the gelu / d-gelu epilogues fits under the tile's MMAs
+    // so the per-element work of the gelu, d-gelu and residual epilogues fits under the tile's MMAs
     const int grp = (warp - 4) >> 2;
     // bf16 rows that are not 16-byte aligned (N or ldc not a multiple of 8: an odd vocabulary) leave through
     // shared memory as runs of 64 columns of one row. A lane storing its own row would touch 32 rows, 32
     // sectors, per 2-byte store: 4096 x 10001 x 512 took 554 us, 153 this way.
     const bool staged = MODE == MODE_NONE && !args.vec_ok && !args.out_fp32 && !args.accumulate;
-    const bool heavy = (args.epi == EPI_BIAS_GELU || args.aux == AUX_MUL_DGELU) && !staged;
+    // (a residual is loads that four warps wait for: by group 0 alone the sum was slower than a launch of its own behind 256-wide
+    // tiles; us, two launches, one, one on both groups: 8192 x 1024 x 1024 27.1, 30.5, 25.0; 4096 x 4096 x 1024 46, 55, 43;
+    // 16384 x 2048 x 2048 118, 113, 101)
+    const bool heavy = (args.epi == EPI_BIAS_GELU || args.aux == AUX_MUL_DGELU || args.aux == AUX_ADD) && !staged;
     float alpha = args.alpha;
     if (args.alpha_dev != nullptr)
       alpha *= args.alpha_fp32 ? *reinterpret_cast<const float*>(args.alpha_dev)
@@ -931,13 +934,20 @@ gemm_bf16_slices_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const long long at = static_cast<long long>(m) * args.ldc + n;
     if (!NB_IN_BOUNDS(NB_SITE_GEMM_STORE, at, static_cast<long long>(args.M - 1) * args.ldc + args.N)) continue;
     const int cols = min(4, args.N - n);
+    float r4[4] = {0.f, 0.f, 0.f, 0.f};              // the residual (2 bytes at a time 2048 x 512 x 2048 took 12.3 us, 10.8 so)
+    const bool whole = cols == 4 && args.vec_ok;
+    if (args.aux == AUX_ADD && whole) {
+      const uint2 a = *reinterpret_cast<const uint2*>(args.aux_in + static_cast<long long>(m) * args.ld_aux + n);
+      r4[0] = __uint_as_float(a.x << 16); r4[1] = __uint_as_float(a.x & 0xffff0000u);
+      r4[2] = __uint_as_float(a.y << 16); r4[3] = __uint_as_float(a.y & 0xffff0000u);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (j >= cols) continue;
       if (args.bias != nullptr && args.epi == EPI_BIAS)
         f[j] += args.bias_fp32 ? reinterpret_cast<const float*>(args.bias)[n + j]
                                : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(args.bias)[n + j]);
-      if (args.aux == AUX_ADD) f[j] += __bfloat162float(args.aux_in[static_cast<long long>(m) * args.ld_aux + n + j]);
+      if (args.aux == AUX_ADD) f[j] += whole ? r4[j] : __bfloat162float(args.aux_in[static_cast<long long>(m) * args.ld_aux + n + j]);
     }
     if (args.out_fp32) {
       float* o = reinterpret_cast<float*>(args.out) + at;

@@ -270,6 +270,22 @@ def test_compiled_products_without_native_kernels(kind, monkeypatch):
     assert kind in str(f.dump_plan()) and gemm.launch_count == n
 
 
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("M,N,K", [(9473, 72, 64), (9600, 200, 64), (9473, 264, 128), (4800, 456, 64), (9473, 8, 64), (300, 328, 64), (130, 1096, 2048), (257, 128, 2048)])
+def test_residual_in_wide_and_sliced_tiles(M, N, K, fp32):
+    """Both epilogue groups read a residual: ends of their 64-column pairs, of tiles of every width and of K slices."""
+    from nabla_b200.native.gemm import gemm_bf16
+
+    torch.manual_seed(M + N)
+    a, b, res = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, K), (K, N), (M, N)))
+    bias = torch.randn(N, device="cuda")
+    ref = a.double() @ b.double() + bias.double() + res.double()
+    out = gemm_bf16(a, b, bias=bias, aux="add", aux_in=res, out_dtype=torch.float32 if fp32 else torch.bfloat16)
+    # fp32: each MMA of 16 products cuts its sum by less than one unit in the last place
+    err = (out.double() - ref).abs().max().item()
+    assert err <= (K / 16 * 2.0 ** -23 + (0 if fp32 else 2.0 ** -8)) * ref.abs().max().item()
+
+
 def test_threads_that_ask_first_agree_on_the_slices():
     """Eight threads of a new process plan their first product at the same time; each has to get what a later call gets."""
     code = """
