@@ -3006,6 +3006,44 @@ int nb_conv2d_wgrad_slices(long long positions, int K, int F) {
   if (z > (positions + 255) / 256) z = (positions + 255) / 256;
   return (int)(z < 1 ? 1 : z);
 }
+// Bands of output rows for the filter gradient from patches, and whether to take it: where a band of some 96 positions (whole
+// rows of one image) fits 48 KB and there are taps to share it (one tap: 256 x 14 x 14 x 16 -> 32 13.0 us without, 15.0 with), and
+// the patches pay. Over 320 sizes in both types (4 to 224 pixels a side, 1 to 64 channels, filters of 2 to 7) they were 0.34 to 1.75
+// times as fast as the gathering kernel, 109 times slower by 3 % or more; with these lines 7 times, by 9 % at most:
+//  - bands of few positions are barriers (us, gathered and from patches: 100 x 4 x 4 x 24 -> 17 of stride 2, 4 positions, 17, 52;
+//    256 x 5 x 5 x 16 -> 32 19.0, 23.2; 64 x 7 x 7 x 16 -> 16, 49 positions, 15.3, 13.2; one channel at a time, where gathering is slow,
+//    64 x 6 x 6 x 5 -> 4 pays from 24 on);
+//  - a slice has to stage less than it would gather, whole bands and halo included (64 x 28 x 28 x 16 -> 32, 2 x 2 of stride 2, every
+//    value once, 19.7, 25.8; 1 x 224 x 224 x 3 -> 16 of stride 2 bf16 20.3, 21.9, fp32 22.5, 20.4), by half where dy comes one value at
+//    a time beside whole pixels (1 x 112 x 112 x 24 -> 17, 5 x 5, 32, 37.5), and with no part of a band too much there for two
+//    filter tiles (16 x 28 x 28 x 16 -> 17 20.2, 22.0);
+//  - on a full chip (z fills it, of which whole bands take less) by no more than a fifth (64 x 28 x 28 x 16 -> 32 31.4, 34.4).
+struct WgradPatches {
+  int th, bands, slices;
+  long long smem;
+  bool take;
+};
+static WgradPatches wgrad_patches(const ConvGeom& g, int z, bool vec, bool dvec, int dtype) {
+  const int K = g.R * g.S * g.C, kt = K <= 16 ? 16 : K <= 32 ? 32 : 64, ft = g.F <= 16 ? 16 : 32, kv = vec ? 4 : 1;
+  const long long image = (long long)g.OH * g.OW, per = ((long long)g.N * image + z - 1) / z;
+  const int nb = image >= 2 * 96 ? (int)min((long long)g.OH, image / 96) : 1, th = g.OH > 0 ? (g.OH + nb - 1) / nb : 1, bands = (g.OH + th - 1) / th;
+  const long long total = (long long)g.N * bands, rounds = (total + z - 1) / z, count = (long long)th * g.OW;
+  const long long spanned = ((long long)kt / kv + g.R * g.S - 2) / (g.R * g.S) + 1, channels = min(spanned * kv, (long long)g.C);
+  const long long staged = ((long long)(th - 1) * g.sh + g.R) * ((long long)(g.OW - 1) * g.sw + g.S) * channels;
+  WgradPatches p{th, bands, z, 4ll * ((staged + 3) / 4 * 4 + count * (ft + 1)), false};
+  if (g.R * g.S <= 1 || p.smem > 48 * 1024 || total <= 0 || total >= 0x7fffffffll) return p;
+  p.slices = (int)((total + rounds - 1) / rounds);           // no more than `part` has
+  const bool scalar_dy = vec && !dvec;
+  const long long tiles = (long long)((K + kt - 1) / kt) * ((g.F + ft - 1) / ft);
+  p.take = count >= (vec || K <= 16 ? 40 : 24) && 100 * per * min(kt, K) >= rounds * staged * (scalar_dy ? 200 : !vec && dtype ? 125 : 110) &&
+           !(scalar_dy && g.F > 16 && 10 * rounds * count > 11 * per) && !(vec && K > 64 && tiles * z >= 444 && 5 * rounds * count > 6 * per);
+  return p;
+}
+// For tests: does nb_conv2d_wgrad_direct take patches (x and dy aligned)?
+int nb_conv2d_wgrad_patches(int N, int H, int W, int C, int R, int S, int F, int OH, int OW, int sh, int sw, int dtype) {
+  const ConvGeom g{N, H, W, C, R, S, F, OH, OW, sh, sw, 0, 0};
+  return wgrad_patches(g, nb_conv2d_wgrad_slices((long long)N * OH * OW, R * S * C, F), C % 4 == 0, F % 4 == 0, dtype).take;
+}
 // part: fp32 scratch of nb_conv2d_wgrad_slices(N * OH * OW, R * S * C, F) * R * S * C * F elements.
 int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part, int N, int H, int W, int C, int R, int S, int F,
                            int OH, int OW, int sh, int sw, int pt, int pl, int dtype, void* stream) {
@@ -3017,17 +3055,11 @@ int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part,
   const long long per = (positions + z - 1) / z;
   const ConvGeom g{N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl};
   const bool vec = C % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & (dtype ? 7 : 15)) == 0;
-  // Patches where a band of some 96 positions (whole rows of one image) fits 48 KB and there are taps to share it (one tap: 256 x
-  // 14 x 14 x 16 -> 32 13.0 us without, 15.0 with); no more slices than `part` has.
-  const int ft = F <= 16 ? 16 : 32;
-  const long long image = (long long)OH * OW;
-  const int nb = image >= 2 * 96 ? (int)min((long long)OH, image / 96) : 1, th = OH > 0 ? (OH + nb - 1) / nb : 1, bands = (OH + th - 1) / th;
-  const long long total = (long long)N * bands;
-  const long long ub = (K <= 16 ? 16 : K <= 32 ? 32 : 64) / (vec ? 4 : 1), spanned = (ub + R * S - 2) / (R * S) + 1, c_max = spanned * (vec ? 4 : 1);
-  const long long smem = 4ll * ((((long long)(th - 1) * sh + R) * ((long long)(OW - 1) * sw + S) * (c_max < C ? c_max : C) + 3) / 4 * 4 + (long long)th * OW * (ft + 1));
-  const bool patch = R * S > 1 && smem <= 48 * 1024 && total > 0 && total < 0x7fffffffll;
-  const int rounds = (int)((total + z - 1) / z), zp = patch ? (int)((total + rounds - 1) / rounds) : z;
   const int dvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(dy) & (dtype ? 7 : 15)) == 0;
+  const WgradPatches pp = wgrad_patches(g, z, vec, dvec, dtype);
+  const bool patch = pp.take;
+  const int zp = patch ? pp.slices : z, th = pp.th, bands = pp.bands;
+  const long long total = (long long)N * bands, smem = pp.smem;
   const size_t dyn = smem < 8192 ? 8192 : (size_t)smem;    // (the sum of the position slices of a block takes 8 KB)
 #define WGRAD_V(T, KG, FG, VEC)                                                                                                          \
   do {                                                                                                                                   \

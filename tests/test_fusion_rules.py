@@ -137,3 +137,18 @@ def test_residual_rows_that_the_epilogue_reads_in_pieces_of_two_bytes_are_added_
     monkeypatch.setattr(gemm, "cluster_slices", lambda *a: slices)
     r = view(torch.zeros(shape, dtype=torch.bfloat16))
     assert gemm.residual_in_epilogue(r.shape[0], r.shape[1], 512, r) == fused
+
+
+@pytest.mark.parametrize("N,H,C,F,R,stride,fp32,bf16", [
+    (256, 28, 1, 16, 3, 1, True, True), (256, 14, 16, 32, 3, 1, True, True), (256, 14, 16, 32, 1, 1, False, False),      # taps to share a band
+    (64, 7, 16, 16, 3, 1, True, True), (256, 6, 16, 32, 3, 1, False, False), (100, 4, 24, 17, 3, 2, False, False),         # positions of a band
+    (64, 6, 5, 4, 5, 1, True, True), (8, 4, 5, 9, 3, 1, False, False), (64, 6, 1, 48, 3, 1, False, False),
+    (64, 28, 16, 32, 2, 2, False, False), (1, 224, 3, 16, 3, 2, True, False), (1, 224, 8, 16, 3, 2, False, False),         # what a slice stages
+    (1, 112, 24, 17, 5, 1, False, False), (16, 28, 16, 17, 3, 1, False, False), (16, 28, 16, 20, 5, 1, True, True),        # dy one value at a time
+    (64, 28, 16, 32, 3, 1, False, False), (1, 512, 64, 8, 7, 1, False, False)])                                              # a full chip; 48 KB
+def test_filter_gradients_that_read_patches(N, H, C, F, R, stride, fp32, bf16):
+    from nabla_b200.native import load
+
+    o = (H + 2 * (R // 2) - R) // stride + 1
+    ask = load("libnb_kernels.so").nb_conv2d_wgrad_patches
+    assert [bool(ask(N, H, H, C, R, R, F, o, o, stride, stride, dtype)) for dtype in (0, 1)] == [fp32, bf16]
