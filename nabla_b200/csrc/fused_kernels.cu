@@ -2917,6 +2917,49 @@ int nb_pool2d_select(const void* x, const void* t, void* y, int N, int H, int W,
   return CHECK_LAUNCH();
 }
 
+// Forward from patches: positions per thread (0: not taken), output rows of a band, and the filter tiles of 4 `fg` channels. Where the patch and
+// the filter tile fit 48 KB, positions fill the threads to 60 % (rows of one image only) and there are blocks enough, but not
+// one channel at a time with a stride (bank conflicts: 16 x 112 x 112 x 3 -> 64, 7 x 7 of stride 2, 59.5 us tiled, 67.2 from patches): 8 positions
+// per thread from two blocks per SM on, 4 from 48 blocks on (148 where a sum has few terms or strides widen the patches: 1 x 224 x 224
+// x 3 -> 16 of stride 2 5.6 us, 7.7 from 112 patches). Of 260 sizes in either type that these lines take the patches were slower in 74, down
+// to 0.66 of the tiled kernel's speed; with the following in 6, at 0.87 and more (us, tiled and from patches):
+//  - channels in fours: whole output vectors and a value staged for at least 1.75 terms, or one tap (64 x 24 x 24 x 32 -> 1, 1 x 1, 4.7,
+//    7.1; 100 x 32 x 32 x 32 -> 32, 1 x 1 of stride 2, 7.2, 9.0; 100 x 40 x 40 x 12 -> 16, 2 x 2 of stride 2, 8.0, 9.6); results one by one only where
+//    sums are longer than 64 terms (256 x 12 x 12 x 8 -> 33, 2 x 2, 14.3, 18.1; 256 x 32 x 32 x 12 -> 33, 3 x 3, 175, 122);
+//  - one channel at a time: whole vectors, one tap or at least 5 terms per value, 56 positions and a tile mostly of channels that exist
+//    (16 x 40 x 40 x 1 -> 32 6.0, 7.7; 100 x 12 x 12 x 1 -> 64 6.0, 7.6; 32 x 112 x 112 x 5 -> 20 80, 92; 128 x 64 x 64 x 1 -> 8 18.6, 14.0), or sums
+//    of 200 terms and more (100 x 64 x 64 x 5 -> 7, 7 x 7, 132, 100).
+struct ConvPatches {
+  int px, th, bands, fg;
+  long long f_tiles;
+};
+static ConvPatches conv_patches(const ConvGeom& g, bool vec, bool fvec) {
+  const int fg = g.F <= 8 ? 2 : g.F <= 16 ? 4 : 8;
+  const long long f_tiles = (g.F + 4 * fg - 1) / (4 * fg), K = (long long)g.R * g.S * g.C;
+  ConvPatches p{0, 0, 0, fg, f_tiles};
+  for (int c = 8; c >= 4 && !p.px && K > 0 && (vec || g.sw == 1); c -= 4) {   // (an empty sum stays tiled)
+    const int mt = 128 / fg * c;
+    if (g.OW > mt) continue;
+    const int nb = (g.OH + mt / g.OW - 1) / (mt / g.OW), rows = (g.OH + nb - 1) / nb, bands = (g.OH + rows - 1) / rows;
+    const long long patch = ((long long)(rows - 1) * g.sh + g.R) * ((long long)(g.OW - 1) * g.sw + g.S) * g.C, count = (long long)rows * g.OW;
+    if (5ll * g.OH * g.OW < 3ll * nb * mt || 4ll * K * 4 * fg + 4 * patch > 48 * 1024 ||
+        (long long)g.N * nb * f_tiles < (c == 8 ? 2 * 148 : K >= 32 && g.sh * g.sw == 1 ? 48 : 148))
+      continue;
+    // terms per staged value: K count / patch
+    const bool tap = g.R * g.S == 1 && g.sh * g.sw == 1;
+    const bool pays = vec ? (fvec ? tap || 4 * K * count >= 7 * patch : K > 64 && 2 * K * count >= 5 * patch)
+                          : K >= 200 || (fvec && (tap || (K * count >= 5 * patch && count >= 56 && 10ll * g.F >= 7 * f_tiles * 4 * fg)));
+    if (!pays || (long long)g.N * bands >= 0x7fffffffll || f_tiles > 65535) break;
+    p = ConvPatches{c, rows, bands, fg, f_tiles};
+  }
+  return p;
+}
+// For tests: positions per thread where nb_conv2d_direct takes patches (all operands aligned), 0 where it does not.
+int nb_conv2d_patches(int N, int H, int W, int C, int R, int S, int F, int OH, int OW, int sh, int sw) {
+  if (OH <= 0 || OW <= 0) return 0;
+  return conv_patches(ConvGeom{N, H, W, C, R, S, F, OH, OW, sh, sw, 0, 0}, C % 4 == 0, F % 4 == 0).px;
+}
+
 int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int R, int S,
                      int F, int OH, int OW, int sh, int sw, int pt, int pl, int dtype, void* stream) {
   const size_t positions = (size_t)N * OH * OW;
@@ -2928,25 +2971,12 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
     const unsigned tiles = (unsigned)((F + 4ll * fg - 1) / (4 * fg));
     return dim3((unsigned)((positions + 256 / fg - 1) / (256 / fg)), tiles < 65535u ? tiles : 65535u, (tiles + 65534u) / 65535u);
   };
-  // Patches where they and the filter tile fit 48 KB, positions fill the threads to 60 % (rows of one image only) and there are
-  // blocks enough, but not one channel at a time with a stride (bank conflicts: 16 x 112 x 112 x 3 -> 64, 7 x 7 of stride 2, 59.5 us
-  // tiled, 67.2 from patches): 8 positions per thread from two blocks per SM on, 4 from 48 blocks on (148
-  // where a sum has few terms or strides widen the patches: 1 x 224 x 224 x 3 -> 16 of stride 2 5.6 us, 7.7 from 112 patches).
-  const int fg_w = F <= 8 ? 2 : F <= 16 ? 4 : 8;
-  const long long f_tiles = (F + 4 * fg_w - 1) / (4 * fg_w);
-  int px = 0, th = 0, bands = 0;
-  for (int c = 8; c >= 4 && !px && R * S * C > 0 && (vec || sw == 1); c -= 4) {   // (an empty sum stays tiled)
-    const int mt = 128 / fg_w * c;
-    if (OW > mt) continue;
-    const int nb = (OH + mt / OW - 1) / (mt / OW), rows = (OH + nb - 1) / nb;
-    const long long smem = 4ll * R * S * C * 4 * fg_w + 4ll * (((long long)(rows - 1) * sh + R) * ((long long)(OW - 1) * sw + S) * C);
-    if (5ll * OH * OW < 3ll * nb * mt || smem > 48 * 1024 || N * (long long)nb * f_tiles < (c == 8 ? 2 * 148 : R * S * C >= 32 && sh * sw == 1 ? 48 : 148)) continue;
-    px = c; th = rows; bands = (OH + rows - 1) / rows;
-  }
-  if (px && (long long)N * bands < 0x7fffffffll && f_tiles <= 65535) {
+  const int low = dtype ? 7 : 15, wvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & low) == 0, yvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & low) == 0;
+  const ConvPatches pp = conv_patches(g, vec, wvec && yvec);
+  if (pp.px) {
+    const int px = pp.px, th = pp.th, bands = pp.bands, fg_w = pp.fg;
     const size_t smem = 4 * ((size_t)R * S * C * 4 * fg_w + (size_t)((th - 1) * sh + R) * ((OW - 1) * sw + S) * C);
-    const int low = dtype ? 7 : 15, wvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & low) == 0, yvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & low) == 0;
-    const dim3 pgrid((unsigned)(N * bands), (unsigned)f_tiles);
+    const dim3 pgrid((unsigned)(N * bands), (unsigned)pp.f_tiles);
 #define PATCH_V(T, FG, PX, VEC) conv2d_patch_kernel<T, FG, PX, VEC><<<pgrid, 128, smem, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec)
 #define PATCH_P(T, FG, PX) do { if (vec) PATCH_V(T, FG, PX, true); else PATCH_V(T, FG, PX, false); } while (0)
 #define PATCH(T, FG) do { if (px == 8) PATCH_P(T, FG, 8); else PATCH_P(T, FG, 4); } while (0)

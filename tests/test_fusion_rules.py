@@ -152,3 +152,16 @@ def test_filter_gradients_that_read_patches(N, H, C, F, R, stride, fp32, bf16):
     o = (H + 2 * (R // 2) - R) // stride + 1
     ask = load("libnb_kernels.so").nb_conv2d_wgrad_patches
     assert [bool(ask(N, H, H, C, R, R, F, o, o, stride, stride, dtype)) for dtype in (0, 1)] == [fp32, bf16]
+
+
+@pytest.mark.parametrize("N,E,C,F,R,stride,px", [
+    (256, 28, 1, 16, 3, 1, 8), (256, 14, 16, 32, 3, 1, 8), (16, 16, 8, 32, 3, 1, 4), (1, 14, 16, 32, 3, 1, 0),                # blocks enough
+    (256, 14, 16, 32, 1, 1, 8), (100, 32, 32, 32, 1, 2, 0), (100, 40, 12, 16, 2, 2, 0), (16, 128, 8, 16, 3, 2, 4),           # terms per value
+    (64, 24, 32, 1, 1, 1, 0), (256, 12, 8, 33, 2, 1, 0), (256, 32, 12, 33, 3, 1, 8),                                          # results one by one
+    (16, 40, 1, 32, 3, 1, 0), (100, 12, 1, 64, 3, 1, 0), (32, 112, 5, 20, 3, 1, 0), (128, 64, 1, 8, 3, 1, 8), (64, 56, 3, 32, 1, 1, 8),
+    (100, 64, 5, 7, 7, 1, 8), (16, 112, 3, 64, 7, 2, 0), (64, 64, 64, 64, 5, 1, 0)])
+def test_convolutions_that_read_patches(N, E, C, F, R, stride, px):
+    from nabla_b200.native import load
+
+    o = (E + 2 * (R // 2) - R) // stride + 1
+    assert load("libnb_kernels.so").nb_conv2d_patches(N, E, E, C, R, R, F, o, o, stride, stride) == px
