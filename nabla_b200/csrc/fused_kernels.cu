@@ -1019,7 +1019,7 @@ __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restri
 // out = base + scatter_add(ids, upd): the gradient of an embedding.
 // Large tables: the ids are bucketed by row (three short launches over the integers), and one launch writes every
 // row of the table once: rows that occur as the fp32 sum of their updates in registers, the others as zeros or as the
-// base's row. No fp32 table that is zeroed, added to with atomics and converted, and no fill of `out` before it.
+// base's row. No fp32 table that is zeroed, added to with atomics and converted, and, but for crowded tables, no fill of `out`.
 // A row with at most SCAT_LIGHT entries is one warp's work (its loads are a list entry and then the rows, two
 // latencies in a chain, so what counts is how many rows the chip has on its way: 4 KB rows by a block each were 1.4 TB/s);
 // a row with more takes the whole block, in segments of SCAT_SEG entries whose fp32 partial rows are added up in two
@@ -1027,12 +1027,13 @@ __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restri
 // groups. One block per row would leave the most frequent id, some 1000 of 16384 tokens (ids of text fall off about as
 // 1 / rank), to one block, and joining them in one step the padding id of a batch (29700 of 33000 ids into 4097 x 2048
 // fp32: 881 us in one step, 128 in two).
-// 16384 ids of text into 32000 x 2048 bf16: fill 23 + rows 34 us before, 49 now (131 MB written, 67 read: 30 us at the
-// copy rate).
+// 16384 ids of text into 32000 x 2048 bf16, bucketing included: fill and rows 68 us, 54 so (131 MB written, 67 read: 30 us at the
+// copy rate); onto a base table 92, 79.
 constexpr int SCAT_SEG = 32, SCAT_GROUP = 32, SCAT_LIGHT = 4;
 struct ScatWs {
   int *counts, *done, *total, *nseg, *nheavy, *nlight;   // zeroed by the launcher
-  int* gdone;                                   // likewise: finished segments of a group, at its first partial row
+  int light;                                    // most entries of a row that one warp adds: SCAT_LIGHT, or 0
+  int* gdone;                                   // likewise zeroed: finished segments of a group, at its first partial row
   int *start, *rank, *list;                     // first list slot per row; place of an entry in its row; entries by row
   int4* seg;                                    // (row, first list slot, entries, partial row or -1): the rows of at most
                                                 // SCAT_LIGHT entries from the end backwards, the others from the start on
@@ -1090,7 +1091,7 @@ __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int n_ids
   if (threadIdx.x == 0) nmany = 0;                   // (the scan below has the barrier)
   const int v = blockIdx.x * 256 + threadIdx.x;
   const int c = v < vocab ? ws.counts[v] : 0;
-  const bool light = c <= SCAT_LIGHT;
+  const bool light = c <= ws.light;
   const int k = light ? 0 : (c + SCAT_SEG - 1) / SCAT_SEG;
   const unsigned long long t = (unsigned long long)(c > 0 && light) << 32 | (unsigned)c;     // (light rows, entries)
   unsigned long long total, heavy = 0;
@@ -1255,9 +1256,21 @@ __device__ __forceinline__ void scatter_idle(const T* __restrict__ base, T* __re
     for (unsigned m = __ballot_sync(0xffffffffu, idle); m; m &= m - 1) {
       const size_t at = (size_t)(v0 + __ffs(m) - 1) * D;
       if (base != nullptr) {
-        for (size_t c = lane * VN; c < D; c += 32 * VN) {
-          if (VN > 1) *reinterpret_cast<uint4*>(out + at + c) = *reinterpret_cast<const uint4*>(base + at + c);
-          else out[at + c] = base[at + c];
+        constexpr int U = 8;                         // loads on their way per lane
+        for (size_t c = lane * VN; c < D; c += 32 * VN * U) {
+          if constexpr (VN > 1) {
+            uint4 r[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (c + u * 32 * VN < D) r[u] = *reinterpret_cast<const uint4*>(base + at + c + u * 32 * VN);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (c + u * 32 * VN < D) *reinterpret_cast<uint4*>(out + at + c + u * 32 * VN) = r[u];
+          } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (c + u * 32 < D) out[at + c + u * 32] = base[at + c + u * 32];
+          }
         }
       } else {
         for (size_t c = lane * VN; c < D; c += 32 * VN) {
@@ -1269,19 +1282,20 @@ __device__ __forceinline__ void scatter_idle(const T* __restrict__ base, T* __re
     if (v0 > vocab - nwarps * SCAT_IDLE) break;      // (the next v0 may not fit an int)
   }
 }
-// Every row of the table, once. The blocks walk the segments of crowded rows, the next descriptor on its way while one is
+// ALL: every row of the table, once. The blocks walk the segments of crowded rows, the next descriptor on its way while one is
 // worked on; then their warps the rows of few entries. Every other block writes its rows without an entry first, the rest
-// last, so that stores and dependent loads run side by side. VN: elements per access (16 bytes, or 1 where rows are not
-// 16-byte aligned).
-template <typename T, int VN>
+// last, so that stores and dependent loads run side by side. Else only the rows that occur, all of them by blocks, over a table that
+// holds the base: what the other form does besides costs this one registers. VN: elements per access (16 bytes, or 1 where rows are
+// not 16-byte aligned).
+template <typename T, int VN, bool ALL>
 __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
                                                           T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
                                                           int D, int vocab) {
   __shared__ int last;
-  const int total = *ws.nseg, lights = *ws.nlight;
+  const int total = *ws.nseg, lights = ALL ? *ws.nlight : 0;
   const int lane = threadIdx.x & 31, nwarps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;         // few rows: spread over the blocks
-  if (blockIdx.x & 1) scatter_idle<T, VN>(base, out, ws.counts, vocab, D, warp, nwarps, lane);
+  if (ALL && (blockIdx.x & 1)) scatter_idle<T, VN>(base, out, ws.counts, vocab, D, warp, nwarps, lane);
   int4 next = make_int4(0, 0, 0, -1);
   if ((int)blockIdx.x < total) next = ws.seg[blockIdx.x];
   for (int s = blockIdx.x; s < total; s += gridDim.x) {
@@ -1333,6 +1347,7 @@ __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(cons
       scatter_write<T, VN>(base, out, (size_t)v * D + c, acc);
     }
   }
+  if (!ALL) return;
   const int4* lseg = ws.seg + n_ids - 1;
   int4 lnext = make_int4(0, 0, 0, -1);
   if (lwarp < lights) lnext = lseg[-lwarp];
@@ -2709,12 +2724,20 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
     else if (!direct) cast_kernel<float, float><<<grid, 256, 0, STREAM>>>(acc, (float*)out, n, (const float*)base);
     return CHECK_LAUNCH();
   }
-  if (n_ids == 0) {
+  // Crowded tables: rows of few entries are few, and the time is that of the long ones. us, all rows in one launch and a copied base
+  // (or zeros) under the rows that occur: 16384 ids into 1000 x 2048 fp32 62, 52, bf16 36.5, 36.6; 33000 with 90 % padding into
+  // 4097 x 2048 fp32 101, 95, bf16 30000 into 4096 58, 60; 65536 into 2000 x 1024 bf16 52, 50; below the line 60000 into 5000 x 1024 60, 67,
+  // 65536 into 32000 x 1024 67, 90, with a base 82, 105.
+  const bool crowded = n_ids >= (dtype == 0 && D >= 1024 ? 4ll : 24ll) * vocab;
+  if (n_ids == 0 || crowded) {
     const size_t bytes = (size_t)vocab * D * (dtype ? 2 : 4);
-    return (base != nullptr ? cudaMemcpyAsync(out, base, bytes, cudaMemcpyDeviceToDevice, STREAM)
-                            : cudaMemsetAsync(out, 0, bytes, STREAM)) == cudaSuccess ? 0 : -1;
+    if ((base != nullptr ? cudaMemcpyAsync(out, base, bytes, cudaMemcpyDeviceToDevice, STREAM)
+                         : cudaMemsetAsync(out, 0, bytes, STREAM)) != cudaSuccess)
+      return -1;
+    if (n_ids == 0) return 0;
   }
   ScatWs ws;
+  ws.light = crowded ? 0 : SCAT_LIGHT;
   ws.counts = work;
   ws.done = ws.counts + vocab;
   ws.total = ws.done + vocab;
@@ -2736,12 +2759,16 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
   const bool vec = D % V == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   int threads = 32;                                  // the power of two that covers a row in one pass, at most 256
   while (threads < 256 && threads * (vec ? V : 1) < D) threads *= 2;
-  // blocks: what the chip holds, or as many as there are entries and groups of SCAT_IDLE rows for their warps
-  const long long held = 148ll * (vec && dtype ? 768 : 1024) / threads, want = ((long long)vocab / SCAT_IDLE + 1) * 32 / threads + 1;
+  // blocks: four times what the chip holds, so that those of short segments make room (one time left the last of the long ones alone:
+  // 16384 ids of text into 32000 x 2048 bf16 62 us, 54 so), or as many as there are entries and groups of SCAT_IDLE rows for their warps
+  const long long held = 148ll * (crowded ? 2048 : 4 * (vec && dtype ? 768 : 1024)) / threads;
+  const long long want = crowded ? n_ids : ((long long)vocab / SCAT_IDLE + 1) * 32 / threads + 1;
   const int grid = (int)(held < n_ids || held < want ? held : n_ids > want ? n_ids : want);
-#define SCAT(T, VN) scatter_rows_kernel<T, VN><<<grid, threads, 0, STREAM>>>((const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D, vocab)
+#define SCAT_R(T, VN, ALL) scatter_rows_kernel<T, VN, ALL><<<grid, threads, 0, STREAM>>>((const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D, vocab)
+#define SCAT(T, VN) do { if (crowded) SCAT_R(T, VN, false); else SCAT_R(T, VN, true); } while (0)
   if (dtype) { if (vec) SCAT(bf16, 8); else SCAT(bf16, 1); }
   else { if (vec) SCAT(float, 4); else SCAT(float, 1); }
+#undef SCAT_R
 #undef SCAT
   return CHECK_LAUNCH();
 }

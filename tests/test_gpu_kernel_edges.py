@@ -439,6 +439,27 @@ def test_embedding_gradient_by_row_counts(dtype, vocab, dim):
     assert not got[idle].any() and _rel2(got[rows], ref[rows]) < STORED[dtype]
 
 
+@pytest.mark.parametrize("dtype,vocab,dim,n", [(torch.float32, 9000, 1048, 35999), (torch.float32, 9000, 1048, 36000), (torch.float32, 1300, 1020, 31200), (torch.float32, 1300, 1020, 31199),
+                                               (torch.bfloat16, 400, 4096, 9600), (torch.bfloat16, 400, 4096, 9599), (torch.bfloat16, 3, 2048, 60000)])
+def test_embedding_gradient_into_crowded_tables(dtype, vocab, dim, n):
+    """Both sides of the line from which on only the rows that occur are written over a copy of the base."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(n)
+    assert kernels._L().nb_embedding_scatter_work(n, dim, vocab, 1 if dtype == torch.bfloat16 else 0) != vocab * dim
+    ids = (vocab * torch.rand(n, device="cuda") ** 3).long().clamp_(max=vocab - 1)
+    ids[ids == 1] = 0                                        # a row without an entry
+    ids[3], ids[7] = -1, vocab                               # outside the table
+    inside = (ids >= 0) & (ids < vocab)
+    upd = torch.randn(n, dim, device="cuda").to(dtype)
+    base = torch.randn(vocab, dim, device="cuda").to(dtype)
+    ref = torch.zeros(vocab, dim, dtype=torch.float64, device="cuda").index_add_(0, ids[inside], upd[inside].double())
+    got = kernels.embedding_scatter_add(base, ids, upd)
+    assert torch.equal(got[1], base[1]) and _rel2(got, ref + base.double()) < STORED[dtype]
+    got = kernels.embedding_scatter_add(None, ids, upd, vocab, dtype)
+    assert not got[1].any() and _rel2(got, ref) < STORED[dtype]
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("ids,add,fused", [
     ((3, 70), (70, 64), True), ((3, 70), (64,), True), ((3, 70), (1, 70, 64), True), ((3, 70), (1, 1, 64), True), ((7,), (7, 64), True),
