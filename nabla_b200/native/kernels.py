@@ -573,6 +573,20 @@ def sgemm_pays(M: int, N: int, K: int) -> bool:
     return min(M, N) > 8 and M * N <= 32768 and 256 <= K <= 4096
 
 
+def sgemm_takes(a: torch.Tensor, b: torch.Tensor) -> bool:
+    """``sgemm_pays`` for the operands at hand. Of up to 16 rows the library has kernels of its own: rows along K times columns along K
+    up to K = 512 (us, library and ``sgemm``: 16 x 64 over 256 3.4, 5.4, over 512 5.1, 5.4, over 700 6.7, 6.3), other orders for few columns
+    of short sums (9 x 9 over 256 4.1, 4.5, 16 x 64 the first transposed 5.1, 5.3) and for many of long ones (16 x 1000 over 512 6.7, 7.1)."""
+    (M, K), N = a.shape, b.shape[1]
+    if not sgemm_pays(M, N, K):
+        return False
+    if M > 16:
+        return True
+    if a.stride(1) == 1 and b.stride(0) == 1:
+        return 512 < K and N <= 512
+    return N <= 512 if K >= 512 else N > 64
+
+
 def sgemm(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor | None:
     """``a @ b [+ bias]`` of small 2-D fp32 matrices of any strides on the CUDA cores; None for anything else."""
     if not (a.is_cuda and a.device == b.device and a.dim() == 2 and b.dim() == 2 and a.dtype == b.dtype == torch.float32

@@ -158,7 +158,7 @@ class MatmulOp(Operation):
         if native.use_native(a) and a.dtype == torch.float32 and a.dim() == 2 and b.dim() == 2:
             from ..native import kernels
 
-            y = kernels.sgemm(a, b) if kernels.sgemm_pays(a.shape[0], b.shape[1], a.shape[1]) else None
+            y = kernels.sgemm(a, b) if kernels.sgemm_takes(a, b) else None
             if y is not None:
                 return y
         return torch.matmul(a, b)
