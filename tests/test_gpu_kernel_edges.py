@@ -668,6 +668,58 @@ def test_attention_with_a_large_common_offset_in_the_mask(S, D, causal):
             assert torch.equal(a, b), offset
 
 
+@pytest.mark.parametrize("S,D,causal", [(700, 64, False), (700, 64, True), (641, 128, False), (700, 128, True), (384, 64, False)])
+def test_attention_with_key_masks_that_are_zero_in_most_tiles(S, D, causal):
+    """Tiles without a mask value between tiles with some, tiles that are hidden whole, and one hidden key in the last of a tile
+    with a remainder: the kernels leave a mask of zeros out tile by tile."""
+    torch.manual_seed(S + D)
+    B = 4
+    m = torch.zeros(B, 1, 1, S, device="cuda")
+    m[0, ..., 256:384] = torch.randn(128, device="cuda")
+    m[1, ..., 128:256] = -float("inf")
+    m[2, ..., 128:384], m[2, ..., -100:] = -1e9, -float("inf")
+    m[3, ..., -1], m[3, ..., 300] = -float("inf"), 2.0
+    if not causal:
+        m[2, ..., :128] = -float("inf")
+        m[2, ..., 200] = 0.0
+    q, k, v = (torch.randn(B, 3, S, D, device="cuda").bfloat16() for _ in range(3))
+    _attention_check(q, k, v, causal, m)
+
+
+@pytest.mark.parametrize("D,keys", [(64, False), (64, True), (128, False)])
+def test_attention_over_key_ranges_that_one_of_two_query_tiles_sees(D, keys):
+    """256 queries over 2048 keys in ranges of one key tile: of the last range the first 128 queries see nothing."""
+    from nabla_b200.native import attention
+
+    torch.manual_seed(D)
+    attention._lib()
+    assert attention._splits(1, 2, 256, 2048, D, int(keys)) == 16
+    q, k, v = (torch.randn(1, 2, s, D, device="cuda").bfloat16() for s in (256, 2048, 2048))
+    m = None
+    if keys:
+        m = torch.zeros(1, 1, 1, 2048, device="cuda")
+        m[..., 700:900], m[..., 2000:] = -float("inf"), 0.5
+    _attention_check(q, k, v, True, m)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_attention_gradients_into_rows_on_16_byte_boundaries(D):
+    """Results whose rows start on 16- and not on 32-byte boundaries are the bits of aligned ones, and nothing beside them is written."""
+    from nabla_b200.native import attention
+
+    torch.manual_seed(0)
+    B, H, S = 2, 3, 200
+    q, k, v, do = (torch.randn(B, H, S, D, device="cuda").bfloat16() for _ in range(4))
+    o, lse = attention.sdpa_fwd(q, k, v, causal=True, scale=0.1)
+    want = attention.sdpa_bwd(do, q, k, v, o, lse, causal=True, scale=0.1)
+    bufs = [torch.zeros(B * S * H * (D + 8) + 8, device="cuda", dtype=torch.bfloat16)[8:].view(B, S, H, D + 8) for _ in range(3)]
+    out = tuple(t[..., :D].permute(0, 2, 1, 3) for t in bufs)
+    assert all(t.data_ptr() % 32 == 16 and t.stride(2) % 16 == 8 for t in out)
+    attention.sdpa_bwd(do, q, k, v, o, lse, causal=True, scale=0.1, out=out)
+    for got, ref, t in zip(out, want, bufs):
+        assert torch.equal(got, ref) and not t[..., D:].any()
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 @pytest.mark.parametrize("S,D", [(130, 64), (300, 128)])
 def test_attention_hides_a_masked_key_that_is_not_finite(S, D, value):
