@@ -255,13 +255,15 @@ def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):
 def embedding_gather(table: torch.Tensor, ids: torch.Tensor, add: torch.Tensor | None = None) -> torch.Tensor | None:
     """Rows of ``table`` (vocab, D) by id. ``add``: a tensor over the trailing dims of the result (at least the
     last), added in the same pass; None when that pass does not take it (the caller then gathers and adds)."""
+    if ids.device != table.device:
+        raise RuntimeError("embedding: expected all tensors to be on the same GPU")
     period = 0
     if add is not None:
         shape = tuple(add.shape)
         while len(shape) > 1 and shape[0] == 1:
             shape = shape[1:]
         full = (*ids.shape, table.shape[1])
-        if add.dtype != table.dtype or not shape or full[len(full) - len(shape):] != shape or not add.numel() \
+        if add.dtype != table.dtype or add.device != table.device or not shape or full[len(full) - len(shape):] != shape or not add.numel() \
                 or not elementwise_enabled():
             return None
         add = add.contiguous()
@@ -284,6 +286,8 @@ def embedding_scatter_add(base: torch.Tensor | None, ids: torch.Tensor, upd: tor
     global launch_count
     from .. import config
 
+    if ids.device != upd.device or (base is not None and base.device != upd.device):
+        raise RuntimeError("embedding: expected all tensors to be on the same GPU")
     if base is None and config.is_deterministic():
         base = torch.zeros((vocab, upd.shape[-1]), dtype=dtype, device=upd.device)
     if base is not None:

@@ -107,6 +107,11 @@ def test_wrappers_refuse_operands_on_the_host():
             gemm.gemm_bf16(*args, **kw)
     with pytest.raises(RuntimeError, match="same GPU"):
         kernels.layernorm_bwd(x, x, None, None, None, add=host)
+    table, ids = _Fake(64, 32, dtype=torch.bfloat16), torch.zeros(5, dtype=torch.int64)
+    with pytest.raises(RuntimeError, match="same GPU"):
+        kernels.embedding_gather(table, ids)
+    with pytest.raises(RuntimeError, match="same GPU"):
+        kernels.embedding_scatter_add(None, ids, table, 64, torch.bfloat16)
 
 
 def test_a_slice_count_that_could_not_be_asked_for_is_not_kept(monkeypatch):
