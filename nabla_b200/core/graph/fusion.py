@@ -705,7 +705,7 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         return
     if kind == "gemm_residual":
         from ... import native
-        from ...native.gemm import gemm_bf16, residual_in_epilogue, split_k_factor
+        from ...native.gemm import cluster_slices, gemm_bf16, residual_in_epilogue, split_k_factor
 
         lin, add = group
         ins = lin.input_impls()
@@ -716,9 +716,11 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         fits = native.use_native(a) and a.numel() > 0 and b.numel() > 0
         if fits:
             m, k, n_out = a.numel() // a.shape[-1], a.shape[-1], b.shape[-1]
-            res = res.reshape(-1, n_out)
             # (a product that is worth cutting into K slices in memory keeps its own launch: the slices are summed by another)
-            fits = (bias is not None or split_k_factor(m, n_out, k) == 1) and residual_in_epilogue(m, n_out, k, res)
+            fits = (bias is not None or split_k_factor(m, n_out, k) == 1) and (n_out % 8 == 0 or cluster_slices(m, n_out, k) > 1)
+        if fits:
+            res = res.reshape(-1, n_out)             # a copy where the rows are not in order: not before it is known to be of use
+            fits = residual_in_epilogue(m, n_out, k, res)
         if fits:
             out = gemm_bf16(a.reshape(-1, k), b, bias=bias, aux="add", aux_in=res).reshape(*a.shape[:-1], n_out)
             _store(add, [[out]], keep_graph)

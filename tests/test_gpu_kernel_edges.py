@@ -271,7 +271,7 @@ def test_compiled_products_without_native_kernels(kind, monkeypatch):
 
 
 @pytest.mark.parametrize("fp32", [False, True])
-@pytest.mark.parametrize("M,N,K", [(9473, 72, 64), (9600, 200, 64), (9473, 264, 128), (4800, 456, 64), (9473, 8, 64), (300, 328, 64), (130, 1096, 2048), (257, 128, 2048)])
+@pytest.mark.parametrize("M,N,K", [(9473, 72, 64), (9600, 200, 64), (9473, 264, 128), (4800, 456, 64), (9473, 8, 64), (300, 328, 64), (130, 1096, 2048), (257, 128, 2048), (9473, 77, 64), (300, 333, 64), (130, 77, 1800)])
 def test_residual_in_wide_and_sliced_tiles(M, N, K, fp32):
     """Both epilogue groups read a residual: ends of their 64-column pairs, of tiles of every width and of K slices."""
     from nabla_b200.native.gemm import gemm_bf16
