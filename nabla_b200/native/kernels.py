@@ -577,18 +577,21 @@ def sgemm_pays(M: int, N: int, K: int) -> bool:
     return min(M, N) > 8 and M * N <= 32768 and 256 <= K <= 4096
 
 
-def sgemm_takes(a: torch.Tensor, b: torch.Tensor) -> bool:
-    """``sgemm_pays`` for the operands at hand. Of up to 16 rows the library has kernels of its own: rows along K times columns along K
-    up to K = 512 (us, library and ``sgemm``: 16 x 64 over 256 3.4, 5.4, over 512 5.1, 5.4, over 700 6.7, 6.3), other orders for few columns
-    of short sums (9 x 9 over 256 4.1, 4.5, 16 x 64 the first transposed 5.1, 5.3) and for many of long ones (16 x 1000 over 512 6.7, 7.1)."""
+def sgemm_takes(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) -> bool:
+    """``sgemm_pays`` for the operands at hand. Of up to 16 rows the library has kernels of its own, quick (us, library and ``sgemm``) at rows along
+    K times columns along K up to K = 512 (16 x 64 over 256 3.4, 5.4, over 512 5.1, 5.4, over 700 6.7, 6.3), at few columns of short sums (9 x 9
+    over 256 4.1, 4.5; 12 x 45 6.4, 5.2; the first operand transposed, 16 x 64 over 400 5.7, 6.3) and at many of long ones (16 x 1000 over 512
+    6.7, 7.1); a bias is a launch more there, so not with one. Over 70
+    sizes of 9 to 32 rows in four orders: 0.85 to 6 times as fast as the library, with a bias 0.88 to 6.4, 8 of 552 below 0.95."""
     (M, K), N = a.shape, b.shape[1]
     if not sgemm_pays(M, N, K):
         return False
-    if M > 16:
+    if M > 16 or bias is not None:
         return True
-    if a.stride(1) == 1 and b.stride(0) == 1:
-        return 512 < K and N <= 512
-    return N <= 512 if K >= 512 else N > 64
+    rows, columns = a.stride(1) == 1, b.stride(0) == 1        # along K
+    if columns:
+        return K > 512 or N >= 1000 if rows else N * K <= 800_000
+    return N * K <= 400_000 and (K >= 512 or N > 64 or (rows and (M > 10 or K >= 320)))
 
 
 def sgemm(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor | None:

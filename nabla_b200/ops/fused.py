@@ -90,7 +90,7 @@ class LinearOp(_Fused):
         if _native(x) and x.dtype == torch.float32 and x.dim() == 2 and w.dim() == 2:
             from ..native import kernels
 
-            z = kernels.sgemm(x, w, b) if kernels.sgemm_takes(x, w) else None
+            z = kernels.sgemm(x, w, b) if kernels.sgemm_takes(x, w, b) else None
         if z is None:
             z = torch.matmul(x, w)
             if b is not None:

@@ -173,12 +173,13 @@ def test_convolutions_that_read_patches(N, E, C, F, R, stride, px):
 
 
 @pytest.mark.parametrize("M,N,K,orders", [            # (rows, rows), (columns, rows), (rows, columns), (columns, columns)
-    (17, 64, 256, [True] * 4), (16, 64, 256, [False] * 4), (16, 65, 256, [True, True, False, True]), (16, 64, 512, [True, True, False, True]),
-    (16, 64, 513, [True] * 4), (16, 513, 600, [False] * 4), (16, 512, 600, [True] * 4), (64, 8, 512, [False] * 4)])
+    (17, 64, 256, [True] * 4), (16, 64, 256, [True, False, False, True]), (10, 64, 256, [False, False, False, True]), (10, 64, 320, [True, False, False, True]),
+    (10, 65, 256, [True, True, False, True]), (16, 64, 512, [True, True, False, True]), (16, 64, 513, [True] * 4), (16, 1000, 400, [True] * 4),
+    (16, 1000, 401, [False, False, True, True]), (16, 1000, 801, [False, False, True, False]), (64, 8, 512, [False] * 4)])
 def test_small_products_of_few_rows_that_the_library_has_kernels_for(M, N, K, orders):
     from nabla_b200.native import kernels
 
     for (ta, tb), takes in zip([(False, False), (True, False), (False, True), (True, True)], orders):
         a = torch.empty(K, M).t() if ta else torch.empty(M, K)
         b = torch.empty(N, K).t() if tb else torch.empty(K, N)
-        assert kernels.sgemm_takes(a, b) == takes
+        assert kernels.sgemm_takes(a, b) == takes and kernels.sgemm_takes(a, b, torch.empty(N)) == kernels.sgemm_pays(M, N, K)
