@@ -582,7 +582,7 @@ def sgemm_takes(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = No
     K times columns along K up to K = 512 (16 x 64 over 256 3.4, 5.4, over 512 5.1, 5.4, over 700 6.7, 6.3), at few columns of short sums (9 x 9
     over 256 4.1, 4.5; 12 x 45 6.4, 5.2; the first operand transposed, 16 x 64 over 400 5.7, 6.3) and at many of long ones (16 x 1000 over 512
     6.7, 7.1); a bias is a launch more there, so not with one. Over 70
-    sizes of 9 to 32 rows in four orders: 0.85 to 6 times as fast as the library, with a bias 0.88 to 6.4, 8 of 552 below 0.95."""
+    sizes of 9 to 32 rows in four orders: 0.85 to 6 times as fast as the library, with a bias 0.88 to 6.4, 7 of 552 below 0.95."""
     (M, K), N = a.shape, b.shape[1]
     if not sgemm_pays(M, N, K):
         return False
