@@ -613,6 +613,18 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
             else:
                 _plain(n_, keep_graph)
         return
+    if kind == "bias_grads":
+        from ... import native
+        from ...native import kernels
+
+        xs = [n_.input_impls()[0]._buffers[0] for n_ in group]
+        if all(native.use_native(x) for x in xs):
+            for n_, o in zip(group, kernels.colsum_group(xs)):
+                _store(n_, [[o]], keep_graph)
+        else:
+            for n_ in group:
+                _plain(n_, keep_graph)
+        return
     if kind == "gather_add":
         from ... import native
 

@@ -14,6 +14,7 @@
 // where the row fits in registers / L1.
 #include <cuda_runtime.h>
 #include <cfloat>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -705,6 +706,95 @@ __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict_
     a[0] += s;
     partial[(size_t)blockIdx.x * N + i] = sum8(a);
   }
+}
+
+// Column sums of several matrices in one launch, without a second one that folds slabs: the blocks of a cluster share a
+// tile of L vectors of columns, walk every row of it between them and meet in distributed shared memory. A block is 256 / L
+// row slots, whose rows are interleaved over the cluster; a thread asks for eight rows before it adds the first and adds
+// them as a tree, so no chain of additions is longer than rows / 64 / (256 / L) + 6. Rows that are not whole aligned
+// vectors go element by element (`vec` of a leaf is 0). Latency bounds it: three dependent rounds (rows, cluster, result) and the
+// launch. 2002 x 512 bf16 5.2 us as slabs and fold, 3.5 so; where the line lies: colsum_clusters in native/kernels.py.
+constexpr int COLSUM_GROUP = 32, COLSUM_CLUSTER = 8;
+struct ColsumGroup {
+  struct Leaf {
+    const void* x;
+    void* out;
+    int rows, N;
+    unsigned tile0;                                  // first column tile of the leaf
+    int vec, out_bf16;
+  } leaf[COLSUM_GROUP];
+  int count;
+};
+template <typename T, int L, bool VEC>
+__device__ __forceinline__ void colsum_slot(const T* __restrict__ x, int rows, int N, int c, int row, float (&acc)[Vec<T>::N]) {
+  constexpr int V = VEC ? Vec<T>::N : 1, STEP = COLSUM_CLUSTER * (256 / L);
+  for (int r = row; r < rows; r += 8 * STEP) {
+    float v[8][V];
+    if constexpr (VEC) {
+      uint4 raw[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        raw[u] = make_uint4(0, 0, 0, 0);
+        if (r + u * STEP < rows && NB_IN_BOUNDS(NB_SITE_REDUCE_INDEX, (long long)(r + u * STEP) * N + c + V - 1, (long long)rows * N))
+          raw[u] = *reinterpret_cast<const uint4*>(x + (size_t)(r + u * STEP) * N + c);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) unpack_vec<T>(raw[u], v[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u][0] = r + u * STEP < rows ? to_f<T>(x[(size_t)(r + u * STEP) * N + c]) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      acc[j] += ((v[0][j] + v[1][j]) + (v[2][j] + v[3][j])) + ((v[4][j] + v[5][j]) + (v[6][j] + v[7][j]));
+  }
+}
+template <typename T, int L>
+__global__ void __launch_bounds__(256) __cluster_dims__(1, COLSUM_CLUSTER, 1) colsum_group_kernel(const __grid_constant__ ColsumGroup g) {
+  constexpr int V = Vec<T>::N;
+  __shared__ float sh[8][L * V];
+  __shared__ float tot[L * V];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  int l = 0;
+  while (l + 1 < g.count && blockIdx.x >= g.leaf[l + 1].tile0) ++l;
+  const ColsumGroup::Leaf& t = g.leaf[l];
+  const int lane = threadIdx.x % L, slot = threadIdx.x / L, rank = blockIdx.y;
+  const int width = t.vec ? L * V : L, c0 = (int)(blockIdx.x - t.tile0) * width, c = c0 + lane * (t.vec ? V : 1);
+  float acc[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = 0.f;
+  if (c < t.N) {
+    const int row = rank * (256 / L) + slot;
+    if (t.vec) colsum_slot<T, L, true>((const T*)t.x, t.rows, t.N, c, row, acc);
+    else colsum_slot<T, L, false>((const T*)t.x, t.rows, t.N, c, row, acc);
+  }
+#pragma unroll
+  for (int o = L; o < 32; o <<= 1)                   // slots that share a warp
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  if ((threadIdx.x & 31) < L) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) sh[threadIdx.x >> 5][lane * V + j] = acc[j];
+  }
+  __syncthreads();
+  // (of a leaf without vectors, element lane * V of a row of `sh` holds column lane)
+  const int i = threadIdx.x, at = t.vec ? i : i * V;
+  if (i < width) {
+    float a[8];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) a[w] = sh[w][at];
+    tot[i] = sum8(a);
+  }
+  cluster.sync();
+  if (rank == 0 && i < width && c0 + i < t.N) {
+    float a[8];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) a[w] = cluster.map_shared_rank(tot, w)[i];
+    const float s = sum8(a);
+    if (t.out_bf16) ((bf16*)t.out)[c0 + i] = __float2bfloat16(s);
+    else ((float*)t.out)[c0 + i] = s;
+  }
+  cluster.sync();                                    // a block's shared memory is read until here
 }
 
 // ============================================================== softmax / log-softmax (last dim)
@@ -2582,6 +2672,34 @@ int nb_colsum(const void* x, void* out, float* partial, int rows, int N, int in_
   if (out_dtype) fold_slices<bf16>(partial, out, (size_t)N, np, STREAM);
   else fold_slices<float>(partial, out, (size_t)N, np, STREAM);
   return CHECK_LAUNCH();
+}
+
+// Column sums of `count` matrices of one type (host arrays of device pointers and sizes) in as few launches as their table
+// has room for; `wide`: tiles of 32 vectors of columns instead of 8. Returns the number of launches, or a negative code.
+int nb_colsum_group(const void* const* x, void* const* out, const int* rows, const int* N, const int* out_dtype, int count, int in_dtype,
+                    int wide, void* stream) {
+  const int V = in_dtype ? 8 : 4, L = wide ? 32 : 8;
+  int launches = 0;
+  for (int k = 0; k < count;) {
+    ColsumGroup g;
+    unsigned tiles = 0;
+    g.count = 0;
+    for (; k < count && g.count < COLSUM_GROUP; ++k) {
+      if (N[k] <= 0) continue;
+      const int vec = N[k] % V == 0 && (reinterpret_cast<uintptr_t>(x[k]) & 15) == 0, width = vec ? L * V : L;
+      g.leaf[g.count++] = ColsumGroup::Leaf{x[k], out[k], rows[k], N[k], tiles, vec, out_dtype[k]};
+      tiles += (N[k] + width - 1) / width;
+    }
+    if (g.count == 0) break;
+    const dim3 grid(tiles, COLSUM_CLUSTER);
+    if (in_dtype) {
+      if (wide) colsum_group_kernel<bf16, 32><<<grid, 256, 0, STREAM>>>(g); else colsum_group_kernel<bf16, 8><<<grid, 256, 0, STREAM>>>(g);
+    } else {
+      if (wide) colsum_group_kernel<float, 32><<<grid, 256, 0, STREAM>>>(g); else colsum_group_kernel<float, 8><<<grid, 256, 0, STREAM>>>(g);
+    }
+    ++launches;
+  }
+  return cudaGetLastError() == cudaSuccess ? launches : -1;
 }
 
 int nb_softmax(const void* x, void* y, int rows, int D, int log, int dtype, void* stream) {

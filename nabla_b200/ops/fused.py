@@ -232,10 +232,11 @@ class BiasGradOp(Operation):
     partial_policy = "any"
 
     def kernel(self, x):
-        if _native(x) and x.dim() == 2 and x.shape[1] % 8 == 0 and x.shape[0] > 0:
+        if _native(x) and x.dim() == 2 and x.shape[0] > 0:
             from ..native import kernels
 
-            return kernels.colsum(x)
+            if x.shape[1] % 8 == 0 or (x.shape[1] and kernels.colsum_clusters(x.shape[0], x.shape[1], x.dtype)):
+                return kernels.colsum(x)
         return x.float().sum(dim=0).to(x.dtype)
 
     def sharding_rule(self, input_shapes, output_shapes, **kw):

@@ -520,7 +520,7 @@ class CompiledFunction:
             rec.steps = _optimizer_steps_last(rec.steps, nodes)
             rec.steps = _bucket_small_all_reduces(rec.steps, nodes)
         if plan is not None:
-            rec.steps = _group_small_updates(rec.steps, nodes)
+            rec.steps = _group_bias_grads(_group_small_updates(rec.steps, nodes), nodes)
         # liveness: free an intermediate after the last step that reads it
         out_ids = {id(i) for i in rec.out_impls if i is not None}
         produced = {id(o): o for outs in rec.keep for o in outs}
@@ -1117,6 +1117,53 @@ def _group_small_updates(steps: list, nodes: list[OpNode], max_elems: int = 1 <<
             gone.update(members)
             out.append(("adamw_group", tuple(steps[si][1][0] for si in members)))
     return [st for si, st in enumerate(steps) if si not in gone] + out if gone else steps
+
+
+def _group_bias_grads(steps: list, nodes: list[OpNode], window: int = 24, max_bytes: int = 1 << 25) -> list:
+    """Bias gradients that lie close together become one step, one launch, where the last of them was: each is a launch of some
+    3 us whatever its size, and they are independent of each other. Only sums that go by clusters on their own, of
+    tensors that are small enough to be kept until then."""
+    from ..native.kernels import colsum_clusters
+    from ..ops.fused import BiasGradOp
+    from ..types import DType
+
+    reader: dict[int, int] = {}                     # impl id -> first step that reads it
+    for si, (kind, idxs) in enumerate(steps):
+        for ni in idxs:
+            for a in nodes[ni].input_impls():
+                reader.setdefault(id(a), si)
+    groups: list[list[int]] = []
+    last: dict = {}                                 # (device, dtype) -> its latest group and the bytes in it
+    for si, (kind, idxs) in enumerate(steps):
+        n = nodes[idxs[0]]
+        if kind != "op" or not isinstance(n.op, BiasGradOp):
+            continue
+        x, o = n.input_impls()[0], n.outputs()[0]
+        if o is None or x.sharding is not None or x.batch_dims or len(x._shape) != 2 or x.device.label != "gpu" \
+                or x.dtype not in (DType.bfloat16, DType.float32):
+            continue
+        rows, cols = (int(d) for d in x._shape)
+        dt = x.dtype.to_torch()
+        if not rows or not cols or colsum_clusters(rows, cols, dt) != 1:
+            continue
+        nbytes, key = rows * cols * dt.itemsize, (x.device, x.dtype)
+        g = last.get(key)
+        if g is not None and si - g[0][0] <= window and g[1] + nbytes <= max_bytes \
+                and all(reader.get(id(nodes[steps[m][1][0]].outputs()[0]), len(steps)) > si for m in g[0]):
+            g[0].append(si)
+            last[key] = (g[0], g[1] + nbytes)
+        else:
+            last[key] = ([si], nbytes)
+            groups.append(last[key][0])
+    at = {g[-1]: g for g in groups if len(g) > 1}
+    gone = {si for g in at.values() for si in g}
+    out = []
+    for si, st in enumerate(steps):
+        if si in at:
+            out.append(("bias_grads", tuple(steps[m][1][0] for m in at[si])))
+        elif si not in gone:
+            out.append(st)
+    return out
 
 
 def compile(fn: Callable | None = None, *, fullgraph: bool = False, max_cache_size: int = 64,

@@ -1049,6 +1049,44 @@ def test_column_sums_around_the_slab_counts():
             assert _rel2(kernels.colsum(x), x.double().sum(0)) < STORED[dtype]
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_column_sums_by_clusters(dtype):
+    """Rows around the slots of a cluster (64 and 256) and eight of them, columns around a tile, odd widths and bases; each alone
+    and all in one launch."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(21)
+    v = 16 // dtype.itemsize
+    xs = []
+    for rows, N, off in ((1, v, 0), (255, 8 * v, 0), (257, 8 * v + v, 0), (512, 1, 0), (2047, 10, 0), (2049, 77, 0), (513, 32 * v, 0),
+                         (100, 8 * v, 3), (4097, 1000, 0), (8191, 3, 1), (300, 2048 + v, 0)):
+        xs.append((torch.randn(rows * N + off, device="cuda").to(dtype))[off:].view(rows, N))
+    for wide in (False, True):
+        for x, s in zip(xs, kernels.colsum_group(xs, torch.float32, wide)):
+            assert _rel2(s, x.double().sum(0)) < STORED[torch.float32]
+    for x, s in zip(xs, kernels.colsum_group(xs * 4)[:len(xs)]):          # more than one launch holds
+        assert s.dtype == dtype and _rel2(s, x.double().sum(0)) < STORED[dtype]
+
+
+def test_compiled_bias_gradients_of_a_step_share_a_launch():
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    torch.manual_seed(22)
+    x, w1, b1, w2, b2, dy = (torch.randn(s, device="cuda").to(torch.bfloat16) for s in ((200, 72), (72, 136), (136,), (136, 9), (9,), (200, 9)))
+
+    def step(x, w1, b1, w2, b2, dy):
+        y, pull = nb.vjp(lambda *a: F.linear(F.linear(*a[:3], activation="relu"), *a[3:]), x, w1, b1, w2, b2, create_graph=False)
+        return (y, *pull(dy))
+
+    f = nb.compile(step)
+    got = [[t.to_torch() for t in f(*(nb.Tensor.from_torch(t) for t in (x, w1, b1, w2, b2, dy)))] for _ in range(2)]
+    assert sum("bias_grads" in line for line in f.dump_plan().splitlines()) == 1
+    plain = [t.to_torch() for t in step(*(nb.Tensor.from_torch(t) for t in (x, w1, b1, w2, b2, dy)))]
+    for a, b, c in zip(*got, plain):
+        assert torch.equal(a, b) and torch.equal(a, c)
+
+
 @pytest.mark.parametrize("rows,N", [(4096, 8), (4099, 124), (12544, 48), (50176, 32), (200704, 16), (700001, 120)])
 def test_narrow_column_sums_are_short_chains(rows, N):
     """The additions one by one: a slab's rows to the slots of a block, the slots in eight sums and in pairs, the slabs to
