@@ -16,6 +16,10 @@ CUDA bf16 tensors:
 * ``layer norm backward -> add``: the gradient that joins dx is added in the same pass (compiled replays).
 * ``matmul -> dact_mul`` (backward of linear + relu/gelu): the activation derivative is applied in
   the GEMM epilogue.
+* ``sub -> [mul with itself ->] sums over all axes -> division by a number``: the mean of a cross-entropy or a squared error, one
+  launch that also leaves the difference where the backward reads it (compiled replays).
+* ``x * y + x * y`` (the gradient of a square): one pass (compiled replays).
+* ``add(number) -> adam_hyper``: the step count and what follows from it, one launch (compiled replays).
 * compiled replays with donated optimizer state: ``matmul -> all_reduce(dp) -> adam_wstep`` becomes a
   GEMM that writes its (unreduced) weight gradient into a symmetric arena plus one kernel that sums
   the ranks' gradients while reading them and applies AdamW in place (``gemm_to_arena`` /
@@ -133,6 +137,34 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
                 if not used[j] and _is_scatter_add_into(nodes[j], o):
                     chain = [i, j]
                     kind = "scatter_zeros"
+        if chain is None and private and n.op.name == "sub":
+            idxs = _mean_of_difference(i, nodes, cons, target_ids, used, producer, private_intermediate)
+            if idxs is not None:
+                for c in idxs:
+                    used[c] = True
+                steps.append((i, ("mean_diff", tuple(idxs))))       # where the difference was made: others may read it
+                continue
+        if chain is None and private and n.op.name == "mul" and _is_plain_binary(n):
+            # x * y + x * y
+            o = sole_output(n)
+            if private_intermediate(o):
+                k = cons[id(o)][0]
+                a_ = nodes[k]
+                if not used[k] and a_.op.name == "add" and _is_plain_binary(a_):
+                    other = [x for x in a_.input_impls() if x is not o]
+                    j = producer.get(id(other[0]), -1) if len(other) == 1 else -1
+                    if j > i and not used[j] and nodes[j].op.name == "mul" and private_intermediate(other[0]) \
+                            and {id(x) for x in nodes[j].input_impls()} == {id(x) for x in n.input_impls()} and len(nodes[j].input_impls()) == 2:
+                        chain = [i, j, k]
+                        kind = "twice_product"
+        if chain is None and private and n.op.name == "add" and _is_plain_binary(n):
+            # step + 1 -> [lr, 1 - b1^t, 1 - b2^t, 1]
+            o = sole_output(n)
+            j = min(cons.get(id(o), [i])) if o is not None else i
+            if j != i and not used[j] and nodes[j].op.name == "adam_hyper" and _is_counted_step(n, o):
+                used[i] = used[j] = True
+                steps.append((i, ("next_step", (i, j))))
+                continue
         if chain is None and n.op.name == "reduce_sum" and _is_plain_sum(n) \
                 and n.kwargs["axis"] < len(n.input_impls()[0]._shape) - 1:
             # sums over neighbouring axes, one after the other (``sum(axis=(0, 1, 2))``): one reduction over
@@ -301,6 +333,68 @@ def _is_cuda_bf16_2d(n: OpNode) -> bool:
 
     return (a.device.label == "gpu" and a.dtype is DType.bfloat16 and b.dtype is DType.bfloat16
             and len(b._shape) == 2 and len(a._shape) >= 2)
+
+
+def _is_plain_binary(n: OpNode) -> bool:
+    """Two unsharded fp32 / bf16 GPU operands of the result's type."""
+    from ...types import DType
+
+    ins, outs = n.input_impls(), n.outputs()
+    o = outs[0] if len(outs) == 1 else None
+    return (len(ins) == 2 and o is not None and o.sharding is None and not o.batch_dims and o.dtype in (DType.bfloat16, DType.float32)
+            and all(x.sharding is None and not x.batch_dims and x.device.label == "gpu" and x.dtype is o.dtype and x.device == o.device
+                    for x in ins))
+
+
+def _mean_of_difference(i: int, nodes, cons, target_ids, used, producer, private_intermediate) -> list[int] | None:
+    """[sub, (mul,) reduce_sum..., div | divide_by_count] when node ``i`` begins a mean over all elements of ``a - b`` or of its
+    square, whose sums nobody else reads. The difference itself may have other readers where it is squared."""
+    n = nodes[i]
+    if not _is_plain_binary(n):
+        return None
+    a, b = n.input_impls()
+    d = n.outputs()[0]
+    numel = math.prod(int(s) for s in d._shape)
+    if tuple(a._shape) != tuple(b._shape) or not 0 < numel <= 1 << 18 or not d._shape:
+        return None
+    idxs, cur = [i], d
+    readers = cons.get(id(d), [])
+    squares = [j for j in dict.fromkeys(readers) if nodes[j].op.name == "mul" and all(x is d for x in nodes[j].input_impls())]
+    if squares:
+        if len(squares) != 1 or used[squares[0]]:
+            return None
+        idxs.append(squares[0])
+        cur = nodes[squares[0]].outputs()[0]
+    while True:
+        if not private_intermediate(cur):
+            return None
+        j = cons[id(cur)][0]
+        m = nodes[j]
+        if used[j]:
+            return None
+        if m.op.name == "reduce_sum" and _is_plain_sum(m):
+            idxs.append(j)
+            cur = m.outputs()[0]
+            if cur is None:
+                return None
+            continue
+        if len(cur._shape) or cur is d:
+            return None
+        if m.op.name == "divide_by_count" and m.outputs()[0] is not None:
+            return idxs + [j]
+        if m.op.name == "div" and _is_plain_binary(m) and m.input_impls()[0] is cur and m.input_impls()[1].literal \
+                and not m.input_impls()[1]._shape:
+            return idxs + [j]
+        return None
+
+
+def _is_counted_step(add: OpNode, o: TensorImpl) -> bool:
+    """``add`` of a number to the one fp32 element of a step count."""
+    from ...types import DType
+
+    ins = add.input_impls()
+    return (o.dtype is DType.float32 and not o._shape and not ins[0]._shape and not ins[1]._shape and ins[0] is not ins[1]
+            and any(x.literal for x in ins))
 
 
 def _is_table_gather(n: OpNode) -> bool:
@@ -624,6 +718,48 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         else:
             for n_ in group:
                 _plain(n_, keep_graph)
+        return
+    if kind == "mean_diff":
+        from ... import native
+        from ...native import kernels
+
+        sub, last = group[0], group[-1]
+        a, b = [x._buffers[0] for x in sub.input_impls()]
+        square = group[1].op.name == "mul"
+        if native.use_native(a) and native.use_native(b) and a.device == b.device and kernels.elementwise_enabled():
+            count = last.kwargs["count"] if last.op.name == "divide_by_count" else last.input_impls()[1]._buffers[0]
+            d, out = kernels.mean_diff(a, b, square, count)
+            _store(sub, [[d]], keep_graph)
+            _store(last, [[out]], keep_graph)
+        else:
+            for n_ in group:
+                _plain(n_, keep_graph)
+        return
+    if kind == "twice_product":
+        from ... import native
+        from ...native import kernels
+
+        x, y = [t._buffers[0] for t in group[0].input_impls()]
+        out = kernels.binary(x, y, "mul2") if native.use_native(x) else None
+        if out is not None:
+            _store(group[-1], [[out]], keep_graph)
+        else:
+            for n_ in group:
+                _plain(n_, keep_graph)
+        return
+    if kind == "next_step":
+        from ... import native
+        from ...native import kernels
+
+        add, hyper = group
+        x, y = [t._buffers[0] for t in add.input_impls()]
+        if native.use_native(x) and native.use_native(y) and x.device == y.device:
+            step, out = kernels.adam_hyper(x, hyper.kwargs["lr"], hyper.kwargs["beta1"], hyper.kwargs["beta2"], plus=y)
+            _store(add, [[step]], keep_graph)
+            _store(hyper, [[out]], keep_graph)
+        else:
+            _plain(add, keep_graph)
+            _plain(hyper, keep_graph)
         return
     if kind == "gather_add":
         from ... import native

@@ -25,7 +25,7 @@ if TYPE_CHECKING:
 class TensorImpl:
     __slots__ = ("_buffers", "_shape", "_dtype", "_device", "sharding", "sharding_constraint", "is_traced",
                  "requires_grad", "grad", "tangent", "cotangent", "dual", "batch_dims", "output_refs",
-                 "output_index", "_local_shapes", "_keepalive", "__weakref__")
+                 "output_index", "_local_shapes", "_keepalive", "literal", "__weakref__")
 
     def __init__(self, buffers: list[torch.Tensor] | torch.Tensor | None = None, *, shape=None, dtype: DType | None = None,
                  device: Device | None = None, sharding: "ShardingSpec | None" = None, batch_dims: int = 0,
@@ -48,6 +48,7 @@ class TensorImpl:
         self.output_index = 0
         self._local_shapes = None
         self._keepalive = None
+        self.literal = False            # a Python number that an op was given
         if buffers is not None and shape is None:
             b0 = buffers[0]
             if sharding is not None:
@@ -75,6 +76,7 @@ class TensorImpl:
         new.sharding_constraint = new.grad = new.tangent = new.cotangent = new.dual = None
         new.output_refs = new._local_shapes = new._keepalive = None
         new.output_index = 0
+        new.literal = False
         return new
 
     # ---- state

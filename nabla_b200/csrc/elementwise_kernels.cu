@@ -47,7 +47,7 @@ __device__ __forceinline__ void store_vec(T* p, const float* in) {
 }
 
 // ------------------------------------------------------------------ binary
-enum BinOp { B_ADD = 0, B_SUB, B_MUL, B_DIV, B_MAX, B_MIN, B_POW };
+enum BinOp { B_ADD = 0, B_SUB, B_MUL, B_DIV, B_MAX, B_MIN, B_POW, B_MUL2 };     // B_MUL2: a * b, rounded, and added to itself
 
 __device__ __forceinline__ float bin_apply(float a, float b, int op) {
   switch (op) {
@@ -57,6 +57,7 @@ __device__ __forceinline__ float bin_apply(float a, float b, int op) {
     case B_DIV: return a / b;
     case B_MAX: return (a != a || b != b) ? NAN : fmaxf(a, b);     // propagate NaN like the framework's oracle
     case B_MIN: return (a != a || b != b) ? NAN : fminf(a, b);
+    case B_MUL2: return 2.f * (a * b);                            // doubling a rounded product is exact
     default: return powf(a, b);
   }
 }
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(256) binary_kernel(const T* __restrict__ a, co
       }
       switch (op) {
 #define NB_CASE(OP) case OP: _Pragma("unroll") for (int j = 0; j < V; ++j) o[j] = bin_apply(x[j], y[j], OP); break;
-        NB_CASE(B_ADD) NB_CASE(B_SUB) NB_CASE(B_MUL) NB_CASE(B_DIV) NB_CASE(B_MAX) NB_CASE(B_MIN)
+        NB_CASE(B_ADD) NB_CASE(B_SUB) NB_CASE(B_MUL) NB_CASE(B_DIV) NB_CASE(B_MAX) NB_CASE(B_MIN) NB_CASE(B_MUL2)
         default: _Pragma("unroll") for (int j = 0; j < V; ++j) o[j] = bin_apply(x[j], y[j], B_POW); break;
 #undef NB_CASE
       }

@@ -33,7 +33,8 @@ def _L():
             "nb_lse_pick_bwd": [c_vp] * 6 + [c_int, c_int, c_int, c_vp],
             "nb_adamw": [c_vp] * 7 + [c_ll] + [c_f] * 8 + [c_vp, c_int, c_int, c_vp],
             "nb_adamw_group": [c_vp] * 8 + [c_int] + [c_f] * 8 + [c_vp, c_int, c_int, c_vp],
-            "nb_adam_hyper": [c_vp, c_vp, c_f, ctypes.c_double, ctypes.c_double, c_vp],
+            "nb_adam_hyper": [c_vp] * 4 + [c_f, ctypes.c_double, ctypes.c_double, c_vp],
+            "nb_mean_diff": [c_vp] * 4 + [c_ll, c_int, c_vp, c_f, c_int, c_vp],
             "nb_sgd": [c_vp] * 5 + [c_ll] + [c_f] * 4 + [c_int, c_int, c_vp],
             "nb_embedding_gather": [c_vp] * 4 + [c_int] * 5 + [c_vp],
             "nb_embedding_scatter_add": [c_vp] * 5 + [c_int] * 4 + [c_vp],
@@ -274,11 +275,13 @@ def adamw_group(leaves: list, *, lr, b1, b2, eps, wd, step: int | None = None, h
     return outs
 
 
-def adam_hyper(step: torch.Tensor, lr: float, b1: float, b2: float) -> torch.Tensor:
-    """[lr, 1 - b1^t, 1 - b2^t, 1] for the fp32 step count ``t`` on the device (one element)."""
+def adam_hyper(step: torch.Tensor, lr: float, b1: float, b2: float, plus: torch.Tensor | None = None):
+    """[lr, 1 - b1^t, 1 - b2^t, 1] for the fp32 step count ``t`` on the device (one element). With ``plus`` (another such
+    element) t is their sum, and (sum, vector) is returned."""
     out = torch.empty(4, dtype=torch.float32, device=step.device)
-    _ok(_L().nb_adam_hyper(ptr(step), ptr(out), float(lr), float(b1), float(b2), stream_ptr()), "adam_hyper")
-    return out
+    total = torch.empty((), dtype=torch.float32, device=step.device) if plus is not None else None
+    _ok(_L().nb_adam_hyper(ptr(step), ptr(plus), ptr(total), ptr(out), float(lr), float(b1), float(b2), stream_ptr()), "adam_hyper")
+    return out if plus is None else (total, out)
 
 
 def sgd(p, g, buf, *, lr, momentum=0.0, wd=0.0, grad_scale=1.0):
@@ -652,6 +655,18 @@ def sgemm(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None) ->
     return out
 
 
+def mean_diff(a: torch.Tensor, b: torch.Tensor, square: bool, count) -> tuple[torch.Tensor, torch.Tensor]:
+    """(d, m): d = a - b, and m the sum of d (or of d * d) over all elements, divided by ``count`` (a number, or an element of a's type
+    on the device), of two fp32 / bf16 tensors of one shape and type. The sum is kept in fp32 and rounded once."""
+    a, b = a.contiguous(), b.contiguous()
+    d = torch.empty_like(a)
+    out = torch.empty((), dtype=a.dtype, device=a.device)
+    on_device = isinstance(count, torch.Tensor)
+    _ok(_L().nb_mean_diff(ptr(a), ptr(b), ptr(d), ptr(out), a.numel(), int(square), ptr(count if on_device else None),
+                          0.0 if on_device else float(max(int(count), 1)), _dt(a), stream_ptr()), "mean_diff")
+    return d, out
+
+
 def sum_slices(part: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     """Sum a contiguous fp32 tensor over its leading dim (the partial products of a split-K GEMM)."""
     s_ = part.shape[0]
@@ -661,7 +676,7 @@ def sum_slices(part: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
 
 
 # ---------------------------------------------------------------- pointwise / reduction families
-BINARY_OPS = {"add": 0, "sub": 1, "mul": 2, "div": 3, "maximum": 4, "minimum": 5, "pow": 6}
+BINARY_OPS = {"add": 0, "sub": 1, "mul": 2, "div": 3, "maximum": 4, "minimum": 5, "pow": 6, "mul2": 7}
 UNARY_OPS = {"neg": 0, "abs": 1, "exp": 2, "log": 3, "sqrt": 4, "rsqrt": 5, "tanh": 6, "sigmoid": 7, "sin": 8, "cos": 9,
              "erf": 10, "log1p": 11, "floor": 12, "trunc": 13, "round": 14, "square": 15, "reciprocal": 16}
 REDUCE_OPS = {"sum": 0, "max": 1, "min": 2, "mean": 3, "argmax": 4, "argmin": 5}

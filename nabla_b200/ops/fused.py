@@ -546,7 +546,7 @@ class LsePickOp(_Fused):
     shards' (lse, picked) with max / sum reductions on small per-row vectors."""
 
     def kernel(self, logits, targets, *, vocab_offset: int = 0):
-        t = targets.long() - vocab_offset
+        t = targets.long() - vocab_offset if vocab_offset else targets.long()
         if logits.device.type != "meta" and _native(logits) and logits.numel():
             from ..native import kernels
 
@@ -608,7 +608,7 @@ class LsePickOp(_Fused):
 
 class LsePickBwdOp(Operation):
     def kernel(self, logits, targets, lse, g_lse, g_pick, *, vocab_offset: int = 0):
-        t = targets.long() - vocab_offset
+        t = targets.long() - vocab_offset if vocab_offset else targets.long()
         if logits.device.type != "meta" and _native(logits) and logits.numel():
             from ..native import kernels
 

@@ -185,6 +185,8 @@ class _Recorded:
         self.copy_in = None                         # (CopyBatch) one-launch copies into the graph's inputs / out of its results
         self.copy_out = None
         self.side_steps: set[int] = set()           # optimizer updates that run on a side stream, under the backward
+        self.constants: list[TensorImpl] = []       # values that follow from numbers alone, made with the plan
+        self.constant_stream = None                 # the stream they were made on
         self.host_sync = False                      # holds a node that reads a device value on the host
         self.sizes: dict[str, int] = {}             # value of every named dynamic dimension in this recording
 
@@ -521,6 +523,7 @@ class CompiledFunction:
             rec.steps = _bucket_small_all_reduces(rec.steps, nodes)
         if plan is not None:
             rec.steps = _group_bias_grads(_group_small_updates(rec.steps, nodes), nodes)
+            rec.steps = _make_constants(rec)
         # liveness: free an intermediate after the last step that reads it
         out_ids = {id(i) for i in rec.out_impls if i is not None}
         produced = {id(o): o for outs in rec.keep for o in outs}
@@ -544,7 +547,7 @@ class CompiledFunction:
         rec.free_after = [[] for _ in rec.steps]
         side_inputs = {id(a) for si in rec.side_steps for ni in rec.steps[si][1] for a in nodes[ni].input_impls()}
         for k, si in last_use.items():
-            if k not in out_ids:
+            if k not in out_ids and produced[k]._buffers is None:
                 # what a side-stream step reads stays allocated until the streams join (end of the schedule)
                 rec.free_after[len(rec.steps) - 1 if k in side_inputs else si].append(produced[k])
         self._stats.graph_nodes = len(nodes)
@@ -688,6 +691,9 @@ class CompiledFunction:
         if self.profile_ops and not torch.cuda.is_current_stream_capturing():
             return self._run_profiled(rec)
         nvtx = _NVTX and torch.cuda.is_available()
+        if rec.constants and torch.cuda.current_stream() != rec.constant_stream and not torch.cuda.is_current_stream_capturing():
+            for o in rec.constants:                 # they may go with the recording while this stream still reads them
+                o._buffers[0].record_stream(torch.cuda.current_stream())
         side = cur = None
         # Measured on the 24-layer benchmark step (1 GPU, power-capped at 1 kW): 155.8 ms with the updates
         # on the side stream, 155.2 ms without: the step is energy bound, so hiding the AdamW kernels
@@ -1117,6 +1123,64 @@ def _group_small_updates(steps: list, nodes: list[OpNode], max_elems: int = 1 <<
             gone.update(members)
             out.append(("adamw_group", tuple(steps[si][1][0] for si in members)))
     return [st for si, st in enumerate(steps) if si not in gone] + out if gone else steps
+
+
+_FROM_NUMBERS = {"full", "add", "sub", "mul", "div", "neg", "divide_by_count", "unsqueeze", "squeeze", "reshape", "broadcast_to", "cast"}
+
+
+def _make_constants(rec: "_Recorded", max_elems: int = 1 << 16) -> list:
+    """Steps that compute from numbers of the program alone (the 1 / n of a mean's gradient, spread over its rows) run once, here, and
+    leave the schedule: at 1 to 2 us a launch they were four of the 41 launches of a classifier's training step. Only small
+    unsharded GPU values that no result of the function can share its memory with: every reader is another such step, an op that writes
+    a new tensor, or a fused step. Returns the steps that stay."""
+    from ..ops.base import BinaryOperation
+
+    nodes = rec.nodes
+    out_ids = {id(i) for i in rec.out_impls if i is not None}
+    step_of = {ni: si for si, (kind, idxs) in enumerate(rec.steps) for ni in idxs}
+    readers: dict[int, list[int]] = {}
+    for ni, n in enumerate(nodes):
+        for a in n.input_impls():
+            readers.setdefault(id(a), []).append(ni)
+    made: dict[int, int] = {}                       # impl id -> its node
+    for si, (kind, idxs) in enumerate(rec.steps):
+        n = nodes[idxs[0]]
+        if kind != "op" or n.op.name not in _FROM_NUMBERS or (not n.input_impls() and n.op.name != "full"):
+            continue
+        outs = n.outputs()
+        if len(outs) != 1 or outs[0] is None or id(outs[0]) in out_ids or outs[0].sharding is not None or outs[0].batch_dims \
+                or outs[0].device.label != "gpu":
+            continue
+        numel = 1
+        for d in outs[0]._shape:
+            numel *= int(d)
+        if numel <= max_elems and all(id(a) in made or (a.literal and a.sharding is None) for a in n.input_impls()):
+            made[id(outs[0])] = idxs[0]
+    while True:                                     # until every reader of what is left is as above
+        bad = [k for k, ni in made.items() if not all(
+            (id(nodes[r].outputs()[0]) in made if nodes[r].outputs()[0] is not None else False) or rec.steps[step_of[r]][0] != "op"
+            or isinstance(nodes[r].op, BinaryOperation) or nodes[r].op.name in ("lse_pick_bwd", "matmul") for r in readers.get(k, []))]
+        if not bad:
+            break
+        for k in bad:
+            del made[k]
+        for k in [k for k, ni in made.items() if not all(id(a) in made or a.literal for a in nodes[ni].input_impls())]:
+            made.pop(k, None)
+    if not made or torch.cuda.is_current_stream_capturing():       # (a capture of the caller's: nothing may be waited for)
+        return rec.steps
+    gone = set(made.values())
+    wanted = {k for k in made if any(r not in gone for r in readers.get(k, []))}
+    kept = []
+    for ni in sorted(gone):
+        o = nodes[ni].outputs()[0]
+        o._buffers = [b.contiguous() for b in nodes[ni].op.execute(nodes[ni])[0]]
+        kept.append(o)
+    torch.cuda.current_stream().synchronize()       # a later call may be on another stream
+    for o in kept:
+        if id(o) in wanted:
+            rec.constants.append(o)
+    rec.constant_stream = torch.cuda.current_stream()
+    return [st for st in rec.steps if not (st[0] == "op" and st[1][0] in gone)]
 
 
 def _group_bias_grads(steps: list, nodes: list[OpNode], window: int = 24, max_bytes: int = 1 << 25) -> list:

@@ -956,6 +956,14 @@ def test_gemm_operands_of_one_row_or_column():
 
 
 # ---------------------------------------------------------------- AdamW bias corrections
+def test_adam_hyper_counts_its_step():
+    from nabla_b200.native import kernels
+
+    for t in (0.0, 1.0, 999.0):
+        s, h = kernels.adam_hyper(torch.tensor(t, device="cuda"), 1e-3, 0.9, 0.999, plus=torch.tensor(1.0, device="cuda"))
+        assert s.item() == t + 1 and torch.equal(h, kernels.adam_hyper(s, 1e-3, 0.9, 0.999))
+
+
 def test_adam_hyper():
     from nabla_b200.native import kernels
 
@@ -1036,6 +1044,57 @@ def test_compiled_step_groups_its_small_updates(donate):
             ref[k] = ref[k] - 1e-2 * ((m[k] / (1 - 0.9 ** t)) / ((v2[k] / (1 - 0.999 ** t)).sqrt() + 1e-8) + 0.1 * ref[k])
             assert _rel2(new[k].to_torch(), ref[k]) < t * STORED[torch.float32]      # a rounding of p, m and v per step
     assert sum("adamw_group" in line for line in str(f.dump_plan()).splitlines()) == 1
+
+
+# ---------------------------------------------------------------- means of a difference
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [1, 31, 1025, 4096, 4097, 70001, 1 << 18])
+def test_mean_of_a_difference_and_of_its_square(dtype, n):
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(23)
+    a, b = (torch.randn(n, device="cuda").to(dtype) for _ in range(2))
+    for square in (False, True):
+        for count in (n, torch.tensor(float(n), device="cuda", dtype=dtype)):
+            d, m = kernels.mean_diff(a, b, square, count)
+            assert torch.equal(d, a - b)
+            terms = d.double() ** 2 if square else d.double()
+            c = float(count)
+            # fp32: the additions of a thread, a warp, a block and a cluster, each rounded to the sum of magnitudes at most
+            bound = (n / 1024 / 8 + 20) * 2.0 ** -24 * terms.abs().sum() / c
+            assert abs(m.double() - terms.sum() / c) <= bound + abs(terms.sum() / c) * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22)
+    x = torch.tensor([1.0, float("nan"), 3.0], device="cuda").to(dtype)
+    assert kernels.mean_diff(x, torch.zeros_like(x), True, 3)[1].isnan()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_compiled_losses_in_one_launch(dtype):
+    """Squared error and cross-entropy with their gradients: compiled against plain calls, twice, and what the plan made of them."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    torch.manual_seed(24)
+    x, y = torch.randn(33, 40, device="cuda").to(dtype), torch.randn(33, 40, device="cuda").to(dtype)
+    t = torch.randint(0, 40, (33,), device="cuda")
+    wrap = nb.Tensor.from_torch
+    for loss, other, steps in ((F.mse_loss, y, ("mean_diff", "twice_product")), (F.cross_entropy_loss, t, ("mean_diff",))):
+        f = nb.compile(lambda a, b, loss=loss: nb.value_and_grad(loss, create_graph=False)(a, b))
+        for k in range(2):
+            arg = (x * (k + 1)).contiguous()
+            v, g = f(wrap(arg), wrap(other))
+            p = arg.double().requires_grad_(True)
+            ref = ((p - other.double()) ** 2).mean() if loss is F.mse_loss else TF.cross_entropy(p, other)
+            ref.backward()
+            assert _rel2(v.to_torch(), ref.detach()) < STORED[dtype] and _rel2(g.to_torch(), p.grad) < 3 * STORED[dtype]
+        plan = f.dump_plan()
+        assert all(sum(s in line for line in plan.splitlines()) == 1 for s in steps)
+        assert " full" not in plan and "broadcast_to" not in plan              # made with the plan
+    # a result that would be the constant itself is made on each call
+    f = nb.compile(lambda a: (nb.broadcast_to(nb.reshape(nb.full((), 2.0, device=a.device), (1,)), (4,)), a + 1.0))
+    for _ in range(2):
+        c, _ = f(wrap(x))
+        assert c.to_torch().tolist() == [2.0] * 4
+        c.to_torch().zero_() if c.to_torch().is_contiguous() else None
 
 
 # ---------------------------------------------------------------- column sums
