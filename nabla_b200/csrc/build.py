@@ -2,8 +2,9 @@
 
 Each `.cu` / `.cpp` translation unit listed in ``TARGETS`` becomes one shared library in
 ``nabla_b200/lib``. The libraries export plain C symbols and are loaded with ctypes
-(`nabla_b200.native`), so there is no dependency on the torch C++ headers and a full rebuild
-takes seconds. nvcc cross-compiles without a GPU present.
+(`nabla_b200.native`), so they do not depend on the torch C++ headers and rebuild in seconds;
+``libnb_replay.so`` alone is a Python extension on torch's C++ interface. nvcc cross-compiles
+without a GPU present.
 
 ``build_all(debug=True)`` (``python -m nabla_b200.csrc.build --debug``) compiles the same sources
 with ``-DNB_DEBUG_CHECKS`` into ``nabla_b200/lib/debug``: every data- or geometry-derived global,
@@ -36,7 +37,19 @@ TARGETS: dict[str, tuple[list[str], list[str]]] = {
     "libnb_comm.so": (["peer_collectives.cu"], []),
     "libnb_runtime.so": (["plan_runtime.cpp"], []),
     "libnb_noalloc.so": (["no_alloc_entry.cu"], []),
+    "libnb_replay.so": (["replay.cpp"], ["torch"]),
 }
+
+
+def _torch_flags() -> list[str]:
+    import sysconfig
+
+    import torch
+
+    base = Path(torch.__file__).resolve().parent
+    inc = [base / "include", base / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"]]
+    return [*(f"-I{p}" for p in inc), f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-L{base / 'lib'}", "-lc10", "-lc10_cuda",
+            "-ltorch_cpu", "-ltorch_python", "-ltorch", f"-DTORCH_OF_BUILD={torch.__version__.replace('+', '_')}"]
 
 
 def _nvcc() -> str:
@@ -69,6 +82,8 @@ def build_all(force: bool = False, verbose: bool = False, debug: bool = False) -
         stamp = lib_dir / (name + ".sha")
         is_cuda = any(p.suffix == ".cu" for p in paths)
         flags = (NVCC_FLAGS if is_cuda else ["-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC"]) + extra
+        if "torch" in flags:
+            flags = [f for f in flags if f != "torch"] + _torch_flags()
         if debug:
             flags = flags + ["-DNB_DEBUG_CHECKS"]
         dig = _digest(paths, flags)

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from pathlib import Path
 
 import torch
@@ -34,6 +35,19 @@ def lib_path(name: str) -> Path:
 
 def available(name: str) -> bool:
     return lib_path(name).exists()
+
+
+_observer = threading.local()
+
+
+def set_recorder(r) -> None:
+    """While ``r`` is set, this thread's calls of launch functions go through ``r.library`` / ``r.function``
+    (``transforms/tape.py``)."""
+    _observer.recorder = r
+
+
+def recorder():
+    return getattr(_observer, "recorder", None)
 
 
 def load(name: str) -> ctypes.CDLL:

@@ -44,6 +44,13 @@ def _lib():
     return _fwd
 
 
+def _launcher(name: str, fn):
+    from . import recorder
+
+    r = recorder()
+    return fn if r is None else r.function(name, fn)
+
+
 def _ok_view(t: torch.Tensor) -> bool:
     if t.dim() != 4:
         return False
@@ -119,7 +126,7 @@ def sdpa_fwd(q, k, v, *, causal: bool, scale: float, mask=None):
     part = torch.empty(ns * B * H * Sq * (D + 1), dtype=torch.float32, device=q.device) if ns > 1 else None
     p_o = 0 if part is None else part.data_ptr()
     p_lse = 0 if part is None else p_o + ns * B * H * Sq * D * 4
-    rc = _lib()(ptr(q), ptr(k), ptr(v), ptr(o_mem), ptr(lse), B, H, Sq, Skv, D,
+    rc = _launcher("nb_attn_fwd", _lib())(ptr(q), ptr(k), ptr(v), ptr(o_mem), ptr(lse), B, H, Sq, Skv, D,
               *q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *o.stride()[:3],
               float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()), m_sb, m_sh, m_sq, ns, c_vp(p_o), c_vp(p_lse),
               ptr(st), stream_ptr())
@@ -153,7 +160,7 @@ def sdpa_bwd(do, q, k, v, o, lse, *, causal: bool, scale: float, out=None, mask=
     strides = []
     for t in (q, k, v, do, o, dq, dk, dv):
         strides += t.stride()[:3]
-    rc = _bwd(*args, B, H, Sq, Skv, D, *strides, float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()),
+    rc = _launcher("nb_attn_bwd", _bwd)(*args, B, H, Sq, Skv, D, *strides, float(scale), int(causal), c_vp(0 if m is None else m.data_ptr()),
               m_sb, m_sh, m_sq, ptr(st), stream_ptr())
     if rc != 0:
         raise RuntimeError(f"nb_attn_bwd failed with code {rc}")

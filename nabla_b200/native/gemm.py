@@ -37,7 +37,10 @@ def _get():
         if os.environ.get("NABLA_B200_GEMM_PAIR", "1") != "0" and torch.cuda.is_available() \
                 and not torch.cuda.is_current_stream_capturing():
             set_pair_mode(True)
-    return _fn
+    from . import recorder
+
+    r = recorder()
+    return _fn if r is None else r.function("nb_gemm_bf16", _fn)
 
 
 def pair_alloc_probe() -> tuple[int, int]:

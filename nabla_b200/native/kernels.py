@@ -10,7 +10,7 @@ import os
 
 import torch
 
-from . import load, ptr, stream_ptr
+from . import load, ptr, recorder, stream_ptr
 
 _lib = None
 launch_count = 0
@@ -75,7 +75,8 @@ def _L():
         # kernels, for comparisons (no row width needs them)
         lib.nb_layernorm_bwd_two_kernels(1 if os.environ.get("NABLA_B200_LN_BWD", "fused") == "two_kernels" else 0)
         _lib = lib
-    return _lib
+    r = recorder()
+    return _lib if r is None else r.library(_lib)
 
 
 def has(name: str) -> bool:
@@ -386,6 +387,7 @@ class CopyBatch:
         self.plain = [use_native(t) and t.device.index == dev and _is_dense(t) for t in fixed]
         self.storages = {t.untyped_storage().data_ptr() for t in fixed} if shared else None
         self.all_sizes = (c_ull * n)(*self.size) if all(self.plain) else None
+        self.launches = -(-sum(1 for s in self.size if s) // 128)          # of a call that copies all of them
 
     def fresh(self) -> list[torch.Tensor]:
         """New tensors like the fixed ones with their contents: what was just allocated for the purpose needs none of the

@@ -49,6 +49,7 @@ from ..core.graph.engine import GRAPH, _STATS, store_outputs
 from ..core.graph.tracing import OpNode, topo_nodes
 from ..core.tensor.api import Tensor
 from ..core.tensor.impl import TensorImpl
+from . import tape
 
 
 import os as _os
@@ -187,6 +188,9 @@ class _Recorded:
         self.side_steps: set[int] = set()           # optimizer updates that run on a side stream, under the backward
         self.constants: list[TensorImpl] = []       # values that follow from numbers alone, made with the plan
         self.constant_stream = None                 # the stream they were made on
+        self.tape = None                            # of later calls without Python (transforms/tape.py); False: none
+        self.tape_counts: tuple = ()                # launches of a taped call: GEMM, fused kernels, attention
+        self.tape_tries = 0
         self.host_sync = False                      # holds a node that reads a device value on the host
         self.sizes: dict[str, int] = {}             # value of every named dynamic dimension in this recording
 
@@ -246,6 +250,8 @@ class CompiledFunction:
         self.op_profile: dict[str, list] = {}
         self._cache: "OrderedDict[Any, dict[Any, _Recorded]]" = OrderedDict()
         self._stats = CompilationStats()
+        self.tape_refused = None        # why the most recent recording of a call was not kept
+        self._taped = None              # (tape, recording, whether CUDA graphs were on) of the most recent call
         self._latest = None             # (structure, signatures, recording, deterministic) of the most recent call
         self.__name__ = getattr(fn, "__name__", "compiled")
         self.__doc__ = getattr(fn, "__doc__", None)
@@ -256,7 +262,7 @@ class CompiledFunction:
 
     def clear_cache(self) -> None:
         self._cache.clear()
-        self._latest = None
+        self._latest = self._taped = None
 
     def release(self) -> None:
         """Drop every recorded schedule together with its CUDA graphs and the buffers they own.
@@ -266,7 +272,7 @@ class CompiledFunction:
             for rec in entry.values():
                 if not isinstance(rec, _Recorded):
                     continue
-                rec.cuda_graph = None
+                rec.cuda_graph = rec.tape = None
                 rec.static_inputs = rec.static_outputs = rec.out_cached = rec.copy_in = rec.copy_out = None
                 for ph in rec.placeholders:
                     ph._buffers = None
@@ -274,7 +280,7 @@ class CompiledFunction:
                     for o in outs:
                         o._buffers = None
         self._cache.clear()
-        self._latest = None
+        self._latest = self._taped = None
 
     def dump_plan(self, file=None) -> str:
         """Text listing of every recorded schedule: one line per step with its kind (``op`` or
@@ -386,7 +392,28 @@ class CompiledFunction:
                 return None
         return leaves
 
+    def _call_taped(self, taped: tuple, args: tuple):
+        """The call without Python in between, or NotImplemented."""
+        handle, rec, graphs = taped
+        if self.profile_ops or graphs is not self.use_cuda_graph or rec.tape is not handle:
+            return NotImplemented
+        t0 = time.perf_counter()
+        out = tape.module().call(handle, args, config.is_deterministic())
+        if out is not NotImplemented:
+            for module, n in zip(_counted_modules(), rec.tape_counts):
+                module.launch_count += n
+            if rec.cuda_graph is None:
+                _STATS["nodes_executed"] += len(rec.nodes)
+            self._stats.hits += 1
+            self._stats.replay_time_s += time.perf_counter() - t0
+        return out
+
     def __call__(self, *args, **kwargs):
+        taped = self._taped             # read once: another thread may replace it
+        if taped is not None and not kwargs:
+            out = self._call_taped(taped, args)
+            if out is not NotImplemented:
+                return out
         args = tuple(_normalize_step_scalars(a) for a in args)
         kwargs = {k: _normalize_step_scalars(v) for k, v in kwargs.items()}
         latest = self._latest           # read once: another thread may replace it
@@ -395,9 +422,10 @@ class CompiledFunction:
             if leaves is not None:
                 self._stats.hits += 1              # the entry is the most recently used one already
                 t0 = time.perf_counter()
-                out = self._replay(latest[2], leaves)
+                out = self._replay(latest[2], leaves, latest[0])
                 self._stats.replay_time_s += time.perf_counter() - t0
                 return out
+        self._taped = None
         self._latest = None
         key, conc, leaves, td = self._keys(args, kwargs)
         pending = [t for t in leaves if isinstance(t, Tensor) and not t._impl.is_realized]
@@ -441,9 +469,10 @@ class CompiledFunction:
             self._stats.compile_time_s += time.perf_counter() - t0
             return result
         t0 = time.perf_counter()
-        out = self._replay(rec, [l for l in leaves if isinstance(l, Tensor)])
+        plain = not kwargs and self.max_cache_size > 0 and all(type(l) is Tensor and l._impl.sharding is None for l in leaves)
+        out = self._replay(rec, [l for l in leaves if isinstance(l, Tensor)], td[0] if plain else None)
         self._stats.replay_time_s += time.perf_counter() - t0
-        if not kwargs and self.max_cache_size > 0 and all(type(l) is Tensor and l._impl.sharding is None for l in leaves):
+        if plain:
             self._latest = (td[0], conc, rec, config.is_deterministic())
         return out
 
@@ -790,14 +819,30 @@ class CompiledFunction:
                 impl._buffers = None
         return pytree.tree_unflatten(rec.out_treedef, outs)
 
-    def _replay(self, rec: _Recorded, tensors: list[Tensor]) -> Any:
+    def _replay(self, rec: _Recorded, tensors: list[Tensor], tds: tuple | None = None) -> Any:
+        """``tds``: the arguments' structures, where nothing but tensors is among them."""
         if self.use_cuda_graph and not rec.host_sync and tensors and tensors[0]._impl.device.label == "gpu":
-            return self._replay_cuda_graph(rec, tensors)
+            out = self._replay_cuda_graph(rec, tensors)
+            if rec.tape is None and rec.cuda_graph is not None and tds is not None and rec.copy_out is not None:
+                rec.tape = tape.graph_call(rec, tensors, tds) or False
+                rec.tape_counts = (0, rec.copy_in.launches + rec.copy_out.launches, 0) if rec.tape else ()
+            self._taped = (rec.tape, rec, True) if rec.tape and tds is not None else None
+            return out
         for ph, t in zip(rec.placeholders, tensors):
             ph._buffers = t._impl._buffers
         try:
-            self._run(rec)
-            return self._collect(rec)
+            if rec.tape is None and tds is not None and not self.profile_ops and not _NVTX and tape.can_record(rec):
+                before = [m.launch_count for m in _counted_modules()]
+                out, rec.tape, self.tape_refused = tape.record(rec, tensors, tds, lambda: self._run(rec), lambda: self._collect(rec))
+                rec.tape_counts = tuple(m.launch_count - b for m, b in zip(_counted_modules(), before))
+                rec.tape_tries += 1
+                if rec.tape is None and rec.tape_tries >= 2:     # arguments that share memory may be told apart on another call
+                    rec.tape = False
+            else:
+                self._run(rec)
+                out = self._collect(rec)
+            self._taped = (rec.tape, rec, False) if rec.tape and tds is not None else None
+            return out
         finally:
             for ph in rec.placeholders:
                 ph._buffers = None
@@ -827,6 +872,7 @@ class CompiledFunction:
                 for ph in rec.placeholders:
                     ph._buffers = None
                 return self._replay(rec, tensors)
+            rec.tape = None
             rec.cuda_graph = g
             self._stats.cuda_graphs += 1
             self._stats.launches_per_graph = total_launches() - n0
@@ -867,6 +913,12 @@ class CompiledFunction:
                 res = [b if b.data_ptr() in rec.static_ptrs else next(taken) for b in bufs] if rec.static_ptrs else [next(taken) for _ in bufs]
                 outs.append(Tensor(impl=TensorImpl.result_like(impl, res)))
         return pytree.tree_unflatten(rec.out_treedef, outs)
+
+
+def _counted_modules() -> tuple:
+    from ..native import attention, gemm, kernels
+
+    return gemm, kernels, attention
 
 
 _OPT_STREAMS: dict = {}

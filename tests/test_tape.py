@@ -1,0 +1,186 @@
+"""Compiled calls that were written down (``transforms/tape.py``) against the same calls run by Python. Needs a B200."""
+import threading
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+def _wrap(t):
+    import nabla_b200 as nb
+
+    return nb.Tensor.from_torch(t)
+
+
+def _leaves(out):
+    from nabla_b200.core.common import pytree
+
+    return [x.to_torch() if hasattr(x, "to_torch") else torch.tensor(x) for x in pytree.tree_leaves(out)]
+
+
+def _taped(f):
+    return f._taped is not None and bool(f._taped[0])
+
+
+def _functions():
+    """(function, inputs of a seed): one per family of launch functions."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    def g(seed):
+        return torch.Generator("cuda").manual_seed(seed)
+
+    def r(s, *shape, dtype=BF16, std=1.0):
+        return (torch.randn(shape, generator=g(s + sum(shape)), device="cuda") * std).to(dtype)
+
+    def grads(f, primals, cot):
+        y, pull = nb.vjp(f, *primals, create_graph=False)
+        return (y, *pull(cot))
+
+    def ids(s, *shape, high=50):
+        return torch.randint(0, high, shape, generator=g(s), device="cuda")
+
+    return {
+        "norm": (lambda x, a, b, dy: grads(lambda *t: F.layer_norm(*t), (x, a, b), dy),
+                 lambda s: [r(s, 70, 256), r(s, 256), r(s + 1, 256), r(s + 2, 70, 256)]),
+        "mlp": (lambda x, w, b, v, dy: {"y": grads(lambda *t: F.linear(F.linear(t[0], t[1], t[2], activation="gelu"), t[3]), (x, w, b, v), dy), "n": [None, 3]},
+                lambda s: [r(s, 100, 64), r(s, 64, 128, std=0.1), r(s, 128), r(s, 128, 64, std=0.1), r(s + 1, 100, 64)]),
+        "attention": (lambda q, k, v, m, do: grads(lambda *t: F.scaled_dot_product_attention(*t, attn_mask=m), (q, k, v), do),
+                      lambda s: [r(s, 2, 4, 130, 64), r(s + 1, 2, 4, 130, 64), r(s + 2, 2, 4, 130, 64), r(s, 2, 1, 1, 130, dtype=F32), r(s + 3, 2, 4, 130, 64)]),
+        "decode": (lambda q, k, v: F.scaled_dot_product_attention(q, k, v, is_causal=True), lambda s: [r(s, 2, 4, 1, 128), r(s, 2, 4, 700, 128), r(s + 1, 2, 4, 700, 128)]),
+        "head": (lambda x, w, t: nb.value_and_grad(lambda x, w: F.cross_entropy_loss(F.linear(x, w), t), argnums=(0, 1), create_graph=False)(x, w),
+                 lambda s: [r(s, 60, 64), r(s, 64, 208, std=0.1), ids(s, 60, high=208)]),
+        "embedding": (lambda t, p, i, dy: grads(lambda a, b: F.embedding(i, a) + b, (t, p), dy),
+                      lambda s: [r(s, 50, 64), r(s, 9, 64), ids(s, 3, 9), r(s, 3, 9, 64)]),
+        "pointwise": (lambda a, b: [nb.exp(a) * b + a, {"s": nb.reduce_sum(a * b, axis=0)}], lambda s: [r(s, 33, 40, dtype=F32), r(s + 1, 33, 40, dtype=F32)]),
+    }
+
+
+@pytest.mark.parametrize("name", ["norm", "mlp", "attention", "decode", "head", "embedding", "pointwise"])
+@pytest.mark.parametrize("graph", [False, True])
+def test_taped_calls_give_what_python_gives(name, graph, monkeypatch):
+    """New inputs and new addresses on every call, results kept: bit for bit but for sums by atomics."""
+    import nabla_b200 as nb
+
+    fn, inputs = _functions()[name]
+    f = nb.compile(fn, cuda_graph=graph)
+    monkeypatch.setenv("NABLA_B200_TAPE", "0")
+    plain = nb.compile(fn, cuda_graph=graph)
+    want = [_leaves(plain(*map(_wrap, inputs(s)))) for s in range(6)]
+    assert not _taped(plain)
+    monkeypatch.delenv("NABLA_B200_TAPE")
+    keep = []
+    for s in range(6):
+        args = inputs(s)
+        out = f(*map(_wrap, args))
+        keep.append((args, out))
+        assert s < 1 or _taped(f), f.tape_refused
+    for (_, out), w in zip(keep, want):
+        got = _leaves(out)
+        assert len(got) == len(w)
+        for a, b in zip(got, w):
+            assert a.shape == b.shape and a.dtype == b.dtype and a.stride() == b.stride()
+            assert torch.equal(a, b) or (name == "embedding" and (a.float() - b.float()).norm() < 4e-3 * b.float().norm())
+    assert f.stats.hits == 5
+
+
+def test_calls_that_are_not_the_one_that_was_written_down(monkeypatch):
+    """Other strides, alignments, shapes, types, structures, shared memory and switches go another way and are right."""
+    import nabla_b200 as nb
+
+    f = nb.compile(lambda d: d["a"] * d["b"][0] + nb.reduce_sum(d["a"], axis=0))
+    x, y = torch.randn(32, 64, device="cuda"), torch.randn(32, 64, device="cuda")
+
+    def check(a, b, container=list):
+        out = f({"a": _wrap(a), "b": container([_wrap(b)])}).to_torch()
+        assert torch.allclose(out, a * b + a.sum(0), atol=1e-4), f.tape_refused
+
+    for _ in range(3):
+        check(x, y)
+    assert _taped(f)
+    check(x, x)                                       # one tensor twice
+    check(x.t().contiguous().t(), y)                  # columns first
+    off = torch.randn(32 * 64 + 1, device="cuda")[1:].view(32, 64)
+    check(off, y)                                     # on a 4-byte boundary
+    check(x, y, tuple)
+    check(x[:16].contiguous(), y[:16].contiguous())
+    for _ in range(3):
+        check(x, y)
+    assert _taped(f)
+    out = f({"a": _wrap(x.to(BF16)), "b": [_wrap(y.to(BF16))]}).to_torch()
+    assert out.dtype == BF16
+    for _ in range(2):
+        check(x, y)
+    monkeypatch.setenv("NABLA_B200_DISABLE_NATIVE", "1")
+    check(x, y)
+    monkeypatch.delenv("NABLA_B200_DISABLE_NATIVE")
+    with pytest.raises(Exception):
+        f({"a": _wrap(x)})
+    check(x, y)
+
+
+def test_arguments_that_share_memory_are_not_written_down():
+    """Written down with both arguments in one place, a call could not tell them apart later."""
+    import nabla_b200 as nb
+
+    f = nb.compile(lambda a, b: a * b + a)
+    x, y, z = (torch.randn(40, 8, device="cuda") for _ in range(3))
+    f(_wrap(x), _wrap(x))
+    f(_wrap(x), _wrap(x))
+    assert not _taped(f) and "share" in f.tape_refused
+    for a, b in ((x, y), (y, z), (z, z), (x, z)):
+        assert torch.equal(f(_wrap(a), _wrap(b)).to_torch(), a * b + a)
+    assert _taped(f)
+
+
+def test_captured_tensors_and_results_that_alias():
+    import nabla_b200 as nb
+
+    w, x = torch.randn(16, 16, device="cuda"), torch.randn(4, 16, device="cuda")
+    held = _wrap(w)
+    f = nb.compile(lambda a: a * 2.0 + nb.reduce_sum(held * 1.0, axis=0))
+    for _ in range(3):
+        assert torch.allclose(f(_wrap(x)).to_torch(), x * 2 + w.sum(0), atol=1e-4)
+    assert _taped(f)
+    w.add_(1.0)                                       # in place: read anew on every call
+    assert torch.allclose(f(_wrap(x)).to_torch(), x * 2 + w.sum(0), atol=1e-4)
+    other = torch.randn(16, 16, device="cuda")
+    held._impl._buffers = [other]
+    assert torch.allclose(f(_wrap(x)).to_torch(), x * 2 + other.sum(0), atol=1e-4)
+    g = nb.compile(lambda a: (a, nb.reshape(a, (-1,)), a + 1.0))
+    for _ in range(4):
+        assert [t.shape for t in _leaves(g(_wrap(x)))] == [x.shape, (x.numel(),), x.shape]
+    assert not _taped(g)
+    h = nb.compile(lambda a: nb.uniform((8,), device=a.device) + a)
+    draws = [h(_wrap(torch.zeros(8, device="cuda"))).to_torch() for _ in range(4)]
+    assert not _taped(h) and not any(torch.equal(draws[0], d) for d in draws[1:])
+
+
+def test_taped_calls_on_streams_and_threads():
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    f = nb.compile(lambda x, a, b: F.layer_norm(F.layer_norm(x, a, b), a, b))
+    args = [(torch.randn(3000, 512, device="cuda") * (k + 1)).to(BF16) for k in range(8)]
+    a, b = torch.ones(512, device="cuda", dtype=BF16), torch.zeros(512, device="cuda", dtype=BF16)
+    want = [f(_wrap(x), _wrap(a), _wrap(b)).to_torch() for x in args]
+    assert _taped(f)
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(30):
+                x = args[(k + i) % 8].clone()
+                out = f(_wrap(x), _wrap(a), _wrap(b)).to_torch()
+                if not torch.equal(out, want[(k + i) % 8]):
+                    bad.append((k, i))
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
