@@ -14,6 +14,7 @@ CUDA bf16 tensors:
 * ``matmul -> mul(one element)`` and ``mul(one element) -> matmul ...`` (the scale of a LoRA adapter and its gradient): the
   factor is applied in the GEMM epilogue (compiled replays).
 * ``layer norm backward -> add``: the gradient that joins dx is added in the same pass (compiled replays).
+* ``linear`` with an activation whose pre-activation nobody reads (inference): it is not written (compiled replays).
 * ``matmul -> dact_mul`` (backward of linear + relu/gelu): the activation derivative is applied in
   the GEMM epilogue.
 * ``sub -> [mul with itself ->] sums over all axes -> division by a number``: the mean of a cross-entropy or a squared error, one
@@ -120,6 +121,12 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
                                 a.op.name == "gelu" and a.kwargs.get("approximate", "none") not in ("none", "tanh")):
                             chain = [i, j, k]
         kind = "linear_epilogue"
+        if chain is None and private and n.op.name == "linear" and n.kwargs.get("activation") in ("relu", "gelu", "gelu_tanh") \
+                and _is_plain_gemm(n) and len(n.outputs()) == 2 and n.outputs()[0] is not None:
+            z = n.outputs()[1]
+            if z is None or (id(z) not in target_ids and not cons.get(id(z))):
+                chain = [i]
+                kind = "linear_act"
         if chain is None and private and n.op.name == "gather" and _is_table_gather(n):
             o = sole_output(n)
             if private_intermediate(o):
@@ -706,6 +713,20 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
                 _store(n_, [[t] for t in o], keep_graph)
             else:
                 _plain(n_, keep_graph)
+        return
+    if kind == "linear_act":
+        from ... import native
+        from ...native.gemm import gemm_bf16
+
+        (lin,) = group
+        ins = [x._buffers[0] for x in lin.input_impls()]
+        x, w = ins[:2]
+        act = lin.kwargs["activation"]
+        if not native.use_native(x) or not x.numel():
+            return _plain(lin, keep_graph)
+        bias = ins[2] if len(ins) > 2 else torch.zeros(w.shape[-1], dtype=w.dtype, device=w.device)
+        out = gemm_bf16(x.reshape(-1, x.shape[-1]), w, bias=bias, epilogue="relu" if act == "relu" else "gelu", gelu_tanh=act == "gelu_tanh")
+        _store(lin, [[out.reshape(*x.shape[:-1], w.shape[-1])], None], keep_graph)
         return
     if kind == "bias_grads":
         from ... import native

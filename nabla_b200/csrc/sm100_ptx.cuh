@@ -327,26 +327,45 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
                "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
 }
-// erf(t) and exp(-t*t) together (Abramowitz & Stegun 7.1.26, |error| < 1.5e-7): one approximate
-// reciprocal, one ex2 and a degree-5 polynomial -- about half the instructions of erff() plus a
-// separate expf(), which matters because the exact-gelu epilogues run on four warps per CTA next
-// to the MMAs. The exponential is also the Gaussian density that d-gelu needs.
-__device__ __forceinline__ float erf_with_gauss(float t, float& gauss) {
-  const float at = fabsf(t);
-  float k;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(k) : "f"(fmaf(0.3275911f, at, 1.0f)));
-  float e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * at * at));
-  gauss = e;
-  float p = fmaf(k, 1.061405429f, -1.453152027f);
-  p = fmaf(k, p, 1.421413741f);
-  p = fmaf(k, p, -0.284496736f);
-  p = fmaf(k, p, 0.254829592f);
-  return copysignf(fmaf(-p * k, e, 1.0f), t);
+// The same for memory that this kernel touches once, and a load of it: first to leave L2, where the operands of a product stay.
+__device__ __forceinline__ void st_global_v8_once(void* p, const uint32_t* w) {
+  asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
 }
-__device__ __forceinline__ float gelu_erf(float x) {
-  float g;
-  return 0.5f * x * (1.0f + erf_with_gauss(x * 0.70710678118654752f, g));
+__device__ __forceinline__ void ld_global_v8_once(const void* p, uint32_t* w) {
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+               : "l"(p));
+}
+// 1 - Phi(|x|) = erfc(|x| / sqrt 2) / 2 and exp(-x * x / 2) of two numbers (Abramowitz & Stegun 7.1.26, |error of erf| < 1.5e-7, with
+// the argument's scale and the half in its constants). The exact-gelu epilogues are bound by instructions where a CTA has one tile and
+// no MMAs to work under. So the polynomial and its surroundings go in the two-wide fp32 instructions, the pair shares one
+// reciprocal, and no sign is taken off and put back: some 11 instructions an element instead of 20. |x| is cut at 40, where the
+// exponential is 0, so that no infinity or NaN of one number reaches the other. us, with the change of the auxiliary loads in the
+// GEMM: 1332 x 512 x 2048 gelu 11.7 -> 11.2, d-gelu 13.7 -> 12.5; 512 x 256 x 256 6.4 -> 5.65, 7.2 -> 5.9. Against 64 bits over [-12, 12]:
+// gelu 1.73e-8 -> 1.55e-8 (relative 2-norm; up to |x| = 5 no element further than 1.6e-3, was 4.9e-2), d-gelu 5.28e-8 -> 5.22e-8.
+__device__ __forceinline__ float2 gauss_tail2(float2 x, float2& cut, float2& gauss) {
+  cut = make_float2(fminf(fabsf(x.x), 40.f), fminf(fabsf(x.y), 40.f));
+  const float2 d = __ffma2_rn(cut, make_float2(0.231641888f, 0.231641888f), make_float2(1.f, 1.f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d.x * d.y));
+  const float2 k = __fmul2_rn(make_float2(r, r), make_float2(d.y, d.x));
+  const float2 e2 = __fmul2_rn(__fmul2_rn(cut, make_float2(-0.72134752044448170f, -0.72134752044448170f)), cut);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(gauss.x) : "f"(e2.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(gauss.y) : "f"(e2.y));
+  float2 p = __ffma2_rn(k, make_float2(0.5307027145f, 0.5307027145f), make_float2(-0.7265760135f, -0.7265760135f));
+  p = __ffma2_rn(k, p, make_float2(0.7107068705f, 0.7107068705f));
+  p = __ffma2_rn(k, p, make_float2(-0.142248368f, -0.142248368f));
+  p = __ffma2_rn(k, p, make_float2(0.127414796f, 0.127414796f));
+  return __fmul2_rn(__fmul2_rn(p, k), gauss);
+}
+// x * Phi(x) = max(x, 0) - |x| * (1 - Phi(|x|)); the maximum as (x + |x|) / 2, which passes NaN on.
+__device__ __forceinline__ float2 gelu_erf2(float2 x) {
+  float2 cut, g;
+  const float2 q = gauss_tail2(x, cut, g), half = make_float2(0.5f, 0.5f);
+  const float2 pos = __ffma2_rn(x, half, __fmul2_rn(make_float2(fabsf(x.x), fabsf(x.y)), half));
+  return __ffma2_rn(make_float2(-cut.x, -cut.y), q, pos);
 }
 __device__ __forceinline__ float gelu_tanh(float x) {
   float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
@@ -354,10 +373,13 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
   return 0.5f * x * (1.0f + t);
 }
-__device__ __forceinline__ float dgelu_erf(float x) {
-  float g;                                                 // exp(-x*x/2)
-  const float cdf = 0.5f * (1.0f + erf_with_gauss(x * 0.70710678118654752f, g));
-  return fmaf(x * 0.3989422804014327f, g, cdf);
+// Phi(x) + x * phi(x)
+__device__ __forceinline__ float2 dgelu_erf2(float2 x) {
+  float2 cut, g;
+  const float2 q = gauss_tail2(x, cut, g);
+  const float2 up = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-q.x, -q.y));
+  return __ffma2_rn(__fmul2_rn(x, make_float2(0.3989422804014327f, 0.3989422804014327f)), g,
+                    make_float2(x.x < 0.f ? q.x : up.x, x.y < 0.f ? q.y : up.y));
 }
 __device__ __forceinline__ float dgelu_tanh(float x) {
   float x2 = x * x;

@@ -1373,3 +1373,47 @@ def test_log_sum_of_rows_around_three_vectors_per_thread(dtype, D):
     assert ((lse.double() - ref)[rows].abs() <= 4e-6 * (1 + ref[rows].abs())).all() and torch.isnan(lse[5])
     assert torch.equal(picked[rows], x[torch.arange(9, device="cuda"), t].float()[rows])
     assert lse[4].item() <= torch.finfo(dtype).min / 2 and not torch.isfinite(lse[6])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (130, 264, 64), (129, 200, 512), (300, 77, 128), (2048, 16400, 64)])
+def test_gelu_epilogues_against_64_bits(M, N, K):
+    """Tiles of each width with ragged ends, one tile per CTA and several, results beyond half of L2; values into both tails, and
+    infinities and NaN, which stay with their own element."""
+    from nabla_b200.native.gemm import gemm_bf16
+
+    torch.manual_seed(25)
+    a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), (torch.randn(K, N, device="cuda") * 3 * K ** -0.5).to(torch.bfloat16)
+    bias, z = torch.randn(N, device="cuda").to(torch.bfloat16), (torch.randn(M, N, device="cuda") * 3).to(torch.bfloat16)
+    x = a.double() @ b.double()
+    phi = lambda t: 0.5 * torch.erfc(-t / 2 ** 0.5)  # noqa: E731
+    y, pre = gemm_bf16(a, b, bias=bias, epilogue="gelu", aux="store_preact")
+    t = x + bias.double()
+    assert _rel2(pre, t) < STORED[torch.bfloat16] and _rel2(y, t * phi(t)) < STORED[torch.bfloat16]
+    assert torch.equal(y, gemm_bf16(a, b, bias=bias, epilogue="gelu"))
+    zd = z.double()
+    d = phi(zd) + zd * torch.exp(-zd * zd / 2) / (2 * torch.pi) ** 0.5
+    assert _rel2(gemm_bf16(a, b, aux="dgelu", aux_in=z), x * d) < STORED[torch.bfloat16]
+    assert _rel2(gemm_bf16(a, b, aux="drelu", aux_in=z), x * (zd > 0)) < STORED[torch.bfloat16]
+    assert _rel2(gemm_bf16(a, b, bias=bias, aux="add", aux_in=z), t + zd) < STORED[torch.bfloat16]
+    odd = torch.tensor([float("nan"), 1.0, float("inf"), -2.0, -3e38, 3e38, 45.0, -45.0], device="cuda").to(torch.bfloat16)
+    bias2 = odd.repeat(-(-N // 8))[:N]
+    y = gemm_bf16(torch.zeros_like(a), b, bias=bias2, epilogue="gelu", out_dtype=torch.float32)
+    want = TF.gelu(bias2.double()).expand(M, N)
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+    ok = want.isfinite()
+    assert ((y.double() - want).abs()[ok] <= 2e-6 * want.abs()[ok] + 1e-6).all()
+
+
+def test_inference_writes_no_pre_activations():
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    torch.manual_seed(26)
+    x, w, b = (torch.randn(s, device="cuda").to(torch.bfloat16) for s in ((3, 50, 64), (64, 200), (200,)))
+    for act, ref in (("relu", torch.relu), ("gelu", TF.gelu), ("gelu_tanh", lambda t: TF.gelu(t, approximate="tanh"))):
+        for args in ((x, w, b), (x, w)):
+            f = nb.compile(lambda *a, act=act: F.linear(*a, activation=act))
+            got = [f(*map(nb.Tensor.from_torch, args)).to_torch() for _ in range(3)][-1]
+            t = x.double() @ w.double() + (b.double() if len(args) == 3 else 0)
+            assert _rel2(got, ref(t)) < STORED[torch.bfloat16] + (2e-3 if act == "gelu_tanh" else 0)
+            assert "linear_act" in f.dump_plan()
