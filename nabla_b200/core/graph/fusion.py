@@ -11,6 +11,8 @@ CUDA bf16 tensors:
   process per GPU: one launch of the fused GEMM + collective kernel (tiles are reduced over
   NVLink while later tiles are still being multiplied).
 * ``linear (+bias) | matmul -> add(residual)``: the residual is added in the GEMM epilogue (compiled replays).
+* ``x @ w [+ b] + (h @ v) [* one element]`` with a K of h of up to 256 (a frozen weight and its adapter): one launch, whose accumulator takes both
+  products (compiled replays).
 * ``matmul -> mul(one element)`` and ``mul(one element) -> matmul ...`` (the scale of a LoRA adapter and its gradient): the
   factor is applied in the GEMM epilogue (compiled replays).
 * ``layer norm backward -> add``: the gradient that joins dx is added in the same pass (compiled replays).
@@ -207,6 +209,11 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
             if dk is not None:
                 chain = [i, dk]
                 kind = "gemm_dact"
+        if chain is None and private and n.op.name in ("matmul", "linear"):
+            dual = _sum_of_products(i, nodes, cons, used, producer, private_intermediate, heads_epilogue)
+            if dual is not None:
+                chain = dual
+                kind = _DUAL[len(dual) - 3]
         if chain is None and private and n.op.name == "matmul" and _is_cuda_bf16_2d(n):
             # x @ w * s with one element s
             o = sole_output(n)
@@ -389,10 +396,54 @@ def _mean_of_difference(i: int, nodes, cons, target_ids, used, producer, private
             return None
         if m.op.name == "divide_by_count" and m.outputs()[0] is not None:
             return idxs + [j]
-        if m.op.name == "div" and _is_plain_binary(m) and m.input_impls()[0] is cur and m.input_impls()[1].literal \
+        if m.op.name == "div" and _is_plain_binary(m) and m.input_impls()[0] is cur and m.input_impls()[1].literal is not None \
                 and not m.input_impls()[1]._shape:
             return idxs + [j]
         return None
+
+
+_DUAL = ("gemm+gemm_residual", "gemm_scale+gemm_residual")       # a sum of two products, without a factor and with one
+
+
+def _sum_of_products(i: int, nodes, cons, used, producer, private_intermediate, heads_epilogue) -> list[int] | None:
+    """[small product, (its scale,) large product, add] in the order of the schedule when product ``i`` is one of two that are added. The
+    small one has the shorter K, of up to 256, and perhaps a one-element factor behind it; nobody else reads either."""
+    def branch(j: int):
+        # (nodes from the product to what is added, the value that is added)
+        if used[j] or nodes[j].op.name not in ("matmul", "linear") or nodes[j].kwargs.get("activation") is not None or not _is_plain_gemm(nodes[j]) \
+                or heads_epilogue(j):
+            return None
+        o = nodes[j].outputs()[0]
+        if not private_intermediate(o):
+            return None
+        k = cons[id(o)][0]
+        if not used[k] and nodes[k].op.name == "mul" and _scalar_factor(nodes[k], o) is not None:
+            v = nodes[k].outputs()[0]
+            return ([j, k], v) if private_intermediate(v) else None
+        return [j], o
+
+    mine = branch(i)
+    if mine is None:
+        return None
+    path, value = mine
+    k = cons[id(value)][0]
+    add = nodes[k]
+    if used[k] or add.op.name != "add" or not _same_layout_addend(add, value):
+        return None
+    other = [x for x in add.input_impls() if x is not value][0]
+    j = producer.get(id(other), -1)
+    if j >= 0 and nodes[j].op.name == "mul" and not used[j]:
+        firsts = [producer[id(x)] for x in nodes[j].input_impls() if id(x) in producer and _scalar_factor(nodes[j], x) is not None]
+        j = firsts[0] if len(firsts) == 1 else -1
+    theirs = branch(j) if j >= 0 and j != i else None
+    if theirs is None or theirs[1] is not other:
+        return None
+    small, large = sorted((path, theirs[0]), key=lambda p: int(nodes[p[0]].input_impls()[0]._shape[-1]))
+    depth = int(nodes[small[0]].input_impls()[0]._shape[-1])
+    if depth > 256 or len(large) > 1 or len(nodes[small[0]].input_impls()) > 2 \
+            or depth >= int(nodes[large[0]].input_impls()[0]._shape[-1]):
+        return None
+    return small + large + [k]
 
 
 def _is_counted_step(add: OpNode, o: TensorImpl) -> bool:
@@ -401,7 +452,7 @@ def _is_counted_step(add: OpNode, o: TensorImpl) -> bool:
 
     ins = add.input_impls()
     return (o.dtype is DType.float32 and not o._shape and not ins[0]._shape and not ins[1]._shape and ins[0] is not ins[1]
-            and any(x.literal for x in ins))
+            and any(x.literal is not None for x in ins))
 
 
 def _is_table_gather(n: OpNode) -> bool:
@@ -871,6 +922,34 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         else:
             _plain(ln, keep_graph)
             _plain(add, keep_graph)
+        return
+    if kind in _DUAL:
+        from ... import native
+        from ...native import kernels
+        from ...native.gemm import dual_takes, gemm_dual
+
+        small, big, add = group[0], group[-2], group[-1]
+        a2, b2 = [x._buffers[0] for x in small.input_impls()]
+        ins = [x._buffers[0] for x in big.input_impls()]
+        a, b = ins[:2]
+        k, k2, n_out = a.shape[-1], a2.shape[-1], b.shape[-1]
+        m = a.numel() // max(k, 1)
+        if native.use_native(a) and a.numel() and b.numel() and dual_takes(m, n_out, k, k2):
+            a2 = a2.reshape(-1, k2)
+            if len(group) == 4:
+                factor = _scalar_factor(group[1], small.outputs()[0])
+                if factor.literal != 1:                    # the thin operand takes the factor
+                    s = factor._buffers[0].reshape(())
+                    scaled = kernels.binary(a2, s, "mul")
+                    a2 = scaled if scaled is not None else a2 * s
+            out = gemm_dual(a.reshape(-1, k), b, a2, b2, ins[2] if len(ins) > 2 else None)
+            _store(add, [[out.reshape(*a.shape[:-1], n_out)]], keep_graph)
+        else:
+            if len(group) == 4:
+                run_fused("gemm_scale", list(group[:2]), keep_graph)
+            else:
+                _plain(small, keep_graph)
+            run_fused("gemm_residual", [big, add], keep_graph)
         return
     if kind == "gemm_residual":
         from ... import native

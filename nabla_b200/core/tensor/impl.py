@@ -48,7 +48,7 @@ class TensorImpl:
         self.output_index = 0
         self._local_shapes = None
         self._keepalive = None
-        self.literal = False            # a Python number that an op was given
+        self.literal = None             # the Python number that an op was given
         if buffers is not None and shape is None:
             b0 = buffers[0]
             if sharding is not None:
@@ -76,7 +76,7 @@ class TensorImpl:
         new.sharding_constraint = new.grad = new.tangent = new.cotangent = new.dual = None
         new.output_refs = new._local_shapes = new._keepalive = None
         new.output_index = 0
-        new.literal = False
+        new.literal = None
         return new
 
     # ---- state

@@ -46,6 +46,7 @@ struct GemmArgs {
   int a_mn, b_mn;           // 1 = MN-major operand
   int out_fp32, bias_fp32;
   int epi, aux, accumulate, gelu_tanh;
+  int K2, a2_mn, b2_mn;                // the second pair of operands of a sum of two products
   int once;                            // results (1) and auxiliary inputs (2) go past L2's order of use
   int vec_ok;               // output/aux rows are 16-byte aligned
   int vec32_ok;             // ... and 32-byte aligned: a lane's 32 columns go out as 32-byte stores (whole sectors)
@@ -193,10 +194,12 @@ __device__ __forceinline__ unsigned ld_acquire_gpu_u32(const unsigned* p) {
 // their row blocks need not be neighbours once a fused mode has re-ordered them), the tensor map of
 // B has a box of BN / 2 rows, the loads of both CTAs complete on the leader's full barriers, and the
 // leader's MMA warp issues for both CTAs.
-template <int BN, int MODE, bool PAIR = false>
+// DUAL: out = epilogue(A B + A2 B2), one accumulator: the k-blocks of the second pair of operands follow those of the first.
+template <int BN, int MODE, bool PAIR = false, bool DUAL = false>
 __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensorMap* tmBp, const GemmArgs& args,
                                          const CommArgs& comm, const int cta, const int nctas,
-                                         const CUtensorMap* tmAownp = nullptr) {
+                                         const CUtensorMap* tmAownp = nullptr, const CUtensorMap* tmA2p = nullptr,
+                                         const CUtensorMap* tmB2p = nullptr) {
   const CUtensorMap& tmA = *tmAp;
   const CUtensorMap& tmB = *tmBp;
   using L = typename SmemSelect<BN, PAIR>::type;
@@ -230,11 +233,15 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
   const int num_m = (args.M + TILE_M - 1) / TILE_M;
   const int num_n = (args.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n * args.batch;
-  const int num_kb = (args.K + BLOCK_K - 1) / BLOCK_K;
+  const int num_kb1 = (args.K + BLOCK_K - 1) / BLOCK_K, num_kb = DUAL ? num_kb1 + (args.K2 + BLOCK_K - 1) / BLOCK_K : num_kb1;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    if (DUAL) {
+      tma_prefetch_desc(tmA2p);
+      tma_prefetch_desc(tmB2p);
+    }
     for (int s = 0; s < STAGES; ++s) {
       // pair: only the leader's full barriers are used; the loads of both CTAs complete on them
       mbar_init(&full_bar[s], 1);
@@ -324,51 +331,53 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
           // pair: the leader expects the bytes of both CTAs on its barrier; the other CTA only loads
           if (!PAIR) mbar_arrive_expect_tx(&full_bar[stage], L::STAGE_BYTES);
           else if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * L::STAGE_BYTES);
-          const int k0 = kb * BLOCK_K;
+          const bool second = DUAL && kb >= num_kb1;
+          const int k0 = (second ? kb - num_kb1 : kb) * BLOCK_K, a_mn = second ? args.a2_mn : args.a_mn, b_mn = second ? args.b2_mn : args.b_mn;
+          const CUtensorMap *mapA = second ? tmA2p : tmAuse, *mapB = second ? tmB2p : tmBp;
           // debug build: every tile origin lies inside its tensor and the innermost coordinate
           // starts on a 16-byte boundary; a failed check skips the copies (the consumers' bounded
           // waits then end the kernel) instead of issuing them
           // (in a pair the second CTA's half tile may start past the edge: those loads read the fill value)
-          if (!(NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, k0, args.K) &&
+          if (!(NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, k0, second ? args.K2 : args.K) &&
                 NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, m0, args.M + (PAIR ? BLOCK_M : 0)) &&
                 NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, n0, args.N + (PAIR ? BNL : 0)) &&
                 NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, b, args.batch) &&
                 NB_IN_BOUNDS(NB_SITE_GEMM_TMA_COORD, ma0, args.M + (PAIR ? BLOCK_M : 0)) &&
-                NB_ALIGNED(NB_SITE_GEMM_TMA_ALIGN, (args.a_mn ? m0 : k0) * 2, 16) &&
-                NB_ALIGNED(NB_SITE_GEMM_TMA_ALIGN, (args.b_mn ? n0 : k0) * 2, 16))) {
+                NB_ALIGNED(NB_SITE_GEMM_TMA_ALIGN, (a_mn ? m0 : k0) * 2, 16) &&
+                NB_ALIGNED(NB_SITE_GEMM_TMA_ALIGN, (b_mn ? n0 : k0) * 2, 16))) {
             ok = false;
             break;
           }
           if (PAIR) {
             const uint32_t lbar = leader_full + 8u * stage;   // the leader's full barrier of this stage
-            if (!args.a_mn) {
-              tma_load_3d_pair(sA, tmAuse, lbar, k0, ma0, b);
+            if (!a_mn) {
+              tma_load_3d_pair(sA, mapA, lbar, k0, ma0, b);
             } else {
 #pragma unroll
               for (int j = 0; j < BLOCK_M / 64; ++j)
-                tma_load_3d_pair(sA + j * (BLOCK_K * 128), &tmA, lbar, m0 + j * 64, k0, b);
+                tma_load_3d_pair(sA + j * (BLOCK_K * 128), mapA, lbar, m0 + j * 64, k0, b);
             }
-            if (!args.b_mn) {
-              tma_load_3d_pair(sB, &tmB, lbar, k0, n0, b);
+            if (!b_mn) {
+              tma_load_3d_pair(sB, mapB, lbar, k0, n0, b);
             } else {
 #pragma unroll
               for (int j = 0; j < BNL / 64; ++j)
-                tma_load_3d_pair(sB + j * (BLOCK_K * 128), &tmB, lbar, n0 + j * 64, k0, b);
+                tma_load_3d_pair(sB + j * (BLOCK_K * 128), mapB, lbar, n0 + j * 64, k0, b);
             }
           } else {
-            if (!args.a_mn) {
-              tma_load_3d(sA, tmAuse, &full_bar[stage], k0, ma0, b);
+            if (!a_mn) {
+              tma_load_3d(sA, mapA, &full_bar[stage], k0, ma0, b);
             } else {
 #pragma unroll
               for (int j = 0; j < BLOCK_M / 64; ++j)
-                tma_load_3d(sA + j * (BLOCK_K * 128), &tmA, &full_bar[stage], m0 + j * 64, k0, b);
+                tma_load_3d(sA + j * (BLOCK_K * 128), mapA, &full_bar[stage], m0 + j * 64, k0, b);
             }
-            if (!args.b_mn) {
-              tma_load_3d(sB, &tmB, &full_bar[stage], k0, n0, b);
+            if (!b_mn) {
+              tma_load_3d(sB, mapB, &full_bar[stage], k0, n0, b);
             } else {
 #pragma unroll
               for (int j = 0; j < BNL / 64; ++j)
-                tma_load_3d(sB + j * (BLOCK_K * 128), &tmB, &full_bar[stage], n0 + j * 64, k0, b);
+                tma_load_3d(sB + j * (BLOCK_K * 128), mapB, &full_bar[stage], n0 + j * 64, k0, b);
             }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -380,13 +389,20 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
     if (PAIR && !leader) {
       // the other CTA of the pair issues nothing: the leader's thread drives both tensor cores
     } else if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(TILE_M, BN, args.a_mn, args.b_mn);
+      uint32_t idesc = make_idesc_bf16(TILE_M, BN, args.a_mn, args.b_mn);
       // Per-operand descriptor constants.
-      const uint32_t a_lbo = args.a_mn ? BLOCK_K * 128 : 16, a_sbo = 1024;
-      const uint32_t b_lbo = args.b_mn ? BLOCK_K * 128 : 16, b_sbo = 1024;
+      uint32_t a_lbo = args.a_mn ? BLOCK_K * 128 : 16, b_lbo = args.b_mn ? BLOCK_K * 128 : 16;
+      constexpr uint32_t a_sbo = 1024, b_sbo = 1024;
       // Descriptor start-address step per UMMA_K (in 16-byte units).
-      const uint32_t a_kstep = args.a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
-      const uint32_t b_kstep = args.b_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      uint32_t a_kstep = args.a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      uint32_t b_kstep = args.b_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      auto use_operands = [&](int a_mn, int b_mn) {
+        idesc = make_idesc_bf16(TILE_M, BN, a_mn, b_mn);
+        a_lbo = a_mn ? BLOCK_K * 128 : 16;
+        b_lbo = b_mn ? BLOCK_K * 128 : 16;
+        a_kstep = a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+        b_kstep = b_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      };
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -408,6 +424,10 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
             break;
           }
           tc_fence_after();
+          if (DUAL && (kb == 0 || kb == num_kb1)) {
+            if (kb == 0) use_operands(args.a_mn, args.b_mn);
+            else use_operands(args.a2_mn, args.b2_mn);
+          }
           const uint32_t sA = smem_u32(ring + stage * L::STAGE_BYTES);
           const uint32_t sB = sA + L::A_BYTES;
           const uint64_t da = make_smem_desc_sw128(sA, a_lbo, a_sbo);
@@ -825,6 +845,24 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
                               const GemmArgs args) {
   CommArgs none{};
   gemm_cta<BN, MODE_NONE, true>(&tmA, &tmB, args, none, blockIdx.x >> 1, gridDim.x >> 1);
+}
+
+// A sum of two products, on lone CTAs and on pairs: a frozen weight and a low-rank adapter beside it. The adapter's product as a launch of its
+// own writes all of M x N once for a K of 16, and the sum reads it: 2048 x 6144 x 2048 with rank 16 18 + 43 us, 43 so; 2048 x 2048 x 6144 9 + 46,
+// 44 so. Like them bound by their waves of tiles (192 on 74 pairs, 128 on 148 SMs).
+template <int BN>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_bf16_dual_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
+                      const __grid_constant__ CUtensorMap tmB2, const GemmArgs args) {
+  CommArgs none{};
+  gemm_cta<BN, MODE_NONE, false, true>(&tmA, &tmB, args, none, blockIdx.x, gridDim.x, nullptr, &tmA2, &tmB2);
+}
+template <int BN>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_bf16_dual_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
+                           const __grid_constant__ CUtensorMap tmB2, const GemmArgs args) {
+  CommArgs none{};
+  gemm_cta<BN, MODE_NONE, true, true>(&tmA, &tmB, args, none, blockIdx.x >> 1, gridDim.x >> 1, nullptr, &tmA2, &tmB2);
 }
 
 // The K range of a tile on a cluster of SLICES CTAs: each multiplies its k-blocks and lays its fp32 tile over the ring that
@@ -1593,6 +1631,34 @@ static int launch_slices(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
   return cudaLaunchKernelEx(&cfg, kernel, ta, tb, a) == cudaSuccess ? 0 : -3;
 }
 
+// A persistent launch of at most one cluster of `cluster` CTAs per as many SMs over `tiles` tiles.
+template <int SMEM, typename Kernel>
+static int launch_with(Kernel kernel, int cluster, long long tiles, cudaStream_t stream, const CUtensorMap* maps, const GemmArgs& a) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -2;
+  long long n = g_num_sms / cluster;
+  if (cluster > 1 && n > 0) {
+    cfg.gridDim = dim3((unsigned)(cluster * n));
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess || fit < 1) return -2;
+    if (fit < n) n = fit;
+  }
+  if (tiles < n) n = tiles;
+  if (n < 1) return 0;
+  cfg.gridDim = dim3((unsigned)(cluster * n));
+  return cudaLaunchKernelEx(&cfg, kernel, maps[0], maps[1], maps[2], maps[3], a) == cudaSuccess ? 0 : -3;
+}
+
 // bit 0: CTA pairs for 256-wide tiles of plain GEMMs with at least one tile pair per two SMs;
 // bit 1: CTA pairs in the fused GEMM + collective kernels (even number of 128-row tiles). 0: lone CTAs only
 static int g_pair_mode = 0;
@@ -1753,6 +1819,53 @@ extern "C" int nb_gemm_bf16(const void* A, const void* B, void* C, const void* b
   if (bn == 256) return launch<256>(ta, tb, g, max_ctas, s);
   if (bn == 128) return launch<128>(ta, tb, g, max_ctas, s);
   return launch<64>(ta, tb, g, max_ctas, s);
+}
+
+// out = A B + A2 B2 (+ bias), bf16, with the second pair of operands as the first is given: one launch of whole tiles. -20: the
+// product of the first pair is one that is cut into slices of K, which the sum does not do.
+extern "C" int nb_gemm_dual_bf16(const void* A, const void* B, const void* A2, const void* B2, void* C, const void* bias, int M, int N, int K,
+                                 int K2, long long lda, long long ldb, long long lda2, long long ldb2, long long ldc, int a_mn, int b_mn,
+                                 int a2_mn, int b2_mn, int bias_fp32, int* status, void* stream) {
+  using namespace nb;
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || K2 <= 0) return -10;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(A2) | reinterpret_cast<uintptr_t>(B2)) & 15)
+    return -11;
+  if ((lda | ldb | lda2 | ldb2) & 7) return -12;
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  const int bn = tile_width(M, N, 1);
+  if (slice_plan(M, N, K, bn).slices > 1) return -20;
+  const bool pair = (g_pair_mode & 1) && bn == 256 && M >= 2 * BLOCK_M &&
+                    (long long)((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + 255) / 256) >= g_num_sms / 2;
+  CUtensorMap maps[4];
+  const void* const base[4] = {A, B, A2, B2};
+  const long long ld[4] = {lda, ldb, lda2, ldb2};
+  const int mn[4] = {a_mn, b_mn, a2_mn, b2_mn};
+  for (int i = 0; i < 4; ++i) {
+    const int k = i < 2 ? K : K2, rows = i & 1 ? N : M, box = i & 1 ? (pair ? bn / 2 : bn) : BLOCK_M;
+    const int r = mn[i] ? make_map(&maps[i], base[i], rows, k, 1, ld[i], 0, BLOCK_K) : make_map(&maps[i], base[i], k, rows, 1, ld[i], 0, box);
+    if (r) return r;
+  }
+  GemmArgs g{};
+  g.M = M; g.N = N; g.K = K; g.K2 = K2; g.batch = 1;
+  g.out = C; g.bias = bias; g.bias_fp32 = bias_fp32; g.epi = bias != nullptr ? EPI_BIAS : EPI_NONE;
+  g.ldc = ldc; g.stride_c = (long long)M * ldc;
+  g.a_mn = a_mn; g.b_mn = b_mn; g.a2_mn = a2_mn; g.b2_mn = b2_mn;
+  g.alpha = 1.f;
+  g.status = status;
+  g.vec_ok = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc % 8 == 0;
+  g.vec32_ok = (reinterpret_cast<uintptr_t>(C) & 31) == 0 && ldc % 16 == 0;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+#define DUAL(BN) launch_with<SmemLayout<BN>::TOTAL>(gemm_bf16_dual_kernel<BN>, 1, (long long)((M + BLOCK_M - 1) / BLOCK_M) * ((N + BN - 1) / BN), s, maps, g)
+  if (pair)
+    return launch_with<SmemLayoutPair<256>::TOTAL>(gemm_bf16_dual_pair_kernel<256>, 2,
+                                                   (long long)((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + 255) / 256), s, maps, g);
+  return bn == 256 ? DUAL(256) : bn == 128 ? DUAL(128) : DUAL(64);
+#undef DUAL
 }
 
 // Fused GEMM + collective over a symmetric workspace (one launch; see FusedMode).

@@ -24,6 +24,8 @@ def _get():
         fn.restype = ctypes.c_int
         fn.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int] * 4 + [ctypes.c_longlong] * 8 + [ctypes.c_int] * 8 + [
             ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+        lib.nb_gemm_dual_bf16.restype = ctypes.c_int
+        lib.nb_gemm_dual_bf16.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int] * 4 + [ctypes.c_longlong] * 5 + [ctypes.c_int] * 5 + [ctypes.c_void_p] * 2
         lib.nb_gemm_slices.argtypes = [ctypes.c_int] * 3
         lib.nb_gemm_slices.restype = ctypes.c_int
         lib.nb_gemm_set_pair_mode.argtypes = [ctypes.c_int]
@@ -314,3 +316,36 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
     if aux == "store_preact":
         return res, (aux_out[0] if squeeze else aux_out)
     return res
+
+
+def dual_takes(M: int, N: int, K: int, K2: int) -> bool:
+    """Is ``a @ b + a2 @ b2`` one launch? Where the first product runs in whole tiles and its rows start on 16-byte boundaries."""
+    return N % 8 == 0 and min(M, N, K, K2) > 0 and cluster_slices(M, N, K) == 1 and split_k_factor(M, N, K) == 1
+
+
+def gemm_dual(a: torch.Tensor, b: torch.Tensor, a2: torch.Tensor, b2: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """``a @ b + a2 @ b2 [+ bias]`` of 2-D bf16 matrices, summed in one accumulator and rounded once (``dual_takes``)."""
+    global launch_count
+    from . import load, ptr, recorder, status_word, stream_ptr
+
+    _get()
+    dev = a.get_device()
+    if dev < 0 or any(t is not None and t.get_device() != dev for t in (b, a2, b2, bias)):
+        raise RuntimeError("gemm_dual: expected all tensors to be on the same GPU")
+    (M, K), N, K2 = a.shape, b.shape[1], a2.shape[1]
+    assert b.shape[0] == K and tuple(a2.shape) == (M, K2) and tuple(b2.shape) == (K2, N)
+    (a, ak, lda, _), (b, bk, ldb, _), (a2, a2k, lda2, _), (b2, b2k, ldb2, _) = (_prep(t.unsqueeze(0)) for t in (a, b, a2, b2))
+    if bias is not None:
+        bias = bias.reshape(-1).contiguous()
+        assert bias.numel() == N
+        if bias.dtype not in (torch.float32, torch.bfloat16):
+            bias = bias.to(torch.bfloat16)
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
+    fn, r = load("libnb_gemm.so").nb_gemm_dual_bf16, recorder()
+    rc = (fn if r is None else r.function("nb_gemm_dual_bf16", fn))(
+        ptr(a), ptr(b), ptr(a2), ptr(b2), ptr(out), ptr(bias), M, N, K, K2, lda, ldb, lda2, ldb2, N, int(ak != "row"), int(bk == "row"),
+        int(a2k != "row"), int(b2k == "row"), int(bias is not None and bias.dtype == torch.float32), ptr(status_word(out.device)), stream_ptr())
+    if rc != 0:
+        raise RuntimeError(f"nb_gemm_dual_bf16 failed with code {rc}")
+    launch_count += 1
+    return out

@@ -58,7 +58,7 @@ def ensure_tensor(x: Any, like: Tensor | None = None) -> Tensor:
         elif isinstance(x, int) and like.dtype is DType.bool:
             dtype = DType.int32            # True + 2 is 3, not True (numpy's promotion of bool with an integer)
         t = constant(x, dtype=dtype, device=like.device)
-        t._impl.literal = isinstance(x, (bool, int, float))
+        t._impl.literal = x if isinstance(x, (bool, int, float)) else None
         return t
     return constant(x)
 

@@ -1206,7 +1206,7 @@ def _make_constants(rec: "_Recorded", max_elems: int = 1 << 16) -> list:
         numel = 1
         for d in outs[0]._shape:
             numel *= int(d)
-        if numel <= max_elems and all(id(a) in made or (a.literal and a.sharding is None) for a in n.input_impls()):
+        if numel <= max_elems and all(id(a) in made or (a.literal is not None and a.sharding is None) for a in n.input_impls()):
             made[id(outs[0])] = idxs[0]
     while True:                                     # until every reader of what is left is as above
         bad = [k for k, ni in made.items() if not all(
@@ -1216,7 +1216,7 @@ def _make_constants(rec: "_Recorded", max_elems: int = 1 << 16) -> list:
             break
         for k in bad:
             del made[k]
-        for k in [k for k, ni in made.items() if not all(id(a) in made or a.literal for a in nodes[ni].input_impls())]:
+        for k in [k for k, ni in made.items() if not all(id(a) in made or a.literal is not None for a in nodes[ni].input_impls())]:
             made.pop(k, None)
     if not made or torch.cuda.is_current_stream_capturing():       # (a capture of the caller's: nothing may be waited for)
         return rec.steps

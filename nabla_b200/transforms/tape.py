@@ -21,7 +21,7 @@ from ..core.tensor.api import Tensor
 from ..core.tensor.impl import TensorImpl
 
 # launch functions: all of their effects are on the device and on the stream that is their last argument
-LAUNCHES = frozenset("""nb_gemm_bf16 nb_attn_fwd nb_attn_bwd nb_layernorm_fwd nb_layernorm_bwd nb_colsum nb_colsum_group nb_softmax
+LAUNCHES = frozenset("""nb_gemm_bf16 nb_gemm_dual_bf16 nb_attn_fwd nb_attn_bwd nb_layernorm_fwd nb_layernorm_bwd nb_colsum nb_colsum_group nb_softmax
     nb_lse_pick_fwd nb_lse_pick_bwd nb_adamw nb_adamw_group nb_adam_hyper nb_mean_diff nb_sgd nb_embedding_gather nb_embedding_scatter_add
     nb_cast nb_activation nb_nf4_dequant nb_nf4_dequant_codes nb_pool2d_fwd nb_pool2d_bwd nb_pool2d_select nb_conv2d_direct
     nb_conv2d_wgrad_direct nb_sgemm nb_sum_slices nb_binary nb_unary nb_reduce nb_cumsum""".split())
@@ -303,7 +303,7 @@ def _tape(rec, tensors, tds, r: _Recorder, result_buffers):
                 out.append(e)
         launches.append((address, rc, name, out))
     return module().make((tuple(tree_of(td) for td in tds), _leaves(tensors), _environment(), device, config.is_deterministic(), launches,
-                          scratch, outs, tree_of(rec.out_treedef), None, [a for a in _captured(rec) if not a.literal]))
+                          scratch, outs, tree_of(rec.out_treedef), None, [a for a in _captured(rec) if a.literal is None]))
 
 
 def _extent(t: torch.Tensor) -> tuple[int, int]:

@@ -1417,3 +1417,50 @@ def test_inference_writes_no_pre_activations():
             t = x.double() @ w.double() + (b.double() if len(args) == 3 else 0)
             assert _rel2(got, ref(t)) < STORED[torch.bfloat16] + (2e-3 if act == "gelu_tanh" else 0)
             assert "linear_act" in f.dump_plan()
+
+
+# ---------------------------------------------------------------- sums of two products
+@pytest.mark.parametrize("M,N,K,K2", [(2048, 1536, 512, 16), (2100, 2056, 1032, 8), (16384, 512, 512, 64), (1300, 520, 456, 1), (9500, 136, 72, 200), (640, 8200, 264, 256)])
+def test_sums_of_two_products(M, N, K, K2):
+    """Lone CTAs of each width and pairs, ragged ends of all four sizes, every order of the operands, with a bias and without."""
+    from nabla_b200.native.gemm import dual_takes, gemm_dual
+
+    torch.manual_seed(27)
+    assert dual_takes(M, N, K, K2)
+    bias = torch.randn(N, device="cuda").to(torch.bfloat16)
+    for order in range(16):
+        ops = []
+        for i, (r, c, std) in enumerate(((M, K, 1.0), (K, N, K ** -0.5), (M, K2, 1.0), (K2, N, K2 ** -0.5))):
+            t = (torch.randn(r, c, device="cuda") * std).to(torch.bfloat16)
+            ops.append(t.t().contiguous().t() if order >> i & 1 else t)
+        a, b, a2, b2 = ops
+        ref = a.double() @ b.double() + a2.double() @ b2.double()
+        assert _rel2(gemm_dual(a, b, a2, b2), ref) < STORED[torch.bfloat16]
+        if order in (0, 15):
+            assert _rel2(gemm_dual(a, b, a2, b2, bias), ref + bias.double()) < STORED[torch.bfloat16]
+
+
+@pytest.mark.parametrize("M,scale", [(1500, 16.0), (1500, 24.0), (100, 16.0), (1500, None)])
+def test_compiled_adapters(M, scale):
+    """A frozen product with an adapter beside it and all gradients; 100 rows run as slices of K and keep their launches."""
+    import nabla_b200 as nb
+
+    torch.manual_seed(28)
+    x, w, a, b, dy = ((torch.randn(s, device="cuda") * std).to(torch.bfloat16) for s, std in (
+        ((M, 520), 1.0), ((520, 1032), 520 ** -0.5), ((520, 16), 0.05), ((16, 1032), 0.3), ((M, 1032), 1.0)))
+
+    def layer(x, w, a, b):
+        h = (x @ a) @ b
+        return x @ w + (h if scale is None else h * (scale / 16))
+
+    def step(x, w, a, b, dy):
+        y, pull = nb.vjp(lambda x, a, b: layer(x, w, a, b), x, a, b, create_graph=False)
+        return (y, *pull(dy))
+
+    f = nb.compile(step)
+    got = [[t.to_torch() for t in f(*map(nb.Tensor.from_torch, (x, w, a, b, dy)))] for _ in range(3)][-1]
+    d = [t.double().requires_grad_(True) for t in (x, a, b)]
+    ref = layer(d[0], w.double(), d[1], d[2])
+    for g, r in zip(got, (ref, *torch.autograd.grad(ref, d, dy.double()))):
+        assert _rel2(g, r.detach()) < 2 * STORED[torch.bfloat16]
+    assert sum("+gemm_residual" in line for line in f.dump_plan().splitlines()) == 2
