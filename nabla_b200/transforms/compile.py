@@ -821,13 +821,15 @@ class CompiledFunction:
 
     def _replay(self, rec: _Recorded, tensors: list[Tensor], tds: tuple | None = None) -> Any:
         """``tds``: the arguments' structures, where nothing but tensors is among them."""
-        if self.use_cuda_graph and not rec.host_sync and tensors and tensors[0]._impl.device.label == "gpu":
+        if self.use_cuda_graph and not rec.host_sync and tensors and tensors[0]._impl.device.label == "gpu" \
+                and not (rec.cuda_graph is None and rec.tape is None and tds is not None and _copies_outweigh_launches(rec) and tape.can_record(rec)):
             out = self._replay_cuda_graph(rec, tensors)
             if rec.tape is None and rec.cuda_graph is not None and tds is not None and rec.copy_out is not None:
                 rec.tape = tape.graph_call(rec, tensors, tds) or False
                 rec.tape_counts = (0, rec.copy_in.launches + rec.copy_out.launches, 0) if rec.tape else ()
             self._taped = (rec.tape, rec, True) if rec.tape and tds is not None else None
             return out
+        # (a call that was to be captured and whose launches are written down instead comes here too)
         for ph, t in zip(rec.placeholders, tensors):
             ph._buffers = t._impl._buffers
         try:
@@ -841,7 +843,7 @@ class CompiledFunction:
             else:
                 self._run(rec)
                 out = self._collect(rec)
-            self._taped = (rec.tape, rec, False) if rec.tape and tds is not None else None
+            self._taped = (rec.tape, rec, self.use_cuda_graph) if rec.tape and tds is not None else None
             return out
         finally:
             for ph in rec.placeholders:
@@ -913,6 +915,21 @@ class CompiledFunction:
                 res = [b if b.data_ptr() in rec.static_ptrs else next(taken) for b in bufs] if rec.static_ptrs else [next(taken) for _ in bufs]
                 outs.append(Tensor(impl=TensorImpl.result_like(impl, res)))
         return pytree.tree_unflatten(rec.out_treedef, outs)
+
+
+def _copies_outweigh_launches(rec: "_Recorded") -> bool:
+    """Is a schedule that is to be replayed from a CUDA graph better written down (``transforms/tape.py``)? A graph owns its arguments and
+    results, so all of them are copied in and out on each call; written-down launches take them where they are, but follow each other some
+    1.6 us later than a graph's. So by the time of the copies at HBM's rate and 2 us a launch: a QLoRA layer of 2048 tokens (80 MB, 7
+    launches) 158 us captured and 142 written down, the logits of a small decoder (66 MB, 31 launches) 260 and 289."""
+    nbytes = 0
+    for im in [*rec.placeholders, *(o for o in rec.out_impls if o is not None)]:
+        n = im.dtype.to_torch().itemsize
+        for d in im._shape:
+            n *= int(d)
+        nbytes += n
+    launches = sum(1 for kind, idxs in rec.steps if kind != "op" or ".ops.view." not in type(rec.nodes[idxs[0]].op).__module__)
+    return 2 * nbytes / 6.4e6 >= 2.0 * launches
 
 
 def _counted_modules() -> tuple:

@@ -184,3 +184,32 @@ def test_taped_calls_on_streams_and_threads():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not bad
+
+
+def test_large_arguments_of_a_captured_function_are_not_copied():
+    """Few launches on large tensors are written down and not captured; a call that does not match is captured and right, and so is
+    the next that matches."""
+    import nabla_b200 as nb
+
+    f = nb.compile(lambda x, w: x @ w, cuda_graph=True)
+    g = torch.Generator("cuda").manual_seed(3)
+    xs = [torch.randn(4096, 4096, generator=g, device="cuda").to(BF16) for _ in range(3)]
+    w = (torch.randn(4096, 2048, generator=g, device="cuda") * 0.02).to(BF16)
+    want = [(x.double() @ w.double()) for x in xs]
+
+    def check(k, x):
+        out = f(_wrap(x), _wrap(w)).to_torch().double()
+        assert (out - want[k]).norm() < 4e-3 * want[k].norm()
+
+    for k, x in enumerate(xs):
+        check(k, x)
+    assert _taped(f) and f.stats.cuda_graphs == 0
+    check(1, xs[1].t().contiguous().t())
+    assert f.stats.cuda_graphs == 1
+    for k, x in enumerate(xs):
+        check(k, x)
+    small = nb.compile(lambda x, w: x @ w, cuda_graph=True)
+    for k in range(3):
+        out = small(_wrap(xs[k][:64]), _wrap(w[:, :64].contiguous())).to_torch().double()
+        assert torch.allclose(out, want[k][:64, :64], atol=0.1)
+    assert small.stats.cuda_graphs == 1 and _taped(small)
