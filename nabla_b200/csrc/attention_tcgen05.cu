@@ -29,6 +29,8 @@
 //   stored once as bf16: no atomics, no fp32 scratch, deterministic.
 // A small kernel before the backward computes delta = rowsum(dO * O) and log2-domain row
 // statistics padded to whole tiles.
+#include <cooperative_groups.h>
+
 #include "sm100_ptx.cuh"
 #include "nb_debug.cuh"
 
@@ -690,7 +692,7 @@ __global__ void __launch_bounds__(128) attn_fwd_combine_kernel(const FwdArgs arg
 // and V: no tile of 128 query rows, no tensor core; K and V go from global memory to registers, 16 bytes per
 // lane, HD / 8 lanes per key, DEC_U keys of K and of V in flight per lane, and every group of lanes keeps its
 // own running maximum, sum and output (fp32), joined at the end of the block and, over the key ranges
-// (gridDim.x), by attn_fwd_combine_kernel. 592 blocks (four per SM) of 4 x 16 B x 8 x 32 lanes hold the bytes
+// (gridDim.x), over the cluster or by attn_fwd_combine_kernel. 592 blocks (four per SM) of 4 x 16 B x 8 x 32 lanes hold the bytes
 // in flight that HBM needs. 64 heads, 1 query, 4001 keys of 128: 68 us with the tile kernel, 42 here with the join
 // (3.1 TB/s); 16 heads, 8000 keys: 120 -> 36 us.
 struct DecodeArgs {
@@ -700,9 +702,9 @@ struct DecodeArgs {
 };
 constexpr int DEC_MAX_Q = 4, DEC_U = 4;
 
-template <int HD, int NQ>
-__global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeArgs a) {
-  constexpr int LPK = HD / 8, KPW = 32 / LPK, G = 4 * KPW;      // lanes per key, keys per warp, lane groups per block
+template <int HD, int NQ, int WARPS, bool CLUSTER>
+__global__ void __launch_bounds__(32 * WARPS) attn_decode_kernel(const DecodeArgs a) {
+  constexpr int LPK = HD / 8, KPW = 32 / LPK, G = WARPS * KPW;      // lanes per key, keys per warp, lane groups per block
   const FwdArgs& f = a.f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LPK, d0 = (lane % LPK) * 8;
   const int grp = warp * KPW + sub;
@@ -794,9 +796,10 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeArgs a) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) so[grp][i][d0 + e] = acc[i][e];
   }
+  __shared__ float to[NQ][HD], tl[NQ];               // this block's range: output and log-sum-exp
   __syncthreads();
   const long long rows = (long long)f.B * f.H * f.Sq;
-  for (int t = threadIdx.x; t < NQ * HD; t += 128) {
+  for (int t = threadIdx.x; t < NQ * HD; t += 32 * WARPS) {
     const int i = t / HD, d = t % HD;
     if (i >= f.Sq) break;
     float mx = -INFINITY, sum = 0.f, o = 0.f;
@@ -814,13 +817,47 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeArgs a) {
     const float lse = have ? (mx + log2f(sum)) * 0.6931471805599453f : -INFINITY;
     const long long row = ((long long)b * f.H + h) * f.Sq + i;
     if (!NB_IN_BOUNDS(NB_SITE_ATTN_STORE, row, rows) || !NB_IN_BOUNDS(NB_SITE_ATTN_STORE, sp, f.nsplit)) continue;
-    if (f.nsplit > 1) {
+    if (CLUSTER) {
+      to[i][d] = o;
+      if (d == 0) tl[i] = lse;
+    } else if (f.nsplit > 1) {
       f.part_o[(sp * rows + row) * HD + d] = o;
       if (d == 0) f.part_lse[sp * rows + row] = lse;
     } else {
       f.O[b * f.o_sb + h * f.o_sh + i * f.o_ss + d] = __float2bfloat16(o);
       if (d == 0) f.lse[row] = lse;
     }
+  }
+  if (CLUSTER) {
+    // the ranges of a (batch, head) are the blocks of a cluster: every block joins its share of the outputs, as
+    // attn_fwd_combine_kernel does from memory
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    for (int t = sp * 32 * WARPS + threadIdx.x; t < NQ * HD; t += f.nsplit * 32 * WARPS) {
+      const int i = t / HD, d = t % HD;
+      if (i >= f.Sq) break;
+      float mx = -INFINITY;
+      bool nan = false;                              // a NaN range makes the row NaN (fmaxf would drop it)
+      for (int r = 0; r < f.nsplit; ++r) {
+        const float v = *cluster.map_shared_rank(&tl[i], r);
+        mx = fmaxf(mx, v);
+        nan |= v != v;
+      }
+      if (nan) mx = NAN;
+      float acc = 0.f, sum = 0.f;
+      if (mx != -INFINITY)
+        for (int r = 0; r < f.nsplit; ++r) {
+          const float w = ex2((*cluster.map_shared_rank(&tl[i], r) - mx) * LOG2E);
+          sum += w;
+          acc = fmaf(w, *cluster.map_shared_rank(&to[i][d], r), acc);
+        }
+      const bool have = !(sum <= 0.f);
+      const long long row = ((long long)b * f.H + h) * f.Sq + i;
+      if (!NB_IN_BOUNDS(NB_SITE_ATTN_STORE, row, rows)) continue;
+      f.O[b * f.o_sb + h * f.o_sh + i * f.o_ss + d] = __float2bfloat16(have ? acc / sum : 0.f);
+      if (d == 0) f.lse[row] = have ? mx + logf(sum) : -INFINITY;
+    }
+    cluster.sync();                                  // a block's shared memory is read until here
   }
 }
 
@@ -1622,14 +1659,37 @@ static void combine(const FwdArgs& a, cudaStream_t stream) {
   attn_fwd_combine_kernel<HD><<<(unsigned)((rows + 3) / 4), 128, 0, stream>>>(a);
 }
 
-template <int HD>
-static int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
+// Blocks of a cluster for so many warps on a (batch, head): of four warps, of eight above 32.
+static int dec_cluster(int warps) { return warps > 32 ? warps / 8 : warps / 4; }
+
+// warps 0: key ranges joined by a second launch.
+template <int HD, int NQ>
+static int launch_decode(const DecodeArgs& a, int warps, cudaStream_t stream) {
   const dim3 grid(a.f.nsplit, a.f.B * a.f.H);
-  if (a.f.Sq == 1) attn_decode_kernel<HD, 1><<<grid, 128, 0, stream>>>(a);
-  else if (a.f.Sq == 2) attn_decode_kernel<HD, 2><<<grid, 128, 0, stream>>>(a);
-  else attn_decode_kernel<HD, 4><<<grid, 128, 0, stream>>>(a);
-  if (a.f.nsplit > 1) combine<HD>(a.f, stream);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  if (warps == 0) {
+    attn_decode_kernel<HD, NQ, 4, false><<<grid, 128, 0, stream>>>(a);
+    if (a.f.nsplit > 1) combine<HD>(a.f, stream);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)a.f.nsplit;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(warps > 32 ? 256 : 128);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const auto kernel = warps > 32 ? attn_decode_kernel<HD, NQ, 8, true> : attn_decode_kernel<HD, NQ, 4, true>;
+  if (a.f.nsplit > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return -2;
+  return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? 0 : -3;
+}
+template <int HD>
+static int launch_decode(const DecodeArgs& a, int warps, cudaStream_t stream) {
+  return a.f.Sq == 1 ? launch_decode<HD, 1>(a, warps, stream) : a.f.Sq == 2 ? launch_decode<HD, 2>(a, warps, stream)
+                                                                            : launch_decode<HD, 4>(a, warps, stream);
 }
 
 template <int HD, UserMask MASK>
@@ -1716,11 +1776,28 @@ extern "C" int nb_attn_fwd_splits(int B, int H, int Sq, int Skv, int D, int has_
   return best;
 }
 
+// Warps that a (batch, head) of the decode kernel is given in a cluster of blocks, which needs no scratch and no second launch (0: key
+// ranges as above). Timed over 4 to 512 pairs, 64 to 8000 keys, one and two queries, both head_dims, every number of warps: as many as
+// leave a warp 8 keys, and as are resident (fewer registers' worth with two queries and in blocks of eight warps). What stays with the
+// ranges: chips that would be left half empty under long walks (us, ranges and clusters: 37 pairs x 4001 keys x 128, two queries 26.2,
+// 30.1), and few keys for many pairs (256 x 300 x 64 9.1, 9.9). us, ranges and clusters, one query: 4 pairs x 8000 keys x 128 21.6,
+// 13.6; 16 x 1000 12.2, 7.9; 32 x 4001 23.9, 19.7; 64 x 512 11.4, 8.8; 148 x 1000 23.3, 21.3; 300 x 4001 116, 114.
+extern "C" int nb_attn_decode_warps(int B, int H, int Sq, int Skv, int D, int has_mask) {
+  if (B <= 0 || H <= 0 || Sq <= 0 || Sq > 2 || Skv < 128 || !attn_decode(B, H, Sq, Skv, D, has_mask != 0)) return 0;
+  const long long bh = (long long)B * H;
+  auto most = [&](int w) { return Sq == 1 ? (w > 32 ? 2400 : 3200) : w > 64 ? 1024 : w > 32 ? 2048 : 2560; };
+  int w = 128;
+  while (w > 4 && (w * bh > most(w) || w * 8 > Skv)) w /= 2;
+  if (w < 8 || (bh > 148 && Skv < (D == 64 ? 512 : 300)) || (bh > 74 && D == 64 && Skv < 192) || (w * bh < 1900 && Skv > 100 * w)) return 0;
+  return w;
+}
+
 // q, k, v: bf16 (B, H, S, D) views, D contiguous, strides in elements (multiples of 8, 16-byte
 // aligned bases). o: bf16 with its own strides. lse: fp32 [B][H][Sq]. D in {64, 128}.
 // mask: optional fp32 additive mask (null = none), element strides m_sb, m_sh, m_sq (0 = broadcast),
 // key stride 1. nsplit = nb_attn_fwd_splits(...) or 1; above 1 part_o / part_lse are fp32 scratch of
-// nsplit * B * H * Sq * D and nsplit * B * H * Sq elements (16-byte aligned).
+// nsplit * B * H * Sq * D and nsplit * B * H * Sq elements (16-byte aligned). nsplit = -nb_attn_decode_warps(...) where that
+// is not 0.
 extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H, int Sq,
                            int Skv, int D, long long q_sb, long long q_sh, long long q_ss, long long k_sb,
                            long long k_sh, long long k_ss, long long v_sb, long long v_sh, long long v_ss,
@@ -1731,7 +1808,12 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   if (D != 64 && D != 128) return -10;
   if (!(scale > 0.f)) return -13;
   if (B <= 0 || H <= 0 || Sq <= 0) return 0;
-  if (nsplit < 1 || (nsplit > 1 && (part_o == nullptr || part_lse == nullptr || (reinterpret_cast<uintptr_t>(part_o) & 15)))) return -14;
+  const int warps = nsplit < 0 ? -nsplit : 0;
+  if (nsplit < 0) {
+    if ((warps != 8 && warps != 16 && warps != 32 && warps != 64 && warps != 128) || Skv <= 0 || !attn_decode(B, H, Sq, Skv, D, mask != nullptr))
+      return -14;
+    nsplit = dec_cluster(warps);
+  } else if (nsplit < 1 || (nsplit > 1 && (part_o == nullptr || part_lse == nullptr || (reinterpret_cast<uintptr_t>(part_o) & 15)))) return -14;
   const long long strides[] = {q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_ss, o_sh, o_sb};
   for (long long s : strides)
     if (s & 7) return -12;
@@ -1754,7 +1836,7 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   if (Skv > 0 && attn_decode(B, H, Sq, Skv, D, mask != nullptr)) {
     const DecodeArgs d{a, reinterpret_cast<const __nv_bfloat16*>(q), reinterpret_cast<const __nv_bfloat16*>(k),
                        reinterpret_cast<const __nv_bfloat16*>(v), q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss};
-    return D == 128 ? launch_decode<128>(d, s) : launch_decode<64>(d, s);
+    return D == 128 ? launch_decode<128>(d, warps, s) : launch_decode<64>(d, warps, s);
   }
   CUtensorMap tq, tk, tv;
   int r;

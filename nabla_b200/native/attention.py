@@ -16,13 +16,14 @@ import torch
 launch_count = 0
 _fwd = None
 _splits = None
+_warps = None
 _bwd = None
 _checked = False
 c_int, c_ll, c_f, c_vp = ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p
 
 
 def _lib():
-    global _fwd, _splits, _bwd, _checked
+    global _fwd, _splits, _warps, _bwd, _checked
     if not _checked:
         _checked = True
         from . import available, load
@@ -35,6 +36,9 @@ def _lib():
             lib.nb_attn_fwd_splits.restype = c_int
             lib.nb_attn_fwd_splits.argtypes = [c_int] * 6
             _splits = functools.lru_cache(1024)(lib.nb_attn_fwd_splits)      # a function of the sizes alone
+            lib.nb_attn_decode_warps.restype = c_int
+            lib.nb_attn_decode_warps.argtypes = [c_int] * 6
+            _warps = functools.lru_cache(1024)(lib.nb_attn_decode_warps)
             _fwd = f
             if hasattr(lib, "nb_attn_bwd"):
                 g = lib.nb_attn_bwd
@@ -121,8 +125,8 @@ def sdpa_fwd(q, k, v, *, causal: bool, scale: float, mask=None):
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
     st = status_word(q.device)
     m, m_sb, m_sh, m_sq = _mask_args(mask, B, H, Sq, Skv)
-    ns = _splits(B, H, Sq, Skv, D, int(m is not None))
-    # fp32 results of the key ranges: nsplit x (output, log-sum-exp)
+    ns = -_warps(B, H, Sq, Skv, D, int(m is not None)) or _splits(B, H, Sq, Skv, D, int(m is not None))
+    # fp32 results of the key ranges: nsplit x (output, log-sum-exp); a cluster of blocks (ns < 0) needs none
     part = torch.empty(ns * B * H * Sq * (D + 1), dtype=torch.float32, device=q.device) if ns > 1 else None
     p_o = 0 if part is None else part.data_ptr()
     p_lse = 0 if part is None else p_o + ns * B * H * Sq * D * 4
@@ -132,7 +136,7 @@ def sdpa_fwd(q, k, v, *, causal: bool, scale: float, mask=None):
               ptr(st), stream_ptr())
     if rc != 0:
         raise RuntimeError(f"nb_attn_fwd failed with code {rc}")
-    launch_count += 1 if ns == 1 else 2
+    launch_count += 1 if ns <= 1 else 2
     return o, lse
 
 

@@ -1464,3 +1464,26 @@ def test_compiled_adapters(M, scale):
     for g, r in zip(got, (ref, *torch.autograd.grad(ref, d, dy.double()))):
         assert _rel2(g, r.detach()) < 2 * STORED[torch.bfloat16]
     assert sum("+gemm_residual" in line for line in f.dump_plan().splitlines()) == 2
+
+
+@pytest.mark.parametrize("B,H,Sq,Skv,D,warps", [(1, 4, 1, 127, 64, 0), (1, 4, 1, 128, 64, 16), (1, 16, 1, 1023, 128, 64), (1, 3, 2, 8001, 64, 128), (2, 32, 1, 4001, 128, 32),
+                                                (4, 16, 2, 300, 128, 32), (37, 1, 2, 3300, 64, 0), (50, 3, 1, 700, 64, 16), (100, 3, 1, 513, 128, 8),
+                                                (16, 10, 2, 400, 64, 0), (401, 1, 1, 2000, 64, 0), (1, 4, 3, 128, 64, 0)])
+def test_few_queries_over_clusters(B, H, Sq, Skv, D, warps):
+    """Both sides of the rule's lines and every number of warps; a NaN key shows, an unseen one does not."""
+    from nabla_b200.native import attention
+
+    attention._lib()
+    assert attention._warps(B, H, Sq, Skv, D, 0) == warps and attention._warps(B, H, Sq, Skv, D, 1) == 0
+    torch.manual_seed(29)
+    q = torch.randn(B, H, Sq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(B, H, Skv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    for causal in (False, True):
+        o, lse = attention.sdpa_fwd(q, k, v, causal=causal, scale=D ** -0.5)
+        s = (q.double() @ k.double().transpose(-1, -2)) * D ** -0.5
+        if causal:
+            s = s.masked_fill(~torch.ones(Sq, Skv, dtype=torch.bool, device="cuda").tril(Skv - Sq), float("-inf"))
+        assert _rel2(o, torch.softmax(s, -1) @ v.double()) < 1.85e-3 and _rel2(lse, torch.logsumexp(s, -1)) < 1e-5
+    k[0, 0, Skv - 1, 0] = float("nan")
+    o, _ = attention.sdpa_fwd(q, k, v, causal=True, scale=D ** -0.5)
+    assert o[0, 0, -1].isnan().all() and not o[0, 0, :-1].isnan().any() and not o.reshape(-1, Sq, D)[1:].isnan().any()
