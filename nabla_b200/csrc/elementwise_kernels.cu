@@ -476,6 +476,7 @@ static bool thin_reduce(long long outer, long long R, long long inner, int V) {
   return R <= 256 && inner % V == 0 && threads >= 148 * 256 && (threads + THIN_THREADS - 1) / THIN_THREADS <= 0x7fffffffll;
 }
 
+// scratch (splits > 1): 3 * outer * splits * inner + 1 floats.
 int nb_reduce(const void* x, void* out, void* scratch, long long outer, long long R, long long inner, int op, int dtype,
               void* stream) {
   if (outer <= 0 || inner <= 0 || R <= 0) return 0;
@@ -510,7 +511,7 @@ int nb_reduce(const void* x, void* out, void* scratch, long long outer, long lon
   const long long tiles = outer * ((inner + 31) / 32);
   const dim3 grid((unsigned)(tiles < 148 * 16 ? tiles : 148 * 16), splits);
   float* pv = reinterpret_cast<float*>(scratch);
-  long long* pi = reinterpret_cast<long long*>(pv + outer * splits * inner);
+  long long* pi = reinterpret_cast<long long*>(pv + (outer * splits * inner + 1) / 2 * 2);      // on an 8-byte boundary
   const int fgrid = grid_for((size_t)(outer * inner), 256);
 #define NB_COL(T, O) do { \
     col_reduce_kernel<T, O><<<grid, 256, 0, STREAM>>>((const T*)x, (O*)out, pv, pi, outer, R, inner, op, splits); \

@@ -794,7 +794,7 @@ def reduce(x: torch.Tensor, axis: int, op: str, keepdims: bool = False):
         shape.pop(axis)
     out = torch.empty(shape, dtype=torch.int64 if op.startswith("arg") else x.dtype, device=x.device)
     splits = _L().nb_reduce_splits(outer, r, inner)
-    scratch = torch.empty(outer * splits * inner * 3, dtype=torch.float32, device=x.device) if splits > 1 else None
+    scratch = torch.empty(outer * splits * inner * 3 + 1, dtype=torch.float32, device=x.device) if splits > 1 else None
     _ok(_L().nb_reduce(ptr(xc), ptr(out), ptr(scratch), outer, r, inner, REDUCE_OPS[op], _dt(xc), stream_ptr()), "reduce")
     return out
 

@@ -1187,6 +1187,18 @@ def test_narrow_column_sums_are_short_chains(rows, N):
     assert torch.equal(kernels.colsum(x), ref)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,inner", [(200, 5), (192, 3), (700, 7), (128, 33)])
+def test_reductions_in_an_odd_number_of_parts(dtype, rows, inner):
+    """An odd number of partial results: their positions, 8 bytes each, lie behind them in the scratch."""
+    from nabla_b200.native import kernels
+
+    torch.manual_seed(31)
+    x = torch.randn(rows, inner, device="cuda").to(dtype)
+    assert _rel2(kernels.reduce(x, 0, "sum"), x.double().sum(0)) < STORED[dtype]
+    assert torch.equal(kernels.reduce(x, 0, "max"), x.amax(0)) and torch.equal(kernels.reduce(x, 0, "argmax"), x.argmax(0))
+
+
 # ---------------------------------------------------------------- pooling
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("mode", ["max", "avg"])
