@@ -29,6 +29,8 @@ CUDA bf16 tensors:
   ``adamw_reduce`` steps, set up by ``transforms/compile.py``).
 * ``all_gather(rows) -> linear | matmul [-> dact_mul]``: one launch that pulls the peers' rows while the tensor
   cores already work on the rows that are there; the gathered tensor is still produced.
+* ``conv2d -> relu`` whose pre-activation is read by nothing but the relu's derivative, and ``max pooling backward -> relu's derivative``:
+  one launch each (compiled replays).
 * ``zeros -> scatter-add``: the gradient of an embedding table without the table of zeros.
 * ``gather -> add`` of a tensor over the trailing dims (token plus position embedding): one pass (compiled replays).
 * ``adamw_group``: the updates of small parameters with the same hyperparameters, one launch at the end of a compiled
@@ -146,6 +148,25 @@ def build_plan(nodes: list[OpNode], targets: list[TensorImpl], private: bool = F
                 if not used[j] and _is_scatter_add_into(nodes[j], o):
                     chain = [i, j]
                     kind = "scatter_zeros"
+        if chain is None and private and n.op.name == "conv2d":
+            k = _relu_behind(n, nodes, cons, target_ids)
+            if k is not None and not used[k]:
+                used[i] = used[k] = True
+                steps.append((i, ("conv_relu", (i, k))))
+                continue
+        if chain is None and private and n.op.name == "pool2d_bwd" and n.kwargs.get("mode") == "max" and _is_plain_gpu(n):
+            o = sole_output(n)
+            if private_intermediate(o):
+                k = cons[id(o)][0]
+                d = nodes[k]
+                x = n.input_impls()[0]
+                if not used[k] and d.op.name == "dact_mul" and d.kwargs.get("activation") == "relu" and d.input_impls()[0] is o \
+                        and len(d.input_impls()) == 2:
+                    z = d.input_impls()[1]
+                    p = nodes[producer[id(x)]] if id(x) in producer else None
+                    if z is x or (p is not None and p.op.name == "relu" and p.input_impls()[0] is z):
+                        chain = [i, k]
+                        kind = "pool_bwd_relu"
         if chain is None and private and n.op.name == "sub":
             idxs = _mean_of_difference(i, nodes, cons, target_ids, used, producer, private_intermediate)
             if idxs is not None:
@@ -347,6 +368,32 @@ def _is_cuda_bf16_2d(n: OpNode) -> bool:
 
     return (a.device.label == "gpu" and a.dtype is DType.bfloat16 and b.dtype is DType.bfloat16
             and len(b._shape) == 2 and len(a._shape) >= 2)
+
+
+def _is_plain_gpu(n: OpNode) -> bool:
+    """Unsharded fp32 / bf16 GPU operands of one type and the result too."""
+    from ...types import DType
+
+    xs = [*n.input_impls(), *n.outputs()]
+    return all(x is not None and x.sharding is None and not x.batch_dims and x.device.label == "gpu" and x.dtype is xs[0].dtype for x in xs) \
+        and xs[0].dtype in (DType.bfloat16, DType.float32)
+
+
+def _relu_behind(n: OpNode, nodes, cons, target_ids) -> int | None:
+    """The relu behind ``n`` when its result z is read by nothing else but derivatives of a relu: those ask whether z is above 0,
+    which the relu's own result answers as well, so z need not exist."""
+    outs = n.outputs()
+    z = outs[0] if len(outs) == 1 else None
+    if z is None or id(z) in target_ids or not _is_plain_gpu(n):
+        return None
+    relus = []
+    for j in dict.fromkeys(cons.get(id(z), [])):
+        m = nodes[j]
+        if m.op.name == "relu" and len(m.input_impls()) == 1:
+            relus.append(j)
+        elif not (m.op.name == "dact_mul" and m.kwargs.get("activation") == "relu" and m.input_impls()[1] is z and m.input_impls()[0] is not z):
+            return None
+    return relus[0] if len(relus) == 1 and nodes[relus[0]].outputs()[0] is not None else None
 
 
 def _is_plain_binary(n: OpNode) -> bool:
@@ -790,6 +837,34 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         else:
             for n_ in group:
                 _plain(n_, keep_graph)
+        return
+    if kind == "conv_relu":
+        from ...ops.convolution import _conv_fwd, _own_kernels
+
+        conv, relu = group
+        ins = [t._buffers[0] for t in conv.input_impls()]
+        if _own_kernels(ins[0]):
+            out = _conv_fwd(ins[0], ins[1], ins[2] if len(ins) > 2 else None, conv.kwargs["stride"], conv.kwargs["padding"], relu=True)
+            _store(conv, [[out]], keep_graph)           # for the relu's derivative, which is all that reads it
+            _store(relu, [[out]], keep_graph)
+        else:
+            _plain(conv, keep_graph)
+            _plain(relu, keep_graph)
+        return
+    if kind == "pool_bwd_relu":
+        from ...native import kernels
+        from ...ops.convolution import _fold
+        from ...ops.pooling import _native_ok
+
+        pool, dact = group
+        x, dy = [t._buffers[0] for t in pool.input_impls()]
+        (kh, kw), (sh, sw), (pt, pb, pl, pr) = pool.kwargs["kernel_size"], pool.kwargs["stride"], pool.kwargs["padding"]
+        x4, dy4 = _fold(x)[0], _fold(dy)[0]
+        if _native_ok(x4) and pt == pb and pl == pr and dy4.dtype == x4.dtype:
+            _store(dact, [[kernels.pool2d_bwd(x4, dy4, kh, kw, sh, sw, pt, pl, "max", relu=True).reshape(x.shape)]], keep_graph)
+        else:
+            _plain(pool, keep_graph)
+            _plain(dact, keep_graph)
         return
     if kind == "mean_diff":
         from ... import native

@@ -1824,7 +1824,9 @@ __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restric
   }
   store_vec<T>(y + (size_t)i * V, acc);
 }
-template <typename T, bool MAX>
+// RELU: x came out of a relu, and its derivative is applied too (what reaches a maximum of 0 or less is multiplied by 0). As a pass of its
+// own it read and wrote all of x's size: 256 x 28 x 28 x 16 fp32 5.4 + 4.7 us, 5.7 so.
+template <typename T, bool MAX, bool RELU = false>
 __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dx,
                                                              const CellGeom g, unsigned total) {
   constexpr int V = Vec<T>::N;
@@ -1854,6 +1856,10 @@ __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restric
             if (v[j] > best[j]) { best[j] = v[j]; where[j] = a * g.kw + b; }
         }
     }
+  }
+  if (RELU) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) d[j] *= best[j] > 0.f ? 1.f : 0.f;
   }
   const float inv = 1.f / (g.kh * g.kw);
   for (int a = 0; a < hh; ++a)
@@ -1912,7 +1918,7 @@ __global__ void __launch_bounds__(256) pool2d_select_kernel(const T* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(256) pool2d_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                         T* __restrict__ dx, int N, int H, int W, int C, int OH,
-                                                        int OW, int kh, int kw, int sh, int sw, int ph, int pw, int mode) {
+                                                        int OW, int kh, int kw, int sh, int sw, int ph, int pw, int mode, int relu) {
   const size_t total = (size_t)N * H * W * C;
   const float inv = 1.f / (kh * kw);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -1947,7 +1953,7 @@ __global__ void __launch_bounds__(256) pool2d_bwd_kernel(const T* __restrict__ x
           if (bh == ih && bw == iw) acc += g;
         }
       }
-    dx[i] = from_f<T>(acc);
+    dx[i] = from_f<T>(relu ? acc * (to_f<T>(x[i]) > 0.f ? 1.f : 0.f) : acc);
   }
 }
 
@@ -1967,6 +1973,15 @@ __global__ void __launch_bounds__(256) pool2d_bwd_kernel(const T* __restrict__ x
 struct ConvGeom {
   int N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl;
 };
+
+// The filter of an input gradient: out[r][s][f][c] = w[R - 1 - r][S - 1 - s][c][f].
+template <typename T>
+__global__ void __launch_bounds__(256) conv_flip_kernel(const T* __restrict__ w, T* __restrict__ out, int taps, int C, int F, unsigned n) {
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= n || !NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, i, n)) return;
+  const unsigned c = i % C, q = i / C, f = q % F, t = q / F;
+  out[i] = w[((size_t)(taps - 1 - t) * C + c) * F + f];
+}
 
 template <typename T>
 __device__ __noinline__ float conv_point(const T* __restrict__ x, const T* __restrict__ w, float acc, const ConvGeom g,
@@ -2020,9 +2035,10 @@ __device__ __forceinline__ ConvTap conv_tap(int k, const ConvGeom& g) {
   return ConvTap{r, s, ((long long)r * g.W + s) * g.C + (k - rs * g.C)};
 }
 
+// relu: below 0 becomes 0, NaN stays.
 template <typename T, int FG, bool VEC>
 __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                           const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g) {
+                                                           const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g, int relu) {
   constexpr int PG = 128 / FG, MT = 2 * PG, FT = 4 * FG, PER = (MT + 127) / 128, KSTEP = MT < 128 ? 128 / MT : 1;
   __shared__ __align__(16) float xs[CONV_KC][MT + 4];
   __shared__ __align__(16) float ws[CONV_KC][FT];
@@ -2117,6 +2133,7 @@ __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict_
       const int f = f0 + fg * 4 + j;
       if (f >= g.F) break;
       if (odd) acc[i][j] = conv_point<T>(x, w, bias ? to_f<T>(bias[f]) : 0.f, g, m, f);
+      if (relu && acc[i][j] < 0.f) acc[i][j] = 0.f;
       y[m * g.F + f] = from_f<T>(acc[i][j]);
     }
   }
@@ -2153,16 +2170,17 @@ __device__ __forceinline__ void stage_patch(const T* __restrict__ image, float* 
 
 // The same sums from a patch: a block stages the input of TH rows of one image's output once, with its halo, and the whole
 // filter tile, and walks (r, s, c) by addresses, where the kernel above stages every input value once per filter tap. A
-// thread has PX positions (lanes take consecutive ones) and 4 channels; VEC: four input channels per shared load, kept as
-// float4 planes so that lanes read consecutive ones. The additions are those of the kernel above, in its order: the same bits.
-// Bound by the shared-memory pipe (71 % of its active time) under 2 PX + 4 wavefronts per 16 PX FMAs, and by the staging before
-// them; 128 registers, so that 512 blocks run at once. us, tiled and from patches, fp32, 3 x 3: 256 x 14 x 14 x 16 -> 32
-// 28.8, 23.2; 256 x 14 x 14 x 32 -> 16 (an input gradient) 40.2, 24.9; 256 x 28 x 28 x 1 -> 16 14.0, 12.5; 16 x 32 x 32 x 8 -> 16
-// 7.5, 5.5; bf16 within a tenth of these.
+// thread has PX positions and 4 channels, the FG channel groups of a position in neighbouring lanes: a warp's loads of input are then
+// few distinct 16-byte pieces, its stores whole rows, and PX + 4 wavefronts serve 16 PX FMAs (with consecutive positions in
+// neighbouring lanes 2 PX + 4 and half-used sectors: 71 % of the shared-memory pipe). The FMAs go two channels at a time. VEC: four
+// input channels per shared load, kept as float4 planes. The additions are those of the kernel above, in its order: the same bits.
+// Bound by the staging, which all blocks do at the same time, and then by issue; 128 registers, so that 512 blocks run at once. us, tiled,
+// from patches with positions in neighbouring lanes, and so, fp32, 3 x 3: 256 x 14 x 14 x 16 -> 32 28.8, 23.7, 20.9; 256 x 14 x 14 x 32 -> 16
+// (an input gradient) 40.2, 25.5, 22.5; 256 x 28 x 28 x 1 -> 16 14.0, 13.1, 11.2.
 template <typename T, int FG, int PX, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                           const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g,
-                                                          int TH, int bands, int wvec, int yvec) {
+                                                          int TH, int bands, int wvec, int yvec, int relu) {
   constexpr int PG = 128 / FG, FT = 4 * FG, KV = VEC ? 4 : 1;
   extern __shared__ __align__(16) float conv_smem[];
   const int tid = threadIdx.x, K = g.R * g.S * g.C, CQ = g.C / KV;
@@ -2190,17 +2208,17 @@ __global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restric
     }
   }
   stage_patch<T, VEC>(x + (size_t)n * g.H * g.W * g.C, xs, g, n, oh0 * g.sh - g.pt, -g.pl, ph, pw, 0, CQ);
-  const int pg = tid % PG, fg = tid / PG;
+  const int fg = tid % FG, pg = tid / FG;
   int at[PX];
-  float acc[PX][4];
+  float2 acc[PX][2];                                 // four channels in two pairs
 #pragma unroll
   for (int i = 0; i < PX; ++i) {
     const int p = pg + i * PG, r = p / g.OW, c = p - r * g.OW;
     at[i] = r < TH ? r * g.sh * pw + c * g.sw : 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int f = f0 + fg * 4 + j;
-      acc[i][j] = bias && f < g.F ? to_f<T>(bias[f]) : 0.f;
+    for (int j = 0; j < 2; ++j) {
+      const int f = f0 + fg * 4 + 2 * j;
+      acc[i][j] = make_float2(bias && f < g.F ? to_f<T>(bias[f]) : 0.f, bias && f + 1 < g.F ? to_f<T>(bias[f + 1]) : 0.f);
     }
   }
   __syncthreads();
@@ -2225,10 +2243,9 @@ __global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restric
           wp += FT;
 #pragma unroll
           for (int i = 0; i < PX; ++i) {
-            acc[i][0] = fmaf(a[i][k], b.x, acc[i][0]);
-            acc[i][1] = fmaf(a[i][k], b.y, acc[i][1]);
-            acc[i][2] = fmaf(a[i][k], b.z, acc[i][2]);
-            acc[i][3] = fmaf(a[i][k], b.w, acc[i][3]);
+            const float2 t = make_float2(a[i][k], a[i][k]);
+            acc[i][0] = __ffma2_rn(t, make_float2(b.x, b.y), acc[i][0]);
+            acc[i][1] = __ffma2_rn(t, make_float2(b.z, b.w), acc[i][1]);
           }
         }
       }
@@ -2238,16 +2255,22 @@ __global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restric
     const int p = pg + i * PG, r = p / g.OW, c = p - r * g.OW, oh = oh0 + r, f = f0 + fg * 4;
     if (r >= TH || oh >= g.OH || f >= g.F) continue;
     const long long m = ((long long)n * g.OH + oh) * g.OW + c;
+    float v[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
     if (odd) {
-      for (int j = 0; j < 4 && f + j < g.F; ++j) acc[i][j] = conv_point<T>(x, w, bias ? to_f<T>(bias[f + j]) : 0.f, g, m, f + j);
+      for (int j = 0; j < 4 && f + j < g.F; ++j) v[j] = conv_point<T>(x, w, bias ? to_f<T>(bias[f + j]) : 0.f, g, m, f + j);
+    }
+    if (relu) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (v[j] < 0.f) v[j] = 0.f;
     }
     T* o = y + m * g.F + f;
     if (yvec) {
-      store4(o, acc[i]);
+      store4(o, v);
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (f + j < g.F) o[j] = from_f<T>(acc[i][j]);
+        if (f + j < g.F) o[j] = from_f<T>(v[j]);
     }
   }
 }
@@ -3081,22 +3104,23 @@ int nb_pool2d_fwd(const void* x, void* y, int N, int H, int W, int C, int OH, in
   return CHECK_LAUNCH();
 }
 int nb_pool2d_bwd(const void* x, const void* dy, void* dx, int N, int H, int W, int C, int OH, int OW, int kh, int kw,
-                  int sh, int sw, int ph, int pw, int mode, int dtype, void* stream) {
+                  int sh, int sw, int ph, int pw, int mode, int relu, int dtype, void* stream) {
   const size_t total = (size_t)N * H * W * C;
   if (!total) return 0;
+  if (relu && mode != 1) return -2;
   const int V = dtype ? 8 : 4;
   CellGeom g;
   if (pool_cells(x, dy, dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g) && (mode == 1 || pool_cells_avg_bwd(N, C, g))) {
     const unsigned n = (unsigned)((size_t)N * g.cells_h * g.cells_w * g.CV);
-#define POOL(T, MAX) pool2d_cell_bwd_kernel<T, MAX><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (const T*)dy, (T*)dx, g, n)
-    if (dtype) { if (mode) POOL(bf16, true); else POOL(bf16, false); }
-    else { if (mode) POOL(float, true); else POOL(float, false); }
+#define POOL(T, ...) pool2d_cell_bwd_kernel<T, __VA_ARGS__><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (const T*)dy, (T*)dx, g, n)
+    if (dtype) { if (relu) POOL(bf16, true, true); else if (mode) POOL(bf16, true); else POOL(bf16, false); }
+    else { if (relu) POOL(float, true, true); else if (mode) POOL(float, true); else POOL(float, false); }
 #undef POOL
     return CHECK_LAUNCH();
   }
   const int grid = grid_for(total, 256);
-  if (dtype) pool2d_bwd_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (const bf16*)dy, (bf16*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
-  else pool2d_bwd_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (const float*)dy, (float*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
+  if (dtype) pool2d_bwd_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (const bf16*)dy, (bf16*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode, relu);
+  else pool2d_bwd_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (const float*)dy, (float*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode, relu);
   return CHECK_LAUNCH();
 }
 
@@ -3153,8 +3177,17 @@ int nb_conv2d_patches(int N, int H, int W, int C, int R, int S, int F, int OH, i
   return conv_patches(ConvGeom{N, H, W, C, R, S, F, OH, OW, sh, sw, 0, 0}, C % 4 == 0, F % 4 == 0).px;
 }
 
+int nb_conv_flip(const void* w, void* out, int R, int S, int C, int F, int dtype, void* stream) {
+  const long long n = (long long)R * S * C * F;
+  if (n <= 0) return 0;
+  if (n > 0x7fffffffll) return -2;
+  const unsigned grid = (unsigned)((n + 255) / 256);
+  if (dtype) conv_flip_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)w, (bf16*)out, R * S, C, F, (unsigned)n);
+  else conv_flip_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)w, (float*)out, R * S, C, F, (unsigned)n);
+  return CHECK_LAUNCH();
+}
 int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int R, int S,
-                     int F, int OH, int OW, int sh, int sw, int pt, int pl, int dtype, void* stream) {
+                     int F, int OH, int OW, int sh, int sw, int pt, int pl, int relu, int dtype, void* stream) {
   const size_t positions = (size_t)N * OH * OW;
   if (!positions || !F) return 0;
   const ConvGeom g{N, H, W, C, R, S, F, OH, OW, sh, sw, pt, pl};
@@ -3170,7 +3203,7 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
     const int px = pp.px, th = pp.th, bands = pp.bands, fg_w = pp.fg;
     const size_t smem = 4 * ((size_t)R * S * C * 4 * fg_w + (size_t)((th - 1) * sh + R) * ((OW - 1) * sw + S) * C);
     const dim3 pgrid((unsigned)(N * bands), (unsigned)pp.f_tiles);
-#define PATCH_V(T, FG, PX, VEC) conv2d_patch_kernel<T, FG, PX, VEC><<<pgrid, 128, smem, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec)
+#define PATCH_V(T, FG, PX, VEC) conv2d_patch_kernel<T, FG, PX, VEC><<<pgrid, 128, smem, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec, relu)
 #define PATCH_P(T, FG, PX) do { if (vec) PATCH_V(T, FG, PX, true); else PATCH_V(T, FG, PX, false); } while (0)
 #define PATCH(T, FG) do { if (px == 8) PATCH_P(T, FG, 8); else PATCH_P(T, FG, 4); } while (0)
     if (dtype) { if (fg_w == 2) PATCH(bf16, 2); else if (fg_w == 4) PATCH(bf16, 4); else PATCH(bf16, 8); }
@@ -3180,7 +3213,7 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
 #undef PATCH_V
     return CHECK_LAUNCH();
   }
-#define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<grid(FG), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g)
+#define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<grid(FG), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, relu)
 #define CONV(T, FG) do { if (vec) CONV_V(T, FG, true); else CONV_V(T, FG, false); } while (0)
   if (dtype) { if (F <= 8) CONV(bf16, 2); else if (F <= 16) CONV(bf16, 4); else CONV(bf16, 8); }
   else { if (F <= 8) CONV(float, 2); else if (F <= 16) CONV(float, 4); else CONV(float, 8); }

@@ -49,9 +49,10 @@ def _L():
             "nb_nf4_dequant": [c_vp] * 3 + [c_ll, c_int, c_int, c_vp],
             "nb_nf4_dequant_codes": [c_vp] * 4 + [c_ll, c_int, c_int, c_vp],
             "nb_pool2d_fwd": [c_vp, c_vp] + [c_int] * 14 + [c_vp],
-            "nb_pool2d_bwd": [c_vp] * 3 + [c_int] * 14 + [c_vp],
+            "nb_pool2d_bwd": [c_vp] * 3 + [c_int] * 15 + [c_vp],
             "nb_pool2d_select": [c_vp] * 3 + [c_int] * 13 + [c_vp],
-            "nb_conv2d_direct": [c_vp] * 4 + [c_int] * 14 + [c_vp],
+            "nb_conv2d_direct": [c_vp] * 4 + [c_int] * 15 + [c_vp],
+            "nb_conv_flip": [c_vp] * 2 + [c_int] * 5 + [c_vp],
             "nb_conv2d_wgrad_slices": [c_ll, c_int, c_int],
             "nb_conv2d_wgrad_direct": [c_vp] * 4 + [c_int] * 14 + [c_vp],
             "nb_sgemm_slices": [c_int] * 3,
@@ -546,14 +547,15 @@ def pool2d_fwd(x, kh, kw, sh, sw, ph, pw, mode: str):
     return y
 
 
-def pool2d_bwd(x, dy, kh, kw, sh, sw, ph, pw, mode: str):
+def pool2d_bwd(x, dy, kh, kw, sh, sw, ph, pw, mode: str, relu: bool = False):
+    """``relu`` (max pooling): x is the output of a relu, whose derivative is applied to the gradient in the same pass."""
     x = x.contiguous()
     dy = dy.contiguous()
     N, H, W, C = x.shape
     _, OH, OW, _ = dy.shape
     dx = torch.empty_like(x)
     _ok(_L().nb_pool2d_bwd(ptr(x), ptr(dy), ptr(dx), N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw,
-                           0 if mode == "avg" else 1, _dt(x), stream_ptr()), "pool2d_bwd")
+                           0 if mode == "avg" else 1, int(relu), _dt(x), stream_ptr()), "pool2d_bwd")
     return dx
 
 
@@ -570,7 +572,16 @@ def pool2d_select(x, t, kh, kw, sh, sw, ph, pw):
     return y
 
 
-def conv2d_direct(x, w, bias, stride, padding):
+def conv_flip(w: torch.Tensor) -> torch.Tensor:
+    """(R, S, C, F) filter -> (R, S, F, C), turned around in both of the first dims: the filter of the input gradient."""
+    R, S, C, F = w.shape
+    w = w.contiguous()
+    out = torch.empty((R, S, F, C), dtype=w.dtype, device=w.device)
+    _ok(_L().nb_conv_flip(ptr(w), ptr(out), R, S, C, F, _dt(w), stream_ptr()), "conv_flip")
+    return out
+
+
+def conv2d_direct(x, w, bias, stride, padding, relu: bool = False):
     """NHWC x RSCF direct convolution; padding = (top, bottom, left, right)."""
     x = x.contiguous()
     w = w.contiguous().to(x.dtype)
@@ -582,7 +593,7 @@ def conv2d_direct(x, w, bias, stride, padding):
     y = torch.empty((N, OH, OW, F), dtype=x.dtype, device=x.device)
     b = bias.contiguous().to(x.dtype).view(-1) if bias is not None else None
     _ok(_L().nb_conv2d_direct(ptr(x), ptr(w), ptr(b), ptr(y), N, H, W, C, R, S, F, OH, OW, stride[0], stride[1], pt, pl,
-                              _dt(x), stream_ptr()), "conv2d_direct")
+                              int(relu), _dt(x), stream_ptr()), "conv2d_direct")
     return y
 
 

@@ -52,7 +52,8 @@ def _fold(x: torch.Tensor):
     return x.reshape(-1, *x.shape[-3:]), lead
 
 
-def _conv_fwd(x, w, bias, stride, padding):
+def _conv_fwd(x, w, bias, stride, padding, relu: bool = False):
+    """``relu`` (GPU only): followed by a relu, where the direct convolution serves in the same launch."""
     from .. import native
 
     x4, lead = _fold(x)
@@ -69,8 +70,10 @@ def _conv_fwd(x, w, bias, stride, padding):
             cols = xp.unfold(1, R, stride[0]).unfold(2, S, stride[1])          # N,OH,OW,C,R,S
             cols = cols.permute(0, 1, 2, 4, 5, 3).reshape(N * OH * OW, R * S * C)
             y = native.gemm_bf16(cols, w.reshape(R * S * C, F), bias=bias)
+            if relu:                                # (the epilogue's relu makes NaN 0)
+                y = torch.relu(y)
             return y.reshape(*lead, OH, OW, F)
-        y = kernels.conv2d_direct(x4, w, bias, stride, padding)
+        y = kernels.conv2d_direct(x4, w, bias, stride, padding, relu)
         return y.reshape(*lead, *y.shape[1:])
     xp = TF.pad(x4.permute(0, 3, 1, 2), (pl, pr, pt, pb))
     y = TF.conv2d(xp, w.permute(3, 2, 0, 1).to(xp.dtype), bias=None if bias is None else bias.to(xp.dtype), stride=stride)
@@ -104,7 +107,9 @@ def _dgrad_as_conv(dy4: torch.Tensor, w: torch.Tensor, out_hw, stride, padding) 
     if min(top, left, bottom, right) < 0:          # padding larger than the filter reach: crop instead
         z = z[:, max(0, -top): hz - max(0, -bottom), max(0, -left): wz - max(0, -right)]
         top, left, bottom, right = max(0, top), max(0, left), max(0, bottom), max(0, right)
-    wf = w.flip(0, 1).permute(0, 1, 3, 2).contiguous()      # (R, S, F, C): in-channels F, out-channels C
+    from ..native import kernels
+
+    wf = kernels.conv_flip(w)                               # (R, S, F, C): in-channels F, out-channels C
     return _conv_fwd(z, wf, None, (1, 1), (top, bottom, left, right))
 
 

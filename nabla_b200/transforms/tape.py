@@ -23,7 +23,7 @@ from ..core.tensor.impl import TensorImpl
 # launch functions: all of their effects are on the device and on the stream that is their last argument
 LAUNCHES = frozenset("""nb_gemm_bf16 nb_gemm_dual_bf16 nb_attn_fwd nb_attn_bwd nb_layernorm_fwd nb_layernorm_bwd nb_colsum nb_colsum_group nb_softmax
     nb_lse_pick_fwd nb_lse_pick_bwd nb_adamw nb_adamw_group nb_adam_hyper nb_mean_diff nb_sgd nb_embedding_gather nb_embedding_scatter_add
-    nb_cast nb_activation nb_nf4_dequant nb_nf4_dequant_codes nb_pool2d_fwd nb_pool2d_bwd nb_pool2d_select nb_conv2d_direct
+    nb_cast nb_activation nb_nf4_dequant nb_nf4_dequant_codes nb_pool2d_fwd nb_pool2d_bwd nb_pool2d_select nb_conv2d_direct nb_conv_flip
     nb_conv2d_wgrad_direct nb_sgemm nb_sum_slices nb_binary nb_unary nb_reduce nb_cumsum""".split())
 # functions of sizes alone
 QUERIES = frozenset("""nb_layernorm_bwd_nblocks nb_colsum_nparts nb_conv2d_wgrad_slices nb_sgemm_slices nb_reduce_splits

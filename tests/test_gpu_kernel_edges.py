@@ -1499,3 +1499,46 @@ def test_few_queries_over_clusters(B, H, Sq, Skv, D, warps):
     k[0, 0, Skv - 1, 0] = float("nan")
     o, _ = attention.sdpa_fwd(q, k, v, causal=True, scale=D ** -0.5)
     assert o[0, 0, -1].isnan().all() and not o[0, 0, :-1].isnan().any() and not o.reshape(-1, Sq, D)[1:].isnan().any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,H,C,F,k,pool,stride", [(3, 12, 1, 8, 3, 2, 2), (2, 11, 4, 12, 3, 2, 2), (2, 9, 3, 5, 2, 3, 2), (5, 16, 8, 32, 3, 2, 2)])
+def test_compiled_convolutions_take_their_relu(dtype, N, H, C, F, k, pool, stride):
+    """Convolution, relu, max pooling (windows apart and overlapping) and all gradients, compiled against plain; and NaN as a plain relu has it."""
+    import nabla_b200 as nb
+
+    torch.manual_seed(30)
+    x, w, b = ((torch.randn(s, device="cuda") * std).to(dtype) for s, std in (((N, H, H, C), 1.0), ((k, k, C, F), 0.3), ((F,), 0.3)))
+
+    def net(x, w, b):
+        h = nb.max_pool2d(nb.relu(nb.conv2d(x, w, bias=b, padding=1)), pool, stride)
+        return h * 1.5
+
+    def step(x, w, b, dy):
+        y, pull = nb.vjp(net, x, w, b, create_graph=False)
+        return (y, *pull(dy))
+
+    ts = [nb.Tensor.from_torch(t) for t in (x, w, b)]
+    dy = nb.Tensor.from_torch(torch.randn_like(net(*ts).to_torch()))
+    f = nb.compile(step)
+    got = [[t.to_torch() for t in f(*ts, dy)] for _ in range(3)][-1]
+    plan = f.dump_plan()
+    assert plan.count("conv_relu") == 1 and plan.count("pool_bwd_relu") == 1
+    for a, c in zip(got, step(*ts, dy)):
+        assert _rel2(a, c.to_torch()) < 4 * STORED[dtype]
+    assert torch.equal(got[0], net(*ts).to_torch())
+    x[0, 0, 0, 0] = float("nan")
+    g = nb.compile(lambda x, w, b: nb.relu(nb.conv2d(x, w, bias=b, padding=1)))
+    for _ in range(2):
+        y = g(nb.Tensor.from_torch(x), *ts[1:]).to_torch()
+        assert torch.equal(y.isnan(), nb.relu(nb.conv2d(nb.Tensor.from_torch(x), ts[1], bias=ts[2], padding=1)).to_torch().isnan())
+    assert "conv_relu" in g.dump_plan()
+
+
+def test_flipped_filters():
+    from nabla_b200.native import kernels
+
+    for shape in ((1, 1, 1, 1), (3, 2, 5, 7), (7, 7, 3, 64)):
+        for dtype in (torch.float32, torch.bfloat16):
+            w = torch.randn(shape, device="cuda").to(dtype)
+            assert torch.equal(kernels.conv_flip(w), w.flip(0, 1).permute(0, 1, 3, 2).contiguous())
