@@ -93,15 +93,43 @@ __device__ __forceinline__ void unpack_vec(const uint4& raw, float* out) {
   for (int i = 0; i < Vec<T>::N; ++i) out[i] = to_f<T>(e[i]);
 }
 
+// 16-byte vector <-> pairs of floats, for the packed two-wide fp32 instructions (fma.rn.f32x2).
+template <typename T> __device__ __forceinline__ void unpack_pairs(const uint4& raw, float2* out);
+template <> __device__ __forceinline__ void unpack_pairs<float>(const uint4& raw, float2* out) {
+  out[0] = make_float2(__uint_as_float(raw.x), __uint_as_float(raw.y));
+  out[1] = make_float2(__uint_as_float(raw.z), __uint_as_float(raw.w));
+}
+template <> __device__ __forceinline__ void unpack_pairs<bf16>(const uint4& raw, float2* out) {
+  const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) out[k] = make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
+}
+template <typename T> __device__ __forceinline__ uint4 pack_pairs(const float2* in);
+template <> __device__ __forceinline__ uint4 pack_pairs<float>(const float2* in) {
+  return make_uint4(__float_as_uint(in[0].x), __float_as_uint(in[0].y), __float_as_uint(in[1].x), __float_as_uint(in[1].y));
+}
+template <> __device__ __forceinline__ uint4 pack_pairs<bf16>(const float2* in) {
+  unsigned w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    __nv_bfloat162 h = __float22bfloat162_rn(in[k]);
+    w[k] = *reinterpret_cast<unsigned*>(&h);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // One warp per row. The row is read once and stays in registers in its packed 16-byte form
 // (D <= 32 * VPL * Vec::N); it is unpacked for the mean, the variance and the output, which keeps
-// the register count low enough for the number of rows in flight that a bandwidth-bound pass needs.
+// the register count low enough for the number of rows in flight that a bandwidth-bound pass needs. The arithmetic on bf16 is two elements wide:
+// that, twice the elements of fp32 in the same bytes, was bound by instructions (16384 x 2048 30.4 us, 26.1 so; HBM's copy rate is
+// 20.5), and wider rows have the registers that they need (8192 x 4096 51.3, 32.8, with 64 they spilled).
 template <typename T, int VPL>
-__global__ void __launch_bounds__(128, 8) layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
+__global__ void __launch_bounds__(128, VPL <= 4 || (VPL <= 8 && sizeof(T) == 4) ? 8 : VPL <= 8 ? 7 : 4) layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
                                                               const T* __restrict__ beta, T* __restrict__ y,
                                                               float* __restrict__ mean, float* __restrict__ rstd,
                                                               int rows, int D, float eps) {
-  constexpr int V = Vec<T>::N;
+  constexpr int V = Vec<T>::N, P = V / 2;
+  constexpr bool PAIRS = sizeof(T) == 2;             // (16384 x 1024 fp32 25.0 us one at a time, 27.4 two)
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -117,20 +145,30 @@ __global__ void __launch_bounds__(128, 8) layernorm_fwd_kernel(const T* __restri
   // reductions issued back to back
   const float shift = __shfl_sync(0xffffffffu, to_f<T>(reinterpret_cast<const T*>(&raw[0])[0]), 0);
   float s = 0.f, q = 0.f;
+  float2 s2 = make_float2(0.f, 0.f), q2 = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int c = (i * 32 + lane) * V;
     if (c < D) {
-      float v[V];
-      unpack_vec<T>(raw[i], v);
+      float2 v[P];
+      unpack_pairs<T>(raw[i], v);
 #pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const float d = v[j] - shift;
-        s += d;
-        q = fmaf(d, d, q);
+      for (int j = 0; j < P; ++j) {
+        if (PAIRS) {
+          const float2 d = __fadd2_rn(v[j], make_float2(-shift, -shift));
+          s2 = __fadd2_rn(s2, d);
+          q2 = __ffma2_rn(d, d, q2);
+        } else {
+          const float a = v[j].x - shift, b = v[j].y - shift;
+          s += a;
+          q = fmaf(a, a, q);
+          s += b;
+          q = fmaf(b, b, q);
+        }
       }
     }
   }
+  if (PAIRS) { s = s2.x + s2.y; q = q2.x + q2.y; }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -144,24 +182,38 @@ __global__ void __launch_bounds__(128, 8) layernorm_fwd_kernel(const T* __restri
     if (rstd) rstd[row] = rs;
   }
   T* yr = y + (size_t)row * D;
-  const float nmr = -mu * rs;
+  const float2 rs2 = make_float2(rs, rs), nmr2 = make_float2(-mu * rs, -mu * rs);
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int c = (i * 32 + lane) * V;
     if (c < D) {
-      float g[V], b[V], o[V], v[V];
-      unpack_vec<T>(raw[i], v);
-      if (gamma) load_vec<T>(gamma + c, g);
-      if (beta) load_vec<T>(beta + c, b);
+      float2 v[P], g[P], b[P];
+      unpack_pairs<T>(raw[i], v);
+      if (gamma) unpack_pairs<T>(*reinterpret_cast<const uint4*>(gamma + c), g);
+      if (beta) unpack_pairs<T>(*reinterpret_cast<const uint4*>(beta + c), b);
 #pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const float n = fmaf(v[j], rs, nmr);
-        o[j] = gamma ? fmaf(n, g[j], beta ? b[j] : 0.f) : (n + (beta ? b[j] : 0.f));
+      for (int j = 0; j < P; ++j) {
+        if (PAIRS) {
+          const float2 n = __ffma2_rn(v[j], rs2, nmr2);
+          v[j] = gamma ? (beta ? __ffma2_rn(n, g[j], b[j]) : __fmul2_rn(n, g[j])) : beta ? __fadd2_rn(n, b[j]) : n;
+        } else {
+          const float m = fmaf(v[j].x, rs, nmr2.x), n = fmaf(v[j].y, rs, nmr2.y);
+          v[j].x = gamma ? fmaf(m, g[j].x, beta ? b[j].x : 0.f) : m + (beta ? b[j].x : 0.f);
+          v[j].y = gamma ? fmaf(n, g[j].y, beta ? b[j].y : 0.f) : n + (beta ? b[j].y : 0.f);
+        }
       }
-      store_vec<T>(yr + c, o);
+      *reinterpret_cast<uint4*>(yr + c) = pack_pairs<T>(v);
     }
   }
 }
+
+// 16 bytes from global to shared memory without a register in between; the copying thread alone waits for them and reads them.
+__device__ __forceinline__ void async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
 // Backward, part 1: dx. One warp per row. The row's x and dy stay in registers in their packed
 // 16-byte form (half the registers of keeping them as floats, so twice as many rows are in flight
@@ -223,31 +275,6 @@ __global__ void __launch_bounds__(128, 4) layernorm_bwd_dx_kernel(const T* __res
       store_vec<T>(dxr + c, o);
     }
   }
-}
-
-// 16-byte vector <-> pairs of floats, for the packed two-wide fp32 instructions (fma.rn.f32x2).
-template <typename T> __device__ __forceinline__ void unpack_pairs(const uint4& raw, float2* out);
-template <> __device__ __forceinline__ void unpack_pairs<float>(const uint4& raw, float2* out) {
-  out[0] = make_float2(__uint_as_float(raw.x), __uint_as_float(raw.y));
-  out[1] = make_float2(__uint_as_float(raw.z), __uint_as_float(raw.w));
-}
-template <> __device__ __forceinline__ void unpack_pairs<bf16>(const uint4& raw, float2* out) {
-  const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) out[k] = make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
-}
-template <typename T> __device__ __forceinline__ uint4 pack_pairs(const float2* in);
-template <> __device__ __forceinline__ uint4 pack_pairs<float>(const float2* in) {
-  return make_uint4(__float_as_uint(in[0].x), __float_as_uint(in[0].y), __float_as_uint(in[1].x), __float_as_uint(in[1].y));
-}
-template <> __device__ __forceinline__ uint4 pack_pairs<bf16>(const float2* in) {
-  unsigned w[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    __nv_bfloat162 h = __float22bfloat162_rn(in[k]);
-    w[k] = *reinterpret_cast<unsigned*>(&h);
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // Backward in one pass (rows of one vector per lane): a persistent grid of warps walks the rows,
@@ -347,8 +374,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
                               const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
                               T* __restrict__ dx, float* __restrict__ partial, int rows, int D, int NW, int RB) {
   constexpr int V = Vec<T>::N, P = V / 2;
-  __shared__ float4 red[2][LN_MAX_WARPS];
-  __shared__ float sh[2][4 * 32 * V];                // RB > 1 means NW <= 4
+  __shared__ float red[2][LN_MAX_WARPS][4];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, slot = wid / NW, c = ((wid - slot * NW) * 32 + lane) * V;
   const bool act = c < D;
   const float inv_d = 1.f / D;
@@ -357,33 +383,53 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
   for (int k = 0; k < P; ++k) { gm[k] = make_float2(1.f, 1.f); ag[k] = ab[k] = make_float2(0.f, 0.f); }
   if (gamma && act) unpack_pairs<T>(*reinterpret_cast<const uint4*>(gamma + c), gm);
   const int stride = gridDim.x * RB;
-  int buf = 0;
-  for (int base = blockIdx.x * RB; base < rows; base += 2 * stride, buf ^= 1) {
-    uint4 xr[2], dr[2], ar[2];
-    float rs[2], nmr[2];
+  // The next pair of rows is on its way to shared memory while a pair is worked on: a thread's own vectors, which it alone waits for
+  // and reads. With the loads in front of their use the memory waited for a block's sums and barrier. us with the column sums' launch, before and
+  // with this and the shorter exchange of the sums: 16384 x 2048 bf16 52.5, 49.3, with `add` 67.9, 57.5; 8192 x 4096 58.8, 51.1; 8192 x 2048 fp32 49.0, 38.1.
+  constexpr int W = ADD ? 3 : 2, AHEAD = 1;
+  extern __shared__ uint4 ln_ring[];
+  auto ask = [&](int base, int stage) {
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int row = base + u * stride + slot;
-      xr[u] = dr[u] = make_uint4(0, 0, 0, 0);
-      rs[u] = nmr[u] = 0.f;
-      if (row < rows) {
-        if (act && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, (long long)row * D + c + V - 1, (long long)rows * D)) {
-          xr[u] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + c);
-          dr[u] = *reinterpret_cast<const uint4*>(dy + (size_t)row * D + c);
-          if (ADD) ar[u] = *reinterpret_cast<const uint4*>(add + (size_t)row * D + c);
-        }
-        rs[u] = rstd[row];
-        nmr[u] = -mean[row] * rs[u];
+      if (row < rows && act && NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, (long long)row * D + c + V - 1, (long long)rows * D)) {
+        uint4* to = ln_ring + ((stage * 2 + u) * W) * blockDim.x + threadIdx.x;
+        async16(to, x + (size_t)row * D + c);
+        async16(to + blockDim.x, dy + (size_t)row * D + c);
+        if (ADD) async16(to + 2 * blockDim.x, add + (size_t)row * D + c);
       }
     }
+    async_commit();
+  };
+  auto moments = [&](int base, float (&m)[2], float (&r)[2]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int row = base + u * stride + slot;
+      m[u] = row < rows ? mean[row] : 0.f;
+      r[u] = row < rows ? rstd[row] : 0.f;
+    }
+  };
+  int buf = 0, stage = 0;
+  float mn[2], rn[2];
+  moments(blockIdx.x * RB, mn, rn);
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k) ask(blockIdx.x * RB + 2 * k * stride, k);
+  for (int base = blockIdx.x * RB; base < rows; base += 2 * stride, buf ^= 1, stage = stage == AHEAD ? 0 : stage + 1) {
+    float rs[2], nmr[2];
+    ask(base + 2 * AHEAD * stride, stage == 0 ? AHEAD : stage - 1);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) { rs[u] = rn[u]; nmr[u] = -mn[u] * rn[u]; }
+    moments(base + 2 * stride, mn, rn);
+    async_wait<AHEAD>();
+    const uint4* from = ln_ring + stage * 2 * W * blockDim.x + threadIdx.x;       // [u][x, dy, add]
     float s[4];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), xv[P], dv[P];
       const float2 rs2 = make_float2(rs[u], rs[u]), nmr2 = make_float2(nmr[u], nmr[u]);
-      unpack_pairs<T>(xr[u], xv);
-      unpack_pairs<T>(dr[u], dv);
-      if (act) {
+      if (act && base + u * stride + slot < rows) {
+        unpack_pairs<T>(from[u * W * blockDim.x], xv);
+        unpack_pairs<T>(from[(u * W + 1) * blockDim.x], dv);
 #pragma unroll
         for (int k = 0; k < P; ++k) {
           const float2 xh = __ffma2_rn(xv[k], rs2, nmr2);              // (x - mean) * rstd
@@ -397,17 +443,26 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
       s[2 * u] = s1.x + s1.y;
       s[2 * u + 1] = s2.x + s2.y;
     }
+    // The four sums over the warp, each to an eighth of its lanes, then over the row's warps by eight lanes each: what an exchange of
+    // all four by all lanes and a loop over the warps take 80 instructions for, of some 230, takes 30.
+    const bool upper = lane & 16, odd8 = lane & 8;
+    const float a0 = (upper ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, upper ? s[0] : s[2], 16);
+    const float a1 = (upper ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, upper ? s[1] : s[3], 16);
+    float a = (odd8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd8 ? a0 : a1, 8);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-    if (lane == 0) red[buf][wid] = make_float4(s[0], s[1], s[2], s[3]);
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    const int which = lane >> 3, of = lane & 7;      // lanes 8 k .. 8 k + 7: sum k
+    if (of == 0) red[buf][wid][which] = a;
     __syncthreads();
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < NW; ++k) {
-      const float4 r = red[buf][slot * NW + k];
-      t.x += r.x; t.y += r.y; t.z += r.z; t.w += r.w;
-    }
+    a = of < NW ? red[buf][slot * NW + of][which] : 0.f;
+    if (of + 8 < NW) a += red[buf][slot * NW + of + 8][which];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    float4 t;
+    t.x = __shfl_sync(0xffffffffu, a, 0);
+    t.y = __shfl_sync(0xffffffffu, a, 8);
+    t.z = __shfl_sync(0xffffffffu, a, 16);
+    t.w = __shfl_sync(0xffffffffu, a, 24);
     const float m1[2] = {t.x * inv_d, t.z * inv_d}, m2[2] = {t.y * inv_d, t.w * inv_d};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -417,14 +472,14 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
         const float2 rs2 = make_float2(rs[u], rs[u]), nmr2 = make_float2(nmr[u], nmr[u]);
         const float2 a2 = make_float2(-rs[u] * m2[u], -rs[u] * m2[u]), b2 = make_float2(-rs[u] * m1[u], -rs[u] * m1[u]);
         float2 xv[P], dv[P], o[P];
-        unpack_pairs<T>(xr[u], xv);
-        unpack_pairs<T>(dr[u], dv);
+        unpack_pairs<T>(from[u * W * blockDim.x], xv);
+        unpack_pairs<T>(from[(u * W + 1) * blockDim.x], dv);
 #pragma unroll
         for (int k = 0; k < P; ++k)
           o[k] = __ffma2_rn(__fmul2_rn(dv[k], gm[k]), rs2, __ffma2_rn(__ffma2_rn(xv[k], rs2, nmr2), a2, b2));
         if (ADD) {
           float2 e[P];
-          unpack_pairs<T>(ar[u], e);
+          unpack_pairs<T>(from[(u * W + 2) * blockDim.x], e);
 #pragma unroll
           for (int k = 0; k < P; ++k) o[k] = __fadd2_rn(o[k], e[k]);
         }
@@ -433,6 +488,9 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
     }
   }
   float* prow = partial + (size_t)blockIdx.x * 2 * D;
+  float(*sh)[4 * 32 * V] = reinterpret_cast<float(*)[4 * 32 * V]>(ln_ring);      // the ring has been read; RB > 1 means NW <= 4
+  async_wait<0>();
+  __syncthreads();
   for (int r = 0; r < RB; ++r) {                     // fold the row slots, in order
     if (slot == r && act) {
 #pragma unroll
@@ -2674,9 +2732,11 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
       layernorm_bwd_fused_kernel<T, ADD><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
                                                                  (const T*)add, (T*)dx, partial, rows, D);            \
     else {                                                                                                            \
-      const int rb = vpl < 8 ? 8 / vpl : 1;                                                                           \
-      layernorm_bwd_rows_kernel<T, ADD><<<nb, 32 * vpl * rb, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
-                                                                          (const T*)add, (T*)dx, partial, rows, D, vpl, rb); \
+      const int rb = vpl < 8 ? 8 / vpl : 1, smem = 32 * vpl * rb * 16 * 2 * 2 * (ADD ? 3 : 2);                        \
+      const auto kernel = layernorm_bwd_rows_kernel<T, ADD>;                                                          \
+      if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
+      kernel<<<nb, 32 * vpl * rb, smem, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)add, (T*)dx, \
+                                                  partial, rows, D, vpl, rb);                                         \
     }                                                                                                                 \
   }
   if (!g_ln_bwd_two_kernels) {
