@@ -1542,3 +1542,36 @@ def test_flipped_filters():
         for dtype in (torch.float32, torch.bfloat16):
             w = torch.randn(shape, device="cuda").to(dtype)
             assert torch.equal(kernels.conv_flip(w), w.flip(0, 1).permute(0, 1, 3, 2).contiguous())
+
+
+def test_captured_leaves_run_beside_the_chain():
+    """Weight and bias gradients of a captured step on streams of their own: the same bits as from one chain, over many replays whose
+    inputs change while the one before may still run; results of earlier calls stay what they were."""
+    import nabla_b200 as nb
+    from nabla_b200.models import transformer as T
+
+    cfg = T.TransformerConfig(n_layers=1, d_model=256, n_heads=4, d_ff=1024)
+    names = ("ln1_g", "ln1_b", "wqkv", "bqkv", "wo", "bo", "ln2_g", "ln2_b", "w1", "b1", "w2", "b2")
+    torch.manual_seed(32)
+    d, f = 256, 1024
+    shapes = ((d,), (d,), (d, 3 * d), (3 * d,), (d, d), (d,), (d,), (d,), (d, f), (f,), (f, d), (d,))
+    p = [(torch.randn(s, device="cuda") * (s[0] ** -0.5 if len(s) == 2 else 0.1)).to(torch.bfloat16) for s in shapes]
+    xs = [torch.randn(2, 200, d, device="cuda").to(torch.bfloat16) for _ in range(12)]
+    dys = [torch.randn(2, 200, d, device="cuda").to(torch.bfloat16) for _ in range(12)]
+
+    def step(x, dy, *q):
+        y, pull = nb.vjp(lambda t, *q: T.block(t, dict(zip(names, q)), cfg), x, *q, create_graph=False)
+        return (y, *pull(dy))
+
+    wrap = nb.Tensor.from_torch
+    g, plain = nb.compile(step, cuda_graph=True), nb.compile(step)
+    want = [[t.to_torch() for t in plain(wrap(x), wrap(dy), *map(wrap, p))] for x, dy in zip(xs, dys)]
+    got = [[t.to_torch() for t in g(wrap(x.clone()), wrap(dy.clone()), *map(wrap, p))] for _ in range(4) for x, dy in zip(xs, dys)]
+    recs = [r for e in g._cache.values() for r in e.values() if hasattr(r, "branch_steps")]
+    assert g.stats.cuda_graphs == 1 and len(recs) == 1 and len(recs[0].branch_steps) >= 5
+    for k, outs in enumerate(got):
+        for a, b in zip(outs, want[k % 12]):
+            assert torch.equal(a, b)
+    h = nb.compile(step, cuda_graph=True, donate_argnums=(0,))
+    h(wrap(xs[0].clone()), wrap(dys[0]), *map(wrap, p))
+    assert not any(r.branch_steps for e in h._cache.values() for r in e.values() if hasattr(r, "branch_steps"))
