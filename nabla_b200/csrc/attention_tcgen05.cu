@@ -195,6 +195,7 @@ struct FwdArgs {
   MaskArg mask;
   int* status;
   int vec32;                    // rows of O start on 32-byte boundaries
+  int q_tiles;                  // query tiles of a CTA: 2, or 1 where those of 2 would leave SMs without a CTA
   int bh_chunk;                 // see tile_order
   int nsplit;                   // the keys are cut into this many ranges, one CTA each (1: no split)
   float* part_o;                // nsplit > 1: [nsplit][B][H][Sq][HD] output over each range, fp32
@@ -252,7 +253,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
   if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return;
-  const int nqt = (args.Sq + 2 * BT - 1) / (2 * BT);
+  const int nqt = (args.Sq + args.q_tiles * BT - 1) / (args.q_tiles * BT);
   int bh_, rank;
   tile_order(blockIdx.x, args.H * args.B * args.nsplit, args.bh_chunk, nqt, bh_, rank);
   const int qt = nqt - 1 - rank;          // the late tiles of a causal problem see the most keys
@@ -260,7 +261,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   bh_ /= args.nsplit;
   const int h = bh_ % args.H;
   const int b = bh_ / args.H;
-  const int q0 = qt * 2 * BT;
+  const int q0 = qt * args.q_tiles * BT;
   const int off = args.Skv - args.Sq;     // causal: row i sees keys <= i + off
   int n_t[2];
 #pragma unroll
@@ -271,7 +272,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int last_key = min(args.Skv - 1, q0t + BT - 1 + off);
       n = last_key < 0 ? 0 : last_key / BT + 1;
     }
-    n_t[t] = q0t < args.Sq ? n : 0;
+    n_t[t] = t < args.q_tiles && q0t < args.Sq ? n : 0;
   }
   // this CTA's range of key tiles: [kt0, kt0 + n_t[t]) of query tile t
   const int per = (max(n_t[0], n_t[1]) + args.nsplit - 1) / args.nsplit;
@@ -602,7 +603,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (ok && q0 + t * BT < args.Sq) {
+    if (ok && t < args.q_tiles && q0 + t * BT < args.Sq) {
       tc_fence_after();
       const bool have = n > 0 && l > 0.f;
       const float inv = have ? 1.f / l : 0.f;
@@ -1715,7 +1716,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     if (set_smem(attn_fwd_kernel<HD, MASK>, L::TOTAL)) return -2;
     configured = true;
   }
-  const int nqt = (a.Sq + 2 * BT - 1) / (2 * BT);
+  const int nqt = (a.Sq + a.q_tiles * BT - 1) / (a.q_tiles * BT);
   const long long grid = (long long)nqt * a.H * a.B * a.nsplit;
   if (grid <= 0) return 0;
   attn_fwd_kernel<HD, MASK><<<(unsigned)grid, NTHREADS, L::TOTAL, stream>>>(tq, tk, tv, a);
@@ -1754,6 +1755,17 @@ static bool attn_decode(int B, int H, int Sq, int Skv, int D, bool mask) {
   if (mask || Sq > nba::DEC_MAX_Q || bh > 65535) return false;
   if (Sq <= 2) return true;
   return D == 64 ? Skv <= nba::BT || bh >= 256 : Skv <= 64 || (bh > 148 && Skv < 256);
+}
+
+// Query tiles that a CTA of the tile kernel owns. Two share the keys that it loads, and one's softmax runs beside the other's
+// products; alone a tile is done sooner (its two math groups' exponentials no longer queue for one SM), so a grid that has an
+// SM for every tile gives it one. us with two and with one: 2 x 8 heads x 1001 x 64, causal, 19.3 and 15.2, full 20.9 and 15.6;
+// 64 x 256 x 128 11.0 and 9.3; 4 x 2048 x 64 under a mask of keys 48.9 and 35.1. A second wave costs more than that (16 x 1500 x
+// 64, full: 28.7 and 38.4). Three causal tiles stay: the last is alone as it is (32 x 333 x 128 10.8 and 11.1).
+static int attn_q_tiles(int B, int H, int Sq, int Skv, int causal, int nsplit) {
+  const long long tiles = (Sq + nba::BT - 1) / nba::BT;
+  if (tiles * B * H * nsplit > 148) return 2;
+  return causal && tiles == 3 && Skv <= Sq ? 2 : 1;
 }
 
 // Key ranges that a forward pass is cut into (1: none).
@@ -1844,6 +1856,7 @@ extern "C" int nb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   a.mask = MaskArg{mask, m_sb, m_sh, m_sq};
   a.status = status;
   a.vec32 = ((reinterpret_cast<uintptr_t>(o) & 31) | ((o_sb | o_sh | o_ss) & 15)) == 0;
+  a.q_tiles = attn_q_tiles(B, H, Sq, Skv, causal, nsplit);
   a.bh_chunk = causal ? l2_chunk(B * H, Skv, D) * nsplit : 1;
   a.nsplit = nsplit; a.part_o = part_o; a.part_lse = part_lse;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

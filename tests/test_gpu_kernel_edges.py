@@ -1299,6 +1299,37 @@ def test_compiled_calls_that_change_between_calls():
 
 
 @pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Sq,Skv", [(2, 148, 128, 128), (2, 74, 129, 200), (3, 37, 300, 300), (3, 37, 300, 400), (2, 37, 512, 512), (2, 16, 1030, 1030)])
+def test_attention_with_one_and_two_query_tiles_per_block(B, H, Sq, Skv, D):
+    """A batch of more tiles than SMs (blocks of two) and each of its items alone (blocks of one) are equal bit for bit."""
+    from nabla_b200.native import attention
+
+    torch.manual_seed(Sq)
+    q = torch.randn(B, H, Sq, D, device="cuda").bfloat16()
+    k, v = (torch.randn(B, H, Skv, D, device="cuda").bfloat16() for _ in range(2))
+    keys = torch.randn(B, 1, 1, Skv, device="cuda")
+    keys[..., 1::3] = -float("inf")
+    for causal in (False, True):
+        for m in (None, keys, keys + torch.randn(B, 1, Sq, Skv, device="cuda")):
+            o, lse = attention.sdpa_fwd(q, k, v, causal=causal, scale=D ** -0.5, mask=m)
+            for b in range(B):
+                one = attention.sdpa_fwd(*(t[b:b + 1] for t in (q, k, v)), causal=causal, scale=D ** -0.5, mask=None if m is None else m[b:b + 1])
+                assert torch.equal(o[b:b + 1], one[0]) and torch.equal(lse[b:b + 1], one[1])
+    _attention_check(q[:, :3], k[:, :3], v[:, :3], True, keys, grads=False)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_attention_over_key_ranges_with_two_query_tiles_per_block(D):
+    """Ranges of three key tiles and one: of the last the first 128 queries of a block see nothing."""
+    from nabla_b200.native import attention
+
+    attention._lib()
+    assert attention._splits(1, 40, 256, 896, D, 0) == 3
+    torch.manual_seed(D)
+    _attention_check(*(torch.randn(1, 40, s, D, device="cuda").bfloat16() for s in (256, 896, 896)), True, grads=False)
+
+
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,H,Sq,Skv", [(1, 1, 1, 1), (2, 3, 1, 31), (1, 2, 2, 127), (1, 2, 3, 128), (2, 1, 4, 257), (1, 4, 1, 4001), (3, 5, 4, 700),
                                         (40, 16, 1, 300), (1, 1, 5, 4000), (2, 4, 33, 2500), (1, 2, 130, 1500), (1, 1, 300, 3000)])
 def test_attention_of_few_queries_over_a_long_prefix(B, H, Sq, Skv, D):
