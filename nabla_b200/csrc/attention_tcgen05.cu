@@ -32,6 +32,7 @@
 #include <cooperative_groups.h>
 
 #include "sm100_ptx.cuh"
+#include "launch.cuh"
 #include "nb_debug.cuh"
 
 namespace nba {
@@ -252,7 +253,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
-  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return;
+  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return follow_grid();
   const int nqt = (args.Sq + args.q_tiles * BT - 1) / (args.q_tiles * BT);
   int bh_, rank;
   tile_order(blockIdx.x, args.H * args.B * args.nsplit, args.bh_chunk, nqt, bh_, rank);
@@ -307,6 +308,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  follow_grid();
   // tile t: scores (and P over their first 64 columns) at t * 128, output accumulator at 256 + t * HD; SPARE: P at 384 + t * 64
 
   if (warp < 4) {
@@ -648,6 +650,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // in which the row sees no key has lse = -inf and weight 0.
 template <int HD>
 __global__ void __launch_bounds__(128) attn_fwd_combine_kernel(const FwdArgs args) {
+  follow_grid();
   constexpr int E = HD / 32;
   const long long rows = (long long)args.B * args.H * args.Sq;
   const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -705,6 +708,7 @@ constexpr int DEC_MAX_Q = 4, DEC_U = 4;
 
 template <int HD, int NQ, int WARPS, bool CLUSTER>
 __global__ void __launch_bounds__(32 * WARPS, NQ == 1 ? (WARPS == 4 ? 4 : 3) : NQ == 2 ? (WARPS == 4 ? 5 : 2) : 1) attn_decode_kernel(const DecodeArgs a) {
+  follow_grid();
   constexpr int LPK = HD / 8, KPW = 32 / LPK, G = WARPS * KPW;      // lanes per key, keys per warp, lane groups per block
   const FwdArgs& f = a.f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LPK, d0 = (lane % LPK) * 8;
@@ -945,10 +949,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
-  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return;
+  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return follow_grid();
   if (smem_u32(smem) & 1023u) {     // the swizzled tiles need it, and the size above leaves no room to align
     if (threadIdx.x == 0) atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER);
-    return;
+    return follow_grid();
   }
   int bh_, jt;             // key tile 0 sees every query tile, the last one only a few
   tile_order(blockIdx.x, args.H * args.B, args.q_chunk, (args.Skv + BT - 1) / BT, bh_, jt);
@@ -996,6 +1000,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  follow_grid();
   constexpr int NREG = HD == 64 ? 3 : 2;
   const uint32_t t_dv = tmem_base + NREG * 128, t_dk = t_dv + HD;
   auto t_s = [&](int it) { return tmem_base + (NREG == 3 ? 2 * it % 3 : it & 1) * 128; };            // S^T of tile it
@@ -1280,7 +1285,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // an earlier bounded wait on this device already failed: leave (uniformly)
-  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return;
+  if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return follow_grid();
   const int nqt = (args.Sq + BT - 1) / BT;
   int bh_, rank;
   tile_order(blockIdx.x, args.H * args.B, args.kv_chunk, nqt, bh_, rank);
@@ -1328,6 +1333,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  follow_grid();
   const uint32_t t_dp = tmem_base + 256, t_dq = tmem_base + 384;   // S buffers at 0 and 128
 
   if (warp == 0) {
@@ -1589,6 +1595,7 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
                                                            float* __restrict__ nlse2, int H, int Sq, int Sq_pad,
                                                            long long do_sb, long long do_sh, long long do_ss,
                                                            long long o_sb, long long o_sh, long long o_ss) {
+  follow_grid();
   constexpr int LPR = D / 8, RPB = 256 / LPR * PREP_U;    // lanes per row: 16 or 8; rows per block: 64 or 128
   static_assert(BT % RPB == 0, "a block stays inside a (batch, head)");
   const int per_bh = Sq_pad / RPB, bh = blockIdx.x / per_bh, q0 = (blockIdx.x - bh * per_bh) * RPB + threadIdx.x / LPR;
@@ -1671,7 +1678,7 @@ static int l2_chunk(int nbh, long long rows, int hd) {
 template <int HD>
 static void combine(const FwdArgs& a, cudaStream_t stream) {
   const long long rows = (long long)a.B * a.H * a.Sq;
-  attn_fwd_combine_kernel<HD><<<(unsigned)((rows + 3) / 4), 128, 0, stream>>>(a);
+  launch_following(attn_fwd_combine_kernel<HD>, (unsigned)((rows + 3) / 4), 128, 0, stream, a);
 }
 
 // Blocks of a cluster for so many warps on a (batch, head): of four warps, of eight above 32.
@@ -1682,12 +1689,12 @@ template <int HD, int NQ>
 static int launch_decode(const DecodeArgs& a, int warps, cudaStream_t stream) {
   const dim3 grid(a.f.nsplit, a.f.B * a.f.H);
   if (warps == 0) {
-    attn_decode_kernel<HD, NQ, 4, false><<<grid, 128, 0, stream>>>(a);
+    launch_following(attn_decode_kernel<HD, NQ, 4, false>, grid, 128, 0, stream, a);
     if (a.f.nsplit > 1) combine<HD>(a.f, stream);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
   }
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)a.f.nsplit;
   attr[0].val.clusterDim.y = 1;
@@ -1699,6 +1706,7 @@ static int launch_decode(const DecodeArgs& a, int warps, cudaStream_t stream) {
   cfg.numAttrs = 1;
   const auto kernel = warps > 32 ? attn_decode_kernel<HD, NQ, 8, true> : attn_decode_kernel<HD, NQ, 4, true>;
   if (a.f.nsplit > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return -2;
+  set_following(cfg);
   return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? 0 : -3;
 }
 template <int HD>
@@ -1719,7 +1727,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   const int nqt = (a.Sq + a.q_tiles * BT - 1) / (a.q_tiles * BT);
   const long long grid = (long long)nqt * a.H * a.B * a.nsplit;
   if (grid <= 0) return 0;
-  attn_fwd_kernel<HD, MASK><<<(unsigned)grid, NTHREADS, L::TOTAL, stream>>>(tq, tk, tv, a);
+  launch_following(attn_fwd_kernel<HD, MASK>, (unsigned)grid, NTHREADS, L::TOTAL, stream, tq, tk, tv, a);
   if (a.nsplit > 1) combine<HD>(a, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -1735,8 +1743,8 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   }
   const long long bh = (long long)a.H * a.B;
   const int nkt = (a.Skv + BT - 1) / BT, nqt = (a.Sq + BT - 1) / BT;
-  attn_bwd_dkdv_kernel<HD, MASK><<<(unsigned)(nkt * bh), NTHREADS, DkvSmem<HD>::TOTAL, stream>>>(tq, tk, tv, tdo, a);
-  attn_bwd_dq_kernel<HD, MASK><<<(unsigned)(nqt * bh), NTHREADS, DqSmem<HD>::TOTAL, stream>>>(tq, tk, tv, tdo, a);
+  launch_following(attn_bwd_dkdv_kernel<HD, MASK>, (unsigned)(nkt * bh), NTHREADS, DkvSmem<HD>::TOTAL, stream, tq, tk, tv, tdo, a);
+  launch_following(attn_bwd_dq_kernel<HD, MASK>, (unsigned)(nqt * bh), NTHREADS, DqSmem<HD>::TOTAL, stream, tq, tk, tv, tdo, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -1905,7 +1913,7 @@ extern "C" int nb_attn_bwd(const void* dO, const void* q, const void* k, const v
   float* nlse2 = stats + rows;
   const long long prep = rows / (256 / (D / 8) * PREP_U);
   if (prep > 0x7fffffffll) return -15;
-#define PREP(HD) attn_bwd_prep_kernel<HD><<<(unsigned)prep, 256, 0, s>>>( \
+#define PREP(HD) launch_following(attn_bwd_prep_kernel<HD>, (unsigned)prep, 256, 0, s,  \
       reinterpret_cast<const __nv_bfloat16*>(dO), reinterpret_cast<const __nv_bfloat16*>(o), lse, ndelta, nlse2, H, Sq, Sq_pad, \
       do_sb, do_sh, do_ss, o_sb, o_sh, o_ss)
   if (D == 128) PREP(128);

@@ -16,6 +16,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "nb_debug.cuh"
 
 namespace nbe {
@@ -87,6 +88,7 @@ constexpr int EW_U = 4;
 template <typename T, int BMODE>
 __global__ void __launch_bounds__(256) binary_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                                                     size_t n, int op, unsigned inner, int swap) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const size_t base = (size_t)blockIdx.x * (256 * V * EW_U) + (size_t)threadIdx.x * V;
   const float bs = BMODE == 1 ? to_f<T>(b[0]) : 0.f;
@@ -163,6 +165,7 @@ __device__ __forceinline__ float un_apply(float x, int op) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) unary_kernel(const T* __restrict__ a, T* __restrict__ out, size_t n, int op) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const size_t base = (size_t)blockIdx.x * (256 * V * EW_U) + (size_t)threadIdx.x * V;
   uint4 ra[EW_U];
@@ -236,6 +239,7 @@ __device__ __forceinline__ Acc warp_red(Acc a, int op) {
 template <typename T, typename O>
 __global__ void __launch_bounds__(256) row_reduce_kernel(const T* __restrict__ x, O* __restrict__ out, long long rows,
                                                         long long R, int op) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const int lane = threadIdx.x & 31;
   for (long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (long long)gridDim.x * 8) {
@@ -287,6 +291,7 @@ template <typename T, typename O>
 __global__ void __launch_bounds__(256) col_reduce_kernel(const T* __restrict__ x, O* __restrict__ out, float* __restrict__ pv,
                                                         long long* __restrict__ pi, long long outer, long long R,
                                                         long long inner, int op, int splits) {
+  nb::follow_grid();
   __shared__ float sv[8][32];
   __shared__ long long si[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -336,6 +341,7 @@ constexpr int THIN_THREADS = 128, THIN_CHAINS = 8;
 template <typename T, int OP, int CH>
 __global__ void __launch_bounds__(THIN_THREADS) thin_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
                                                          int R, long long inner) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N, U = 4, STEP = CH > U ? CH : U;
   const long long nv = inner / V, t = (long long)blockIdx.x * THIN_THREADS + threadIdx.x;
   if (t >= outer * nv) return;
@@ -386,6 +392,7 @@ template <typename T, typename O>
 __global__ void __launch_bounds__(256) col_reduce_finish_kernel(const float* __restrict__ pv, const long long* __restrict__ pi,
                                                                O* __restrict__ out, long long outer, long long R,
                                                                long long inner, int op, int splits) {
+  nb::follow_grid();
   const long long total = outer * inner;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const long long o = t / inner, i = t - o * inner;
@@ -400,6 +407,7 @@ __global__ void __launch_bounds__(256) col_reduce_finish_kernel(const float* __r
 template <typename T>
 __global__ void __launch_bounds__(256) cumsum_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
                                                     long long R, long long inner, int exclusive, int reverse) {
+  nb::follow_grid();
   const long long total = outer * inner;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const long long o = t / inner, i = t - o * inner;
@@ -439,7 +447,7 @@ int nb_binary(const void* a, const void* b, void* out, long long n, int op, int 
   const size_t blocks = ((size_t)n + 256 * V * EW_U - 1) / (256 * V * EW_U);
   if (blocks > 0x7fffffffull) return -4;
   const unsigned grid = (unsigned)blocks;
-#define NB_BIN(T, M) binary_kernel<T, M><<<grid, 256, 0, STREAM>>>((const T*)a, (const T*)b, (T*)out, (size_t)n, op, (unsigned)inner, swap)
+#define NB_BIN(T, M) nb::launch_following(binary_kernel<T, M>, grid, 256, 0, STREAM, (const T*)a, (const T*)b, (T*)out, (size_t)n, op, (unsigned)inner, swap)
   if (dtype) { if (bmode == 0) NB_BIN(bf16, 0); else if (bmode == 1) NB_BIN(bf16, 1); else NB_BIN(bf16, 2); }
   else { if (bmode == 0) NB_BIN(float, 0); else if (bmode == 1) NB_BIN(float, 1); else NB_BIN(float, 2); }
 #undef NB_BIN
@@ -452,8 +460,8 @@ int nb_unary(const void* a, void* out, long long n, int op, int dtype, void* str
   const size_t blocks = ((size_t)n + 256 * V * EW_U - 1) / (256 * V * EW_U);
   if (blocks > 0x7fffffffull) return -4;
   const unsigned grid = (unsigned)blocks;
-  if (dtype) unary_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)a, (bf16*)out, (size_t)n, op);
-  else unary_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)a, (float*)out, (size_t)n, op);
+  if (dtype) nb::launch_following(unary_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)a, (bf16*)out, (size_t)n, op);
+  else nb::launch_following(unary_kernel<float>, grid, 256, 0, STREAM, (const float*)a, (float*)out, (size_t)n, op);
   return CHECK_LAUNCH();
 }
 
@@ -485,18 +493,18 @@ int nb_reduce(const void* x, void* out, void* scratch, long long outer, long lon
     const long long want = (outer + 7) / 8;
     const int grid = (int)(want < 148 * 16 ? want : 148 * 16);
     if (dtype) {
-      if (arg) row_reduce_kernel<bf16, long long><<<grid, 256, 0, STREAM>>>((const bf16*)x, (long long*)out, outer, R, op);
-      else row_reduce_kernel<bf16, bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (bf16*)out, outer, R, op);
+      if (arg) nb::launch_following(row_reduce_kernel<bf16, long long>, grid, 256, 0, STREAM, (const bf16*)x, (long long*)out, outer, R, op);
+      else nb::launch_following(row_reduce_kernel<bf16, bf16>, grid, 256, 0, STREAM, (const bf16*)x, (bf16*)out, outer, R, op);
     } else {
-      if (arg) row_reduce_kernel<float, long long><<<grid, 256, 0, STREAM>>>((const float*)x, (long long*)out, outer, R, op);
-      else row_reduce_kernel<float, float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)out, outer, R, op);
+      if (arg) nb::launch_following(row_reduce_kernel<float, long long>, grid, 256, 0, STREAM, (const float*)x, (long long*)out, outer, R, op);
+      else nb::launch_following(row_reduce_kernel<float, float>, grid, 256, 0, STREAM, (const float*)x, (float*)out, outer, R, op);
     }
     return CHECK_LAUNCH();
   }
   const int V = dtype ? 8 : 4;
   if (!arg && thin_reduce(outer, R, inner, V) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
     const unsigned grid_t = (unsigned)((outer * (inner / V) + THIN_THREADS - 1) / THIN_THREADS);
-#define NB_THIN(T, OP, CH) thin_reduce_kernel<T, OP, CH><<<grid_t, THIN_THREADS, 0, STREAM>>>((const T*)x, (T*)out, outer, (int)R, inner)
+#define NB_THIN(T, OP, CH) nb::launch_following(thin_reduce_kernel<T, OP, CH>, grid_t, THIN_THREADS, 0, STREAM, (const T*)x, (T*)out, outer, (int)R, inner)
 #define NB_THIN_S(T, OP) do { if (R <= THIN_CHAINS) NB_THIN(T, OP, 1); else NB_THIN(T, OP, THIN_CHAINS); } while (0)
 #define NB_THIN_T(T) do { if (op == R_SUM) NB_THIN_S(T, R_SUM); else if (op == R_MAX) NB_THIN(T, R_MAX, 1); \
                           else if (op == R_MIN) NB_THIN(T, R_MIN, 1); else NB_THIN_S(T, R_MEAN); } while (0)
@@ -514,8 +522,8 @@ int nb_reduce(const void* x, void* out, void* scratch, long long outer, long lon
   long long* pi = reinterpret_cast<long long*>(pv + (outer * splits * inner + 1) / 2 * 2);      // on an 8-byte boundary
   const int fgrid = grid_for((size_t)(outer * inner), 256);
 #define NB_COL(T, O) do { \
-    col_reduce_kernel<T, O><<<grid, 256, 0, STREAM>>>((const T*)x, (O*)out, pv, pi, outer, R, inner, op, splits); \
-    if (splits > 1) col_reduce_finish_kernel<T, O><<<fgrid, 256, 0, STREAM>>>(pv, pi, (O*)out, outer, R, inner, op, splits); \
+    nb::launch_following(col_reduce_kernel<T, O>, grid, 256, 0, STREAM, (const T*)x, (O*)out, pv, pi, outer, R, inner, op, splits); \
+    if (splits > 1) nb::launch_following(col_reduce_finish_kernel<T, O>, fgrid, 256, 0, STREAM, pv, pi, (O*)out, outer, R, inner, op, splits); \
   } while (0)
   if (dtype) { if (arg) NB_COL(bf16, long long); else NB_COL(bf16, bf16); }
   else { if (arg) NB_COL(float, long long); else NB_COL(float, float); }
@@ -527,8 +535,8 @@ int nb_cumsum(const void* x, void* out, long long outer, long long R, long long 
               void* stream) {
   if (outer <= 0 || inner <= 0 || R <= 0) return 0;
   const int grid = grid_for((size_t)(outer * inner), 256);
-  if (dtype) cumsum_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (bf16*)out, outer, R, inner, exclusive, reverse);
-  else cumsum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)out, outer, R, inner, exclusive, reverse);
+  if (dtype) nb::launch_following(cumsum_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, (bf16*)out, outer, R, inner, exclusive, reverse);
+  else nb::launch_following(cumsum_kernel<float>, grid, 256, 0, STREAM, (const float*)x, (float*)out, outer, R, inner, exclusive, reverse);
   return CHECK_LAUNCH();
 }
 

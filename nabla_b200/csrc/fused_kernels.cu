@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "nb_debug.cuh"
 
 namespace nbk {
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(128, VPL <= 4 || (VPL <= 8 && sizeof(T) == 4) 
                                                               const T* __restrict__ beta, T* __restrict__ y,
                                                               float* __restrict__ mean, float* __restrict__ rstd,
                                                               int rows, int D, float eps) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N, P = V / 2;
   constexpr bool PAIRS = sizeof(T) == 2;             // (16384 x 1024 fp32 25.0 us one at a time, 27.4 two)
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -223,6 +225,7 @@ __global__ void __launch_bounds__(128, 4) layernorm_bwd_dx_kernel(const T* __res
                                                               const T* __restrict__ gamma, const float* __restrict__ mean,
                                                               const float* __restrict__ rstd, T* __restrict__ dx,
                                                               int rows, int D) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(128, 4)
     layernorm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                                const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
                                T* __restrict__ dx, float* __restrict__ partial, int rows, int D) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N, P = V / 2;
   __shared__ float sh[2][32 * V];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = lane * V;
@@ -373,6 +377,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
     layernorm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                               const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
                               T* __restrict__ dx, float* __restrict__ partial, int rows, int D, int NW, int RB) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N, P = V / 2;
   __shared__ float red[2][LN_MAX_WARPS][4];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, slot = wid / NW, c = ((wid - slot * NW) * 32 + lane) * V;
@@ -522,6 +527,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_dgb_kernel(const T* __restr
                                                                const float* __restrict__ rstd,
                                                                float* __restrict__ partial, int rows, int D,
                                                                int rows_per_block) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   __shared__ float sh[2][8][32 * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -564,6 +570,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_dgb_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __restrict__ partial, T* __restrict__ out0,
                                                               T* __restrict__ out1, int nblocks, int D) {
+  nb::follow_grid();
   __shared__ float sh[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -588,6 +595,7 @@ __device__ __forceinline__ float sum8(const float (&a)[8]) { return ((a[0] + a[1
 template <typename T, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
                                                                 int slices) {
+  nb::follow_grid();
   __shared__ float sh[WARPS][33];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   const size_t i0 = (size_t)blockIdx.x * 32, i = i0 + lane;
@@ -611,8 +619,8 @@ __global__ void __launch_bounds__(32 * WARPS) fold_slices_kernel(const float* __
 template <typename T>
 static void fold_slices(const float* part, void* out, size_t n, int slices, cudaStream_t stream) {
   const unsigned grid = (unsigned)((n + 31) / 32);
-  if (slices < 64) fold_slices_kernel<T, 8><<<grid, 256, 0, stream>>>(part, (T*)out, n, slices);
-  else fold_slices_kernel<T, 32><<<grid, 1024, 0, stream>>>(part, (T*)out, n, slices);
+  if (slices < 64) nb::launch_following(fold_slices_kernel<T, 8>, grid, 256, 0, stream, part, (T*)out, n, slices);
+  else nb::launch_following(fold_slices_kernel<T, 32>, grid, 1024, 0, stream, part, (T*)out, n, slices);
 }
 
 // ============================================================== small fp32 products
@@ -629,6 +637,7 @@ struct SgemmArgs {
   long long a_m, a_k, b_k, b_n;
 };
 __global__ void __launch_bounds__(256) sgemm_kernel(const SgemmArgs g) {
+  nb::follow_grid();
   __shared__ float sa[SG][SG + 1], sb[SG][SG + 1];   // [k][m], [k][n]
   const int t = threadIdx.x, m0 = blockIdx.y * SG, n0 = blockIdx.x * SG;
   const int k_lo = blockIdx.z * g.per, k_hi = min(g.K, k_lo + g.per);
@@ -678,6 +687,7 @@ __global__ void __launch_bounds__(256) sgemm_kernel(const SgemmArgs g) {
 // out[m][n] = sum of the slices + bias[n]; eight lanes per result.
 __global__ void __launch_bounds__(256) sgemm_fold_kernel(const float* __restrict__ part, const float* __restrict__ bias,
                                                         float* __restrict__ out, int MN, int N, int slices) {
+  nb::follow_grid();
   const int i = (blockIdx.x * 256 + threadIdx.x) % 32 + blockIdx.x * 32, q = threadIdx.x >> 5;
   __shared__ float sh[8][33];
   float s = 0.f;
@@ -698,6 +708,7 @@ __global__ void __launch_bounds__(256) sgemm_fold_kernel(const float* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
                                                     int N, int rows_per_block) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   __shared__ float sh[8][32 * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -732,6 +743,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
                                                            int N, int rows_per_block) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   __shared__ float sh[256 * V];
   const int nv = N / V, rpp = 256 / nv, r_in = threadIdx.x / nv, c = threadIdx.x % nv;
@@ -809,6 +821,7 @@ __device__ __forceinline__ void colsum_slot(const T* __restrict__ x, int rows, i
 }
 template <typename T, int L>
 __global__ void __launch_bounds__(256) __cluster_dims__(1, COLSUM_CLUSTER, 1) colsum_group_kernel(const __grid_constant__ ColsumGroup g) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   __shared__ float sh[8][L * V];
   __shared__ float tot[L * V];
@@ -858,6 +871,7 @@ __global__ void __launch_bounds__(256) __cluster_dims__(1, COLSUM_CLUSTER, 1) co
 // ============================================================== softmax / log-softmax (last dim)
 template <typename T, bool LOG>
 __global__ void __launch_bounds__(256) softmax_kernel(const T* __restrict__ x, T* __restrict__ y, int rows, int D) {
+  nb::follow_grid();
   __shared__ float sh[8];
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
@@ -902,6 +916,7 @@ template <typename T, bool WHOLE, bool WIDE>
 __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__ logits,
                                                           const long long* __restrict__ tgt, float* __restrict__ lse_out,
                                                           float* __restrict__ picked, int rows, int D) {
+  nb::follow_grid();
   __shared__ float sh[8];
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
@@ -960,6 +975,7 @@ __global__ void __launch_bounds__(256) lse_pick_bwd_kernel(const T* __restrict__
                                                           const float* __restrict__ lse, const float* __restrict__ g_lse,
                                                           const float* __restrict__ g_pick, T* __restrict__ dlogits,
                                                           int rows, int D) {
+  nb::follow_grid();
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
   const T* xr = logits + (size_t)row * D;
@@ -1069,6 +1085,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const TP* __restrict__ p, co
                                                    TP* __restrict__ p_out, float* __restrict__ m_out,
                                                    float* __restrict__ v_out, size_t n, AdamHyper h,
                                                    const float* __restrict__ hyper) {
+  nb::follow_grid();
   adamw_device_hyper(h, hyper);
   const float ibc1 = 1.f / h.bc1, ibc2 = 1.f / h.bc2;
   const size_t i0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -1091,6 +1108,7 @@ struct AdamGroup {
 template <typename TP, typename TG>
 __global__ void __launch_bounds__(256) adamw_group_kernel(const __grid_constant__ AdamGroup c, AdamHyper h,
                                                          const float* __restrict__ hyper) {
+  nb::follow_grid();
   adamw_device_hyper(h, hyper);
   int l = 0;
   while (l + 1 < c.count && blockIdx.x >= c.leaf[l + 1].block0) ++l;
@@ -1104,6 +1122,7 @@ __global__ void __launch_bounds__(256) adamw_group_kernel(const __grid_constant_
 // as the updates of a small model (13 us of a 180 us training step; 2.8 now). `plus`: t is the sum of two counts, kept in `total`.
 __global__ void adam_hyper_kernel(const float* __restrict__ step, const float* __restrict__ plus, float* __restrict__ total,
                                   float* __restrict__ hyper, float lr, double b1, double b2) {
+  nb::follow_grid();
   const float sum = plus != nullptr ? step[0] + plus[0] : step[0];
   if (total != nullptr) total[0] = sum;
   const double t = (double)sum;
@@ -1121,6 +1140,7 @@ template <typename T, int C>
 __global__ void __launch_bounds__(MEAN_THREADS) __cluster_dims__(C, 1, 1)
     mean_diff_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ d, T* __restrict__ out, int n, int square,
                      const T* __restrict__ count_at, float count) {
+  nb::follow_grid();
   __shared__ float sh[MEAN_THREADS / 32], tot;
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int rank = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1153,6 +1173,7 @@ __global__ void __launch_bounds__(256) sgd_kernel(const TP* __restrict__ p, cons
                                                  const float* __restrict__ buf, TP* __restrict__ p_out,
                                                  float* __restrict__ buf_out, size_t n, float lr, float momentum,
                                                  float wd, float grad_scale) {
+  nb::follow_grid();
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t k = i0; k < n; k += stride) {
@@ -1174,6 +1195,7 @@ template <typename T, bool ADD>
 __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restrict__ table,
                                                               const long long* __restrict__ ids, const T* __restrict__ add,
                                                               T* __restrict__ out, int n_ids, int D, int vocab, int period) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
@@ -1261,6 +1283,7 @@ __device__ __forceinline__ unsigned long long scatter_scan(unsigned long long x,
 }
 
 __global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
+  nb::follow_grid();
   const int i = blockIdx.x * 256 + threadIdx.x;
   const long long id = i < n_ids ? ids[i] : -1;
   const bool ok = id >= 0 && id < vocab;
@@ -1270,6 +1293,7 @@ __global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __r
 // List slots and segments of every row; the rows of a block come in order, the blocks in any. A row of many
 // segments is written by the whole block.
 __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int n_ids, int vocab) {
+  nb::follow_grid();
   constexpr int FEW = 4;
   struct Row { int v, c, at, sg, h; };
   __shared__ unsigned long long wsum[8], wsum2[8];
@@ -1310,6 +1334,7 @@ __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int n_ids
   }
 }
 __global__ void __launch_bounds__(256) scatter_place_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
+  nb::follow_grid();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n_ids) return;
   const long long id = ids[i];
@@ -1478,6 +1503,7 @@ template <typename T, int VN, bool ALL>
 __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
                                                           T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
                                                           int D, int vocab) {
+  nb::follow_grid();
   __shared__ int last;
   const int total = *ws.nseg, lights = ALL ? *ws.nlight : 0;
   const int lane = threadIdx.x & 31, nwarps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1552,6 +1578,7 @@ __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(cons
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) embedding_scatter_add_kernel(float* __restrict__ acc, const long long* __restrict__ ids,
                                                                    const T* __restrict__ upd, int n_ids, int D, int vocab) {
+  nb::follow_grid();
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
   const long long id = ids[i];
@@ -1582,6 +1609,7 @@ __global__ void __launch_bounds__(128) embedding_scatter_sorted_kernel(const lon
                                                                       const long long* __restrict__ perm,
                                                                       const T* __restrict__ upd, const T* __restrict__ base,
                                                                       T* __restrict__ out, int n_ids, int D, int vocab) {
+  nb::follow_grid();
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;
   const long long id = sorted_ids[i];
@@ -1602,6 +1630,7 @@ __global__ void __launch_bounds__(128) embedding_scatter_sorted_kernel(const lon
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256) cast_kernel(const TI* __restrict__ in, TO* __restrict__ out, size_t n,
                                                   const TO* __restrict__ add_to) {
+  nb::follow_grid();
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t k = i0; k < n; k += stride) {
@@ -1627,6 +1656,7 @@ __device__ __forceinline__ float dgelu_tanh_f(float x) {
 template <typename T, bool BWD>
 __global__ void __launch_bounds__(256) act_kernel(const T* __restrict__ z, const T* __restrict__ dy, T* __restrict__ out,
                                                  size_t n, int mode) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const size_t i0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
   const size_t stride = (size_t)gridDim.x * blockDim.x * V;
@@ -1698,12 +1728,14 @@ __device__ __forceinline__ void rng_resolve(const unsigned long long* state, uin
     offset = state[1] << 32;
   }
 }
-__global__ void rng_bump_kernel(unsigned long long* state) { state[1] += 1ull; }
+__global__ void rng_bump_kernel(unsigned long long* state) {
+  nb::follow_grid(); state[1] += 1ull; }
 
 // mode 0: uniform in [a, b); mode 1: gaussian mean a std b
 template <typename T>
 __global__ void __launch_bounds__(256) rng_kernel(T* __restrict__ out, size_t n, uint64_t seed, uint64_t offset,
                                                  int mode, float a, float b, const unsigned long long* state) {
+  nb::follow_grid();
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
   rng_resolve(state, seed, offset);
@@ -1729,6 +1761,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dropout_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                      uint8_t* __restrict__ mask, size_t n, float p, uint64_t seed,
                                                      uint64_t offset, const unsigned long long* state) {
+  nb::follow_grid();
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
   rng_resolve(state, seed, offset);
@@ -1759,6 +1792,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) nf4_dequant_kernel(const uint8_t* __restrict__ packed,
                                                          const float* __restrict__ absmax, T* __restrict__ out,
                                                          size_t n, int block) {
+  nb::follow_grid();
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t b = i0; b * 2 < n; b += stride) {
@@ -1780,6 +1814,7 @@ __global__ void __launch_bounds__(256) nf4_dequant_codes_kernel(const uint8_t* _
                                                                const float* __restrict__ absmax,
                                                                const float* __restrict__ codebook, T* __restrict__ out,
                                                                size_t n, int block) {
+  nb::follow_grid();
   __shared__ float cb[16];
   if (threadIdx.x < 16) cb[threadIdx.x] = codebook[threadIdx.x];
   __syncthreads();
@@ -1824,6 +1859,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pool2d_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int N, int H, int W,
                                                         int C, int OH, int OW, int kh, int kw, int sh, int sw, int ph,
                                                         int pw, int mode) {
+  nb::follow_grid();
   const size_t total = (size_t)N * OH * OW * C;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = i % C;
@@ -1858,6 +1894,7 @@ struct CellGeom {
 };
 template <typename T, bool MAX>
 __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, const CellGeom g, unsigned total) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
@@ -1887,6 +1924,7 @@ __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restric
 template <typename T, bool MAX, bool RELU = false>
 __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dx,
                                                              const CellGeom g, unsigned total) {
+  nb::follow_grid();
   constexpr int V = Vec<T>::N;
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
@@ -1946,6 +1984,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pool2d_select_kernel(const T* __restrict__ x, const T* __restrict__ t,
                                                            T* __restrict__ y, int N, int H, int W, int C, int OH, int OW,
                                                            int kh, int kw, int sh, int sw, int ph, int pw) {
+  nb::follow_grid();
   const size_t total = (size_t)N * OH * OW * C;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = i % C;
@@ -1977,6 +2016,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pool2d_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                         T* __restrict__ dx, int N, int H, int W, int C, int OH,
                                                         int OW, int kh, int kw, int sh, int sw, int ph, int pw, int mode, int relu) {
+  nb::follow_grid();
   const size_t total = (size_t)N * H * W * C;
   const float inv = 1.f / (kh * kw);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -2035,6 +2075,7 @@ struct ConvGeom {
 // The filter of an input gradient: out[r][s][f][c] = w[R - 1 - r][S - 1 - s][c][f].
 template <typename T>
 __global__ void __launch_bounds__(256) conv_flip_kernel(const T* __restrict__ w, T* __restrict__ out, int taps, int C, int F, unsigned n) {
+  nb::follow_grid();
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= n || !NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, i, n)) return;
   const unsigned c = i % C, q = i / C, f = q % F, t = q / F;
@@ -2097,6 +2138,7 @@ __device__ __forceinline__ ConvTap conv_tap(int k, const ConvGeom& g) {
 template <typename T, int FG, bool VEC>
 __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                            const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g, int relu) {
+  nb::follow_grid();
   constexpr int PG = 128 / FG, MT = 2 * PG, FT = 4 * FG, PER = (MT + 127) / 128, KSTEP = MT < 128 ? 128 / MT : 1;
   __shared__ __align__(16) float xs[CONV_KC][MT + 4];
   __shared__ __align__(16) float ws[CONV_KC][FT];
@@ -2239,6 +2281,7 @@ template <typename T, int FG, int PX, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                           const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g,
                                                           int TH, int bands, int wvec, int yvec, int relu) {
+  nb::follow_grid();
   constexpr int PG = 128 / FG, FT = 4 * FG, KV = VEC ? 4 : 1;
   extern __shared__ __align__(16) float conv_smem[];
   const int tid = threadIdx.x, K = g.R * g.S * g.C, CQ = g.C / KV;
@@ -2350,6 +2393,7 @@ template <typename T, int KG, int FG, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                                  float* __restrict__ part, const ConvGeom g,
                                                                  long long per_block) {
+  nb::follow_grid();
   constexpr int SL = 128 / (KG * FG), KT = 4 * KG, FT = 4 * FG;
   constexpr int RED = SL > 1 ? 128 * 16 : 4, STAGE = WG_MC * (KT + FT);
   __shared__ __align__(16) float sm[RED > STAGE ? RED : STAGE];
@@ -2473,6 +2517,7 @@ template <typename T, int KG, int FG, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_wgrad_patch_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                                 float* __restrict__ part, const ConvGeom g, int TH,
                                                                 int bands, int total, int dvec) {
+  nb::follow_grid();
   constexpr int SL = 128 / (KG * FG), KT = 4 * KG, FT = 4 * FG, KV = VEC ? 4 : 1;
   extern __shared__ __align__(16) float conv_smem[];
   const int tid = threadIdx.x;
@@ -2590,6 +2635,7 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_patch_kernel(const T* __r
 template <typename T>
 __global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
                                                         int slices) {
+  nb::follow_grid();
   const size_t nv = n / 4;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x) {
     float4 acc = reinterpret_cast<const float4*>(part)[i];
@@ -2633,6 +2679,7 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, unsigned 
     reinterpret_cast<uint8_t*>(dst)[b] = reinterpret_cast<const uint8_t*>(src)[b];
 }
 __global__ void __launch_bounds__(256) copy_batch_kernel(const __grid_constant__ CopyBatch c) {
+  nb::follow_grid();
   int lo = 0, hi = c.n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
@@ -2672,7 +2719,7 @@ int nb_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y
   if (D % V) return -2;
   const int vpl = (D / V + 31) / 32;
   dim3 grid((rows + 3) / 4), block(128);
-#define LN_FWD(T, VPL) layernorm_fwd_kernel<T, VPL><<<grid, block, 0, STREAM>>>((const T*)x, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, D, eps)
+#define LN_FWD(T, VPL) nb::launch_following(layernorm_fwd_kernel<T, VPL>, grid, block, 0, STREAM, (const T*)x, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, D, eps)
   if (dtype) {
     if (vpl <= 1) LN_FWD(bf16, 1); else if (vpl <= 2) LN_FWD(bf16, 2); else if (vpl <= 4) LN_FWD(bf16, 4);
     else if (vpl <= 8) LN_FWD(bf16, 8); else if (vpl <= 16) LN_FWD(bf16, 16); else return -3;
@@ -2721,21 +2768,21 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
   dim3 grid_gb((D + 32 * V - 1) / (32 * V), nb);
 #define LN_BWD(T, VPL)                                                                                                \
   {                                                                                                                   \
-    layernorm_bwd_dx_kernel<T, VPL><<<grid_dx, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean,    \
+    nb::launch_following(layernorm_bwd_dx_kernel<T, VPL>, grid_dx, 128, 0, STREAM, (const T*)dy, (const T*)x, (const T*)gamma, mean,    \
                                                                   rstd, (T*)dx, rows, D);                            \
-    layernorm_bwd_dgb_kernel<T><<<grid_gb, 256, 0, STREAM>>>((const T*)dy, (const T*)x, mean, rstd, partial, rows, D, \
+    nb::launch_following(layernorm_bwd_dgb_kernel<T>, grid_gb, 256, 0, STREAM, (const T*)dy, (const T*)x, mean, rstd, partial, rows, D, \
                                                               rpb);                                                   \
   }
 #define LN_BWD_ONE_PASS(T, ADD)                                                                                       \
   {                                                                                                                   \
     if (vpl == 1)                                                                                                     \
-      layernorm_bwd_fused_kernel<T, ADD><<<nb, 128, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
+      nb::launch_following(layernorm_bwd_fused_kernel<T, ADD>, nb, 128, 0, STREAM, (const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
                                                                  (const T*)add, (T*)dx, partial, rows, D);            \
     else {                                                                                                            \
       const int rb = vpl < 8 ? 8 / vpl : 1, smem = 32 * vpl * rb * 16 * 2 * 2 * (ADD ? 3 : 2);                        \
       const auto kernel = layernorm_bwd_rows_kernel<T, ADD>;                                                          \
       if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
-      kernel<<<nb, 32 * vpl * rb, smem, STREAM>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)add, (T*)dx, \
+      nb::launch_following(kernel, nb, 32 * vpl * rb, smem, STREAM, (const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)add, (T*)dx, \
                                                   partial, rows, D, vpl, rb);                                         \
     }                                                                                                                 \
   }
@@ -2752,8 +2799,8 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
 #undef LN_BWD
 #undef LN_BWD_ONE_PASS
   const dim3 grid_fold((D + 31) / 32, 2);
-  if (dtype) colsum_partials_kernel<bf16><<<grid_fold, 1024, 0, STREAM>>>(partial, (bf16*)dgamma, (bf16*)dbeta, nb, D);
-  else colsum_partials_kernel<float><<<grid_fold, 1024, 0, STREAM>>>(partial, (float*)dgamma, (float*)dbeta, nb, D);
+  if (dtype) nb::launch_following(colsum_partials_kernel<bf16>, grid_fold, 1024, 0, STREAM, partial, (bf16*)dgamma, (bf16*)dbeta, nb, D);
+  else nb::launch_following(colsum_partials_kernel<float>, grid_fold, 1024, 0, STREAM, partial, (float*)dgamma, (float*)dbeta, nb, D);
   return CHECK_LAUNCH();
 }
 
@@ -2784,12 +2831,12 @@ int nb_colsum(const void* x, void* out, float* partial, int rows, int N, int in_
   const int np = nb_colsum_nparts(rows, N, in_dtype);
   const int rpb = (rows + np - 1) / np;
   if (colsum_narrow(rows, N, V)) {
-    if (in_dtype) colsum_narrow_kernel<bf16><<<np, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
-    else colsum_narrow_kernel<float><<<np, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
+    if (in_dtype) nb::launch_following(colsum_narrow_kernel<bf16>, np, 256, 0, STREAM, (const bf16*)x, partial, rows, N, rpb);
+    else nb::launch_following(colsum_narrow_kernel<float>, np, 256, 0, STREAM, (const float*)x, partial, rows, N, rpb);
   } else {
     const dim3 grid((N + 32 * V - 1) / (32 * V), np);
-    if (in_dtype) colsum_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, partial, rows, N, rpb);
-    else colsum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, partial, rows, N, rpb);
+    if (in_dtype) nb::launch_following(colsum_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, partial, rows, N, rpb);
+    else nb::launch_following(colsum_kernel<float>, grid, 256, 0, STREAM, (const float*)x, partial, rows, N, rpb);
   }
   if (out_dtype) fold_slices<bf16>(partial, out, (size_t)N, np, STREAM);
   else fold_slices<float>(partial, out, (size_t)N, np, STREAM);
@@ -2815,9 +2862,9 @@ int nb_colsum_group(const void* const* x, void* const* out, const int* rows, con
     if (g.count == 0) break;
     const dim3 grid(tiles, COLSUM_CLUSTER);
     if (in_dtype) {
-      if (wide) colsum_group_kernel<bf16, 32><<<grid, 256, 0, STREAM>>>(g); else colsum_group_kernel<bf16, 8><<<grid, 256, 0, STREAM>>>(g);
+      if (wide) nb::launch_following(colsum_group_kernel<bf16, 32>, grid, 256, 0, STREAM, g); else nb::launch_following(colsum_group_kernel<bf16, 8>, grid, 256, 0, STREAM, g);
     } else {
-      if (wide) colsum_group_kernel<float, 32><<<grid, 256, 0, STREAM>>>(g); else colsum_group_kernel<float, 8><<<grid, 256, 0, STREAM>>>(g);
+      if (wide) nb::launch_following(colsum_group_kernel<float, 32>, grid, 256, 0, STREAM, g); else nb::launch_following(colsum_group_kernel<float, 8>, grid, 256, 0, STREAM, g);
     }
     ++launches;
   }
@@ -2827,11 +2874,11 @@ int nb_colsum_group(const void* const* x, void* const* out, const int* rows, con
 int nb_softmax(const void* x, void* y, int rows, int D, int log, int dtype, void* stream) {
   if (rows <= 0) return 0;
   if (dtype) {
-    if (log) softmax_kernel<bf16, true><<<rows, 256, 0, STREAM>>>((const bf16*)x, (bf16*)y, rows, D);
-    else softmax_kernel<bf16, false><<<rows, 256, 0, STREAM>>>((const bf16*)x, (bf16*)y, rows, D);
+    if (log) nb::launch_following(softmax_kernel<bf16, true>, rows, 256, 0, STREAM, (const bf16*)x, (bf16*)y, rows, D);
+    else nb::launch_following(softmax_kernel<bf16, false>, rows, 256, 0, STREAM, (const bf16*)x, (bf16*)y, rows, D);
   } else {
-    if (log) softmax_kernel<float, true><<<rows, 256, 0, STREAM>>>((const float*)x, (float*)y, rows, D);
-    else softmax_kernel<float, false><<<rows, 256, 0, STREAM>>>((const float*)x, (float*)y, rows, D);
+    if (log) nb::launch_following(softmax_kernel<float, true>, rows, 256, 0, STREAM, (const float*)x, (float*)y, rows, D);
+    else nb::launch_following(softmax_kernel<float, false>, rows, 256, 0, STREAM, (const float*)x, (float*)y, rows, D);
   }
   return CHECK_LAUNCH();
 }
@@ -2841,7 +2888,7 @@ int nb_lse_pick_fwd(const void* logits, const long long* tgt, float* lse, float*
   if (rows <= 0) return 0;
   const bool whole = D % (dtype ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
   const bool wide = D >= 8 * 256 * (dtype ? 8 : 4);
-#define LSE_V(T, W, WIDE) lse_pick_fwd_kernel<T, W, WIDE><<<rows, 256, 0, STREAM>>>((const T*)logits, tgt, lse, picked, rows, D)
+#define LSE_V(T, W, WIDE) nb::launch_following(lse_pick_fwd_kernel<T, W, WIDE>, rows, 256, 0, STREAM, (const T*)logits, tgt, lse, picked, rows, D)
 #define LSE(T, W) do { if (wide) LSE_V(T, W, true); else LSE_V(T, W, false); } while (0)
   if (dtype) { if (whole) LSE(bf16, true); else LSE(bf16, false); }
   else { if (whole) LSE(float, true); else LSE(float, false); }
@@ -2853,7 +2900,7 @@ int nb_lse_pick_bwd(const void* logits, const long long* tgt, const float* lse, 
                     void* dlogits, int rows, int D, int dtype, void* stream) {
   if (rows <= 0) return 0;
   const bool whole = D % (dtype ? 8 : 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0;
-#define LSE(T, W) lse_pick_bwd_kernel<T, W><<<rows, 256, 0, STREAM>>>((const T*)logits, tgt, lse, g_lse, g_pick, (T*)dlogits, rows, D)
+#define LSE(T, W) nb::launch_following(lse_pick_bwd_kernel<T, W>, rows, 256, 0, STREAM, (const T*)logits, tgt, lse, g_lse, g_pick, (T*)dlogits, rows, D)
   if (dtype) { if (whole) LSE(bf16, true); else LSE(bf16, false); }
   else { if (whole) LSE(float, true); else LSE(float, false); }
 #undef LSE
@@ -2866,7 +2913,7 @@ int nb_adamw(const void* p, const void* g, const float* m, const float* v, void*
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)n, 256 * 8, 148 * 8);
   const AdamHyper h{lr, b1, b2, eps, wd, bc1, bc2, grad_scale};
-#define ADAMW(TP, TG) adamw_kernel<TP, TG><<<grid, 256, 0, STREAM>>>((const TP*)p, (const TG*)g, m, v, (TP*)p_out, m_out, v_out, (size_t)n, h, hyper)
+#define ADAMW(TP, TG) nb::launch_following(adamw_kernel<TP, TG>, grid, 256, 0, STREAM, (const TP*)p, (const TG*)g, m, v, (TP*)p_out, m_out, v_out, (size_t)n, h, hyper)
   if (p_dtype) { if (g_dtype) ADAMW(bf16, bf16); else ADAMW(bf16, float); }
   else { if (g_dtype) ADAMW(float, bf16); else ADAMW(float, float); }
 #undef ADAMW
@@ -2893,7 +2940,7 @@ int nb_adamw_group(const void* const* p, const void* const* g, const float* cons
       blocks += ((unsigned)n[k] + 2047) / 2048;
     }
     if (c.count == 0) break;
-#define ADAMW(TP, TG) adamw_group_kernel<TP, TG><<<blocks, 256, 0, STREAM>>>(c, h, hyper)
+#define ADAMW(TP, TG) nb::launch_following(adamw_group_kernel<TP, TG>, blocks, 256, 0, STREAM, c, h, hyper)
     if (p_dtype) { if (g_dtype) ADAMW(bf16, bf16); else ADAMW(bf16, float); }
     else { if (g_dtype) ADAMW(float, bf16); else ADAMW(float, float); }
 #undef ADAMW
@@ -2901,13 +2948,13 @@ int nb_adamw_group(const void* const* p, const void* const* g, const float* cons
   return CHECK_LAUNCH();
 }
 int nb_adam_hyper(const float* step, const float* plus, float* total, float* hyper, float lr, double b1, double b2, void* stream) {
-  adam_hyper_kernel<<<1, 1, 0, STREAM>>>(step, plus, total, hyper, lr, b1, b2);
+  nb::launch_following(adam_hyper_kernel, 1, 1, 0, STREAM, step, plus, total, hyper, lr, b1, b2);
   return CHECK_LAUNCH();
 }
 int nb_mean_diff(const void* a, const void* b, void* d, void* out, long long n, int square, const void* count_at, float count, int dtype,
                  void* stream) {
   if (n <= 0 || n > (1 << 20)) return -2;
-#define MEAN(T, C) mean_diff_kernel<T, C><<<C, MEAN_THREADS, 0, STREAM>>>((const T*)a, (const T*)b, (T*)d, (T*)out, (int)n, square, (const T*)count_at, count)
+#define MEAN(T, C) nb::launch_following(mean_diff_kernel<T, C>, C, MEAN_THREADS, 0, STREAM, (const T*)a, (const T*)b, (T*)d, (T*)out, (int)n, square, (const T*)count_at, count)
   if (n <= 4 * MEAN_THREADS) { if (dtype) MEAN(bf16, 1); else MEAN(float, 1); }
   else { if (dtype) MEAN(bf16, 8); else MEAN(float, 8); }
 #undef MEAN
@@ -2917,7 +2964,7 @@ int nb_sgd(const void* p, const void* g, const float* buf, void* p_out, float* b
            float momentum, float wd, float grad_scale, int p_dtype, int g_dtype, void* stream) {
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)n, 256);
-#define SGD(TP, TG) sgd_kernel<TP, TG><<<grid, 256, 0, STREAM>>>((const TP*)p, (const TG*)g, buf, (TP*)p_out, buf_out, (size_t)n, lr, momentum, wd, grad_scale)
+#define SGD(TP, TG) nb::launch_following(sgd_kernel<TP, TG>, grid, 256, 0, STREAM, (const TP*)p, (const TG*)g, buf, (TP*)p_out, buf_out, (size_t)n, lr, momentum, wd, grad_scale)
   if (p_dtype && g_dtype) SGD(bf16, bf16);
   else if (p_dtype) SGD(bf16, float);
   else if (g_dtype) SGD(float, bf16);
@@ -2929,7 +2976,7 @@ int nb_embedding_gather(const void* table, const long long* ids, const void* add
                         int period, int dtype, void* stream) {
   if (n_ids <= 0) return 0;
   if (add != nullptr && period <= 0) return -2;
-#define GATHER(T, ADD) embedding_gather_kernel<T, ADD><<<n_ids, 128, 0, STREAM>>>((const T*)table, ids, (const T*)add, (T*)out, n_ids, D, vocab, period)
+#define GATHER(T, ADD) nb::launch_following(embedding_gather_kernel<T, ADD>, n_ids, 128, 0, STREAM, (const T*)table, ids, (const T*)add, (T*)out, n_ids, D, vocab, period)
   if (dtype) { if (add) GATHER(bf16, true); else GATHER(bf16, false); }
   else { if (add) GATHER(float, true); else GATHER(float, false); }
 #undef GATHER
@@ -2964,13 +3011,13 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
     float* acc = direct ? (float*)out : reinterpret_cast<float*>(work);
     if (cudaMemsetAsync(acc, 0, n * sizeof(float), STREAM) != cudaSuccess) return -1;
     const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(acc)) & 15) == 0;
-#define SCAT(T, VEC) embedding_scatter_add_kernel<T, VEC><<<n_ids, 128, 0, STREAM>>>(acc, ids, (const T*)upd, n_ids, D, vocab)
+#define SCAT(T, VEC) nb::launch_following(embedding_scatter_add_kernel<T, VEC>, n_ids, 128, 0, STREAM, acc, ids, (const T*)upd, n_ids, D, vocab)
     if (dtype) { if (vec) SCAT(bf16, true); else SCAT(bf16, false); }
     else { if (vec) SCAT(float, true); else SCAT(float, false); }
 #undef SCAT
     const int grid = grid_for(n, 256);
-    if (dtype) cast_kernel<float, bf16><<<grid, 256, 0, STREAM>>>(acc, (bf16*)out, n, (const bf16*)base);
-    else if (!direct) cast_kernel<float, float><<<grid, 256, 0, STREAM>>>(acc, (float*)out, n, (const float*)base);
+    if (dtype) nb::launch_following(cast_kernel<float, bf16>, grid, 256, 0, STREAM, acc, (bf16*)out, n, (const bf16*)base);
+    else if (!direct) nb::launch_following(cast_kernel<float, float>, grid, 256, 0, STREAM, acc, (float*)out, n, (const float*)base);
     return CHECK_LAUNCH();
   }
   // Crowded tables: rows of few entries are few, and the time is that of the long ones. us, all rows in one launch and a copied base
@@ -3001,9 +3048,9 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
   float* part = reinterpret_cast<float*>(ws.seg + n_ids);
   const int idb = (n_ids + 255) / 256;
   if (cudaMemsetAsync(work, 0, (2 * (size_t)vocab + 4 + scat_max_heavy(n_ids)) * sizeof(int), STREAM) != cudaSuccess) return -1;
-  scatter_count_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
-  scatter_slots_kernel<<<(vocab + 255) / 256, 256, 0, STREAM>>>(ws, n_ids, vocab);
-  scatter_place_kernel<<<idb, 256, 0, STREAM>>>(ids, ws, n_ids, vocab);
+  nb::launch_following(scatter_count_kernel, idb, 256, 0, STREAM, ids, ws, n_ids, vocab);
+  nb::launch_following(scatter_slots_kernel, (vocab + 255) / 256, 256, 0, STREAM, ws, n_ids, vocab);
+  nb::launch_following(scatter_place_kernel, idb, 256, 0, STREAM, ids, ws, n_ids, vocab);
   const int V = dtype ? 8 : 4;
   const bool vec = D % V == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   int threads = 32;                                  // the power of two that covers a row in one pass, at most 256
@@ -3013,7 +3060,7 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
   const long long held = 148ll * (crowded ? 2048 : 4 * (vec && dtype ? 768 : 1024)) / threads;
   const long long want = crowded ? n_ids : ((long long)vocab / SCAT_IDLE + 1) * 32 / threads + 1;
   const int grid = (int)(held < n_ids || held < want ? held : n_ids > want ? n_ids : want);
-#define SCAT_R(T, VN, ALL) scatter_rows_kernel<T, VN, ALL><<<grid, threads, 0, STREAM>>>((const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D, vocab)
+#define SCAT_R(T, VN, ALL) nb::launch_following(scatter_rows_kernel<T, VN, ALL>, grid, threads, 0, STREAM, (const T*)upd, (const T*)base, (T*)out, ws, part, n_ids, D, vocab)
 #define SCAT(T, VN) do { if (crowded) SCAT_R(T, VN, false); else SCAT_R(T, VN, true); } while (0)
   if (dtype) { if (vec) SCAT(bf16, 8); else SCAT(bf16, 1); }
   else { if (vec) SCAT(float, 4); else SCAT(float, 1); }
@@ -3026,8 +3073,8 @@ int nb_embedding_scatter_add(int* work, const long long* ids, const void* upd, c
 int nb_embedding_scatter_sorted(const long long* sorted_ids, const long long* perm, const void* upd, const void* base,
                                 void* out, int n_ids, int D, int vocab, int dtype, void* stream) {
   if (n_ids <= 0) return 0;
-  if (dtype) embedding_scatter_sorted_kernel<bf16><<<n_ids, 128, 0, STREAM>>>(sorted_ids, perm, (const bf16*)upd, (const bf16*)base, (bf16*)out, n_ids, D, vocab);
-  else embedding_scatter_sorted_kernel<float><<<n_ids, 128, 0, STREAM>>>(sorted_ids, perm, (const float*)upd, (const float*)base, (float*)out, n_ids, D, vocab);
+  if (dtype) nb::launch_following(embedding_scatter_sorted_kernel<bf16>, n_ids, 128, 0, STREAM, sorted_ids, perm, (const bf16*)upd, (const bf16*)base, (bf16*)out, n_ids, D, vocab);
+  else nb::launch_following(embedding_scatter_sorted_kernel<float>, n_ids, 128, 0, STREAM, sorted_ids, perm, (const float*)upd, (const float*)base, (float*)out, n_ids, D, vocab);
   return CHECK_LAUNCH();
 }
 
@@ -3054,7 +3101,7 @@ int nb_copy_batch(void* const* dst, const void* const* src, const unsigned long 
     }
     if (c.n == 0) break;
     c.first[c.n] = (unsigned)blocks;
-    copy_batch_kernel<<<(unsigned)blocks, 256, 0, STREAM>>>(c);
+    nb::launch_following(copy_batch_kernel, (unsigned)blocks, 256, 0, STREAM, c);
     ++launches;
   }
   return cudaGetLastError() == cudaSuccess ? launches : -1;
@@ -3063,8 +3110,8 @@ int nb_copy_batch(void* const* dst, const void* const* src, const unsigned long 
 int nb_cast(const void* in, void* out, long long n, int in_dtype, int out_dtype, void* stream) {
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)n, 256);
-  if (in_dtype && !out_dtype) cast_kernel<bf16, float><<<grid, 256, 0, STREAM>>>((const bf16*)in, (float*)out, (size_t)n, nullptr);
-  else if (!in_dtype && out_dtype) cast_kernel<float, bf16><<<grid, 256, 0, STREAM>>>((const float*)in, (bf16*)out, (size_t)n, nullptr);
+  if (in_dtype && !out_dtype) nb::launch_following(cast_kernel<bf16, float>, grid, 256, 0, STREAM, (const bf16*)in, (float*)out, (size_t)n, nullptr);
+  else if (!in_dtype && out_dtype) nb::launch_following(cast_kernel<float, bf16>, grid, 256, 0, STREAM, (const float*)in, (bf16*)out, (size_t)n, nullptr);
   else return -2;
   return CHECK_LAUNCH();
 }
@@ -3074,11 +3121,11 @@ int nb_activation(const void* z, const void* dy, void* out, long long n, int mod
   const int V = dtype ? 8 : 4;
   const int grid = grid_for((size_t)n, 256 * V);
   if (dtype) {
-    if (bwd) act_kernel<bf16, true><<<grid, 256, 0, STREAM>>>((const bf16*)z, (const bf16*)dy, (bf16*)out, (size_t)n, mode);
-    else act_kernel<bf16, false><<<grid, 256, 0, STREAM>>>((const bf16*)z, nullptr, (bf16*)out, (size_t)n, mode);
+    if (bwd) nb::launch_following(act_kernel<bf16, true>, grid, 256, 0, STREAM, (const bf16*)z, (const bf16*)dy, (bf16*)out, (size_t)n, mode);
+    else nb::launch_following(act_kernel<bf16, false>, grid, 256, 0, STREAM, (const bf16*)z, nullptr, (bf16*)out, (size_t)n, mode);
   } else {
-    if (bwd) act_kernel<float, true><<<grid, 256, 0, STREAM>>>((const float*)z, (const float*)dy, (float*)out, (size_t)n, mode);
-    else act_kernel<float, false><<<grid, 256, 0, STREAM>>>((const float*)z, nullptr, (float*)out, (size_t)n, mode);
+    if (bwd) nb::launch_following(act_kernel<float, true>, grid, 256, 0, STREAM, (const float*)z, (const float*)dy, (float*)out, (size_t)n, mode);
+    else nb::launch_following(act_kernel<float, false>, grid, 256, 0, STREAM, (const float*)z, nullptr, (float*)out, (size_t)n, mode);
   }
   return CHECK_LAUNCH();
 }
@@ -3087,16 +3134,16 @@ int nb_rng(void* out, long long n, unsigned long long seed, unsigned long long o
            int dtype, void* stream) {
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)n, 256 * 4, 148 * 8);
-  if (dtype) rng_kernel<bf16><<<grid, 256, 0, STREAM>>>((bf16*)out, (size_t)n, seed, offset, mode, a, b, nullptr);
-  else rng_kernel<float><<<grid, 256, 0, STREAM>>>((float*)out, (size_t)n, seed, offset, mode, a, b, nullptr);
+  if (dtype) nb::launch_following(rng_kernel<bf16>, grid, 256, 0, STREAM, (bf16*)out, (size_t)n, seed, offset, mode, a, b, nullptr);
+  else nb::launch_following(rng_kernel<float>, grid, 256, 0, STREAM, (float*)out, (size_t)n, seed, offset, mode, a, b, nullptr);
   return CHECK_LAUNCH();
 }
 int nb_dropout(const void* x, void* y, unsigned char* mask, long long n, float p, unsigned long long seed,
                unsigned long long offset, int dtype, void* stream) {
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)n, 256 * 4, 148 * 8);
-  if (dtype) dropout_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (bf16*)y, mask, (size_t)n, p, seed, offset, nullptr);
-  else dropout_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)y, mask, (size_t)n, p, seed, offset, nullptr);
+  if (dtype) nb::launch_following(dropout_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, (bf16*)y, mask, (size_t)n, p, seed, offset, nullptr);
+  else nb::launch_following(dropout_kernel<float>, grid, 256, 0, STREAM, (const float*)x, (float*)y, mask, (size_t)n, p, seed, offset, nullptr);
   return CHECK_LAUNCH();
 }
 // Variants whose stream position lives on the device: `state` = [seed, draws so far] (two 64-bit
@@ -3106,20 +3153,20 @@ int nb_rng_dev(void* out, long long n, unsigned long long* state, unsigned long 
                int dtype, void* stream) {
   if (n > 0) {
     const int grid = grid_for((size_t)n, 256 * 4, 148 * 8);
-    if (dtype) rng_kernel<bf16><<<grid, 256, 0, STREAM>>>((bf16*)out, (size_t)n, salt, 0, mode, a, b, state);
-    else rng_kernel<float><<<grid, 256, 0, STREAM>>>((float*)out, (size_t)n, salt, 0, mode, a, b, state);
+    if (dtype) nb::launch_following(rng_kernel<bf16>, grid, 256, 0, STREAM, (bf16*)out, (size_t)n, salt, 0, mode, a, b, state);
+    else nb::launch_following(rng_kernel<float>, grid, 256, 0, STREAM, (float*)out, (size_t)n, salt, 0, mode, a, b, state);
   }
-  rng_bump_kernel<<<1, 1, 0, STREAM>>>(state);
+  nb::launch_following(rng_bump_kernel, 1, 1, 0, STREAM, state);
   return CHECK_LAUNCH();
 }
 int nb_dropout_dev(const void* x, void* y, unsigned char* mask, long long n, float p, unsigned long long* state,
                    unsigned long long salt, int dtype, void* stream) {
   if (n > 0) {
     const int grid = grid_for((size_t)n, 256 * 4, 148 * 8);
-    if (dtype) dropout_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (bf16*)y, mask, (size_t)n, p, salt, 0, state);
-    else dropout_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)y, mask, (size_t)n, p, salt, 0, state);
+    if (dtype) nb::launch_following(dropout_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, (bf16*)y, mask, (size_t)n, p, salt, 0, state);
+    else nb::launch_following(dropout_kernel<float>, grid, 256, 0, STREAM, (const float*)x, (float*)y, mask, (size_t)n, p, salt, 0, state);
   }
-  rng_bump_kernel<<<1, 1, 0, STREAM>>>(state);
+  nb::launch_following(rng_bump_kernel, 1, 1, 0, STREAM, state);
   return CHECK_LAUNCH();
 }
 
@@ -3127,8 +3174,8 @@ int nb_nf4_dequant(const unsigned char* packed, const float* absmax, void* out, 
                    void* stream) {
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)(n + 1) / 2, 256);
-  if (dtype) nf4_dequant_kernel<bf16><<<grid, 256, 0, STREAM>>>(packed, absmax, (bf16*)out, (size_t)n, block);
-  else nf4_dequant_kernel<float><<<grid, 256, 0, STREAM>>>(packed, absmax, (float*)out, (size_t)n, block);
+  if (dtype) nb::launch_following(nf4_dequant_kernel<bf16>, grid, 256, 0, STREAM, packed, absmax, (bf16*)out, (size_t)n, block);
+  else nb::launch_following(nf4_dequant_kernel<float>, grid, 256, 0, STREAM, packed, absmax, (float*)out, (size_t)n, block);
   return CHECK_LAUNCH();
 }
 
@@ -3137,7 +3184,7 @@ int nb_nf4_dequant_codes(const unsigned char* codes, const float* absmax, const 
   if (n <= 0) return 0;
   const int grid = grid_for((size_t)(n + 15) / 16, 256);
   const bool whole = block % 16 == 0 && ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-#define NF4(T, W) nf4_dequant_codes_kernel<T, W><<<grid, 256, 0, STREAM>>>(codes, absmax, codebook, (T*)out, (size_t)n, block)
+#define NF4(T, W) nb::launch_following(nf4_dequant_codes_kernel<T, W>, grid, 256, 0, STREAM, codes, absmax, codebook, (T*)out, (size_t)n, block)
   if (dtype) { if (whole) NF4(bf16, true); else NF4(bf16, false); }
   else { if (whole) NF4(float, true); else NF4(float, false); }
 #undef NF4
@@ -3152,15 +3199,15 @@ int nb_pool2d_fwd(const void* x, void* y, int N, int H, int W, int C, int OH, in
   CellGeom g;
   if (pool_cells(x, y, nullptr, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g)) {
     const unsigned n = (unsigned)(total / V);
-#define POOL(T, MAX) pool2d_cell_fwd_kernel<T, MAX><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (T*)y, g, n)
+#define POOL(T, MAX) nb::launch_following(pool2d_cell_fwd_kernel<T, MAX>, (n + 255) / 256, 256, 0, STREAM, (const T*)x, (T*)y, g, n)
     if (dtype) { if (mode) POOL(bf16, true); else POOL(bf16, false); }
     else { if (mode) POOL(float, true); else POOL(float, false); }
 #undef POOL
     return CHECK_LAUNCH();
   }
   const int grid = grid_for(total, 256);
-  if (dtype) pool2d_fwd_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (bf16*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
-  else pool2d_fwd_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (float*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
+  if (dtype) nb::launch_following(pool2d_fwd_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, (bf16*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
+  else nb::launch_following(pool2d_fwd_kernel<float>, grid, 256, 0, STREAM, (const float*)x, (float*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode);
   return CHECK_LAUNCH();
 }
 int nb_pool2d_bwd(const void* x, const void* dy, void* dx, int N, int H, int W, int C, int OH, int OW, int kh, int kw,
@@ -3172,15 +3219,15 @@ int nb_pool2d_bwd(const void* x, const void* dy, void* dx, int N, int H, int W, 
   CellGeom g;
   if (pool_cells(x, dy, dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, V, g) && (mode == 1 || pool_cells_avg_bwd(N, C, g))) {
     const unsigned n = (unsigned)((size_t)N * g.cells_h * g.cells_w * g.CV);
-#define POOL(T, ...) pool2d_cell_bwd_kernel<T, __VA_ARGS__><<<(n + 255) / 256, 256, 0, STREAM>>>((const T*)x, (const T*)dy, (T*)dx, g, n)
+#define POOL(T, ...) nb::launch_following(pool2d_cell_bwd_kernel<T, __VA_ARGS__>, (n + 255) / 256, 256, 0, STREAM, (const T*)x, (const T*)dy, (T*)dx, g, n)
     if (dtype) { if (relu) POOL(bf16, true, true); else if (mode) POOL(bf16, true); else POOL(bf16, false); }
     else { if (relu) POOL(float, true, true); else if (mode) POOL(float, true); else POOL(float, false); }
 #undef POOL
     return CHECK_LAUNCH();
   }
   const int grid = grid_for(total, 256);
-  if (dtype) pool2d_bwd_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (const bf16*)dy, (bf16*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode, relu);
-  else pool2d_bwd_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (const float*)dy, (float*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode, relu);
+  if (dtype) nb::launch_following(pool2d_bwd_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, (const bf16*)dy, (bf16*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode, relu);
+  else nb::launch_following(pool2d_bwd_kernel<float>, grid, 256, 0, STREAM, (const float*)x, (const float*)dy, (float*)dx, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw, mode, relu);
   return CHECK_LAUNCH();
 }
 
@@ -3189,8 +3236,8 @@ int nb_pool2d_select(const void* x, const void* t, void* y, int N, int H, int W,
   const size_t total = (size_t)N * OH * OW * C;
   if (!total) return 0;
   const int grid = grid_for(total, 256);
-  if (dtype) pool2d_select_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)x, (const bf16*)t, (bf16*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw);
-  else pool2d_select_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)x, (const float*)t, (float*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw);
+  if (dtype) nb::launch_following(pool2d_select_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)x, (const bf16*)t, (bf16*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw);
+  else nb::launch_following(pool2d_select_kernel<float>, grid, 256, 0, STREAM, (const float*)x, (const float*)t, (float*)y, N, H, W, C, OH, OW, kh, kw, sh, sw, ph, pw);
   return CHECK_LAUNCH();
 }
 
@@ -3242,8 +3289,8 @@ int nb_conv_flip(const void* w, void* out, int R, int S, int C, int F, int dtype
   if (n <= 0) return 0;
   if (n > 0x7fffffffll) return -2;
   const unsigned grid = (unsigned)((n + 255) / 256);
-  if (dtype) conv_flip_kernel<bf16><<<grid, 256, 0, STREAM>>>((const bf16*)w, (bf16*)out, R * S, C, F, (unsigned)n);
-  else conv_flip_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)w, (float*)out, R * S, C, F, (unsigned)n);
+  if (dtype) nb::launch_following(conv_flip_kernel<bf16>, grid, 256, 0, STREAM, (const bf16*)w, (bf16*)out, R * S, C, F, (unsigned)n);
+  else nb::launch_following(conv_flip_kernel<float>, grid, 256, 0, STREAM, (const float*)w, (float*)out, R * S, C, F, (unsigned)n);
   return CHECK_LAUNCH();
 }
 int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int R, int S,
@@ -3263,7 +3310,7 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
     const int px = pp.px, th = pp.th, bands = pp.bands, fg_w = pp.fg;
     const size_t smem = 4 * ((size_t)R * S * C * 4 * fg_w + (size_t)((th - 1) * sh + R) * ((OW - 1) * sw + S) * C);
     const dim3 pgrid((unsigned)(N * bands), (unsigned)pp.f_tiles);
-#define PATCH_V(T, FG, PX, VEC) conv2d_patch_kernel<T, FG, PX, VEC><<<pgrid, 128, smem, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec, relu)
+#define PATCH_V(T, FG, PX, VEC) nb::launch_following(conv2d_patch_kernel<T, FG, PX, VEC>, pgrid, 128, smem, STREAM, (const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec, relu)
 #define PATCH_P(T, FG, PX) do { if (vec) PATCH_V(T, FG, PX, true); else PATCH_V(T, FG, PX, false); } while (0)
 #define PATCH(T, FG) do { if (px == 8) PATCH_P(T, FG, 8); else PATCH_P(T, FG, 4); } while (0)
     if (dtype) { if (fg_w == 2) PATCH(bf16, 2); else if (fg_w == 4) PATCH(bf16, 4); else PATCH(bf16, 8); }
@@ -3273,7 +3320,7 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
 #undef PATCH_V
     return CHECK_LAUNCH();
   }
-#define CONV_V(T, FG, VEC) conv2d_direct_kernel<T, FG, VEC><<<grid(FG), 128, 0, STREAM>>>((const T*)x, (const T*)w, (const T*)bias, (T*)y, g, relu)
+#define CONV_V(T, FG, VEC) nb::launch_following(conv2d_direct_kernel<T, FG, VEC>, grid(FG), 128, 0, STREAM, (const T*)x, (const T*)w, (const T*)bias, (T*)y, g, relu)
 #define CONV(T, FG) do { if (vec) CONV_V(T, FG, true); else CONV_V(T, FG, false); } while (0)
   if (dtype) { if (F <= 8) CONV(bf16, 2); else if (F <= 16) CONV(bf16, 4); else CONV(bf16, 8); }
   else { if (F <= 8) CONV(float, 2); else if (F <= 16) CONV(float, 4); else CONV(float, 8); }
@@ -3299,8 +3346,8 @@ int nb_sgemm(const float* a, const float* b, const float* bias, float* out, floa
   const int per = ((K + z - 1) / z + SG - 1) / SG * SG;
   z = (K + per - 1) / per;
   const SgemmArgs g{a, b, bias, z > 1 ? partial : out, M, N, K, per, a_m, a_k, b_k, b_n};
-  sgemm_kernel<<<dim3((N + SG - 1) / SG, (M + SG - 1) / SG, z), 256, 0, STREAM>>>(g);
-  if (z > 1) sgemm_fold_kernel<<<(M * N + 31) / 32, 256, 0, STREAM>>>(partial, bias, out, M * N, N, z);
+  nb::launch_following(sgemm_kernel, dim3((N + SG - 1) / SG, (M + SG - 1) / SG, z), 256, 0, STREAM, g);
+  if (z > 1) nb::launch_following(sgemm_fold_kernel, (M * N + 31) / 32, 256, 0, STREAM, partial, bias, out, M * N, N, z);
   return CHECK_LAUNCH();
 }
 
@@ -3308,8 +3355,8 @@ int nb_sum_slices(const float* part, void* out, long long n, int slices, int dty
   if (n <= 0 || slices <= 0) return 0;
   if (n & 3) return -2;
   const int grid = grid_for((size_t)n / 4, 256, 148 * 8);
-  if (dtype) sum_slices_kernel<bf16><<<grid, 256, 0, STREAM>>>(part, (bf16*)out, (size_t)n, slices);
-  else sum_slices_kernel<float><<<grid, 256, 0, STREAM>>>(part, (float*)out, (size_t)n, slices);
+  if (dtype) nb::launch_following(sum_slices_kernel<bf16>, grid, 256, 0, STREAM, part, (bf16*)out, (size_t)n, slices);
+  else nb::launch_following(sum_slices_kernel<float>, grid, 256, 0, STREAM, part, (float*)out, (size_t)n, slices);
   return CHECK_LAUNCH();
 }
 
@@ -3379,8 +3426,8 @@ int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part,
   const size_t dyn = smem < 8192 ? 8192 : (size_t)smem;    // (the sum of the position slices of a block takes 8 KB)
 #define WGRAD_V(T, KG, FG, VEC)                                                                                                          \
   do {                                                                                                                                   \
-    if (patch) conv2d_wgrad_patch_kernel<T, KG, FG, VEC><<<dim3((K + 4 * KG - 1) / (4 * KG), (F + 4 * FG - 1) / (4 * FG), zp), 128, dyn, STREAM>>>((const T*)x, (const T*)dy, part, g, th, bands, (int)total, dvec); \
-    else conv2d_wgrad_direct_kernel<T, KG, FG, VEC><<<dim3((K + 4 * KG - 1) / (4 * KG), (F + 4 * FG - 1) / (4 * FG), z), 128, 0, STREAM>>>((const T*)x, (const T*)dy, part, g, per);  \
+    if (patch) nb::launch_following(conv2d_wgrad_patch_kernel<T, KG, FG, VEC>, dim3((K + 4 * KG - 1) / (4 * KG), (F + 4 * FG - 1) / (4 * FG), zp), 128, dyn, STREAM, (const T*)x, (const T*)dy, part, g, th, bands, (int)total, dvec); \
+    else nb::launch_following(conv2d_wgrad_direct_kernel<T, KG, FG, VEC>, dim3((K + 4 * KG - 1) / (4 * KG), (F + 4 * FG - 1) / (4 * FG), z), 128, 0, STREAM, (const T*)x, (const T*)dy, part, g, per);  \
   } while (0)
 #define WGRAD(T, KG, FG) do { if (vec) WGRAD_V(T, KG, FG, true); else WGRAD_V(T, KG, FG, false); } while (0)
 #define WGRAD_T(T)                                                                            \

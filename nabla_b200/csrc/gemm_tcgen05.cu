@@ -20,6 +20,7 @@
 // Replaces what the reference obtains from MAX's matmul (nabla/ops/binary.py:197-198) and the
 // matmul + add + relu/gelu composition of nabla/nn/functional/layers.py:30-35.
 #include "sm100_ptx.cuh"
+#include "launch.cuh"
 #include "nb_debug.cuh"
 #include <atomic>
 #include <stdio.h>
@@ -273,6 +274,7 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
   if (PAIR) cluster_sync_all();      // the other CTA's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (MODE == MODE_NONE) follow_grid();
   if (!PAIR && s_abort != 0) {               // uniform for the whole CTA
     if (warp == 2) tmem_dealloc(tmem_base, 2 * BN);
     return false;
@@ -914,6 +916,7 @@ gemm_bf16_slices_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  follow_grid();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -1537,7 +1540,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
   long long tiles = (long long)num_m * num_n * a.batch;
   int grid = (int)(tiles < max_ctas ? tiles : max_ctas);
   if (grid < 1) return 0;
-  gemm_bf16_tcgen05_kernel<BN><<<grid, NUM_THREADS, L::TOTAL, stream>>>(ta, tb, a);
+  launch_following(gemm_bf16_tcgen05_kernel<BN>, grid, NUM_THREADS, L::TOTAL, stream, ta, tb, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -1616,7 +1619,7 @@ static SlicePlan slice_plan(int M, int N, int K, int bn) {
 template <int BN>
 static int launch_slices(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, int slices, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = slices;
   attr[0].val.clusterDim.y = 1;
@@ -1628,6 +1631,7 @@ static int launch_slices(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const auto kernel = slices == 2 ? gemm_bf16_slices_kernel<BN, 2> : slices == 4 ? gemm_bf16_slices_kernel<BN, 4> : gemm_bf16_slices_kernel<BN, 8>;
+  set_following(cfg);
   return cudaLaunchKernelEx(&cfg, kernel, ta, tb, a) == cudaSuccess ? 0 : -3;
 }
 
@@ -1635,7 +1639,7 @@ static int launch_slices(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
 template <int SMEM, typename Kernel>
 static int launch_with(Kernel kernel, int cluster, long long tiles, cudaStream_t stream, const CUtensorMap* maps, const GemmArgs& a) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)cluster;
   attr[0].val.clusterDim.y = 1;
@@ -1656,6 +1660,7 @@ static int launch_with(Kernel kernel, int cluster, long long tiles, cudaStream_t
   if (tiles < n) n = tiles;
   if (n < 1) return 0;
   cfg.gridDim = dim3((unsigned)(cluster * n));
+  set_following(cfg);
   return cudaLaunchKernelEx(&cfg, kernel, maps[0], maps[1], maps[2], maps[3], a) == cudaSuccess ? 0 : -3;
 }
 
@@ -1670,7 +1675,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   using L = SmemLayoutPair<BN>;
   int& max_clusters = g_pair_max_clusters;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -1695,6 +1700,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   if (tiles < pairs) pairs = (int)tiles;
   if (pairs < 1) return 0;
   cfg.gridDim = dim3(2 * pairs);
+  set_following(cfg);
   return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_pair_kernel<BN>, ta, tb, a) == cudaSuccess ? 0 : -3;
 }
 

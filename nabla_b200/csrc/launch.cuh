@@ -1,0 +1,47 @@
+// Launches that follow each other closely. A kernel that starts with follow_grid() and is launched by launch_following() is
+// resident, with its set-up done, before the launch ahead of it in the stream has ended: its blocks take the SMs as that
+// one's leave them, and the start of a grid lies under the last blocks ahead of it. Captured steps, us before and after: a
+// transformer block of 2 x 1001 x 512 199 and 184, four layers of 4 x 333 x 512 257 and 241, two small layers and their Adam
+// 61.5 and 55.9, three attention kernels of 8 x 12 heads x 777 209 and 200; from a tape: an adapter's step at 2048 141 and 130.
+//
+// Rules that keep this the order of the stream:
+//  - nothing in global memory is read or written before follow_grid() (nor loaded into shared memory); it returns when every
+//    grid ahead has ended and its writes are visible. All blocks call it, on every path out of the kernel.
+//  - only then does it let the next launch begin, so no more than two grids of a stream are on the chip. A kernel that takes
+//    tensor memory has it by then: a waiting block may wait for the tensor memory of a running one, never the other way.
+//  - a kernel without follow_grid() is launched with <<< >>> and waits for the end of all that is ahead of it, as before.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace nb {
+
+__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_grid_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void follow_grid() {
+  wait_for_previous_grid();
+  let_next_grid_start();
+}
+
+// Adds the attribute to a launch whose attribute array has room for one more.
+inline void set_following(cudaLaunchConfig_t& cfg) {
+  cudaLaunchAttribute& a = cfg.attrs[cfg.numAttrs++];
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  set_following(cfg);
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+}  // namespace nb

@@ -52,6 +52,32 @@ def test_every_kernel_source_includes_the_check_header_and_uses_it():
     assert "#define NB_ALIGNED(site, value, align) true" in header
 
 
+def test_every_kernel_of_a_following_launch_waits_for_the_grid_ahead():
+    """A kernel that is launched before the grid ahead of it has ended calls follow_grid(), and before any path out of it."""
+    import re
+
+    csrc = ROOT / "nabla_b200" / "csrc"
+    for name in ("gemm_tcgen05.cu", "attention_tcgen05.cu", "fused_kernels.cu", "elementwise_kernels.cu"):
+        src = re.sub(r"//[^\n]*", "", (csrc / name).read_text())
+        cta = src[src.index("bool gemm_cta("):] if "bool gemm_cta(" in src else ""
+        bodies = {}
+        for m in re.finditer("__global__", src):
+            kernel = re.compile(r"(\w+_kernel)\s*\(").search(src, m.end())
+            brace = src.index("{", kernel.end())
+            bodies[kernel.group(1)] = src[brace:src.index("\n}\n", brace)]
+        launched = set(re.findall(r"launch_following\((\w+)", src)) - {"kernel"}
+        launched |= {k for k in bodies if re.match(r"gemm_bf16_|layernorm_bwd_rows", k)}        # (through a pointer to the kernel)
+        assert launched and launched <= set(bodies), name
+        for k in launched:
+            body = bodies[k]
+            if "gemm_cta<" in body:
+                assert "gemm_cta<BN, MODE_NONE" in body
+                body = cta
+            body = body.replace("return follow_grid();", "follow_grid_and_leave;")
+            ahead = re.sub(r"\[&?\]\([^)]*\)[^{;]*\{ return [^}]*\}", "", body[:body.index("follow_grid();")])      # (without lambdas)
+            assert not re.search(r"\breturn\b", ahead), (name, k)
+
+
 @pytest.mark.parametrize("source,kernels", [
     ("fused_kernels.cu", ["layernorm_bwd_rows_kernel", "colsum_narrow_kernel", "scatter_count_kernel", "scatter_slots_kernel", "scatter_place_kernel",
                           "scatter_rows_kernel", "nf4_dequant_codes_kernel", "pool2d_cell_fwd_kernel", "pool2d_cell_bwd_kernel", "pool2d_bwd_kernel",

@@ -601,6 +601,62 @@ def test_rule_of_joined_sums(args, joined):
     assert kernels.joined_sum(*args) == joined
 
 
+# ---------------------------------------------------------------- launches that follow each other
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("rows,width", [(64, 128), (1001, 512), (4096, 1024)])
+def test_launches_that_start_before_the_one_ahead_has_ended(rows, width, captured):
+    """A chain in which every kernel reads what the one ahead of it wrote, in memory that the allocator hands out again at once, and a
+    fork and join of two streams: equal, bit for bit, to the same calls with a synchronisation after each."""
+    from nabla_b200.native import attention, gemm, kernels
+
+    torch.manual_seed(rows)
+    x0 = torch.randn(rows, width, device="cuda").bfloat16()
+    w = (torch.randn(width, width, device="cuda") * width ** -0.5).bfloat16()
+    g, b = (torch.randn(width, device="cuda").bfloat16() for _ in range(2))
+    side = torch.cuda.Stream()
+
+    def chain(between, fork):
+        x, sums = x0, []
+        for _ in range(12):
+            y = kernels.layernorm_fwd(x, g, b, 1e-5)[0]
+            between()
+            main = torch.cuda.current_stream()
+            if fork:
+                side.wait_stream(main)
+                y.record_stream(side)
+            with torch.cuda.stream(side if fork else main):
+                z = gemm.gemm_bf16(y, w)
+            u = gemm.gemm_bf16(y, w.t())
+            if fork:
+                main.wait_stream(side)
+                z.record_stream(main)
+            between()
+            h = [t.view(1, rows, width // 64, 64).transpose(1, 2) for t in (u, z, y)]
+            o, lse = attention.sdpa_fwd(*h, causal=True, scale=0.125)
+            between()
+            d = attention.sdpa_bwd(o, *h, o, lse, causal=True, scale=0.125)
+            between()
+            x = gemm.gemm_bf16(d[0].transpose(1, 2).reshape(rows, width) + o.transpose(1, 2).reshape(rows, width), w)
+            sums += [kernels.colsum(x), d[1].sum(), d[2].sum()]
+            between()
+        return [x, *sums]
+
+    want = chain(torch.cuda.synchronize, False)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        chain(lambda: None, True)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            got = chain(lambda: None, True)
+        for _ in range(3):
+            graph.replay()
+    else:
+        got = chain(lambda: None, True)
+    torch.cuda.synchronize()
+    for p, q in zip(got, want):
+        assert torch.equal(p, q)
+
+
 # ---------------------------------------------------------------- attention
 def _attention64(q, k, v, causal, mask=None):
     s = q.double() @ k.double().transpose(-1, -2) * q.shape[-1] ** -0.5
