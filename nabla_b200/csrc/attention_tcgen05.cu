@@ -1333,7 +1333,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  follow_grid();
+  // The dK / dV kernel ahead writes nothing that is read here, and it lets this grid begin only when the statistics and all before them
+  // are in memory: so the blocks work beside its last ones and wait for its end before their own. (Reads go to L2, past lines that this SM
+  // may hold; a mask of rows is read through them.) us: 2 x 8 heads x 1001 x 64 causal 184 -> 176 in
+  // a block's training step, 8 x 12 x 777 x 64 with a mask of keys 200 -> 198 and 4 x 16 x 2048 x 128 397 -> 394, both with their forward pass.
+  constexpr bool BESIDE = MASK != MASK_ROWS;
+  if (BESIDE) let_next_grid_start();
+  else follow_grid();
   const uint32_t t_dp = tmem_base + 256, t_dq = tmem_base + 384;   // S buffers at 0 and 128
 
   if (warp == 0) {
@@ -1418,8 +1424,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint32_t a_dp = t_dp + lane_addr + grp * 64;
     // padded to whole tiles, so always in range (the debug build checks it and reads nothing otherwise)
     const bool stat_ok = NB_IN_BOUNDS(NB_SITE_ATTN_STAT_INDEX, q_idx, args.Sq_pad);
-    const float nlse2 = stat_ok ? args.nlse2[bh * args.Sq_pad + q_idx] : -INFINITY;
-    const float ndelta = stat_ok ? args.ndelta[bh * args.Sq_pad + q_idx] : 0.f;
+    const float nlse2 = stat_ok ? __ldcg(args.nlse2 + bh * args.Sq_pad + q_idx) : -INFINITY;
+    const float ndelta = stat_ok ? __ldcg(args.ndelta + bh * args.Sq_pad + q_idx) : 0.f;
     // user mask: one row for all queries goes through shared memory (64 values per group and key tile) and is
     // added on the way into the exponent, with the forward's roundings (see the dK / dV kernel); a row per query is
     // read by its own thread in the mask pass
@@ -1431,7 +1437,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     float* smask = reinterpret_cast<float*>(smem + L::OFF_MASK) + grp * 128;
     const float mask_mul = LOG2E / args.scale_log2;
     const float2 mul2 = make_float2(mask_mul, mask_mul);
-    float mnext = mkey && r < 64 && grp * 64 + r < args.Skv ? mkeys[grp * 64 + r] : 0.f;
+    float mnext = mkey && r < 64 && grp * 64 + r < args.Skv ? __ldcg(mkeys + grp * 64 + r) : 0.f;
     const int lim = args.causal ? min(args.Skv - 1, q_idx + off) : args.Skv - 1;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
@@ -1440,7 +1446,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (mkey) {
         if (r < 64) smask[(j & 1) * 64 + r] = mnext;
         masked = named_bar_or(2 + grp, 128, mnext != 0.f);
-        mnext = j + 1 < n && r < 64 && kv0 + BT + r < args.Skv ? mkeys[kv0 + BT + r] : 0.f;
+        mnext = j + 1 < n && r < 64 && kv0 + BT + r < args.Skv ? __ldcg(mkeys + kv0 + BT + r) : 0.f;
       }
       if (ok && !mbar_wait(&s_full[j & 1], (j >> 1) & 1)) {
         atomicExch(args.status, NB_ERR_TIMEOUT_EPILOGUE);
@@ -1580,6 +1586,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  if (BESIDE) wait_for_previous_grid();
 }
 
 // ndelta[b][h][q] = -sum_d dO * O and nlse2 = -lse * log2(e), both padded to Sq_pad rows per
