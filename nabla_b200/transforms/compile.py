@@ -939,9 +939,10 @@ class CompiledFunction:
 
 def _copies_outweigh_launches(rec: "_Recorded") -> bool:
     """Is a schedule that is to be replayed from a CUDA graph better written down (``transforms/tape.py``)? A graph owns its arguments and
-    results, so all of them are copied in and out on each call; written-down launches take them where they are, but follow each other some
-    1.6 us later than a graph's. So by the time of the copies at HBM's rate and 2 us a launch: a QLoRA layer of 2048 tokens (80 MB, 7
-    launches) 158 us captured and 142 written down, the logits of a small decoder (66 MB, 31 launches) 260 and 289."""
+    results, so all of them are copied in and out on each call; written-down launches take them where they are, but leave no steps beside
+    each other. So by the time of the copies at HBM's rate and 0.5 us a launch: a QLoRA layer of 2048 tokens (80 MB, 7 launches) 158 us
+    captured and 130 written down, the logits of a small decoder (66 MB, 31 launches) 241 and 231, the training step of one of its layers
+    (19 MB, 22 launches) 184 and 191."""
     nbytes = 0
     for im in [*rec.placeholders, *(o for o in rec.out_impls if o is not None)]:
         n = im.dtype.to_torch().itemsize
@@ -949,7 +950,7 @@ def _copies_outweigh_launches(rec: "_Recorded") -> bool:
             n *= int(d)
         nbytes += n
     launches = sum(1 for kind, idxs in rec.steps if kind != "op" or ".ops.view." not in type(rec.nodes[idxs[0]].op).__module__)
-    return 2 * nbytes / 6.4e6 >= 2.0 * launches
+    return 2 * nbytes / 6.4e6 >= 0.5 * launches
 
 
 def _counted_modules() -> tuple:
