@@ -1602,7 +1602,7 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
                                                            float* __restrict__ nlse2, int H, int Sq, int Sq_pad,
                                                            long long do_sb, long long do_sh, long long do_ss,
                                                            long long o_sb, long long o_sh, long long o_ss) {
-  follow_grid();
+  follow_grid(dO, O, lse);
   constexpr int LPR = D / 8, RPB = 256 / LPR * PREP_U;    // lanes per row: 16 or 8; rows per block: 64 or 128
   static_assert(BT % RPB == 0, "a block stays inside a (batch, head)");
   const int per_bh = Sq_pad / RPB, bh = blockIdx.x / per_bh, q0 = (blockIdx.x - bh * per_bh) * RPB + threadIdx.x / LPR;

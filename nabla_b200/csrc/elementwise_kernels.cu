@@ -88,7 +88,7 @@ constexpr int EW_U = 4;
 template <typename T, int BMODE>
 __global__ void __launch_bounds__(256) binary_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                                                     size_t n, int op, unsigned inner, int swap) {
-  nb::follow_grid();
+  nb::follow_grid(a, b);
   constexpr int V = Vec<T>::N;
   const size_t base = (size_t)blockIdx.x * (256 * V * EW_U) + (size_t)threadIdx.x * V;
   const float bs = BMODE == 1 ? to_f<T>(b[0]) : 0.f;
@@ -165,7 +165,7 @@ __device__ __forceinline__ float un_apply(float x, int op) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) unary_kernel(const T* __restrict__ a, T* __restrict__ out, size_t n, int op) {
-  nb::follow_grid();
+  nb::follow_grid(a);
   constexpr int V = Vec<T>::N;
   const size_t base = (size_t)blockIdx.x * (256 * V * EW_U) + (size_t)threadIdx.x * V;
   uint4 ra[EW_U];
@@ -239,7 +239,7 @@ __device__ __forceinline__ Acc warp_red(Acc a, int op) {
 template <typename T, typename O>
 __global__ void __launch_bounds__(256) row_reduce_kernel(const T* __restrict__ x, O* __restrict__ out, long long rows,
                                                         long long R, int op) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   constexpr int V = Vec<T>::N;
   const int lane = threadIdx.x & 31;
   for (long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (long long)gridDim.x * 8) {
@@ -291,7 +291,7 @@ template <typename T, typename O>
 __global__ void __launch_bounds__(256) col_reduce_kernel(const T* __restrict__ x, O* __restrict__ out, float* __restrict__ pv,
                                                         long long* __restrict__ pi, long long outer, long long R,
                                                         long long inner, int op, int splits) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   __shared__ float sv[8][32];
   __shared__ long long si[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -341,7 +341,7 @@ constexpr int THIN_THREADS = 128, THIN_CHAINS = 8;
 template <typename T, int OP, int CH>
 __global__ void __launch_bounds__(THIN_THREADS) thin_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
                                                          int R, long long inner) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   constexpr int V = Vec<T>::N, U = 4, STEP = CH > U ? CH : U;
   const long long nv = inner / V, t = (long long)blockIdx.x * THIN_THREADS + threadIdx.x;
   if (t >= outer * nv) return;
@@ -392,7 +392,7 @@ template <typename T, typename O>
 __global__ void __launch_bounds__(256) col_reduce_finish_kernel(const float* __restrict__ pv, const long long* __restrict__ pi,
                                                                O* __restrict__ out, long long outer, long long R,
                                                                long long inner, int op, int splits) {
-  nb::follow_grid();
+  nb::follow_grid(pv, pi);
   const long long total = outer * inner;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const long long o = t / inner, i = t - o * inner;
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(256) col_reduce_finish_kernel(const float* __r
 template <typename T>
 __global__ void __launch_bounds__(256) cumsum_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
                                                     long long R, long long inner, int exclusive, int reverse) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   const long long total = outer * inner;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const long long o = t / inner, i = t - o * inner;

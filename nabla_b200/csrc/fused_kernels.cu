@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128, VPL <= 4 || (VPL <= 8 && sizeof(T) == 4) 
                                                               const T* __restrict__ beta, T* __restrict__ y,
                                                               float* __restrict__ mean, float* __restrict__ rstd,
                                                               int rows, int D, float eps) {
-  nb::follow_grid();
+  nb::follow_grid(x, gamma, beta);
   constexpr int V = Vec<T>::N, P = V / 2;
   constexpr bool PAIRS = sizeof(T) == 2;             // (16384 x 1024 fp32 25.0 us one at a time, 27.4 two)
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(128, 4) layernorm_bwd_dx_kernel(const T* __res
                                                               const T* __restrict__ gamma, const float* __restrict__ mean,
                                                               const float* __restrict__ rstd, T* __restrict__ dx,
                                                               int rows, int D) {
-  nb::follow_grid();
+  nb::follow_grid(dy, x, gamma, mean, rstd);
   constexpr int V = Vec<T>::N;
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128, 4)
     layernorm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                                const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
                                T* __restrict__ dx, float* __restrict__ partial, int rows, int D) {
-  nb::follow_grid();
+  nb::follow_grid(dy, x, gamma, mean, rstd, add);
   constexpr int V = Vec<T>::N, P = V / 2;
   __shared__ float sh[2][32 * V];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = lane * V;
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(32 * LN_MAX_WARPS, 2)
     layernorm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                               const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ add,
                               T* __restrict__ dx, float* __restrict__ partial, int rows, int D, int NW, int RB) {
-  nb::follow_grid();
+  nb::follow_grid(dy, x, gamma, mean, rstd, add);
   constexpr int V = Vec<T>::N, P = V / 2;
   __shared__ float red[2][LN_MAX_WARPS][4];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, slot = wid / NW, c = ((wid - slot * NW) * 32 + lane) * V;
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_dgb_kernel(const T* __restr
                                                                const float* __restrict__ rstd,
                                                                float* __restrict__ partial, int rows, int D,
                                                                int rows_per_block) {
-  nb::follow_grid();
+  nb::follow_grid(dy, x, mean, rstd);
   constexpr int V = Vec<T>::N;
   __shared__ float sh[2][8][32 * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_dgb_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __restrict__ partial, T* __restrict__ out0,
                                                               T* __restrict__ out1, int nblocks, int D) {
-  nb::follow_grid();
+  nb::follow_grid(partial);
   __shared__ float sh[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -595,7 +595,7 @@ __device__ __forceinline__ float sum8(const float (&a)[8]) { return ((a[0] + a[1
 template <typename T, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) fold_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
                                                                 int slices) {
-  nb::follow_grid();
+  nb::follow_grid(part);
   __shared__ float sh[WARPS][33];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   const size_t i0 = (size_t)blockIdx.x * 32, i = i0 + lane;
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(256) sgemm_kernel(const SgemmArgs g) {
 // out[m][n] = sum of the slices + bias[n]; eight lanes per result.
 __global__ void __launch_bounds__(256) sgemm_fold_kernel(const float* __restrict__ part, const float* __restrict__ bias,
                                                         float* __restrict__ out, int MN, int N, int slices) {
-  nb::follow_grid();
+  nb::follow_grid(part, bias);
   const int i = (blockIdx.x * 256 + threadIdx.x) % 32 + blockIdx.x * 32, q = threadIdx.x >> 5;
   __shared__ float sh[8][33];
   float s = 0.f;
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(256) sgemm_fold_kernel(const float* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
                                                     int N, int rows_per_block) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   constexpr int V = Vec<T>::N;
   __shared__ float sh[8][32 * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict__ x, float* __restrict__ partial, int rows,
                                                            int N, int rows_per_block) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   constexpr int V = Vec<T>::N;
   __shared__ float sh[256 * V];
   const int nv = N / V, rpp = 256 / nv, r_in = threadIdx.x / nv, c = threadIdx.x % nv;
@@ -871,7 +871,7 @@ __global__ void __launch_bounds__(256) __cluster_dims__(1, COLSUM_CLUSTER, 1) co
 // ============================================================== softmax / log-softmax (last dim)
 template <typename T, bool LOG>
 __global__ void __launch_bounds__(256) softmax_kernel(const T* __restrict__ x, T* __restrict__ y, int rows, int D) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   __shared__ float sh[8];
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
@@ -916,7 +916,7 @@ template <typename T, bool WHOLE, bool WIDE>
 __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__ logits,
                                                           const long long* __restrict__ tgt, float* __restrict__ lse_out,
                                                           float* __restrict__ picked, int rows, int D) {
-  nb::follow_grid();
+  nb::follow_grid(logits, tgt);
   __shared__ float sh[8];
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
@@ -975,7 +975,7 @@ __global__ void __launch_bounds__(256) lse_pick_bwd_kernel(const T* __restrict__
                                                           const float* __restrict__ lse, const float* __restrict__ g_lse,
                                                           const float* __restrict__ g_pick, T* __restrict__ dlogits,
                                                           int rows, int D) {
-  nb::follow_grid();
+  nb::follow_grid(logits, tgt, lse, g_lse, g_pick);
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
   const T* xr = logits + (size_t)row * D;
@@ -1085,7 +1085,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const TP* __restrict__ p, co
                                                    TP* __restrict__ p_out, float* __restrict__ m_out,
                                                    float* __restrict__ v_out, size_t n, AdamHyper h,
                                                    const float* __restrict__ hyper) {
-  nb::follow_grid();
+  nb::follow_grid(p, g, m, v, hyper);
   adamw_device_hyper(h, hyper);
   const float ibc1 = 1.f / h.bc1, ibc2 = 1.f / h.bc2;
   const size_t i0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -1108,7 +1108,7 @@ struct AdamGroup {
 template <typename TP, typename TG>
 __global__ void __launch_bounds__(256) adamw_group_kernel(const __grid_constant__ AdamGroup c, AdamHyper h,
                                                          const float* __restrict__ hyper) {
-  nb::follow_grid();
+  nb::follow_grid(hyper);
   adamw_device_hyper(h, hyper);
   int l = 0;
   while (l + 1 < c.count && blockIdx.x >= c.leaf[l + 1].block0) ++l;
@@ -1122,7 +1122,7 @@ __global__ void __launch_bounds__(256) adamw_group_kernel(const __grid_constant_
 // as the updates of a small model (13 us of a 180 us training step; 2.8 now). `plus`: t is the sum of two counts, kept in `total`.
 __global__ void adam_hyper_kernel(const float* __restrict__ step, const float* __restrict__ plus, float* __restrict__ total,
                                   float* __restrict__ hyper, float lr, double b1, double b2) {
-  nb::follow_grid();
+  nb::follow_grid(step, plus);
   const float sum = plus != nullptr ? step[0] + plus[0] : step[0];
   if (total != nullptr) total[0] = sum;
   const double t = (double)sum;
@@ -1140,7 +1140,7 @@ template <typename T, int C>
 __global__ void __launch_bounds__(MEAN_THREADS) __cluster_dims__(C, 1, 1)
     mean_diff_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ d, T* __restrict__ out, int n, int square,
                      const T* __restrict__ count_at, float count) {
-  nb::follow_grid();
+  nb::follow_grid(a, b, count_at);
   __shared__ float sh[MEAN_THREADS / 32], tot;
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int rank = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1173,7 +1173,7 @@ __global__ void __launch_bounds__(256) sgd_kernel(const TP* __restrict__ p, cons
                                                  const float* __restrict__ buf, TP* __restrict__ p_out,
                                                  float* __restrict__ buf_out, size_t n, float lr, float momentum,
                                                  float wd, float grad_scale) {
-  nb::follow_grid();
+  nb::follow_grid(p, g, buf);
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t k = i0; k < n; k += stride) {
@@ -1195,7 +1195,7 @@ template <typename T, bool ADD>
 __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restrict__ table,
                                                               const long long* __restrict__ ids, const T* __restrict__ add,
                                                               T* __restrict__ out, int n_ids, int D, int vocab, int period) {
-  nb::follow_grid();
+  nb::follow_grid(table, ids, add);
   constexpr int V = Vec<T>::N;
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
@@ -1283,7 +1283,7 @@ __device__ __forceinline__ unsigned long long scatter_scan(unsigned long long x,
 }
 
 __global__ void __launch_bounds__(256) scatter_count_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
-  nb::follow_grid();
+  nb::follow_grid(ids);
   const int i = blockIdx.x * 256 + threadIdx.x;
   const long long id = i < n_ids ? ids[i] : -1;
   const bool ok = id >= 0 && id < vocab;
@@ -1334,7 +1334,7 @@ __global__ void __launch_bounds__(256) scatter_slots_kernel(ScatWs ws, int n_ids
   }
 }
 __global__ void __launch_bounds__(256) scatter_place_kernel(const long long* __restrict__ ids, ScatWs ws, int n_ids, int vocab) {
-  nb::follow_grid();
+  nb::follow_grid(ids);
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n_ids) return;
   const long long id = ids[i];
@@ -1503,7 +1503,7 @@ template <typename T, int VN, bool ALL>
 __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
                                                           T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
                                                           int D, int vocab) {
-  nb::follow_grid();
+  nb::follow_grid(upd, base, part);
   __shared__ int last;
   const int total = *ws.nseg, lights = ALL ? *ws.nlight : 0;
   const int lane = threadIdx.x & 31, nwarps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1578,7 +1578,7 @@ __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(cons
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) embedding_scatter_add_kernel(float* __restrict__ acc, const long long* __restrict__ ids,
                                                                    const T* __restrict__ upd, int n_ids, int D, int vocab) {
-  nb::follow_grid();
+  nb::follow_grid(acc, ids, upd);
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
   const long long id = ids[i];
@@ -1609,7 +1609,7 @@ __global__ void __launch_bounds__(128) embedding_scatter_sorted_kernel(const lon
                                                                       const long long* __restrict__ perm,
                                                                       const T* __restrict__ upd, const T* __restrict__ base,
                                                                       T* __restrict__ out, int n_ids, int D, int vocab) {
-  nb::follow_grid();
+  nb::follow_grid(sorted_ids, perm, upd, base);
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;
   const long long id = sorted_ids[i];
@@ -1630,7 +1630,7 @@ __global__ void __launch_bounds__(128) embedding_scatter_sorted_kernel(const lon
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256) cast_kernel(const TI* __restrict__ in, TO* __restrict__ out, size_t n,
                                                   const TO* __restrict__ add_to) {
-  nb::follow_grid();
+  nb::follow_grid(in, add_to);
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t k = i0; k < n; k += stride) {
@@ -1656,7 +1656,7 @@ __device__ __forceinline__ float dgelu_tanh_f(float x) {
 template <typename T, bool BWD>
 __global__ void __launch_bounds__(256) act_kernel(const T* __restrict__ z, const T* __restrict__ dy, T* __restrict__ out,
                                                  size_t n, int mode) {
-  nb::follow_grid();
+  nb::follow_grid(z, dy);
   constexpr int V = Vec<T>::N;
   const size_t i0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
   const size_t stride = (size_t)gridDim.x * blockDim.x * V;
@@ -1729,13 +1729,13 @@ __device__ __forceinline__ void rng_resolve(const unsigned long long* state, uin
   }
 }
 __global__ void rng_bump_kernel(unsigned long long* state) {
-  nb::follow_grid(); state[1] += 1ull; }
+  nb::follow_grid(state); state[1] += 1ull; }
 
 // mode 0: uniform in [a, b); mode 1: gaussian mean a std b
 template <typename T>
 __global__ void __launch_bounds__(256) rng_kernel(T* __restrict__ out, size_t n, uint64_t seed, uint64_t offset,
                                                  int mode, float a, float b, const unsigned long long* state) {
-  nb::follow_grid();
+  nb::follow_grid(state);
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
   rng_resolve(state, seed, offset);
@@ -1761,7 +1761,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dropout_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                      uint8_t* __restrict__ mask, size_t n, float p, uint64_t seed,
                                                      uint64_t offset, const unsigned long long* state) {
-  nb::follow_grid();
+  nb::follow_grid(x, state);
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
   rng_resolve(state, seed, offset);
@@ -1792,7 +1792,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) nf4_dequant_kernel(const uint8_t* __restrict__ packed,
                                                          const float* __restrict__ absmax, T* __restrict__ out,
                                                          size_t n, int block) {
-  nb::follow_grid();
+  nb::follow_grid(packed, absmax);
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t b = i0; b * 2 < n; b += stride) {
@@ -1814,7 +1814,7 @@ __global__ void __launch_bounds__(256) nf4_dequant_codes_kernel(const uint8_t* _
                                                                const float* __restrict__ absmax,
                                                                const float* __restrict__ codebook, T* __restrict__ out,
                                                                size_t n, int block) {
-  nb::follow_grid();
+  nb::follow_grid(codes, absmax, codebook);
   __shared__ float cb[16];
   if (threadIdx.x < 16) cb[threadIdx.x] = codebook[threadIdx.x];
   __syncthreads();
@@ -1859,7 +1859,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pool2d_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int N, int H, int W,
                                                         int C, int OH, int OW, int kh, int kw, int sh, int sw, int ph,
                                                         int pw, int mode) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   const size_t total = (size_t)N * OH * OW * C;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = i % C;
@@ -1894,7 +1894,7 @@ struct CellGeom {
 };
 template <typename T, bool MAX>
 __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, const CellGeom g, unsigned total) {
-  nb::follow_grid();
+  nb::follow_grid(x);
   constexpr int V = Vec<T>::N;
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
@@ -1924,7 +1924,7 @@ __global__ void __launch_bounds__(256) pool2d_cell_fwd_kernel(const T* __restric
 template <typename T, bool MAX, bool RELU = false>
 __global__ void __launch_bounds__(256) pool2d_cell_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dx,
                                                              const CellGeom g, unsigned total) {
-  nb::follow_grid();
+  nb::follow_grid(x, dy);
   constexpr int V = Vec<T>::N;
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
@@ -1984,7 +1984,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pool2d_select_kernel(const T* __restrict__ x, const T* __restrict__ t,
                                                            T* __restrict__ y, int N, int H, int W, int C, int OH, int OW,
                                                            int kh, int kw, int sh, int sw, int ph, int pw) {
-  nb::follow_grid();
+  nb::follow_grid(x, t);
   const size_t total = (size_t)N * OH * OW * C;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = i % C;
@@ -2016,7 +2016,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pool2d_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                         T* __restrict__ dx, int N, int H, int W, int C, int OH,
                                                         int OW, int kh, int kw, int sh, int sw, int ph, int pw, int mode, int relu) {
-  nb::follow_grid();
+  nb::follow_grid(x, dy);
   const size_t total = (size_t)N * H * W * C;
   const float inv = 1.f / (kh * kw);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -2075,7 +2075,7 @@ struct ConvGeom {
 // The filter of an input gradient: out[r][s][f][c] = w[R - 1 - r][S - 1 - s][c][f].
 template <typename T>
 __global__ void __launch_bounds__(256) conv_flip_kernel(const T* __restrict__ w, T* __restrict__ out, int taps, int C, int F, unsigned n) {
-  nb::follow_grid();
+  nb::follow_grid(w);
   const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= n || !NB_IN_BOUNDS(NB_SITE_FLAT_INDEX, i, n)) return;
   const unsigned c = i % C, q = i / C, f = q % F, t = q / F;
@@ -2138,7 +2138,7 @@ __device__ __forceinline__ ConvTap conv_tap(int k, const ConvGeom& g) {
 template <typename T, int FG, bool VEC>
 __global__ void __launch_bounds__(128) conv2d_direct_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                            const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g, int relu) {
-  nb::follow_grid();
+  nb::follow_grid(x, w, bias);
   constexpr int PG = 128 / FG, MT = 2 * PG, FT = 4 * FG, PER = (MT + 127) / 128, KSTEP = MT < 128 ? 128 / MT : 1;
   __shared__ __align__(16) float xs[CONV_KC][MT + 4];
   __shared__ __align__(16) float ws[CONV_KC][FT];
@@ -2281,7 +2281,7 @@ template <typename T, int FG, int PX, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_patch_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                           const T* __restrict__ bias, T* __restrict__ y, const ConvGeom g,
                                                           int TH, int bands, int wvec, int yvec, int relu) {
-  nb::follow_grid();
+  nb::follow_grid(x, w, bias);
   constexpr int PG = 128 / FG, FT = 4 * FG, KV = VEC ? 4 : 1;
   extern __shared__ __align__(16) float conv_smem[];
   const int tid = threadIdx.x, K = g.R * g.S * g.C, CQ = g.C / KV;
@@ -2393,7 +2393,7 @@ template <typename T, int KG, int FG, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_wgrad_direct_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                                  float* __restrict__ part, const ConvGeom g,
                                                                  long long per_block) {
-  nb::follow_grid();
+  nb::follow_grid(x, dy);
   constexpr int SL = 128 / (KG * FG), KT = 4 * KG, FT = 4 * FG;
   constexpr int RED = SL > 1 ? 128 * 16 : 4, STAGE = WG_MC * (KT + FT);
   __shared__ __align__(16) float sm[RED > STAGE ? RED : STAGE];
@@ -2517,7 +2517,7 @@ template <typename T, int KG, int FG, bool VEC>
 __global__ void __launch_bounds__(128, 4) conv2d_wgrad_patch_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                                 float* __restrict__ part, const ConvGeom g, int TH,
                                                                 int bands, int total, int dvec) {
-  nb::follow_grid();
+  nb::follow_grid(x, dy);
   constexpr int SL = 128 / (KG * FG), KT = 4 * KG, FT = 4 * FG, KV = VEC ? 4 : 1;
   extern __shared__ __align__(16) float conv_smem[];
   const int tid = threadIdx.x;
@@ -2635,7 +2635,7 @@ __global__ void __launch_bounds__(128, 4) conv2d_wgrad_patch_kernel(const T* __r
 template <typename T>
 __global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict__ part, T* __restrict__ out, size_t n,
                                                         int slices) {
-  nb::follow_grid();
+  nb::follow_grid(part);
   const size_t nv = n / 4;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x) {
     float4 acc = reinterpret_cast<const float4*>(part)[i];

@@ -7,6 +7,10 @@
 // Rules that keep this the order of the stream:
 //  - nothing in global memory is read or written before follow_grid() (nor loaded into shared memory); it returns when every
 //    grid ahead has ended and its writes are visible. All blocks call it, on every path out of the kernel.
+//  - pointers that a kernel takes as parameters and reads through go in as arguments of follow_grid(). What lies behind a `const T*
+//    __restrict__` counts as constant for the whole kernel, so the compiler may read it ahead of the wait, and by the load for constants,
+//    whose lines the wait need not drop; the pointers that come back from it are no longer known to be those. (Members of a
+//    struct parameter never were.)
 //  - only then does it let the next launch begin, so no more than two grids of a stream are on the chip. A kernel that takes
 //    tensor memory has it by then: a waiting block may wait for the tensor memory of a running one, never the other way.
 //  - a kernel without follow_grid() is launched with <<< >>> and waits for the end of all that is ahead of it, as before.
@@ -19,9 +23,13 @@ namespace nb {
 
 __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_grid_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void follow_grid() {
+template <typename Pointer>
+__device__ __forceinline__ void as_of_now(Pointer& p) { asm volatile("" : "+l"(p) : : "memory"); }
+template <typename... Pointers>
+__device__ __forceinline__ void follow_grid(Pointers&... read) {
   wait_for_previous_grid();
   let_next_grid_start();
+  (as_of_now(read), ...);
 }
 
 // Adds the attribute to a launch whose attribute array has room for one more.

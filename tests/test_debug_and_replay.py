@@ -53,17 +53,19 @@ def test_every_kernel_source_includes_the_check_header_and_uses_it():
 
 
 def test_every_kernel_of_a_following_launch_waits_for_the_grid_ahead():
-    """A kernel that is launched before the grid ahead of it has ended calls follow_grid(), and before any path out of it."""
+    """A kernel that is launched before the grid ahead of it has ended calls follow_grid(), before any path out of it, and with every pointer
+    parameter that the compiler would take for constant."""
     import re
 
     csrc = ROOT / "nabla_b200" / "csrc"
     for name in ("gemm_tcgen05.cu", "attention_tcgen05.cu", "fused_kernels.cu", "elementwise_kernels.cu"):
         src = re.sub(r"//[^\n]*", "", (csrc / name).read_text())
         cta = src[src.index("bool gemm_cta("):] if "bool gemm_cta(" in src else ""
-        bodies = {}
+        bodies, params = {}, {}
         for m in re.finditer("__global__", src):
             kernel = re.compile(r"(\w+_kernel)\s*\(").search(src, m.end())
             brace = src.index("{", kernel.end())
+            params[kernel.group(1)] = src[kernel.end():brace]
             bodies[kernel.group(1)] = src[brace:src.index("\n}\n", brace)]
         launched = set(re.findall(r"launch_following\((\w+)", src)) - {"kernel"}
         launched |= {k for k in bodies if re.match(r"gemm_bf16_|layernorm_bwd_rows", k)}        # (through a pointer to the kernel)
@@ -74,8 +76,11 @@ def test_every_kernel_of_a_following_launch_waits_for_the_grid_ahead():
                 assert "gemm_cta<BN, MODE_NONE" in body
                 body = cta
             body = body.replace("return follow_grid();", "follow_grid_and_leave;")
-            ahead = re.sub(r"\[&?\]\([^)]*\)[^{;]*\{ return [^}]*\}", "", body[:body.index("follow_grid();")])      # (without lambdas)
+            ahead = re.sub(r"\[&?\]\([^)]*\)[^{;]*\{ return [^}]*\}", "", body[:body.index("follow_grid(")])      # (without lambdas)
             assert not re.search(r"\breturn\b", ahead), (name, k)
+            given = re.search(r"follow_grid\(([^)]*)\)", body).group(1).replace(" ", "").split(",")
+            constant = re.findall(r"const [\w ]+\* ?__restrict__ (\w+)", params.get(k, ""))
+            assert set(constant) <= set(given), (name, k)
 
 
 @pytest.mark.parametrize("source,kernels", [

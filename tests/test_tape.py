@@ -213,3 +213,65 @@ def test_large_arguments_of_a_captured_function_are_not_copied():
         out = small(_wrap(xs[k][:64]), _wrap(w[:, :64].contiguous())).to_torch().double()
         assert torch.allclose(out, want[k][:64, :64], atol=0.1)
     assert small.stats.cuda_graphs == 1 and _taped(small)
+
+
+@pytest.mark.parametrize("name", list(_functions()) if torch.cuda.is_available() else ["norm"])
+@pytest.mark.parametrize("graph", [False, True])
+def test_calls_in_a_row_read_their_own_inputs(name, graph):
+    """Launches that are resident before the ones ahead have ended: forty calls without a synchronisation, each on other values in the same
+    memory, give what calls alone give."""
+    import nabla_b200 as nb
+
+    fn, inputs = _functions()[name]
+    f, plain = nb.compile(fn, cuda_graph=graph), nb.compile(fn)
+    sets = [inputs(k) for k in range(4)]
+    want = []
+    for s in sets:
+        want.append([t.clone() for t in _leaves(plain(*map(_wrap, s)))])
+        torch.cuda.synchronize()
+    held = [t.clone() for t in sets[0]]
+    got = []
+    for k in range(40):
+        for h, t in zip(held, sets[k % 4]):
+            h.copy_(t)
+        got.append([t.clone() for t in _leaves(f(*map(_wrap, held)))])
+    torch.cuda.synchronize()
+    for k, outs in enumerate(got):
+        for a, b in zip(outs, want[k % 4]):
+            assert torch.equal(a, b), k
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_training_run_of_calls_in_a_row(graph):
+    """Two hundred steps of a small network with AdamW, parameters, moments and step count from each to the next, against the same steps
+    with a synchronisation after each: equal bit for bit."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    def step(params, state, x, y):
+        def loss(p):
+            return F.mse_loss(F.linear(F.linear(x, p["w0"], p["b0"], activation="relu"), p["w1"], p["b1"]), y)
+
+        value, grads = nb.value_and_grad(loss, create_graph=False)(params)
+        params, state = nb.nn.adamw_update(params, grads, state, lr=1e-2, weight_decay=0.01, realize=False)
+        return value, params, state
+
+    def run(f, pause):
+        gen = torch.Generator("cuda").manual_seed(5)
+        shapes = {"w0": (64, 256), "b0": (256,), "w1": (256, 8), "b1": (8,)}
+        p = {k: _wrap((torch.randn(s, generator=gen, device="cuda") * 0.1).to(BF16)) for k, s in shapes.items()}
+        st = {"m": {k: _wrap(torch.zeros(s, device="cuda")) for k, s in shapes.items()},
+              "v": {k: _wrap(torch.zeros(s, device="cuda")) for k, s in shapes.items()}, "step": _wrap(torch.tensor(0.0, device="cuda"))}
+        losses = []
+        for k in range(200):
+            x = torch.rand(100, 64, generator=gen, device="cuda").to(BF16)
+            value, p, st = f(p, st, _wrap(x), _wrap(torch.sin(x[:, :8].float() * 6).to(BF16)))
+            losses.append(value)
+            pause()
+        return [t.clone() for t in _leaves([losses, p, st])]
+
+    got, want = run(nb.compile(step, cuda_graph=graph), lambda: None), run(nb.compile(step), torch.cuda.synchronize)
+    torch.cuda.synchronize()
+    assert float(want[199]) < float(want[0])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
