@@ -1592,9 +1592,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // ndelta[b][h][q] = -sum_d dO * O and nlse2 = -lse * log2(e), both padded to Sq_pad rows per
 // (b, h): padding rows and rows whose lse is -inf (no visible key) get nlse2 = -inf (probability 0)
 // and ndelta = 0. D / 8 lanes per row, 16-byte loads, PREP_U rows per group of lanes on their way; a block's rows lie in
-// one (b, h) (they divide a tile of 128), so there is one division per block. 64 heads x 2048 x 128: 21.8 us with a row and two
-// 64-bit divisions per group, 17.8 so.
-constexpr int PREP_U = 4;
+// one (b, h) (they divide a tile of 128), so there is one division per block; the heads of the same rows, which lie side by side in
+// memory, are neighbouring blocks. Whole backward pass, us, with 4 rows and the rows of a head as neighbours, and so: 4 x 16 x 2048 x
+// 128 259.6, 256.7; 8 x 12 x 777 x 64 86.1, 84.4; 2 x 8 x 1001 x 64 23.0, 21.9; 4 x 16 x 4096 x 64 672, 662.
+constexpr int PREP_U = 2;
 template <int D>
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dO,
                                                            const __nv_bfloat16* __restrict__ O,
@@ -1603,10 +1604,10 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
                                                            long long do_sb, long long do_sh, long long do_ss,
                                                            long long o_sb, long long o_sh, long long o_ss) {
   follow_grid(dO, O, lse);
-  constexpr int LPR = D / 8, RPB = 256 / LPR * PREP_U;    // lanes per row: 16 or 8; rows per block: 64 or 128
+  constexpr int LPR = D / 8, RPB = 256 / LPR * PREP_U;    // lanes per row: 16 or 8; rows per block: 32 or 64
   static_assert(BT % RPB == 0, "a block stays inside a (batch, head)");
-  const int per_bh = Sq_pad / RPB, bh = blockIdx.x / per_bh, q0 = (blockIdx.x - bh * per_bh) * RPB + threadIdx.x / LPR;
-  const int b = bh / H, h = bh - b * H, sub = threadIdx.x % LPR;
+  const int per_bh = Sq_pad / RPB, rows = blockIdx.x / H, h = blockIdx.x - rows * H, b = rows / per_bh, bh = b * H + h;
+  const int q0 = (rows - b * per_bh) * RPB + threadIdx.x / LPR, sub = threadIdx.x % LPR;
   const __nv_bfloat16* pd = dO + b * do_sb + h * do_sh + sub * 8;
   const __nv_bfloat16* po = O + b * o_sb + h * o_sh + sub * 8;
   uint4 ra[PREP_U], rc[PREP_U];
