@@ -18,8 +18,8 @@
 // operand from TMEM. Shared memory then only feeds Q / K / V / dO, which halves the operand
 // traffic of the PV-type products.
 //
-// forward (attn_fwd_kernel): one CTA owns TWO query tiles (2 x 128 rows) that share the K / V
-//   stream. Group A works on the softmax of tile A while the tensor core runs tile B's products
+// forward (attn_fwd_kernel): one CTA owns TWO query tiles (2 x 128 rows; one where the grid has an
+//   SM for every tile) that share the K / V stream. Group A works on the softmax of tile A while the tensor core runs tile B's products
 //   and vice versa (S_A, S_B, O_A, O_B = 512 TMEM columns at head_dim 128).
 // backward, dK / dV (attn_bwd_dkdv_kernel): one CTA owns 128 keys and walks over the query
 //   tiles: S^T = K Q^T, dP^T = V dO^T, P^T and dS^T written back into TMEM as A operands of
@@ -1788,7 +1788,7 @@ static int attn_q_tiles(int B, int H, int Sq, int Skv, int causal, int nsplit) {
 // Decode kernel: ranges of at least 128 keys, for four blocks per SM; at head_dim 64 none below 512 keys, where a block walks
 // them before a second launch would have started (64 pairs x 300 keys: 12.3 us whole, 15.4 in two ranges; 16.4 and 15.4 at
 // head_dim 128).
-// Otherwise a CTA owns 256 queries of one (batch, head), so a short query block against a long prefix gives one
+// Otherwise a CTA owns up to 256 queries of one (batch, head), so a short query block against a long prefix gives one
 // CTA per (batch, head), each walking all key tiles alone. The rule counts what the busiest SM walks: waves *
 // (key tiles per CTA + 3), the 3 standing for a CTA's start and end, and 3 more for the launch that joins the
 // ranges (a tile is 1.7 us at head_dim 128, the join 5): 500 keys 16.4 us whole and 17.4 in four ranges, 520 keys 18.4 and
