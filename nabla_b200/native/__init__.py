@@ -179,6 +179,11 @@ except AttributeError:             # a torch build without CUDA
     _raw_stream = None
 
 
+def raw_stream(device: int) -> int:
+    """Handle of the current stream of a GPU."""
+    return _raw_stream(device) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
+
+
 def stream_ptr() -> ctypes.c_void_p:
     if _raw_stream is not None:
         return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))

@@ -42,7 +42,7 @@ from typing import Any, Callable
 
 import torch
 
-from .. import config
+from .. import config, native
 from ..core.common import pytree
 from ..core.graph import fusion
 from ..core.graph.engine import GRAPH, _STATS, store_outputs
@@ -189,7 +189,8 @@ class _Recorded:
         self.branch_steps: set[int] = set()         # captured beside the others (see _branch_leaves)
         self.side_steps: set[int] = set()           # optimizer updates that run on a side stream, under the backward
         self.constants: list[TensorImpl] = []       # values that follow from numbers alone, made with the plan
-        self.constant_stream = None                 # the stream they were made on
+        self.owned: list[torch.Tensor] | None = None     # GPU tensors that go with the recording: its constants and the numbers in it
+        self.told: set[int] = set()                 # raw streams that the allocator knows to read them
         self.tape = None                            # of later calls without Python (transforms/tape.py); False: none
         self.tape_counts: tuple = ()                # launches of a taped call: GEMM, fused kernels, attention
         self.tape_tries = 0
@@ -275,7 +276,7 @@ class CompiledFunction:
                 if not isinstance(rec, _Recorded):
                     continue
                 rec.cuda_graph = rec.tape = None
-                rec.static_inputs = rec.static_outputs = rec.out_cached = rec.copy_in = rec.copy_out = None
+                rec.static_inputs = rec.static_outputs = rec.out_cached = rec.copy_in = rec.copy_out = rec.owned = None
                 for ph in rec.placeholders:
                     ph._buffers = None
                 for outs in rec.keep:
@@ -400,6 +401,7 @@ class CompiledFunction:
         if self.profile_ops or graphs is not self.use_cuda_graph or rec.tape is not handle:
             return NotImplemented
         t0 = time.perf_counter()
+        _tell_stream(rec)
         out = tape.module().call(handle, args, config.is_deterministic())
         if out is not NotImplemented:
             for module, n in zip(_counted_modules(), rec.tape_counts):
@@ -716,6 +718,7 @@ class CompiledFunction:
         new.out_impls = [mapping.get(id(i), i) if i is not None else None for i in base.out_impls]
         new.targets = [mapping[id(t)] for t in base.targets]
         self._plan(new)
+        _tell_stream(new)                           # the numbers are those of the first recording, perhaps of another stream
         self._run(new)
         return new, self._collect(new)
 
@@ -726,9 +729,6 @@ class CompiledFunction:
         if self.profile_ops and not torch.cuda.is_current_stream_capturing():
             return self._run_profiled(rec)
         nvtx = _NVTX and torch.cuda.is_available()
-        if rec.constants and torch.cuda.current_stream() != rec.constant_stream and not torch.cuda.is_current_stream_capturing():
-            for o in rec.constants:                 # they may go with the recording while this stream still reads them
-                o._buffers[0].record_stream(torch.cuda.current_stream())
         side = cur = None
         # Measured on the 24-layer benchmark step (1 GPU, power-capped at 1 kW): 155.8 ms with the updates
         # on the side stream, 155.2 ms without: the step is energy bound, so hiding the AdamW kernels
@@ -841,6 +841,7 @@ class CompiledFunction:
 
     def _replay(self, rec: _Recorded, tensors: list[Tensor], tds: tuple | None = None) -> Any:
         """``tds``: the arguments' structures, where nothing but tensors is among them."""
+        _tell_stream(rec)
         if self.use_cuda_graph and not rec.host_sync and tensors and tensors[0]._impl.device.label == "gpu" \
                 and not (rec.cuda_graph is None and rec.tape is None and tds is not None and _copies_outweigh_launches(rec) and tape.can_record(rec)):
             out = self._replay_cuda_graph(rec, tensors)
@@ -951,6 +952,22 @@ def _copies_outweigh_launches(rec: "_Recorded") -> bool:
         nbytes += n
     launches = sum(1 for kind, idxs in rec.steps if kind != "op" or ".ops.view." not in type(rec.nodes[idxs[0]].op).__module__)
     return 2 * nbytes / 6.4e6 >= 0.5 * launches
+
+
+def _tell_stream(rec: "_Recorded") -> None:
+    """Before the current stream reads what the recording owns: the recording may go, and the allocator hand its memory out again, while
+    that stream is still at it, so each stream is made known to the allocator once. (A capture runs nothing.)"""
+    if rec.owned is None:
+        placeholders = {id(p) for p in rec.placeholders}
+        numbers = [a for n in rec.nodes for a in n.input_impls() if a.literal is not None and id(a) not in placeholders and a._buffers]
+        rec.owned = list({id(b): b for a in [*rec.constants, *numbers] for b in a._buffers if b.is_cuda}.values())
+    if rec.owned:
+        index = rec.owned[0].device.index
+        stream = native.raw_stream(index)
+        if stream not in rec.told and not torch.cuda.is_current_stream_capturing():
+            for b in rec.owned:
+                b.record_stream(torch.cuda.current_stream(b.device))
+            rec.told.add(stream)
 
 
 def _counted_modules() -> tuple:
@@ -1371,7 +1388,6 @@ def _make_constants(rec: "_Recorded", max_elems: int = 1 << 16) -> list:
     for o in kept:
         if id(o) in wanted:
             rec.constants.append(o)
-    rec.constant_stream = torch.cuda.current_stream()
     return [st for st in rec.steps if not (st[0] == "op" and st[1][0] in gone)]
 
 

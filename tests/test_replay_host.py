@@ -1,0 +1,69 @@
+"""Host side of compiled calls (``transforms/compile.py``, ``transforms/tape.py``) with stand-ins for the GPU's part."""
+import importlib
+
+import pytest
+import torch
+
+import nabla_b200 as nb
+from nabla_b200 import native
+from nabla_b200.transforms import tape
+
+C = importlib.import_module("nabla_b200.transforms.compile")
+
+
+class _Owned:
+    """A GPU tensor that a recording owns, as far as the host sees it."""
+    is_cuda, device = True, torch.device("cuda", 0)
+
+    def __init__(self, log):
+        self.log = log
+
+    def record_stream(self, stream):
+        self.log.append(("told", stream))
+
+
+class _Impl:
+    literal = None
+
+    def __init__(self, log):
+        self._buffers = [_Owned(log)]
+
+
+@pytest.fixture
+def gpu(monkeypatch):
+    """(log, set the current stream, say whether it is capturing) of a GPU that is not there."""
+    state, log = {"stream": 1, "capturing": False}, []
+    monkeypatch.setattr(native, "raw_stream", lambda device: state["stream"], raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: state["stream"])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state["capturing"])
+    return state, log
+
+
+class _Module:
+    def __init__(self, log, out):
+        self.log, self.out = log, out
+
+    def call(self, handle, args, deterministic):
+        self.log.append(("call", handle))
+        return self.out
+
+
+def _taped_function(monkeypatch, log):
+    f = nb.compile(lambda x: x)
+    rec = C._Recorded()
+    rec.constants = [_Impl(log)]
+    rec.tape, rec.tape_counts = "handle", ()
+    f._taped = (rec.tape, rec, f.use_cuda_graph)
+    monkeypatch.setattr(tape, "module", lambda: _Module(log, "out"))
+    return f, rec
+
+
+def test_each_stream_is_told_of_the_constants_before_a_taped_call(gpu, monkeypatch):
+    """What was made with the plan may be freed while another stream still reads it: once per stream, ahead of the launches."""
+    state, log = gpu
+    f, _ = _taped_function(monkeypatch, log)
+    x = nb.Tensor.from_torch(torch.zeros(2))
+    for stream in (1, 1, 2, 1):
+        state["stream"] = stream
+        assert f(x) == "out"
+    assert log == [("told", 1), ("call", "handle"), ("call", "handle"), ("told", 2), ("call", "handle"), ("call", "handle")]

@@ -275,3 +275,38 @@ def test_a_training_run_of_calls_in_a_row(graph):
     assert float(want[199]) < float(want[0])
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_constants_outlive_the_calls_of_other_streams(graph):
+    """Traced on one stream, called on another that is behind, and released: the memory of what was made with the plan is not handed
+    out again before that stream has read it."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    def fn(x, y):
+        return nb.value_and_grad(lambda x: F.mse_loss(x, y), create_graph=False)(x)
+
+    x, y = torch.randn(512, 8, device="cuda"), torch.randn(512, 8, device="cuda")
+    want = 2 * (x.double() - y.double()) / x.numel()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    f = nb.compile(fn, cuda_graph=graph)
+    with torch.cuda.stream(first):
+        f(_wrap(x), _wrap(y))
+        rec = next(iter(next(iter(f._cache.values())).values()))
+        shapes = {tuple(b.shape) for o in rec.constants for b in o._buffers}
+        assert shapes
+        del rec
+        f(_wrap(x), _wrap(y))
+        assert _taped(f), f.tape_refused
+    torch.cuda.synchronize()
+    with torch.cuda.stream(second):
+        torch.cuda._sleep(100_000_000)                # some 50 ms
+        _, g = f(_wrap(x), _wrap(y))
+    f.release()
+    del f
+    with torch.cuda.stream(first):
+        held = [torch.full(s, 1e6, device="cuda") for s in shapes for _ in range(400)]
+    torch.cuda.synchronize()
+    assert torch.allclose(g.to_torch().double(), want, rtol=1e-4, atol=1e-9) and held
