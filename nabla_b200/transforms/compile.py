@@ -189,6 +189,7 @@ class _Recorded:
         self.branch_steps: set[int] = set()         # captured beside the others (see _branch_leaves)
         self.side_steps: set[int] = set()           # optimizer updates that run on a side stream, under the backward
         self.constants: list[TensorImpl] = []       # values that follow from numbers alone, made with the plan
+        self.constant_nodes: list[int] = []         # their nodes, in order
         self.owned: list[torch.Tensor] | None = None     # GPU tensors that go with the recording: its constants and the numbers in it
         self.told: set[int] = set()                 # raw streams that the allocator knows to read them
         self.tape = None                            # of later calls without Python (transforms/tape.py); False: none
@@ -398,7 +399,8 @@ class CompiledFunction:
     def _call_taped(self, taped: tuple, args: tuple):
         """The call without Python in between, or NotImplemented."""
         handle, rec, graphs = taped
-        if self.profile_ops or graphs is not self.use_cuda_graph or rec.tape is not handle:
+        if self.profile_ops or graphs is not self.use_cuda_graph or rec.tape is not handle \
+                or (rec.constants and torch.cuda.is_current_stream_capturing()):     # see _run
             return NotImplemented
         t0 = time.perf_counter()
         _tell_stream(rec)
@@ -723,7 +725,16 @@ class CompiledFunction:
         return new, self._collect(new)
 
     # ---- execution of a recorded graph
-    def _run(self, rec: _Recorded) -> None:
+    def _run(self, rec: _Recorded, own_capture: bool = False) -> None:
+        if rec.constants and not own_capture and torch.cuda.is_current_stream_capturing():
+            # the caller's graph may outlive the recording: it gets constants in its own memory
+            made = [(o, o._buffers) for o in rec.constants]
+            try:
+                _compute_constants(rec)
+                return self._run(rec, own_capture=True)
+            finally:
+                for o, buffers in made:
+                    o._buffers = buffers
         nodes = rec.nodes
         _STATS["nodes_executed"] += len(nodes)
         if self.profile_ops and not torch.cuda.is_current_stream_capturing():
@@ -884,7 +895,7 @@ class CompiledFunction:
 
                 n0 = total_launches()
                 with torch.cuda.graph(g, capture_error_mode="thread_local"):
-                    self._run(rec)
+                    self._run(rec, own_capture=True)
                     rec.static_outputs = [list(i._buffers) if i is not None else None for i in rec.out_impls]
             except Exception as e:
                 import warnings
@@ -1379,16 +1390,24 @@ def _make_constants(rec: "_Recorded", max_elems: int = 1 << 16) -> list:
         return rec.steps
     gone = set(made.values())
     wanted = {k for k in made if any(r not in gone for r in readers.get(k, []))}
-    kept = []
-    for ni in sorted(gone):
-        o = nodes[ni].outputs()[0]
-        o._buffers = [b.contiguous() for b in nodes[ni].op.execute(nodes[ni])[0]]
-        kept.append(o)
+    rec.constant_nodes = sorted(gone)
+    rec.constants = [o for o in (nodes[ni].outputs()[0] for ni in rec.constant_nodes) if id(o) in wanted]
+    _compute_constants(rec)
     torch.cuda.current_stream().synchronize()       # a later call may be on another stream
-    for o in kept:
-        if id(o) in wanted:
-            rec.constants.append(o)
     return [st for st in rec.steps if not (st[0] == "op" and st[1][0] in gone)]
+
+
+def _compute_constants(rec: "_Recorded") -> None:
+    """Run the steps that compute ``rec.constants`` and drop what only they read."""
+    outs = []
+    for ni in rec.constant_nodes:
+        n = rec.nodes[ni]
+        outs.append(n.outputs()[0])
+        outs[-1]._buffers = [b.contiguous() for b in n.op.execute(n)[0]]
+    kept = {id(o) for o in rec.constants}
+    for o in outs:
+        if id(o) not in kept:
+            o._buffers = None
 
 
 def _group_bias_grads(steps: list, nodes: list[OpNode], window: int = 24, max_bytes: int = 1 << 25) -> list:

@@ -67,3 +67,36 @@ def test_each_stream_is_told_of_the_constants_before_a_taped_call(gpu, monkeypat
         state["stream"] = stream
         assert f(x) == "out"
     assert log == [("told", 1), ("call", "handle"), ("call", "handle"), ("told", 2), ("call", "handle"), ("call", "handle")]
+
+
+def test_a_graph_of_the_callers_gets_constants_of_its_own(gpu, monkeypatch):
+    """It may outlive the function, so nothing that goes with the recording is in it."""
+    state, log = gpu
+    f, rec = _taped_function(monkeypatch, log)
+    state["capturing"] = True
+    assert f._call_taped(f._taped, (nb.Tensor.from_torch(torch.zeros(2)),)) is NotImplemented and log == []
+
+    class Op:
+        def __init__(self, execute):
+            self.execute = execute
+
+    class Node:
+        def __init__(self, out, execute):
+            self.out, self.op, self.out_refs = out, Op(execute), []
+
+        def outputs(self):
+            return [self.out]
+
+    class Impl:
+        literal = _buffers = None
+
+    constant, helper, seen = Impl(), Impl(), []
+    rec.nodes = [Node(helper, lambda n: [[torch.ones(3)]]), Node(constant, lambda n: [[helper._buffers[0] + 1]]),
+                 Node(None, lambda n: seen.append(constant._buffers[0]) or [])]
+    rec.constants, rec.constant_nodes, rec.steps, rec.free_after = [constant], [0, 1], [("op", (2,))], [[]]
+    constant._buffers = [made := torch.full((3,), 2.0)]
+    f._run(rec)
+    state["capturing"] = False
+    f._run(rec)
+    assert seen[0] is not made and torch.equal(seen[0], made) and seen[1] is made and constant._buffers[0] is made
+    assert helper._buffers is None

@@ -310,3 +310,30 @@ def test_constants_outlive_the_calls_of_other_streams(graph):
         held = [torch.full(s, 1e6, device="cuda") for s in shapes for _ in range(400)]
     torch.cuda.synchronize()
     assert torch.allclose(g.to_torch().double(), want, rtol=1e-4, atol=1e-9) and held
+
+
+def test_a_graph_of_the_callers_outlives_the_function():
+    """A compiled function in a capture of the caller's own: dropped, its constants are still the graph's."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    x, y = torch.randn(512, 8, device="cuda"), torch.randn(512, 8, device="cuda")
+    f = nb.compile(lambda x, y: nb.value_and_grad(lambda x: F.mse_loss(x, y), create_graph=False)(x))
+    for _ in range(3):                                # traced, written down, taped
+        f(_wrap(x), _wrap(y))
+    assert _taped(f), f.tape_refused
+    rec = next(iter(next(iter(f._cache.values())).values()))
+    shapes = {tuple(b.shape) for o in rec.constants for b in o._buffers}
+    assert shapes
+    del rec
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        _, grad = f(_wrap(x), _wrap(y))
+    f.release()
+    del f
+    held = [torch.full(s, 1e6, device="cuda") for s in shapes for _ in range(400)]
+    x.mul_(3.0)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.allclose(grad.to_torch().double(), 2 * (x.double() - y.double()) / x.numel(), rtol=1e-4, atol=1e-9) and held
