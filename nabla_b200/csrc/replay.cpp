@@ -57,6 +57,13 @@ struct Ref {                                         // owned reference
   ~Ref() { Py_XDECREF(p); }
 };
 
+// Launches wait for the device when the stream's queue is full, and allocations may; other threads of Python run meanwhile (and so does
+// a host function on the stream that needs Python), as they do while ctypes or torch calls a library.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 struct Tree {                                        // structure of an argument or of the result
   char kind = 'n';                                   // n None, x a leaf, l list, t tuple, d dict
   Ref keys;                                          // tuple
@@ -105,6 +112,7 @@ struct Tape {
   std::vector<Leaf> leaves;
   std::vector<std::pair<std::string, Ref>> env;      // (name, bytes or None)
   std::vector<Pin> pins;
+  std::vector<at::Tensor> kept;                      // what the launches' fixed addresses lie in: alive as long as a call is at it
   int device = 0;
   bool deterministic = false;
   std::vector<Launch> launches;
@@ -172,7 +180,7 @@ Tree read_tree(PyObject* o) {                        // (kind, keys or None, chi
 
 void release(PyObject* cap) { delete static_cast<Tape*>(PyCapsule_GetPointer(cap, "nb_tape")); }
 
-// make(args, leaves, env, device, deterministic, launches, scratch, outs, out_tree, graph, captured impls): see transforms/tape.py
+// make(args, leaves, env, device, deterministic, launches, scratch, outs, out_tree, graph, captured impls, kept tensors): see transforms/tape.py
 PyObject* make(PyObject*, PyObject* a) {
   auto t = std::make_unique<Tape>();
   try {
@@ -293,6 +301,8 @@ PyObject* make(PyObject*, PyObject* a) {
       p.strides = x.strides().vec();
       t->pins.push_back(std::move(p));
     }
+    o = item(a, 11);
+    for (Py_ssize_t i = 0; i < size(o); ++i) t->kept.push_back(tensor(item(o, i)));
   } catch (const Fail&) {
     return nullptr;
   } catch (const std::exception& e) {
@@ -387,92 +397,12 @@ PyObject* build(const Tree& t, std::vector<Ref>& leaves, size_t& at) {
   }
 }
 
-// call(tape, args, deterministic) -> result, or NotImplemented when the call is not the one that was written down
-PyObject* call(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
-  HANDLE_TH_ERRORS
-  if (argc != 3 || !PyTuple_CheckExact(argv[1])) { PyErr_SetString(PyExc_TypeError, "call(tape, args, deterministic)"); return nullptr; }
-  Tape* t = static_cast<Tape*>(PyCapsule_GetPointer(argv[0], "nb_tape"));
-  if (t == nullptr) return nullptr;
-  if (PyTuple_GET_SIZE(argv[1]) != static_cast<Py_ssize_t>(t->args.size()) || (argv[2] == Py_True) != t->deterministic) Py_RETURN_NOTIMPLEMENTED;
-  std::vector<PyObject*> leaves;
-  leaves.reserve(t->leaves.size());
-  for (size_t i = 0; i < t->args.size(); ++i)
-    if (!gather(t->args[i], PyTuple_GET_ITEM(argv[1], i), leaves)) Py_RETURN_NOTIMPLEMENTED;
-  if (leaves.size() != t->leaves.size()) Py_RETURN_NOTIMPLEMENTED;
-  if (c10::cuda::current_device() != t->device) Py_RETURN_NOTIMPLEMENTED;
-  for (const auto& e : t->env) {
-    const char* v = std::getenv(e.first.c_str());
-    if (v == nullptr ? e.second.p != Py_None : (e.second.p == Py_None || std::strcmp(v, PyBytes_AS_STRING(e.second.p)) != 0)) Py_RETURN_NOTIMPLEMENTED;
-  }
-  for (const Pin& p : t->pins) {
-    PyObject* b = slot(p.impl.p, o_buffers);
-    if (b == nullptr || !PyList_CheckExact(b) || PyList_GET_SIZE(b) != 1 || !THPVariable_Check(PyList_GET_ITEM(b, 0))) Py_RETURN_NOTIMPLEMENTED;
-    const at::Tensor& x = THPVariable_Unpack(PyList_GET_ITEM(b, 0));
-    if (x.data_ptr() != p.ptr || x.sizes() != at::IntArrayRef(p.sizes) || x.strides() != at::IntArrayRef(p.strides)) Py_RETURN_NOTIMPLEMENTED;
-  }
-  std::vector<char*> bases(leaves.size() + t->outs.size() + 1, nullptr);
-  std::vector<at::Tensor> held;                      // arguments stay alive whatever an allocation may run
-  held.reserve(leaves.size());
-  for (size_t i = 0; i < leaves.size(); ++i) {
-    const at::Tensor* x = buffer(t->leaves[i], leaves[i], t->device);
-    if (x == nullptr) Py_RETURN_NOTIMPLEMENTED;
-    held.push_back(*x);
-    bases[i] = static_cast<char*>(x->data_ptr());
-  }
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(t->device)).stream();
+// The launches in their order. Returns the first that failed (`code`: with what), else null.
+const Launch* run_launches(const Tape& t, const std::vector<char*>& bases, cudaStream_t stream, int& code) {
   long ints[REG_INTS + STACK_INTS];
   double floats[FLOATS];
-  auto launch_copies = [&](void* const* dst, void* const* src, const unsigned long long* bytes, size_t n) -> bool {
-    std::memset(ints, 0, sizeof(ints));
-    std::memset(floats, 0, sizeof(floats));
-    ints[0] = reinterpret_cast<long>(dst);
-    ints[1] = reinterpret_cast<long>(src);
-    ints[2] = reinterpret_cast<long>(bytes);
-    ints[3] = static_cast<long>(n);
-    ints[4] = reinterpret_cast<long>(stream);
-    const int k = call_launcher(t->copy_batch, ints, floats);
-    if (k < 0) PyErr_Format(PyExc_RuntimeError, "copy_batch failed with code %d", k);
-    return k >= 0;
-  };
-  if (t->replay.p != nullptr) {
-    const size_t n = leaves.size();
-    std::vector<void*> src(n, nullptr);
-    std::vector<unsigned long long> bytes(n, 0);
-    bool any = false;
-    for (size_t i = 0; i < n; ++i)
-      if (bases[i] != t->in_ptrs[i]) {
-        src[i] = bases[i];
-        bytes[i] = t->in_bytes[i];
-        any = any || bytes[i] > 0;
-      }
-    if (any && !launch_copies(t->in_ptrs.data(), src.data(), bytes.data(), n)) return nullptr;
-    Ref r(PyObject_CallNoArgs(t->replay.p));
-    if (r.p == nullptr) return nullptr;
-  }
-  std::vector<at::Tensor> results;
-  results.reserve(t->outs.size());
-  at::Tensor scratch;
-  {
-    at::AutoDispatchBelowAutograd guard;
-    for (size_t i = 0; i < t->outs.size(); ++i) {
-      const Out& o = t->outs[i];
-      if (o.is_static) { results.emplace_back(); continue; }
-      results.push_back(at::empty_strided(o.sizes, o.strides, o.options));
-      bases[leaves.size() + i] = static_cast<char*>(results.back().data_ptr());
-    }
-    if (t->scratch) {
-      scratch = at::empty({static_cast<int64_t>(t->scratch)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, t->device));
-      bases.back() = static_cast<char*>(scratch.data_ptr());
-    }
-  }
-  if (t->replay.p != nullptr && !t->out_ptrs.empty()) {
-    std::vector<void*> dst;
-    for (size_t i = 0; i < t->outs.size(); ++i)
-      if (!t->outs[i].is_static) dst.push_back(bases[leaves.size() + i]);
-    if (!launch_copies(dst.data(), t->out_ptrs.data(), t->out_bytes.data(), dst.size())) return nullptr;
-  }
   std::vector<std::string> blobs;
-  for (const Launch& l : t->launches) {
+  for (const Launch& l : t.launches) {
     std::memset(ints, 0, sizeof(ints));
     std::memset(floats, 0, sizeof(floats));
     blobs.clear();
@@ -504,11 +434,103 @@ PyObject* call(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
         }
       }
     }
-    const int rc = call_launcher(l.fn, ints, floats);
-    if (rc != l.rc) {
-      PyErr_Format(PyExc_RuntimeError, "%s failed with code %d", l.name.c_str(), rc);
-      return nullptr;
+    code = call_launcher(l.fn, ints, floats);
+    if (code != l.rc) return &l;
+  }
+  return nullptr;
+}
+
+// One launch that copies for a graph; a negative code when it failed.
+int run_copies(void* copy_batch, void* const* dst, void* const* src, const unsigned long long* bytes, size_t n, cudaStream_t stream) {
+  long ints[REG_INTS + STACK_INTS] = {reinterpret_cast<long>(dst), reinterpret_cast<long>(src), reinterpret_cast<long>(bytes), static_cast<long>(n),
+                                      reinterpret_cast<long>(stream)};
+  double floats[FLOATS] = {};
+  return call_launcher(copy_batch, ints, floats);
+}
+
+// call(tape, args, deterministic) -> result, or NotImplemented when the call is not the one that was written down
+PyObject* call(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
+  HANDLE_TH_ERRORS
+  if (argc != 3 || !PyTuple_CheckExact(argv[1])) { PyErr_SetString(PyExc_TypeError, "call(tape, args, deterministic)"); return nullptr; }
+  Tape* t = static_cast<Tape*>(PyCapsule_GetPointer(argv[0], "nb_tape"));
+  if (t == nullptr) return nullptr;
+  if (PyTuple_GET_SIZE(argv[1]) != static_cast<Py_ssize_t>(t->args.size()) || (argv[2] == Py_True) != t->deterministic) Py_RETURN_NOTIMPLEMENTED;
+  std::vector<PyObject*> leaves;
+  leaves.reserve(t->leaves.size());
+  for (size_t i = 0; i < t->args.size(); ++i)
+    if (!gather(t->args[i], PyTuple_GET_ITEM(argv[1], i), leaves)) Py_RETURN_NOTIMPLEMENTED;
+  if (leaves.size() != t->leaves.size()) Py_RETURN_NOTIMPLEMENTED;
+  if (c10::cuda::current_device() != t->device) Py_RETURN_NOTIMPLEMENTED;
+  for (const auto& e : t->env) {
+    const char* v = std::getenv(e.first.c_str());
+    if (v == nullptr ? e.second.p != Py_None : (e.second.p == Py_None || std::strcmp(v, PyBytes_AS_STRING(e.second.p)) != 0)) Py_RETURN_NOTIMPLEMENTED;
+  }
+  std::vector<at::Tensor> held;                      // stay alive whatever else runs while this waits
+  held.reserve(leaves.size() + t->pins.size());
+  for (const Pin& p : t->pins) {
+    PyObject* b = slot(p.impl.p, o_buffers);
+    if (b == nullptr || !PyList_CheckExact(b) || PyList_GET_SIZE(b) != 1 || !THPVariable_Check(PyList_GET_ITEM(b, 0))) Py_RETURN_NOTIMPLEMENTED;
+    const at::Tensor& x = THPVariable_Unpack(PyList_GET_ITEM(b, 0));
+    if (x.data_ptr() != p.ptr || x.sizes() != at::IntArrayRef(p.sizes) || x.strides() != at::IntArrayRef(p.strides)) Py_RETURN_NOTIMPLEMENTED;
+    held.push_back(x);
+  }
+  std::vector<char*> bases(leaves.size() + t->outs.size() + 1, nullptr);
+  for (size_t i = 0; i < leaves.size(); ++i) {
+    const at::Tensor* x = buffer(t->leaves[i], leaves[i], t->device);
+    if (x == nullptr) Py_RETURN_NOTIMPLEMENTED;
+    held.push_back(*x);
+    bases[i] = static_cast<char*>(x->data_ptr());
+  }
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(t->device)).stream();
+  int code = 0;
+  if (t->replay.p != nullptr) {
+    const size_t n = leaves.size();
+    std::vector<void*> src(n, nullptr);
+    std::vector<unsigned long long> bytes(n, 0);
+    bool any = false;
+    for (size_t i = 0; i < n; ++i)
+      if (bases[i] != t->in_ptrs[i]) {
+        src[i] = bases[i];
+        bytes[i] = t->in_bytes[i];
+        any = any || bytes[i] > 0;
+      }
+    if (any) {
+      WithoutGil free;
+      code = run_copies(t->copy_batch, t->in_ptrs.data(), src.data(), bytes.data(), n, stream);
     }
+    if (code < 0) return PyErr_Format(PyExc_RuntimeError, "copy_batch failed with code %d", code);
+    Ref r(PyObject_CallNoArgs(t->replay.p));
+    if (r.p == nullptr) return nullptr;
+  }
+  std::vector<at::Tensor> results;
+  results.reserve(t->outs.size());
+  at::Tensor scratch;
+  const Launch* failed = nullptr;
+  {
+    WithoutGil free;
+    at::AutoDispatchBelowAutograd guard;
+    for (size_t i = 0; i < t->outs.size(); ++i) {
+      const Out& o = t->outs[i];
+      if (o.is_static) { results.emplace_back(); continue; }
+      results.push_back(at::empty_strided(o.sizes, o.strides, o.options));
+      bases[leaves.size() + i] = static_cast<char*>(results.back().data_ptr());
+    }
+    if (t->scratch) {
+      scratch = at::empty({static_cast<int64_t>(t->scratch)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, t->device));
+      bases.back() = static_cast<char*>(scratch.data_ptr());
+    }
+    if (t->replay.p != nullptr && !t->out_ptrs.empty()) {
+      std::vector<void*> dst;
+      for (size_t i = 0; i < t->outs.size(); ++i)
+        if (!t->outs[i].is_static) dst.push_back(bases[leaves.size() + i]);
+      code = run_copies(t->copy_batch, dst.data(), t->out_ptrs.data(), t->out_bytes.data(), dst.size(), stream);
+    }
+    if (code >= 0) failed = run_launches(*t, bases, stream, code);
+  }
+  if (failed == nullptr && code < 0) return PyErr_Format(PyExc_RuntimeError, "copy_batch failed with code %d", code);
+  if (failed != nullptr) {
+    PyErr_Format(PyExc_RuntimeError, "%s failed with code %d", failed->name.c_str(), code);
+    return nullptr;
   }
   std::vector<Ref> wrapped;
   wrapped.reserve(t->outs.size());

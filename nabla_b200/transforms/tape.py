@@ -303,7 +303,7 @@ def _tape(rec, tensors, tds, r: _Recorder, result_buffers):
                 out.append(e)
         launches.append((address, rc, name, out))
     return module().make((tuple(tree_of(td) for td in tds), _leaves(tensors), _environment(), device, config.is_deterministic(), launches,
-                          scratch, outs, tree_of(rec.out_treedef), None, [a for a in _captured(rec) if a.literal is None]))
+                          scratch, outs, tree_of(rec.out_treedef), None, [a for a in _captured(rec) if a.literal is None], rec.owned or []))
 
 
 def _extent(t: torch.Tensor) -> tuple[int, int]:
@@ -354,6 +354,6 @@ def graph_call(rec, tensors: list, tds: tuple):
         graph = (rec.cuda_graph.replay, address, [(t.data_ptr(), n) for t, n in zip(ins.fixed, ins.size)],
                  [(t.data_ptr(), n) for t, n in zip(outs_.fixed, outs_.size)])
         return module().make((tuple(tree_of(td) for td in tds), _leaves(tensors), _environment(), device, config.is_deterministic(), [], 0, outs,
-                              tree_of(rec.out_treedef), graph, []))
+                              tree_of(rec.out_treedef), graph, [], [*ins.fixed, *outs_.fixed, *(rec.owned or [])]))
     except _Refused:
         return None

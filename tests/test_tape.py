@@ -337,3 +337,40 @@ def test_a_graph_of_the_callers_outlives_the_function():
     g.replay()
     torch.cuda.synchronize()
     assert torch.allclose(grad.to_torch().double(), 2 * (x.double() - y.double()) / x.numel(), rtol=1e-4, atol=1e-9) and held
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """More launches than a stream's queue holds behind a kernel of half a second: the caller waits, and Python goes on elsewhere."""
+    import time
+
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    f = nb.compile(lambda x, a, b: F.layer_norm(F.layer_norm(x, a, b), a, b))
+    args = [_wrap(t) for t in (torch.randn(8, 512, device="cuda"), torch.ones(512, device="cuda"), torch.zeros(512, device="cuda"))]
+    for _ in range(3):
+        f(*args)
+    assert _taped(f), f.tape_refused
+    torch.cuda.synchronize()
+    done, gaps = threading.Event(), [0.0]
+
+    def tick():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    other = threading.Thread(target=tick)
+    other.start()
+    torch.cuda._sleep(1_000_000_000)
+    t0 = time.perf_counter()
+    for _ in range(2500):
+        f(*args)
+    waited = time.perf_counter() - t0
+    done.set()
+    other.join()
+    torch.cuda.synchronize()
+    assert waited > 0.3, "the queue was never full"
+    assert max(gaps) < 0.2 * waited
