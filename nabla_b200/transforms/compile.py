@@ -193,6 +193,7 @@ class _Recorded:
         self.owned: list[torch.Tensor] | None = None     # GPU tensors that go with the recording: its constants and the numbers in it
         self.told: set[int] = set()                 # raw streams that the allocator knows to read them
         self.tape = None                            # of later calls without Python (transforms/tape.py); False: none
+        self.tape_of_graph = False                  # it replays the graph
         self.tape_counts: tuple = ()                # launches of a taped call: GEMM, fused kernels, attention
         self.tape_tries = 0
         self.host_sync = False                      # holds a node that reads a device value on the host
@@ -402,23 +403,23 @@ class CompiledFunction:
         if self.profile_ops or graphs is not self.use_cuda_graph or rec.tape is not handle \
                 or (rec.constants and torch.cuda.is_current_stream_capturing()):     # see _run
             return NotImplemented
-        t0 = time.perf_counter()
         _tell_stream(rec)
         out = tape.module().call(handle, args, config.is_deterministic())
         if out is not NotImplemented:
             for module, n in zip(_counted_modules(), rec.tape_counts):
                 module.launch_count += n
-            if rec.cuda_graph is None:
+            if not rec.tape_of_graph:
                 _STATS["nodes_executed"] += len(rec.nodes)
-            self._stats.hits += 1
-            self._stats.replay_time_s += time.perf_counter() - t0
         return out
 
     def __call__(self, *args, **kwargs):
         taped = self._taped             # read once: another thread may replace it
         if taped is not None and not kwargs:
+            t0 = time.perf_counter()
             out = self._call_taped(taped, args)
             if out is not NotImplemented:
+                self._stats.hits += 1
+                self._stats.replay_time_s += time.perf_counter() - t0
                 return out
         args = tuple(_normalize_step_scalars(a) for a in args)
         kwargs = {k: _normalize_step_scalars(v) for k, v in kwargs.items()}
@@ -428,7 +429,7 @@ class CompiledFunction:
             if leaves is not None:
                 self._stats.hits += 1              # the entry is the most recently used one already
                 t0 = time.perf_counter()
-                out = self._replay(latest[2], leaves, latest[0])
+                out = self._replay(latest[2], leaves, latest[0], args)
                 self._stats.replay_time_s += time.perf_counter() - t0
                 return out
         self._taped = None
@@ -476,7 +477,7 @@ class CompiledFunction:
             return result
         t0 = time.perf_counter()
         plain = not kwargs and self.max_cache_size > 0 and all(type(l) is Tensor and l._impl.sharding is None for l in leaves)
-        out = self._replay(rec, [l for l in leaves if isinstance(l, Tensor)], td[0] if plain else None)
+        out = self._replay(rec, [l for l in leaves if isinstance(l, Tensor)], td[0] if plain else None, args)
         self._stats.replay_time_s += time.perf_counter() - t0
         if plain:
             self._latest = (td[0], conc, rec, config.is_deterministic())
@@ -850,14 +851,21 @@ class CompiledFunction:
                 impl._buffers = None
         return pytree.tree_unflatten(rec.out_treedef, outs)
 
-    def _replay(self, rec: _Recorded, tensors: list[Tensor], tds: tuple | None = None) -> Any:
-        """``tds``: the arguments' structures, where nothing but tensors is among them."""
+    def _replay(self, rec: _Recorded, tensors: list[Tensor], tds: tuple | None = None, args: tuple = ()) -> Any:
+        """``tds``: the structures of the arguments ``args``, where nothing but tensors is among them."""
+        if rec.tape and tds is not None:            # written down already, whatever was called in between
+            taped = (rec.tape, rec, self.use_cuda_graph)
+            out = self._call_taped(taped, args)
+            if out is not NotImplemented:
+                self._taped = taped
+                return out
         _tell_stream(rec)
         if self.use_cuda_graph and not rec.host_sync and tensors and tensors[0]._impl.device.label == "gpu" \
                 and not (rec.cuda_graph is None and rec.tape is None and tds is not None and _copies_outweigh_launches(rec) and tape.can_record(rec)):
             out = self._replay_cuda_graph(rec, tensors)
             if rec.tape is None and rec.cuda_graph is not None and tds is not None and rec.copy_out is not None:
                 rec.tape = tape.graph_call(rec, tensors, tds) or False
+                rec.tape_of_graph = bool(rec.tape)
                 rec.tape_counts = (0, rec.copy_in.launches + rec.copy_out.launches, 0) if rec.tape else ()
             self._taped = (rec.tape, rec, True) if rec.tape and tds is not None else None
             return out
@@ -906,7 +914,7 @@ class CompiledFunction:
                 for ph in rec.placeholders:
                     ph._buffers = None
                 return self._replay(rec, tensors)
-            rec.tape = None
+            rec.tape = rec.tape or None             # launches that were written down serve on, the graph the calls that they do not match
             rec.cuda_graph = g
             self._stats.cuda_graphs += 1
             self._stats.launches_per_graph = total_launches() - n0

@@ -374,3 +374,38 @@ def test_other_threads_run_while_a_launch_waits():
     torch.cuda.synchronize()
     assert waited > 0.3, "the queue was never full"
     assert max(gaps) < 0.2 * waited
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_calls_of_several_signatures_in_turn(graph, monkeypatch):
+    """Each signature keeps its tape whatever is called in between, an odd call of its own included; none of them is run by Python again."""
+    import nabla_b200 as nb
+    from nabla_b200.transforms.compile import CompiledFunction
+
+    f = nb.compile(lambda x, w: x @ w, cuda_graph=graph)
+    g = torch.Generator("cuda").manual_seed(4)
+    xs = [torch.randn(n, 4096, generator=g, device="cuda").to(BF16) for n in (2048, 4096)]
+    w = (torch.randn(4096, 2048, generator=g, device="cuda") * 0.02).to(BF16)
+    want = [x.double() @ w.double() for x in xs]
+
+    def check(k, x):
+        assert (f(_wrap(x), _wrap(w)).to_torch().double() - want[k]).norm() < 4e-3 * want[k].norm()
+
+    for k in (0, 0, 1, 1):                            # traced and written down, one after the other
+        check(k, xs[k])
+    by_python = []
+    for name in ("_run", "_replay_cuda_graph"):
+        monkeypatch.setattr(CompiledFunction, name, lambda self, *a, _f=getattr(CompiledFunction, name), **k: by_python.append(1) or _f(self, *a, **k))
+    hits = f.stats.hits
+    for _ in range(4):
+        for k in (0, 1):
+            check(k, xs[k])
+            assert _taped(f), f.tape_refused
+    assert not by_python and f.stats.hits == hits + 8 and f.stats.cuda_graphs == 0
+    check(1, xs[1].t().contiguous().t())              # columns first
+    assert by_python
+    by_python.clear()
+    for k in (1, 0, 1):
+        check(k, xs[k])
+        assert _taped(f)
+    assert not by_python
