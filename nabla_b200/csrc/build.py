@@ -3,7 +3,7 @@
 Each `.cu` / `.cpp` translation unit listed in ``TARGETS`` becomes one shared library in
 ``nabla_b200/lib``. The libraries export plain C symbols and are loaded with ctypes
 (`nabla_b200.native`), so they do not depend on the torch C++ headers and rebuild in seconds;
-``libnb_replay.so`` alone is a Python extension on torch's C++ interface. nvcc cross-compiles
+``libnb_replay.so`` alone is a Python extension on torch's C++ interface, and is left out where it cannot be built. nvcc cross-compiles
 without a GPU present.
 
 ``build_all(debug=True)`` (``python -m nabla_b200.csrc.build --debug``) compiles the same sources
@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -41,15 +42,29 @@ TARGETS: dict[str, tuple[list[str], list[str]]] = {
 }
 
 
-def _torch_flags() -> list[str]:
+def replay_built_for() -> str:
+    """The Python and torch whose binary interfaces ``libnb_replay.so`` uses, as it names them itself."""
+    import torch
+
+    return re.sub(r"\W", "_", f"python{sys.version_info[0]}.{sys.version_info[1]}_torch{torch.__version__}")
+
+
+def _torch_flags() -> list[str] | None:
+    """Flags of a target on torch's C++ interface; None where it cannot be built (its calls know one calling convention; Python's or
+    torch's headers may not be there): compiled calls are replayed by Python then."""
+    import platform
     import sysconfig
 
     import torch
 
     base = Path(torch.__file__).resolve().parent
-    inc = [base / "include", base / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"]]
+    python = Path(sysconfig.get_paths()["include"])
+    if sys.platform != "linux" or platform.machine() not in ("x86_64", "AMD64") or not (python / "Python.h").exists() \
+            or not (base / "include" / "torch" / "csrc" / "autograd" / "python_variable.h").exists() or not (base / "lib" / "libc10_cuda.so").exists():
+        return None
+    inc = [base / "include", base / "include" / "torch" / "csrc" / "api" / "include", python]
     return [*(f"-I{p}" for p in inc), f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-L{base / 'lib'}", "-lc10", "-lc10_cuda",
-            "-ltorch_cpu", "-ltorch_python", "-ltorch", f"-DTORCH_OF_BUILD={torch.__version__.replace('+', '_')}"]
+            "-ltorch_cpu", "-ltorch_python", "-ltorch", f"-DNB_BUILT_FOR={replay_built_for()}"]
 
 
 def _nvcc() -> str:
@@ -83,7 +98,10 @@ def build_all(force: bool = False, verbose: bool = False, debug: bool = False) -
         is_cuda = any(p.suffix == ".cu" for p in paths)
         flags = (NVCC_FLAGS if is_cuda else ["-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC"]) + extra
         if "torch" in flags:
-            flags = [f for f in flags if f != "torch"] + _torch_flags()
+            more = _torch_flags()
+            if more is None:
+                continue
+            flags = [f for f in flags if f != "torch"] + more
         if debug:
             flags = flags + ["-DNB_DEBUG_CHECKS"]
         dig = _digest(paths, flags)

@@ -578,4 +578,13 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "libnb_replay", nullptr, -1, method
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_libnb_replay() { return PyModule_Create(&module); }
+#define NB_TEXT_(x) #x
+#define NB_TEXT(x) NB_TEXT_(x)
+PyMODINIT_FUNC PyInit_libnb_replay() {
+  PyObject* m = PyModule_Create(&module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", NB_TEXT(NB_BUILT_FOR)) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

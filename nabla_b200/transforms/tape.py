@@ -42,23 +42,34 @@ _module = None
 
 
 def module():
-    """The extension, or None where it is not built."""
+    """The extension, or None where it is not built, or not for this Python and torch (then Python replays)."""
     global _module
     if _module is None:
-        path = native.lib_path("libnb_replay.so")
-        if not path.exists():
-            _module = False
-        else:
-            import importlib.machinery
-            import importlib.util
-
-            loader = importlib.machinery.ExtensionFileLoader("libnb_replay", str(path))
-            spec = importlib.util.spec_from_file_location("libnb_replay", str(path), loader=loader)
-            m = importlib.util.module_from_spec(spec)
-            loader.exec_module(m)
-            m.classes(Tensor, TensorImpl)
-            _module = m
+        _module = _load() or False
     return _module or None
+
+
+def _load():
+    import importlib.machinery
+    import importlib.util
+    import warnings
+
+    from ..csrc.build import replay_built_for
+
+    path = native.lib_path("libnb_replay.so")
+    if not path.exists():
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("libnb_replay", str(path))
+    try:
+        m = importlib.util.module_from_spec(importlib.util.spec_from_file_location("libnb_replay", str(path), loader=loader))
+        loader.exec_module(m)
+        if m.built_for != replay_built_for():
+            raise ImportError(f"it was built for {m.built_for}, this is {replay_built_for()}")
+        m.classes(Tensor, TensorImpl)
+    except (ImportError, OSError, AttributeError) as e:
+        warnings.warn(f"{path.name} cannot be used, compiled calls are replayed by Python (python -m nabla_b200.csrc.build builds it anew): {e}")
+        return None
+    return m
 
 
 class _Refused(Exception):

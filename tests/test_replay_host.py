@@ -100,3 +100,34 @@ def test_a_graph_of_the_callers_gets_constants_of_its_own(gpu, monkeypatch):
     f._run(rec)
     assert seen[0] is not made and torch.equal(seen[0], made) and seen[1] is made and constant._buffers[0] is made
     assert helper._buffers is None
+
+
+@pytest.mark.parametrize("what", ["garbage", "other version"])
+def test_an_extension_that_does_not_load_is_one_that_is_not_there(what, tmp_path, monkeypatch):
+    """Built for another Python or torch, or broken: said once, and calls go on by Python."""
+    path = native.lib_path("libnb_replay.so")
+    if what == "garbage":
+        path = tmp_path / "libnb_replay.so"
+        path.write_bytes(b"no library")
+        monkeypatch.setattr(native, "lib_path", lambda name: path)
+    else:
+        if not path.exists():
+            pytest.skip("not built")
+        from nabla_b200.csrc import build
+
+        monkeypatch.setattr(build, "replay_built_for", lambda: "another", raising=False)
+    monkeypatch.setattr(tape, "_module", None)
+    with pytest.warns(UserWarning, match="replayed by Python"):
+        assert tape.module() is None
+    assert tape.module() is None                     # and not a second time
+
+
+def test_build_leaves_the_extension_out_where_it_cannot_be_built(tmp_path, monkeypatch):
+    import platform
+
+    from nabla_b200.csrc import build
+
+    monkeypatch.setattr(platform, "machine", lambda: "aarch64")
+    monkeypatch.setattr(build, "LIB", tmp_path)
+    monkeypatch.setattr(build, "TARGETS", {"libnb_replay.so": build.TARGETS["libnb_replay.so"]})
+    assert build.build_all() == [] and not list(tmp_path.iterdir())
