@@ -146,14 +146,25 @@ def _value(arg) -> int:
 
 
 def can_record(rec) -> bool:
-    """Is the schedule one whose launches all go through the wrappers that are observed?"""
-    return (module() is not None and os.environ.get("NABLA_B200_TAPE", "1") != "0" and not rec.host_sync and not rec.side_steps and not any(rec.donated)
-            and not rec.arena_blocks and rec.placeholders and all(p.sharding is None and p.device.label == "gpu" for p in rec.placeholders)
-            and all(type(n.op).__module__.startswith(("nabla_b200.ops.", "nabla_b200.nn.finetune.")) and not type(n.op).__module__.endswith((".custom", ".custom_op", ".communication"))
-                    and ".communication." not in type(n.op).__module__
-                    and all(o is None or o.sharding is None for o in n.outputs()) for n in rec.nodes)
+    """Is this a call whose launches all go through the wrappers that are observed? A recording of which none is says so once (``rec.tape``)."""
+    if not _recordable(rec):
+        rec.tape = False
+        return False
+    return (module() is not None and os.environ.get("NABLA_B200_TAPE", "1") != "0" and not rec.arena_blocks
             and not torch.cuda.is_current_stream_capturing() and _get_current_dispatch_mode() is None
             and not config.get_flag("VERIFY_EAGER_SHAPES"))
+
+
+def _recordable(rec) -> bool:
+    """What of it the recording decides."""
+    def own(op) -> bool:
+        m = type(op).__module__
+        return m.startswith(("nabla_b200.ops.", "nabla_b200.nn.finetune.")) and not m.endswith((".custom", ".custom_op", ".communication")) \
+            and ".communication." not in m
+
+    return bool(not rec.host_sync and not rec.side_steps and not any(rec.donated)
+                and rec.placeholders and all(p.sharding is None and p.device.label == "gpu" for p in rec.placeholders)
+                and all(own(n.op) and all(o is None or o.sharding is None for o in n.outputs()) for n in rec.nodes))
 
 
 def _leaves(tensors) -> list:

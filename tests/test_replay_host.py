@@ -122,6 +122,21 @@ def test_an_extension_that_does_not_load_is_one_that_is_not_there(what, tmp_path
     assert tape.module() is None                     # and not a second time
 
 
+def test_a_recording_that_cannot_be_taped_says_so_once(monkeypatch):
+    """Without the extension being looked for, and without its nodes being looked over on every call."""
+    def unexpected():
+        raise AssertionError("looked for the extension")
+
+    monkeypatch.setattr(tape, "module", unexpected)
+    f = nb.compile(lambda x: x * 2.0 + 1.0)
+    x = nb.Tensor.from_torch(torch.ones(3))
+    for _ in range(3):
+        assert f(x).to_torch().tolist() == [3.0, 3.0, 3.0]
+    (entry,) = f._cache.values()
+    (rec,) = entry.values()
+    assert rec.tape is False
+
+
 def test_build_leaves_the_extension_out_where_it_cannot_be_built(tmp_path, monkeypatch):
     import platform
 
