@@ -252,7 +252,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // an earlier bounded wait on this device already failed: leave (uniformly)
+  // an earlier bounded wait on this device already failed, as far as is known before the grid ahead has ended: leave (uniformly)
   if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return follow_grid();
   const int nqt = (args.Sq + args.q_tiles * BT - 1) / (args.q_tiles * BT);
   int bh_, rank;
@@ -948,7 +948,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // an earlier bounded wait on this device already failed: leave (uniformly)
+  // an earlier bounded wait on this device already failed, as far as is known before the grid ahead has ended: leave (uniformly)
   if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return follow_grid();
   if (smem_u32(smem) & 1023u) {     // the swizzled tiles need it, and the size above leaves no room to align
     if (threadIdx.x == 0) atomicExch(args.status, NB_ERR_TIMEOUT_PRODUCER);
@@ -1284,7 +1284,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // an earlier bounded wait on this device already failed: leave (uniformly)
+  // an earlier bounded wait on this device already failed, as far as is known before the grid ahead has ended: leave (uniformly)
   if (__syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(args.status) : 0)) return follow_grid();
   const int nqt = (args.Sq + BT - 1) / BT;
   int bh_, rank;
@@ -1333,7 +1333,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // The dK / dV kernel ahead writes nothing that is read here, and it lets this grid begin only when the statistics and all before them
+  // (An exception to the rule, see launch.cuh.) The dK / dV kernel ahead writes nothing that is read here, and it lets this grid begin only when the statistics and all before them
   // are in memory: so the blocks work beside its last ones and wait for its end before their own. (Reads go to L2, past lines that this SM
   // may hold; a mask of rows is read through them.) us: 2 x 8 heads x 1001 x 64 causal 184 -> 176 in
   // a block's training step, 8 x 12 x 777 x 64 with a mask of keys 200 -> 198 and 4 x 16 x 2048 x 128 397 -> 394, both with their forward pass.

@@ -222,7 +222,7 @@ __device__ __forceinline__ bool gemm_cta(const CUtensorMap* tmAp, const CUtensor
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // a previous bounded wait failed on this device: do not pile more waits on top of it
+  // a previous bounded wait failed on this device (as far as is known before the grid ahead has ended): do not pile more waits on top of it
   // (a pair does not leave early: both CTAs must reach the cluster barriers below, and their waits
   // are bounded anyway). The word is fetched under the set-up below and looked at after it: half a microsecond of a small
   // product's five

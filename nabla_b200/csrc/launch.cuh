@@ -14,6 +14,14 @@
 //  - only then does it let the next launch begin, so no more than two grids of a stream are on the chip. A kernel that takes
 //    tensor memory has it by then: a waiting block may wait for the tensor memory of a running one, never the other way.
 //  - a kernel without follow_grid() is launched with <<< >>> and waits for the end of all that is ahead of it, as before.
+// Two exceptions, and what they rest on:
+//  - kernels with bounded waits look at the device's status word while they set up, half a microsecond that a launch would otherwise
+//    pay behind its wait. They see it as of then: the launch right behind one whose wait ran out may still start, and meets the limits
+//    of its own waits; the one behind it leaves. Nothing else follows from the word on the device.
+//  - attn_bwd_dq_kernel, unless it reads a mask of a row per query, works and lets the next launch begin before it has waited. The kernel ahead of it, dK / dV,
+//    writes nothing that it reads and reads nothing that it writes, and begins it only behind its own wait, so all that came before is
+//    complete; what it reads goes past L1; and its blocks wait before they end, so whoever waits for it has dK and dV too. Three grids
+//    are on the chip then. A second kernel of this kind directly behind it would not have that ground to stand on.
 #pragma once
 #include <cuda_runtime.h>
 
