@@ -58,6 +58,8 @@ def test_every_kernel_of_a_following_launch_waits_for_the_grid_ahead():
     import re
 
     csrc = ROOT / "nabla_b200" / "csrc"
+    as_of_now = (csrc / "launch.cuh").read_text().split("void as_of_now(")[1].split("\n}\n")[0]
+    assert "__cvta_generic_to_global(" in as_of_now and "__cvta_global_to_generic(" in as_of_now      # still pointers to global memory
     for name in ("gemm_tcgen05.cu", "attention_tcgen05.cu", "fused_kernels.cu", "elementwise_kernels.cu"):
         src = re.sub(r"//[^\n]*", "", (csrc / name).read_text())
         cta = src[src.index("bool gemm_cta("):] if "bool gemm_cta(" in src else ""
