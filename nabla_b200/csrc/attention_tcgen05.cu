@@ -706,8 +706,11 @@ struct DecodeArgs {
 };
 constexpr int DEC_MAX_Q = 4, DEC_U = 4;
 
-template <int HD, int NQ, int WARPS, bool CLUSTER>
-__global__ void __launch_bounds__(32 * WARPS, NQ == 1 ? (WARPS == 4 ? 4 : 3) : NQ == 2 ? (WARPS == 4 ? 5 : 2) : 1) attn_decode_kernel(const DecodeArgs a) {
+// AHEAD (one query, blocks of four warps): the next keys and values are on their way while the current ones are worked on, for which four
+// blocks fit an SM instead of seven: for grids that need no more (dec_ahead). Of eight warps with so many registers fewer clusters of 16 fit
+// the chip (16 x 8000 18.1, 24.2), and two queries have the registers no more.
+template <int HD, int NQ, int WARPS, bool CLUSTER, bool AHEAD>
+__global__ void __launch_bounds__(32 * WARPS, NQ == 1 ? (WARPS == 4 ? (AHEAD ? 4 : 7) : 3) : NQ == 2 ? (WARPS == 4 ? 5 : 2) : 1) attn_decode_kernel(const DecodeArgs a) {
   follow_grid();
   constexpr int LPK = HD / 8, KPW = 32 / LPK, G = WARPS * KPW;      // lanes per key, keys per warp, lane groups per block
   const FwdArgs& f = a.f;
@@ -743,10 +746,6 @@ __global__ void __launch_bounds__(32 * WARPS, NQ == 1 ? (WARPS == 4 ? 4 : 3) : N
       }
     }
   };
-  // One query, blocks of four warps: the next keys and values are on their way while the current ones are worked on (64 heads x 4001 keys
-  // of 128 28.1 -> 26.9 us, 256 x 8000 178 -> 167). Of eight warps with so many registers fewer clusters of 16 fit the chip (16 x 8000
-  // 18.1, 24.2), and two queries have the registers no more.
-  constexpr bool AHEAD = NQ == 1 && WARPS == 4;
   uint4 kr[DEC_U], vr[DEC_U], kn[DEC_U], vn[DEC_U];
   if (AHEAD) fetch(k0 + grp, kn, vn);
   for (int kb = k0 + grp; kb - grp < k1; kb += G * DEC_U) {
@@ -1692,12 +1691,19 @@ static void combine(const FwdArgs& a, cudaStream_t stream) {
 // Blocks of a cluster for so many warps on a (batch, head): of four warps, of eight above 32.
 static int dec_cluster(int warps) { return warps > 32 ? warps / 8 : warps / 4; }
 
+// Blocks that load ahead hold 592 of four warps on the chip, clusters of more than two of them 512 (not every group of SMs divides into whole ones). us,
+// one query, loading ahead and not: clusters of 64 pairs x 4001 keys x 128 26.9, 28.1, of 148 (592 blocks) 76, 61; ranges of 148 pairs x 4001 55, 60, of
+// 300 (600 blocks) 137, 107.
+static bool dec_ahead(int queries, int warps, long long blocks) { return queries == 1 && warps <= 32 && blocks <= (warps > 8 ? 512 : 592); }
+
 // warps 0: key ranges joined by a second launch.
 template <int HD, int NQ>
 static int launch_decode(const DecodeArgs& a, int warps, cudaStream_t stream) {
+  constexpr bool ONE = NQ == 1;
   const dim3 grid(a.f.nsplit, a.f.B * a.f.H);
+  const bool ahead = dec_ahead(a.f.Sq, warps, (long long)grid.x * grid.y);
   if (warps == 0) {
-    launch_following(attn_decode_kernel<HD, NQ, 4, false>, grid, 128, 0, stream, a);
+    launch_following(ahead ? attn_decode_kernel<HD, NQ, 4, false, ONE> : attn_decode_kernel<HD, NQ, 4, false, false>, grid, 128, 0, stream, a);
     if (a.f.nsplit > 1) combine<HD>(a.f, stream);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
   }
@@ -1712,7 +1718,8 @@ static int launch_decode(const DecodeArgs& a, int warps, cudaStream_t stream) {
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const auto kernel = warps > 32 ? attn_decode_kernel<HD, NQ, 8, true> : attn_decode_kernel<HD, NQ, 4, true>;
+  const auto kernel = warps > 32 ? attn_decode_kernel<HD, NQ, 8, true, false>
+                      : ahead    ? attn_decode_kernel<HD, NQ, 4, true, ONE> : attn_decode_kernel<HD, NQ, 4, true, false>;
   if (a.f.nsplit > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return -2;
   set_following(cfg);
   return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? 0 : -3;
@@ -1819,18 +1826,37 @@ extern "C" int nb_attn_fwd_splits(int B, int H, int Sq, int Skv, int D, int has_
 }
 
 // Warps that a (batch, head) of the decode kernel is given in a cluster of blocks, which needs no scratch and no second launch (0: key
-// ranges as above). Timed over 4 to 512 pairs, 64 to 8000 keys, one and two queries, both head_dims, every number of warps: as many as
-// leave a warp 8 keys, and as are resident (fewer registers' worth with two queries and in blocks of eight warps). What stays with the
-// ranges: chips that would be left half empty under long walks (us, ranges and clusters: 37 pairs x 4001 keys x 128, two queries 26.2,
-// 30.1), and few keys for many pairs (256 x 300 x 64 9.1, 9.9). us, ranges and clusters, one query: 4 pairs x 8000 keys x 128 21.6,
-// 13.6; 16 x 1000 12.2, 7.9; 32 x 4001 23.9, 19.7; 64 x 512 11.4, 8.8; 148 x 1000 23.3, 21.3; 300 x 4001 116, 114.
+// ranges as above). Timed for every number of warps and the ranges over 4 to 512 pairs, 128 to 8000 keys, one and two queries, both head_dims (826
+// sizes, calls in a row): as many warps as have eight keys each and as leave no cluster waiting for its turn. The lines:
+//  - blocks of eight warps take few pairs, by 3 (one query) and 2 blocks an SM; a pair on 16 of them wants keys enough for the larger exchange.
+//  - of four warps 512 blocks load ahead, up to 800 do not, and those of larger clusters pay under more keys only. Two queries: 600 blocks.
+//  - ranges win where they fill the chip evenly and clusters do not (148 pairs x 4001 x 128 55 us, clusters 61), where clusters would leave it half
+//    empty under long walks (two queries, 37 x 4001 x 128 26.2, 30.1), and under few keys (256 x 300 x 64 9.1, 9.9).
+// us, ranges and clusters, one query: 4 pairs x 8000 keys x 128 21.6, 13.6; 16 x 1000 12.2, 7.9; 32 x 4001 23.9, 19.7; 64 x 512 11.4, 8.8.
 extern "C" int nb_attn_decode_warps(int B, int H, int Sq, int Skv, int D, int has_mask) {
   if (B <= 0 || H <= 0 || Sq <= 0 || Sq > 2 || Skv < 128 || !attn_decode(B, H, Sq, Skv, D, has_mask != 0)) return 0;
   const long long bh = (long long)B * H;
-  auto most = [&](int w) { return Sq == 1 ? (w > 32 ? 2400 : 3200) : w > 64 ? 1024 : w > 32 ? 2048 : 2560; };
+  const bool one = Sq == 1, wide = D == 128;
+  auto takes = [&](int w) {
+    if (w == 128) return bh <= (one ? 16 : 8) && Skv >= (bh <= 4 ? 1500 : 3000);
+    if (w == 64) return bh <= (one ? 48 : 32) && Skv >= (wide ? 300 : 700) && (one || !wide || Skv < 8000);
+    const long long blocks = bh * w / 4;
+    return w * 8 <= Skv && (one ? blocks <= 512 || (blocks <= 800 && Skv >= (w == 8 ? 128 : w == 16 ? 700 : 1000)) : blocks <= 600);
+  };
   int w = 128;
-  while (w > 4 && (w * bh > most(w) || w * 8 > Skv)) w /= 2;
-  if (w < 8 || (bh > 148 && Skv < (D == 64 ? 512 : 300)) || (bh > 74 && D == 64 && Skv < 192) || (w * bh < 1900 && Skv > 100 * w)) return 0;
+  while (w >= 8 && !takes(w)) w /= 2;
+  if (w < 8) return 0;
+  if (one) {
+    if (w <= 32 && 592 % bh == 0 && (Skv >= 1500 || w * bh > 4 * 512)) return 0;
+    if (wide ? (Skv < 160 && bh > 8) || (Skv < 300 && bh > 256) : (Skv < 200 && bh > 4) || (Skv < 300 && bh > 16) || (Skv < 320 && bh > 24 && bh < 64)) return 0;
+    if (!wide && bh > 148 && Skv < 512) return 0;
+  } else {
+    if (w == 32 && Skv >= (w * bh < 1300 ? 3000 : wide ? 4000 : 6000)) return 0;
+    if (w == 16 && bh > 74 && Skv >= (wide ? 700 : 1500)) return 0;
+    if (w == 8 && w * bh < 1900 && Skv >= 1000) return 0;
+    if (wide ? Skv < 160 && bh > 24 : Skv < 160 || (Skv < 300 && bh > 16) || (Skv < 512 && bh > 24 && bh < 64)) return 0;
+    if (bh >= 148 && Skv < (wide ? 300 : 512)) return 0;
+  }
   return w;
 }
 

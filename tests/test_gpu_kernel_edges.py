@@ -1588,6 +1588,26 @@ def test_few_queries_over_clusters(B, H, Sq, Skv, D, warps):
     assert o[0, 0, -1].isnan().all() and not o[0, 0, :-1].isnan().any() and not o.reshape(-1, Sq, D)[1:].isnan().any()
 
 
+@pytest.mark.parametrize("bh,Sq,Skv,D,warps", [(148, 1, 2001, 128, 0), (149, 1, 2001, 128, 16), (128, 1, 901, 64, 16), (129, 1, 901, 64, 16), (96, 1, 999, 64, 16),
+                                               (96, 1, 1001, 64, 32), (296, 1, 700, 64, 0), (297, 1, 700, 64, 8), (290, 1, 700, 64, 8), (400, 1, 700, 128, 8), (16, 1, 2999, 128, 64), (16, 1, 3000, 128, 128), (300, 1, 130, 64, 0),
+                                               (192, 2, 999, 64, 8), (192, 2, 1000, 64, 0), (24, 2, 8000, 128, 0)])
+def test_few_queries_by_what_fits_the_chip(bh, Sq, Skv, D, warps):
+    """Grids that load ahead and that do not, in clusters (up to 512 blocks) and in ranges (592), one block to either side, against 64 bits."""
+    from nabla_b200.native import attention
+
+    attention._lib()
+    assert attention._warps(1, bh, Sq, Skv, D, 0) == warps
+    torch.manual_seed(31)
+    q = torch.randn(1, bh, Sq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(1, bh, Skv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    o, lse = attention.sdpa_fwd(q, k, v, causal=True, scale=D ** -0.5)
+    for h in range(0, bh, 64):
+        w = slice(h, h + 64)
+        s = (q[:, w].double() @ k[:, w].double().transpose(-1, -2)) * D ** -0.5
+        s = s.masked_fill(~torch.ones(Sq, Skv, dtype=torch.bool, device="cuda").tril(Skv - Sq), float("-inf"))
+        assert _rel2(o[:, w], torch.softmax(s, -1) @ v[:, w].double()) < 1.85e-3 and _rel2(lse[:, w], torch.logsumexp(s, -1)) < 1e-5
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("N,H,C,F,k,pool,stride", [(3, 12, 1, 8, 3, 2, 2), (2, 11, 4, 12, 3, 2, 2), (2, 9, 3, 5, 2, 3, 2), (5, 16, 8, 32, 3, 2, 2)])
 def test_compiled_convolutions_take_their_relu(dtype, N, H, C, F, k, pool, stride):
