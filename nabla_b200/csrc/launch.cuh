@@ -53,8 +53,11 @@ inline void set_following(cudaLaunchConfig_t& cfg) {
   a.val.programmaticStreamSerializationAllowed = 1;
 }
 
+// A kernel with follow_grid() may also be launched behind all that is ahead of it (`following` false). Blocks that start in the room that running ones
+// leave are not spread evenly: where a grid is less than the SMs could hold, some of them get several blocks and others none, and a
+// kernel that runs for long then pays more than the start of a launch.
 template <typename... Params, typename... Args>
-inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_when(bool following, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.gridDim = grid;
@@ -62,8 +65,12 @@ inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 b
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  set_following(cfg);
+  if (following) set_following(cfg);
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_when(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace nb
