@@ -11,7 +11,7 @@ CUDA bf16 tensors:
   process per GPU: one launch of the fused GEMM + collective kernel (tiles are reduced over
   NVLink while later tiles are still being multiplied).
 * ``linear (+bias) | matmul -> add(residual)``: the residual is added in the GEMM epilogue (compiled replays).
-* ``x @ w [+ b] + (h @ v) [* one element]`` with a K of h of up to 256 (a frozen weight and its adapter): one launch, whose accumulator takes both
+* ``x @ w [+ b] + (h @ v) [* a power of two]`` with a K of h of up to 256 (a frozen weight and its adapter): one launch, whose accumulator takes both
   products (compiled replays).
 * ``matmul -> mul(one element)`` and ``mul(one element) -> matmul ...`` (the scale of a LoRA adapter and its gradient): the
   factor is applied in the GEMM epilogue (compiled replays).
@@ -491,6 +491,11 @@ def _sum_of_products(i: int, nodes, cons, used, producer, private_intermediate, 
             or depth >= int(nodes[large[0]].input_impls()[0]._shape[-1]):
         return None
     return small + large + [k]
+
+
+def _is_power_of_two(x) -> bool:
+    """A number that scales bf16 values without rounding them."""
+    return x is not None and 2.0 ** -64 <= x <= 2.0 ** 64 and math.frexp(x)[0] == 0.5
 
 
 def _is_counted_step(add: OpNode, o: TensorImpl) -> bool:
@@ -1009,11 +1014,12 @@ def run_fused(kind: str, group: list[OpNode], keep_graph: bool = False, arena_bl
         a, b = ins[:2]
         k, k2, n_out = a.shape[-1], a2.shape[-1], b.shape[-1]
         m = a.numel() // max(k, 1)
-        if native.use_native(a) and a.numel() and b.numel() and dual_takes(m, n_out, k, k2):
+        # the thin operand takes a factor that does not round it; any other is applied to the fp32 product, in launches of their own
+        factor = _scalar_factor(group[1], small.outputs()[0]) if len(group) == 4 else None
+        if native.use_native(a) and a.numel() and b.numel() and dual_takes(m, n_out, k, k2) and (factor is None or _is_power_of_two(factor.literal)):
             a2 = a2.reshape(-1, k2)
-            if len(group) == 4:
-                factor = _scalar_factor(group[1], small.outputs()[0])
-                if factor.literal != 1:                    # the thin operand takes the factor
+            if factor is not None:
+                if factor.literal != 1:
                     s = factor._buffers[0].reshape(())
                     scaled = kernels.binary(a2, s, "mul")
                     a2 = scaled if scaled is not None else a2 * s

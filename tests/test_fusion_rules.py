@@ -191,3 +191,13 @@ def test_column_sums_go_by_clusters_where_these_fill_the_chip(rows, cols, bf16, 
     from nabla_b200.native.kernels import colsum_clusters
 
     assert colsum_clusters(rows, cols, torch.bfloat16 if bf16 else torch.float32) == how
+
+
+def test_factors_that_a_thin_operand_takes_do_not_round_it():
+    """Beside a larger product a low-rank one is scaled before it: by powers of two alone, whose products with bf16 values are exact."""
+    h = torch.randn(1000).bfloat16()
+    for x, takes in ((1, True), (1.0, True), (2.0, True), (0.25, True), (0.75, False), (4 / 3, False), (-2.0, False), (0.0, False), (True, True), (None, False),
+                     (float("inf"), False), (float("nan"), False), (2.0 ** 100, False), (10 ** 400, False)):
+        assert fusion._is_power_of_two(x) is takes, x
+        if takes:
+            assert torch.equal((h * x).double(), h.double() * x)
