@@ -781,7 +781,8 @@ __global__ void __launch_bounds__(256) colsum_narrow_kernel(const T* __restrict_
 // Column sums of several matrices in one launch, without a second one that folds slabs: the blocks of a cluster share a
 // tile of L vectors of columns, walk every row of it between them and meet in distributed shared memory. A block is 256 / L
 // row slots, whose rows are interleaved over the cluster; a thread asks for eight rows before it adds the first and adds
-// them as a tree, so no chain of additions is longer than rows / 64 / (256 / L) + 6. Rows that are not whole aligned
+// them as a tree, so no value goes through more than ceil(rows / (64 * 256 / L)) + 8 + log2(32 / L) additions that round (three in the tree, one a
+// round, the slots of a warp, eight warps, eight blocks): 14 for 8192 rows and L = 8, 16 for 4096 and L = 32. Rows that are not whole aligned
 // vectors go element by element (`vec` of a leaf is 0). Latency bounds it: three dependent rounds (rows, cluster, result) and the
 // launch. 2002 x 512 bf16 5.2 us as slabs and fold, 3.5 so; where the line lies: colsum_clusters in native/kernels.py.
 constexpr int COLSUM_GROUP = 32, COLSUM_CLUSTER = 8;
