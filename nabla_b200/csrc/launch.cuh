@@ -39,12 +39,15 @@ __device__ __forceinline__ void as_of_now(Pointer& p) {
   asm volatile("" : "+l"(global) : : "memory");
   p = static_cast<Pointer>(__cvta_global_to_generic(global));
 }
+// (`early` false, for every block of a grid: the next launch begins as these blocks end, which counts as much as saying so.)
 template <typename... Pointers>
-__device__ __forceinline__ void follow_grid(Pointers&... read) {
+__device__ __forceinline__ void follow_grid_when(bool early, Pointers&... read) {
   wait_for_previous_grid();
-  let_next_grid_start();
+  if (early) let_next_grid_start();
   (as_of_now(read), ...);
 }
+template <typename... Pointers>
+__device__ __forceinline__ void follow_grid(Pointers&... read) { follow_grid_when(true, read...); }
 
 // Adds the attribute to a launch whose attribute array has room for one more.
 inline void set_following(cudaLaunchConfig_t& cfg) {
