@@ -2757,6 +2757,15 @@ int nb_layernorm_bwd_nblocks(int rows, int D, int dtype) {
   return nb < 1 ? 1 : nb;
 }
 
+// Dynamic shared memory that lets no SM take more than its share of the `nb` blocks of `warps` warps, where registers (64 and 56 a thread) would:
+// blocks begin in the room that the launch ahead leaves, and pile up where it leaves it first. us in chains, before launches followed each other, piled up
+// and so: 100 x 4096 bf16 8.7, 10.7, 8.0; 4096 x 1536 fp32 22.1, 20.1, 16.4. Where all that fit are there the share is no help and shared memory
+// is lost to the L1: 16384 x 2048 with its forward pass 74.8 us, 75.9 so.
+static int ln_share(int nb, int warps, int dtype) {
+  const int share = (nb + 147) / 148, fit = 65536 / ((dtype ? 64 : 56) * 32 * warps);
+  return share < fit ? 227 * 1024 / (share + 1) + 1024 : 0;
+}
+
 int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* add, void* dx,
                      void* dgamma, void* dbeta, float* partial, int rows, int D, int dtype, void* stream) {
   if (rows <= 0) return 0;
@@ -2782,7 +2791,8 @@ int nb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const flo
       nb::launch_following(layernorm_bwd_fused_kernel<T, ADD>, nb, 128, 0, STREAM, (const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, \
                                                                  (const T*)add, (T*)dx, partial, rows, D);            \
     else {                                                                                                            \
-      const int rb = vpl < 8 ? 8 / vpl : 1, smem = 32 * vpl * rb * 16 * 2 * 2 * (ADD ? 3 : 2);                        \
+      const int rb = vpl < 8 ? 8 / vpl : 1, ring = 32 * vpl * rb * 16 * 2 * 2 * (ADD ? 3 : 2);                        \
+      const int share = ln_share(nb, vpl * rb, dtype), smem = ring > share ? ring : share;                                             \
       const auto kernel = layernorm_bwd_rows_kernel<T, ADD>;                                                          \
       if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
       nb::launch_following(kernel, nb, 32 * vpl * rb, smem, STREAM, (const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)add, (T*)dx, \

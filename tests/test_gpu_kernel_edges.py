@@ -1682,3 +1682,25 @@ def test_captured_leaves_run_beside_the_chain():
     h = nb.compile(step, cuda_graph=True, donate_argnums=(0,))
     h(wrap(xs[0].clone()), wrap(dys[0]), *map(wrap, p))
     assert not any(r.branch_steps for e in h._cache.values() for r in e.values() if hasattr(r, "branch_steps"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,D", [(1, 512), (100, 4096), (296, 3072), (297, 3072), (700, 1536), (5000, 1536), (2047, 1000), (601, 264)])
+@pytest.mark.parametrize("add", [False, True])
+def test_layer_norm_backward_of_less_than_a_chipful_of_blocks(rows, D, dtype, add):
+    """Grids whose blocks are kept apart by their shared memory and grids that are not, with and without a gradient that joins, twice in a row."""
+    from nabla_b200.native import kernels
+
+    if D > (2048 if dtype == torch.float32 else 4096):
+        pytest.skip("rows of at most 16 warps")
+    g = torch.Generator("cuda").manual_seed(rows + D)
+    x, dy, extra = ((torch.randn(rows, D, generator=g, device="cuda") + 0.1).to(dtype) for _ in range(3))
+    gamma = torch.randn(D, generator=g, device="cuda").to(dtype)
+    _, mean, rstd = kernels.layernorm_fwd(x, gamma, None, 1e-5)
+    d = x.double().requires_grad_(True)
+    w = gamma.double().requires_grad_(True)
+    dx64, dw64 = torch.autograd.grad(TF.layer_norm(d, (D,), w, None, 1e-5), (d, w), dy.double())
+    tol = 2.5e-3 if dtype == torch.bfloat16 else 2e-6         # stored to 2^-9 / 2^-24; sums of up to 5000 rows in fp32
+    for _ in range(2):
+        dx, dw, db = kernels.layernorm_bwd(dy, x, gamma, mean, rstd, add=extra if add else None)
+        assert _rel2(dx, dx64 + extra.double() if add else dx64) < tol and _rel2(dw, dw64) < tol and _rel2(db, dy.double().sum(0)) < tol
