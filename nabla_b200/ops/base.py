@@ -16,6 +16,7 @@ Execution happens later in ``execute``: the kernel runs once per locally held sh
 """
 from __future__ import annotations
 
+import functools
 import weakref
 from typing import Any, Sequence
 
@@ -63,6 +64,19 @@ def ensure_tensor(x: Any, like: Tensor | None = None) -> Tensor:
     return constant(x)
 
 
+@functools.lru_cache(None)
+def _snake_case(n: str) -> str:
+    """Name of an op of a class: a plan asks for the names of its nodes some thousand times."""
+    if n.endswith("Op"):
+        n = n[:-2]
+    out = []
+    for i, ch in enumerate(n):
+        if ch.isupper() and i and (not n[i - 1].isupper()):
+            out.append("_")
+        out.append(ch.lower())
+    return "".join(out)
+
+
 class Operation:
     """Base class of all ops. Subclasses implement ``kernel`` plus optional rules."""
 
@@ -75,17 +89,7 @@ class Operation:
     # ------------------------------------------------------------------ identity
     @property
     def name(self) -> str:
-        if self._name is not None:
-            return self._name
-        n = type(self).__name__
-        if n.endswith("Op"):
-            n = n[:-2]
-        out = []
-        for i, ch in enumerate(n):
-            if ch.isupper() and i and (not n[i - 1].isupper()):
-                out.append("_")
-            out.append(ch.lower())
-        return "".join(out)
+        return self._name if self._name is not None else _snake_case(type(self).__name__)
 
     def __repr__(self) -> str:
         return f"<op {self.name}>"
