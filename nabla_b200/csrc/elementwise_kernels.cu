@@ -239,7 +239,7 @@ __device__ __forceinline__ Acc warp_red(Acc a, int op) {
 template <typename T, typename O>
 __global__ void __launch_bounds__(256) row_reduce_kernel(const T* __restrict__ x, O* __restrict__ out, long long rows,
                                                         long long R, int op) {
-  nb::follow_grid(x);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS, x);
   constexpr int V = Vec<T>::N;
   const int lane = threadIdx.x & 31;
   for (long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (long long)gridDim.x * 8) {
@@ -341,7 +341,7 @@ constexpr int THIN_THREADS = 128, THIN_CHAINS = 8;
 template <typename T, int OP, int CH>
 __global__ void __launch_bounds__(THIN_THREADS) thin_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, long long outer,
                                                          int R, long long inner) {
-  nb::follow_grid(x);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS, x);
   constexpr int V = Vec<T>::N, U = 4, STEP = CH > U ? CH : U;
   const long long nv = inner / V, t = (long long)blockIdx.x * THIN_THREADS + threadIdx.x;
   if (t >= outer * nv) return;

@@ -129,9 +129,8 @@ __global__ void __launch_bounds__(128, VPL <= 4 || (VPL <= 8 && sizeof(T) == 4) 
                                                               const T* __restrict__ beta, T* __restrict__ y,
                                                               float* __restrict__ mean, float* __restrict__ rstd,
                                                               int rows, int D, float eps) {
-  // Thousands of blocks of four short rows each spend a fifth of their time on letting the next launch begin early: 40000 x 64 fp32 11.2 us so, 8.4
-  // without (9.0 before launches followed each other), bf16 11.4, 9.6; 16384 x 256 bf16 5.9, 5.3.
-  nb::follow_grid_when(VPL > 1 || gridDim.x <= 2048, x, gamma, beta);
+  // (of wider rows 16384 x 2048 24.2 us, 25.7 by ending)
+  nb::follow_grid_when(VPL > 1 || gridDim.x <= nb::MANY_BLOCKS, x, gamma, beta);
   constexpr int V = Vec<T>::N, P = V / 2;
   constexpr bool PAIRS = sizeof(T) == 2;             // (16384 x 1024 fp32 25.0 us one at a time, 27.4 two)
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -874,7 +873,7 @@ __global__ void __launch_bounds__(256) __cluster_dims__(1, COLSUM_CLUSTER, 1) co
 // ============================================================== softmax / log-softmax (last dim)
 template <typename T, bool LOG>
 __global__ void __launch_bounds__(256) softmax_kernel(const T* __restrict__ x, T* __restrict__ y, int rows, int D) {
-  nb::follow_grid(x);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS || D > 4096, x);
   __shared__ float sh[8];
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
@@ -919,7 +918,7 @@ template <typename T, bool WHOLE, bool WIDE>
 __global__ void __launch_bounds__(256) lse_pick_fwd_kernel(const T* __restrict__ logits,
                                                           const long long* __restrict__ tgt, float* __restrict__ lse_out,
                                                           float* __restrict__ picked, int rows, int D) {
-  nb::follow_grid(logits, tgt);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS || D > 4096, logits, tgt);
   __shared__ float sh[8];
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
@@ -978,7 +977,7 @@ __global__ void __launch_bounds__(256) lse_pick_bwd_kernel(const T* __restrict__
                                                           const float* __restrict__ lse, const float* __restrict__ g_lse,
                                                           const float* __restrict__ g_pick, T* __restrict__ dlogits,
                                                           int rows, int D) {
-  nb::follow_grid(logits, tgt, lse, g_lse, g_pick);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS || D > 4096, logits, tgt, lse, g_lse, g_pick);
   const int row = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, row, rows)) return;   // debug build: one block per row
   const T* xr = logits + (size_t)row * D;
@@ -1198,7 +1197,7 @@ template <typename T, bool ADD>
 __global__ void __launch_bounds__(128) embedding_gather_kernel(const T* __restrict__ table,
                                                               const long long* __restrict__ ids, const T* __restrict__ add,
                                                               T* __restrict__ out, int n_ids, int D, int vocab, int period) {
-  nb::follow_grid(table, ids, add);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS, table, ids, add);
   constexpr int V = Vec<T>::N;
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
@@ -1506,7 +1505,7 @@ template <typename T, int VN, bool ALL>
 __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(const T* __restrict__ upd, const T* __restrict__ base,
                                                           T* __restrict__ out, ScatWs ws, float* __restrict__ part, int n_ids,
                                                           int D, int vocab) {
-  nb::follow_grid(upd, base, part);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS, upd, base, part);
   __shared__ int last;
   const int total = *ws.nseg, lights = ALL ? *ws.nlight : 0;
   const int lane = threadIdx.x & 31, nwarps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1581,7 +1580,7 @@ __global__ void __launch_bounds__(256, VN == 8 ? 3 : 4) scatter_rows_kernel(cons
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) embedding_scatter_add_kernel(float* __restrict__ acc, const long long* __restrict__ ids,
                                                                    const T* __restrict__ upd, int n_ids, int D, int vocab) {
-  nb::follow_grid(acc, ids, upd);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS, acc, ids, upd);
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;   // debug build: one block per id
   const long long id = ids[i];
@@ -1612,7 +1611,7 @@ __global__ void __launch_bounds__(128) embedding_scatter_sorted_kernel(const lon
                                                                       const long long* __restrict__ perm,
                                                                       const T* __restrict__ upd, const T* __restrict__ base,
                                                                       T* __restrict__ out, int n_ids, int D, int vocab) {
-  nb::follow_grid(sorted_ids, perm, upd, base);
+  nb::follow_grid_when(gridDim.x <= nb::MANY_BLOCKS, sorted_ids, perm, upd, base);
   const int i = blockIdx.x;
   if (!NB_IN_BOUNDS(NB_SITE_ROW_INDEX, i, n_ids)) return;
   const long long id = sorted_ids[i];

@@ -39,7 +39,10 @@ __device__ __forceinline__ void as_of_now(Pointer& p) {
   asm volatile("" : "+l"(global) : : "memory");
   p = static_cast<Pointer>(__cvta_global_to_generic(global));
 }
-// (`early` false, for every block of a grid: the next launch begins as these blocks end, which counts as much as saying so.)
+// `early` false, for every block of a grid: the next launch begins as these blocks end, which counts as much as saying so. Thousands of small blocks
+// spend up to a third of their time on saying so. us in chains, before launches followed each other, with every block saying so, and by ending:
+// layer norm of 40000 x 64 fp32 9.0, 11.2, 8.4; 11368 rows of 256 fp32 from a table 8.2, 13.1, 7.2; gradient of the cross-entropy of 6410 x 100 bf16 5.8, 8.0, 5.4.
+constexpr unsigned MANY_BLOCKS = 2048;
 template <typename... Pointers>
 __device__ __forceinline__ void follow_grid_when(bool early, Pointers&... read) {
   wait_for_previous_grid();

@@ -77,7 +77,8 @@ def test_every_kernel_of_a_following_launch_waits_for_the_grid_ahead():
             if "gemm_cta<" in body:
                 assert "gemm_cta<BN, MODE_NONE" in body
                 body = cta
-            body = re.sub(r"follow_grid_when\(VPL > 1 \|\| gridDim.x <= 2048, ", "follow_grid(", body.replace("return follow_grid();", "follow_grid_and_leave;"))
+            body = re.sub(r"follow_grid_when\((?:VPL > 1 \|\| )?gridDim.x <= nb::MANY_BLOCKS(?: \|\| D > 4096)?, ", "follow_grid(",
+                          body.replace("return follow_grid();", "follow_grid_and_leave;"))
             if k == "attn_bwd_dq_kernel":             # works beside the kernel ahead of it: launch.cuh says on what grounds
                 beside = "  if (BESIDE) let_next_grid_start();\n  else follow_grid();\n"
                 assert body.count(beside) == 1 and "constexpr bool BESIDE = MASK != MASK_ROWS;" in body

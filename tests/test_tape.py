@@ -409,3 +409,35 @@ def test_calls_of_several_signatures_in_turn(graph, monkeypatch):
         check(k, xs[k])
         assert _taped(f)
     assert not by_python
+
+
+@pytest.mark.parametrize("rows,dim", [(2048, 96), (2049, 96), (8196, 96), (600, 8200)])
+def test_many_small_blocks_in_a_row(rows, dim):
+    """Grids that let the next launch begin by ending, and rows that begin when all ahead has ended, between others that do neither: thirty calls
+    in a row on changing inputs, against the same calls with a synchronisation after each."""
+    import nabla_b200 as nb
+    from nabla_b200.nn import functional as F
+
+    def fn(table, ids, a, b, t):
+        x = F.layer_norm(F.embedding(ids, table), a, b)
+        return (x, *nb.value_and_grad(lambda x: F.cross_entropy_loss(x, t), create_graph=False)(x), nb.softmax(x))
+
+    g = torch.Generator("cuda").manual_seed(rows)
+    table = torch.randn(500, dim, generator=g, device="cuda")
+    a, b = torch.ones(dim, device="cuda"), torch.zeros(dim, device="cuda")
+    sets = [(torch.randint(0, 500, (rows,), generator=g, device="cuda"), torch.randint(0, dim, (rows,), generator=g, device="cuda")) for _ in range(3)]
+    f, plain = nb.compile(fn), nb.compile(fn)
+    want = []
+    for i, t in sets:
+        want.append([x.clone() for x in _leaves(plain(*map(_wrap, (table, i, a, b, t))))])
+        torch.cuda.synchronize()
+    ids, tgt, got = sets[0][0].clone(), sets[0][1].clone(), []
+    for k in range(30):
+        ids.copy_(sets[k % 3][0])
+        tgt.copy_(sets[k % 3][1])
+        got.append(_leaves(f(*map(_wrap, (table, ids, a, b, tgt)))))
+    torch.cuda.synchronize()
+    for k, outs in enumerate(got):
+        assert all(torch.equal(x, y) for x, y in zip(outs, want[k % 3])), k
+    x = want[0][0].double()
+    assert torch.allclose(want[0][1].double(), torch.nn.functional.cross_entropy(x, sets[0][1]), rtol=1e-5)
