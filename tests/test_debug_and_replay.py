@@ -69,7 +69,7 @@ def test_every_kernel_of_a_following_launch_waits_for_the_grid_ahead():
             brace = src.index("{", kernel.end())
             params[kernel.group(1)] = src[kernel.end():brace]
             bodies[kernel.group(1)] = src[brace:src.index("\n}\n", brace)]
-        launched = set(re.findall(r"launch_(?:following\(|when\(following, )(\w+)", src)) - {"kernel", "ahead"}
+        launched = set(re.findall(r"launch_(?:following\(|when\((?:following|rows_follow\(rows, D\)), )(\w+)", src)) - {"kernel", "ahead"}
         launched |= {k for k in bodies if re.match(r"gemm_bf16_|layernorm_bwd_rows|attn_decode", k)}        # (through a pointer to the kernel)
         assert launched and launched <= set(bodies), name
         for k in launched:
