@@ -3324,11 +3324,14 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
   };
   const int low = dtype ? 7 : 15, wvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & low) == 0, yvec = F % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & low) == 0;
   const ConvPatches pp = conv_patches(g, vec, wvec && yvec);
+  // (as for the filter gradient: from 3e8 multiply-adds on following gains 0.4 % in the mean and may cost a quarter, 256 x 28 x 28 x 16 -> 16, 5 x 5 of
+  // stride 2, 55.4 and 70.7 us; a classifier's 256 x 14 x 14 x 16 -> 32, of 2.3e8, gains 1.5 us a launch in its step)
+  const bool following = (double)positions * F * R * S * C < 3e8;
   if (pp.px) {
     const int px = pp.px, th = pp.th, bands = pp.bands, fg_w = pp.fg;
     const size_t smem = 4 * ((size_t)R * S * C * 4 * fg_w + (size_t)((th - 1) * sh + R) * ((OW - 1) * sw + S) * C);
     const dim3 pgrid((unsigned)(N * bands), (unsigned)pp.f_tiles);
-#define PATCH_V(T, FG, PX, VEC) nb::launch_following(conv2d_patch_kernel<T, FG, PX, VEC>, pgrid, 128, smem, STREAM, (const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec, relu)
+#define PATCH_V(T, FG, PX, VEC) nb::launch_when(following, conv2d_patch_kernel<T, FG, PX, VEC>, pgrid, 128, smem, STREAM, (const T*)x, (const T*)w, (const T*)bias, (T*)y, g, th, bands, wvec, yvec, relu)
 #define PATCH_P(T, FG, PX) do { if (vec) PATCH_V(T, FG, PX, true); else PATCH_V(T, FG, PX, false); } while (0)
 #define PATCH(T, FG) do { if (px == 8) PATCH_P(T, FG, 8); else PATCH_P(T, FG, 4); } while (0)
     if (dtype) { if (fg_w == 2) PATCH(bf16, 2); else if (fg_w == 4) PATCH(bf16, 4); else PATCH(bf16, 8); }
@@ -3338,7 +3341,7 @@ int nb_conv2d_direct(const void* x, const void* w, const void* bias, void* y, in
 #undef PATCH_V
     return CHECK_LAUNCH();
   }
-#define CONV_V(T, FG, VEC) nb::launch_following(conv2d_direct_kernel<T, FG, VEC>, grid(FG), 128, 0, STREAM, (const T*)x, (const T*)w, (const T*)bias, (T*)y, g, relu)
+#define CONV_V(T, FG, VEC) nb::launch_when(following, conv2d_direct_kernel<T, FG, VEC>, grid(FG), 128, 0, STREAM, (const T*)x, (const T*)w, (const T*)bias, (T*)y, g, relu)
 #define CONV(T, FG) do { if (vec) CONV_V(T, FG, true); else CONV_V(T, FG, false); } while (0)
   if (dtype) { if (F <= 8) CONV(bf16, 2); else if (F <= 16) CONV(bf16, 4); else CONV(bf16, 8); }
   else { if (F <= 8) CONV(float, 2); else if (F <= 16) CONV(float, 4); else CONV(float, 8); }
@@ -3443,8 +3446,9 @@ int nb_conv2d_wgrad_direct(const void* x, const void* dy, void* dw, float* part,
   const long long total = (long long)N * bands, smem = pp.smem;
   const size_t dyn = smem < 8192 ? 8192 : (size_t)smem;    // (the sum of the position slices of a block takes 8 KB)
   // Long ones start evenly spread (see launch_when). 220 sizes in chains, behind the launch ahead and following it: below 1e7 multiply-adds 1.07 times the
-  // time, from 6e7 on 0.95 (64 x 56 x 56 x 32 -> 32, 3 x 3, 163 and 181 us; 256 x 16 x 16 x 4 -> 64, 5 x 5 of stride 2, 20.5 and 29.0).
-  const bool following = (double)positions * K * F < 6e7;
+  // time, from 4e7 on 0.95 (64 x 56 x 56 x 32 -> 32, 3 x 3, 163 and 181 us; 256 x 16 x 16 x 4 -> 64, 5 x 5 of stride 2, 20.5 and 29.0; 100 x 16 x 16 x
+  // 4 -> 64 17.4 and 21.0).
+  const bool following = (double)positions * K * F < 4e7;
 #define WGRAD_V(T, KG, FG, VEC)                                                                                                          \
   do {                                                                                                                                   \
     if (patch) nb::launch_when(following, conv2d_wgrad_patch_kernel<T, KG, FG, VEC>, dim3((K + 4 * KG - 1) / (4 * KG), (F + 4 * FG - 1) / (4 * FG), zp), 128, dyn, STREAM, (const T*)x, (const T*)dy, part, g, th, bands, (int)total, dvec); \

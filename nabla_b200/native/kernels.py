@@ -155,7 +155,7 @@ def colsum_clusters(rows: int, N: int, dtype: torch.dtype) -> int:
     and their fold pays until the slabs' many more blocks do (us, slabs + fold, 8, 32; bf16 unless said): 512 x 256 4.1, 3.3, 3.5;
     2002 x 512 5.2, 3.5, 5.4; 2002 x 2048 5.7, 4.2, 5.4, fp32 5.7, 6.5, 5.1; 8192 x 512 5.9, 5.1, 10.9; 4096 x 8192 10.8, 13.2,
     9.0, fp32 25.7, 37, 30; 16384 x 8192 44, 55, 52; 65536 x 256 17, 18, 63. Fewer than 16 tiles of 32 vectors leave a third of the chip idle, which
-    longer sums do not make up for: in chains 4096 x 3072 12.3, -, 13.6, fp32 4096 x 1536 11.3, -, 12.6, of 3000 rows 10.7, -, 10.8 and 10.1, -, 10.1. Rows that are not whole vectors took a
+    longer sums do not make up for: in chains 4096 x 3072 12.3, -, 13.6, fp32 4096 x 1536 11.3, -, 12.6, of 3000 rows 10.7, -, 10.8 and 9.5, -, 10.2. Rows that are not whole vectors took a
     cast, a sum and a cast, or in fp32 one sum: 512 x 10 5.4, 3.1, fp32 3.0, 2.9; 512 x 1 fp32 2.2, 2.9; 3000 x 777 24, 9.8, 5.6, fp32 11.6,
     8.9, 4.7. Of whole vectors no value goes through more additions that round than as slabs (counted for every number of rows and slabs); of
     others the sums are as near to 64 bits as the cast's."""
@@ -170,7 +170,7 @@ def colsum_clusters(rows: int, N: int, dtype: torch.dtype) -> int:
         return 0                                     # tall and narrow: slabs of a few rows at a time
     if -(-N // (8 * v)) <= 40:
         return 1
-    return 2 if rows <= (4096 if N >= 16 * 32 * v else 3000) and N <= (8192 if v == 8 else 2048) else 0
+    return 2 if rows <= (4096 if N >= 16 * 32 * v else 2500) and N <= (8192 if v == 8 else 2048) else 0
 
 
 def colsum_group(xs: list[torch.Tensor], out_dtype: torch.dtype | None = None, wide: bool = False) -> list[torch.Tensor]:
