@@ -181,7 +181,11 @@ except AttributeError:             # a torch build without CUDA
 
 def raw_stream(device: int) -> int:
     """Handle of the current stream of a GPU."""
-    return _raw_stream(device) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
+    return torch.cuda.current_stream(device).cuda_stream
+
+
+if _raw_stream is not None:
+    raw_stream = _raw_stream  # noqa: F811
 
 
 def stream_ptr() -> ctypes.c_void_p:

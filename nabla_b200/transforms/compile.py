@@ -52,6 +52,7 @@ from ..core.tensor.impl import TensorImpl
 from . import tape
 
 
+import functools as _functools
 import os as _os
 import threading as _threading
 
@@ -191,6 +192,7 @@ class _Recorded:
         self.constants: list[TensorImpl] = []       # values that follow from numbers alone, made with the plan
         self.constant_nodes: list[int] = []         # their nodes, in order
         self.owned: list[torch.Tensor] | None = None     # GPU tensors that go with the recording: its constants and the numbers in it
+        self.owned_on = 0                           # their device
         self.told: set[int] = set()                 # raw streams that the allocator knows to read them
         self.tape = None                            # of later calls without Python (transforms/tape.py); False: none
         self.tape_of_graph = False                  # it replays the graph
@@ -401,9 +403,10 @@ class CompiledFunction:
         """The call without Python in between, or NotImplemented."""
         handle, rec, graphs = taped
         if self.profile_ops or graphs is not self.use_cuda_graph or rec.tape is not handle \
-                or (rec.constants and torch.cuda.is_current_stream_capturing()):     # see _run
+                or (rec.constants and not rec.tape_of_graph and torch.cuda.is_current_stream_capturing()):     # see _run
             return NotImplemented
-        _tell_stream(rec)
+        if rec.owned is None or (rec.owned and native.raw_stream(rec.owned_on) not in rec.told):
+            _tell_stream(rec)
         out = tape.module().call(handle, args, config.is_deterministic())
         if out is not NotImplemented:
             for module, n in zip(_counted_modules(), rec.tape_counts):
@@ -979,16 +982,18 @@ def _tell_stream(rec: "_Recorded") -> None:
     if rec.owned is None:
         placeholders = {id(p) for p in rec.placeholders}
         numbers = [a for n in rec.nodes for a in n.input_impls() if a.literal is not None and id(a) not in placeholders and a._buffers]
-        rec.owned = list({id(b): b for a in [*rec.constants, *numbers] for b in a._buffers if b.is_cuda}.values())
+        owned = list({id(b): b for a in [*rec.constants, *numbers] for b in a._buffers if b.is_cuda}.values())
+        rec.owned_on = owned[0].device.index if owned else 0
+        rec.owned = owned
     if rec.owned:
-        index = rec.owned[0].device.index
-        stream = native.raw_stream(index)
+        stream = native.raw_stream(rec.owned_on)
         if stream not in rec.told and not torch.cuda.is_current_stream_capturing():
             for b in rec.owned:
                 b.record_stream(torch.cuda.current_stream(b.device))
             rec.told.add(stream)
 
 
+@_functools.lru_cache(None)                         # (a taped call asks)
 def _counted_modules() -> tuple:
     from ..native import attention, gemm, kernels
 
