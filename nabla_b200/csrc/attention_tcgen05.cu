@@ -1827,7 +1827,7 @@ extern "C" int nb_attn_fwd_splits(int B, int H, int Sq, int Skv, int D, int has_
 
 // Warps that a (batch, head) of the decode kernel is given in a cluster of blocks, which needs no scratch and no second launch (0: key
 // ranges as above). Timed for every number of warps and the ranges over 4 to 512 pairs, 128 to 8000 keys, one and two queries, both head_dims (826
-// sizes, calls in a row): as many warps as have eight keys each and as leave no cluster waiting for its turn. The lines:
+// sizes, calls in a row): as many warps as leave no cluster waiting for its turn, of four warps with eight keys each. The lines:
 //  - blocks of eight warps take few pairs, by 3 (one query) and 2 blocks an SM; a pair on 16 of them wants keys enough for the larger exchange.
 //  - of four warps 512 blocks load ahead, up to 800 do not, and those of larger clusters pay under more keys only. Two queries: 600 blocks.
 //  - ranges win where they fill the chip evenly and clusters do not (148 pairs x 4001 x 128 55 us, clusters 61), where clusters would leave it half

@@ -66,7 +66,7 @@ def _load():
         if m.built_for != replay_built_for():
             raise ImportError(f"it was built for {m.built_for}, this is {replay_built_for()}")
         m.classes(Tensor, TensorImpl)
-    except (ImportError, OSError, AttributeError) as e:
+    except (ImportError, OSError, AttributeError, TypeError) as e:
         warnings.warn(f"{path.name} cannot be used, compiled calls are replayed by Python (python -m nabla_b200.csrc.build builds it anew): {e}")
         return None
     return m

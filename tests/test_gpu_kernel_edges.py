@@ -1590,7 +1590,8 @@ def test_few_queries_over_clusters(B, H, Sq, Skv, D, warps):
 
 @pytest.mark.parametrize("bh,Sq,Skv,D,warps", [(148, 1, 2001, 128, 0), (149, 1, 2001, 128, 16), (128, 1, 901, 64, 16), (129, 1, 901, 64, 16), (96, 1, 999, 64, 16),
                                                (96, 1, 1001, 64, 32), (296, 1, 700, 64, 0), (297, 1, 700, 64, 8), (290, 1, 700, 64, 8), (400, 1, 700, 128, 8), (16, 1, 2999, 128, 64), (16, 1, 3000, 128, 128), (300, 1, 130, 64, 0),
-                                               (192, 2, 999, 64, 8), (192, 2, 1000, 64, 0), (24, 2, 8000, 128, 0)])
+                                               (192, 2, 999, 64, 8), (192, 2, 1000, 64, 0), (24, 2, 8000, 128, 0),
+                                               (48, 1, 300, 128, 64), (32, 2, 301, 128, 64), (1, 1, 1500, 64, 128)])
 def test_few_queries_by_what_fits_the_chip(bh, Sq, Skv, D, warps):
     """Grids that load ahead and that do not, in clusters (up to 512 blocks) and in ranges (592), one block to either side, against 64 bits."""
     from nabla_b200.native import attention
